@@ -49,9 +49,12 @@ constexpr int kUmmaK = 32;       // K elements one f8 MMA consumes
 constexpr int kRowTile = 128;    // MMA M
 constexpr int kATileBytes = kRowTile * kBK;   // 16 KiB
 constexpr int kMaxSmem = 232448;              // 227 KiB opt-in limit per CTA
+#ifndef BQ_STREAM_THREADS
+#define BQ_STREAM_THREADS 384
+#endif
+constexpr int kStreamThreads = BQ_STREAM_THREADS;   // weight-streaming kernel: warps 0 / 1 load and
+constexpr int kStreamWarps = kStreamThreads / 32;   // issue MMAs, ALL warps run the epilogue
 constexpr int kBarrierBytes = 1024;           // mbarriers + tmem slot + flags
-constexpr int kMaxArgmaxSlots = 768;          // greedy pick: pairs per batch row a launch may leave
-constexpr int kNoIndex = 0x7fffffff;          // greedy pick: "nothing yet", loses against any real column
 
 struct Segment {
   const float* sw;     // device: weight dequant scale
@@ -65,16 +68,16 @@ struct Segment {
                        // unquantized activation (kind::f16 MMA, no scales), 0 = e4m3 weight
   int y_tma;           // pair kernel: the output can be described to TMA (16-byte aligned base and pitch)
   int n;               // weight rows (output columns) of this segment
-  int tile_begin;      // pair kernel: index of the segment's first tile
-  int un;              // stream kernel: weight rows per unit (gate/up form: output columns per unit)
-  int unit_begin;      // stream kernel: index of the segment's first unit
-  int split;           // stream kernel: K slices with accumulators of their own
-  int wide;            // stream kernel: output (and residual) rows are 16-byte aligned
+  int tile_begin;      // tile kernel: index of the segment's first tile
+  int split;           // stream kernel: K slices of this weight (1, 2, 4 or 8)
+  int split_forced;    // stream kernel: non-zero = use this split instead of the shape rule
+  int cluster_begin;   // stream kernel: index of the segment's first cluster
 };
 
-// SiLU(gate)*up and the quantization of the product, done in the epilogue of ONE GEMM that
-// multiplies the gate rows and the up rows of the same output columns in one CTA (or pair) -- two
-// TMA boxes per pipeline stage, read from the two weights where they lie (the reference keeps gate_proj and up_proj as two tensors, braid/model/mlp.py:27-29; nothing is
+// SiLU(gate)*up and the quantization of the product, done in the epilogue of ONE GEMM whose
+// 128-row MMA tiles are put together from 64 gate rows and the 64 up rows of the same output
+// columns -- two TMA boxes per pipeline stage, read from the two weights where they lie (the
+// reference keeps gate_proj and up_proj as two tensors, braid/model/mlp.py:27-29; nothing is
 // repacked or copied).
 struct PairSilu {
   int on;
@@ -86,17 +89,18 @@ struct PairSilu {
   long long ld_hq;
   float* sh;               // device: the scale of h
   unsigned int* words;     // [0] amax bits [1] arrivals [2] departures ([3] is the sticky status)
+  unsigned int expected;   // CTAs that take part in the exchange (the active ones)
 };
 
-// Greedy pick fused into the lm_head GEMM: every epilogue thread keeps, for its batch row, the
-// largest of the logits it has seen over all units of its CTA -- taken after the rounding to the
+// Greedy pick fused into the lm_head GEMM: every CTA (one 128-row tile of the vocabulary, K not
+// split) reduces, per batch row, the largest of ITS 128 logits -- taken after the rounding to the
 // output type the logits tensor would have had, lowest index winning ties, NaN winning over
 // everything, which is `logits.argmax(-1)` as torch evaluates it -- and writes one (value,
-// index) pair at the end; a second, tiny kernel reduces the pairs of a row.
+// index) pair per row; a second, tiny kernel reduces the pairs of all tiles.
 struct ArgmaxOut {
   int on;
   int store_logits;          // 0 = the logits themselves are not written at all
-  uint2* partial;            // device: [slots][M] pairs {value as fp32 bits, vocabulary index}
+  uint2* partial;            // device: [tiles][M] pairs {value as fp32 bits, vocabulary index}
 };
 
 // a beats b: NaN first, then the larger value, then the lower index
@@ -131,14 +135,17 @@ struct GemmParams {
   int n_seg;
   const float* sx;     // device: activation dequant scale
   int M;               // activation rows
+  int mma_n;           // stream kernel: padded batch = MMA N (multiple of 16)
   int k_blocks;        // ceil(K / 128)
   int k_blocks_dense;  // stream kernel: 128-byte K blocks of a 16-bit row, ceil(2K / 128)
-  int flat;            // stream kernel: K is not a multiple of 128 bytes
   int dense_fmt;       // stream kernel: tcgen05 operand format of the 16-bit segments (0 f16, 1 bf16)
+  int cluster;         // stream kernel: CTAs per cluster = largest split of the launch
+  int stages;          // stream kernel: depth of the weight ring; pair kernel: pipeline depth
+  int b_stages;        // stream kernel: depth of the activation ring
   int out_dtype;
-  int m_tiles;         // pair kernel: tile rows
+  int m_tiles;         // tile kernel: ceil(M / 128)
   int pair_n;          // pair kernel, plain form: output columns per tile, 256 or 128
-  int total_tiles;     // pair kernel
+  int total_tiles;     // tile kernel
   unsigned int* status;
   ArgmaxOut argmax;
   unsigned long long* phase_ring;   // development builds (BQ_PHASES) only, else nullptr
@@ -159,18 +166,181 @@ __device__ __forceinline__ int find_segment(const GemmParams& p, int tile) {
   return s;
 }
 
+__device__ __forceinline__ void store_out4(void* y, long long idx, int out_dtype, float4 v) {
+  if (out_dtype == BQ_DTYPE_BF16) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y);
+    const __nv_bfloat162 hi = __floats2bfloat162_rn(v.z, v.w);
+    uint2 w;
+    w.x = *reinterpret_cast<const uint32_t*>(&lo);
+    w.y = *reinterpret_cast<const uint32_t*>(&hi);
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(y) + idx) = w;
+  } else if (out_dtype == BQ_DTYPE_F16) {
+    const __half2 lo = __floats2half2_rn(v.x, v.y);
+    const __half2 hi = __floats2half2_rn(v.z, v.w);
+    uint2 w;
+    w.x = *reinterpret_cast<const uint32_t*>(&lo);
+    w.y = *reinterpret_cast<const uint32_t*>(&hi);
+    *reinterpret_cast<uint2*>(static_cast<__half*>(y) + idx) = w;
+  } else {
+    *reinterpret_cast<float4*>(static_cast<float*>(y) + idx) = v;
+  }
+}
+
+struct EpilogueArgs {
+  const float* part;       // this CTA's staging buffer [mma_n][128] fp32
+  uint32_t part_addr;      // its shared-memory address
+  int peer0;               // cluster rank of K slice 0 of this tile
+  int m_begin, m_end;      // output rows this CTA reduces and writes
+  int warp, lane;
+  int row0;                // first weight row (output column) of the tile
+  float scale;
+  bool col_ok;
+  void* y;
+  long long ldy;
+  int out_dtype;
+  const void* res;
+  long long ld_res;
+  const PushParams* push;
+};
+
+// Four residual values of the output type, as raw bits (16 bytes cover the widest case).
+__device__ __forceinline__ uint4 load_res4(const void* res, long long idx, int out_dtype) {
+  uint4 r = make_uint4(0u, 0u, 0u, 0u);
+  if (out_dtype == BQ_DTYPE_F32) {
+    r = __ldg(reinterpret_cast<const uint4*>(static_cast<const float*>(res) + idx));
+  } else {
+    const uint2 h = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(res) + idx));
+    r.x = h.x; r.y = h.y;
+  }
+  return r;
+}
+
+// out = T(float(T(v)) + float(res)): the GEMM's own rounding, then the add's.
+__device__ __forceinline__ float4 add_res4(float4 v, uint4 raw, int out_dtype) {
+  if (out_dtype == BQ_DTYPE_BF16) {
+    const __nv_bfloat162 r0 = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
+    const __nv_bfloat162 r1 = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+    v.x = __bfloat162float(__float2bfloat16_rn(v.x)) + __bfloat162float(r0.x);
+    v.y = __bfloat162float(__float2bfloat16_rn(v.y)) + __bfloat162float(r0.y);
+    v.z = __bfloat162float(__float2bfloat16_rn(v.z)) + __bfloat162float(r1.x);
+    v.w = __bfloat162float(__float2bfloat16_rn(v.w)) + __bfloat162float(r1.y);
+  } else if (out_dtype == BQ_DTYPE_F16) {
+    const __half2 r0 = *reinterpret_cast<const __half2*>(&raw.x);
+    const __half2 r1 = *reinterpret_cast<const __half2*>(&raw.y);
+    v.x = __half2float(__float2half_rn(v.x)) + __half2float(r0.x);
+    v.y = __half2float(__float2half_rn(v.y)) + __half2float(r0.y);
+    v.z = __half2float(__float2half_rn(v.z)) + __half2float(r1.x);
+    v.w = __half2float(__float2half_rn(v.w)) + __half2float(r1.y);
+  } else {
+    // intrinsics: a plain + would be contracted with the scaling multiply into one fma
+    v.x = __fadd_rn(v.x, __uint_as_float(raw.x)); v.y = __fadd_rn(v.y, __uint_as_float(raw.y));
+    v.z = __fadd_rn(v.z, __uint_as_float(raw.z)); v.w = __fadd_rn(v.w, __uint_as_float(raw.w));
+  }
+  return v;
+}
+
+// Sums the SPLIT partial tiles of this CTA's rows in rank order (fixed order:
+// the result does not depend on timing) and stores them.  Every thread asks
+// for all the partials of a batch of rows before it uses any of them, so the
+// remote shared-memory latency is paid once per batch, not once per load.
+template <int SPLIT, bool RES>
+__device__ __forceinline__ void reduce_store(const EpilogueArgs& e) {
+  // rows in flight per thread (half as many when residual values are held as well)
+  constexpr int kRows = ((RES && SPLIT < 8) ? 8 / SPLIT : 16 / SPLIT) > (kStreamWarps > 8 ? 2 : 1)
+                            ? ((RES && SPLIT < 8) ? 8 / SPLIT : 16 / SPLIT) / (kStreamWarps > 8 ? 2 : 1)
+                            : 1;
+  constexpr int kWarps = kStreamWarps;
+  const int n4 = e.lane * 4;                 // 4 consecutive output columns
+  for (int m0 = e.m_begin + e.warp; m0 < e.m_end; m0 += kWarps * kRows) {
+    float4 v[kRows][SPLIT];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int m = m0 + i * kWarps;
+      if (m < e.m_end) {
+        const uint32_t off = e.part_addr + static_cast<uint32_t>(m * kRowTile + n4) * 4u;
+#pragma unroll
+        for (int r = 0; r < SPLIT; ++r) {
+          if constexpr (SPLIT == 1)
+            v[i][0] = *reinterpret_cast<const float4*>(e.part + m * kRowTile + n4);
+          else
+            v[i][r] = ld_cluster_f4(map_to_cta(off, e.peer0 + r));
+        }
+      }
+    }
+    uint4 rraw[RES ? kRows : 1];
+    if constexpr (RES) {
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        const int m = m0 + i * kWarps;
+        if (m < e.m_end && e.col_ok)
+          rraw[i] = load_res4(e.res, (long long)m * e.ld_res + e.row0 + n4, e.out_dtype);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int m = m0 + i * kWarps;
+      if (m < e.m_end) {
+        float4 acc = v[i][0];
+#pragma unroll
+        for (int r = 1; r < SPLIT; ++r) {
+          acc.x += v[i][r].x; acc.y += v[i][r].y; acc.z += v[i][r].z; acc.w += v[i][r].w;
+        }
+        acc.x *= e.scale; acc.y *= e.scale; acc.z *= e.scale; acc.w *= e.scale;
+        if constexpr (RES) {
+          if (e.col_ok) acc = add_res4(acc, rraw[i], e.out_dtype);
+        }
+        if (e.col_ok) {
+          if (e.push->n == 0) {
+            store_out4(e.y, (long long)m * e.ldy + e.row0 + n4, e.out_dtype, acc);
+          } else {
+            for (int d = 0; d < e.push->n; ++d)
+              store_out4(e.push->dst[d], (long long)m * e.push->ld + e.row0 + n4, e.out_dtype, acc);
+          }
+        }
+      }
+    }
+  }
+}
+
+// Per batch row of this CTA's share: the best of the tile's 128 logits (see ArgmaxOut).  K is
+// not split in an argmax launch, so the staged tile is final.
+template <typename T>
+__device__ __forceinline__ void argmax_rows(const EpilogueArgs& e, int n_total, uint2* partial_tile) {
+  using namespace bq::qd;
+  const int n4 = e.lane * 4;
+  for (int m = e.m_begin + e.warp; m < e.m_end; m += kStreamWarps) {
+    const float4 v = *reinterpret_cast<const float4*>(e.part + m * kRowTile + n4);
+    const float r[4] = {widen(narrow<T>(v.x * e.scale)), widen(narrow<T>(v.y * e.scale)),
+                        widen(narrow<T>(v.z * e.scale)), widen(narrow<T>(v.w * e.scale))};
+    float bv = 0.0f;
+    int bi = 0x7fffffff;                      // "nothing yet": loses against any real column
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int idx = e.row0 + n4 + j;
+      if (idx < n_total && (bi == 0x7fffffff || argmax_beats(r[j], idx, bv, bi))) { bv = r[j]; bi = idx; }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+      if (oi != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+    }
+    if (e.lane == 0) partial_tile[m] = make_uint2(__float_as_uint(bv), static_cast<unsigned int>(bi));
+  }
+}
+
 // Second stage of the greedy pick: one CTA per batch row reduces the pairs of all tiles.
 __global__ void __launch_bounds__(128) argmax_finish_kernel(const uint2* partial, int tiles, int M,
                                                             long long* idx_out) {
   pdl_wait_prior_grids();
   const int m = blockIdx.x;
   float bv = 0.0f;
-  int bi = kNoIndex;
+  int bi = 0x7fffffff;
   for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
     const uint2 pr = __ldcg(partial + static_cast<size_t>(t) * M + m);
     const float ov = __uint_as_float(pr.x);
     const int oi = static_cast<int>(pr.y);
-    if (oi != kNoIndex && (bi == kNoIndex || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+    if (oi != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
   }
   __shared__ float s_v[4];
   __shared__ int s_i[4];
@@ -178,13 +348,13 @@ __global__ void __launch_bounds__(128) argmax_finish_kernel(const uint2* partial
   for (int off = 16; off > 0; off >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
     const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-    if (oi != kNoIndex && (bi == kNoIndex || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+    if (oi != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
   }
   if ((threadIdx.x & 31) == 0) { s_v[threadIdx.x >> 5] = bv; s_i[threadIdx.x >> 5] = bi; }
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < 4; ++w)
-      if (s_i[w] != kNoIndex && (bi == kNoIndex || argmax_beats(s_v[w], s_i[w], bv, bi))) {
+      if (s_i[w] != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(s_v[w], s_i[w], bv, bi))) {
         bv = s_v[w];
         bi = s_i[w];
       }
@@ -192,7 +362,464 @@ __global__ void __launch_bounds__(128) argmax_finish_kernel(const uint2* partial
   }
 }
 
-#include "gemm_stream.cuh"
+// Interleaved gate/up tile: columns 0..63 of the tile are gate rows, 64..127 the up rows of the
+// same 64 output columns.  Sums the K slices like reduce_store, rounds both halves to the
+// activation type T exactly as the plain GEMM would have stored them, forms
+// h = T(T(silu(gate)) * up) (the two roundings of the separate torch kernels,
+// braid/model/mlp.py:48), and parks h (64 values of T per row) at the start of the row's
+// staging slot in THIS CTA's buffer -- rows of this CTA's share are read by no peer.
+// Lane L < 16 ends up with columns 4L, 4L+1; lane L+16 with 4L+2, 4L+3.  Returns max |h|.
+template <int SPLIT, typename T>
+__device__ __forceinline__ float silu_pair_rows(const EpilogueArgs& e, float scale_up, float* part_rw) {
+  using namespace bq::qd;
+  constexpr int kRows = ((SPLIT < 8) ? 8 / SPLIT : 1) > (kStreamWarps > 8 ? 2 : 1)
+                            ? ((SPLIT < 8) ? 8 / SPLIT : 1) / (kStreamWarps > 8 ? 2 : 1)
+                            : 1;
+  constexpr int kWarps = kStreamWarps;
+  const int n4 = e.lane * 4;
+  const bool up_half = e.lane >= 16;
+  const float sc = up_half ? scale_up : e.scale;
+  const int hcol = (e.lane & 15) * 4 + (up_half ? 2 : 0);
+  float mx = 0.0f;
+  for (int m0 = e.m_begin + e.warp; m0 < e.m_end; m0 += kWarps * kRows) {
+    float4 v[kRows][SPLIT];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int m = m0 + i * kWarps;
+      if (m < e.m_end) {
+        const uint32_t off = e.part_addr + static_cast<uint32_t>(m * kRowTile + n4) * 4u;
+#pragma unroll
+        for (int r = 0; r < SPLIT; ++r) {
+          if constexpr (SPLIT == 1)
+            v[i][0] = *reinterpret_cast<const float4*>(e.part + m * kRowTile + n4);
+          else
+            v[i][r] = ld_cluster_f4(map_to_cta(off, e.peer0 + r));
+        }
+      }
+    }
+    __syncwarp();   // every lane has its slice of the rows before any lane overwrites them
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int m = m0 + i * kWarps;    // warp-uniform
+      if (m < e.m_end) {
+        float4 acc = v[i][0];
+#pragma unroll
+        for (int r = 1; r < SPLIT; ++r) {
+          acc.x += v[i][r].x; acc.y += v[i][r].y; acc.z += v[i][r].z; acc.w += v[i][r].w;
+        }
+        // the value the plain GEMM would have stored: one rounding to T
+        const float r0 = widen(narrow<T>(acc.x * sc)), r1 = widen(narrow<T>(acc.y * sc));
+        const float r2 = widen(narrow<T>(acc.z * sc)), r3 = widen(narrow<T>(acc.w * sc));
+        const float got0 = __shfl_xor_sync(0xffffffffu, up_half ? r0 : r2, 16);
+        const float got1 = __shfl_xor_sync(0xffffffffu, up_half ? r1 : r3, 16);
+        const float g0 = up_half ? got0 : r0, g1 = up_half ? got1 : r1;
+        const float u0 = up_half ? r2 : got0, u1 = up_half ? r3 : got1;
+        const T s0 = silu_to<T>(g0);
+        const T s1 = silu_to<T>(g1);
+        const T h0 = narrow<T>(widen(s0) * u0);
+        const T h1 = narrow<T>(widen(s1) * u1);
+        mx = nan_max(mx, fabsf(widen(h0)));
+        mx = nan_max(mx, fabsf(widen(h1)));
+        T* hrow = reinterpret_cast<T*>(part_rw + m * kRowTile);
+        hrow[hcol] = h0;
+        hrow[hcol + 1] = h1;
+      }
+    }
+  }
+  return mx;
+}
+
+// After the grid-wide scale is known: cast the parked h of this CTA's rows and write the codes.
+template <typename T>
+__device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const float* part, float scale,
+                                               uint8_t* hq, long long ld_hq, int col0) {
+  using namespace bq::qd;
+  const ScaleDiv sc(scale);
+  const int hcol = (e.lane & 15) * 4 + (e.lane >= 16 ? 2 : 0);
+  for (int m = e.m_begin + e.warp; m < e.m_end; m += kStreamWarps) {
+    const T* hrow = reinterpret_cast<const T*>(part + m * kRowTile);
+    float f[2] = {widen(hrow[hcol]), widen(hrow[hcol + 1])};
+    divide_group<2, true>(sc, f);   // the scale is that of these very values
+    const uint32_t pair = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
+    *reinterpret_cast<uint16_t*>(hq + static_cast<long long>(m) * ld_hq + col0 + hcol) =
+        static_cast<uint16_t>(pair & 0xFFFFu);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Weight-streaming kernel (swap-AB, cluster split-K)
+// ---------------------------------------------------------------------------
+// Shared memory, after aligning the dynamic base to 1024 bytes:
+//   [stages x 16 KiB weight tiles][b_stages x (mma_n*128) activation tiles] ... [barrier block]
+// Two rings with their own barriers and their own producer thread.  The weight ring is as deep
+// as the shared memory allows: its tiles come from HBM, and the bytes in flight per SM are what
+// sets the streaming rate.  The activation ring is shallow (2 to 4 tiles at wide batches): its
+// tiles are L2 hits shared by every row tile, and a wide batch tile is as large as a weight
+// tile, so every activation slot given up is a weight tile more in flight.
+// The tile area is reused after the main loop as the fp32 staging buffer
+// part[m][128] that the cluster reduction reads.
+#ifndef BQ_STREAM_MIN_CTAS
+#define BQ_STREAM_MIN_CTAS 2
+#endif
+__global__ void __launch_bounds__(kStreamThreads, BQ_STREAM_MIN_CTAS)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xd,
+                   const __grid_constant__ WeightMaps tm_w, const __grid_constant__ GemmParams p,
+                   const int smem_tile_bytes) {
+  extern __shared__ uint8_t smem_dyn[];
+  const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+  uint8_t* const base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
+  const int b_tile_bytes = p.mma_n * kBK;
+  const uint32_t a_base = base;
+  const uint32_t b_base = base + p.stages * kATileBytes;
+  const uint32_t bar_base = base + smem_tile_bytes;          // 8-byte aligned
+  // barrier block: weight ring full / empty, activation ring full, accumulator.  One
+  // tcgen05.commit per K block: it arrives on the weight slot's "empty" barrier, and the
+  // activation producer watches the same barrier for the block whose activation slot it wants
+  // to refill.
+  const int n_bars = 2 * p.stages + p.b_stages;
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (p.stages + s); };
+  auto full_bar_b = [&](int s) { return bar_base + 8u * (2 * p.stages + s); };
+  const uint32_t accum_bar = bar_base + 8u * n_bars;
+  volatile uint32_t* const tmem_slot =
+      reinterpret_cast<volatile uint32_t*>(base_ptr + smem_tile_bytes + 8 * (n_bars + 1));
+  volatile uint32_t* const abort_flag = tmem_slot + 1;
+  float* const s_quant = reinterpret_cast<float*>(const_cast<uint32_t*>(tmem_slot) + 2);   // one float per warp
+
+  if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 0); }
+  pdl_launch_dependents();   // the next kernel may start its own set-up right away
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // A cluster of p.cluster CTAs works on p.cluster / split row tiles of one weight
+  // at a time: CTAs [g*split, (g+1)*split) of the cluster hold the K slices of
+  // tile g and reduce among themselves.
+  const int crank = (p.cluster > 1) ? static_cast<int>(cluster_ctarank()) : 0;
+  const int cluster_id = blockIdx.x / p.cluster;
+  int sg = 0;
+#pragma unroll
+  for (int i = 1; i < BQ_MAX_SEGMENTS; ++i)
+    if (i < p.n_seg && cluster_id >= p.seg[i].cluster_begin) sg = i;
+  const Segment seg = p.seg[sg];
+  const int split = seg.split;
+  const int group = crank / split;              // which tile of the cluster
+  const int krank = crank - group * split;      // which K slice of that tile
+  const int tile_in_seg = (cluster_id - seg.cluster_begin) * (p.cluster / split) + group;
+  const int row0 = tile_in_seg * kRowTile;
+  const bool active = row0 < seg.n;             // padding CTAs only keep the cluster barriers
+
+  // this CTA's K slice, balanced to within one block
+  // a 16-bit segment (a weight the reference keeps unquantized) walks 128-byte K blocks of
+  // 64 elements over the dense activation; everything else about the pipeline is the same
+  const bool dense = seg.dense != 0;
+  const int seg_k_blocks = dense ? p.k_blocks_dense : p.k_blocks;
+  const CUtensorMap* const x_map = dense ? &tm_xd : &tm_x;
+  const int kb_base = seg_k_blocks / split, kb_rem = seg_k_blocks % split;
+  const int kb_count = active ? kb_base + (krank < kb_rem ? 1 : 0) : 0;
+  const int kb_begin = krank * kb_base + (krank < kb_rem ? krank : kb_rem);
+
+  uint32_t tmem_cols = 32;
+  while (tmem_cols < static_cast<uint32_t>(p.mma_n)) tmem_cols <<= 1;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(x_map);
+    tma_prefetch_desc(&tm_w.w[sg]);
+    if (p.pair.on) tma_prefetch_desc(&tm_w.w[1]);
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int s = 0; s < p.b_stages; ++s) mbar_init(full_bar_b(s), 1);
+    mbar_init(accum_bar, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1 && active) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  if (threadIdx.x == 0) BQ_STAMP(p, 1);
+
+  if (!active) {
+    // nothing to multiply: it only matches the two cluster barriers of the working CTAs
+    if (p.cluster > 1) { cluster_sync_all(); cluster_sync_all(); }
+    return;
+  }
+
+  if (warp == 0) {
+    if (elect_one()) {
+      // Weights do not depend on any earlier kernel: this thread never waits for the kernel
+      // that produces the activation, it only follows the MMAs through the weight ring.
+      // weights are read once: evict first
+      const uint64_t pol_w = policy_evict_first();
+      // one 128-row box, or (paired gate/up) two 64-row boxes from the two weights
+      const bool paired = p.pair.on != 0;
+      const int half_row0 = tile_in_seg * (kRowTile / 2);
+      // slot and phase are carried along: an integer division by a run-time depth costs a
+      // single issuing thread more than the loads it issues
+      int s = 0;
+      uint32_t phase = 1;                      // parity of the completion that frees slot s
+      for (int i = 0; i < kb_count; ++i) {
+        if (i >= p.stages && !mbar_wait(empty_bar(s), phase)) {
+          *abort_flag = 1;
+          break;
+        }
+        mbar_expect_tx(full_bar(s), kATileBytes);
+        const int kx = (kb_begin + i) * kBK;
+        const uint32_t dst = a_base + s * kATileBytes;
+        if (paired) {
+          tma_load_2d(dst, &tm_w.w[0], full_bar(s), kx, half_row0, pol_w);
+          tma_load_2d(dst + kATileBytes / 2, &tm_w.w[1], full_bar(s), kx, half_row0, pol_w);
+        } else {
+          tma_load_2d(dst, &tm_w.w[sg], full_bar(s), kx, row0, pol_w);
+        }
+        if (++s == p.stages) { s = 0; phase ^= 1u; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    if (elect_one()) {
+      // the activation tile is shared by every row tile: keep it in L2
+      const uint64_t pol_x = policy_evict_last();
+      pdl_wait_prior_grids();   // the kernel that produces the activation has completed
+      BQ_STAMP(p, 2);
+      // Activation slot s was last read by the MMAs of block j = i - b_stages, whose completion
+      // is completion number j / stages of weight slot j % stages.  That barrier cannot complete
+      // a second time before this thread has looked: block j + stages >= i needs THIS load first
+      // (the host keeps b_stages <= stages).
+      int s = 0, js = 0;                       // activation slot of block i, weight slot of block j
+      uint32_t jphase = 0;                     // parity of completion j / stages
+      for (int i = 0; i < kb_count; ++i) {
+        if (i >= p.b_stages) {
+          if (!mbar_wait(empty_bar(js), jphase)) {
+            *abort_flag = 1;
+            break;
+          }
+          if (++js == p.stages) { js = 0; jphase ^= 1u; }
+        }
+        mbar_expect_tx(full_bar_b(s), b_tile_bytes);
+        tma_load_2d(b_base + s * b_tile_bytes, x_map, full_bar_b(s), (kb_begin + i) * kBK, 0, pol_x);
+        if (++s == p.b_stages) s = 0;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = dense ? idesc_f16(kRowTile, p.mma_n, p.dense_fmt)
+                                   : idesc_e4m3(kRowTile, p.mma_n);
+      int s = 0, sb = 0;
+      uint32_t phase = 0, phase_b = 0;
+      for (int i = 0; i < kb_count; ++i) {
+        if (!mbar_wait(full_bar(s), phase) || !mbar_wait(full_bar_b(sb), phase_b)) {
+          *abort_flag = 1;
+          break;
+        }
+        tc_fence_after();
+        if (i == 0) BQ_STAMP(p, 3);
+        const uint64_t da = smem_desc_sw128(a_base + s * kATileBytes);
+        const uint64_t db = smem_desc_sw128(b_base + sb * b_tile_bytes);
+#pragma unroll
+        for (int j = 0; j < kBK / kUmmaK; ++j) {
+          // +32 bytes along K inside the swizzle span = +2 in descriptor units (32 e4m3 or 16
+          // 16-bit elements: one MMA's K either way)
+          if (dense) mma_f16(tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
+          else mma_f8(tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
+        }
+        mma_commit(empty_bar(s));   // both slots are free once these MMAs retire
+        if (++s == p.stages) { s = 0; phase ^= 1u; }
+        if (++sb == p.b_stages) { sb = 0; phase_b ^= 1u; }
+      }
+      mma_commit(accum_bar);        // accumulator complete
+    }
+    __syncwarp();
+  }
+
+  // ---- epilogue: TMEM -> fp32 staging in shared memory ----------------------
+  pdl_wait_prior_grids();   // scales are read and outputs written only after this
+  // the epilogue warps get here at once and have the scale ready long before
+  // the accumulator is
+  const float sw = dense ? 1.0f : __ldg(seg.sw);
+  const float sx_ready = dense ? 1.0f : __ldg(p.sx);
+  bool ok = mbar_wait(accum_bar, 0);
+  tc_fence_after();
+  if (threadIdx.x == 0) BQ_STAMP(p, 4);
+  if (!ok) *abort_flag = 1;
+  __syncthreads();
+  ok = (*abort_flag == 0);
+  const float scale = sx_ready * sw;
+  float* const part = reinterpret_cast<float*>(base_ptr);   // [mma_n][128]
+  if (ok) {
+    // 8 warps: warp w reads TMEM lanes 32*(w%4).. (the only ones it may touch)
+    // and every other 16-column chunk, starting at chunk w/4
+    const int quad = warp & 3;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const int n_local = quad * 32 + lane;
+    for (int c = (warp >> 2) * 16; c < p.mma_n; c += 4 * kStreamWarps) {
+      uint32_t r[16];
+      tmem_ld16(lane_addr + c, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) part[(c + j) * kRowTile + n_local] = __uint_as_float(r[j]);
+    }
+  } else if (threadIdx.x == 0) {
+    atomicExch(p.status, (unsigned int)kErrDeviceWait);
+  }
+  tc_fence_before();
+  if (p.cluster > 1) cluster_sync_all(); else __syncthreads();
+  if (threadIdx.x == 0) BQ_STAMP(p, 5);
+
+  // ---- reduce the K slices in rank order and write this CTA's share of rows --
+  float pair_max = 0.0f;
+  const int per = (p.M + split - 1) / split;
+  const int m_begin = krank * per;
+  const int m_end = (m_begin + per < p.M) ? (m_begin + per) : p.M;
+  if (ok) {
+    const bool col_ok = (row0 + lane * 4) < seg.n;      // n is a multiple of 16
+    const uint32_t part_addr = smem_u32(part);
+    const int peer0 = group * split;
+    const EpilogueArgs ea{part, part_addr, peer0, m_begin, m_end, warp, lane, row0, scale, col_ok,
+                          seg.y, seg.ldy, p.out_dtype, seg.res, seg.ld_res, &p.push};
+    if (p.pair.on) {
+      const float scale_up = sx_ready * __ldg(p.pair.sw_up);
+      float mx;
+#define BQ_PAIR_ROWS(TT)                                                          \
+      switch (split) {                                                             \
+        case 1: mx = silu_pair_rows<1, TT>(ea, scale_up, part); break;             \
+        case 2: mx = silu_pair_rows<2, TT>(ea, scale_up, part); break;             \
+        case 4: mx = silu_pair_rows<4, TT>(ea, scale_up, part); break;             \
+        default: mx = silu_pair_rows<8, TT>(ea, scale_up, part); break;            \
+      }
+      if (p.out_dtype == BQ_DTYPE_BF16) { BQ_PAIR_ROWS(__nv_bfloat16) }
+      else if (p.out_dtype == BQ_DTYPE_F16) { BQ_PAIR_ROWS(__half) }
+      else { BQ_PAIR_ROWS(float) }
+#undef BQ_PAIR_ROWS
+      pair_max = mx;
+    } else if (p.argmax.on) {
+      uint2* const mine = p.argmax.partial + static_cast<size_t>(tile_in_seg) * p.M;
+      if (p.out_dtype == BQ_DTYPE_BF16) argmax_rows<__nv_bfloat16>(ea, seg.n, mine);
+      else if (p.out_dtype == BQ_DTYPE_F16) argmax_rows<__half>(ea, seg.n, mine);
+      else argmax_rows<float>(ea, seg.n, mine);
+      if (p.argmax.store_logits) reduce_store<1, false>(ea);
+    } else if (seg.res == nullptr) {
+      switch (split) {
+        case 1: reduce_store<1, false>(ea); break;
+        case 2: reduce_store<2, false>(ea); break;
+        case 4: reduce_store<4, false>(ea); break;
+        default: reduce_store<8, false>(ea); break;
+      }
+    } else {
+      switch (split) {
+        case 1: reduce_store<1, true>(ea); break;
+        case 2: reduce_store<2, true>(ea); break;
+        case 4: reduce_store<4, true>(ea); break;
+        default: reduce_store<8, true>(ea); break;
+      }
+    }
+  }
+  if (threadIdx.x == 0) BQ_STAMP(p, 6);
+  // nobody leaves while a peer may still read its staging buffer
+  if (p.cluster > 1) cluster_sync_all(); else __syncthreads();
+  if (p.pair.on && p.push.n > 0) {
+    // ---- column-parallel form: h itself goes to every rank's gathered buffer; the amax needs
+    // all ranks' shards and is taken by the quantizer that follows the exchange ----
+    __syncthreads();   // parked rows are complete
+    if (ok) {
+      const int col0 = tile_in_seg * (kRowTile / 2);
+      const int hcol = (lane & 15) * 4 + (lane >= 16 ? 2 : 0);
+      for (int m = m_begin + warp; m < m_end; m += kStreamWarps) {
+        const long long at = static_cast<long long>(m) * p.push.ld + col0 + hcol;
+        if (p.out_dtype == BQ_DTYPE_F32) {
+          const float2 v = *reinterpret_cast<const float2*>(part + m * kRowTile + hcol);
+          for (int d = 0; d < p.push.n; ++d)
+            *reinterpret_cast<float2*>(static_cast<float*>(p.push.dst[d]) + at) = v;
+        } else {
+          const uint32_t v = *reinterpret_cast<const uint32_t*>(
+              reinterpret_cast<const uint16_t*>(part + m * kRowTile) + hcol);
+          for (int d = 0; d < p.push.n; ++d)
+            *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.push.dst[d]) + at) = v;
+        }
+      }
+    }
+  } else if (p.pair.on) {
+    // ---- grid-wide max |h| -> scale -> codes of this CTA's rows (h is parked in `part`) ----
+    using namespace bq::qd;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+      pair_max = nan_max(pair_max, __shfl_xor_sync(0xffffffffu, pair_max, off));
+    if (lane == 0) s_quant[warp] = pair_max;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float w = s_quant[0];
+#pragma unroll
+      for (int i = 1; i < kStreamWarps; ++i) w = nan_max(w, s_quant[i]);
+      unsigned int* const words = p.pair.words;
+      if (p.pair.expected > 1) {
+        // an aborted CTA still arrives (with 0), so the others are not left waiting
+        atomicMax(&words[0], __float_as_uint(w));
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&words[1]) : "memory");
+        unsigned int amax_bits = 0, arrived = 0;
+        const long long t0 = clock64();
+        for (;;) {
+          asm volatile("ld.acquire.gpu.global.v2.u32 {%0, %1}, [%2];"
+                       : "=r"(amax_bits), "=r"(arrived)
+                       : "l"(words)
+                       : "memory");
+          if (arrived >= p.pair.expected) break;
+          if (clock64() - t0 > kSpinLimitCycles) {
+            atomicExch(p.status, (unsigned int)kErrDeviceWait);
+            break;
+          }
+        }
+        w = __uint_as_float(amax_bits);
+      }
+      const float sc = scale_from_amax(w);
+      if (blockIdx.x == 0) p.pair.sh[0] = sc;
+      s_quant[0] = sc;
+    }
+    __syncthreads();
+    const float sc = s_quant[0];
+    if (ok) {
+      const EpilogueArgs ea{part, smem_u32(part), 0, m_begin, m_end, warp, lane, row0, 0.0f, true,
+                            nullptr, 0, p.out_dtype, nullptr, 0, &p.push};
+      const int col0 = tile_in_seg * (kRowTile / 2);
+      if (p.out_dtype == BQ_DTYPE_BF16)
+        silu_pair_emit<__nv_bfloat16>(ea, part, sc, p.pair.hq, p.pair.ld_hq, col0);
+      else if (p.out_dtype == BQ_DTYPE_F16)
+        silu_pair_emit<__half>(ea, part, sc, p.pair.hq, p.pair.ld_hq, col0);
+      else
+        silu_pair_emit<float>(ea, part, sc, p.pair.hq, p.pair.ld_hq, col0);
+    }
+    if (threadIdx.x == 0 && p.pair.expected > 1) {
+      unsigned int* const words = p.pair.words;
+      const unsigned int old = atomicAdd(&words[2], 1u);
+      if (old == p.pair.expected - 1) {
+        words[0] = 0u; words[1] = 0u; words[2] = 0u;
+        __threadfence();
+      }
+    }
+  }
+  if (p.push.n > 0) {
+    // The stores of all threads of this CTA are ordered before thread 0's fence by the barrier
+    // (fences are cumulative); the fence orders them before this CTA's count; the last CTA sees
+    // every count, fences again and only then signals the ranks: every store of the launch
+    // happens before every arrival.
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence_system();
+      const unsigned int old = atomicAdd(p.push.done, 1u);
+      if (old == p.push.expected - 1u) {
+        *p.push.done = 0u;                       // ready for the next launch on this scratch
+        __threadfence_system();
+        for (int d = 0; d < p.push.n; ++d)
+          asm volatile("red.release.sys.global.add.u32 [%0], 1;" ::"l"(p.push.flag[d]) : "memory");
+      }
+    }
+  }
+  if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);
+  if (threadIdx.x == 0) BQ_STAMP(p, 7);
+}
 
 // Waits (bounded) until `flag` has counted `count` more arrivals than at the end of the
 // previous wait, i.e. until every CTA of every rank's push launch has stored its share into
@@ -329,44 +956,18 @@ template <typename T>
 __device__ __forceinline__ void silu16(const uint32_t (&g)[16], const uint32_t (&u)[16], float sg,
                                        float su, uint4 (&out)[sizeof(T) == 4 ? 4 : 2], float& mx) {
   using namespace bq::qd;
+  T h[16];
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    float gg[8], uu[8];
-    if constexpr (sizeof(T) == 2) {
-#pragma unroll
-      for (int i = 0; i < 8; i += 2) {
-        const int j = half * 8 + i;
-        const float2 a = unpack2<T>(pack2<T>(__uint_as_float(g[j]) * sg, __uint_as_float(g[j + 1]) * sg));
-        const float2 b = unpack2<T>(pack2<T>(__uint_as_float(u[j]) * su, __uint_as_float(u[j + 1]) * su));
-        gg[i] = a.x; gg[i + 1] = a.y;
-        uu[i] = b.x; uu[i + 1] = b.y;
-      }
-      gated_product<T, kSilu, 8>(gg, uu);
-      uint32_t w[4], m = 0u;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        w[i] = pack2<T>(gg[2 * i], gg[2 * i + 1]);
-        m = absmax2<T>(m, w[i]);
-      }
-      const float2 mm = unpack2<T>(m);
-      mx = nan_max(mx, mm.x);
-      mx = nan_max(mx, mm.y);
-      out[half] = make_uint4(w[0], w[1], w[2], w[3]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        gg[i] = __uint_as_float(g[half * 8 + i]) * sg;
-        uu[i] = __uint_as_float(u[half * 8 + i]) * su;
-      }
-      gated_product<T, kSilu, 8>(gg, uu);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) mx = nan_max(mx, fabsf(gg[i]));
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-        out[half * 2 + q] = make_uint4(__float_as_uint(gg[4 * q]), __float_as_uint(gg[4 * q + 1]),
-                                       __float_as_uint(gg[4 * q + 2]), __float_as_uint(gg[4 * q + 3]));
-    }
+  for (int i = 0; i < 16; ++i) {
+    const float gg = widen(narrow<T>(__uint_as_float(g[i]) * sg));
+    const float uu = widen(narrow<T>(__uint_as_float(u[i]) * su));
+    const T sl = silu_to<T>(gg);
+    h[i] = narrow<T>(widen(sl) * uu);
+    mx = nan_max(mx, fabsf(widen(h[i])));
   }
+  const uint4* raw = reinterpret_cast<const uint4*>(h);
+#pragma unroll
+  for (int q = 0; q < (sizeof(T) == 4 ? 4 : 2); ++q) out[q] = raw[q];
 }
 
 // The epilogue of one warp for one tile: 32 rows x 256 accumulator columns.  SILU: the tile's
@@ -737,25 +1338,6 @@ int make_map(CUtensorMap* out, const void* ptr, long long rows, long long K, int
   return rc == CUDA_SUCCESS ? kOk : kErrUnsupported;
 }
 
-// The same tensor seen as [K / 128][rows][128 bytes], so that one box brings `kb` K blocks of
-// box_rows rows (blocks beyond K read as zero): a box costs the copy engine 62 clocks however
-// few rows it has, which is more than the MMAs of one K block.  `flat` (K not a multiple of 128):
-// one K block per box, addressed by x.
-int make_map_kb(CUtensorMap* out, const void* ptr, long long rows, long long K, int box_rows, int kb, bool flat) {
-  EncodeTiledFn fn = encode_fn();
-  if (fn == nullptr) return kErrNoDriver;
-  const cuuint64_t dims[3] = {flat ? (cuuint64_t)K : (cuuint64_t)kBK, (cuuint64_t)rows,
-                              flat ? 1 : (cuuint64_t)(K / kBK)};
-  const cuuint64_t strides[2] = {(cuuint64_t)K, flat ? (cuuint64_t)K : (cuuint64_t)kBK};
-  const cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, (cuuint32_t)kb};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult rc = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims,
-                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return rc == CUDA_SUCCESS ? kOk : kErrUnsupported;
-}
-
 // [M, N] output of the prefill kernel, row pitch ldy elements: boxes of 32 rows x 128 bytes,
 // 128-byte swizzle; rows beyond M and columns beyond N are clipped by the store.
 int make_out_map(CUtensorMap* out, void* ptr, long long M, long long N, long long ldy, int out_dtype) {
@@ -787,14 +1369,12 @@ int device_sms() {
   return sms[dev];
 }
 
-long long g_opt_split = 0, g_opt_stages = 0, g_opt_stream_max_m = 256;
-long long g_opt_pair_from = 32;      // decode: batches above this many rows run on CTA pairs
+long long g_opt_split = 0, g_opt_stages = 0, g_opt_stream_max_m = 256, g_opt_cta_target = 160;
 long long g_opt_push_tma = 1;   // prefill push epilogue: bulk tensor stores (0: 16-byte plain stores)
 long long g_opt_pair_narrow = -1;   // prefill: 128-column tiles for a lone narrow weight (-1 auto, 0 never, 1 always)
 long long g_opt_pdl = 1;   // programmatic dependent launch on by default
-long long g_opt_b_stages = 0;   // activation ring depth: 0 = heuristic
+long long g_opt_b_stages = 0;   // activation ring depth: 0 = heuristic, -1 = as deep as the weight ring
 long long g_opt_smem_cap = 0;   // 0 = no cap on pipeline bytes per CTA
-thread_local int g_argmax_slots = 0;     // pairs per batch row the last stream launch wrote (greedy pick)
 thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
 
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
@@ -802,202 +1382,183 @@ inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintp
 int configure_once() {
   static int rc = -1;
   if (rc < 0) {
-    auto opt_in = [](auto kernel) {
-      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) == cudaSuccess;
-    };
-    rc = opt_in(gemm_stream_kernel<0>) && opt_in(gemm_stream_kernel<1>) && opt_in(gemm_stream_kernel<2>) &&
-                 opt_in(gemm_pair_kernel)
-             ? kOk : kErrLaunch;
+    cudaError_t e1 = cudaFuncSetAttribute(gemm_stream_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    cudaError_t e3 = cudaFuncSetAttribute(gemm_pair_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    rc = (e1 == cudaSuccess && e3 == cudaSuccess) ? kOk : kErrLaunch;
     if (rc != kOk) (void)cudaGetLastError();
   }
   return rc;
 }
 
-// CTA pairs of the stream kernel that are resident at once (one CTA per SM).
-int max_pairs() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (cached[dev] == 0) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(2, 1, 1);
-    cfg.blockDim = dim3(kStreamThreads, 1, 1);
-    cfg.dynamicSmemBytes = kMaxSmem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_stream_kernel<2>, &cfg) != cudaSuccess || clusters < 1) {
-      (void)cudaGetLastError();
-      clusters = device_sms() / 2;
-    }
-    cached[dev] = clusters;
+// Largest grid of the stream kernel that is resident at once with this cluster
+// size and shared-memory footprint (the paired gate/up epilogue has a grid-wide wait).
+int max_resident_ctas(int cluster, int smem) {
+  struct Entry { int cluster, smem, cap; };
+  static Entry cache[64];
+  static int n_cached = 0;
+  for (int i = 0; i < n_cached; ++i)
+    if (cache[i].cluster == cluster && cache[i].smem == smem) return cache[i].cap;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(cluster * 64), 1, 1);
+  cfg.blockDim = dim3(kStreamThreads, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_stream_kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    clusters = 0;
   }
-  return cached[dev];
+  // The occupancy calculator reports one CTA per SM for this kernel even where two
+  // demonstrably run side by side (all 256 CTAs of a 100 KB launch start within 1.3 us of
+  // each other), so the per-SM count is derived from the resources themselves: shared
+  // memory (1 KB reserved per CTA), registers, and the two-CTA cap of the launch bounds.
+  cudaFuncAttributes fa;
+  memset(&fa, 0, sizeof(fa));
+  int regs = 128;
+  if (cudaFuncGetAttributes(&fa, gemm_stream_kernel) == cudaSuccess && fa.numRegs > 0)
+    regs = fa.numRegs;
+  else
+    (void)cudaGetLastError();
+  int per_sm = 233472 / (smem + 1024);
+  const int by_regs = 65536 / (((regs + 7) / 8) * 8 * kStreamThreads);
+  if (per_sm > by_regs) per_sm = by_regs;
+  if (per_sm > 2) per_sm = 2;
+  if (per_sm < 1) per_sm = 1;
+  int cap = clusters * cluster * per_sm > 0 ? clusters * cluster * per_sm : -1;
+  if (getenv("BQ_DEBUG"))
+    fprintf(stderr, "[bq] residency: cluster %d smem %d regs %d -> %d clusters x %d per SM = %d CTAs\n",
+            cluster, smem, regs, clusters, per_sm, cap);
+  if (n_cached < 64) cache[n_cached++] = Entry{cluster, smem, cap};
+  return cap;
 }
 
-// K slices of one weight.  A function of the weight's own shape only -- never of what else shares
-// the launch or of the batch -- so an output element is summed in the same order whether its
-// weight is multiplied alone or grouped with others.
+// K slices of one weight.  A function of the weight's own shape only -- never of
+// what else shares the launch or of the batch -- so an output element is summed
+// in the same order whether its weight is multiplied alone or grouped with
+// others (`project` stays bit-identical to per-weight calls).  Small weights
+// are sliced so that their tiles x slices cover most of the SMs.
 int split_for_weight(long long n_rows, int k_blocks) {
   const long long tiles = (n_rows + kRowTile - 1) / kRowTile;
+  // at most 4: clusters of 8 leave a fifth of the SMs unusable (15 clusters of 8 fit on the
+  // 148 SMs, against 33 clusters of 4)
   int s = 1;
+  while (s < 4 && tiles * (s * 2) <= g_opt_cta_target && (s * 2) * 2 <= k_blocks) s *= 2;
   if (g_opt_split > 0) {
-    while (s * 2 <= g_opt_split && s < 8 && s * 2 <= k_blocks) s *= 2;
-  } else {
-    while (s < 4 && tiles * (s * 2) <= 160 && (s * 2) * 2 <= k_blocks) s *= 2;
+    s = 1;
+    while (s * 2 <= g_opt_split && s < 8) s *= 2;
+    while (s > 1 && s > k_blocks) s /= 2;
   }
   return s;
 }
 
-// How a launch of the stream kernel is laid out; the sums do not depend on any of it.
-int plan_stream(GemmParams& p, StreamShape& sh) {
+int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightMaps& maps,
+                  GemmParams& p, cudaStream_t stream) {
   const int sms = device_sms();
   if (sms <= 0) return kErrLaunch;
-  memset(&sh, 0, sizeof(sh));
-  const bool silu = p.pair.on != 0;
-  sh.mode = p.M > 128 ? 2 : (p.M > g_opt_pair_from ? 1 : 0);
-  const int cg = sh.mode == 0 ? 1 : 2;
-  sh.nm = silu ? 2 : 1;
-  sh.m_half = ((p.M + cg - 1) / cg + 7) / 8 * 8;
-  const int step = cg == 2 ? 32 : 16;                    // MMA N granularity
-  const int max_units = cg == 2 ? max_pairs() : sms;
-  if (max_units < 1) return kErrLaunch;
-  auto round_up = [&](int n) { return (n + step - 1) / step * step; };
-  // tensor-memory columns per weight row: a pair of 128 keeps half of a unit's columns in each half
-  // of the lanes
-  const int row_cols_x2 = sh.mode == 1 ? 1 : 2;
-  int buffers = 1;
-  for (int i = 0; i < p.n_seg; ++i)
-    p.seg[i].split = split_for_weight(p.seg[i].n, p.seg[i].dense ? p.k_blocks_dense : p.k_blocks);
-  auto seg_un = [&](const Segment& s, int un) {
-    int most = 1024 / (row_cols_x2 * buffers * sh.nm * s.split) / step * step;
-    if (most > 256) most = 256;
-    if (s.dense && round_up(s.n) < most) most = round_up(s.n);
-    return un < most ? un : most;
-  };
-  auto count = [&](int un) {
-    long long units = 0;
-    for (int i = 0; i < p.n_seg; ++i) units += (p.seg[i].n + seg_un(p.seg[i], un) - 1) / seg_un(p.seg[i], un);
-    return units;
-  };
-  // rows per unit: the fewest that make the launch one round; where one MMA (N <= 256) or tensor
-  // memory does not reach that far, two accumulators and the rows with the least padding
-  int un = 0;
-  for (int u = step; u <= 256; u += step)
-    if (count(u) <= max_units) { un = u; break; }
-  if (un == 0) {
-    if (silu) return kErrUnsupported;                    // h waits for a grid-wide exchange inside its CTA
-    buffers = 2;
-    long long best = 0;
-    for (int u = 256; u >= 64; u -= step) {
-      const long long cost = (count(u) + max_units - 1) / max_units * (u + 8);   // 8: what a round costs by itself
-      if (un == 0 || cost < best) { un = u; best = cost; }
-    }
-  }
-  const long long units = count(un);
-  if (units > 0x3fffffffLL) return kErrTooLarge;
-  sh.units = (int)units;
-  sh.rounds = (int)((units + max_units - 1) / max_units);
-  sh.grid = (int)(units < max_units ? units : max_units) * cg;
-  int at = 0, k_blocks[2] = {0, 0}, w_rows[2] = {0, 0};
+  p.mma_n = ((p.M + 15) / 16) * 16;
+  const int b_tile = p.mma_n * kBK;
+  const int stage_bytes = kATileBytes + b_tile;
+  int cluster = 1, min_split = 8;
   for (int i = 0; i < p.n_seg; ++i) {
-    Segment& s = p.seg[i];
-    s.un = seg_un(s, un);
-    s.unit_begin = at;
-    at += (s.n + s.un - 1) / s.un;
-    const int d = s.dense && sh.rounds == 1 ? 1 : 0;
-    const int kb = s.dense ? p.k_blocks_dense : p.k_blocks;
-    if (kb > k_blocks[d]) k_blocks[d] = kb;
-    if (s.un > w_rows[d]) w_rows[d] = s.un;
-    const int cols = s.un * row_cols_x2 / 2 * sh.nm * s.split;
-    if (cols > sh.acc_cols) sh.acc_cols = cols;
+    p.seg[i].split = p.seg[i].split_forced > 0 ? p.seg[i].split_forced
+                                               : split_for_weight(p.seg[i].n, p.seg[i].dense ? p.k_blocks_dense
+                                                                                             : p.k_blocks);
+    if (p.seg[i].split > cluster) cluster = p.seg[i].split;
+    if (p.seg[i].split < min_split) min_split = p.seg[i].split;
   }
-  sh.tmem_cols = 32;
-  while (sh.tmem_cols < sh.acc_cols * buffers) sh.tmem_cols *= 2;
-  if (sh.tmem_cols > 512) return kErrUnsupported;
-  sh.flat = p.flat;
-  const int budget = g_opt_smem_cap > 0 && g_opt_smem_cap < kMaxSmem - 1024 - kStreamBarrierBytes
-                         ? (int)g_opt_smem_cap : kMaxSmem - 1024 - kStreamBarrierBytes;
-  for (int d = 0; d < 2; ++d) {
-    if (w_rows[d] == 0) continue;
-    RingShape& r = sh.ring[d];
-    r.a_block = sh.m_half * kBK;
-    r.w_block = sh.nm * (w_rows[d] / cg) * kBK;
-    // a stage holds 16 KB of weights or more: what the issuing threads spend per stage is fixed
-    r.kb_stage = r.w_block >= 16384 || p.flat ? 1 : (r.w_block >= 8192 ? 2 : 4);
-    while (r.kb_stage > 1 && (r.kb_stage > k_blocks[d] || r.kb_stage * r.a_block > 32768)) r.kb_stage /= 2;
-    const int a_bytes = r.kb_stage * r.a_block, w_bytes = r.kb_stage * r.w_block;
-    const int want = (k_blocks[d] + r.kb_stage - 1) / r.kb_stage * sh.rounds;   // stages of a CTA's work
-    // 96 KB of activation tiles in flight, four stages at least: once the previous kernel is done every
-    // CTA walks the same tiles of L2 at the same time, and that latency under load is what a wide
-    // batch waits for (128 rows, 4096 x 12288: 16.9 / 14.3 / 13.4 us with 2 / 3 / 4 stages of 32 KB).
-    // The weight ring gets the rest; it streams at full rate from about 100 KB on.
-    int a_stages = 98304 / a_bytes;
-    if (a_stages < 4) a_stages = 4;
-    if (a_stages > 16) a_stages = 16;
-    if (g_opt_b_stages > 0) a_stages = (int)g_opt_b_stages;
-    if (a_stages > want) a_stages = want;
-    int w_stages = (budget - a_stages * a_bytes) / w_bytes;
-    if (w_stages > 40) w_stages = 40;
-    if (w_stages > want) w_stages = want;
-    if (g_opt_stages > 0 && w_stages > g_opt_stages) w_stages = (int)g_opt_stages;
-    if (w_stages < 1) return kErrUnsupported;
-    if (a_stages > w_stages) a_stages = w_stages;
-    r.a_stages = a_stages;
-    r.w_stages = w_stages;
-    // an MMA reads 64 or 128 rows from the start of any batch tile, whatever the batch
-    const int reach = (a_stages * r.kb_stage - 1) * r.a_block + (sh.mode == 2 ? 128 : 64) * kBK;
-    const int bytes = a_stages * a_bytes + w_stages * w_bytes;
-    if (bytes > sh.ring_bytes) sh.ring_bytes = bytes;
-    if (reach > sh.ring_bytes) sh.ring_bytes = reach;
+  p.cluster = cluster;
+  int clusters = 0;
+  for (int i = 0; i < p.n_seg; ++i) {
+    const int tiles = (p.seg[i].n + kRowTile - 1) / kRowTile;
+    const int per_cluster = cluster / p.seg[i].split;
+    p.seg[i].cluster_begin = clusters;
+    clusters += (tiles + per_cluster - 1) / per_cluster;
   }
-  if (w_rows[1] == 0) sh.ring[1] = sh.ring[0];
-  const int es = p.out_dtype == BQ_DTYPE_F32 ? 4 : 2;
-  if (silu && sh.ring_bytes < sh.m_half * (2 * un * es + 16)) sh.ring_bytes = sh.m_half * (2 * un * es + 16);
-  sh.ring_bytes = (sh.ring_bytes + 127) / 128 * 128;
-  if (sh.ring_bytes + kStreamBarrierBytes + 1024 > kMaxSmem) return kErrUnsupported;
-  return kOk;
-}
+  const long long grid = (long long)clusters * cluster;
+  if (grid > 0x7fffffffLL) return kErrTooLarge;
+  int kb_max = (p.k_blocks + min_split - 1) / min_split;
+  for (int i = 0; i < p.n_seg; ++i)
+    if (p.seg[i].dense) {
+      const int kb = (p.k_blocks_dense + p.seg[i].split - 1) / p.seg[i].split;
+      if (kb > kb_max) kb_max = kb;
+    }
+  const int staging = p.mma_n * kRowTile * 4;
+  // Shared memory per CTA: small enough that the whole grid is resident at once
+  // (up to 2 CTAs per SM: 256 threads x ~128 registers each), so one CTA's
+  // epilogue overlaps its neighbour's loads.
+  int per_sm = (int)((grid + sms - 1) / sms);
+  if (per_sm < 1) per_sm = 1;
+  if (per_sm > 2) per_sm = 2;
+  int budget = kMaxSmem / per_sm - 1024 - kBarrierBytes - 1024;
+  // Leave room for the NEXT kernel's CTAs: with programmatic dependent launch they
+  // become resident while this kernel still runs and pre-load their weights.
+  if (g_opt_smem_cap > 0 && budget > g_opt_smem_cap) budget = (int)g_opt_smem_cap;
+  int stages = budget / stage_bytes;            // both rings equally deep: the starting point
+  if (stages > kb_max) stages = kb_max;
+  if (stages > 24) stages = 24;
+  if (stages < 2) stages = kb_max < 2 ? kb_max : 2;
+  if (g_opt_stages > 0 && g_opt_stages < stages) stages = (int)g_opt_stages;
+  int b_stages = stages;
+  // Wide batch tiles: a shallow activation ring (its tiles are L2 hits), the rest goes to
+  // weight tiles in flight.  Two slots cover the L2 latency at the rate one CTA of a two-per-SM
+  // launch consumes tiles; a CTA that has the SM to itself consumes twice as fast.
+  long long want_b = g_opt_b_stages;
+  if (want_b == 0) want_b = b_tile >= 8192 ? (per_sm == 2 ? 2 : 4) : -1;
+  if (want_b > 0 && want_b < b_stages && !(g_opt_stages > 0)) {
+    b_stages = (int)want_b;
+    stages = (budget - b_stages * b_tile) / kATileBytes;
+    if (stages > kb_max) stages = kb_max;
+    if (stages > 24) stages = 24;
+    if (b_stages > stages) b_stages = stages;
+  }
+  p.stages = stages;
+  p.b_stages = b_stages;
+  int tile_bytes = stages * kATileBytes + b_stages * b_tile;
+  if (tile_bytes < staging) tile_bytes = staging;
+  const int smem = tile_bytes + kBarrierBytes + 1024;
+  if (smem > kMaxSmem) return kErrUnsupported;
+  if (p.pair.on) p.pair.expected = (unsigned)((p.seg[0].n / kRowTile) * p.seg[0].split);
+  if (p.push.n > 0)
+    p.push.expected = (unsigned)(((p.seg[0].n + kRowTile - 1) / kRowTile) * p.seg[0].split);
+  if (p.pair.on && p.push.n == 0) {
+    // the epilogue's amax exchange waits on the whole grid: every CTA must be resident
+    const int cap = max_resident_ctas(cluster, smem);
+    if (getenv("BQ_DEBUG"))
+      fprintf(stderr, "[bq] paired launch: grid %lld cluster %d smem %d resident cap %d\n", grid,
+              cluster, smem, cap);
+    if (cap <= 0 || grid > cap) return kErrUnsupported;
+  }
 
-int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightMaps& maps,
-                  GemmParams& p, const StreamShape& sh, cudaStream_t stream) {
-  const int smem = sh.ring_bytes + kStreamBarrierBytes + 1024;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)sh.grid, 1, 1);
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
   cfg.blockDim = dim3(kStreamThreads, 1, 1);
   cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  int n_attr = g_opt_pdl ? 1 : 0;
-  if (sh.mode > 0) {
-    attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-    attr[n_attr].val.clusterDim.x = 2;
-    attr[n_attr].val.clusterDim.y = 1;
-    attr[n_attr].val.clusterDim.z = 1;
-    ++n_attr;
-  }
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = n_attr;
-  g_last_launch[0] = 0; g_last_launch[1] = sh.grid; g_last_launch[2] = p.seg[0].split;
-  g_last_launch[3] = sh.ring[0].w_stages; g_last_launch[4] = smem; g_last_launch[5] = p.seg[0].un;
-  g_argmax_slots = (sh.mode > 0 ? sh.grid / 2 : sh.grid) * (sh.mode == 1 ? 2 : 1) *
-                   (sh.rounds > 1 ? (kStreamWarps - 4) / 4 : kStreamWarps / 4);
+  cfg.numAttrs = g_opt_pdl ? 2 : 1;
+  g_last_launch[0] = 0; g_last_launch[1] = grid; g_last_launch[2] = cluster;
+  g_last_launch[3] = stages; g_last_launch[4] = smem; g_last_launch[5] = p.mma_n;
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
 #endif
-  cudaError_t e;
-  if (sh.mode == 0) e = cudaLaunchKernelEx(&cfg, gemm_stream_kernel<0>, tm_x, tm_xd, maps, p, sh);
-  else if (sh.mode == 1) e = cudaLaunchKernelEx(&cfg, gemm_stream_kernel<1>, tm_x, tm_xd, maps, p, sh);
-  else e = cudaLaunchKernelEx(&cfg, gemm_stream_kernel<2>, tm_x, tm_xd, maps, p, sh);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_stream_kernel, tm_x, tm_xd, maps, p, tile_bytes);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
 }
@@ -1047,9 +1608,9 @@ int bq::gemm_set_option(const char* key, long long value) {
   if (strcmp(key, "push_tma") == 0) { g_opt_push_tma = value ? 1 : 0; return kOk; }
   if (strcmp(key, "pair_narrow") == 0) { g_opt_pair_narrow = value < 0 ? -1 : (value ? 1 : 0); return kOk; }
   if (strcmp(key, "decode_smem_cap") == 0) { g_opt_smem_cap = value; return kOk; }
-  if (strcmp(key, "decode_pair_from") == 0) {
-    if (value < 0 || value > 64) return kErrBadArg;
-    g_opt_pair_from = value;
+  if (strcmp(key, "decode_cta_target") == 0) {
+    if (value < 1) return kErrBadArg;
+    g_opt_cta_target = value;
     return kOk;
   }
   if (strcmp(key, "stream_max_m") == 0) {
@@ -1080,7 +1641,7 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
                 const int64_t* ldy, int out_dtype, void* ws, size_t ws_bytes, void* stream_v,
                 const void* const* res = nullptr,
                 const int64_t* ld_res = nullptr, const PairSilu* pair = nullptr,
-                const PushParams* push = nullptr,
+                int split_forced = 0, const PushParams* push = nullptr,
                 const DenseArgs* dn = nullptr, const ArgmaxOut* am = nullptr) {
   if (!xq || !sx || !wq || !sw || !y || !N || !ldy || M <= 0 || K <= 0) return kErrBadArg;
   if (n_seg < 1 || n_seg > BQ_MAX_SEGMENTS) return kErrBadArg;
@@ -1137,7 +1698,6 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   p.M = (int)M;
   p.k_blocks = (int)((K + kBK - 1) / kBK);
   p.k_blocks_dense = (int)((2 * K + kBK - 1) / kBK);
-  p.flat = K % kBK != 0;
   p.dense_fmt = (dn != nullptr && dn->dtype == BQ_DTYPE_BF16) ? 1 : 0;
   p.out_dtype = out_dtype;
   // the sticky status word is the 4th word of the scratch, as in the quantizer
@@ -1160,7 +1720,7 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   }
 
   const bool pair_path = !stream_path;
-  p.m_tiles = (int)((M + kPairTile - 1) / kPairTile);
+  p.m_tiles = pair_path ? (int)((M + kPairTile - 1) / kPairTile) : (int)((M + kRowTile - 1) / kRowTile);
   // plain prefill form of ONE narrow weight: 128-column tiles when all of them still run at once,
   // i.e. when 256-column ones would leave half of the CTA pairs without a tile (the sums are the
   // same, tile by tile; a 128-column tile takes 0.6-0.75 of a 256-column one, so a second round
@@ -1172,8 +1732,8 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     const bool narrow = g_opt_pair_narrow > 0 || (g_opt_pair_narrow < 0 && wide_tiles * 2 <= pairs);
     if (narrow) p.pair_n = kPairTile / 2;
   }
-  const int w_box_rows = pair == nullptr ? p.pair_n / 2 : kRowTile;
-  const int tile_n = pair ? kPairTile / 2 : p.pair_n;
+  const int w_box_rows = (pair_path && pair == nullptr) ? p.pair_n / 2 : kRowTile;
+  const int tile_n = pair_path ? ((pair && pair->prefill) ? kPairTile / 2 : p.pair_n) : kRowTile;
   OutMaps ymaps;
   memset(&ymaps, 0, sizeof(ymaps));
   int tiles = 0;
@@ -1182,68 +1742,50 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     const bool no_y = (pair && !pair->prefill) || push || (am != nullptr && !am->store_logits);
     p.seg[i].y = no_y ? nullptr : y[i];
     p.seg[i].ldy = no_y ? 0 : ldy[i];
+    p.seg[i].split_forced = split_forced;
     p.seg[i].res = res ? res[i] : nullptr;
     p.seg[i].ld_res = res ? ld_res[i] : 0;
     p.seg[i].n = (int)N[i];
     p.seg[i].dense = (dn != nullptr && dn->kind[i] != 0) ? 1 : 0;
     p.seg[i].tile_begin = tiles;
     const long long nt = (N[i] + tile_n - 1) / tile_n;
-    if (stream_path) {
-      const long long es = out_dtype == BQ_DTYPE_F32 ? 4 : 2;
-      bool wide = true;
-      if (push) {
-        wide = (push->ld * es) % 16 == 0;
-        for (int d = 0; d < push->n; ++d) wide = wide && aligned_to(push->dst[d], 16);
-      } else if (!no_y) {
-        wide = aligned_to(y[i], 16) && (ldy[i] * es) % 16 == 0;
-      }
-      if (p.seg[i].res) wide = wide && aligned_to(res[i], 16) && (ld_res[i] * es) % 16 == 0;
-      p.seg[i].wide = wide ? 1 : 0;
-      continue;
-    }
-    const long long add = nt * p.m_tiles;
+    const long long add = stream_path ? nt : nt * p.m_tiles;
     if (tiles + add > 0x3fffffffLL) return kErrTooLarge;
     tiles += (int)add;
-    if (!no_y) {
+    if (pair_path && !no_y) {
       const size_t es = out_dtype == BQ_DTYPE_F32 ? 4 : 2;
       p.seg[i].y_tma = aligned_to(y[i], 16) && (ldy[i] * es) % 16 == 0 &&
                        make_out_map(&ymaps.y[i], y[i], M, N[i], ldy[i], out_dtype) == kOk;
     }
-    if (push && g_opt_push_tma) {
+    if (pair_path && push && g_opt_push_tma) {
       // one map per destination rank over its [M, N shard] window (n_seg is 1 for a push)
       bool ok = true;
       for (int d = 0; d < push->n && ok; ++d)
         ok = make_out_map(&ymaps.y[d], push->dst[d], M, N[i], push->ld, out_dtype) == kOk;
       p.seg[i].y_tma = ok ? 1 : 0;
     }
-    if (pair) {
+    if (pair && pair->prefill) {
       // two maps over the two weights, 128-row boxes: one CTA of a pair loads gate rows, the other
       // the up rows of the same output columns
       if (int rc = make_map(&maps.w[0], wq[0], N[0], K, kRowTile)) return rc;
       if (int rc = make_map(&maps.w[1], pair->wq_up, N[0], K, kRowTile)) return rc;
-    } else if (int rc = make_map(&maps.w[i], wq[i], N[i], K, w_box_rows)) {
-      return rc;
+    } else if (pair) {
+      // two maps over the two weights, 64-row boxes: the kernel puts a tile together from both
+      if (int rc = make_map(&maps.w[0], wq[0], N[0] / 2, K, kRowTile / 2)) return rc;
+      if (int rc = make_map(&maps.w[1], pair->wq_up, N[0] / 2, K, kRowTile / 2)) return rc;
+    } else if (int rc = make_map(&maps.w[i], wq[i], N[i], p.seg[i].dense ? 2 * K : K, w_box_rows)) {
+      return rc;     // a 16-bit weight is described by its bytes: [N, 2K]
     }
   }
   p.total_tiles = tiles;
   CUtensorMap tm_x;
   if (stream_path) {
-    StreamShape sh;
-    if (int rc = plan_stream(p, sh)) return rc;
-    const int cg = sh.mode ? 2 : 1;
-    auto map = [&](CUtensorMap* m, const void* ptr, long long rows, bool dense, int box_rows) {
-      // a 16-bit operand is described by its bytes: [rows, 2K]
-      return make_map_kb(m, ptr, rows, dense ? 2 * K : K, box_rows, sh.ring[dense ? 1 : 0].kb_stage, sh.flat != 0);
-    };
-    for (int i = 0; i < n_seg; ++i)
-      if (int rc = map(&maps.w[i], wq[i], N[i], p.seg[i].dense != 0, p.seg[i].un / cg)) return rc;
-    if (pair)
-      if (int rc = map(&maps.w[1], pair->wq_up, N[0], false, p.seg[0].un / cg)) return rc;
-    if (int rc = map(&tm_x, xq, M, false, sh.m_half)) return rc;
+    const int mma_n = (int)(((M + 15) / 16) * 16);
+    if (int rc = make_map(&tm_x, xq, M, K, mma_n)) return rc;
     CUtensorMap tm_xd = tm_x;
     if (dn != nullptr)
-      if (int rc = map(&tm_xd, dn->x, M, true, sh.m_half)) return rc;
-    return launch_stream(tm_x, tm_xd, maps, p, sh, stream);
+      if (int rc = make_map(&tm_xd, dn->x, M, 2 * K, mma_n)) return rc;
+    return launch_stream(tm_x, tm_xd, maps, p, stream);
   }
   if (int rc = make_map(&tm_x, xq, M, K, kRowTile)) return rc;
   return launch_pair(tm_x, maps, ymaps, p, stream);
@@ -1271,7 +1813,7 @@ extern "C" int bq_project_mixed(const void* xq, const float* sx, const void* x_d
   if (out_dtype != dense_dtype) return kErrUnsupported;   // F.linear returns the activation's type
   const DenseArgs dn{x_dense, dense_dtype, kind};
   return run_grouped(xq, sx, M, K, n_seg, w, sw, y, N, ldy, out_dtype, ws, ws_bytes, stream_v,
-                     nullptr, nullptr, nullptr, nullptr, &dn);
+                     nullptr, nullptr, nullptr, 0, nullptr, &dn);
 }
 
 extern "C" int bq_gemm_w8a8(const void* xq, const void* wq, const float* sx, const float* sw,
@@ -1288,11 +1830,7 @@ extern "C" int bq_gemm_w8a8(const void* xq, const void* wq, const float* sx, con
 
 extern "C" size_t bq_lm_head_argmax_workspace_bytes(int64_t M, int64_t N) {
   if (M <= 0 || N <= 0) return 0;
-  // one pair per batch row and column group: at most three groups per CTA, at most one CTA per SM
-  // and per 16 weight rows (a CTA pair per 32)
-  const int64_t rows = (N + 15) / 16 + 1;
-  const int64_t slots = rows < kMaxArgmaxSlots / 3 ? 3 * rows : kMaxArgmaxSlots;
-  return static_cast<size_t>(slots) * static_cast<size_t>(M) * sizeof(uint2);
+  return static_cast<size_t>((N + kRowTile - 1) / kRowTile) * static_cast<size_t>(M) * sizeof(uint2);
 }
 
 extern "C" int bq_lm_head_argmax(const void* xq, const void* wq, const float* sx, const float* sw,
@@ -1313,9 +1851,11 @@ extern "C" int bq_lm_head_argmax(const void* xq, const void* wq, const float* sx
   void* ys[1] = {logits_or_null};
   const int64_t Ns[1] = {N};
   const int64_t ldys[1] = {ldy};
+  // K is not split: every tile's logits are final inside one CTA
   if (int rc = run_grouped(xq, sx, M, K, 1, wqs, sws, ys, Ns, ldys, out_dtype, ws, ws_bytes, stream,
-                           nullptr, nullptr, nullptr, nullptr, nullptr, &am))
+                           nullptr, nullptr, nullptr, 1, nullptr, nullptr, &am))
     return rc;
+  const int tiles = (int)((N + kRowTile - 1) / kRowTile);
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)M, 1, 1);
@@ -1326,7 +1866,7 @@ extern "C" int bq_lm_head_argmax(const void* xq, const void* wq, const float* sx
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_opt_pdl ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_finish_kernel, am.partial, g_argmax_slots, (int)M,
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_finish_kernel, am.partial, tiles, (int)M,
                                            reinterpret_cast<long long*>(idx_out));
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
@@ -1349,10 +1889,14 @@ extern "C" int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const
   const void* wqs[1] = {wq_gate};
   const float* sws[1] = {sw_gate};
   void* ys[1] = {nullptr};
-  const int64_t Ns[1] = {I};
+  const int64_t Ns[1] = {2 * I};
   const int64_t ldys[1] = {0};
+  // K slices as the gate weight alone would get them: every dot product is then summed in the
+  // order of the separate gate and up GEMMs
+  const int k_blocks = (int)((K + kBK - 1) / kBK);
+  const int split = (K > 0 && K <= 0x7fffff00LL) ? split_for_weight((int)I, k_blocks) : 1;
   return run_grouped(xq, sx, M, K, 1, wqs, sws, ys, Ns, ldys, act_dtype, ws, ws_bytes, stream,
-                     nullptr, nullptr, &pair);
+                     nullptr, nullptr, &pair, split);
 }
 
 extern "C" int bq_gate_up_silu_w8a8(const void* xq, const float* sx, const void* wq_gate,
@@ -1413,7 +1957,7 @@ extern "C" int bq_gemm_w8a8_push(const void* xq, const void* wq, const float* sx
   const int64_t Ns[1] = {N};
   const int64_t ldys[1] = {0};
   return run_grouped(xq, sx, M, K, 1, wqs, sws, ys, Ns, ldys, out_dtype, ws, ws_bytes, stream,
-                     nullptr, nullptr, nullptr, &push);
+                     nullptr, nullptr, nullptr, 0, &push);
 }
 
 extern "C" int bq_gate_up_silu_push_w8a8(const void* xq, const float* sx, const void* wq_gate,
@@ -1445,11 +1989,13 @@ extern "C" int bq_gate_up_silu_push_w8a8(const void* xq, const float* sx, const 
     pair.prefill = 1;
     const int64_t Ns[1] = {I};
     return run_grouped(xq, sx, M, K, 1, wqs, sws, ys, Ns, ldys, act_dtype, ws, ws_bytes, stream,
-                       nullptr, nullptr, &pair, &push);
+                       nullptr, nullptr, &pair, 0, &push);
   }
-  const int64_t Ns[1] = {I};
+  const int64_t Ns[1] = {2 * I};
+  const int k_blocks = (int)((K + kBK - 1) / kBK);
+  const int split = (K > 0 && K <= 0x7fffff00LL) ? split_for_weight(I, k_blocks) : 1;
   return run_grouped(xq, sx, M, K, 1, wqs, sws, ys, Ns, ldys, act_dtype, ws, ws_bytes, stream,
-                     nullptr, nullptr, &pair, &push);
+                     nullptr, nullptr, &pair, split, &push);
 }
 
 extern "C" int bq_wait_flag(const void* flag, void* seen, unsigned int count, void* status_word,

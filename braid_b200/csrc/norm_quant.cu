@@ -49,8 +49,6 @@ struct NormParams {
   int rows, cols;
   long long ld_x, ld_h;
   float eps;
-  unsigned long long* phase_ring;   // development builds (BQ_PHASES) only, else nullptr
-  int phase_seq;
 };
 
 template <typename T> struct Vec4 { T v[kVec]; };
@@ -78,13 +76,12 @@ __device__ __forceinline__ void store4(T* p, const Vec4<T>& v) {
 }
 
 template <typename T>
-__device__ __forceinline__ void emit4(const Vec4<T>& v, const ScaleDiv& sc, uint8_t* dst, bool live) {
+__device__ __forceinline__ void emit4(const Vec4<T>& v, const ScaleDiv& sc, uint8_t* dst) {
   float f[4] = {widen(v.v[0]), widen(v.v[1]), widen(v.v[2]), widen(v.v[3])};
   divide_group<4, true>(sc, f);   // the scale is that of these very values
   const uint32_t a = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
   const uint32_t b = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
-  const uint32_t w = (a & 0xFFFFu) | ((b & 0xFFFFu) << 16);
-  if (live) *reinterpret_cast<uint32_t*>(dst) = w;
+  *reinterpret_cast<uint32_t*>(dst) = (a & 0xFFFFu) | ((b & 0xFFFFu) << 16);
 }
 
 // Lane 0 of the warp ends up with the shuffle-down tree sum (the other lanes hold partial
@@ -100,7 +97,6 @@ __device__ __forceinline__ float warp_tree_sum(float s) {
 // ---------------------------------------------------------------------------------------------
 template <typename T, int VPT>
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormParams p) {
-  if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
   __shared__ float s_red[4];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -117,21 +113,12 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormP
       g[i][0] = f.x; g[i][1] = f.y; g[i][2] = f.z; g[i][3] = f.w;
     }
   }
-  // Pass 0 is a rehearsal on zeros while the CTA waits for the previous kernel anyway: the same
-  // instructions without a store, so that pass 1 finds them in the instruction cache.
-#pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-  const bool live = pass != 0;
+  bq::pdl_wait_prior_grids();
   Vec4<T> x[VPT];
-  if (live) {
-    bq::pdl_wait_prior_grids();
-    if (threadIdx.x == 0) BQ_STAMP(p, 2);
-  }
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = t + i * kNormThreads;
-    if (live && v < n_vec) x[i] = load4(xr + v * kVec);
-    else x[i] = Vec4<T>{};
+    if (v < n_vec) x[i] = load4(xr + v * kVec);
   }
   float s = 0.0f;
 #pragma unroll
@@ -169,7 +156,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormP
       }
     }
   }
-  if (live && p.h_out != nullptr) {
+  if (p.h_out != nullptr) {
     T* hr = reinterpret_cast<T*>(p.h_out) + static_cast<long long>(row) * p.ld_h;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -177,20 +164,16 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormP
       if (v < n_vec) store4(hr + v * kVec, x[i]);
     }
   }
-  if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
-  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), live));
-  if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
+  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
   const ScaleDiv dv(sc);
-  if (live && blockIdx.x == 0 && t == 0) p.scale[0] = sc;
+  if (blockIdx.x == 0 && t == 0) p.scale[0] = sc;
   uint8_t* qr = p.q + static_cast<long long>(row) * p.cols;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = t + i * kNormThreads;
-    if (v < n_vec) emit4(x[i], dv, qr + v * kVec, live);
-  }
+    if (v < n_vec) emit4(x[i], dv, qr + v * kVec);
   }
   grid_depart(static_cast<QuantWs*>(p.ws));
-  if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -301,8 +284,6 @@ struct GatedParams {
   int rows, heads;
   long long ld_y, ld_z;
   float eps;
-  unsigned long long* phase_ring;   // development builds (BQ_PHASES) only, else nullptr
-  int phase_seq;
 };
 
 constexpr int kHeadDim = 128;
@@ -311,28 +292,18 @@ constexpr int kMaxHeadsPerWarp = 8;    // up to 64 heads
 
 template <typename T, bool Y_F32, int HPW>
 __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_quant_kernel(const GatedParams p) {
-  if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x;
   const float4 gm = __ldg(reinterpret_cast<const float4*>(p.gamma) + lane);
   const float gmv[kVec] = {gm.x, gm.y, gm.z, gm.w};
-  // pass 0 is a rehearsal on zeros (see rmsnorm_quant_kernel)
-#pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-  const bool live = pass != 0;
+  bq::pdl_wait_prior_grids();
   Vec4<T> core[HPW];
   Vec4<T> gate[HPW];
-  if (live) {
-    bq::pdl_wait_prior_grids();
-    if (threadIdx.x == 0) BQ_STAMP(p, 2);
-  }
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
     const int head = warp + i * kGatedWarps;
-    core[i] = Vec4<T>{};
-    gate[i] = Vec4<T>{};
-    if (live && head < p.heads) {
+    if (head < p.heads) {
       const long long off = static_cast<long long>(head) * kHeadDim + lane * kVec;
       if constexpr (Y_F32) {
         // the reference rounds the scan output to the activation type first (gdn.py:383)
@@ -362,39 +333,32 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_quant_kernel(c
       // the three idle warps of the restated kernel contribute exact zeros
       const float sigma2 = __fdiv_rn(s, static_cast<float>(kHeadDim));
       const float rstd = rsqrtf(__fadd_rn(sigma2, p.eps));
-      float silu[kVec] = {widen(gate[i].v[0]), widen(gate[i].v[1]), widen(gate[i].v[2]), widen(gate[i].v[3])};
-      gate_group<T, kSilu, kVec>(silu);
 #pragma unroll
       for (int j = 0; j < kVec; ++j) {
         const T xn = narrow<T>(__fmul_rn(rstd, widen(core[i].v[j])));
-        const float h = __fmul_rn(__fmul_rn(gmv[j], widen(xn)), silu[j]);
+        const float zf = widen(gate[i].v[j]);
+        const float silu = __fdiv_rn(zf, 1.0f + expf(-zf));
+        const float h = __fmul_rn(__fmul_rn(gmv[j], widen(xn)), silu);
         core[i].v[j] = narrow<T>(h);
         m = nan_max(m, fabsf(widen(core[i].v[j])));
       }
     }
   }
-  if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
-  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), live));
-  if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
+  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
   const ScaleDiv dv(sc);
-  if (live && blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
+  if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
   uint8_t* qr = p.q + static_cast<long long>(row) * p.heads * kHeadDim;
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
     const int head = warp + i * kGatedWarps;
-    if (head < p.heads) emit4(core[i], dv, qr + head * kHeadDim + lane * kVec, live);
-  }
+    if (head < p.heads) emit4(core[i], dv, qr + head * kHeadDim + lane * kVec);
   }
   grid_depart(static_cast<QuantWs*>(p.ws));
-  if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
 // ---------------------------------------------------------------------------------------------
 template <typename Kernel, typename Params>
-int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t stream) {
-#ifdef BQ_PHASES
-  p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
-#endif
+int launch_rows(Kernel kernel, int rows, int threads, const Params& p, cudaStream_t stream) {
   // every CTA waits for every other: the whole grid must fit on the device at once
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -485,12 +449,12 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_scale_kernel(c
     s = __shfl_sync(0xffffffffu, s, 0);
     const float sigma2 = __fdiv_rn(s, static_cast<float>(kHeadDim));
     const float rstd = rsqrtf(__fadd_rn(sigma2, p.eps));
-    float silu[kVec] = {widen(gate.v[0]), widen(gate.v[1]), widen(gate.v[2]), widen(gate.v[3])};
-    gate_group<T, kSilu, kVec>(silu);
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
       const T xn = narrow<T>(__fmul_rn(rstd, widen(core.v[j])));
-      const float h = __fmul_rn(__fmul_rn(gmv[j], widen(xn)), silu[j]);
+      const float zf = widen(gate.v[j]);
+      const float silu = __fdiv_rn(zf, 1.0f + expf(-zf));
+      const float h = __fmul_rn(__fmul_rn(gmv[j], widen(xn)), silu);
       core.v[j] = narrow<T>(h);
       m = nan_max(m, fabsf(widen(core.v[j])));
     }
