@@ -22,7 +22,8 @@ struct QuantWs {
 // thread.  A single-CTA grid never touches global memory here.  Thread 0 of every
 // CTA of a multi-CTA grid owes the scratch a grid_depart() call afterwards; that
 // part is kept off the critical path on purpose.
-__device__ __forceinline__ float grid_amax(float m, QuantWs* ws) {
+// `live` = false: the CTA's own max without the exchange (a rehearsal pass, see norm_quant.cu).
+__device__ __forceinline__ float grid_amax(float m, QuantWs* ws, bool live = true) {
   __shared__ float s_warp[32];
   __shared__ float s_amax;
 #pragma unroll
@@ -36,7 +37,7 @@ __device__ __forceinline__ float grid_amax(float m, QuantWs* ws) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) w = nan_max(w, __shfl_xor_sync(0xffffffffu, w, off));
     if (lane == 0) {
-      if (gridDim.x == 1) {
+      if (gridDim.x == 1 || !live) {
         s_amax = w;
       } else {
         // |x| >= 0 or NaN with the sign cleared: the unsigned order of the bit

@@ -235,3 +235,45 @@ def test_norm_quant_survives_capture_and_replays_identically(Q):
     for e, r in zip(eager, outs):
         assert torch.equal(u8(e), u8(r))
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,dt", [(1, torch.bfloat16), (27, torch.float16), (128, torch.bfloat16)],
+                         ids=["1", "27-fp16", "128"])
+def test_norms_behind_a_running_gemm_read_its_output(Q, rows, dt):
+    """Launched back to back from a graph, the norm kernels start before the kernel that writes their
+    input has finished: they must see its output, not what the buffer held before."""
+    hidden = 2048
+    w1, w2 = (Q.quantize_weight((randn_cpu((hidden, hidden), seed=s, dtype=torch.bfloat16) * 0.05).cuda())
+              for s in (1, 2))
+    gamma, gamma_h = _gamma(hidden, 3), _gamma(128, 4)
+    x0 = randn_cpu((rows, hidden), seed=5, dtype=dt).cuda()
+    y = randn_cpu((rows, hidden), seed=6).cuda().float()
+
+    def chain(wait=lambda t: t):
+        x = x0
+        for _ in range(6):
+            z = wait(Q.linear(wait(Q.rms_norm_quant(x, gamma, EPS)), w1))
+            x = wait(Q.linear(wait(Q.gated_rms_norm_quant(y, z, gamma_h, EPS, 128)), w2, residual=x))
+        return z, x
+
+    def one_at_a_time(t):
+        torch.cuda.synchronize()
+        return t
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        chain()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain()
+    ref = chain(one_at_a_time)
+    for _ in range(10):
+        for t in out:
+            t.zero_()
+        graph.replay()
+        graph.replay()
+        for got, want in zip(out, ref):
+            assert torch.equal(u8(got), u8(want))
+    assert Q.device_status() == 0
