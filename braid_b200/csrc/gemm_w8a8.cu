@@ -956,18 +956,44 @@ template <typename T>
 __device__ __forceinline__ void silu16(const uint32_t (&g)[16], const uint32_t (&u)[16], float sg,
                                        float su, uint4 (&out)[sizeof(T) == 4 ? 4 : 2], float& mx) {
   using namespace bq::qd;
-  T h[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float gg = widen(narrow<T>(__uint_as_float(g[i]) * sg));
-    const float uu = widen(narrow<T>(__uint_as_float(u[i]) * su));
-    const T sl = silu_to<T>(gg);
-    h[i] = narrow<T>(widen(sl) * uu);
-    mx = nan_max(mx, fabsf(widen(h[i])));
+  for (int half = 0; half < 2; ++half) {
+    float gg[8], uu[8];
+    if constexpr (sizeof(T) == 2) {
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        const int j = half * 8 + i;
+        const float2 a = unpack2<T>(pack2<T>(__uint_as_float(g[j]) * sg, __uint_as_float(g[j + 1]) * sg));
+        const float2 b = unpack2<T>(pack2<T>(__uint_as_float(u[j]) * su, __uint_as_float(u[j + 1]) * su));
+        gg[i] = a.x; gg[i + 1] = a.y;
+        uu[i] = b.x; uu[i + 1] = b.y;
+      }
+      gated_product<T, kSilu, 8>(gg, uu);
+      uint32_t w[4], m = 0u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        w[i] = pack2<T>(gg[2 * i], gg[2 * i + 1]);
+        m = absmax2<T>(m, w[i]);
+      }
+      const float2 mm = unpack2<T>(m);
+      mx = nan_max(mx, mm.x);
+      mx = nan_max(mx, mm.y);
+      out[half] = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        gg[i] = __uint_as_float(g[half * 8 + i]) * sg;
+        uu[i] = __uint_as_float(u[half * 8 + i]) * su;
+      }
+      gated_product<T, kSilu, 8>(gg, uu);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx = nan_max(mx, fabsf(gg[i]));
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        out[half * 2 + q] = make_uint4(__float_as_uint(gg[4 * q]), __float_as_uint(gg[4 * q + 1]),
+                                       __float_as_uint(gg[4 * q + 2]), __float_as_uint(gg[4 * q + 3]));
+    }
   }
-  const uint4* raw = reinterpret_cast<const uint4*>(h);
-#pragma unroll
-  for (int q = 0; q < (sizeof(T) == 4 ? 4 : 2); ++q) out[q] = raw[q];
 }
 
 // The epilogue of one warp for one tile: 32 rows x 256 accumulator columns.  SILU: the tile's

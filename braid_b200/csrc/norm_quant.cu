@@ -495,12 +495,12 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_scale_kernel(c
     s = __shfl_sync(0xffffffffu, s, 0);
     const float sigma2 = __fdiv_rn(s, static_cast<float>(kHeadDim));
     const float rstd = rsqrtf(__fadd_rn(sigma2, p.eps));
+    float silu[kVec] = {widen(gate.v[0]), widen(gate.v[1]), widen(gate.v[2]), widen(gate.v[3])};
+    gate_group<T, kSilu, kVec>(silu);
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
       const T xn = narrow<T>(__fmul_rn(rstd, widen(core.v[j])));
-      const float zf = widen(gate.v[j]);
-      const float silu = __fdiv_rn(zf, 1.0f + expf(-zf));
-      const float h = __fmul_rn(__fmul_rn(gmv[j], widen(xn)), silu);
+      const float h = __fmul_rn(__fmul_rn(gmv[j], widen(xn)), silu[j]);
       core.v[j] = narrow<T>(h);
       m = nan_max(m, fabsf(widen(core.v[j])));
     }

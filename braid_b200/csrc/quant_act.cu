@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       for (int u = 0; u < kUnroll; ++u) {
         const unsigned long long g = (unsigned long long)g0 + (unsigned long long)u * nthreads;
         if (g < p.n_groups) {
-          apply_prologue<T, MODE>(a[u], b[MODE == kPlain ? 0 : u]);
+          apply_prologue<T, MODE, true>(a[u], b[MODE == kPlain ? 0 : u]);
           m = absmax8(a[u], m);
         }
       }
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       for (int u = 0; u < kUnroll; ++u) {
         const long long g = g0 + (long long)u * nthreads;
         if (g < (long long)p.n_groups) {
-          apply_prologue<T, MODE>(a[u], b[MODE == kPlain ? 0 : u]);
+          apply_prologue<T, MODE, true>(a[u], b[MODE == kPlain ? 0 : u]);
           emit8<T, PHASE == kBoth>(a[u], dv, p.q + static_cast<size_t>(g) * kGroup);
         }
       }
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(256) prologue_dense_kernel(const QParams p, T*
   for (unsigned long long g = blockIdx.x * blockDim.x + threadIdx.x; g < p.n_groups; g += nthreads) {
     Pack8<T> a, b;
     load_raw<T, MODE, false>(p, (unsigned int)g, a, b);
-    apply_prologue<T, MODE>(a, b);
+    apply_prologue<T, MODE, true>(a, b);
     m = absmax8(a, m);
     if constexpr (sizeof(T) == 4) {
       float4* dst = reinterpret_cast<float4*>(out + g * kGroup);

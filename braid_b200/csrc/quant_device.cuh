@@ -193,14 +193,91 @@ __device__ __forceinline__ float scale_from_amax(float amax) {
 
 // x / (1 + exp(-x)) and 1 / (1 + exp(-x)) rounded to T as torch evaluates F.silu and
 // torch.sigmoid of a T tensor on a CUDA device: fp32, expf, an IEEE division, one rounding.
-// (Taking ex2/rcp approximations wherever the rounding to a 16-bit T hides them, with the exact
-// instructions for values near a rounding tie, passed the exhaustive test but measured slower:
-// the guard and the divergent exact path cost what the approximations saved.)
 template <typename T> __device__ __forceinline__ T silu_to(float x) {
   return narrow<T>(__fdiv_rn(x, 1.0f + expf(-x)));
 }
 template <typename T> __device__ __forceinline__ T sigmoid_to(float x) {
   return narrow<T>(__fdiv_rn(1.0f, 1.0f + expf(-x)));
+}
+
+// The same two functions of N values, the rounding to T left to the caller.
+// For 16-bit T the division is a reciprocal estimate and one residual correction of the quotient
+// (q = x y, q + (x - d q) y; Markstein, IBM J. Res. Dev. 34(1), 1990): with |x| <= 80 the divisor lies
+// in [1, 2^116] and nothing leaves the normal range, and x takes only 65,536 values, all of which
+// were compared on the device: the fp32 quotients are the IEEE ones, bit for bit, for both
+// functions and both types.  (-0 needs the sign put back.)  Values beyond 80, infinities and NaN
+// take the division itself, decided once per group of N.  For the kernels that run the arithmetic
+// many times over; those of small decode batches run it once from a cold instruction cache, where
+// the shorter code of silu_to / sigmoid_to is the faster one (four graphed decoder layers of 27 fp16
+// rows: 291.4 us with them, 297.5 with this).
+__device__ __forceinline__ float corrected_quotient(float x, float d) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  const float q = __fmul_rn(x, y);
+  return copysignf(__fmaf_rn(__fmaf_rn(-d, q, x), y, q), x);
+}
+
+enum Gate { kSilu, kSigmoid };
+
+template <typename T, Gate G, int N>
+__device__ __forceinline__ void gate_group(float (&x)[N]) {
+  if constexpr (sizeof(T) == 2) {
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < N; ++i) ok = ok && fabsf(x[i]) <= 80.0f;
+    if (ok) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) x[i] = corrected_quotient(G == kSilu ? x[i] : 1.0f, 1.0f + expf(-x[i]));
+      return;
+    }
+  }
+  // rare for 16-bit types: kept rolled so that it costs little code
+#pragma unroll(sizeof(T) == 2 ? 1 : N)
+  for (int i = 0; i < N; ++i) x[i] = __fdiv_rn(G == kSilu ? x[i] : 1.0f, 1.0f + expf(-x[i]));
+}
+
+// two values rounded to a 16-bit T and packed, low half first
+template <typename T>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  if constexpr (std::is_same<T, __half>::value) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+template <typename T>
+__device__ __forceinline__ float2 unpack2(uint32_t w) {
+  if constexpr (std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+  else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+}
+// running |.| maximum of packed pairs, NaN-propagating; starts at 0
+template <typename T>
+__device__ __forceinline__ uint32_t absmax2(uint32_t m, uint32_t w) {
+  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+  const T2 r = __hmax2_nan(*reinterpret_cast<const T2*>(&m), __habs2(*reinterpret_cast<const T2*>(&w)));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// N values of `gated` pass through the gate function, are rounded to T, multiplied by `other` in fp32
+// and rounded again (the two roundings of the separate torch kernels).  Results in `gated`, as
+// values of T widened.
+template <typename T, Gate G, int N>
+__device__ __forceinline__ void gated_product(float (&gated)[N], const float (&other)[N]) {
+  gate_group<T, G, N>(gated);
+  if constexpr (sizeof(T) == 2) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const float2 s = unpack2<T>(pack2<T>(gated[i], gated[i + 1]));
+      const float2 h = unpack2<T>(pack2<T>(s.x * other[i], s.y * other[i + 1]));
+      gated[i] = h.x;
+      gated[i + 1] = h.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) gated[i] = gated[i] * other[i];
+  }
 }
 
 // Raw operands of one group: one 8-pack for the plain mode, two for the prologues.
@@ -226,9 +303,21 @@ __device__ __forceinline__ void load_raw(const QParams& p, unsigned int g, Pack8
 }
 
 // a <- the activation values (in place); plain mode is the identity.
-template <typename T, int MODE>
+// LARGE: the kernel runs this many times over (see gate_group).
+template <typename T, int MODE, bool LARGE = false>
 __device__ __forceinline__ void apply_prologue(Pack8<T>& a, const Pack8<T>& b) {
-  if constexpr (MODE != kPlain) {
+  if constexpr (MODE != kPlain && LARGE) {
+    float x[8], y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      // the operand of the gate function first: gate of SiLU(gate) * up, gate of o * sigmoid(gate)
+      x[i] = widen(MODE == kSiluMul ? a.v[i] : b.v[i]);
+      y[i] = widen(MODE == kSiluMul ? b.v[i] : a.v[i]);
+    }
+    gated_product<T, MODE == kSiluMul ? kSilu : kSigmoid, 8>(x, y);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a.v[i] = narrow<T>(x[i]);   // exact: values of T already
+  } else if constexpr (MODE != kPlain) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       if constexpr (MODE == kSiluMul) {
