@@ -100,6 +100,33 @@ def _weight_scale(t: torch.Tensor) -> torch.Tensor:
 _CAST_CHUNK_BYTES = 256 * 2 ** 20
 
 
+def _quantize_weight_fused(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor] | None:
+    """Codes and scale of a weight from the activation quantizer's kernel: one launch that reads the
+    weight from memory once (a second time from L2 where it is larger than shared memory) instead of
+    two reductions, a division, a clamp and a conversion through fp32 temporaries.  A 12288 x 4096
+    bf16 weight: 485 -> 50 us; its 150 MB take 22.7 us at 6.65 TB/s.  Scale and codes are the
+    bits of the torch spelling: both take max |w| / 448 and divide.
+
+    `None` -- the torch spelling -- for whatever the kernel does not take: no CUDA tensor of the current
+    device, another type, a strided or unaligned view, a weight that records gradients, a tensor
+    subclass (tracing), no library, a capture before the scratch exists, or the parity arm."""
+    if (type(w) not in (torch.Tensor, torch.nn.Parameter) or not w.is_cuda or w.dtype not in _DTYPE_CODE
+            or not w.is_contiguous() or w.data_ptr() % 16 or w.numel() == 0 or _quantizers_off()
+            or (w.requires_grad and torch.is_grad_enabled())
+            or w.device.index != torch.cuda.current_device()):
+        return None
+    try:
+        lib = _require_lib()
+        slot = _take_slot(w.device, counted=False)
+    except (OSError, RuntimeError):
+        return None
+    q = torch.empty(w.shape, dtype=FP8, device=w.device)
+    scale = torch.empty((1, 1), dtype=torch.float32, device=w.device)
+    rc = lib.bq_quantize_act(w.data_ptr(), _DTYPE_CODE[w.dtype], w.numel(), q.data_ptr(), scale.data_ptr(),
+                             slot, 16, _stream_ptr(w.device))
+    return (q, scale) if rc == 0 else None
+
+
 def quantize_weight(w: torch.Tensor) -> FP8Weight:
     """`[N, K]` -> e4m3 + one per-tensor scale, once, at load (braid/model/quant.py:139-154)."""
     if w.dim() != 2:
@@ -109,6 +136,9 @@ def quantize_weight(w: torch.Tensor) -> FP8Weight:
         raise ValueError(
             f"_scaled_mm needs both weight dims to be multiples of 16; got "
             f"[{N}, {K}]. Leave this projection in bf16.")
+    fused = _quantize_weight_fused(w)
+    if fused is not None:
+        return FP8Weight(data=fused[0], scale=fused[1], shape=(N, K))
     scale = _weight_scale(w)
     data = torch.empty((N, K), dtype=FP8, device=w.device)
     rows = max(1, min(N, _CAST_CHUNK_BYTES // (K * 4)))
@@ -215,13 +245,14 @@ def _scratch_for(device_index: int) -> torch.Tensor:
     return buf
 
 
-def _take_slot(device: torch.device) -> int:
-    """Device address of the next scratch slot of this device."""
+def _take_slot(device: torch.device, counted: bool = True) -> int:
+    """Device address of the next scratch slot of this device.  `counted` = False: the launch is not one
+    of the forward path that `launch_count` reports (loading a weight)."""
     global _launches
     idx = device.index if device.index is not None else torch.cuda.current_device()
     buf = _scratch_for(idx)
     with _LOCK:
-        _launches += 1
+        _launches += counted
         slot = _next_slot[idx]
         _next_slot[idx] = (slot + 1) % _SLOTS
     return buf.data_ptr() + slot * _SLOT_BYTES

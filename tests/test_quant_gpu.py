@@ -396,3 +396,27 @@ def test_bad_arguments_raise(Q):
         Q.silu_mul_quant(torch.zeros(4, 12, device="cuda", dtype=torch.bfloat16),
                          torch.zeros(4, 12, device="cuda", dtype=torch.bfloat16))
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", DTYPES, ids=DT_IDS)
+@pytest.mark.parametrize("shape", [(16, 16), (272, 1040), (4096, 4096), (12288, 4096)])
+def test_quantize_weight_gives_the_bits_of_the_torch_spelling(Q, dt, shape):
+    """One launch against the parity arm, infinities and NaN included; strided views keep the torch
+    spelling."""
+    w = randn_cpu(shape, seed=shape[0], dtype=dt, scale=0.02).cuda()
+    cases = [w, w * 1e-3, torch.zeros_like(w), w[:, : shape[1] // 32 * 16] if shape[1] > 16 else w.t()]
+    for bad in (float("inf"), float("nan")):
+        v = w.clone()
+        v[shape[0] // 2, 3] = bad
+        cases.append(v)
+    for i, v in enumerate(cases):
+        got = Q.quantize_weight(v)
+        assert (Q._quantize_weight_fused(v) is not None) == v.is_contiguous()
+        try:
+            Q.warm_fused(False)
+            want = Q.quantize_weight(v)
+        finally:
+            Q.warm_fused(True)
+        assert got.shape == want.shape and got.data.shape == want.data.shape
+        assert torch.equal(u8(got.scale), u8(want.scale)), f"{dt} {shape} case {i}"
+        assert torch.equal(u8(got.data), u8(want.data)), f"{dt} {shape} case {i}"
