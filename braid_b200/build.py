@@ -27,7 +27,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libbraid_b200.so"
 SOURCES = ("quant_act.cu", "norm_quant.cu", "gemm_w8a8.cu", "cabi.cu")
-HEADERS = (CSRC / "ptx.cuh", CSRC / "quant_device.cuh", CSRC / "grid_amax.cuh",
+HEADERS = (CSRC / "ptx.cuh", CSRC / "gemm_wide.cuh", CSRC / "quant_device.cuh", CSRC / "grid_amax.cuh",
            PKG.parent / "include" / "braid_b200.h")
 
 

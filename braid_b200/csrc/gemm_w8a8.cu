@@ -55,6 +55,7 @@ constexpr int kMaxSmem = 232448;              // 227 KiB opt-in limit per CTA
 constexpr int kStreamThreads = BQ_STREAM_THREADS;   // weight-streaming kernel: warps 0 / 1 load and
 constexpr int kStreamWarps = kStreamThreads / 32;   // issue MMAs, ALL warps run the epilogue
 constexpr int kBarrierBytes = 1024;           // mbarriers + tmem slot + flags
+constexpr int kNoIndex = 0x7fffffff;          // greedy pick: "nothing yet", loses against any real column
 
 struct Segment {
   const float* sw;     // device: weight dequant scale
@@ -72,6 +73,9 @@ struct Segment {
   int split;           // stream kernel: K slices of this weight (1, 2, 4 or 8)
   int split_forced;    // stream kernel: non-zero = use this split instead of the shape rule
   int cluster_begin;   // stream kernel: index of the segment's first cluster
+  int un;              // wide kernel: weight rows per unit (gate/up form: output columns per unit)
+  int unit_begin;      // wide kernel: index of the segment's first unit
+  int wide;            // wide kernel: output (and residual) rows are 16-byte aligned
 };
 
 // SiLU(gate)*up and the quantization of the product, done in the epilogue of ONE GEMM whose
@@ -313,17 +317,17 @@ __device__ __forceinline__ void argmax_rows(const EpilogueArgs& e, int n_total, 
     const float r[4] = {widen(narrow<T>(v.x * e.scale)), widen(narrow<T>(v.y * e.scale)),
                         widen(narrow<T>(v.z * e.scale)), widen(narrow<T>(v.w * e.scale))};
     float bv = 0.0f;
-    int bi = 0x7fffffff;                      // "nothing yet": loses against any real column
+    int bi = kNoIndex;                      // "nothing yet": loses against any real column
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int idx = e.row0 + n4 + j;
-      if (idx < n_total && (bi == 0x7fffffff || argmax_beats(r[j], idx, bv, bi))) { bv = r[j]; bi = idx; }
+      if (idx < n_total && (bi == kNoIndex || argmax_beats(r[j], idx, bv, bi))) { bv = r[j]; bi = idx; }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
       const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-      if (oi != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+      if (oi != kNoIndex && (bi == kNoIndex || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
     }
     if (e.lane == 0) partial_tile[m] = make_uint2(__float_as_uint(bv), static_cast<unsigned int>(bi));
   }
@@ -335,12 +339,12 @@ __global__ void __launch_bounds__(128) argmax_finish_kernel(const uint2* partial
   pdl_wait_prior_grids();
   const int m = blockIdx.x;
   float bv = 0.0f;
-  int bi = 0x7fffffff;
+  int bi = kNoIndex;
   for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
     const uint2 pr = __ldcg(partial + static_cast<size_t>(t) * M + m);
     const float ov = __uint_as_float(pr.x);
     const int oi = static_cast<int>(pr.y);
-    if (oi != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+    if (oi != kNoIndex && (bi == kNoIndex || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
   }
   __shared__ float s_v[4];
   __shared__ int s_i[4];
@@ -348,13 +352,13 @@ __global__ void __launch_bounds__(128) argmax_finish_kernel(const uint2* partial
   for (int off = 16; off > 0; off >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
     const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-    if (oi != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+    if (oi != kNoIndex && (bi == kNoIndex || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
   }
   if ((threadIdx.x & 31) == 0) { s_v[threadIdx.x >> 5] = bv; s_i[threadIdx.x >> 5] = bi; }
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < 4; ++w)
-      if (s_i[w] != 0x7fffffff && (bi == 0x7fffffff || argmax_beats(s_v[w], s_i[w], bv, bi))) {
+      if (s_i[w] != kNoIndex && (bi == kNoIndex || argmax_beats(s_v[w], s_i[w], bv, bi))) {
         bv = s_v[w];
         bi = s_i[w];
       }
@@ -1325,6 +1329,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
+#include "gemm_wide.cuh"
+
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -1364,6 +1370,25 @@ int make_map(CUtensorMap* out, const void* ptr, long long rows, long long K, int
   return rc == CUDA_SUCCESS ? kOk : kErrUnsupported;
 }
 
+// The same tensor seen as [K / 128][rows][128 bytes], so that one box brings `kb` K blocks of
+// box_rows rows (blocks beyond K read as zero): a box costs the copy engine 62 clocks however
+// few rows it has, which is more than the MMAs of one K block.  `flat` (K not a multiple of 128):
+// one K block per box, addressed by x.
+int make_map_kb(CUtensorMap* out, const void* ptr, long long rows, long long K, int box_rows, int kb, bool flat) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return kErrNoDriver;
+  const cuuint64_t dims[3] = {flat ? (cuuint64_t)K : (cuuint64_t)kBK, (cuuint64_t)rows,
+                              flat ? 1 : (cuuint64_t)(K / kBK)};
+  const cuuint64_t strides[2] = {(cuuint64_t)K, flat ? (cuuint64_t)K : (cuuint64_t)kBK};
+  const cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, (cuuint32_t)kb};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult rc = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims,
+                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return rc == CUDA_SUCCESS ? kOk : kErrUnsupported;
+}
+
 // [M, N] output of the prefill kernel, row pitch ldy elements: boxes of 32 rows x 128 bytes,
 // 128-byte swizzle; rows beyond M and columns beyond N are clipped by the store.
 int make_out_map(CUtensorMap* out, void* ptr, long long M, long long N, long long ldy, int out_dtype) {
@@ -1396,11 +1421,13 @@ int device_sms() {
 }
 
 long long g_opt_split = 0, g_opt_stages = 0, g_opt_stream_max_m = 256, g_opt_cta_target = 160;
+long long g_opt_wide = -1;   // decode: CTA-pair kernel (-1 by batch, 0 never, 1 always)
 long long g_opt_push_tma = 1;   // prefill push epilogue: bulk tensor stores (0: 16-byte plain stores)
 long long g_opt_pair_narrow = -1;   // prefill: 128-column tiles for a lone narrow weight (-1 auto, 0 never, 1 always)
 long long g_opt_pdl = 1;   // programmatic dependent launch on by default
 long long g_opt_b_stages = 0;   // activation ring depth: 0 = heuristic, -1 = as deep as the weight ring
 long long g_opt_smem_cap = 0;   // 0 = no cap on pipeline bytes per CTA
+thread_local int g_argmax_slots = 0;     // pairs per batch row the last launch wrote (greedy pick)
 thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
 
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
@@ -1412,7 +1439,11 @@ int configure_once() {
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     cudaError_t e3 = cudaFuncSetAttribute(gemm_pair_kernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    rc = (e1 == cudaSuccess && e3 == cudaSuccess) ? kOk : kErrLaunch;
+    cudaError_t e4 = cudaFuncSetAttribute(gemm_wide_kernel<1>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    cudaError_t e5 = cudaFuncSetAttribute(gemm_wide_kernel<2>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    rc = (e1 == cudaSuccess && e3 == cudaSuccess && e4 == cudaSuccess && e5 == cudaSuccess) ? kOk : kErrLaunch;
     if (rc != kOk) (void)cudaGetLastError();
   }
   return rc;
@@ -1581,10 +1612,186 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   cfg.numAttrs = g_opt_pdl ? 2 : 1;
   g_last_launch[0] = 0; g_last_launch[1] = grid; g_last_launch[2] = cluster;
   g_last_launch[3] = stages; g_last_launch[4] = smem; g_last_launch[5] = p.mma_n;
+  g_argmax_slots = (p.seg[0].n + kRowTile - 1) / kRowTile;   // one pair per row tile
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
 #endif
   const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_stream_kernel, tm_x, tm_xd, maps, p, tile_bytes);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
+  return kOk;
+}
+
+// CTA pairs of the wide kernel that are resident at once (one CTA per SM).
+int max_pairs() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (cached[dev] == 0) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(2, 1, 1);
+    cfg.blockDim = dim3(kWideThreads, 1, 1);
+    cfg.dynamicSmemBytes = kMaxSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_wide_kernel<2>, &cfg) != cudaSuccess || clusters < 1) {
+      (void)cudaGetLastError();
+      clusters = device_sms() / 2;
+    }
+    cached[dev] = clusters;
+  }
+  return cached[dev];
+}
+
+// How a launch of the wide kernel is laid out; the sums do not depend on any of it.
+// kErrUnsupported: no one-round layout of a form that needs one, or a shape that leaves no room for
+// the rings; the K-sliced kernel takes those.
+int plan_wide(GemmParams& p, WideShape& sh, bool flat) {
+  memset(&sh, 0, sizeof(sh));
+  const bool silu = p.pair.on != 0;
+  sh.mode = p.M > 128 ? 2 : 1;
+  constexpr int cg = 2;
+  sh.nm = silu ? 2 : 1;
+  sh.m_half = ((p.M + cg - 1) / cg + 7) / 8 * 8;
+  constexpr int step = 32;                               // MMA N granularity
+  const int max_units = max_pairs();
+  if (max_units < 1) return kErrLaunch;
+  auto round_up = [&](int n) { return (n + step - 1) / step * step; };
+  // tensor-memory columns per weight row: a pair of 128 keeps half of a unit's columns in each half
+  // of the lanes
+  const int row_cols_x2 = sh.mode == 1 ? 1 : 2;
+  int buffers = 1;
+  for (int i = 0; i < p.n_seg; ++i)
+    p.seg[i].split =    // the greedy pick: K in one piece, as on the K-sliced kernel
+        p.argmax.on ? 1 : split_for_weight(p.seg[i].n, p.seg[i].dense ? p.k_blocks_dense : p.k_blocks);
+  auto seg_un = [&](const Segment& s, int un) {
+    int most = 1024 / (row_cols_x2 * buffers * sh.nm * s.split) / step * step;
+    if (most > 256) most = 256;
+    if (s.dense && round_up(s.n) < most) most = round_up(s.n);
+    return un < most ? un : most;
+  };
+  auto count = [&](int un) {
+    long long units = 0;
+    for (int i = 0; i < p.n_seg; ++i) units += (p.seg[i].n + seg_un(p.seg[i], un) - 1) / seg_un(p.seg[i], un);
+    return units;
+  };
+  // rows per unit: the fewest that make the launch one round; where one MMA (N <= 256) or tensor
+  // memory does not reach that far, two accumulators and the rows with the least padding
+  int un = 0;
+  for (int u = step; u <= 256; u += step)
+    if (count(u) <= max_units) { un = u; break; }
+  if (un == 0) {
+    if (silu) return kErrUnsupported;                    // h waits for a grid-wide exchange inside its CTA
+    buffers = 2;
+    long long best = 0;
+    for (int u = 256; u >= 64; u -= step) {
+      const long long cost = (count(u) + max_units - 1) / max_units * (u + 8);   // 8: what a round costs by itself
+      if (un == 0 || cost < best) { un = u; best = cost; }
+    }
+  }
+  const long long units = count(un);
+  if (units > 0x3fffffffLL) return kErrTooLarge;
+  sh.units = (int)units;
+  sh.rounds = (int)((units + max_units - 1) / max_units);
+  sh.grid = (int)(units < max_units ? units : max_units) * cg;
+  int at = 0, k_blocks[2] = {0, 0}, w_rows[2] = {0, 0};
+  for (int i = 0; i < p.n_seg; ++i) {
+    Segment& s = p.seg[i];
+    s.un = seg_un(s, un);
+    s.unit_begin = at;
+    at += (s.n + s.un - 1) / s.un;
+    const int d = s.dense && sh.rounds == 1 ? 1 : 0;
+    const int kb = s.dense ? p.k_blocks_dense : p.k_blocks;
+    if (kb > k_blocks[d]) k_blocks[d] = kb;
+    if (s.un > w_rows[d]) w_rows[d] = s.un;
+    const int cols = s.un * row_cols_x2 / 2 * sh.nm * s.split;
+    if (cols > sh.acc_cols) sh.acc_cols = cols;
+  }
+  sh.tmem_cols = 32;
+  while (sh.tmem_cols < sh.acc_cols * buffers) sh.tmem_cols *= 2;
+  if (sh.tmem_cols > 512) return kErrUnsupported;
+  sh.flat = flat;
+  const int budget = g_opt_smem_cap > 0 && g_opt_smem_cap < kMaxSmem - 1024 - kBarrierBytes
+                         ? (int)g_opt_smem_cap : kMaxSmem - 1024 - kBarrierBytes;
+  for (int d = 0; d < 2; ++d) {
+    if (w_rows[d] == 0) continue;
+    RingShape& r = sh.ring[d];
+    r.a_block = sh.m_half * kBK;
+    r.w_block = sh.nm * (w_rows[d] / cg) * kBK;
+    // a stage holds 16 KB of weights or more: what the issuing threads spend per stage is fixed
+    r.kb_stage = r.w_block >= 16384 || flat ? 1 : (r.w_block >= 8192 ? 2 : 4);
+    while (r.kb_stage > 1 && (r.kb_stage > k_blocks[d] || r.kb_stage * r.a_block > 32768)) r.kb_stage /= 2;
+    const int a_bytes = r.kb_stage * r.a_block, w_bytes = r.kb_stage * r.w_block;
+    const int want = (k_blocks[d] + r.kb_stage - 1) / r.kb_stage * sh.rounds;   // stages of a CTA's work
+    // 96 KB of activation tiles in flight, four stages at least: once the previous kernel is done every
+    // CTA walks the same tiles of L2 at the same time, and that latency under load is what a wide
+    // batch waits for (128 rows, 4096 x 12288: 16.9 / 14.3 / 13.4 us with 2 / 3 / 4 stages of 32 KB).
+    // The weight ring gets the rest; it streams at full rate from about 100 KB on.
+    int a_stages = 98304 / a_bytes;
+    if (a_stages < 4) a_stages = 4;
+    if (a_stages > 16) a_stages = 16;
+    if (g_opt_b_stages > 0) a_stages = (int)g_opt_b_stages;
+    if (a_stages > want) a_stages = want;
+    int w_stages = (budget - a_stages * a_bytes) / w_bytes;
+    if (w_stages > 40) w_stages = 40;
+    if (w_stages > want) w_stages = want;
+    if (g_opt_stages > 0 && w_stages > g_opt_stages) w_stages = (int)g_opt_stages;
+    if (w_stages < 1) return kErrUnsupported;
+    if (a_stages > w_stages) a_stages = w_stages;
+    r.a_stages = a_stages;
+    r.w_stages = w_stages;
+    // an MMA reads 64 or 128 rows from the start of any batch tile, whatever the batch
+    const int reach = (a_stages * r.kb_stage - 1) * r.a_block + (sh.mode == 2 ? 128 : 64) * kBK;
+    const int bytes = a_stages * a_bytes + w_stages * w_bytes;
+    if (bytes > sh.ring_bytes) sh.ring_bytes = bytes;
+    if (reach > sh.ring_bytes) sh.ring_bytes = reach;
+  }
+  if (w_rows[1] == 0) sh.ring[1] = sh.ring[0];
+  const int es = p.out_dtype == BQ_DTYPE_F32 ? 4 : 2;
+  if (silu && sh.ring_bytes < sh.m_half * (2 * un * es + 16)) sh.ring_bytes = sh.m_half * (2 * un * es + 16);
+  sh.ring_bytes = (sh.ring_bytes + 127) / 128 * 128;
+  if (sh.ring_bytes + kBarrierBytes + 1024 > kMaxSmem) return kErrUnsupported;
+  return kOk;
+}
+
+// (value, index) pairs per batch row that the greedy pick of a launch leaves: one per unit walker and
+// column group (a pair of 128 holds a row's columns in two lane quarters).
+int argmax_slots(const WideShape& sh) {
+  return sh.grid / 2 * (sh.mode == 1 ? 2 : 1) * (sh.rounds > 1 ? (kWideWarps - 4) / 4 : kWideWarps / 4);
+}
+
+int launch_wide(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightMaps& maps,
+                  GemmParams& p, const WideShape& sh, cudaStream_t stream) {
+  const int smem = sh.ring_bytes + kBarrierBytes + 1024;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)sh.grid, 1, 1);
+  cfg.blockDim = dim3(kWideThreads, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_opt_pdl ? 2 : 1;
+  g_last_launch[0] = 0; g_last_launch[1] = sh.grid; g_last_launch[2] = p.seg[0].split;
+  g_last_launch[3] = sh.ring[0].w_stages; g_last_launch[4] = smem; g_last_launch[5] = p.seg[0].un;
+  g_argmax_slots = argmax_slots(sh);
+#ifdef BQ_PHASES
+  p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
+#endif
+  const cudaError_t e = sh.mode == 1 ? cudaLaunchKernelEx(&cfg, gemm_wide_kernel<1>, tm_x, tm_xd, maps, p, sh)
+                                     : cudaLaunchKernelEx(&cfg, gemm_wide_kernel<2>, tm_x, tm_xd, maps, p, sh);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
 }
@@ -1634,6 +1841,7 @@ int bq::gemm_set_option(const char* key, long long value) {
   if (strcmp(key, "push_tma") == 0) { g_opt_push_tma = value ? 1 : 0; return kOk; }
   if (strcmp(key, "pair_narrow") == 0) { g_opt_pair_narrow = value < 0 ? -1 : (value ? 1 : 0); return kOk; }
   if (strcmp(key, "decode_smem_cap") == 0) { g_opt_smem_cap = value; return kOk; }
+  if (strcmp(key, "decode_wide") == 0) { g_opt_wide = value < 0 ? -1 : (value ? 1 : 0); return kOk; }
   if (strcmp(key, "decode_cta_target") == 0) {
     if (value < 1) return kErrBadArg;
     g_opt_cta_target = value;
@@ -1661,6 +1869,73 @@ struct DenseArgs {
   int dtype;
   const int* kind;
 };
+
+// Which launches the wide kernel takes: batches that fill its MMA shape (128 rows, or 256) well enough.
+// K-sliced kernel / wide kernel in us, graphed, one decoder layer of hidden 4096 (and 2560):
+//     48 rows 78.6 / 76.3 (69.8 / 69.3)      56 rows 83.1 / 77.4 (71.9 / 70.9)     64 rows 83.5 / 76.4
+//    128 rows 91.5 / 82.8                   144 rows 95.6 / 96.0                  160 rows 98.6 / 98.1
+//    176 rows 108.8 / 99.6 (92.7 / 86.4)    256 rows 166.3 / 104.1 (137.4 / 104.3)
+// with the MLP alone at 40 and 48 rows 0.94 to 0.99 as fast here and at 129 to 160 0.94 to 1.00.
+// Weights of several rounds (a vocabulary) pay an epilogue per round: where K is long it is hidden and
+// the line lies lower (124000 x 4096: 32 rows 103.1 / 92.8, 40 rows 106.7 / 89.4, 136 rows
+// 155.5 / 124.7; 60016 x 4096: 54.0 / 54.8, 57.0 / 54.0, 81.3 / 69.2), where K is short higher
+// (60016 x 1024: 48 rows 32.5 / 39.1, 64 rows 36.6 / 38.6, 136 rows 50.9 / 55.0, 256 rows 123.7 / 56.8).
+bool wide_applies(const GemmParams& p, const WideShape& sh) {
+  if (g_opt_wide >= 0) return g_opt_wide != 0;
+  if (sh.rounds > 1 && p.k_blocks >= 16) return p.M > 32;
+  return p.M > (sh.rounds > 1 ? 64 : 48) && (p.M <= 128 || p.M > 160);
+}
+
+// The launch on the wide kernel; kErrUnsupported where it has no layout for it or the K-sliced one is
+// the faster.  `p` holds everything but
+// the segments.
+int run_wide(GemmParams p, const void* xq, int64_t K, const void* const* wq, const float* const* sw,
+             void* const* y, const int64_t* N, const int64_t* ldy, const void* const* res,
+             const int64_t* ld_res, const DenseArgs* dn, cudaStream_t stream) {
+  const bool silu = p.pair.on != 0, flat = K % kBK != 0;
+  const bool no_y = silu || p.push.n > 0 || (p.argmax.on && !p.argmax.store_logits);
+  const long long es = p.out_dtype == BQ_DTYPE_F32 ? 4 : 2;
+  for (int i = 0; i < p.n_seg; ++i) {
+    Segment& s = p.seg[i];
+    s.sw = sw[i];
+    s.n = (int)(silu ? N[i] / 2 : N[i]);      // the gate/up form's N counts gate and up rows
+    s.dense = (dn != nullptr && dn->kind[i] != 0) ? 1 : 0;
+    s.y = no_y ? nullptr : y[i];
+    s.ldy = no_y ? 0 : ldy[i];
+    s.res = res ? res[i] : nullptr;
+    s.ld_res = res ? ld_res[i] : 0;
+    bool wide = true;
+    if (p.push.n > 0) {
+      wide = (p.push.ld * es) % 16 == 0;
+      for (int d = 0; d < p.push.n; ++d) wide = wide && aligned_to(p.push.dst[d], 16);
+    } else if (!no_y) {
+      wide = aligned_to(y[i], 16) && (ldy[i] * es) % 16 == 0;
+    }
+    if (s.res) wide = wide && aligned_to(s.res, 16) && (s.ld_res * es) % 16 == 0;
+    s.wide = wide ? 1 : 0;
+  }
+  WideShape sh;
+  if (int rc = plan_wide(p, sh, flat)) return rc;
+  if (!wide_applies(p, sh)) return kErrUnsupported;
+  // the caller's scratch for the greedy pick has a pair per row and 128 vocabulary rows
+  if (p.argmax.on && argmax_slots(sh) > (p.seg[0].n + kRowTile - 1) / kRowTile) return kErrUnsupported;
+  auto map = [&](CUtensorMap* m, const void* ptr, long long rows, bool dense, int box_rows) {
+    // a 16-bit operand is described by its bytes: [rows, 2K]
+    return make_map_kb(m, ptr, rows, dense ? 2 * K : K, box_rows, sh.ring[dense ? 1 : 0].kb_stage, flat);
+  };
+  WeightMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  CUtensorMap tm_x;
+  for (int i = 0; i < p.n_seg; ++i)
+    if (int rc = map(&maps.w[i], wq[i], p.seg[i].n, p.seg[i].dense != 0, p.seg[i].un / 2)) return rc;
+  if (silu)
+    if (int rc = map(&maps.w[1], p.pair.wq_up, p.seg[0].n, false, p.seg[0].un / 2)) return rc;
+  if (int rc = map(&tm_x, xq, p.M, false, sh.m_half)) return rc;
+  CUtensorMap tm_xd = tm_x;
+  if (dn != nullptr)
+    if (int rc = map(&tm_xd, dn->x, p.M, true, sh.m_half)) return rc;
+  return launch_wide(tm_x, tm_xd, maps, p, sh, stream);
+}
 
 int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg,
                 const void* const* wq, const float* const* sw, void* const* y, const int64_t* N,
@@ -1745,6 +2020,10 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     p.push.amax_local = (push->amax_dst[0] != nullptr) ? static_cast<unsigned int*>(ws) + 1 : nullptr;
   }
 
+  if (stream_path && (p.M > 32 || g_opt_wide > 0)) {
+    const int rc = run_wide(p, xq, K, wq, sw, y, N, ldy, res, ld_res, dn, stream);
+    if (rc != kErrUnsupported) return rc;
+  }
   const bool pair_path = !stream_path;
   p.m_tiles = pair_path ? (int)((M + kPairTile - 1) / kPairTile) : (int)((M + kRowTile - 1) / kRowTile);
   // plain prefill form of ONE narrow weight: 128-column tiles when all of them still run at once,
@@ -1881,7 +2160,6 @@ extern "C" int bq_lm_head_argmax(const void* xq, const void* wq, const float* sx
   if (int rc = run_grouped(xq, sx, M, K, 1, wqs, sws, ys, Ns, ldys, out_dtype, ws, ws_bytes, stream,
                            nullptr, nullptr, nullptr, 1, nullptr, nullptr, &am))
     return rc;
-  const int tiles = (int)((N + kRowTile - 1) / kRowTile);
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)M, 1, 1);
@@ -1892,7 +2170,7 @@ extern "C" int bq_lm_head_argmax(const void* xq, const void* wq, const float* sx
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_opt_pdl ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_finish_kernel, am.partial, tiles, (int)M,
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_finish_kernel, am.partial, g_argmax_slots, (int)M,
                                            reinterpret_cast<long long*>(idx_out));
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;

@@ -555,6 +555,7 @@ int bq_read_device_status(void* ws, void* stream, int* status_out);
  * bq_set_option("decode_split_k", v)    0 = heuristic, else force the K slices per tile
  * bq_set_option("decode_stages", v)     0 = heuristic, else cap the pipeline depth
  * bq_set_option("decode_b_stages", v)   activation ring depth: 0 = heuristic, -1 = as the weight ring
+ * bq_set_option("decode_wide", v)       decode batches on the CTA-pair kernel: -1 by size, 0 never, 1 always
  * bq_set_option("decode_cta_target", v) CTAs a small weight is sliced to reach (default 160)
  * bq_set_option("decode_smem_cap", v)   0 = none, else cap pipeline bytes per CTA
  * bq_set_option("stream_max_m", v)      largest M the weight-streaming kernel takes (<= 256)

@@ -13,7 +13,7 @@ import torch.nn.functional as F
 
 import oracle
 from oracle import torch_spelling as TS
-from _util import codes_np, config1_inputs, from_bits16, from_bits32, max_rel, randn_cpu
+from _util import codes_np, config1_inputs, from_bits16, from_bits32, max_rel, randn_cpu, u8
 
 pytestmark = pytest.mark.gpu
 
@@ -619,3 +619,85 @@ def test_paired_mlp_equals_the_four_launch_mlp_and_replays(Q):
         graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, eager) and Q.device_status() == 0
+
+
+def _pitched(Q, xq, sx, w, M, n):
+    buf = torch.full((M, n + 4), 7.0, dtype=torch.bfloat16, device="cuda")
+    Q.fp8_matmul_grouped(xq, sx, [w], out=[buf[:, :n]])
+    return buf
+
+
+@pytest.fixture
+def wide(Q):
+    Q.set_option("decode_wide", 1)
+    yield
+    Q.set_option("decode_wide", -1)
+
+
+@pytest.mark.parametrize("M,ns,K", [(1, (48,), 256), (33, (16,), 128), (40, (48, 1040), 4096), (64, (4096, 1024), 1040),
+                                    (65, (272,), 2560), (127, (4096,), 16), (128, (8192, 1024, 1024), 4096),
+                                    (129, (4736,), 512), (200, (1040, 32), 2064), (256, (12288, 4096), 1024)])
+def test_wide_batches_on_cta_pairs_agree_with_the_k_sliced_kernel(Q, M, ns, K):
+    """Wide decode batches run on CTA pairs (one round of units over the whole of K); the option selects
+    that kernel or the K-sliced one for any batch.  Edges: one unit, the last unit short, K below and beyond a 128-byte block,
+    batches that fill half of a pair's rows, all of them, and one row more."""
+    x = randn_cpu((M, K), seed=M + K).cuda()
+    xq, sx = Q.quantize_act(x)
+    ws = [Q.quantize_weight((randn_cpu((n, K), seed=n) * 0.02).cuda()) for n in ns]
+    a = xq.float().double() * sx.double()
+
+    def both(fn):
+        out = []
+        try:
+            for wide in (1, 0):
+                Q.set_option("decode_wide", wide)
+                out.append(fn())
+        finally:
+            Q.set_option("decode_wide", -1)
+        return out
+
+    got, want = both(lambda: Q.fp8_matmul_grouped(xq, sx, ws, out_dtype=torch.float32))
+    for y, z, w in zip(got, want, ws):
+        b = w.data.float().double() * w.scale.double()
+        # an fp32 sum of K products, 32 of them per step of the accumulator, each step off by at most
+        # two units of the last place of the sum of magnitudes; the scaling adds two more
+        bound = (K / 32 + 2) * 2.0 ** -22 * (a.abs() @ b.abs().t()) + 1e-30
+        for t in (y, z):
+            assert ((t.double() - a @ b.t()).abs() <= bound).all()
+        for t, alone in zip((y, z), both(lambda: Q.fp8_matmul(xq, sx, w, out_dtype=torch.float32))):
+            assert torch.equal(t, alone)
+    # a residual, and an output row pitch that allows 8-byte accesses only
+    n = ns[0]
+    res = randn_cpu((M, n), seed=9).cuda()
+    got, want = both(lambda: Q.linear(x, ws[0], residual=res))
+    assert max_rel(got, want.double()) <= TOL_BF16
+    for buf, plain in zip(both(lambda: _pitched(Q, xq, sx, ws[0], M, n)), both(lambda: Q.fp8_matmul(xq, sx, ws[0]))):
+        assert torch.equal(buf[:, :n], plain) and bool((buf[:, n:] == 7.0).all())
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("M,I,K,dt", [(33, 64, 128, torch.bfloat16), (64, 4736, 1040, torch.float16),
+                                      (96, 1024, 2048, torch.float32), (130, 192, 256, torch.bfloat16),
+                                      (256, 12288, 1024, torch.bfloat16)])
+def test_wide_gate_up_codes_equal_the_separate_kernels(Q, wide, M, I, K, dt):
+    x = randn_cpu((M, K), seed=1, dtype=dt).cuda()
+    xq, sx = Q.quantize_act(x)
+    g, u = (Q.quantize_weight((randn_cpu((I, K), seed=s) * 0.05).cuda()) for s in (2, 3))
+    got = Q.gate_up_silu_quant(xq, sx, g, u, dt)
+    gate, up = Q.fp8_matmul_grouped(xq, sx, (g, u), out_dtype=dt)
+    q, s = Q.silu_mul_quant(gate, up)
+    assert got is not None and torch.equal(got[1], s) and torch.equal(u8(got[0]), u8(q))
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("M", [33, 64, 129])
+def test_wide_greedy_pick_over_several_rounds(Q, wide, M):
+    V, K = 60016, 256
+    w = Q.quantize_weight((randn_cpu((V, K), seed=3) * 0.02).cuda())
+    w.data.view(torch.uint8)[V - 16:] = w.data.view(torch.uint8)[:16]      # equal logits: the lower index wins
+    x = randn_cpu((M, K), seed=M).cuda()
+    idx, logits = Q.lm_head_argmax(x, w, return_logits=True)
+    assert torch.equal(idx.flatten(), logits.argmax(-1).flatten())
+    xq, sx = Q.quantize_act(x)
+    assert torch.equal(logits, Q.fp8_matmul(xq, sx, w))
+    assert Q.device_status() == 0
