@@ -22,22 +22,48 @@ struct QuantWs {
 // thread.  A single-CTA grid never touches global memory here.  Thread 0 of every
 // CTA of a multi-CTA grid owes the scratch a grid_depart() call afterwards; that
 // part is kept off the critical path on purpose.
-// `live` = false: the CTA's own max without the exchange (a rehearsal pass, see norm_quant.cu).
-__device__ __forceinline__ float grid_amax(float m, QuantWs* ws, bool live = true) {
-  __shared__ float s_warp[32];
-  __shared__ float s_amax;
+struct WholeCta {
+  static constexpr bool live = true;
+  __device__ int warp() const { return threadIdx.x >> 5; }
+  __device__ int warps() const { return (blockDim.x + 31) >> 5; }
+  __device__ int slot() const { return 0; }
+  __device__ void sync() const { __syncthreads(); }
+};
+
+// A CTA of THREADS working threads and, where it was launched with 32 more, a warp that only rehearses
+// (see norm_quant.cu): that one runs the code of warp 0 on its own words of shared memory, and the
+// others never wait for it.
+template <int THREADS>
+struct RehearsingCta {
+  bool live;
+  __device__ int warp() const { return live ? threadIdx.x >> 5 : 0; }
+  __device__ int warps() const { return live ? THREADS / 32 : 1; }
+  __device__ int slot() const { return live ? 0 : 1; }
+  __device__ void sync() const {
+    if (live) asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    else __syncwarp();
+  }
+};
+
+// `cta.live` = false: this warp's own max without the exchange.
+template <typename Cta = WholeCta>
+__device__ __forceinline__ float grid_amax(float m, QuantWs* ws, const Cta& cta = Cta{}) {
+  __shared__ float s_warp_of[2][32];
+  __shared__ float s_amax_of[2];
+  float* const s_warp = s_warp_of[cta.slot()];
+  float& s_amax = s_amax_of[cta.slot()];
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = cta.warp();
   if (lane == 0) s_warp[warp] = m;
-  __syncthreads();
+  cta.sync();
   if (warp == 0) {
-    const int nwarps = (blockDim.x + 31) >> 5;
+    const int nwarps = cta.warps();
     float w = (lane < nwarps) ? s_warp[lane] : 0.0f;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) w = nan_max(w, __shfl_xor_sync(0xffffffffu, w, off));
     if (lane == 0) {
-      if (gridDim.x == 1 || !live) {
+      if (gridDim.x == 1 || !cta.live) {
         s_amax = w;
       } else {
         // |x| >= 0 or NaN with the sign cleared: the unsigned order of the bit
@@ -63,7 +89,7 @@ __device__ __forceinline__ float grid_amax(float m, QuantWs* ws, bool live = tru
       }
     }
   }
-  __syncthreads();
+  cta.sync();
   return s_amax;
 }
 

@@ -53,7 +53,7 @@ struct NormParams {
   int phase_seq;
 };
 
-constexpr unsigned int kRehearseRows = 32;   // see rmsnorm_quant_kernel; one CTA per row
+constexpr int kRehearseRows = 32;   // see rmsnorm_quant_kernel; one CTA per row
 
 template <typename T> struct Vec4 { T v[kVec]; };
 
@@ -103,11 +103,14 @@ __device__ __forceinline__ float warp_tree_sum(float s) {
 // plain RMSNorm -> quantize.  One CTA of 128 threads per row; VPT = vectors held per thread.
 // ---------------------------------------------------------------------------------------------
 template <typename T, int VPT>
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormParams p) {
+__global__ void __launch_bounds__(kNormThreads + 32) rmsnorm_quant_kernel(const NormParams p) {
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
-  __shared__ float s_red[4];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  __shared__ float s_red_of[2][4];
+  const RehearsingCta<kNormThreads> cta{threadIdx.x < kNormThreads};
+  const bool live = cta.live;
+  float* const s_red = s_red_of[cta.slot()];
+  const int lane = threadIdx.x & 31, warp = cta.warp(), t = warp * 32 + lane;
   const int row = blockIdx.x;
   const int n_vec = p.cols / kVec;
   const T* xr = reinterpret_cast<const T*>(p.x) + static_cast<long long>(row) * p.ld_x;
@@ -122,16 +125,15 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormP
     }
   }
   // What bounds this kernel at a decode batch is neither bytes nor arithmetic but one dependent chain
-  // run once from a cold instruction cache (the previous kernel's code was there).  Pass 0 is a
-  // rehearsal on zeros while the CTA waits for the previous kernel anyway: the same instructions
-  // without a load, store or exchange, so that pass 1 finds them in the cache.  Four graphed decoder
-  // layers (eight of these, three gated ones): 264.5 -> 248.6 us at 1 row, 297.5 -> 289.9 at 27.
-  // Only up to kRehearseRows rows: with 128 CTAs the rehearsal competes with the GEMM that is being
-  // waited for (379.5 -> 378.0 us there, 344 -> 350 in front of a faster GEMM), and at 64 rows
-  // in front of a vocabulary, with nothing to wait for, it cost 2.4 us.
-#pragma unroll 1
-  for (int pass = gridDim.x <= kRehearseRows ? 0 : 1; pass < 2; ++pass) {
-  const bool live = pass != 0;
+  // run once from a cold instruction cache (the previous kernel's code was there).  So a fifth
+  // warp rehearses: it runs the same instructions on zeros, without a load, store or exchange, while
+  // the others wait for the previous kernel, and they find the code in the cache.  A warp of its own,
+  // because there may be nothing to wait for (behind a kernel that was not launched with early
+  // starts): a second pass of all warps gave more in
+  // an unbroken chain (hidden 4096, four graphed layers, 1 row: 262 -> 244 us, here 256) but cost 3 us
+  // per launch in a broken one (hidden 2560: 194 -> 203 us, here 193).
+  // Only up to kRehearseRows rows: beyond, the rehearsal competes with the GEMM that is waited for
+  // (344 -> 350 us at 128 rows).
   Vec4<T> x[VPT];
   if (live) {
     bq::pdl_wait_prior_grids();
@@ -157,13 +159,13 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormP
   }
   s = warp_tree_sum(s);
   if (lane == 0 && warp >= 2) s_red[warp - 2] = s;
-  __syncthreads();
+  cta.sync();
   if (lane == 0 && warp < 2) s = __fadd_rn(s, s_red[warp]);
-  __syncthreads();
+  cta.sync();
   if (lane == 0 && warp == 1) s_red[0] = s;
-  __syncthreads();
+  cta.sync();
   if (t == 0) s_red[1] = __fdiv_rn(__fadd_rn(s, s_red[0]), static_cast<float>(p.cols));
-  __syncthreads();
+  cta.sync();
   const float rstd = rsqrtf(__fadd_rn(s_red[1], p.eps));
 
   float m = 0.0f;
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormP
     }
   }
   if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
-  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), live));
+  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), cta));
   if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
   const ScaleDiv dv(sc);
   if (live && blockIdx.x == 0 && t == 0) p.scale[0] = sc;
@@ -197,7 +199,6 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_quant_kernel(const NormP
   for (int i = 0; i < VPT; ++i) {
     const int v = t + i * kNormThreads;
     if (v < n_vec) emit4(x[i], dv, qr + v * kVec, live);
-  }
   }
   grid_depart(static_cast<QuantWs*>(p.ws));
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
@@ -320,17 +321,15 @@ constexpr int kGatedWarps = 8;
 constexpr int kMaxHeadsPerWarp = 8;    // up to 64 heads
 
 template <typename T, bool Y_F32, int HPW>
-__global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_quant_kernel(const GatedParams p) {
+__global__ void __launch_bounds__(kGatedWarps * 32 + 32) gated_rmsnorm_quant_kernel(const GatedParams p) {
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const RehearsingCta<kGatedWarps * 32> cta{threadIdx.x < kGatedWarps * 32};   // see rmsnorm_quant_kernel
+  const bool live = cta.live;
+  const int lane = threadIdx.x & 31, warp = cta.warp();
   const int row = blockIdx.x;
   const float4 gm = __ldg(reinterpret_cast<const float4*>(p.gamma) + lane);
   const float gmv[kVec] = {gm.x, gm.y, gm.z, gm.w};
-  // pass 0 is a rehearsal on zeros (see rmsnorm_quant_kernel)
-#pragma unroll 1
-  for (int pass = gridDim.x <= kRehearseRows ? 0 : 1; pass < 2; ++pass) {
-  const bool live = pass != 0;
   Vec4<T> core[HPW];
   Vec4<T> gate[HPW];
   if (live) {
@@ -384,7 +383,7 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_quant_kernel(c
     }
   }
   if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
-  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), live));
+  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), cta));
   if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
   const ScaleDiv dv(sc);
   if (live && blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
@@ -393,7 +392,6 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_quant_kernel(c
   for (int i = 0; i < HPW; ++i) {
     const int head = warp + i * kGatedWarps;
     if (head < p.heads) emit4(core[i], dv, qr + head * kHeadDim + lane * kVec, live);
-  }
   }
   grid_depart(static_cast<QuantWs*>(p.ws));
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
@@ -405,6 +403,7 @@ int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t str
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
 #endif
+  if (rows <= kRehearseRows) threads += 32;   // the rehearsing warp
   // every CTA waits for every other: the whole grid must fit on the device at once
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
