@@ -15,7 +15,7 @@
 // K / 32 of them one after another.  That chain is why small batches stay on the K-sliced kernel
 // (gemm_w8a8.cu): a 64-row form of this one took 3.6 us instead of 2.5 from the activation's arrival
 // to the last MMA of a 4096 x 4096 weight, and four graphed decoder layers 254.6 instead of 245.0 us
-// at 1 row, 290.3 instead of 288.1 at 27.  At 128 rows they take 333.9 instead of 362.9 us here, a
+// at 1 row, 290.3 instead of 288.1 at 27.  At 128 rows they take 344 instead of 379 us here, a
 // 248320-row vocabulary 178 instead of 233 us at 64 rows and 267 instead of 665 at 256.
 //
 // Sums.  Weights of few rows are summed in 2 or 4 K slices, each with an accumulator of its own,
