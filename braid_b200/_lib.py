@@ -34,6 +34,8 @@ SIGNATURES = {
     "bq_scratchless_status": (_int, [ctypes.POINTER(ctypes.c_int)]),
     "bq_quant_workspace_bytes": (_sz, []),
     "bq_quantize_act": (_int, [_vp, _int, _i64, _vp, _vp, _vp, _sz, _vp]),
+    "bq_quantize_weight_workspace_bytes": (_sz, []),
+    "bq_quantize_weight": (_int, [_vp, _int, _i64, _vp, _vp, _vp, _sz, _vp]),
     "bq_quantize_act_static": (_int, [_vp, _int, _i64, _vp, _vp, _vp]),
     "bq_silu_mul_quant": (_int, [_vp, _vp, _int, _i64, _i64, _i64, _i64, _vp, _vp, _vp, _sz, _vp]),
     "bq_silu_mul_scale": (_int, [_vp, _vp, _int, _i64, _i64, _i64, _i64, _vp, _vp, _sz, _vp]),

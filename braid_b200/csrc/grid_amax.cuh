@@ -93,6 +93,18 @@ __device__ __forceinline__ float grid_amax(float m, QuantWs* ws, const Cta& cta 
   return s_amax;
 }
 
+// CTA-wide max alone, to every thread.  Blocks of whole warps, 1024 threads at most.
+__device__ __forceinline__ float cta_amax(float m) {
+  __shared__ float s_warp[32];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
+  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = s_warp[0];
+  for (unsigned int i = 1; i < blockDim.x / 32; ++i) m = nan_max(m, s_warp[i]);
+  return m;
+}
+
 // Column-parallel form: every CTA waits (bounded, thread 0 polls with a system-scope acquire)
 // until the arrival counter has advanced by `count` beyond *seen -- i.e. until every rank's push
 // launch has stored its share of the buffer this kernel is about to read.  *seen is advanced by

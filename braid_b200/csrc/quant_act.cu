@@ -112,7 +112,11 @@ __global__ void __launch_bounds__(512, 1) quant_hold_kernel(const QParams p) {
 // column-parallel MLP: every rank takes the scale of its own shard, the ranks combine the
 // scales with a MAX all-reduce (max is exact and order-free, and the scale is a monotone
 // function of the amax), and every rank casts its shard with the combined scale.
-enum Phase { kBoth = 0, kScaleOnly = 1, kCastOnly = 2 };
+// kMaxOnly and kWeightCast are the two launches of the weight quantizer (ring kernel only): pass 1
+// leaves every CTA's maximum in a caller-owned array, pass 2 folds them and casts.  A weight may be
+// loaded on any stream while others decode, so nothing here waits for another CTA and no word
+// is shared with another launch.
+enum Phase { kBoth = 0, kScaleOnly = 1, kCastOnly = 2, kMaxOnly = 3, kWeightCast = 4 };
 
 template <typename T, int MODE, int PHASE>
 __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
@@ -196,9 +200,9 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
     grid_depart(static_cast<QuantWs*>(p.ws), coherent ? p.wait_seen : nullptr, p.wait_count);
 }
 
-// Sticky status of the launches that run without scratch from the caller (the cast half alone):
-// a bounded wait that ran out there has no status word of the caller's to raise, so it raises
-// this one; bq_scratchless_status() reads and clears it.
+// Sticky status of the launches that run without scratch words from the caller (the cast half alone,
+// the weight quantizer): a bounded wait that ran out there has no status word of the caller's to
+// raise, so it raises this one; bq_scratchless_status() reads and clears it.
 __device__ unsigned int g_scratchless_status = 0u;
 
 // ---- plain quantizer at prefill sizes: bulk copies into a shared-memory ring --------------
@@ -286,17 +290,27 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
   auto fail = [&]() { atomicExch(&s_failed, 1u); };
   // what a later pass (or the cast launch that follows a scale launch) reads again stays in
   // L2 as long as L2 likes; measured, the hint makes no difference at any size
-  const uint64_t policy = (PHASE == kCastOnly) ? bq::policy_evict_first() : bq::policy_evict_last();
+  constexpr bool kCasts = PHASE == kCastOnly || PHASE == kWeightCast;   // the forward pass casts
+  const uint64_t policy = kCasts ? bq::policy_evict_first() : bq::policy_evict_last();
+  // the weight's cast walks backwards: what the launch before read last is the likeliest to be in L2
+  auto chunk_at = [&](int k) { return PHASE == kWeightCast ? count - 1 - k : k; };
   // the elements after the last whole group belong to consumer thread 0 of CTA 0
   const bool owns_tail = p.tail != 0 && blockIdx.x == 0 && threadIdx.x == 0;
   const T* tail_src = reinterpret_cast<const T*>(p.a) + static_cast<size_t>(p.n_groups) * kGroup;
   constexpr int kPerUnit = 16 / (int)sizeof(T);   // elements (and code bytes) per 16 bytes of input
 
-  float sc;
-  // ---- forward pass: |x| max (kBoth, kScaleOnly) or the cast itself (kCastOnly) ----
+  float sc = 1.0f;
+  // ---- forward pass: |x| max (kBoth, kScaleOnly, kMaxOnly) or the cast itself ----
   if constexpr (PHASE == kCastOnly) sc = __ldcg(p.scale);
+  if constexpr (PHASE == kWeightCast) {
+    // the launch before had this one's grid: one maximum per CTA
+    float w = 0.0f;
+    for (unsigned int i = threadIdx.x; i < gridDim.x; i += blockDim.x) w = nan_max(w, __ldcg(p.partial + i));
+    sc = scale_from_amax(cta_amax(w));
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
+  }
   {
-    const ScaleDiv dv(PHASE == kCastOnly ? sc : 1.0f);
+    const ScaleDiv dv(sc);
     float m = 0.0f;
     if (producer) {
       if (lane == 0) {
@@ -307,9 +321,9 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
             fail();
             break;
           }
-          const uint32_t bytes = chunk_bytes(k);
+          const uint32_t bytes = chunk_bytes(chunk_at(k));
           bq::mbar_expect_tx(bq::smem_u32(&bars[0][s]), bytes);
-          bq::bulk_load_1d(bq::smem_u32(ring + s * kRingChunk), src + chunk_offset(k), bytes,
+          bq::bulk_load_1d(bq::smem_u32(ring + s * kRingChunk), src + chunk_offset(chunk_at(k)), bytes,
                            bq::smem_u32(&bars[0][s]), policy);
         }
       }
@@ -320,7 +334,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
           fail();
           break;
         }
-        const uint32_t have = chunk_bytes(k);
+        const uint32_t have = chunk_bytes(chunk_at(k));
         uint4 raw[kRingUnits];
 #pragma unroll
         for (int u = 0; u < kRingUnits; ++u) {
@@ -331,8 +345,9 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
         for (int u = 0; u < kRingUnits; ++u) {
           const uint32_t unit = threadIdx.x + u * kRingThreads;
           if (unit * 16u < have) {
-            if constexpr (PHASE == kCastOnly) {
-              unit_emit<T, false>(raw[u], dv, p.q + (chunk_offset(k) / 16 + unit) * kPerUnit);
+            if constexpr (kCasts) {
+              unit_emit<T, PHASE == kWeightCast>(raw[u], dv,
+                                                 p.q + (chunk_offset(chunk_at(k)) / 16 + unit) * kPerUnit);
             } else {
               m = unit_absmax<T>(raw[u], m);
             }
@@ -345,12 +360,15 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
         }
       }
     }
-    if constexpr (PHASE == kCastOnly) {
+    if constexpr (kCasts) {
       if (owns_tail) {
         uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;
         for (unsigned int i = 0; i < p.tail; ++i)
           dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(tail_src[i]), dv), __NV_SATFINITE, __NV_E4M3);
       }
+    } else if constexpr (PHASE == kMaxOnly) {
+      m = cta_amax(m);
+      if (threadIdx.x == 0) p.partial[blockIdx.x] = m;
     } else {
       if (owns_tail)
         for (unsigned int i = 0; i < p.tail; ++i) m = nan_max(m, fabsf(widen(tail_src[i])));
@@ -414,7 +432,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
   __syncthreads();
   if (s_failed != 0u) {
     if (threadIdx.x == 0) {
-      // the cast half alone runs without scratch: it raises the library's own sticky word
+      // the cast half alone and the weight quantizer have none: they raise the library's own
       if (p.ws != nullptr)
         atomicExch(&static_cast<QuantWs*>(p.ws)->status, (unsigned int)bq::kErrDeviceWait);
       else
@@ -424,7 +442,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
     }
     __syncthreads();
   }
-  if constexpr (PHASE != kCastOnly) grid_depart(static_cast<QuantWs*>(p.ws));
+  if constexpr (PHASE == kBoth || PHASE == kScaleOnly) grid_depart(static_cast<QuantWs*>(p.ws));
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
@@ -633,6 +651,15 @@ int launch_ring(const QParams& p, int sms, cudaStream_t stream) {
   return launch_with_pdl(quant_ring_kernel<T, PHASE, 1>, grid, block, p, stream, kRingSmem);
 }
 
+constexpr int kWeightCtas = 1024;   // room for one maximum per CTA of the weight quantizer's first launch
+
+// Two launches where the activation quantizer takes one: nothing is exchanged while they run.
+template <typename T>
+int launch_weight(const QParams& p, int sms, cudaStream_t stream) {
+  if (int rc = launch_ring<T, kMaxOnly>(p, sms, stream)) return rc;
+  return launch_ring<T, kWeightCast>(p, sms, stream);
+}
+
 template <typename T, int MODE>
 int launch_quant(QParams p, cudaStream_t stream) {
   const int sms = device_sms();
@@ -765,6 +792,33 @@ extern "C" int bq_quantize_act(const void* x, int dtype, int64_t n, void* q_out,
   p.tail = static_cast<unsigned int>(n % kGroup);
   p.groups_per_row = 1;
   return dispatch_dtype<kPlain>(dtype, p, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" size_t bq_quantize_weight_workspace_bytes(void) { return kWeightCtas * sizeof(float); }
+
+extern "C" int bq_quantize_weight(const void* w, int dtype, int64_t n, void* q_out, float* scale_out,
+                                  void* ws, size_t ws_bytes, void* stream) {
+  if (w == nullptr || q_out == nullptr || scale_out == nullptr || n <= 0) return bq::kErrBadArg;
+  if (dtype != BQ_DTYPE_F32 && dtype != BQ_DTYPE_BF16 && dtype != BQ_DTYPE_F16) return bq::kErrBadArg;
+  if (ws == nullptr || ws_bytes < kWeightCtas * sizeof(float) || !aligned_to(ws, 4)) return bq::kErrWorkspace;
+  if (n % kGroup || !aligned_to(w, 16) || !aligned_to(q_out, 8)) return bq::kErrUnsupported;
+  if (n / kGroup >= 0x7fffffffLL) return bq::kErrTooLarge;
+  const int sms = device_sms();
+  if (sms <= 0) return bq::kErrLaunch;
+  if (2 * sms > kWeightCtas) return bq::kErrUnsupported;
+  QParams p{};
+  p.a = w;
+  p.q = static_cast<uint8_t*>(q_out);
+  p.scale = scale_out;
+  p.partial = static_cast<float*>(ws);
+  p.n_groups = static_cast<unsigned int>(n / kGroup);
+  p.groups_per_row = 1;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case BQ_DTYPE_F32: return launch_weight<float>(p, sms, s);
+    case BQ_DTYPE_BF16: return launch_weight<__nv_bfloat16>(p, sms, s);
+    default: return launch_weight<__half>(p, sms, s);
+  }
 }
 
 extern "C" int bq_quantize_act_after(const void* x, int dtype, int64_t n, void* q_out,

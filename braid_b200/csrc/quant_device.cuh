@@ -31,6 +31,7 @@ struct QParams {
   uint8_t* q;
   float* scale;
   void* ws;             // kernel-specific scratch words
+  float* partial;       // weight quantizer: the CTAs' maxima, from its first launch to its second
   unsigned int n_groups;      // full groups of 8
   unsigned int tail;          // plain mode only: leftover elements (< 8)
   unsigned int groups_per_row;

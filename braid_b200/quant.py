@@ -16,8 +16,9 @@ unchanged; what is underneath is replaced:
     `mlp_forward`, `gated_output_projection` — the fused prologues the reference
     leaves as separate bf16 kernels (braid/model/mlp.py:48, attention.py:215).
 
-Weights are quantized with the reference's own torch spelling (load-time work,
-braid/model/quant.py:118-154), on whatever device the weight lives on.
+Weights are quantized on whatever device they live on: contiguous CUDA weights by two launches
+of this library (`bq_quantize_weight`), all others with the reference's own torch spelling
+(braid/model/quant.py:118-154); the bits are the same.
 
 There is no CPU implementation of the kernels: activations must be CUDA
 tensors, and a missing library is an error, not a silent slow path.  The only
@@ -101,29 +102,30 @@ _CAST_CHUNK_BYTES = 256 * 2 ** 20
 
 
 def _quantize_weight_fused(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor] | None:
-    """Codes and scale of a weight from the activation quantizer's kernel: one launch that reads the
-    weight from memory once (a second time from L2 where it is larger than shared memory) instead of
-    two reductions, a division, a clamp and a conversion through fp32 temporaries.  A 12288 x 4096
-    bf16 weight: 485 -> 50 us; its 150 MB take 22.7 us at 6.65 TB/s.  Scale and codes are the
-    bits of the torch spelling: both take max |w| / 448 and divide.
+    """Codes and scale of a weight from two launches of the ring kernel (`quant_act.cu`): every CTA's
+    max |w|, then the cast under their maximum.  Scale and codes are the bits of the torch
+    spelling: both take max |w| / 448 and divide.
 
-    `None` -- the torch spelling -- for whatever the kernel does not take: no CUDA tensor of the current
+    Weights may be loaded on any stream, in any number, while others decode, as with plain torch
+    operations: the launches share no scratch with the forward path and wait for no other CTA.
+
+    `None` -- the torch spelling -- for whatever the kernels do not take: no CUDA tensor of the current
     device, another type, a strided or unaligned view, a weight that records gradients, a tensor
-    subclass (tracing), no library, a capture before the scratch exists, or the parity arm."""
+    subclass (tracing), no library, or the parity arm."""
     if (type(w) not in (torch.Tensor, torch.nn.Parameter) or not w.is_cuda or w.dtype not in _DTYPE_CODE
             or not w.is_contiguous() or w.data_ptr() % 16 or w.numel() == 0 or _quantizers_off()
             or (w.requires_grad and torch.is_grad_enabled())
             or w.device.index != torch.cuda.current_device()):
         return None
     try:
-        lib = _require_lib()
-        slot = _take_slot(w.device, counted=False)
+        lib = _lib.load()
     except (OSError, RuntimeError):
         return None
     q = torch.empty(w.shape, dtype=FP8, device=w.device)
     scale = torch.empty((1, 1), dtype=torch.float32, device=w.device)
-    rc = lib.bq_quantize_act(w.data_ptr(), _DTYPE_CODE[w.dtype], w.numel(), q.data_ptr(), scale.data_ptr(),
-                             slot, 16, _stream_ptr(w.device))
+    ws = torch.empty(lib.bq_quantize_weight_workspace_bytes(), dtype=torch.uint8, device=w.device)
+    rc = lib.bq_quantize_weight(w.data_ptr(), _DTYPE_CODE[w.dtype], w.numel(), q.data_ptr(), scale.data_ptr(),
+                                ws.data_ptr(), ws.numel(), _stream_ptr(w.device))
     return (q, scale) if rc == 0 else None
 
 
@@ -245,14 +247,13 @@ def _scratch_for(device_index: int) -> torch.Tensor:
     return buf
 
 
-def _take_slot(device: torch.device, counted: bool = True) -> int:
-    """Device address of the next scratch slot of this device.  `counted` = False: the launch is not one
-    of the forward path that `launch_count` reports (loading a weight)."""
+def _take_slot(device: torch.device) -> int:
+    """Device address of the next scratch slot of this device."""
     global _launches
     idx = device.index if device.index is not None else torch.cuda.current_device()
     buf = _scratch_for(idx)
     with _LOCK:
-        _launches += counted
+        _launches += 1
         slot = _next_slot[idx]
         _next_slot[idx] = (slot + 1) % _SLOTS
     return buf.data_ptr() + slot * _SLOT_BYTES

@@ -46,7 +46,7 @@ int bq_version(void);
 
 /*
  * Synchronises the current device and returns, through *status_out, the sticky status of the
- * launches that take no scratch from the caller (bq_cast_act): 0, or BQ_ERR_DEVICE_WAIT when a
+ * launches that keep no status word of the caller's (bq_cast_act, bq_quantize_weight): 0, or BQ_ERR_DEVICE_WAIT when a
  * bounded wait of such a launch ran out since the last call; clears it.  Never during capture.
  */
 int bq_scratchless_status(int* status_out);
@@ -82,6 +82,18 @@ size_t bq_quant_workspace_bytes(void);
  */
 int bq_quantize_act(const void* x, int dtype, int64_t n, void* q_out, float* scale_out,
                     void* ws, size_t ws_bytes, void* stream);
+
+/*
+ * The quantizer for a weight, once, at load: the same arithmetic as bq_quantize_act with the same
+ * bits, for callers that load weights while other streams decode.  Two launches that wait for no
+ * other CTA and keep nothing between calls: `ws` is any bq_quantize_weight_workspace_bytes() bytes
+ * of device memory, uninitialised, private to the call until the stream has passed it.  n % 8 == 0.
+ *
+ * Replaces: braid/model/quant.py:139-154 (`quantize_weight`).
+ */
+size_t bq_quantize_weight_workspace_bytes(void);
+int bq_quantize_weight(const void* w, int dtype, int64_t n, void* q_out, float* scale_out,
+                       void* ws, size_t ws_bytes, void* stream);
 
 /*
  * The same quantizer for callers that cannot give the library a scratch buffer.

@@ -126,6 +126,11 @@ def test_argument_validation_returns_before_any_cuda_call(lib):
     assert lib.bq_cast_act_push(16, 1, 4, 12, 16, 16, 2, ptrs, 64, ptrs, 16, 16, None) == _lib.BQ_ERR_UNSUPPORTED
     assert lib.bq_rows_push(16, 1, 4, 16, 16, 2, bad, 64, ptrs, 16, 16, None) == _lib.BQ_ERR_BAD_ARG
     assert lib.bq_rows_push(16, 1, 4, 16, 16, 2, ptrs, 64, ptrs, None, 0, None) == _lib.BQ_ERR_WORKSPACE
+    room = lib.bq_quantize_weight_workspace_bytes()
+    assert lib.bq_quantize_weight(16, 1, 64, None, 16, 16, room, None) == _lib.BQ_ERR_BAD_ARG
+    assert lib.bq_quantize_weight(16, 1, 64, 16, 16, 16, room - 1, None) == _lib.BQ_ERR_WORKSPACE
+    assert lib.bq_quantize_weight(16, 1, 68, 16, 16, 16, room, None) == _lib.BQ_ERR_UNSUPPORTED
+    assert lib.bq_quantize_weight(24, 1, 64, 16, 16, 16, room, None) == _lib.BQ_ERR_UNSUPPORTED
     assert lib.bq_scratchless_status(None) == _lib.BQ_ERR_BAD_ARG
     assert lib.bq_set_option(b"no_such_option", 1) == _lib.BQ_ERR_BAD_ARG
     assert lib.bq_set_option(b"quant_ring", 1) == _lib.BQ_OK and lib.bq_set_option(b"push_tma", 1) == _lib.BQ_OK

@@ -420,3 +420,47 @@ def test_quantize_weight_gives_the_bits_of_the_torch_spelling(Q, dt, shape):
         assert got.shape == want.shape and got.data.shape == want.data.shape
         assert torch.equal(u8(got.scale), u8(want.scale)), f"{dt} {shape} case {i}"
         assert torch.equal(u8(got.data), u8(want.data)), f"{dt} {shape} case {i}"
+
+
+def test_weights_load_on_a_side_stream_while_a_graph_replays(Q):
+    """Loading shares no state with the forward path: it takes none of its scratch slots, and 300
+    weights (more than there are slots) quantized beside a replaying graph leave both sides' bits as
+    they are alone.  It works inside a capture too."""
+    hidden = 1024
+    x = randn_cpu((64, hidden), seed=1).cuda()
+    fw = Q.quantize_weight((randn_cpu((hidden, hidden), seed=2) * 0.02).cuda())
+    raw = [(randn_cpu((hidden, n), seed=n) * 0.02).cuda() for n in (16, 272, 8192)]
+    want = [Q.quantize_weight(w) for w in raw]
+    slots = dict(Q._next_slot)
+
+    def step():
+        y = x
+        for _ in range(8):
+            y = Q.linear(y, fw)
+        return y, Q.quantize_weight(raw[1]).data
+
+    with torch.cuda.stream(torch.cuda.Stream()):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step()
+    graph.replay()
+    torch.cuda.synchronize()
+    alone = [t.clone() for t in out]
+    assert torch.equal(u8(alone[1]), u8(want[1].data))
+    taken = dict(Q._next_slot)
+    assert taken != slots
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for i in range(100):
+        graph.replay()
+        with torch.cuda.stream(side):
+            got = [Q.quantize_weight(w) for w in raw]
+    torch.cuda.synchronize()
+    assert Q._next_slot == taken
+    for a, b in zip(out, alone):
+        assert torch.equal(u8(a), u8(b))
+    for a, b in zip(got, want):
+        assert torch.equal(u8(a.data), u8(b.data)) and torch.equal(u8(a.scale), u8(b.scale))
+    assert Q.device_status() == 0
