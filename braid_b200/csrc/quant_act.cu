@@ -256,7 +256,10 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
   // [0] full / [1] empty of the forward pass, [2] full / [3] empty of the backward pass
   __shared__ __align__(8) uint64_t bars[4][12];
   __shared__ unsigned int s_failed;
-  bq::pdl_launch_dependents();
+  // The GEMMs fetch their weights without waiting for the kernels before them.  The launch that
+  // writes a weight's codes therefore never lets a dependent start early: the next launch, and any
+  // behind it, starts when these codes are complete.
+  if constexpr (PHASE != kWeightCast) bq::pdl_launch_dependents();
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool producer = warp == kRingThreads / 32;

@@ -88,6 +88,8 @@ int bq_quantize_act(const void* x, int dtype, int64_t n, void* q_out, float* sca
  * bits, for callers that load weights while other streams decode.  Two launches that wait for no
  * other CTA and keep nothing between calls: `ws` is any bq_quantize_weight_workspace_bytes() bytes
  * of device memory, uninitialised, private to the call until the stream has passed it.  n % 8 == 0.
+ * A GEMM may follow on the same stream at once: the launch after this one starts only when the
+ * codes are complete (see `wq` of bq_gemm_w8a8).
  *
  * Replaces: braid/model/quant.py:139-154 (`quantize_weight`).
  */
@@ -297,7 +299,10 @@ size_t bq_gemm_workspace_bytes(int64_t M, int64_t N_total, int64_t K);
  * `torch._scaled_mm(xq, w.data.t(), scale_a=sx, scale_b=w.scale, out_dtype=...)`.
  *
  *   xq   device, [M,K] e4m3fn codes, contiguous, 16-byte aligned, K % 16 == 0
- *   wq   device, [N,K] e4m3fn codes, contiguous, 16-byte aligned, N % 16 == 0
+ *   wq   device, [N,K] e4m3fn codes, contiguous, 16-byte aligned, N % 16 == 0.  Read ahead of the
+ *        kernels before this one, here and in every entry point that takes weights: written by
+ *        bq_quantize_weight, by a copy or by kernels outside this library on the same stream, or
+ *        synchronised; never the codes of another quantizer of this library that may still run
  *   sx   device, one float (activation dequant scale)
  *   sw   device, one float (weight dequant scale)
  *   y    device, [M,N] of out_dtype, row stride ldy elements (ldy >= N)

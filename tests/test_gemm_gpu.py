@@ -701,3 +701,60 @@ def test_wide_greedy_pick_over_several_rounds(Q, wide, M):
     xq, sx = Q.quantize_act(x)
     assert torch.equal(logits, Q.fp8_matmul(xq, sx, w))
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("n,k", [(272, 1040), (1024, 512), (12288, 4096)])
+def test_a_fresh_weight_is_complete_before_a_queued_gemm_reads_it(Q, n, k):
+    """The GEMMs fetch weights ahead of the kernels before them.  With the host far ahead of the device,
+    quantize_weight -> GEMM -- directly, and with a quantizer or a norm in between -- must still see
+    whole weights: eagerly, where a weight's memory held another one's codes, and in a graph whose
+    source weights change between replays."""
+    srcs = [(randn_cpu((n, k), seed=10 + i) * 0.02).cuda() for i in range(4)]
+    x = randn_cpu((64, k), seed=1).cuda()
+    gamma = torch.ones(k, device="cuda")
+    xq, sx = Q.quantize_act(x)
+    busy = torch.randn(4096, 4096, device="cuda")
+
+    def chain(src, wait=lambda: None):
+        out = []
+        for rows in (8, 64):
+            q8, xr = xq[:rows], x[:rows]
+            w = Q.quantize_weight(src)
+            wait()
+            out.append(Q.fp8_matmul(q8, sx, w))
+            w = Q.quantize_weight(src)
+            wait()
+            out.append(Q.linear(xr, w))                                  # a quantizer in between
+            w = Q.quantize_weight(src)
+            wait()
+            out.append(Q.linear(Q.rms_norm_quant(xr, gamma, 1e-6), w))   # a norm in between
+            w = Q.quantize_weight(src)
+            wait()
+            out.append(Q.lm_head_argmax(xr, w))
+            g, u = Q.quantize_weight(src), Q.quantize_weight(src.neg())
+            wait()
+            if n % 64 == 0:
+                out.extend(Q.gate_up_silu_quant(q8, sx, g, u, torch.bfloat16) or ())
+        return out
+
+    want = [chain(s, torch.cuda.synchronize) for s in srcs]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for src, ref in zip(srcs, want):
+            for _ in range(8):
+                busy = (busy @ busy).clamp(-1, 1)                        # the device falls behind
+            for a, b in zip(chain(src), ref, strict=True):
+                assert torch.equal(u8(a), u8(b))
+    src = srcs[0].clone()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        chain(src)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain(src)
+    for s, ref in zip(srcs, want):
+        src.copy_(s)
+        graph.replay()
+        for a, b in zip(out, ref, strict=True):
+            assert torch.equal(u8(a), u8(b))
+    assert Q.device_status() == 0
