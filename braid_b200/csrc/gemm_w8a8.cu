@@ -207,13 +207,14 @@ struct EpilogueArgs {
   const PushParams* push;
 };
 
-// Four residual values of the output type, as raw bits (16 bytes cover the widest case).
+// Four residual values of the output type, as raw bits (16 bytes cover the widest case).  The residual
+// and the activation scale come from kernels this one runs ahead of: no `__ldg` (see ld_coherent4).
 __device__ __forceinline__ uint4 load_res4(const void* res, long long idx, int out_dtype) {
   uint4 r = make_uint4(0u, 0u, 0u, 0u);
   if (out_dtype == BQ_DTYPE_F32) {
-    r = __ldg(reinterpret_cast<const uint4*>(static_cast<const float*>(res) + idx));
+    r = ld_coherent16(static_cast<const float*>(res) + idx);
   } else {
-    const uint2 h = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(res) + idx));
+    const uint2 h = ld_coherent8(static_cast<const uint16_t*>(res) + idx);
     r.x = h.x; r.y = h.y;
   }
   return r;
@@ -256,6 +257,16 @@ __device__ __forceinline__ void reduce_store(const EpilogueArgs& e) {
   constexpr int kWarps = kStreamWarps;
   const int n4 = e.lane * 4;                 // 4 consecutive output columns
   for (int m0 = e.m_begin + e.warp; m0 < e.m_end; m0 += kWarps * kRows) {
+    // the residual first: these loads keep their place before the others'
+    uint4 rraw[RES ? kRows : 1];
+    if constexpr (RES) {
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        const int m = m0 + i * kWarps;
+        if (m < e.m_end && e.col_ok)
+          rraw[i] = load_res4(e.res, (long long)m * e.ld_res + e.row0 + n4, e.out_dtype);
+      }
+    }
     float4 v[kRows][SPLIT];
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
@@ -269,15 +280,6 @@ __device__ __forceinline__ void reduce_store(const EpilogueArgs& e) {
           else
             v[i][r] = ld_cluster_f4(map_to_cta(off, e.peer0 + r));
         }
-      }
-    }
-    uint4 rraw[RES ? kRows : 1];
-    if constexpr (RES) {
-#pragma unroll
-      for (int i = 0; i < kRows; ++i) {
-        const int m = m0 + i * kWarps;
-        if (m < e.m_end && e.col_ok)
-          rraw[i] = load_res4(e.res, (long long)m * e.ld_res + e.row0 + n4, e.out_dtype);
       }
     }
 #pragma unroll
@@ -645,7 +647,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   // the epilogue warps get here at once and have the scale ready long before
   // the accumulator is
   const float sw = dense ? 1.0f : __ldg(seg.sw);
-  const float sx_ready = dense ? 1.0f : __ldg(p.sx);
+  const float sx_ready = dense ? 1.0f : ld_coherent4(p.sx);
   bool ok = mbar_wait(accum_bar, 0);
   tc_fence_after();
   if (threadIdx.x == 0) BQ_STAMP(p, 4);
@@ -1222,7 +1224,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
       const int n0 = n_idx * n_step;
       if (!mbar_wait(acc_full(b), use_b & 1)) { ok = false; break; }
       tc_fence_after();
-      const float sx = __ldg(p.sx);
+      const float sx = ld_coherent4(p.sx);
       const float scale = sx * __ldg(seg.sw);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + b * kPairTile;
       const bool use_tma = seg.y_tma != 0;

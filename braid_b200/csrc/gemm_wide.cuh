@@ -111,13 +111,13 @@ __device__ __forceinline__ void add_res16(float (&v)[16], const T* res, bool wid
   alignas(16) T r[16];
   if constexpr (sizeof(T) == 4) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) reinterpret_cast<float4*>(r)[q] = __ldg(reinterpret_cast<const float4*>(res) + q);
+    for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(r)[q] = ld_coherent16(res + 4 * q);
   } else if (wide) {
-    reinterpret_cast<uint4*>(r)[0] = __ldg(reinterpret_cast<const uint4*>(res));
-    reinterpret_cast<uint4*>(r)[1] = __ldg(reinterpret_cast<const uint4*>(res) + 1);
+    reinterpret_cast<uint4*>(r)[0] = ld_coherent16(res);
+    reinterpret_cast<uint4*>(r)[1] = ld_coherent16(res + 8);
   } else {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) reinterpret_cast<uint2*>(r)[q] = __ldg(reinterpret_cast<const uint2*>(res) + q);
+    for (int q = 0; q < 4; ++q) reinterpret_cast<uint2*>(r)[q] = ld_coherent8(res + 4 * q);
   }
   // the intrinsic: a plain + would be contracted with the scaling multiply for fp32 outputs
 #pragma unroll
@@ -546,7 +546,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     const int rows = p.M - m0 < sh.m_half ? p.M - m0 : sh.m_half;   // may be <= 0 in a pair's second CTA
     const bool row_ok = row < rows;
     const bool warp_ok = Lanes::row0(quad) < rows;            // some lane of the warp holds a real row
-    const float sx = __ldg(p.sx);
+    const float sx = ld_coherent4(p.sx);
     float bv = 0.0f;
     int bi = kNoIndex;
     int round = 0;

@@ -57,8 +57,7 @@ constexpr int kRehearseRows = 32;   // see rmsnorm_quant_kernel; one CTA per row
 
 template <typename T> struct Vec4 { T v[kVec]; };
 
-// Coherent loads on purpose: the kernels run ahead of the one that writes `p`, and a load the
-// compiler takes for one of constant memory (__ldg) may be moved above the wait for it.
+// Coherent loads on purpose (see load8).
 template <typename T>
 __device__ __forceinline__ Vec4<T> load4(const T* p) {
   Vec4<T> r;
@@ -476,7 +475,7 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_scale_kernel(c
     const long long off = static_cast<long long>(head) * kHeadDim + lane * kVec;
     Vec4<T> core;
     if constexpr (Y_F32) {
-      const float4 f = __ldg(reinterpret_cast<const float4*>(
+      const float4 f = __ldcg(reinterpret_cast<const float4*>(
           reinterpret_cast<const float*>(p.y) + row * p.ld_y + off));
       core.v[0] = narrow<T>(f.x); core.v[1] = narrow<T>(f.y);
       core.v[2] = narrow<T>(f.z); core.v[3] = narrow<T>(f.w);

@@ -53,17 +53,13 @@ __global__ void __launch_bounds__(512, 1) quant_hold_kernel(const QParams p) {
   Pack8<T> other[MODE == kPlain ? 1 : MAXH];
   bq::pdl_wait_prior_grids();   // the activation is the previous kernel's output
   if (threadIdx.x == 0) BQ_STAMP(p, 2);
-  // a gathered buffer that peers store into while this kernel is resident is read with
-  // coherent loads, after the arrival wait
-  const bool coherent = p.wait_flag != nullptr;
-  if (coherent)
+  if (p.wait_flag != nullptr)   // a gathered buffer that peers store into while this kernel is resident
     grid_wait_arrivals(p.wait_flag, p.wait_seen, p.wait_count, static_cast<QuantWs*>(p.ws));
 #pragma unroll
   for (int i = 0; i < MAXH; ++i) {
     const unsigned int g = tid + static_cast<unsigned int>(i) * nthreads;
     if (i < p.held && g < p.n_groups) {
-      if (coherent) load_raw<T, MODE, true>(p, g, held[i], other[MODE == kPlain ? 0 : i]);
-      else load_raw<T, MODE, false>(p, g, held[i], other[MODE == kPlain ? 0 : i]);
+      load_raw<T, MODE>(p, g, held[i], other[MODE == kPlain ? 0 : i]);
     }
   }
   float m = 0.0f;
@@ -81,7 +77,7 @@ __global__ void __launch_bounds__(512, 1) quant_hold_kernel(const QParams p) {
   if (owns_tail) {
     const T* src = reinterpret_cast<const T*>(p.a) + static_cast<size_t>(p.n_groups) * kGroup;
     for (unsigned int i = 0; i < p.tail; ++i) {
-      tail_v[i] = widen(coherent ? __ldcg(src + i) : src[i]);
+      tail_v[i] = widen(__ldcg(src + i));
       m = nan_max(m, fabsf(tail_v[i]));
     }
   }
@@ -125,8 +121,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
   const unsigned int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned int nthreads = gridDim.x * blockDim.x;
   bq::pdl_wait_prior_grids();
-  const bool coherent = p.wait_flag != nullptr;
-  if (coherent)
+  if (p.wait_flag != nullptr)
     grid_wait_arrivals(p.wait_flag, p.wait_seen, p.wait_count, static_cast<QuantWs*>(p.ws));
   const bool owns_tail = (MODE == kPlain) && p.tail != 0 && tid == nthreads - 1;
   float sc;
@@ -140,8 +135,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       for (int u = 0; u < kUnroll; ++u) {
         const unsigned long long g = (unsigned long long)g0 + (unsigned long long)u * nthreads;
         if (g < p.n_groups) {
-          if (coherent) load_raw<T, MODE, true>(p, (unsigned int)g, a[u], b[MODE == kPlain ? 0 : u]);
-          else load_raw<T, MODE, false>(p, (unsigned int)g, a[u], b[MODE == kPlain ? 0 : u]);
+          load_raw<T, MODE>(p, (unsigned int)g, a[u], b[MODE == kPlain ? 0 : u]);
         }
       }
 #pragma unroll
@@ -156,7 +150,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
     if (owns_tail) {
       const T* src = reinterpret_cast<const T*>(p.a) + static_cast<size_t>(p.n_groups) * kGroup;
       for (unsigned int i = 0; i < p.tail; ++i)
-        m = nan_max(m, fabsf(widen(coherent ? __ldcg(src + i) : src[i])));
+        m = nan_max(m, fabsf(widen(__ldcg(src + i))));
     }
     sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
     if (tid == 0) p.scale[0] = sc;
@@ -175,8 +169,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       for (int u = 0; u < kUnroll; ++u) {
         const long long g = g0 + (long long)u * nthreads;
         if (g < (long long)p.n_groups) {
-          if (coherent) load_raw<T, MODE, true>(p, (unsigned int)g, a[u], b[MODE == kPlain ? 0 : u]);
-          else load_raw<T, MODE, false>(p, (unsigned int)g, a[u], b[MODE == kPlain ? 0 : u]);
+          load_raw<T, MODE>(p, (unsigned int)g, a[u], b[MODE == kPlain ? 0 : u]);
         }
       }
 #pragma unroll
@@ -192,12 +185,12 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       const T* src = reinterpret_cast<const T*>(p.a) + static_cast<size_t>(p.n_groups) * kGroup;
       uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;
       for (unsigned int i = 0; i < p.tail; ++i)
-        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(coherent ? __ldcg(src + i) : src[i]), dv),
+        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(src + i)), dv),
                                        __NV_SATFINITE, __NV_E4M3);
     }
   }
   if constexpr (PHASE != kCastOnly)
-    grid_depart(static_cast<QuantWs*>(p.ws), coherent ? p.wait_seen : nullptr, p.wait_count);
+    grid_depart(static_cast<QuantWs*>(p.ws), p.wait_flag != nullptr ? p.wait_seen : nullptr, p.wait_count);
 }
 
 // Sticky status of the launches that run without scratch words from the caller (the cast half alone,
@@ -367,14 +360,14 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
       if (owns_tail) {
         uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;
         for (unsigned int i = 0; i < p.tail; ++i)
-          dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(tail_src[i]), dv), __NV_SATFINITE, __NV_E4M3);
+          dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(tail_src + i)), dv), __NV_SATFINITE, __NV_E4M3);
       }
     } else if constexpr (PHASE == kMaxOnly) {
       m = cta_amax(m);
       if (threadIdx.x == 0) p.partial[blockIdx.x] = m;
     } else {
       if (owns_tail)
-        for (unsigned int i = 0; i < p.tail; ++i) m = nan_max(m, fabsf(widen(tail_src[i])));
+        for (unsigned int i = 0; i < p.tail; ++i) m = nan_max(m, fabsf(widen(__ldcg(tail_src + i))));
       if (threadIdx.x == 0) BQ_STAMP(p, 3);
       sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
       if (threadIdx.x == 0) BQ_STAMP(p, 4);
@@ -426,7 +419,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
     if (owns_tail) {
       uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;
       for (unsigned int i = 0; i < p.tail; ++i)
-        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(tail_src[i]), dv), __NV_SATFINITE, __NV_E4M3);
+        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(tail_src + i)), dv), __NV_SATFINITE, __NV_E4M3);
     }
   }
   // no bulk copy is in flight here unless a wait ran out: every issued copy was waited for by
@@ -461,7 +454,7 @@ __global__ void __launch_bounds__(256) prologue_dense_kernel(const QParams p, T*
   float m = 0.0f;
   for (unsigned long long g = blockIdx.x * blockDim.x + threadIdx.x; g < p.n_groups; g += nthreads) {
     Pack8<T> a, b;
-    load_raw<T, MODE, false>(p, (unsigned int)g, a, b);
+    load_raw<T, MODE>(p, (unsigned int)g, a, b);
     apply_prologue<T, MODE, true>(a, b);
     m = absmax8(a, m);
     if constexpr (sizeof(T) == 4) {
@@ -531,8 +524,8 @@ __global__ void __launch_bounds__(256) row_push_kernel(const RowPush p) {
       // two groups per thread, one 16-byte store per destination: a warp writes 512 contiguous
       // bytes of the row on every rank
       for (int g = 2 * threadIdx.x; g < p.groups_per_row; g += 2 * blockDim.x) {
-        const Pack8<T> v0 = load8<T, false>(src + g * kGroup);
-        const Pack8<T> v1 = load8<T, false>(src + (g + 1) * kGroup);
+        const Pack8<T> v0 = load8<T>(src + g * kGroup);
+        const Pack8<T> v1 = load8<T>(src + (g + 1) * kGroup);
         const uint2 c0 = codes8<T, false>(v0, dv), c1 = codes8<T, false>(v1, dv);
         const uint4 c = make_uint4(c0.x, c0.y, c1.x, c1.y);
         const long long at = (long long)row * p.ld_dst + g * kGroup;
@@ -541,7 +534,7 @@ __global__ void __launch_bounds__(256) row_push_kernel(const RowPush p) {
       continue;
     }
     for (int g = threadIdx.x; g < p.groups_per_row; g += blockDim.x) {
-      const Pack8<T> v = load8<T, false>(src + g * kGroup);
+      const Pack8<T> v = load8<T>(src + g * kGroup);
       const long long at = (long long)row * p.ld_dst + g * kGroup;
       if constexpr (CAST) {
         const uint2 c = codes8<T, false>(v, dv);

@@ -64,22 +64,21 @@ template <> __device__ __forceinline__ __nv_bfloat16 narrow<__nv_bfloat16>(float
 // NaN-propagating max: once either side is NaN the result is NaN.
 __device__ __forceinline__ float nan_max(float m, float v) { return (v != v || v > m) ? v : m; }
 
-// COHERENT = false: read-only path (`ld.global.nc`), for inputs nobody writes while the kernel
-// is resident.  COHERENT = true: L2-coherent loads (`ld.global.cg`), for a gathered buffer that
-// other GPUs (and this GPU's own push launch) are still storing into while this kernel waits
-// for their arrival -- the non-coherent path promises nothing for such data.
-template <typename T, bool COHERENT = false>
+// What an earlier kernel writes is read with `ld.global.cg` (volatile to the compiler): the kernels
+// run ahead of that kernel, and a load of what the compiler takes for constant memory (`__ldg`)
+// may be moved above the wait for it.  For gathered buffers the load also has to see what other
+// GPUs stored while this kernel was waiting for their arrival.
+template <typename T>
 __device__ __forceinline__ Pack8<T> load8(const T* p) {
   Pack8<T> r;
   if constexpr (sizeof(T) == 4) {
     const float4* q = reinterpret_cast<const float4*>(p);
-    const float4 lo = COHERENT ? __ldcg(q) : __ldg(q);
-    const float4 hi = COHERENT ? __ldcg(q + 1) : __ldg(q + 1);
+    const float4 lo = __ldcg(q);
+    const float4 hi = __ldcg(q + 1);
     r.v[0] = lo.x; r.v[1] = lo.y; r.v[2] = lo.z; r.v[3] = lo.w;
     r.v[4] = hi.x; r.v[5] = hi.y; r.v[6] = hi.z; r.v[7] = hi.w;
   } else {
-    const uint4* q = reinterpret_cast<const uint4*>(p);
-    const uint4 raw = COHERENT ? __ldcg(q) : __ldg(q);
+    const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(p));
     *reinterpret_cast<uint4*>(&r) = raw;
   }
   return r;
@@ -282,10 +281,10 @@ __device__ __forceinline__ void gated_product(float (&gated)[N], const float (&o
 }
 
 // Raw operands of one group: one 8-pack for the plain mode, two for the prologues.
-template <typename T, int MODE, bool COHERENT = false>
+template <typename T, int MODE>
 __device__ __forceinline__ void load_raw(const QParams& p, unsigned int g, Pack8<T>& a, Pack8<T>& b) {
   if constexpr (MODE == kPlain) {
-    a = load8<T, COHERENT>(reinterpret_cast<const T*>(p.a) + static_cast<size_t>(g) * kGroup);
+    a = load8<T>(reinterpret_cast<const T*>(p.a) + static_cast<size_t>(g) * kGroup);
   } else {
     const unsigned int row = g / p.groups_per_row;
     const unsigned int col = (g - row * p.groups_per_row) * kGroup;
@@ -298,8 +297,8 @@ __device__ __forceinline__ void load_raw(const QParams& p, unsigned int g, Pack8
       pb = reinterpret_cast<const T*>(p.b) + static_cast<long long>(row) * p.ld_b +
            static_cast<long long>(head) * p.chunk_stride + (col - head * p.chunk);
     }
-    a = load8<T, COHERENT>(pa);
-    b = load8<T, COHERENT>(pb);
+    a = load8<T>(pa);
+    b = load8<T>(pb);
   }
 }
 

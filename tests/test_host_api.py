@@ -260,3 +260,19 @@ def test_push_entry_points_check_their_arguments():
                                  None, 0, None) == _lib.BQ_ERR_BAD_ARG
     assert lib.bq_peer_open(None, None) == _lib.BQ_ERR_BAD_ARG
     assert lib.bq_peer_alloc(0, None, None) == _lib.BQ_ERR_BAD_ARG
+
+
+def test_the_read_only_load_path_is_kept_for_load_time_constants():
+    """Kernels start ahead of the ones whose outputs they read; a load the compiler takes for one of
+    constant memory (`__ldg`) may be moved above the wait.  Only norm weights and weight scales,
+    which no kernel of a forward pass writes, may be read that way."""
+    csrc = ROOT / "braid_b200" / "csrc"
+    seen = 0
+    for f in sorted(csrc.iterdir()):
+        for i, line in enumerate(f.read_text().splitlines(), 1):
+            code = line.split("//")[0]
+            assert "ld.global.nc" not in code, f"{f.name}:{i}"
+            for arg in re.findall(r"__ldg\((.*)", code):
+                seen += 1
+                assert re.match(r"reinterpret_cast<const float4\*>\(p\.gamma\)|seg\.sw\)|p\.pair\.sw_up\)", arg), f"{f.name}:{i}: {line}"
+    assert seen > 0
