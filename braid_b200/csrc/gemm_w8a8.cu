@@ -1738,10 +1738,10 @@ int plan_wide(GemmParams& p, WideShape& sh, bool flat) {
     int a_stages = 98304 / a_bytes;
     if (a_stages < 4) a_stages = 4;
     if (a_stages > 16) a_stages = 16;
-    if (g_opt_b_stages > 0) a_stages = (int)g_opt_b_stages;
+    if (g_opt_b_stages > 0) a_stages = g_opt_b_stages < kWideMaxA ? (int)g_opt_b_stages : kWideMaxA;
     if (a_stages > want) a_stages = want;
     int w_stages = (budget - a_stages * a_bytes) / w_bytes;
-    if (w_stages > 40) w_stages = 40;
+    if (w_stages > kWideMaxW) w_stages = kWideMaxW;
     if (w_stages > want) w_stages = want;
     if (g_opt_stages > 0 && w_stages > g_opt_stages) w_stages = (int)g_opt_stages;
     if (w_stages < 1) return kErrUnsupported;

@@ -51,6 +51,10 @@ struct WideShape {
 
 constexpr int kWideThreads = 384;     // warps 0 / 1 / 2 load weights, issue MMAs, load activations
 constexpr int kWideWarps = kWideThreads / 32;
+// Deepest rings: two barriers per weight slot, one per activation slot and four for the accumulators
+// lie before the last 128 bytes of the barrier area (tensor-memory slot, abort flag, s_red).
+constexpr int kWideMaxW = 40, kWideMaxA = 28;
+static_assert(8 * (2 * kWideMaxW + kWideMaxA + 4) <= kBarrierBytes - 128, "the barriers overrun the flags");
 
 // Where the accumulators of a CTA's batch rows lie in tensor memory (lanes x columns):
 //   pair of 128   rows 0..63 in lanes 0..63 (columns of CTA 0's weight rows) and again in lanes

@@ -676,6 +676,24 @@ def test_wide_batches_on_cta_pairs_agree_with_the_k_sliced_kernel(Q, M, ns, K):
     assert Q.device_status() == 0
 
 
+def test_forced_ring_depths_leave_the_flags_of_the_wide_kernel_alone(Q, wide):
+    """The deepest rings that options can ask for: 40 weight stages and as many activation stages as
+    the barrier area has room for (its last bytes hold the tensor-memory address)."""
+    M, n, K = 8, 48, 41 * 128 + 16
+    x = randn_cpu((M, K), seed=1).cuda()
+    xq, sx = Q.quantize_act(x)
+    w = Q.quantize_weight((randn_cpu((n, K), seed=2) * 0.02).cuda())
+    base = Q.fp8_matmul(xq, sx, w, out_dtype=torch.float32)
+    try:
+        for depth in (28, 29, 40, 1000):
+            Q.set_option("decode_b_stages", depth)
+            assert torch.equal(base, Q.fp8_matmul(xq, sx, w, out_dtype=torch.float32))
+            assert Q.last_gemm_launch()["stages"] == 40
+    finally:
+        Q.set_option("decode_b_stages", 0)
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("M,I,K,dt", [(33, 64, 128, torch.bfloat16), (64, 4736, 1040, torch.float16),
                                       (96, 1024, 2048, torch.float32), (130, 192, 256, torch.bfloat16),
                                       (256, 12288, 1024, torch.bfloat16)])
