@@ -1786,8 +1786,8 @@ int launch_wide(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_opt_pdl ? 2 : 1;
-  g_last_launch[0] = 0; g_last_launch[1] = sh.grid; g_last_launch[2] = p.seg[0].split;
-  g_last_launch[3] = sh.ring[0].w_stages; g_last_launch[4] = smem; g_last_launch[5] = p.seg[0].un;
+  g_last_launch[0] = 1; g_last_launch[1] = sh.grid; g_last_launch[2] = p.seg[0].split;
+  g_last_launch[3] = sh.ring[0].w_stages; g_last_launch[4] = smem; g_last_launch[5] = 64 << sh.mode;
   g_argmax_slots = argmax_slots(sh);
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);

@@ -588,8 +588,9 @@ int bq_set_option(const char* key, int64_t value);
 
 /*
  * Describes the launch the last GEMM call on this thread chose:
- * out[0]=kernel (0 weight-streaming cluster kernel, 2 CTA-pair tile kernel) out[1]=grid out[2]=cluster/split
- * out[3]=stages out[4]=dynamic smem bytes out[5]=batch tile (MMA N)
+ * out[0]=kernel (decode: 0 K-sliced cluster kernel, 1 CTA-pair kernel; prefill: 2 CTA-pair tile kernel)
+ * out[1]=grid out[2]=K slices (0: of the cluster; 1: of the first weight) out[3]=stages (of the weight ring)
+ * out[4]=dynamic smem bytes out[5]=batch rows of one MMA (0, 1) or weight rows of one tile (2)
  */
 int bq_last_gemm_launch(int64_t out[6]);
 

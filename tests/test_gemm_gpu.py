@@ -652,6 +652,7 @@ def test_wide_batches_on_cta_pairs_agree_with_the_k_sliced_kernel(Q, M, ns, K):
             for wide in (1, 0):
                 Q.set_option("decode_wide", wide)
                 out.append(fn())
+                assert Q.last_gemm_launch()["wide"] == bool(wide)
         finally:
             Q.set_option("decode_wide", -1)
         return out
@@ -688,7 +689,7 @@ def test_forced_ring_depths_leave_the_flags_of_the_wide_kernel_alone(Q, wide):
         for depth in (28, 29, 40, 1000):
             Q.set_option("decode_b_stages", depth)
             assert torch.equal(base, Q.fp8_matmul(xq, sx, w, out_dtype=torch.float32))
-            assert Q.last_gemm_launch()["stages"] == 40
+            assert Q.last_gemm_launch()["stages"] == 40 and Q.last_gemm_launch()["wide"]
     finally:
         Q.set_option("decode_b_stages", 0)
     assert Q.device_status() == 0
@@ -702,6 +703,7 @@ def test_wide_gate_up_codes_equal_the_separate_kernels(Q, wide, M, I, K, dt):
     xq, sx = Q.quantize_act(x)
     g, u = (Q.quantize_weight((randn_cpu((I, K), seed=s) * 0.05).cuda()) for s in (2, 3))
     got = Q.gate_up_silu_quant(xq, sx, g, u, dt)
+    assert Q.last_gemm_launch()["wide"]
     gate, up = Q.fp8_matmul_grouped(xq, sx, (g, u), out_dtype=dt)
     q, s = Q.silu_mul_quant(gate, up)
     assert got is not None and torch.equal(got[1], s) and torch.equal(u8(got[0]), u8(q))
@@ -715,9 +717,48 @@ def test_wide_greedy_pick_over_several_rounds(Q, wide, M):
     w.data.view(torch.uint8)[V - 16:] = w.data.view(torch.uint8)[:16]      # equal logits: the lower index wins
     x = randn_cpu((M, K), seed=M).cuda()
     idx, logits = Q.lm_head_argmax(x, w, return_logits=True)
+    assert Q.last_gemm_launch()["wide"]
     assert torch.equal(idx.flatten(), logits.argmax(-1).flatten())
     xq, sx = Q.quantize_act(x)
     assert torch.equal(logits, Q.fp8_matmul(xq, sx, w))
+    assert Q.device_status() == 0
+
+
+def test_what_the_wide_kernel_has_no_layout_for_runs_on_the_k_sliced_one(Q, wide):
+    """A vocabulary so small that the picks of the unit walkers do not fit the caller's scratch (a pair
+    per row and 128 vocabulary rows), with the option that asks for the wide kernel."""
+    x = randn_cpu((64, 256), seed=1).cuda()
+    w = Q.quantize_weight((randn_cpu((1024, 256), seed=2) * 0.02).cuda())
+    idx, logits = Q.lm_head_argmax(x, w, return_logits=True)
+    assert not Q.last_gemm_launch()["wide"]
+    assert torch.equal(idx.flatten(), logits.argmax(-1).flatten())
+    # gate and up of more rows than one round of units holds: refused, as without the option
+    xq, sx = Q.quantize_act(x)
+    g, u = (Q.quantize_weight((randn_cpu((20480, 256), seed=s) * 0.05).cuda()) for s in (3, 4))
+    assert Q.gate_up_silu_quant(xq, sx, g, u, torch.bfloat16) is None
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("M", [33, 64, 200])
+@pytest.mark.parametrize("K", [192, 1040, 4096])
+def test_wide_16_bit_segments_over_several_rounds(Q, wide, M, K):
+    """Segments of 16-bit weights beside FP8 ones in a launch of more units than are resident: both kinds
+    share one ring layout, the first and the last unit of a walker may be of either kind."""
+    dt = torch.bfloat16
+    x = randn_cpu((M, K), seed=M + K, dtype=dt).cuda()
+    a, b = (randn_cpu((n, K), seed=n, dtype=dt, scale=0.02).cuda() for n in (32, 272))
+    w = Q.quantize_weight(randn_cpu((40960, K), seed=1, dtype=dt, scale=0.02).cuda())
+    ya, yw, yb = Q.project(x, a, w, b)
+    launch = Q.last_gemm_launch()
+    assert launch["wide"] and launch["grid"] % 2 == 0 and 40960 // 256 > launch["grid"] // 2   # several rounds
+    xq, sx = Q.quantize_act(x)
+    assert torch.equal(yw, Q.fp8_matmul(xq, sx, w, out_dtype=dt))
+    for y, d in ((ya, a), (yb, b)):
+        # products of 16-bit values are exact in fp32; what is left is one rounding to the output type
+        # and fp32 sums of K products
+        ref = x.double() @ d.double().t()
+        bound = 2.0 ** -8 * ref.abs() + K * 2.0 ** -22 * (x.double().abs() @ d.double().abs().t())
+        assert ((y.double() - ref).abs() <= bound).all()
     assert Q.device_status() == 0
 
 
