@@ -35,6 +35,7 @@ from collections.abc import Iterable, Sequence
 from dataclasses import dataclass
 
 import torch
+import torch.autograd.forward_ad as forward_ad
 import torch.nn.functional as F
 
 from . import _lib
@@ -101,6 +102,14 @@ def _weight_scale(t: torch.Tensor) -> torch.Tensor:
 _CAST_CHUNK_BYTES = 256 * 2 ** 20
 
 
+def _transformed() -> bool:
+    """Is this call seen through a dispatch mode (make_fx, fake tensors), a functorch transform
+    (functionalize, jvp), forward-mode differentiation or a tracer?  Those follow torch operations
+    only, and their tensors may have no memory behind `data_ptr()`."""
+    return (torch._C._len_torch_dispatch_stack() > 0 or torch._C._functorch.maybe_current_level() is not None
+            or forward_ad._current_level >= 0 or torch.jit.is_tracing())
+
+
 def _quantize_weight_fused(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor] | None:
     """Codes and scale of a weight from two launches of the ring kernel (`quant_act.cu`): every CTA's
     max |w|, then the cast under their maximum.  Scale and codes are the bits of the torch
@@ -111,9 +120,9 @@ def _quantize_weight_fused(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]
 
     `None` -- the torch spelling -- for whatever the kernels do not take: no CUDA tensor of the current
     device, another type, a strided or unaligned view, a weight that records gradients, a tensor
-    subclass (tracing), no library, or the parity arm."""
+    subclass, a call that is traced or transformed, no library, or the parity arm."""
     if (type(w) not in (torch.Tensor, torch.nn.Parameter) or not w.is_cuda or w.dtype not in _DTYPE_CODE
-            or not w.is_contiguous() or w.data_ptr() % 16 or w.numel() == 0 or _quantizers_off()
+            or _transformed() or w.is_neg() or not w.is_contiguous() or w.data_ptr() % 16 or w.numel() == 0 or _quantizers_off()
             or (w.requires_grad and torch.is_grad_enabled())
             or w.device.index != torch.cuda.current_device()):
         return None

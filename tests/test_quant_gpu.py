@@ -464,3 +464,30 @@ def test_weights_load_on_a_side_stream_while_a_graph_replays(Q):
     for a, b in zip(got, want):
         assert torch.equal(u8(a.data), u8(b.data)) and torch.equal(u8(a.scale), u8(b.scale))
     assert Q.device_status() == 0
+
+
+def test_quantize_weight_can_be_traced_and_transformed(Q):
+    """A call that is seen through a tracer or a transform takes the torch spelling: a kernel launched
+    by pointer is invisible to them, and a functional tensor's pointer is no memory."""
+    import torch.autograd.forward_ad as fwad
+    from torch.fx.experimental.proxy_tensor import make_fx
+    a, b = ((randn_cpu((32, 48), seed=s) * 0.02).cuda() for s in (1, 2))
+
+    def f(w):
+        r = Q.quantize_weight(w)
+        return r.data, r.scale
+
+    def same(got, w):
+        return all(torch.equal(u8(x), u8(y)) for x, y in zip(got, f(w), strict=True))
+
+    assert Q._quantize_weight_fused(a) is not None
+    assert same(make_fx(f)(a)(b), b)
+    assert same(torch.jit.trace(f, (a,), check_trace=False)(b), b)
+    assert same(torch.func.functionalize(f)(b), b)
+    with fwad.dual_level():
+        assert Q._quantize_weight_fused(fwad.make_dual(b, a)) is None
+    assert torch.func.jvp(lambda w: Q.quantize_weight(w).scale, (b,), (a,))[0].equal(f(b)[1])
+    neg = torch._neg_view(b)
+    assert same(f(neg), b.neg())
+    with pytest.raises(RuntimeError):          # as with the torch spelling
+        torch.func.vmap(f)(torch.stack([a, b]))
