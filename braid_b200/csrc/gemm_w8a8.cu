@@ -1873,19 +1873,49 @@ struct DenseArgs {
 };
 
 // Which launches the wide kernel takes: batches that fill its MMA shape (128 rows, or 256) well enough.
-// K-sliced kernel / wide kernel in us, graphed, one decoder layer of hidden 4096 (and 2560):
-//     48 rows 78.6 / 76.3 (69.8 / 69.3)      56 rows 83.1 / 77.4 (71.9 / 70.9)     64 rows 83.5 / 76.4
-//    128 rows 91.5 / 82.8                   144 rows 95.6 / 96.0                  160 rows 98.6 / 98.1
-//    176 rows 108.8 / 99.6 (92.7 / 86.4)    256 rows 166.3 / 104.1 (137.4 / 104.3)
-// with the MLP alone at 40 and 48 rows 0.94 to 0.99 as fast here and at 129 to 160 0.94 to 1.00.
-// Weights of several rounds (a vocabulary) pay an epilogue per round: where K is long it is hidden and
-// the line lies lower (124000 x 4096: 32 rows 103.1 / 92.8, 40 rows 106.7 / 89.4, 136 rows
-// 155.5 / 124.7; 60016 x 4096: 54.0 / 54.8, 57.0 / 54.0, 81.3 / 69.2), where K is short higher
-// (60016 x 1024: 48 rows 32.5 / 39.1, 64 rows 36.6 / 38.6, 136 rows 50.9 / 55.0, 256 rows 123.7 / 56.8).
+// All figures are the K-sliced kernel's time over this one's, graphed, weights from HBM (banks larger
+// than L2); where a line says nothing, it lies between 1.0 and 1.4, beyond 208 rows up to 2.5.
+//
+// One round.  One decoder layer of hidden 1024 / 2048 / 2560 / 4096 / 5120: 33 to 48 rows 1.03 / 1.00 / 0.99 /
+// 1.00 / 1.04, 49 rows 1.09 / 1.03 / 1.01 / 1.06 / 1.07, 128 rows 1.21 / 1.13 / 1.09 / 1.10 / 1.09, 129 rows
+// 1.15 / 1.04 / 1.00 / 0.98 / 0.99, 161 rows 1.20 / 1.11 / 1.07 / 1.09 / 1.14: 49 rows on, without 129 to 160.
+// Within that, what the K-sliced kernel does better:
+//  * gate/up in units of more than 128 columns up to 80 rows, where SiLU is the longer part
+//    (K = 4096, 16384 columns: 49 rows 0.96, 65 rows 0.98; 128-column units 1.02);
+//  * weights of many rows and short K up to 80 rows (9472 x 1024: 49 rows 0.87);
+//  * units of 256 weight rows beyond 160 rows, whose epilogue nothing hides unless K is long
+//    (18944 x 2048: 0.94 to 0.97; x 4096: 0.96 to 0.98, 256 rows 1.05; x 12288: 1.06);
+//  * few rows and long K beyond 160 rows: one thread's chain of MMAs against a quarter of it
+//    (1024 x 7680: 161 rows 0.96, 208 rows 1.04; 4096 x 12288: 0.93, 224 rows 0.99, 240 rows 1.03).
+//
+// Several rounds (a vocabulary) pay an epilogue per round.  Where K is long it is hidden (60016 x 4096:
+// 33 rows 1.05, 129 rows 1.09), where K is short the batch has to be larger (60016 x 1024: 65 rows 1.14,
+// 129 rows 1.06).  The K-sliced kernel holds up to two CTAs per SM at once; while its tiles fit and fill
+// three quarters of that room, only its wide accumulators (more than 96 rows, and again more than 160) are
+// slower (32000 x 4096: 49 rows 0.95, 97 rows 1.01, 129 rows 0.88, 161 rows 1.06; 24576 x 4096: 1.08,
+// 1.12, 0.97, 1.24), and with K below 1536 only those that no longer fit twice (20480 x 1024: 65 rows
+// 0.80, 192 rows 0.95, 256 rows 1.62).
 bool wide_applies(const GemmParams& p, const WideShape& sh) {
   if (g_opt_wide >= 0) return g_opt_wide != 0;
-  if (sh.rounds > 1 && p.k_blocks >= 16) return p.M > 32;
-  return p.M > (sh.rounds > 1 ? 64 : 48) && (p.M <= 128 || p.M > 160);
+  const int sms = device_sms();
+  long long ctas = 0;                                  // of the K-sliced kernel
+  for (int i = 0; i < p.n_seg; ++i)
+    ctas += (long long)((p.seg[i].n + kRowTile - 1) / kRowTile) * p.seg[i].split;
+  const bool between = p.M > 128 && p.M <= 160;
+  const bool short_k = p.k_blocks < 12;
+  if (sh.rounds > 1) {
+    if (ctas <= 2 * sms && short_k) return p.M > 208;
+    if (ctas <= 2 * sms && 2 * ctas > 3 * sms && p.k_blocks >= 16) return p.M > 96 && !between;
+    return p.k_blocks >= 16 ? p.M > 32 : p.M > 64 && !between;
+  }
+  if (p.M <= 48 || between) return false;
+  const int un = p.seg[0].un;
+  if (p.pair.on) return un <= 128 || p.M > 80;
+  if (short_k && un >= 128 && p.M <= 80) return false;
+  if (un > 224 && p.M > 160) return p.k_blocks >= 64 || (p.k_blocks >= 32 && p.M > 192);
+  if (p.seg[0].split == 4 && ctas <= sms && p.k_blocks > 48 && p.M > 160)
+    return p.M > (p.k_blocks > 64 ? 224 : 192);
+  return true;
 }
 
 // The launch on the wide kernel; kErrUnsupported where it has no layout for it or the K-sliced one is

@@ -724,6 +724,40 @@ def test_wide_greedy_pick_over_several_rounds(Q, wide, M):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("n,k,on,off", [
+    (4096, 4096, (49, 128, 161, 256), (48, 129, 160)),        # one round
+    (9472, 1024, (81,), (64, 80)),                            # many rows, short K
+    (18944, 1024, (), (161, 256)), (18944, 4096, (160 + 33,), (192,)), (18944, 8192, (161,), ()),   # 256-row units
+    (1024, 6144, (161,), ()), (1024, 7680, (193,), (161, 192)), (1024, 12288, (225,), (224,)),    # long K, few rows
+    (20480, 1024, (209,), (65, 208)), (32000, 1536, (65, 161), (64, 129)),                        # two rounds
+    (32000, 2048, (97, 161), (96, 129)), (24576, 2048, (33, 129), (32,)), (49152, 2048, (33, 129), (32,))])
+def test_which_decode_batches_run_on_cta_pairs(Q, n, k, on, off):
+    """Both sides of every line of the dispatch; whichever kernel is taken gives its own bits."""
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    data = torch.randint(0, 120, (n, k), generator=g, device="cuda", dtype=torch.uint8)
+    w = Q.FP8Weight(data=data.view(Q.FP8), scale=torch.full((1, 1), 1e-3, device="cuda"), shape=(n, k))
+    torch.cuda.synchronize()
+    for M, wide in [(m, True) for m in on] + [(m, False) for m in off]:
+        xq, sx = Q.quantize_act(randn_cpu((M, k), seed=M).cuda())
+        y = Q.fp8_matmul(xq, sx, w)
+        assert Q.last_gemm_launch()["wide"] == wide, f"{M} x {n} x {k}"
+        try:
+            Q.set_option("decode_wide", int(wide))
+            assert torch.equal(y, Q.fp8_matmul(xq, sx, w))
+        finally:
+            Q.set_option("decode_wide", -1)
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("M,I,wide", [(64, 16384, False), (80, 16384, False), (81, 16384, True), (49, 9472, True)])
+def test_which_gate_up_batches_run_on_cta_pairs(Q, M, I, wide):
+    xq, sx = Q.quantize_act(randn_cpu((M, 256), seed=M).cuda())
+    g, u = (Q.quantize_weight((randn_cpu((I, 256), seed=s) * 0.05).cuda()) for s in (1, 2))
+    assert Q.gate_up_silu_quant(xq, sx, g, u, torch.bfloat16) is not None
+    assert Q.last_gemm_launch()["wide"] == wide
+    assert Q.device_status() == 0
+
+
 def test_what_the_wide_kernel_has_no_layout_for_runs_on_the_k_sliced_one(Q, wide):
     """A vocabulary so small that the picks of the unit walkers do not fit the caller's scratch (a pair
     per row and 128 vocabulary rows), with the option that asks for the wide kernel."""
