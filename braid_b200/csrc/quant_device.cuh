@@ -203,9 +203,10 @@ template <typename T> __device__ __forceinline__ T sigmoid_to(float x) {
 // The same two functions of N values, the rounding to T left to the caller.
 // For 16-bit T the division is a reciprocal estimate and one residual correction of the quotient
 // (q = x y, q + (x - d q) y; Markstein, IBM J. Res. Dev. 34(1), 1990): with |x| <= 80 the divisor lies
-// in [1, 2^116] and nothing leaves the normal range, and x takes only 65,536 values, all of which
-// were compared on the device: the fp32 quotients are the IEEE ones, bit for bit, for both
-// functions and both types.  (-0 needs the sign put back.)  Values beyond 80, infinities and NaN
+// in [1, 2^116] and nothing leaves the normal range, and x takes only 65,536 values: the fp32
+// quotients are the IEEE ones, bit for bit (tested for SiLU down to quotients of 2^-120, where its
+// fp32 value is used; for the value rounded to T over all inputs of both functions and types).
+// (-0 needs the sign put back.)  Values beyond 80, infinities and NaN
 // take the division itself, decided once per group of N.  For the kernels that run the arithmetic
 // many times over; those of small decode batches run it once from a cold instruction cache, where
 // the shorter code of silu_to / sigmoid_to is the faster one (four graphed decoder layers of 27 fp16

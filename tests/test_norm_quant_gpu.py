@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import pytest
 import torch
+import torch.nn.functional as F
 
 from oracle import torch_spelling as TS
 from _util import randn_cpu, u8
@@ -277,3 +278,46 @@ def test_norms_behind_a_running_gemm_read_its_output(Q, rows, dt):
         for got, want in zip(out, ref):
             assert torch.equal(u8(got), u8(want))
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+def test_silu_of_the_looped_gated_norm_is_the_ieee_quotient(Q, lib, dt):
+    """The looped kernel multiplies the fp32 quotient z / (1 + exp(-z)) by gamma before it rounds to 16
+    bits, and takes that quotient without the division instruction up to |z| = 80.  For every such z a
+    gamma is chosen whose product lands one fp32 step below a rounding boundary of the 16-bit type,
+    and one that lands on it: a quotient one step too large or too small changes the output."""
+    z = torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(dt)
+    z = z[z.float().abs() <= 80]
+    s = F.silu(z.cuda().float()).cpu()                 # fp32, expf, an IEEE division
+    keep = s.abs() >= 2.0 ** -120                      # gamma stays finite
+    z, s = z[keep], s[keep].double()
+    ulp = 2.0 ** -7 if dt is torch.bfloat16 else 2.0 ** -10
+    for above in (False, True):
+        wrong = torch.nextafter(s.float(), torch.zeros(()) if above else torch.full((), torch.inf).copysign(s.float()))
+        gamma, want = torch.zeros(len(s)), torch.zeros(len(s))
+        sharp = torch.zeros(len(s), dtype=torch.bool)
+        for i in range(16):
+            upper = 1.9375 - 2 * i * ulp               # even: the boundary itself rounds to it
+            tie = upper - ulp / 2
+            target = tie if above else tie - 2.0 ** -23
+            for step in range(-3, 4):
+                g = ((target / s) * (1 + step * 2.0 ** -24)).float()
+                hit = (g.double() * s).float() == target           # exact products, one rounding
+                hit &= ((g.double() * wrong.double()).float() >= tie) != above
+                gamma = torch.where(hit & ~sharp, g, gamma)
+                want = torch.where(hit & ~sharp, upper if above else upper - ulp, want)
+                sharp |= hit
+        assert sharp.float().mean() > 0.99             # (a few quotients have no such gamma)
+        zs, gs, want = z[sharp], gamma[sharp], want[sharp]
+        whole = torch.arange(-(-len(zs) // 128) * 128) % len(zs)   # the last row filled from the front
+        zs, gs, want = zs[whole].cuda().reshape(-1, 128), gs[whole].cuda().reshape(-1, 128), want[whole]
+        y = torch.ones(1, 128, device="cuda", dtype=dt)
+        h, scale = torch.empty_like(zs), torch.empty(1, device="cuda")
+        ws = torch.zeros(16, dtype=torch.uint8, device="cuda")
+        stream = torch.cuda.current_stream().cuda_stream
+        code = {torch.bfloat16: 1, torch.float16: 2}[dt]
+        for i in range(len(zs)):
+            assert lib.bq_gated_rmsnorm_scale(y.data_ptr(), code, 128, zs[i].data_ptr(), code, 128, gs[i].data_ptr(), 0.0,
+                                              1, 1, 128, h[i].data_ptr(), 128, scale.data_ptr(), ws.data_ptr(), 16,
+                                              stream) == 0
+        assert torch.equal(h.float().cpu().flatten(), want)
