@@ -583,12 +583,13 @@ def main():
     n1 = Q.launch_count()
     g_gemm, _ = capture(lambda: ps.gemms_only_b200(xq, sx, coreq, oq, hq, bufs))
     gemm_launches = (Q.launch_count() - n1) // 4
+    gemm_kernel = "gemm_wide_kernel" if Q.last_gemm_launch()["wide"] else "gemm_stream_kernel"
     ms_gemm, _ = timed_replays(g_gemm.replay, args.steps, args.warmup, dist=None)
     peaks = measured_peaks()
     gemm_bytes = ps.gemm_algorithmic_bytes()
     achieved = gemm_bytes / (ms_gemm / args.steps * 1e-3) / 1e9
     traffic = ps.gemm_measured_traffic_bytes()
-    roofline = {"bound": "hbm", "kernel": "gemm_stream_kernel", "achieved": achieved,
+    roofline = {"bound": "hbm", "kernel": gemm_kernel, "achieved": achieved,
                 "peak": peaks["hbm_gbs"], "peak_source": peaks["source"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"],
                 "traffic": traffic["bytes"] / max(1, gemm_launches),

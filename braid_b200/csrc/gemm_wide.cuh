@@ -14,9 +14,11 @@
 // what loading its M rows costs (measured 22 and 40 clocks for N <= 32 x K = 32), and a CTA issues
 // K / 32 of them one after another.  That chain is why small batches stay on the K-sliced kernel
 // (gemm_w8a8.cu): a 64-row form of this one took 3.6 us instead of 2.5 from the activation's arrival
-// to the last MMA of a 4096 x 4096 weight, and four graphed decoder layers 254.6 instead of 245.0 us
-// at 1 row, 290.3 instead of 288.1 at 27.  At 128 rows they take 344 instead of 379 us here, a
-// 248320-row vocabulary 178 instead of 233 us at 64 rows and 267 instead of 665 at 256.
+// to the last MMA of a 4096 x 4096 weight; four graphed decoder layers were 4 % slower with it at
+// 1 row and 1 % at 27, and it was not kept.  At 128 rows those layers (hidden 4096, bf16) take 341 us
+// here and 376 on the K-sliced kernel.  Graphed norm + greedy pick with logits over a 248320 x 4096
+// vocabulary: 180 and 223 us at 64 rows, 273 and 742 at 256; eager calls add their host time (212 us at
+// 64 rows).
 //
 // Sums.  Weights of few rows are summed in 2 or 4 K slices, each with an accumulator of its own,
 // added in order at the end: the order of summation is a function of the weight's shape alone and

@@ -129,10 +129,13 @@ __global__ void __launch_bounds__(kNormThreads + 32) rmsnorm_quant_kernel(const 
   // the others wait for the previous kernel, and they find the code in the cache.  A warp of its own,
   // because there may be nothing to wait for (behind a kernel that was not launched with early
   // starts): a second pass of all warps gave more in
-  // an unbroken chain (hidden 4096, four graphed layers, 1 row: 262 -> 244 us, here 256) but cost 3 us
+  // an unbroken chain (hidden 4096, four graphed layers, 1 row: 262 -> 244 us, here 255) but cost 3 us
   // per launch in a broken one (hidden 2560: 194 -> 203 us, here 193).
   // Only up to kRehearseRows rows: beyond, the rehearsal competes with the GEMM that is waited for
   // (344 -> 350 us at 128 rows).
+  // The two-pass build was also 4 % faster at 128 rows (334 us, here 348), where neither form rehearses:
+  // its compiled kernels differ (118 and 80 registers for the two norms; 72 and 56 here).  What in
+  // them makes the difference has not been shown.
   Vec4<T> x[VPT];
   if (live) {
     bq::pdl_wait_prior_grids();

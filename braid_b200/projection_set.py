@@ -117,13 +117,15 @@ class ProjectionSet:
                 total += M * k + sum(ws[n].shape[0] * k + 2 * M * ws[n].shape[0] for n in grp)
         return total
 
-    # dram__bytes_read.sum + dram__bytes_write.sum of one gemm_stream_kernel launch at 128 rows,
+    # dram__bytes_read.sum + dram__bytes_write.sum of one gemm_wide_kernel launch at 128 rows,
     # measured with ncu on a 4-layer stack (weights larger than L2), per launch shape: every
     # weight byte and the activation codes cross HBM once; the outputs are still in L2 when the
-    # kernel ends, so they do not show.  Other row counts use the mean measured/algorithmic ratio.
+    # kernel ends, so they do not show.  (qkv|z: less the 1.57 MB of the two 16-bit gate weights and the
+    # dense activation that the measured launch also reads; gate|up: the form with SiLU and codes in
+    # the epilogue.)  Other row counts use the mean measured/algorithmic ratio.
     MEASURED_TRAFFIC_M128 = {
-        ("qkv", "z"): 50.98e6, ("out",): 17.39e6, ("gate", "up"): 101.45e6, ("down",): 51.99e6,
-        ("q", "k", "v"): 42.57e6,
+        ("qkv", "z"): 50.94e6, ("out",): 17.38e6, ("gate", "up"): 101.33e6, ("down",): 51.99e6,
+        ("q", "k", "v"): 42.55e6,
     }
 
     def gemm_measured_traffic_bytes(self) -> dict:

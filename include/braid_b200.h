@@ -290,10 +290,11 @@ size_t bq_gemm_workspace_bytes(int64_t M, int64_t N_total, int64_t K);
  * Per-tensor W8A8 GEMM:  Y[M,N] = (Xq[M,K] . Wq[N,K]^T) * sx * sw, fp32
  * accumulation in tensor memory, scales applied in the epilogue, output cast
  * to `out_dtype`.  Both operands are K-major, exactly the layout the reference
- * keeps (`FP8Weight.data` is [N,K] row-major).  M <= 256 takes the
- * weight-streaming kernel (weight rows on the MMA M side, batch on the N side,
- * deterministic split-K over a thread-block cluster); larger M takes the
- * persistent compute-bound kernel.
+ * keeps (`FP8Weight.data` is [N,K] row-major).  M <= 256 takes one of two
+ * weight-streaming kernels: small batches the K-sliced one (weight rows on the
+ * MMA M side, batch on the N side, deterministic split-K over a thread-block
+ * cluster), wide ones the CTA-pair one (batch on the M side, K in one CTA
+ * pair); larger M takes the persistent compute-bound kernel.
  *
  * Replaces: braid/model/quant.py:232-241 (`fp8_matmul`), i.e. the call
  * `torch._scaled_mm(xq, w.data.t(), scale_a=sx, scale_b=w.scale, out_dtype=...)`.
