@@ -1876,17 +1876,18 @@ struct DenseArgs {
 // All figures are the K-sliced kernel's time over this one's, graphed, weights from HBM (banks larger
 // than L2); where a line says nothing, it lies between 1.0 and 1.4, beyond 208 rows up to 2.5.
 //
-// One round.  One decoder layer of hidden 1024 / 2048 / 2560 / 4096 / 5120: 33 to 48 rows 1.03 / 1.00 / 0.99 /
+// One round.  Four decoder layers of hidden 1024 / 2048 / 2560 / 4096 / 5120: 33 to 48 rows 1.03 / 1.00 / 0.99 /
 // 1.00 / 1.04, 49 rows 1.09 / 1.03 / 1.01 / 1.06 / 1.07, 128 rows 1.21 / 1.13 / 1.09 / 1.10 / 1.09, 129 rows
 // 1.15 / 1.04 / 1.00 / 0.98 / 0.99, 161 rows 1.20 / 1.11 / 1.07 / 1.09 / 1.14: 49 rows on, without 129 to 160.
+// (Gate/up of 16384 columns alone measures 0.96 at 49 rows, but in the chain of a layer it is the
+// faster one: hidden 4096, 312 us here, 324 with that launch on the K-sliced kernel.)
 // Within that, what the K-sliced kernel does better:
-//  * gate/up in units of more than 128 columns up to 80 rows, where SiLU is the longer part
-//    (K = 4096, 16384 columns: 49 rows 0.96, 65 rows 0.98; 128-column units 1.02);
-//  * weights of many rows and short K up to 80 rows (9472 x 1024: 49 rows 0.87);
-//  * units of 256 weight rows beyond 160 rows, whose epilogue nothing hides unless K is long
-//    (18944 x 2048: 0.94 to 0.97; x 4096: 0.96 to 0.98, 256 rows 1.05; x 12288: 1.06);
+//  * short K in units that leave no pair of SMs free: up to 64 rows (9472 x 1024 behind a norm: 49 rows
+//    0.83, 80 rows 1.05), and in the longest units from 177 rows on (18944 x 1024: 176 rows 1.00,
+//    192 rows 0.97, 256 rows 0.96);
 //  * few rows and long K beyond 160 rows: one thread's chain of MMAs against a quarter of it
-//    (1024 x 7680: 161 rows 0.96, 208 rows 1.04; 4096 x 12288: 0.93, 224 rows 0.99, 240 rows 1.03).
+//    (4096 x 12288: 161 rows 0.93, 224 rows 0.99, 240 rows 1.03, and four layers of hidden 4096 393 -> 390 us
+//    at 161 rows; 2560 x 7680: 0.96 alone, but the layers 324 -> 328 us: the line lies between).
 //
 // Several rounds (a vocabulary) pay an epilogue per round.  Where K is long it is hidden (60016 x 4096:
 // 33 rows 1.05, 129 rows 1.09), where K is short the batch has to be larger (60016 x 1024: 65 rows 1.14,
@@ -1909,12 +1910,9 @@ bool wide_applies(const GemmParams& p, const WideShape& sh) {
     return p.k_blocks >= 16 ? p.M > 32 : p.M > 64 && !between;
   }
   if (p.M <= 48 || between) return false;
-  const int un = p.seg[0].un;
-  if (p.pair.on) return un <= 128 || p.M > 80;
-  if (short_k && un >= 128 && p.M <= 80) return false;
-  if (un > 224 && p.M > 160) return p.k_blocks >= 64 || (p.k_blocks >= 32 && p.M > 192);
-  if (p.seg[0].split == 4 && ctas <= sms && p.k_blocks > 48 && p.M > 160)
-    return p.M > (p.k_blocks > 64 ? 224 : 192);
+  if (p.pair.on) return true;
+  if (short_k && sh.units >= max_pairs() && (p.seg[0].un > 224 ? p.M > 176 : p.M <= 64)) return false;
+  if (p.seg[0].split == 4 && ctas <= sms && p.k_blocks > 64 && p.M > 160) return p.M > 224;
   return true;
 }
 

@@ -726,9 +726,8 @@ def test_wide_greedy_pick_over_several_rounds(Q, wide, M):
 
 @pytest.mark.parametrize("n,k,on,off", [
     (4096, 4096, (49, 128, 161, 256), (48, 129, 160)),        # one round
-    (9472, 1024, (81,), (64, 80)),                            # many rows, short K
-    (18944, 1024, (), (161, 256)), (18944, 4096, (160 + 33,), (192,)), (18944, 8192, (161,), ()),   # 256-row units
-    (1024, 6144, (161,), ()), (1024, 7680, (193,), (161, 192)), (1024, 12288, (225,), (224,)),    # long K, few rows
+    (9472, 1024, (65,), (49, 64)), (9472, 2048, (49,), ()), (18944, 1024, (49, 176), (177, 256)),  # all pairs, short K
+    (1024, 8192, (161,), ()), (1024, 12288, (225,), (161, 224)),                                  # long K, few rows
     (20480, 1024, (209,), (65, 208)), (32000, 1536, (65, 161), (64, 129)),                        # two rounds
     (32000, 2048, (97, 161), (96, 129)), (24576, 2048, (33, 129), (32,)), (49152, 2048, (33, 129), (32,))])
 def test_which_decode_batches_run_on_cta_pairs(Q, n, k, on, off):
@@ -749,7 +748,7 @@ def test_which_decode_batches_run_on_cta_pairs(Q, n, k, on, off):
     assert Q.device_status() == 0
 
 
-@pytest.mark.parametrize("M,I,wide", [(64, 16384, False), (80, 16384, False), (81, 16384, True), (49, 9472, True)])
+@pytest.mark.parametrize("M,I,wide", [(48, 16384, False), (49, 16384, True), (160, 9472, False), (161, 9472, True)])
 def test_which_gate_up_batches_run_on_cta_pairs(Q, M, I, wide):
     xq, sx = Q.quantize_act(randn_cpu((M, 256), seed=M).cuda())
     g, u = (Q.quantize_weight((randn_cpu((I, 256), seed=s) * 0.05).cuda()) for s in (1, 2))
