@@ -659,6 +659,7 @@ def test_wide_batches_on_cta_pairs_agree_with_the_k_sliced_kernel(Q, M, ns, K):
 
     got, want = both(lambda: Q.fp8_matmul_grouped(xq, sx, ws, out_dtype=torch.float32))
     for y, z, w in zip(got, want, ws):
+        assert torch.equal(y, z)      # the same sums in the same order: the choice of a kernel shows in no result
         b = w.data.float().double() * w.scale.double()
         # an fp32 sum of K products, 32 of them per step of the accumulator, each step off by at most
         # two units of the last place of the sum of magnitudes; the scaling adds two more
@@ -731,18 +732,19 @@ def test_wide_greedy_pick_over_several_rounds(Q, wide, M):
     (20480, 1024, (209,), (65, 208)), (32000, 1536, (65, 161), (64, 129)),                        # two rounds
     (32000, 2048, (97, 161), (96, 129)), (24576, 2048, (33, 129), (32,)), (49152, 2048, (33, 129), (32,))])
 def test_which_decode_batches_run_on_cta_pairs(Q, n, k, on, off):
-    """Both sides of every line of the dispatch; whichever kernel is taken gives its own bits."""
+    """Both sides of every line of the dispatch.  Both kernels give the same bits, so that a grouped launch
+    and per-weight calls agree although the lines may part them."""
     g = torch.Generator(device="cuda").manual_seed(n + k)
     data = torch.randint(0, 120, (n, k), generator=g, device="cuda", dtype=torch.uint8)
     w = Q.FP8Weight(data=data.view(Q.FP8), scale=torch.full((1, 1), 1e-3, device="cuda"), shape=(n, k))
     torch.cuda.synchronize()
     for M, wide in [(m, True) for m in on] + [(m, False) for m in off]:
         xq, sx = Q.quantize_act(randn_cpu((M, k), seed=M).cuda())
-        y = Q.fp8_matmul(xq, sx, w)
+        y = Q.fp8_matmul(xq, sx, w, out_dtype=torch.float32)
         assert Q.last_gemm_launch()["wide"] == wide, f"{M} x {n} x {k}"
         try:
-            Q.set_option("decode_wide", int(wide))
-            assert torch.equal(y, Q.fp8_matmul(xq, sx, w))
+            Q.set_option("decode_wide", int(not wide))
+            assert torch.equal(y, Q.fp8_matmul(xq, sx, w, out_dtype=torch.float32))
         finally:
             Q.set_option("decode_wide", -1)
     assert Q.device_status() == 0
