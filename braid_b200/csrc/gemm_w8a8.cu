@@ -445,7 +445,7 @@ __device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const floa
   for (int m = e.m_begin + e.warp; m < e.m_end; m += kStreamWarps) {
     const T* hrow = reinterpret_cast<const T*>(part + m * kRowTile);
     float f[2] = {widen(hrow[hcol]), widen(hrow[hcol + 1])};
-    divide_group<2, true>(sc, f);   // the scale is that of these very values
+    divide_group<T, 2, true>(sc, f);   // the scale is that of these very values
     const uint32_t pair = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
     *reinterpret_cast<uint16_t*>(hq + static_cast<long long>(m) * ld_hq + col0 + hcol) =
         static_cast<uint16_t>(pair & 0xFFFFu);

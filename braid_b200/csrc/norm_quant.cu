@@ -83,7 +83,7 @@ __device__ __forceinline__ void store4(T* p, const Vec4<T>& v) {
 template <typename T>
 __device__ __forceinline__ void emit4(const Vec4<T>& v, const ScaleDiv& sc, uint8_t* dst, bool live) {
   float f[4] = {widen(v.v[0]), widen(v.v[1]), widen(v.v[2]), widen(v.v[3])};
-  divide_group<4, true>(sc, f);   // the scale is that of these very values
+  divide_group<T, 4, true>(sc, f);   // the scale is that of these very values
   const uint32_t a = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
   const uint32_t b = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
   const uint32_t w = (a & 0xFFFFu) | ((b & 0xFFFFu) << 16);

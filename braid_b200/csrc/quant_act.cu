@@ -230,7 +230,7 @@ __device__ __forceinline__ void unit_emit(const uint4& raw, const ScaleDiv& dv, 
   } else {
     float f[4] = {__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z),
                   __uint_as_float(raw.w)};
-    divide_group<4, OWN_SCALE>(dv, f);
+    divide_group<T, 4, OWN_SCALE>(dv, f);
     const uint32_t a = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
     const uint32_t b = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
     *reinterpret_cast<uint32_t*>(dst) = (a & 0xFFFFu) | ((b & 0xFFFFu) << 16);

@@ -114,6 +114,11 @@ __device__ __forceinline__ float absmax8(const Pack8<T>& v, float m) {
 // takes the division instruction instead, and quotients too small for the corrections to be
 // exact are far below half of the smallest e4m3 step, where only the sign reaches the code
 // (hence the copysign, which also keeps -0).
+// Values of a 16-bit type take one correction: over all 2^23 divisor mantissas and all dividend
+// mantissas of 8 (bf16) and of 11 bits (fp16), checked one by one, the quotient after the first
+// correction is the IEEE one.  Two instructions of about ten per element: the weight loader's cast, a
+// 12288 x 4096 weight in all, 48.6 -> 44.5 us; a prompt layer of 9658 rows 2,260 -> 2,235 us, four graphed
+// decoder layers of 128 rows 344.9 -> 341.9 us.
 struct ScaleDiv {
   float sc, inv;
   bool fast;
@@ -123,12 +128,12 @@ struct ScaleDiv {
     fast = s >= 0x1p-60f && s <= 0x1p60f;
   }
   // The quotient by the corrections alone; NaN where the division instruction has to decide.
+  template <int CORRECTIONS>
   __device__ __forceinline__ float corrected(float x) const {
     float q = __fmul_rn(x, inv);
-    float r = __fmaf_rn(-q, sc, x);
-    q = __fmaf_rn(r, inv, q);
-    r = __fmaf_rn(-q, sc, x);
-    return copysignf(__fmaf_rn(r, inv, q), x);
+#pragma unroll
+    for (int i = 0; i < CORRECTIONS; ++i) q = __fmaf_rn(__fmaf_rn(-q, sc, x), inv, q);
+    return copysignf(q, x);
   }
 };
 
@@ -140,13 +145,14 @@ struct ScaleDiv {
 // the bare quotient: the reference clamps to +-448 before its (non-saturating) cast,
 // `cvt.rn.satfinite` does the same clamp itself (finite values and infinities beyond the
 // range become +-448, NaN stays NaN).
-template <int N, bool OWN_SCALE = false>
+// T is the type the x are values of.
+template <typename T, int N, bool OWN_SCALE = false>
 __device__ __forceinline__ void divide_group(const ScaleDiv& d, float (&x)[N]) {
   float q[N];
   bool ok = d.fast;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    q[i] = d.corrected(x[i]);
+    q[i] = d.corrected<sizeof(T) == 2 ? 1 : 2>(x[i]);
     if constexpr (!OWN_SCALE) ok = ok && (q[i] == q[i]);
   }
   if (ok) {
@@ -160,7 +166,7 @@ __device__ __forceinline__ void divide_group(const ScaleDiv& d, float (&x)[N]) {
 
 __device__ __forceinline__ float quant_one(float x, const ScaleDiv& d) {
   float v[1] = {x};
-  divide_group<1>(d, v);
+  divide_group<float, 1>(d, v);
   return v[0];
 }
 
@@ -170,7 +176,7 @@ __device__ __forceinline__ uint2 codes8(const Pack8<T>& v, const ScaleDiv& sc) {
   float f[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) f[i] = widen(v.v[i]);
-  divide_group<8, OWN_SCALE>(sc, f);
+  divide_group<T, 8, OWN_SCALE>(sc, f);
   uint32_t w[2];
 #pragma unroll
   for (int half = 0; half < 2; ++half) {

@@ -422,6 +422,21 @@ def test_quantize_weight_gives_the_bits_of_the_torch_spelling(Q, dt, shape):
         assert torch.equal(u8(got.data), u8(want.data)), f"{dt} {shape} case {i}"
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+def test_cast_of_every_16_bit_value_under_many_scales(Q, dt):
+    """The cast divides with one residual correction for 16-bit types: all 65,536 values (NaN, infinities
+    and subnormals too) under scales of every kind give the codes of the IEEE division."""
+    x = torch.arange(65536, dtype=torch.int32, device="cuda").to(torch.int16).view(dt)
+    g = torch.Generator().manual_seed(3)
+    scales = (torch.rand(400, generator=g) + 1.0) * 2.0 ** torch.randint(-40, 20, (400,), generator=g).float()
+    special = torch.tensor([1.0, 3.0, 448.0, 1.0 / 448.0, 1e-12, 2.0 ** -61, 2.0 ** 61, 1.9999999, 1.0000001])
+    for s in torch.cat([scales, special]).cuda():
+        s = s.reshape(1, 1)
+        want = (x.float() / s[0]).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
+        got = Q.cast_act(x, s)
+        assert torch.equal(u8(got), u8(want)), f"scale {s.item():.9e}"
+
+
 def test_weights_load_on_a_side_stream_while_a_graph_replays(Q):
     """Loading shares no state with the forward path: it takes none of its scratch slots, and 300
     weights (more than there are slots) quantized beside a replaying graph leave both sides' bits as
