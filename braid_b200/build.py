@@ -3,7 +3,8 @@
 The reference engine JIT-builds its extension on first use
 (braid/kernels/loader.py:10-44: `torch.utils.cpp_extension.load`, `-O3 -lineinfo`,
 no fast-math).  Here the library is built once, in-tree, for sm_100a only, and
-loaded with ctypes — it has no torch or Python dependency at all.  Flags keep
+loaded with ctypes — it has no torch or Python dependency at all.  A second, small
+one (`_host.so`, g++) holds the native calls of `quant.py` and does link torch.  Flags keep
 the reference's numerics contract: no `--use_fast_math`, IEEE division and
 square root, no flush-to-zero.
 
@@ -38,6 +39,33 @@ def nvcc_path() -> str:
     return cand
 
 
+HOST_SRC = CSRC / "host_calls.cpp"
+HOST = PKG / "_host.so"
+
+
+def build_host(force: bool = False) -> Path:
+    """Compile the native calls of quant.py against the torch that is installed."""
+    deps = (HOST_SRC, PKG.parent / "include" / "braid_b200.h")
+    if not force and HOST.exists() and all(d.stat().st_mtime <= HOST.stat().st_mtime for d in deps):
+        return HOST
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    torch_lib = Path(torch.__file__).resolve().parent / "lib"
+    cuda = Path(nvcc_path()).resolve().parent.parent
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
+    cmd = ["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(arg for path in includes for arg in ("-isystem", path)),
+           str(HOST_SRC), "-o", str(HOST), f"-L{torch_lib}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + proc.stdout + proc.stderr)
+    return HOST
+
+
 def is_stale() -> bool:
     if not LIB.exists():
         return True
@@ -52,6 +80,8 @@ PHASES_LIB = PKG / "libbraid_b200_phases.so"
 def build(force: bool = False, verbose: bool = False, defines: tuple[str, ...] = (),
           out: Path | None = None) -> Path:
     """Compile the CUDA sources for sm_100a into one shared library."""
+    if out is None and not defines:
+        build_host(force)
     if out is None and not defines and not force and not is_stale():
         return LIB
     LIB = out if out is not None else globals()["LIB"]

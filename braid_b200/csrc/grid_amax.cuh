@@ -149,18 +149,36 @@ __device__ __forceinline__ void grid_depart(QuantWs* ws, unsigned int* wait_seen
   }
 }
 
+// Host side: CTAs of a kernel that an SM of the current device holds at once, 0 where CUDA cannot say.  The
+// answer is a property of the compiled kernel; asking costs a launch's host time a third over, so
+// each thread keeps the last few.
+template <typename Kernel>
+inline int resident_per_sm(Kernel kernel, int threads, size_t dynamic_smem) {
+  struct Known { const void* kernel; int dev, threads; size_t smem; int per_sm; };
+  static thread_local Known known[32];
+  static thread_local unsigned int next = 0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  const void* const key = reinterpret_cast<const void*>(kernel);
+  for (const Known& k : known)
+    if (k.kernel == key && k.dev == dev && k.threads == threads && k.smem == dynamic_smem) return k.per_sm;
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dynamic_smem) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  known[next++ % 32] = Known{key, dev, threads, dynamic_smem, per_sm};
+  return per_sm;
+}
+
 // Host side: launches a grid-stride kernel with at most as many CTAs as the device holds at
 // once (`want` CTAs if that is fewer), so that no partial second wave trails the first -- a grid
 // of 8 CTAs per SM where five fit ran 1.6 waves.  Programmatic dependent launch on request.
 template <typename Kernel, typename... Args>
 inline cudaError_t launch_resident_smem(Kernel kernel, long long want, int threads, int sms, bool pdl,
                                         size_t dynamic_smem, cudaStream_t stream, Args... args) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dynamic_smem) != cudaSuccess ||
-      per_sm < 1) {
-    (void)cudaGetLastError();
-    per_sm = 4;
-  }
+  int per_sm = resident_per_sm(kernel, threads, dynamic_smem);
+  if (per_sm < 1) per_sm = 4;
   const long long cap = static_cast<long long>(per_sm) * sms;
   long long grid = want < cap ? want : cap;
   if (grid < 1) grid = 1;

@@ -407,10 +407,10 @@ int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t str
 #endif
   if (rows <= kRehearseRows) threads += 32;   // the rehearsing warp
   // every CTA waits for every other: the whole grid must fit on the device at once
-  int dev = 0, sms = 0, per_sm = 0;
+  int dev = 0, sms = 0;
+  const int per_sm = resident_per_sm(kernel, threads, 0);
   if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess) {
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1) {
     (void)cudaGetLastError();
     return bq::kErrLaunch;
   }

@@ -31,7 +31,7 @@ from __future__ import annotations
 
 import ctypes
 import threading
-from collections.abc import Iterable, Sequence
+from collections.abc import Iterable, Mapping, Sequence
 from dataclasses import dataclass
 
 import torch
@@ -176,13 +176,56 @@ _SLOTS = 256
 _TWO_LAUNCH_FROM = 1 << 22
 _SLOT_BYTES = 64
 _scratch: dict[int, torch.Tensor] = {}
-_next_slot: dict[int, int] = {}
+_taken: dict[int, int] = {}      # slots taken per device, where the native calls do not count them
 _launches = 0      # kernels of this library launched (or captured) so far
+
+# `csrc/host_calls.cpp`: the plain case of the calls below, checks, allocations and launch in one native
+# call (a launch from here costs about 18 us of host time, from there about 5; figures there).  Each returns None for
+# whatever is not plain, and the code below decides.  `_HOST` is the module, None where it cannot be
+# loaded (another torch build): everything then runs through the code below.  `_NATIVE` is the
+# same module while the kernels are active.
+_HOST = None
+_NATIVE = None
+
+
+class _NextSlots(Mapping):
+    """Device index -> index of the scratch slot its next launch takes."""
+
+    def __getitem__(self, device):
+        if device not in _scratch:
+            raise KeyError(device)
+        return _HOST.next_slot(device) if _HOST is not None else _taken.get(device, 0) % _SLOTS
+
+    def __iter__(self):
+        return iter(_scratch)
+
+    def __len__(self):
+        return len(_scratch)
+
+
+_next_slot = _NextSlots()
 
 
 def launch_count() -> int:
     """How many kernels of this library have been launched or captured by this process."""
-    return _launches
+    return _launches + (_HOST.launch_count() if _HOST is not None else 0)
+
+
+def _load_host(lib) -> None:
+    """Load the native calls once and give them the library's functions and the slots made so far."""
+    global _HOST
+    if _HOST is not None:
+        return
+    try:
+        from . import _host
+    except ImportError:
+        return
+    _host.init({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _lib.SIGNATURES},
+               _SLOTS, _SLOT_BYTES, _TWO_LAUNCH_FROM)
+    with _LOCK:
+        for index, buf in _scratch.items():
+            _host.set_scratch(index, buf.data_ptr())
+        _HOST = _host
 
 
 def warm_fused(enable: bool = True) -> bool:
@@ -195,9 +238,9 @@ def warm_fused(enable: bool = True) -> bool:
     loaded RAISES: there is no slower arm that would make a benchmark look
     plausible without the kernels.
     """
-    global _FUSED, _FUSED_STATE
+    global _FUSED, _FUSED_STATE, _NATIVE
     if not enable:
-        _FUSED, _FUSED_STATE = None, "disabled by caller"
+        _FUSED, _FUSED_STATE, _NATIVE = None, "disabled by caller", None
         return False
     if _FUSED is not None:
         return True
@@ -207,7 +250,8 @@ def warm_fused(enable: bool = True) -> bool:
         _FUSED = None
         _FUSED_STATE = f"unavailable: {type(e).__name__}: {str(e).split(chr(10), 1)[0][:120]}"
         raise
-    _FUSED, _FUSED_STATE = lib, "active"
+    _load_host(lib)
+    _FUSED, _FUSED_STATE, _NATIVE = lib, "active", _HOST
     if torch.cuda.is_available():
         _scratch_for(torch.cuda.current_device())
     return True
@@ -252,7 +296,8 @@ def _scratch_for(device_index: int) -> torch.Tensor:
                                   device=torch.device("cuda", device_index))
                 torch.cuda.synchronize(device_index)
                 _scratch[device_index] = buf
-                _next_slot[device_index] = 0
+                if _HOST is not None:
+                    _HOST.set_scratch(device_index, buf.data_ptr())
     return buf
 
 
@@ -261,10 +306,12 @@ def _take_slot(device: torch.device) -> int:
     global _launches
     idx = device.index if device.index is not None else torch.cuda.current_device()
     buf = _scratch_for(idx)
+    if _HOST is not None:
+        return _HOST.take_slot(idx)
     with _LOCK:
         _launches += 1
-        slot = _next_slot[idx]
-        _next_slot[idx] = (slot + 1) % _SLOTS
+        slot = _taken.get(idx, 0) % _SLOTS
+        _taken[idx] = slot + 1
     return buf.data_ptr() + slot * _SLOT_BYTES
 
 
@@ -337,6 +384,10 @@ def quantize_act(x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     fp16 take the one-launch kernel; a non-contiguous or 16-byte-misaligned view
     takes the torch spelling, as the reference does (`tests/test_quant.py:424-449`).
     """
+    if _NATIVE is not None:
+        got = _NATIVE.quantize_act(x)
+        if got is not None:
+            return got
     _check_cuda(x, "quantize_act")
     if _quantizers_off():
         return _torch_quantize(x)
@@ -470,6 +521,10 @@ def sigmoid_gate_quant(o: torch.Tensor, gate: torch.Tensor,
     `qg.view(B, T, H, 2*D).chunk(2, dim=-1)` (braid/model/attention.py:177), which
     is read in place — no `reshape` copy.
     """
+    if _NATIVE is not None:
+        got = _NATIVE.sigmoid_gate_quant(o, gate)
+        if got is not None:
+            return got
     _check_cuda(o, "sigmoid_gate_quant")
     if _quantizers_off():
         return _torch_quantize(o * torch.sigmoid(gate.reshape(o.shape)))
@@ -610,7 +665,11 @@ def rms_norm_quant(x: torch.Tensor, gamma: torch.Tensor, eps: float,
     """`quantize_act(rms_norm(x, gamma, eps))` in one launch (braid/model/layer.py:49,59 feeding
     `project` / the MLP).  Bit-identical to the two steps.  More rows than fit on the device at
     once (prefill) take two launches: the norm with rows looped per CTA, which also leaves the
-    scale, and the cast pass; inputs with odd strides run the two torch-spelled steps."""
+    scale, and the cast; inputs with odd strides run the two torch-spelled steps."""
+    if _NATIVE is not None:
+        got = _NATIVE.rms_norm_quant(x, gamma, eps, keep_dense)
+        if got is not None:
+            return QuantizedActivation(got[0], got[1], x.shape, x.dtype, got[2])
     _check_cuda(x, "rms_norm_quant")
     K = x.shape[-1]
     code = _DTYPE_CODE.get(x.dtype)
@@ -657,6 +716,10 @@ def gated_rms_norm_quant(y: torch.Tensor, z: torch.Tensor, gamma: torch.Tensor, 
     """`quantize_act(rms_norm_gated(y.to(z.dtype), z, gamma, eps))` in one launch: the GDN readout
     feeding out_proj (braid/model/gdn.py:373-387).  `y` is `[..., H, D]` or `[..., H*D]`, the fp32
     scan output or already of `z`'s type; `z` is `[..., H*D]`.  Returns the `[..., H*D]` activation."""
+    if _NATIVE is not None:
+        got = _NATIVE.gated_rms_norm_quant(y, z, gamma, eps, head_dim)
+        if got is not None:
+            return QuantizedActivation(got[0], got[1], z.shape, z.dtype)
     _check_cuda(z, "gated_rms_norm_quant")
     width = z.shape[-1]
     heads = width // head_dim
@@ -743,6 +806,10 @@ def fp8_matmul(xq: torch.Tensor, sx: torch.Tensor, w: FP8Weight,
     (`[M, N]`, `out_dtype`) the result is `residual + that`, the add running in the GEMM's
     epilogue with the two roundings of the separate kernels (decode sizes; larger M adds after).
     """
+    if _NATIVE is not None and isinstance(w, FP8Weight):
+        y = _NATIVE.matmul(xq, sx, w.data, w.scale, out_dtype, residual)
+        if y is not None:
+            return y
     if residual is None:
         return fp8_matmul_grouped(xq, sx, (w,), out_dtype=out_dtype)[0]
     _check_gemm_inputs(xq, sx)
@@ -839,6 +906,11 @@ def lm_head_argmax(x, w: FP8Weight, return_logits: bool = False):
         logits = fp8_matmul(xq, sx, w, out_dtype=dt)
         idx = logits.argmax(-1).reshape(lead)
         return (idx, logits.reshape(*lead, N)) if return_logits else idx
+    if _NATIVE is not None:
+        got = _NATIVE.lm_head_argmax(xq, sx, w.data, w.scale, dt, return_logits)
+        if got is not None:
+            idx = got[0].reshape(lead)
+            return (idx, got[1].reshape(*lead, N)) if return_logits else idx
     lib = _require_lib()
     if not xq.is_contiguous():
         xq = xq.contiguous()
@@ -901,6 +973,10 @@ def fp8_linear(x: torch.Tensor, w: FP8Weight, residual: torch.Tensor | None = No
     if isinstance(x, QuantizedActivation):
         return fp8_matmul(x.q, x.scale, w, out_dtype=x.dtype, residual=res2).reshape(*lead, N)
     pre = _attached(x)
+    if pre is None and _NATIVE is not None:
+        y = _NATIVE.linear(x, w.data, w.scale, res2)
+        if y is not None:
+            return y
     xq, sx = (pre[0].reshape(-1, K), pre[1]) if pre is not None else quantize_act(x.reshape(-1, K))
     return fp8_matmul(xq, sx, w, out_dtype=x.dtype, residual=res2).reshape(*lead, N)
 
@@ -965,6 +1041,17 @@ def _project_mixed(xq, sx, dense: torch.Tensor, weights, lead, K):
     return [y.reshape(*lead, y.shape[1]) for y in outs]
 
 
+def _project_native(xq, sx, dense, dtype, weights, lead):
+    """All members in one launch, or None where that is for `project` to decide."""
+    if _NATIVE is None or (dense is not None and not _DENSE_SEGMENTS):
+        return None
+    ys = _NATIVE.project(xq, sx, dense, dtype, tuple([w.data if isinstance(w, FP8Weight) else w for w in weights]),
+                         tuple([w.scale if isinstance(w, FP8Weight) else None for w in weights]))
+    if ys is None or len(lead) == 1:
+        return ys
+    return [y.reshape(*lead, y.shape[1]) for y in ys]
+
+
 def project(x: torch.Tensor, *weights: torch.Tensor | FP8Weight) -> list[torch.Tensor]:
     """`F.linear(x, w)` for several projections that share one activation.
 
@@ -986,15 +1073,18 @@ def project(x: torch.Tensor, *weights: torch.Tensor | FP8Weight) -> list[torch.T
         else:
             dense = x
             xq, sx = quantize_act(x.reshape(-1, K))
-        mixed = _project_mixed(xq, sx, dense, weights, lead, K)
+        mixed = _project_native(xq, sx, dense, dense.dtype, weights, lead)
+        if mixed is None:
+            mixed = _project_mixed(xq, sx, dense, weights, lead, K)
         if mixed is not None:
             return mixed
         pre = QuantizedActivation(xq, sx, x.shape, x.dtype, dense)     # do not quantize twice
-    if pre is not None:
-        ys = iter(fp8_matmul_grouped(pre.q, pre.scale, fp8, out_dtype=pre.dtype))
-    else:
-        xq, sx = quantize_act(x.reshape(-1, K))
-        ys = iter(fp8_matmul_grouped(xq, sx, fp8, out_dtype=x.dtype))
+    xq, sx = (pre.q, pre.scale) if pre is not None else quantize_act(x.reshape(-1, K))
+    if len(fp8) == len(weights):
+        ys = _project_native(xq, sx, None, x.dtype, weights, lead)
+        if ys is not None:
+            return ys
+    ys = iter(fp8_matmul_grouped(xq, sx, fp8, out_dtype=x.dtype))
     out = []
     for w in weights:
         if isinstance(w, FP8Weight):
@@ -1241,6 +1331,14 @@ def mlp_forward(x: torch.Tensor, gate_proj: FP8Weight, up_proj: FP8Weight,
     M = pre.q.shape[0] if pre is not None else x2.shape[0]
     I = gate_proj.shape[0]
     res2 = residual.reshape(-1, down_proj.shape[0]) if residual is not None else None
+    if (_PAIR_MLP and _NATIVE is not None and isinstance(gate_proj, FP8Weight) and isinstance(up_proj, FP8Weight)
+            and isinstance(down_proj, FP8Weight)):
+        xq, sx = (pre.q, pre.scale) if pre is not None else quantize_act(x2)
+        y = _NATIVE.mlp(xq, sx, x.dtype, gate_proj.data, gate_proj.scale, up_proj.data, up_proj.scale,
+                        down_proj.data, down_proj.scale, res2)
+        if y is not None:
+            return y if len(lead) == 1 else y.reshape(*lead, down_proj.shape[0])
+        pre = QuantizedActivation(xq, sx, x.shape, x.dtype)     # do not quantize twice
     if _PAIR_MLP and M <= 256 and x.device.type == "cuda":
         xq, sx = (pre.q, pre.scale) if pre is not None else quantize_act(x2)
         paired = gate_up_silu_quant(xq, sx, gate_proj, up_proj, x.dtype)

@@ -1,0 +1,128 @@
+"""The native calls (`csrc/host_calls.cpp`) against the Python code they stand in for: same bits, same
+shapes, same launches, and whatever they do not take is decided by that code."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from _util import randn_cpu, u8
+
+pytestmark = pytest.mark.gpu
+
+
+def _flat(out):
+    if isinstance(out, torch.Tensor):
+        return [out]
+    if out is None:
+        return []
+    if isinstance(out, (list, tuple)):
+        return [t for o in out for t in _flat(o)]
+    return _flat([out.q, out.scale, out.dense])          # QuantizedActivation
+
+
+def _both(Q, monkeypatch, fn):
+    """`fn()` through the native calls and through the Python code alone, with the launches of each."""
+    assert Q._NATIVE is not None, "the native calls are not built for this torch"
+    n0 = Q.launch_count()
+    native = _flat(fn())
+    n1 = Q.launch_count()
+    with monkeypatch.context() as m:
+        m.setattr(Q, "_NATIVE", None)
+        python = _flat(fn())
+    assert n1 - n0 == Q.launch_count() - n1
+    assert len(native) == len(python)
+    for a, b in zip(native, python):
+        assert a.shape == b.shape and a.dtype is b.dtype and a.stride() == b.stride()
+        assert torch.equal(u8(a), u8(b))
+    return native
+
+
+@pytest.fixture(scope="module")
+def weights(request):
+    from braid_b200 import quant as Q
+    Q.warm_fused(True)
+    mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
+    H = 512
+    return {"a": mk(H, H, 1), "b": mk(1024, H, 2), "gate": mk(1536, H, 3), "up": mk(1536, H, 4), "down": mk(H, 1536, 5),
+            "odd_gate": mk(1040, H, 6), "odd_up": mk(1040, H, 7), "odd_down": mk(H, 1040, 8)}
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("M", [1, 17, 256, 257, 2500])
+def test_native_calls_give_the_bits_of_the_python_code(Q, monkeypatch, weights, dt, M):
+    H, w = 512, weights
+    x = randn_cpu((M, H), seed=M, dtype=dt).cuda()
+    x3 = x.view(M, 1, H)
+    res = randn_cpu((M, H), seed=1, dtype=dt).cuda()
+    strided = randn_cpu((M, 2 * H), seed=2, dtype=dt).cuda()[:, H:]
+    gates = [randn_cpu((16, H), seed=s, dtype=dt, scale=0.02).cuda() for s in (3, 4)]
+    gamma = 1 + 0.1 * randn_cpu((H,), seed=5, dtype=torch.float32).cuda()
+    gamma_h = 1 + 0.1 * randn_cpu((128,), seed=6, dtype=torch.float32).cuda()
+    scan = randn_cpu((M, H), seed=7, dtype=torch.float32).cuda()
+    both = lambda fn: _both(Q, monkeypatch, fn)  # noqa: E731
+    both(lambda: Q.quantize_act(x3))
+    both(lambda: Q.quantize_act(strided))                               # the torch spelling, either way
+    both(lambda: Q.linear(x, w["a"]))
+    both(lambda: Q.linear(x3, w["a"], residual=res.view(M, 1, H)))
+    both(lambda: Q.linear(x, w["a"], residual=strided))
+    both(lambda: Q.linear(strided, w["a"]))
+    both(lambda: Q.project(x, w["a"], w["b"]))
+    both(lambda: Q.project(x3, w["a"], *gates, w["b"]))
+    h = Q.rms_norm_quant(x, gamma, 1e-6, keep_dense=True)
+    both(lambda: Q.rms_norm_quant(x3, gamma, 1e-6, keep_dense=True))
+    both(lambda: Q.rms_norm_quant(strided, gamma, 1e-6))
+    both(lambda: Q.project(h, w["a"], *gates))
+    both(lambda: Q.gated_rms_norm_quant(scan.view(M, H // 128, 128), x, gamma_h, 1e-6, 128))
+    both(lambda: Q.gated_rms_norm_quant(x, strided, gamma_h, 1e-6, 128))
+    qg = randn_cpu((M, 2 * H), seed=8, dtype=dt).cuda().view(M, 2, H)
+    both(lambda: Q.sigmoid_gate_quant(x, qg[..., H // 2:]))
+    both(lambda: Q.sigmoid_gate_quant(x, res))
+    both(lambda: Q.gated_output_projection(x, qg[..., H // 2:], w["a"]))
+    both(lambda: Q.mlp_forward(x3, w["gate"], w["up"], w["down"], residual=res.view(M, 1, H)))
+    both(lambda: Q.mlp_forward(h, w["gate"], w["up"], w["down"], residual=strided))
+    both(lambda: Q.mlp_forward(x, w["odd_gate"], w["odd_up"], w["odd_down"]))
+    both(lambda: Q.lm_head_argmax(h, w["b"], return_logits=True))
+    both(lambda: [Q.lm_head_argmax(x3, w["b"])])
+    assert Q.device_status() == 0
+
+
+def test_what_the_python_code_refuses_stays_refused(Q, weights):
+    w = weights
+    x = randn_cpu((8, 512), seed=1).cuda()
+    for bad in (lambda: Q.linear(x.cpu(), w["a"]), lambda: Q.quantize_act(x.cpu())):
+        with pytest.raises(RuntimeError):
+            bad()
+    for bad in (lambda: Q.linear(x.double(), w["a"]), lambda: Q.quantize_act(x[:0]),
+                lambda: Q.linear(x, w["a"], residual=x.float()), lambda: Q.linear(x, w["a"], residual=x[:4]),
+                lambda: Q.rms_norm_quant(x, torch.ones(4, device="cuda"), 1e-6),
+                lambda: Q.rms_norm_quant(x, torch.ones(512, device="cuda").half(), 1e-6),
+                lambda: Q.project(x[:, :256].contiguous(), w["a"], w["b"])):
+        with pytest.raises(ValueError):
+            bad()
+
+
+def test_native_calls_from_threads_and_streams(Q, weights):
+    """Slots are counted in one place whichever way a call takes; threads on their own streams get the
+    bits of a lone call."""
+    import threading
+    w, x = weights, randn_cpu((4, 512), seed=1).cuda()
+    want = Q.mlp_forward(x, w["gate"], w["up"], w["down"])
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(200):
+                got = Q.linear(x, w["a"])
+            out = [Q.fp8_matmul(*Q.quantize_act(x), w["a"]) for _ in range(20)]
+            torch.cuda.current_stream().synchronize()
+            wrong.extend(i for i, o in enumerate(out) if not torch.equal(o, got))
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    assert torch.equal(want, Q.mlp_forward(x, w["gate"], w["up"], w["down"]))
+    assert Q.device_status() == 0
