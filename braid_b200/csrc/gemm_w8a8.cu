@@ -158,6 +158,18 @@ struct GemmParams {
   PushParams push;
 };
 
+// What a launch's epilogue does and the type it writes, as template parameters of the kernels.  A decode
+// launch runs its epilogue once per CTA, on the critical path and through an instruction cache that
+// other kernels have used since, and a prefill launch's MMA and epilogue loops should carry no branch that
+// the launch cannot take: one kernel with every form in it was 285 KB of code (the K-sliced one), of
+// which a launch runs a tenth (35 to 52 KB now).  Four graphed decoder layers, one kernel -> these: hidden
+// 4096, 1 row 252 -> 246 us, 128 rows 339 -> 334; hidden 2560, 16 rows 231 -> 224; hidden 5120, 64 rows
+// 449 -> 435; hidden 1024, 8 rows 157 -> 149.  At prefill sizes the residual and 16-bit forms in the one
+// kernel had cost every launch 8 %.  kAny, with the type taken at run time, is the column-parallel and greedy
+// forms, and launches whose segments differ in their form.
+enum Epi { kAny = -1, kPlain = 0, kResidual = 1, kGateUp = 2, kMixed = 3 };
+constexpr int kAnyType = -1;
+
 struct alignas(64) WeightMaps {
   CUtensorMap w[BQ_MAX_SEGMENTS];
 };
@@ -296,7 +308,7 @@ __device__ __forceinline__ void reduce_store(const EpilogueArgs& e) {
           if (e.col_ok) acc = add_res4(acc, rraw[i], e.out_dtype);
         }
         if (e.col_ok) {
-          if (e.push->n == 0) {
+          if (e.push == nullptr) {
             store_out4(e.y, (long long)m * e.ldy + e.row0 + n4, e.out_dtype, acc);
           } else {
             for (int d = 0; d < e.push->n; ++d)
@@ -467,11 +479,16 @@ __device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const floa
 #ifndef BQ_STREAM_MIN_CTAS
 #define BQ_STREAM_MIN_CTAS 2
 #endif
+template <int EPI, int DT>
 __global__ void __launch_bounds__(kStreamThreads, BQ_STREAM_MIN_CTAS)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xd,
                    const __grid_constant__ WeightMaps tm_w, const __grid_constant__ GemmParams p,
                    const int smem_tile_bytes) {
   extern __shared__ uint8_t smem_dyn[];
+  const bool pair_on = EPI == kAny ? p.pair.on != 0 : EPI == kGateUp;
+  const bool argmax_on = EPI == kAny && p.argmax.on;
+  const PushParams* const push = EPI == kAny && p.push.n > 0 ? &p.push : nullptr;
+  const int out_dtype = DT == kAnyType ? p.out_dtype : DT;
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
   const int b_tile_bytes = p.mma_n * kBK;
@@ -528,7 +545,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   if (threadIdx.x == 0) {
     tma_prefetch_desc(x_map);
     tma_prefetch_desc(&tm_w.w[sg]);
-    if (p.pair.on) tma_prefetch_desc(&tm_w.w[1]);
+    if (pair_on) tma_prefetch_desc(&tm_w.w[1]);
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -561,7 +578,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       // weights are read once: evict first
       const uint64_t pol_w = policy_evict_first();
       // one 128-row box, or (paired gate/up) two 64-row boxes from the two weights
-      const bool paired = p.pair.on != 0;
+      const bool paired = pair_on;
       const int half_row0 = tile_in_seg * (kRowTile / 2);
       // slot and phase are carried along: an integer division by a run-time depth costs a
       // single issuing thread more than the loads it issues
@@ -686,8 +703,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     const uint32_t part_addr = smem_u32(part);
     const int peer0 = group * split;
     const EpilogueArgs ea{part, part_addr, peer0, m_begin, m_end, warp, lane, row0, scale, col_ok,
-                          seg.y, seg.ldy, p.out_dtype, seg.res, seg.ld_res, &p.push};
-    if (p.pair.on) {
+                          seg.y, seg.ldy, out_dtype, seg.res, seg.ld_res, push};
+    if (pair_on) {
       const float scale_up = sx_ready * __ldg(p.pair.sw_up);
       float mx;
 #define BQ_PAIR_ROWS(TT)                                                          \
@@ -697,18 +714,18 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         case 4: mx = silu_pair_rows<4, TT>(ea, scale_up, part); break;             \
         default: mx = silu_pair_rows<8, TT>(ea, scale_up, part); break;            \
       }
-      if (p.out_dtype == BQ_DTYPE_BF16) { BQ_PAIR_ROWS(__nv_bfloat16) }
-      else if (p.out_dtype == BQ_DTYPE_F16) { BQ_PAIR_ROWS(__half) }
+      if (out_dtype == BQ_DTYPE_BF16) { BQ_PAIR_ROWS(__nv_bfloat16) }
+      else if (out_dtype == BQ_DTYPE_F16) { BQ_PAIR_ROWS(__half) }
       else { BQ_PAIR_ROWS(float) }
 #undef BQ_PAIR_ROWS
       pair_max = mx;
-    } else if (p.argmax.on) {
+    } else if (argmax_on) {
       uint2* const mine = p.argmax.partial + static_cast<size_t>(tile_in_seg) * p.M;
-      if (p.out_dtype == BQ_DTYPE_BF16) argmax_rows<__nv_bfloat16>(ea, seg.n, mine);
-      else if (p.out_dtype == BQ_DTYPE_F16) argmax_rows<__half>(ea, seg.n, mine);
+      if (out_dtype == BQ_DTYPE_BF16) argmax_rows<__nv_bfloat16>(ea, seg.n, mine);
+      else if (out_dtype == BQ_DTYPE_F16) argmax_rows<__half>(ea, seg.n, mine);
       else argmax_rows<float>(ea, seg.n, mine);
       if (p.argmax.store_logits) reduce_store<1, false>(ea);
-    } else if (seg.res == nullptr) {
+    } else if (EPI == kPlain || (EPI == kAny && seg.res == nullptr)) {
       switch (split) {
         case 1: reduce_store<1, false>(ea); break;
         case 2: reduce_store<2, false>(ea); break;
@@ -727,7 +744,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   if (threadIdx.x == 0) BQ_STAMP(p, 6);
   // nobody leaves while a peer may still read its staging buffer
   if (p.cluster > 1) cluster_sync_all(); else __syncthreads();
-  if (p.pair.on && p.push.n > 0) {
+  if (pair_on && push != nullptr) {
     // ---- column-parallel form: h itself goes to every rank's gathered buffer; the amax needs
     // all ranks' shards and is taken by the quantizer that follows the exchange ----
     __syncthreads();   // parked rows are complete
@@ -736,7 +753,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       const int hcol = (lane & 15) * 4 + (lane >= 16 ? 2 : 0);
       for (int m = m_begin + warp; m < m_end; m += kStreamWarps) {
         const long long at = static_cast<long long>(m) * p.push.ld + col0 + hcol;
-        if (p.out_dtype == BQ_DTYPE_F32) {
+        if (out_dtype == BQ_DTYPE_F32) {
           const float2 v = *reinterpret_cast<const float2*>(part + m * kRowTile + hcol);
           for (int d = 0; d < p.push.n; ++d)
             *reinterpret_cast<float2*>(static_cast<float*>(p.push.dst[d]) + at) = v;
@@ -748,7 +765,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         }
       }
     }
-  } else if (p.pair.on) {
+  } else if (pair_on) {
     // ---- grid-wide max |h| -> scale -> codes of this CTA's rows (h is parked in `part`) ----
     using namespace bq::qd;
 #pragma unroll
@@ -788,11 +805,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     const float sc = s_quant[0];
     if (ok) {
       const EpilogueArgs ea{part, smem_u32(part), 0, m_begin, m_end, warp, lane, row0, 0.0f, true,
-                            nullptr, 0, p.out_dtype, nullptr, 0, &p.push};
+                            nullptr, 0, out_dtype, nullptr, 0, push};
       const int col0 = tile_in_seg * (kRowTile / 2);
-      if (p.out_dtype == BQ_DTYPE_BF16)
+      if (out_dtype == BQ_DTYPE_BF16)
         silu_pair_emit<__nv_bfloat16>(ea, part, sc, p.pair.hq, p.pair.ld_hq, col0);
-      else if (p.out_dtype == BQ_DTYPE_F16)
+      else if (out_dtype == BQ_DTYPE_F16)
         silu_pair_emit<__half>(ea, part, sc, p.pair.hq, p.pair.ld_hq, col0);
       else
         silu_pair_emit<float>(ea, part, sc, p.pair.hq, p.pair.ld_hq, col0);
@@ -806,7 +823,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       }
     }
   }
-  if (p.push.n > 0) {
+  if (push != nullptr) {
     // The stores of all threads of this CTA are ordered before thread 0's fence by the barrier
     // (fences are cumulative); the fence orders them before this CTA's count; the last CTA sees
     // every count, fences again and only then signals the ranks: every store of the launch
@@ -1002,26 +1019,78 @@ __device__ __forceinline__ void silu16(const uint32_t (&g)[16], const uint32_t (
   }
 }
 
+// 16 bytes of the output type, already rounded to it, plus 16 residual bytes, rounded again.
+template <int ES>
+__device__ __forceinline__ uint4 add_res_piece(const uint4& v, const uint4& r, int out_dtype) {
+  using namespace bq::qd;
+  const uint32_t a[4] = {v.x, v.y, v.z, v.w}, b[4] = {r.x, r.y, r.z, r.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (ES == 4) {
+      o[i] = __float_as_uint(__fadd_rn(__uint_as_float(a[i]), __uint_as_float(b[i])));
+    } else if (out_dtype == BQ_DTYPE_BF16) {
+      const float2 x = unpack2<__nv_bfloat16>(a[i]), y = unpack2<__nv_bfloat16>(b[i]);
+      o[i] = pack2<__nv_bfloat16>(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y));
+    } else {
+      const float2 x = unpack2<__half>(a[i]), y = unpack2<__half>(b[i]);
+      o[i] = pack2<__half>(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y));
+    }
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // The epilogue of one warp for one tile: 32 rows x 256 accumulator columns.  SILU: the tile's
 // columns [0,128) are gate and [128,256) up of the same 128 output columns, and the output is
 // h = silu(gate) * up (128 columns); max |h| is folded into `mx`.
-template <int ES, bool SILU>
+// RES: the residual's rows come in as coalesced 128-byte pieces (asked for before the box is free), go
+// through the box into the lane-per-row order of the accumulator, and the sums replace them there.  The
+// reads hide behind the next tile's MMAs; a separate add moved three times the bytes (38 us at 9658 x
+// 4096, and a launch).
+template <int ES, bool SILU, bool RES, bool PUSH>
 __device__ __forceinline__ void pair_epilogue_rows(const GemmParams& p, const Segment& seg,
                                                    const CUtensorMap* ymap, bool use_tma,
                                                    uint32_t taddr, float scale, float scale_up,
-                                                   int m_row0, int n0, uint8_t* box,
+                                                   int out_dtype, int m_row0, int n0, uint8_t* box,
                                                    uint32_t box_addr, int lane, int col_half,
                                                    float& mx) {
   constexpr int kCols = 128 / ES;              // output columns per 128-byte piece
   constexpr int kPieces = ES == 4 ? 4 : 2;     // 16-byte pieces per 16 accumulator columns
-  const int out_cols = SILU ? kPairTile / 2 : p.pair_n;
-  const int c_end = (col_half + 1) * (out_cols / 2);
-  for (int c = col_half * (out_cols / 2); c < c_end; c += kCols) {
+  const int out_cols = SILU ? kPairTile / 2 : (seg.dense ? seg.un : p.pair_n);
+  const int half_cols = (out_cols / 2 + kCols - 1) / kCols * kCols;   // whole pieces: 16-bit weights may be narrow
+  const int c_end = (col_half + 1) * half_cols;
+  for (int c = col_half * half_cols; c < c_end; c += kCols) {
     // pieces beyond this weight's rows are never stored (warp-uniform)
     if ((n0 + c) >= seg.n) break;
+    uint4 rv[RES ? 8 : 1];
+    if constexpr (RES) {
+      const int col = n0 + c + (lane & 7) * (16 / ES);
+#pragma unroll
+      for (int pass = 0; pass < 8; ++pass) {
+        const int m = m_row0 + pass * 4 + (lane >> 3);
+        rv[pass] = make_uint4(0u, 0u, 0u, 0u);
+        if (m < p.M && col < seg.n) {
+          const uint8_t* src = static_cast<const uint8_t*>(seg.res) + ((long long)m * seg.ld_res + col) * ES;
+          if (seg.wide) {
+            rv[pass] = ld_coherent16(src);
+          } else {                              // rows are 8-byte aligned at least (checked by the host)
+            const uint2 lo = ld_coherent8(src), hi = ld_coherent8(src + 8);
+            rv[pass] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+          }
+        }
+      }
+    }
     // the TMA store of the previous piece must have finished reading the box
     if (use_tma && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     __syncwarp();
+    if constexpr (RES) {
+#pragma unroll
+      for (int pass = 0; pass < 8; ++pass) {
+        const int row = pass * 4 + (lane >> 3);
+        *reinterpret_cast<uint4*>(box + row * 128 + (((lane & 7) ^ (row & 7)) << 4)) = rv[pass];
+      }
+      __syncwarp();
+    }
 #pragma unroll
     for (int j = 0; j < kCols; j += 16) {
       uint32_t r[16];
@@ -1032,16 +1101,18 @@ __device__ __forceinline__ void pair_epilogue_rows(const GemmParams& p, const Se
         tmem_ld16(taddr + kPairTile / 2 + c + j, up);
         tmem_ld_wait();
         if constexpr (ES == 4) silu16<float>(r, up, scale, scale_up, v, mx);
-        else if (p.out_dtype == BQ_DTYPE_BF16) silu16<__nv_bfloat16>(r, up, scale, scale_up, v, mx);
+        else if (out_dtype == BQ_DTYPE_BF16) silu16<__nv_bfloat16>(r, up, scale, scale_up, v, mx);
         else silu16<__half>(r, up, scale, scale_up, v, mx);
       } else {
         tmem_ld_wait();
-        cast16<ES>(r, scale, p.out_dtype, v);
+        cast16<ES>(r, scale, out_dtype, v);
       }
 #pragma unroll
       for (int q = 0; q < kPieces; ++q) {
         const int piece = (j * ES) / 16 + q;                  // 0..7 along the 128-byte row
-        *reinterpret_cast<uint4*>(box + lane * 128 + ((piece ^ (lane & 7)) << 4)) = v[q];
+        uint4* const at = reinterpret_cast<uint4*>(box + lane * 128 + ((piece ^ (lane & 7)) << 4));
+        if constexpr (RES) *at = add_res_piece<ES>(v[q], *at, out_dtype);
+        else *at = v[q];
       }
     }
     if (use_tma) {
@@ -1051,7 +1122,7 @@ __device__ __forceinline__ void pair_epilogue_rows(const GemmParams& p, const Se
         // column-parallel form: the same box into every rank's gathered buffer (ymap[d] then
         // describes rank d's buffer at this rank's columns; peers' buffers are reached through
         // peer-mapped addresses by plain, non-multicast bulk stores)
-        const int n_dst = p.push.n > 0 ? p.push.n : 1;
+        const int n_dst = PUSH && p.push.n > 0 ? p.push.n : 1;
         for (int d = 0; d < n_dst; ++d) tma_store_2d(ymap + d, box_addr, n0 + c, m_row0);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
@@ -1067,7 +1138,7 @@ __device__ __forceinline__ void pair_epilogue_rows(const GemmParams& p, const Se
         const uint4 v = *reinterpret_cast<const uint4*>(box + row * 128 + ((piece ^ (row & 7)) << 4));
         if (m < p.M && col < seg.n) {         // n is a multiple of 16: a piece is in or out as a whole
           // rows are 8-byte aligned at least (checked by the host)
-          if (p.push.n == 0) {
+          if (!PUSH || p.push.n == 0) {
             uint8_t* dst = static_cast<uint8_t*>(seg.y) + ((long long)m * seg.ldy + col) * ES;
             *reinterpret_cast<uint2*>(dst) = make_uint2(v.x, v.y);
             *reinterpret_cast<uint2*>(dst + 8) = make_uint2(v.z, v.w);
@@ -1088,11 +1159,14 @@ __device__ __forceinline__ void pair_epilogue_rows(const GemmParams& p, const Se
   }
 }
 
+template <int EPI, int DT>
 __global__ void __launch_bounds__(kTileThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xd,
                  const __grid_constant__ WeightMaps tm_w, const __grid_constant__ OutMaps tm_y,
                  const __grid_constant__ GemmParams p) {
   extern __shared__ uint8_t smem_dyn[];
+  const int out_dtype = DT == kAnyType ? p.out_dtype : DT;
+  const int push_n = EPI == kAny ? p.push.n : 0;
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
   const uint32_t bar_base = base + kPairStages * kPairStageBytes;
@@ -1113,7 +1187,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
   const int rank = static_cast<int>(cluster_ctarank());     // 0 = leader of the pair
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int m_tiles = (p.M + kPairTile - 1) / kPairTile;
-  const bool silu = p.pair.on != 0;                       // gate/up tiles, h = silu(gate) * up out
+  const bool silu = EPI == kAny ? p.pair.on != 0 : EPI == kGateUp;                       // gate/up tiles, h = silu(gate) * up out
   // output columns per tile: 128 of h in the SiLU form; 256 in the plain form, or 128 for a weight
   // so narrow that 256-wide tiles would leave CTA pairs without work (same sums, more tiles)
   const int n_step = silu ? kPairTile / 2 : p.pair_n;
@@ -1153,18 +1227,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
       for (int t = pair; t < p.total_tiles && ok; t += n_pairs) {
         const int sg = find_segment(p, t);
         const int local = t - p.seg[sg].tile_begin;
+        const bool dense = EPI == kMixed && p.seg[sg].dense != 0;
         int m_idx, n_idx;
-        pair_tile_coords(local, m_tiles, (p.seg[sg].n + n_step - 1) / n_step, m_idx, n_idx);
+        pair_tile_coords(local, m_tiles, dense ? 1 : (p.seg[sg].n + n_step - 1) / n_step, m_idx, n_idx);
         const int m0 = m_idx * kPairTile + rank * kRowTile;
         // plain: this CTA's half of the tile's 256 weight rows; SiLU form: the leader loads 128
         // gate rows, its peer the 128 up rows of the same output columns
-        const int n0 = silu ? n_idx * kRowTile : n_idx * n_step + rank * b_rows;
+        const int rows = dense ? p.seg[sg].un / 2 : b_rows;
+        const int n0 = silu ? n_idx * kRowTile : n_idx * n_step + rank * rows;
         const CUtensorMap* const w_map = silu ? &tm_w.w[rank] : &tm_w.w[sg];
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        const CUtensorMap* const x_map = dense ? &tm_xd : &tm_x;
+        const int blocks = dense ? p.k_blocks_dense : p.k_blocks;
+        for (int kb = 0; kb < blocks; ++kb, ++it) {
           const int s = it % kPairStages, use = it / kPairStages;
           if (use > 0 && !mbar_wait(empty_bar(s), (use - 1) & 1)) { ok = false; break; }
-          if (rank == 0) mbar_expect_tx(full_bar(s), 2u * (kATileBytes + (uint32_t)b_rows * kBK));
-          tma_load_2d_pair(a_tile(s), &tm_x, full_bar(s), kb * kBK, m0, pol);
+          if (rank == 0) mbar_expect_tx(full_bar(s), 2u * (kATileBytes + (uint32_t)rows * kBK));
+          tma_load_2d_pair(a_tile(s), x_map, full_bar(s), kb * kBK, m0, pol);
           tma_load_2d_pair(b_tile(s), w_map, full_bar(s), kb * kBK, n0, pol);
         }
       }
@@ -1182,15 +1260,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
         if (use_b > 0 && !mbar_wait(acc_empty(b), (use_b - 1) & 1)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + b * kPairTile;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        const Segment& seg = p.seg[find_segment(p, t)];
+        const bool dense = EPI == kMixed && seg.dense != 0;
+        const uint32_t idesc_d = dense ? idesc_f16(kPairTile, seg.un, p.dense_fmt) : 0u;
+        const int blocks = dense ? p.k_blocks_dense : p.k_blocks;
+        for (int kb = 0; kb < blocks; ++kb, ++it) {
           const int s = it % kPairStages, use = it / kPairStages;
           if (!mbar_wait(full_bar(s), use & 1)) { ok = false; break; }
           tc_fence_after();
           const uint64_t da = smem_desc_sw128(a_tile(s));
           const uint64_t db = smem_desc_sw128(b_tile(s));
 #pragma unroll
-          for (int j = 0; j < kBK / kUmmaK; ++j)
-            mma_f8_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
+          for (int j = 0; j < kBK / kUmmaK; ++j) {
+            if (dense) mma_f16_pair(tmem_d, da + 2u * j, db + 2u * j, idesc_d, (kb | j) != 0 ? 1u : 0u);
+            else mma_f8_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
+          }
           // the stage is free in BOTH CTAs once these MMAs retire
           mma_commit_pair(empty_bar(s));
           mma_commit_pair(map_to_cta(empty_bar(s), 1));
@@ -1219,30 +1303,30 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
       const Segment seg = p.seg[sg];
       const int local = t - seg.tile_begin;
       int m_idx, n_idx;
-      pair_tile_coords(local, m_tiles, (seg.n + n_step - 1) / n_step, m_idx, n_idx);
+      pair_tile_coords(local, m_tiles, seg.dense ? 1 : (seg.n + n_step - 1) / n_step, m_idx, n_idx);
       const int m0 = m_idx * kPairTile + rank * kRowTile;
       const int n0 = n_idx * n_step;
       if (!mbar_wait(acc_full(b), use_b & 1)) { ok = false; break; }
       tc_fence_after();
       const float sx = ld_coherent4(p.sx);
-      const float scale = sx * __ldg(seg.sw);
+      const float scale = EPI == kMixed && seg.dense ? 1.0f : sx * __ldg(seg.sw);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + b * kPairTile;
       const bool use_tma = seg.y_tma != 0;
-      if (silu) {
-        const float scale_up = sx * __ldg(p.pair.sw_up);
-        if (p.out_dtype == BQ_DTYPE_F32)
-          pair_epilogue_rows<4, true>(p, seg, &tm_y.y[p.push.n > 0 ? 0 : sg], use_tma, taddr, scale, scale_up,
-                                      m0 + quad * 32, n0, stage, stage_addr, lane, col_half, h_max);
-        else
-          pair_epilogue_rows<2, true>(p, seg, &tm_y.y[p.push.n > 0 ? 0 : sg], use_tma, taddr, scale, scale_up,
-                                      m0 + quad * 32, n0, stage, stage_addr, lane, col_half, h_max);
-      } else if (p.out_dtype == BQ_DTYPE_F32) {
-        pair_epilogue_rows<4, false>(p, seg, &tm_y.y[p.push.n > 0 ? 0 : sg], use_tma, taddr, scale, 0.0f, m0 + quad * 32,
-                                     n0, stage, stage_addr, lane, col_half, h_max);
+      const CUtensorMap* const ymap = &tm_y.y[push_n > 0 ? 0 : sg];
+      const float scale_up = silu ? sx * __ldg(p.pair.sw_up) : 0.0f;
+#define BQ_ROWS(ES, SILU, RES)                                                                                          \
+  pair_epilogue_rows<ES, SILU, RES, EPI == kAny>(p, seg, ymap, use_tma, taddr, scale, scale_up, out_dtype, m0 + quad * 32, \
+                                                 n0, stage, stage_addr, lane, col_half, h_max)
+      if constexpr (DT == BQ_DTYPE_F32) {
+        BQ_ROWS(4, EPI == kGateUp, EPI == kResidual);
+      } else if constexpr (DT != kAnyType) {
+        BQ_ROWS(2, EPI == kGateUp, EPI == kResidual);
+      } else if (out_dtype == BQ_DTYPE_F32) {
+        if (silu) BQ_ROWS(4, true, false); else BQ_ROWS(4, false, false);
       } else {
-        pair_epilogue_rows<2, false>(p, seg, &tm_y.y[p.push.n > 0 ? 0 : sg], use_tma, taddr, scale, 0.0f, m0 + quad * 32,
-                                     n0, stage, stage_addr, lane, col_half, h_max);
+        if (silu) BQ_ROWS(2, true, false); else BQ_ROWS(2, false, false);
       }
+#undef BQ_ROWS
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(b == 0 ? leader_acc_empty0 : leader_acc_empty1);
@@ -1251,11 +1335,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x,
     // form the wait also means the stores have been written, before anybody is told to look
     if (lane == 0) {
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-      if (p.push.n > 0) asm volatile("fence.proxy.async;" ::: "memory");
+      if (push_n > 0) asm volatile("fence.proxy.async;" ::: "memory");
     }
     __syncwarp();
     if (!ok) *abort_flag = 1;
-    if (p.push.n > 0) {
+    if (push_n > 0) {
       // The stores of all epilogue threads are ordered before the elected thread's fence by the
       // barrier (fences are cumulative); the fence orders them before this CTA's count; the
       // last CTA sees every count, fences again and only then signals the ranks: every store of
@@ -1434,18 +1518,65 @@ thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
 
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
+using StreamKernel = decltype(&gemm_stream_kernel<kAny, kAnyType>);
+using WideKernel = decltype(&gemm_wide_kernel<1, kAny, kAnyType>);
+using PairKernel = decltype(&gemm_pair_kernel<kAny, kAnyType>);
+
+// The kernels by [epilogue][type]; the types are BQ_DTYPE_F32, BF16, F16 = 0, 1, 2.
+const StreamKernel kStream[3][3] = {
+    {gemm_stream_kernel<kPlain, 0>, gemm_stream_kernel<kPlain, 1>, gemm_stream_kernel<kPlain, 2>},
+    {gemm_stream_kernel<kResidual, 0>, gemm_stream_kernel<kResidual, 1>, gemm_stream_kernel<kResidual, 2>},
+    {gemm_stream_kernel<kGateUp, 0>, gemm_stream_kernel<kGateUp, 1>, gemm_stream_kernel<kGateUp, 2>}};
+const StreamKernel kStreamAny = gemm_stream_kernel<kAny, kAnyType>;
+template <int MODE>
+struct WideKernels {
+  static constexpr WideKernel any = gemm_wide_kernel<MODE, kAny, kAnyType>;
+  static constexpr WideKernel of[3][3] = {
+      {gemm_wide_kernel<MODE, kPlain, 0>, gemm_wide_kernel<MODE, kPlain, 1>, gemm_wide_kernel<MODE, kPlain, 2>},
+      {gemm_wide_kernel<MODE, kResidual, 0>, gemm_wide_kernel<MODE, kResidual, 1>, gemm_wide_kernel<MODE, kResidual, 2>},
+      {gemm_wide_kernel<MODE, kGateUp, 0>, gemm_wide_kernel<MODE, kGateUp, 1>, gemm_wide_kernel<MODE, kGateUp, 2>}};
+};
+const PairKernel kPair[4][3] = {
+    {gemm_pair_kernel<kPlain, 0>, gemm_pair_kernel<kPlain, 1>, gemm_pair_kernel<kPlain, 2>},
+    {gemm_pair_kernel<kResidual, 0>, gemm_pair_kernel<kResidual, 1>, gemm_pair_kernel<kResidual, 2>},
+    {gemm_pair_kernel<kGateUp, 0>, gemm_pair_kernel<kGateUp, 1>, gemm_pair_kernel<kGateUp, 2>},
+    {nullptr, gemm_pair_kernel<kMixed, 1>, gemm_pair_kernel<kMixed, 2>}};
+const PairKernel kPairAny = gemm_pair_kernel<kAny, kAnyType>;
+
+// The form all segments of a launch share, or kAny.  `mixed`: does the kernel have a form for 16-bit
+// segments (elsewhere they are a matter of a segment)?
+int epilogue_of(const GemmParams& p, bool mixed) {
+  if (p.push.n > 0 || p.argmax.on) return kAny;
+  if (p.pair.on) return kGateUp;
+  int with = 0, dense = 0;
+  for (int i = 0; i < p.n_seg; ++i) {
+    with += p.seg[i].res != nullptr;
+    dense += p.seg[i].dense != 0;
+  }
+  if (mixed && dense > 0) return kMixed;               // never with a residual
+  return with == 0 ? kPlain : (with == p.n_seg ? kResidual : kAny);
+}
+
 int configure_once() {
   static int rc = -1;
   if (rc < 0) {
-    cudaError_t e1 = cudaFuncSetAttribute(gemm_stream_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    cudaError_t e3 = cudaFuncSetAttribute(gemm_pair_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    cudaError_t e4 = cudaFuncSetAttribute(gemm_wide_kernel<1>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    cudaError_t e5 = cudaFuncSetAttribute(gemm_wide_kernel<2>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    rc = (e1 == cudaSuccess && e3 == cudaSuccess && e4 == cudaSuccess && e5 == cudaSuccess) ? kOk : kErrLaunch;
+    bool ok = true;
+    auto set = [&](const void* kernel) {
+      ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) == cudaSuccess;
+    };
+    set((const void*)kStreamAny);
+    set((const void*)WideKernels<1>::any);
+    set((const void*)WideKernels<2>::any);
+    set((const void*)kPairAny);
+    for (int e = 0; e < 4; ++e)
+      for (int d = 0; d < 3; ++d) {
+        if (kPair[e][d] != nullptr) set((const void*)kPair[e][d]);
+        if (e == 3) continue;
+        set((const void*)kStream[e][d]);
+        set((const void*)WideKernels<1>::of[e][d]);
+        set((const void*)WideKernels<2>::of[e][d]);
+      }
+    rc = ok ? kOk : kErrLaunch;
     if (rc != kOk) (void)cudaGetLastError();
   }
   return rc;
@@ -1453,12 +1584,12 @@ int configure_once() {
 
 // Largest grid of the stream kernel that is resident at once with this cluster
 // size and shared-memory footprint (the paired gate/up epilogue has a grid-wide wait).
-int max_resident_ctas(int cluster, int smem) {
-  struct Entry { int cluster, smem, cap; };
+int max_resident_ctas(StreamKernel kernel, int cluster, int smem) {
+  struct Entry { StreamKernel kernel; int cluster, smem, cap; };
   static Entry cache[64];
   static int n_cached = 0;
   for (int i = 0; i < n_cached; ++i)
-    if (cache[i].cluster == cluster && cache[i].smem == smem) return cache[i].cap;
+    if (cache[i].kernel == kernel && cache[i].cluster == cluster && cache[i].smem == smem) return cache[i].cap;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(cluster * 64), 1, 1);
@@ -1472,7 +1603,7 @@ int max_resident_ctas(int cluster, int smem) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_stream_kernel, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     clusters = 0;
   }
@@ -1483,7 +1614,7 @@ int max_resident_ctas(int cluster, int smem) {
   cudaFuncAttributes fa;
   memset(&fa, 0, sizeof(fa));
   int regs = 128;
-  if (cudaFuncGetAttributes(&fa, gemm_stream_kernel) == cudaSuccess && fa.numRegs > 0)
+  if (cudaFuncGetAttributes(&fa, kernel) == cudaSuccess && fa.numRegs > 0)
     regs = fa.numRegs;
   else
     (void)cudaGetLastError();
@@ -1496,7 +1627,7 @@ int max_resident_ctas(int cluster, int smem) {
   if (getenv("BQ_DEBUG"))
     fprintf(stderr, "[bq] residency: cluster %d smem %d regs %d -> %d clusters x %d per SM = %d CTAs\n",
             cluster, smem, regs, clusters, per_sm, cap);
-  if (n_cached < 64) cache[n_cached++] = Entry{cluster, smem, cap};
+  if (n_cached < 64) cache[n_cached++] = Entry{kernel, cluster, smem, cap};
   return cap;
 }
 
@@ -1585,12 +1716,14 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   if (tile_bytes < staging) tile_bytes = staging;
   const int smem = tile_bytes + kBarrierBytes + 1024;
   if (smem > kMaxSmem) return kErrUnsupported;
+  const int epi = epilogue_of(p, false);
+  const StreamKernel kernel = epi == kAny ? kStreamAny : kStream[epi][p.out_dtype];
   if (p.pair.on) p.pair.expected = (unsigned)((p.seg[0].n / kRowTile) * p.seg[0].split);
   if (p.push.n > 0)
     p.push.expected = (unsigned)(((p.seg[0].n + kRowTile - 1) / kRowTile) * p.seg[0].split);
   if (p.pair.on && p.push.n == 0) {
     // the epilogue's amax exchange waits on the whole grid: every CTA must be resident
-    const int cap = max_resident_ctas(cluster, smem);
+    const int cap = max_resident_ctas(kernel, cluster, smem);
     if (getenv("BQ_DEBUG"))
       fprintf(stderr, "[bq] paired launch: grid %lld cluster %d smem %d resident cap %d\n", grid,
               cluster, smem, cap);
@@ -1618,7 +1751,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
 #endif
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_stream_kernel, tm_x, tm_xd, maps, p, tile_bytes);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm_x, tm_xd, maps, p, tile_bytes);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
 }
@@ -1642,7 +1775,7 @@ int max_pairs() {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_wide_kernel<2>, &cfg) != cudaSuccess || clusters < 1) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, WideKernels<2>::any, &cfg) != cudaSuccess || clusters < 1) {
       (void)cudaGetLastError();
       clusters = device_sms() / 2;
     }
@@ -1792,13 +1925,16 @@ int launch_wide(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
 #endif
-  const cudaError_t e = sh.mode == 1 ? cudaLaunchKernelEx(&cfg, gemm_wide_kernel<1>, tm_x, tm_xd, maps, p, sh)
-                                     : cudaLaunchKernelEx(&cfg, gemm_wide_kernel<2>, tm_x, tm_xd, maps, p, sh);
+  const int epi = epilogue_of(p, false);
+  const WideKernel kernel =
+      sh.mode == 1 ? (epi == kAny ? WideKernels<1>::any : WideKernels<1>::of[epi][p.out_dtype])
+                   : (epi == kAny ? WideKernels<2>::any : WideKernels<2>::of[epi][p.out_dtype]);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm_x, tm_xd, maps, p, sh);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
 }
 
-int launch_pair(const CUtensorMap& tm_x, const WeightMaps& maps, const OutMaps& ymaps, GemmParams& p,
+int launch_pair(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightMaps& maps, const OutMaps& ymaps, GemmParams& p,
                 cudaStream_t stream) {
   const int sms = device_sms();
   if (sms <= 0) return kErrLaunch;
@@ -1807,6 +1943,7 @@ int launch_pair(const CUtensorMap& tm_x, const WeightMaps& maps, const OutMaps& 
                 "pair kernel: pipeline + store boxes exceed the shared memory of an SM");
   int pairs = p.total_tiles < sms / 2 ? p.total_tiles : sms / 2;
   if (pairs < 1) pairs = 1;
+  const int epi = epilogue_of(p, true);
   if (p.push.n > 0) p.push.expected = (unsigned)(2 * pairs);   // every CTA has a tile and stores
   g_last_launch[0] = 2; g_last_launch[1] = 2 * pairs; g_last_launch[2] = 2;
   g_last_launch[3] = kPairStages; g_last_launch[4] = smem; g_last_launch[5] = p.pair_n;
@@ -1825,7 +1962,7 @@ int launch_pair(const CUtensorMap& tm_x, const WeightMaps& maps, const OutMaps& 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_opt_pdl ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel, tm_x, maps, ymaps, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, epi == kAny ? kPairAny : kPair[epi][p.out_dtype], tm_x, tm_xd, maps, ymaps, p);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
 }
@@ -1994,8 +2131,11 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     if (N[i] > 0x7fffff00LL) return kErrTooLarge;
   }
   const bool stream_path = M <= g_opt_stream_max_m;
-  if (dn != nullptr) {    // 16-bit segments exist in the weight-streaming kernel only
-    if (!stream_path || pair || push || res) return kErrUnsupported;
+  if (dn != nullptr) {
+    if (pair || push || res) return kErrUnsupported;
+    // prefill sizes: 16-bit weights of one tile column (gates); wider ones are a library GEMM's business
+    for (int i = 0; i < n_seg && !stream_path; ++i)
+      if (dn->kind[i] != 0 && N[i] > kPairTile) return kErrUnsupported;
     if (!dn->x || (dn->dtype != BQ_DTYPE_BF16 && dn->dtype != BQ_DTYPE_F16)) return kErrBadArg;
     if (!aligned_to(dn->x, 16)) return kErrUnsupported;
   }
@@ -2011,8 +2151,8 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
         if (!aligned_to(push->dst[d], 16)) return kErrUnsupported;
     }
   }
-  if (res != nullptr) {   // the residual epilogue exists in the weight-streaming kernel only
-    if (!stream_path || ld_res == nullptr) return kErrUnsupported;
+  if (res != nullptr) {
+    if (ld_res == nullptr) return kErrUnsupported;
     for (int i = 0; i < n_seg; ++i)
       if (res[i] && (ld_res[i] < N[i] || ld_res[i] % 4 || !aligned_to(res[i], out_align)))
         return kErrUnsupported;
@@ -2083,7 +2223,12 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     p.seg[i].n = (int)N[i];
     p.seg[i].dense = (dn != nullptr && dn->kind[i] != 0) ? 1 : 0;
     p.seg[i].tile_begin = tiles;
-    const long long nt = (N[i] + tile_n - 1) / tile_n;
+    if (pair_path && p.seg[i].dense) p.seg[i].un = (int)((N[i] + 31) / 32 * 32);   // MMA N granularity of a pair
+    if (pair_path && res != nullptr && res[i] != nullptr) {
+      const size_t es = out_dtype == BQ_DTYPE_F32 ? 4 : 2;
+      p.seg[i].wide = aligned_to(res[i], 16) && (ld_res[i] * es) % 16 == 0 ? 1 : 0;
+    }
+    const long long nt = pair_path && p.seg[i].dense ? 1 : (N[i] + tile_n - 1) / tile_n;
     const long long add = stream_path ? nt : nt * p.m_tiles;
     if (tiles + add > 0x3fffffffLL) return kErrTooLarge;
     tiles += (int)add;
@@ -2108,8 +2253,10 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
       // two maps over the two weights, 64-row boxes: the kernel puts a tile together from both
       if (int rc = make_map(&maps.w[0], wq[0], N[0] / 2, K, kRowTile / 2)) return rc;
       if (int rc = make_map(&maps.w[1], pair->wq_up, N[0] / 2, K, kRowTile / 2)) return rc;
-    } else if (int rc = make_map(&maps.w[i], wq[i], N[i], p.seg[i].dense ? 2 * K : K, w_box_rows)) {
-      return rc;     // a 16-bit weight is described by its bytes: [N, 2K]
+    } else {
+      // a 16-bit weight is described by its bytes: [N, 2K]
+      const int box_rows = pair_path && p.seg[i].dense ? p.seg[i].un / 2 : w_box_rows;
+      if (int rc = make_map(&maps.w[i], wq[i], N[i], p.seg[i].dense ? 2 * K : K, box_rows)) return rc;
     }
   }
   p.total_tiles = tiles;
@@ -2123,7 +2270,10 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     return launch_stream(tm_x, tm_xd, maps, p, stream);
   }
   if (int rc = make_map(&tm_x, xq, M, K, kRowTile)) return rc;
-  return launch_pair(tm_x, maps, ymaps, p, stream);
+  CUtensorMap tm_xd = tm_x;
+  if (dn != nullptr)
+    if (int rc = make_map(&tm_xd, dn->x, M, 2 * K, kRowTile)) return rc;
+  return launch_pair(tm_x, tm_xd, maps, ymaps, p, stream);
 }
 
 }  // namespace

@@ -139,14 +139,14 @@ struct UnitOut {
   bool row_ok;
 };
 
-template <typename T>
+template <typename T, int EPI>
 __device__ __forceinline__ void store_chunk(const UnitOut& o, int c, float (&v)[16]) {
   const int col = o.row0 + c;
   if (!o.row_ok || col >= o.seg.n) return;        // n is a multiple of 16: a chunk is in or out
   const bool wide = o.seg.wide != 0;
-  if (o.seg.res != nullptr)
+  if (EPI == kResidual || (EPI == kAny && o.seg.res != nullptr))
     add_res16<T>(v, static_cast<const T*>(o.seg.res) + (long long)o.m * o.seg.ld_res + col, wide);
-  if (o.p.push.n == 0) {
+  if (EPI != kAny || o.p.push.n == 0) {
     store16<T>(static_cast<T*>(o.seg.y) + (long long)o.m * o.seg.ldy + col, v, wide);
   } else {
     for (int d = 0; d < o.p.push.n; ++d)
@@ -261,7 +261,7 @@ __device__ __forceinline__ void pair_push(const PairTile<T>& t, const PushParams
 }
 
 // Everything after the accumulator of the gate/up form is complete.  All threads of the CTA.
-template <typename T, int MODE>
+template <typename T, int MODE, int EPI>
 __device__ __forceinline__ void pair_finish(const GemmParams& p, uint8_t* smem, float* s_red, uint32_t taddr, int unit,
                                             int m0, int rows, bool ok, float sg, float su) {
   using namespace bq::qd;
@@ -276,7 +276,7 @@ __device__ __forceinline__ void pair_finish(const GemmParams& p, uint8_t* smem, 
   if (threadIdx.x == 0) BQ_STAMP(p, 1);
   float mx = ok ? pair_silu(t) : 0.0f;
   const int col0 = unit * un, cols = p.seg[0].n;
-  if (p.push.n > 0) {
+  if (EPI == kAny && p.push.n > 0) {
     __syncthreads();
     if (ok) pair_push(t, p.push, m0, col0, cols);
     return;      // the amax needs every rank's shard: the quantizer behind the exchange takes it
@@ -390,12 +390,14 @@ __device__ __forceinline__ bool issue_unit(const GemmParams& p, const RingShape&
   return true;
 }
 
-template <int MODE>
+template <int MODE, int EPI, int DT>
 __global__ void __launch_bounds__(kWideThreads, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xd,
                    const __grid_constant__ WeightMaps tm_w, const __grid_constant__ GemmParams p,
                    const __grid_constant__ WideShape sh) {
   using Lanes = LaneMap<MODE>;
+  const int out_dtype = DT == kAnyType ? p.out_dtype : DT;
+  const bool argmax_on = EPI == kAny && p.argmax.on;
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
@@ -428,7 +430,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int crank = static_cast<int>(cluster_ctarank());
   const bool many = sh.rounds > 1;                           // two accumulators, dedicated epilogue warps
-  const bool paired = p.pair.on != 0;
+  const bool paired = EPI == kAny ? p.pair.on != 0 : EPI == kGateUp;
   const int m0 = crank * sh.m_half;                          // first batch row of this CTA
 
   if (threadIdx.x == 0) {
@@ -561,10 +563,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       const float sw = seg.dense ? 1.0f : __ldg(seg.sw);
       const float sw_up = paired ? __ldg(p.pair.sw_up) : 0.0f;
       const int b = many ? round & 1 : 0;
-      if (seg.res != nullptr && row_ok) {
+      if ((EPI == kResidual || (EPI == kAny && seg.res != nullptr)) && row_ok) {
         // the residual's lines on their way while the MMAs run
         const int col = (unit - seg.unit_begin) * seg.un + Lanes::col0(quad, seg.un) + col_group * 16;
-        const int es = p.out_dtype == BQ_DTYPE_F32 ? 4 : 2;
+        const int es = out_dtype == BQ_DTYPE_F32 ? 4 : 2;
         if (col < seg.n)
           asm volatile("prefetch.global.L1 [%0];" ::"l"(static_cast<const uint8_t*>(seg.res) +
                                                          ((long long)(m0 + row) * seg.ld_res + col) * es));
@@ -581,12 +583,12 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       const float scale = seg.dense ? 1.0f : sx * sw;
       if (paired) {
         const float su = sx * sw_up;
-        if (p.out_dtype == BQ_DTYPE_BF16)
-          pair_finish<__nv_bfloat16, MODE>(p, base_ptr, s_red, taddr, unit, m0, rows, ok, scale, su);
-        else if (p.out_dtype == BQ_DTYPE_F16)
-          pair_finish<__half, MODE>(p, base_ptr, s_red, taddr, unit, m0, rows, ok, scale, su);
+        if (out_dtype == BQ_DTYPE_BF16)
+          pair_finish<__nv_bfloat16, MODE, EPI>(p, base_ptr, s_red, taddr, unit, m0, rows, ok, scale, su);
+        else if (out_dtype == BQ_DTYPE_F16)
+          pair_finish<__half, MODE, EPI>(p, base_ptr, s_red, taddr, unit, m0, rows, ok, scale, su);
         else
-          pair_finish<float, MODE>(p, base_ptr, s_red, taddr, unit, m0, rows, ok, scale, su);
+          pair_finish<float, MODE, EPI>(p, base_ptr, s_red, taddr, unit, m0, rows, ok, scale, su);
       } else if (ok && warp_ok) {
         const int cols = Lanes::cols(seg.un);
         const UnitOut o{p, seg, (unit - seg.unit_begin) * seg.un + Lanes::col0(quad, seg.un), m0 + row, row_ok};
@@ -596,15 +598,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           load_sums(taddr + c, seg.split, cols, v);
 #pragma unroll
           for (int q = 0; q < 16; ++q) v[q] *= scale;
-          if (p.argmax.on) {
-            if (p.out_dtype == BQ_DTYPE_BF16) argmax_chunk<__nv_bfloat16>(o, c, v, bv, bi);
-            else if (p.out_dtype == BQ_DTYPE_F16) argmax_chunk<__half>(o, c, v, bv, bi);
+          if (argmax_on) {
+            if (out_dtype == BQ_DTYPE_BF16) argmax_chunk<__nv_bfloat16>(o, c, v, bv, bi);
+            else if (out_dtype == BQ_DTYPE_F16) argmax_chunk<__half>(o, c, v, bv, bi);
             else argmax_chunk<float>(o, c, v, bv, bi);
             if (!p.argmax.store_logits) continue;
           }
-          if (p.out_dtype == BQ_DTYPE_BF16) store_chunk<__nv_bfloat16>(o, c, v);
-          else if (p.out_dtype == BQ_DTYPE_F16) store_chunk<__half>(o, c, v);
-          else store_chunk<float>(o, c, v);
+          if (out_dtype == BQ_DTYPE_BF16) store_chunk<__nv_bfloat16, EPI>(o, c, v);
+          else if (out_dtype == BQ_DTYPE_F16) store_chunk<__half, EPI>(o, c, v);
+          else store_chunk<float, EPI>(o, c, v);
         }
       }
       if (many) {
@@ -614,7 +616,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(b), 0));
       }
     }
-    if (p.argmax.on && row_ok) {
+    if (argmax_on && row_ok) {
       // a pair of 128 holds a row's columns in two lane quarters: two slots per column group
       const int slot = (unit0 * n_groups + col_group) * (MODE == 1 ? 2 : 1) + (MODE == 1 ? quad >> 1 : 0);
       p.argmax.partial[static_cast<size_t>(slot) * p.M + m0 + row] =
@@ -624,7 +626,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   }
   tc_fence_before();
   cluster_sync_all();   // nobody frees tensor memory while the peer may still use the pair
-  if (p.push.n > 0 && threadIdx.x == 0) {
+  if (EPI == kAny && p.push.n > 0 && threadIdx.x == 0) {
     // The stores of all threads of this CTA are ordered before thread 0's fence by the barrier
     // (fences are cumulative); the fence orders them before this CTA's count; the last CTA sees
     // every count, fences again and only then signals the ranks: every store of the launch

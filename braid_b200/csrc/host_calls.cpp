@@ -53,8 +53,6 @@ struct Lib {
 bool g_ready = false;
 int64_t g_two_launch_from = 0;
 
-constexpr int64_t kDecodeRows = 256;     // residuals and 16-bit members ride in the GEMM up to here
-
 constexpr int kMaxDevices = 64;
 struct Scratch {
   std::atomic<uint64_t> base{0};      // device address of the slots, 0 = none yet
@@ -351,7 +349,6 @@ at::Tensor gemm(const Here& h, const at::Tensor& xq, const at::Tensor& sx, const
   if (code < 0 || !is_codes(h, xq) || !is_scale(h, sx) || !is_scale(h, sw) || !is_weight(h, w, xq.size(1))) return {};
   const int64_t M = xq.size(0), K = xq.size(1), N = w.size(0);
   const bool res = residual.defined();
-  if (res && M > kDecodeRows) return {};       // added separately there
   if (res && (!plain(h, residual) || residual.dim() != 2 || residual.size(0) != M || residual.size(1) != N ||
               residual.scalar_type() != out || residual.stride(1) != 1 || recorded(residual)))
     return {};
@@ -396,7 +393,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !aligned(w.data_ptr(), 16))
     Py_RETURN_NONE;
   if (res) {
-    if (x.numel() / K > kDecodeRows || !plain(h, residual) || recorded(residual) || residual.numel() != x.numel() / K * N) Py_RETURN_NONE;
+    if (!plain(h, residual) || recorded(residual) || residual.numel() != x.numel() / K * N) Py_RETURN_NONE;
     if (residual.dim() != 2) {
       if (!residual.is_contiguous()) Py_RETURN_NONE;
       residual = residual.view({-1, N});
@@ -482,7 +479,7 @@ PyObject* project(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const void* dp = nullptr;
   at::Tensor d2;
   if (mixed) {
-    if (M > kDecodeRows || !dense.defined() || !plain(h, dense) || dense.scalar_type() != out || code == BQ_DTYPE_F32 ||
+    if (!dense.defined() || !plain(h, dense) || dense.scalar_type() != out || code == BQ_DTYPE_F32 ||
         !dense.is_contiguous() || dense.numel() != M * K || !aligned(dense.data_ptr(), 16) || (M > 256 && recorded(dense)))
       Py_RETURN_NONE;
     dp = dense.data_ptr();
@@ -529,7 +526,7 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   // what the down projection would refuse is refused before anything runs
   if (I % 64 || N % 16 || !aligned(wd.data_ptr(), 16)) Py_RETURN_NONE;
   if (residual.defined() &&
-      (M > kDecodeRows || !plain(h, residual) || residual.dim() != 2 || residual.size(0) != M || residual.size(1) != N ||
+      (!plain(h, residual) || residual.dim() != 2 || residual.size(0) != M || residual.size(1) != N ||
        residual.scalar_type() != out || residual.stride(1) != 1 || residual.stride(0) < N || residual.stride(0) % 4 ||
        !aligned(residual.data_ptr(), out == at::kFloat ? 16 : 8) || recorded(residual)))
     Py_RETURN_NONE;

@@ -110,6 +110,14 @@ def _transformed() -> bool:
             or forward_ad._current_level >= 0 or torch.jit.is_tracing())
 
 
+def _recorded(*tensors: torch.Tensor) -> bool:
+    """Would torch follow an operation on these (gradients, a subclass, a transform, autocast), or read
+    them other than as the memory says (a negated view)?  Then it stays a torch operation."""
+    return ((torch.is_grad_enabled() and any(t.requires_grad for t in tensors)) or torch.is_autocast_enabled("cuda")
+            or any(type(t) not in (torch.Tensor, torch.nn.Parameter) or t.is_neg() for t in tensors)
+            or _transformed())
+
+
 def _quantize_weight_fused(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor] | None:
     """Codes and scale of a weight from two launches of the ring kernel (`quant_act.cu`): every CTA's
     max |w|, then the cast under their maximum.  Scale and codes are the bits of the torch
@@ -804,7 +812,7 @@ def fp8_matmul(xq: torch.Tensor, sx: torch.Tensor, w: FP8Weight,
 
     `(xq * sx) @ (w.data * w.scale)^T`, fp32 accumulation, `out_dtype` result.  With `residual`
     (`[M, N]`, `out_dtype`) the result is `residual + that`, the add running in the GEMM's
-    epilogue with the two roundings of the separate kernels (decode sizes; larger M adds after).
+    epilogue with the two roundings of the separate kernels.
     """
     if _NATIVE is not None and isinstance(w, FP8Weight):
         y = _NATIVE.matmul(xq, sx, w.data, w.scale, out_dtype, residual)
@@ -819,7 +827,8 @@ def fp8_matmul(xq: torch.Tensor, sx: torch.Tensor, w: FP8Weight,
         raise ValueError(f"residual must be a [{M}, {N}] {out_dtype} CUDA tensor")
     code = _DTYPE_CODE.get(out_dtype)
     if (M == 0 or code is None or residual.stride(1) != 1 or w.data.shape[1] != K
-            or not w.data.is_contiguous()):
+            or not w.data.is_contiguous()
+            or (M > 256 and (residual.device != xq.device or _recorded(residual)))):
         return residual + fp8_matmul_grouped(xq, sx, (w,), out_dtype=out_dtype)[0]
     lib = _require_lib()
     if not xq.is_contiguous():
@@ -1006,8 +1015,10 @@ def _project_mixed(xq, sx, dense: torch.Tensor, weights, lead, K):
     """One launch for FP8 and 16-bit weights together, or None when the set does not qualify."""
     M = xq.shape[0]
     dt = dense.dtype
-    if (not _DENSE_SEGMENTS or M == 0 or M > 256 or dt not in (torch.bfloat16, torch.float16)
+    if (not _DENSE_SEGMENTS or M == 0 or dt not in (torch.bfloat16, torch.float16)
             or len(weights) > _lib.BQ_MAX_SEGMENTS):
+        return None
+    if M > 256 and _recorded(dense, *(w for w in weights if not isinstance(w, FP8Weight))):
         return None
     d2 = dense.reshape(-1, K)
     if not d2.is_contiguous() or d2.data_ptr() % 16:
@@ -1017,7 +1028,8 @@ def _project_mixed(xq, sx, dense: torch.Tensor, weights, lead, K):
             if w.data.shape[1] != K or not w.data.is_contiguous():
                 return None
         elif (w.dtype != dt or w.dim() != 2 or w.shape[1] != K or w.shape[0] % 16
-              or not w.is_contiguous() or w.data_ptr() % 16 or not w.is_cuda):
+              or not w.is_contiguous() or w.data_ptr() % 16 or not w.is_cuda
+              or (M > 256 and (w.shape[0] > 256 or w.device != dense.device))):
             return None
     lib = _require_lib()
     n = len(weights)
@@ -1057,8 +1069,8 @@ def project(x: torch.Tensor, *weights: torch.Tensor | FP8Weight) -> list[torch.T
 
     The activation is quantized once (braid/model/quant.py:260-286) and all FP8 weights of
     the call go through one grouped launch.  Weights left in bf16 (GDN's a/b gates beside its
-    FP8 qkv/z) ride in the same launch at decode sizes, as 16-bit tensor-core segments over
-    the unquantized activation; where that does not apply (larger M, fp32 engines,
+    FP8 qkv/z) ride in the same launch, as 16-bit tensor-core segments over
+    the unquantized activation; where that does not apply (more than 256 columns at M > 256, fp32 engines,
     `set_dense_segments(False)`) they take `F.linear`, as in the reference.
     """
     pre = x if isinstance(x, QuantizedActivation) else None

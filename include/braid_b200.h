@@ -316,8 +316,7 @@ int bq_gemm_w8a8(const void* xq, const void* wq, const float* sx, const float* s
  * bq_gemm_w8a8 with the residual add of the decoder layer in the epilogue:
  *   y = T(float(T(acc * sx * sw)) + float(residual))
  * i.e. the GEMM's own rounding to the output type T followed by the add's rounding, which is
- * what the reference's separate kernels produce.  Decode regime only (M <= 256): larger M
- * returns BQ_ERR_UNSUPPORTED and the caller adds separately.
+ * what the reference's separate kernels produce.
  *
  * Replaces: `x = x + h` after the mixer's output projection and `x + self.mlp(h)`
  * (braid/model/layer.py:57,60), fused into `linear(core, out_proj)` (braid/model/gdn.py:387),
@@ -538,7 +537,7 @@ int bq_gemm_w8a8_grouped(const void* xq, const float* sx, int64_t M, int64_t K, 
                          void* ws, size_t ws_bytes, void* stream);
 
 /*
- * `project` with a mixed set of weights in ONE launch (decode regime, M <= 256): segments
+ * `project` with a mixed set of weights in ONE launch: segments
  * with kind[i] == 0 are e4m3 weights multiplied with the quantized activation exactly as in
  * bq_gemm_w8a8_grouped; segments with kind[i] != 0 are weights the reference leaves
  * unquantized (bf16 / fp16, [N_i, K] row-major) and are multiplied with the UNQUANTIZED
@@ -553,7 +552,8 @@ int bq_gemm_w8a8_grouped(const void* xq, const float* sx, int64_t M, int64_t K, 
  *   x_dense      device, [M, K] of dense_dtype (BQ_DTYPE_BF16 or BQ_DTYPE_F16), contiguous,
  *                16-byte aligned; out_dtype must equal dense_dtype when a 16-bit segment exists
  *   w[i]         device, e4m3 codes (kind 0) or 16-bit values (kind != 0), contiguous [N_i, K]
- * Returns BQ_ERR_UNSUPPORTED for M > 256: call bq_gemm_w8a8_grouped and a dense GEMM instead.
+ * Returns BQ_ERR_UNSUPPORTED for M > 256 with a 16-bit segment of more than 256 rows: call
+ * bq_gemm_w8a8_grouped and a dense GEMM instead.
  */
 int bq_project_mixed(const void* xq, const float* sx, const void* x_dense, int dense_dtype, int64_t M,
                      int64_t K, int n_seg, const void* const* w, const float* const* sw,

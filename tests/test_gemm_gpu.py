@@ -370,6 +370,33 @@ def test_gdn_input_projection_as_one_launch(Q, dt, M):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("M,K,widths", [(257, 4096, (32, 32)), (300, 1040, (16, 256)), (513, 512, (240, 80)),
+                                        (1500, 2048, (48,))])
+def test_prefill_mixed_projection_as_one_launch(Q, dt, M, K, widths):
+    """M > 256: 16-bit weights of up to 256 rows are tiles of the one launch.  FP8 members bit-equal to
+    their own launch, 16-bit ones within half a unit of the type of the exact product (fp32 sums over K
+    add far less); wider ones and those that record gradients go through `F.linear`."""
+    x = randn_cpu((M, K), seed=M, dtype=dt).cuda()
+    w = Q.quantize_weight(randn_cpu((2 * K, K), seed=1, scale=0.02).cuda())
+    dense = [randn_cpu((n, K), seed=2 + n, dtype=dt, scale=0.02).cuda() for n in widths]
+    n0 = Q.launch_count()
+    ys = Q.project(x, w, *dense)
+    assert Q.launch_count() - n0 == 2 and Q.last_gemm_launch()["kernel"] == "pair"
+    xq, sx = Q.quantize_act(x)
+    assert torch.equal(ys[0], Q.fp8_matmul(xq, sx, w, out_dtype=dt))
+    for y, d in zip(ys[1:], dense):
+        assert y.dtype is dt and y.shape == (M, d.shape[0])
+        assert max_rel(y, F.linear(x.double(), d.double())) <= (2 ** -8 if dt is torch.bfloat16 else 2 ** -10)
+    assert all(torch.equal(p, q) for p, q in zip(ys, Q.project(x, w, *dense)))
+    wide = randn_cpu((272, K), seed=5, dtype=dt, scale=0.02).cuda()
+    assert torch.equal(Q.project(x, w, wide)[1], F.linear(x, wide))
+    d = dense[0].clone().requires_grad_()
+    got = Q.project(x, w, d)[1]
+    assert got.requires_grad and torch.equal(got, F.linear(x, d))
+    assert Q.device_status() == 0
+
+
 def test_leading_dims_and_dispatch(Q):
     x = randn_cpu((2, 3, 256), seed=19).cuda()
     w = randn_cpu((512, 256), seed=20, scale=0.02).cuda()
@@ -497,6 +524,22 @@ def test_residual_epilogue_equals_gemm_then_add(Q, dt, M, N, K):
     got = Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=res)
     assert got.dtype is dt and got.shape == (M, N)
     assert torch.equal(got, want), f"{int((got != want).sum())} of {got.numel()} differ"
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("M,N,K", [(257, 4096, 512), (300, 272, 256), (413, 1040, 1040), (512, 16, 16), (1000, 4112, 2048)])
+def test_prefill_residual_epilogue_over_row_pitches(Q, dt, M, N, K):
+    """M > 256: ragged rows and columns, residual rows that start on 16 bytes or only on 8 (16-bit types),
+    one that is a column block of a wider buffer; bit-equal to the separate add.  What records gradients
+    stays a torch addition."""
+    _, _, xq, sx, fw = _operands(Q, M, N, K, seed=M + N)
+    y = Q.fp8_matmul(xq, sx, fw, out_dtype=dt)
+    for off, pitch in ((0, N), (4, N + 20), (8, N + 16), (3, N + 8)):
+        res = randn_cpu((M, pitch), seed=off, dtype=dt, scale=0.5).cuda()[:, off:off + N]
+        assert torch.equal(Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=res), res + y)
+    res = randn_cpu((M, N), seed=9, dtype=dt).cuda().requires_grad_()
+    assert Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=res).requires_grad
+    assert Q.device_status() == 0
 
 
 def test_residual_strided_scoped_and_through_the_sublayers(Q):
