@@ -73,7 +73,8 @@ struct Segment {
   int split;           // stream kernel: K slices of this weight (1, 2, 4 or 8)
   int split_forced;    // stream kernel: non-zero = use this split instead of the shape rule
   int cluster_begin;   // stream kernel: index of the segment's first cluster
-  int un;              // wide kernel: weight rows per unit (gate/up form: output columns per unit)
+  int un;              // wide kernel: weight rows per unit (gate/up form: output columns per unit);
+                       // pair kernel, plain form: output columns per tile
   int unit_begin;      // wide kernel: index of the segment's first unit
   int wide;            // wide kernel: output (and residual) rows are 16-byte aligned
 };
@@ -148,7 +149,6 @@ struct GemmParams {
   int b_stages;        // stream kernel: depth of the activation ring
   int out_dtype;
   int m_tiles;         // tile kernel: ceil(M / 128)
-  int pair_n;          // pair kernel, plain form: output columns per tile, 256 or 128
   int total_tiles;     // tile kernel
   unsigned int* status;
   ArgmaxOut argmax;
@@ -1056,9 +1056,9 @@ __device__ __forceinline__ void pair_epilogue_rows(const GemmParams& p, const Se
                                                    float& mx) {
   constexpr int kCols = 128 / ES;              // output columns per 128-byte piece
   constexpr int kPieces = ES == 4 ? 4 : 2;     // 16-byte pieces per 16 accumulator columns
-  const int out_cols = SILU ? kPairTile / 2 : (seg.dense ? seg.un : p.pair_n);
+  const int out_cols = SILU ? kPairTile / 2 : seg.un;
   const int half_cols = (out_cols / 2 + kCols - 1) / kCols * kCols;   // whole pieces: 16-bit weights may be narrow
-  const int c_end = (col_half + 1) * half_cols;
+  const int c_end = (col_half + 1) * half_cols < out_cols ? (col_half + 1) * half_cols : out_cols;   // of this tile
   for (int c = col_half * half_cols; c < c_end; c += kCols) {
     // pieces beyond this weight's rows are never stored (warp-uniform)
     if ((n0 + c) >= seg.n) break;
@@ -1188,10 +1188,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int m_tiles = (p.M + kPairTile - 1) / kPairTile;
   const bool silu = EPI == kAny ? p.pair.on != 0 : EPI == kGateUp;                       // gate/up tiles, h = silu(gate) * up out
-  // output columns per tile: 128 of h in the SiLU form; 256 in the plain form, or 128 for a weight
-  // so narrow that 256-wide tiles would leave CTA pairs without work (same sums, more tiles)
-  const int n_step = silu ? kPairTile / 2 : p.pair_n;
-  const int b_rows = silu ? kRowTile : p.pair_n / 2;       // weight rows this CTA loads per K block
+  // output columns per tile: 128 of h in the SiLU form, in the plain form what the host chose for the
+  // segment (the sums are the same either way)
+  auto tile_cols = [&](const Segment& g) { return silu ? kPairTile / 2 : g.un; };
   float* const s_amax = reinterpret_cast<float*>(base_ptr + kPairStages * kPairStageBytes + 512);
 
   if (threadIdx.x == 0) {
@@ -1229,11 +1228,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         const int local = t - p.seg[sg].tile_begin;
         const bool dense = EPI == kMixed && p.seg[sg].dense != 0;
         int m_idx, n_idx;
-        pair_tile_coords(local, m_tiles, dense ? 1 : (p.seg[sg].n + n_step - 1) / n_step, m_idx, n_idx);
+        const int n_step = tile_cols(p.seg[sg]);
+        pair_tile_coords(local, m_tiles, (p.seg[sg].n + n_step - 1) / n_step, m_idx, n_idx);
         const int m0 = m_idx * kPairTile + rank * kRowTile;
-        // plain: this CTA's half of the tile's 256 weight rows; SiLU form: the leader loads 128
+        // plain: this CTA's half of the tile's weight rows; SiLU form: the leader loads 128
         // gate rows, its peer the 128 up rows of the same output columns
-        const int rows = dense ? p.seg[sg].un / 2 : b_rows;
+        const int rows = silu ? kRowTile : n_step / 2;
         const int n0 = silu ? n_idx * kRowTile : n_idx * n_step + rank * rows;
         const CUtensorMap* const w_map = silu ? &tm_w.w[rank] : &tm_w.w[sg];
         const CUtensorMap* const x_map = dense ? &tm_xd : &tm_x;
@@ -1251,8 +1251,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     __syncwarp();
   } else if (warp == 1) {
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc = (silu || p.pair_n == kPairTile) ? idesc_e4m3(kPairTile, kPairTile)
-                                                             : idesc_e4m3(kPairTile, kPairTile / 2);
       int it = 0, tile_iter = 0;
       bool ok = true;
       for (int t = pair; t < p.total_tiles && ok; t += n_pairs, ++tile_iter) {
@@ -1262,7 +1260,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         const uint32_t tmem_d = tmem_base + b * kPairTile;
         const Segment& seg = p.seg[find_segment(p, t)];
         const bool dense = EPI == kMixed && seg.dense != 0;
-        const uint32_t idesc_d = dense ? idesc_f16(kPairTile, seg.un, p.dense_fmt) : 0u;
+        const uint32_t idesc = dense ? idesc_f16(kPairTile, seg.un, p.dense_fmt)
+                                     : idesc_e4m3(kPairTile, silu ? kPairTile : seg.un);
         const int blocks = dense ? p.k_blocks_dense : p.k_blocks;
         for (int kb = 0; kb < blocks; ++kb, ++it) {
           const int s = it % kPairStages, use = it / kPairStages;
@@ -1272,7 +1271,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           const uint64_t db = smem_desc_sw128(b_tile(s));
 #pragma unroll
           for (int j = 0; j < kBK / kUmmaK; ++j) {
-            if (dense) mma_f16_pair(tmem_d, da + 2u * j, db + 2u * j, idesc_d, (kb | j) != 0 ? 1u : 0u);
+            if (dense) mma_f16_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
             else mma_f8_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
           }
           // the stage is free in BOTH CTAs once these MMAs retire
@@ -1303,7 +1302,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       const Segment seg = p.seg[sg];
       const int local = t - seg.tile_begin;
       int m_idx, n_idx;
-      pair_tile_coords(local, m_tiles, seg.dense ? 1 : (seg.n + n_step - 1) / n_step, m_idx, n_idx);
+      const int n_step = tile_cols(seg);
+      pair_tile_coords(local, m_tiles, (seg.n + n_step - 1) / n_step, m_idx, n_idx);
       const int m0 = m_idx * kPairTile + rank * kRowTile;
       const int n0 = n_idx * n_step;
       if (!mbar_wait(acc_full(b), use_b & 1)) { ok = false; break; }
@@ -1509,7 +1509,7 @@ int device_sms() {
 long long g_opt_split = 0, g_opt_stages = 0, g_opt_stream_max_m = 256, g_opt_cta_target = 160;
 long long g_opt_wide = -1;   // decode: CTA-pair kernel (-1 by batch, 0 never, 1 always)
 long long g_opt_push_tma = 1;   // prefill push epilogue: bulk tensor stores (0: 16-byte plain stores)
-long long g_opt_pair_narrow = -1;   // prefill: 128-column tiles for a lone narrow weight (-1 auto, 0 never, 1 always)
+long long g_opt_pair_narrow = -1;   // prefill: columns of a plain launch's tiles (-1 by rule, 0: 256, 1: 128, else so many)
 long long g_opt_pdl = 1;   // programmatic dependent launch on by default
 long long g_opt_b_stages = 0;   // activation ring depth: 0 = heuristic, -1 = as deep as the weight ring
 long long g_opt_smem_cap = 0;   // 0 = no cap on pipeline bytes per CTA
@@ -1946,7 +1946,7 @@ int launch_pair(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
   const int epi = epilogue_of(p, true);
   if (p.push.n > 0) p.push.expected = (unsigned)(2 * pairs);   // every CTA has a tile and stores
   g_last_launch[0] = 2; g_last_launch[1] = 2 * pairs; g_last_launch[2] = 2;
-  g_last_launch[3] = kPairStages; g_last_launch[4] = smem; g_last_launch[5] = p.pair_n;
+  g_last_launch[3] = kPairStages; g_last_launch[4] = smem; g_last_launch[5] = p.pair.on ? kPairTile : p.seg[0].un;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
@@ -1978,7 +1978,11 @@ int bq::gemm_set_option(const char* key, long long value) {
   if (strcmp(key, "decode_b_stages") == 0) { g_opt_b_stages = value; return kOk; }
   if (strcmp(key, "gemm_pdl") == 0) { g_opt_pdl = value ? 1 : 0; return kOk; }
   if (strcmp(key, "push_tma") == 0) { g_opt_push_tma = value ? 1 : 0; return kOk; }
-  if (strcmp(key, "pair_narrow") == 0) { g_opt_pair_narrow = value < 0 ? -1 : (value ? 1 : 0); return kOk; }
+  if (strcmp(key, "pair_narrow") == 0) {
+    if (value > 1 && (value % 64 || value > kPairTile)) return kErrBadArg;
+    g_opt_pair_narrow = value < 0 ? -1 : value;
+    return kOk;
+  }
   if (strcmp(key, "decode_smem_cap") == 0) { g_opt_smem_cap = value; return kOk; }
   if (strcmp(key, "decode_wide") == 0) { g_opt_wide = value < 0 ? -1 : (value ? 1 : 0); return kOk; }
   if (strcmp(key, "decode_cta_target") == 0) {
@@ -2104,6 +2108,71 @@ int run_wide(GemmParams p, const void* xq, int64_t K, const void* const* wq, con
   return launch_wide(tm_x, tm_xd, maps, p, sh, stream);
 }
 
+// Tiles of a plain prefill launch: 256, 192 or 128 columns (the sums are the same, tile by tile; whole
+// 128-byte pieces of 16-bit output), and the last columns of its widest weight as 128-column tiles that
+// are visited last, where that evens out the last round.  A launch takes as long as its busiest CTA pair
+// (tiles are dealt out in turn), a tile its columns plus a part that does not shrink with them: the
+// activation rows' loads and MMA passes, the epilogue.  Measured, us with tiles of 256 / 192 / 128 columns:
+// 4096 x 12288 at 300 rows 45.0 / 37.9 / 31.6, at 600 45.1 / 38.2 / 56.5, at 1024 45.6 / 67.9 / 56.8, at 1500
+// 81.7 / 68.9 / 81.9, at 3000 126.5 / 138.2 / 182.8: one round of n columns costs n + 128, within the launch's
+// own 3 us.  64 columns never won by more than 2 %.  Split: q, k and v of 8192 + 1024 + 1024 columns at 1500 rows
+// 58.0 -> 54.8, 2560 x 7680 at 4096 rows 76.8 -> 69.7.
+struct TilePlan {
+  int cols;            // columns of a tile
+  int split;           // weight whose end becomes a segment of 128-column tiles, -1: none
+  int64_t split_at;    // its first column there
+};
+constexpr int kTileFixedCols = 128;
+
+TilePlan plan_tiles(const int64_t* N, const int* dense, int n_seg, int m_tiles, int k_blocks, bool may_split) {
+  TilePlan best{kPairTile, -1, 0};
+  if (g_opt_pair_narrow >= 0) {
+    best.cols = g_opt_pair_narrow == 0 ? kPairTile : (g_opt_pair_narrow == 1 ? kPairTile / 2 : (int)g_opt_pair_narrow);
+    return best;
+  }
+  const long long pairs = device_sms() / 2 > 0 ? device_sms() / 2 : 1;
+  int widest = -1;
+  for (int i = 0; i < n_seg; ++i)
+    if ((dense == nullptr || dense[i] == 0) && (widest < 0 || N[i] > N[widest])) widest = i;
+  if (widest < 0) return best;
+  // cost of `wide` tiles of n columns, then `small` ones of 128, dealt out in turn
+  auto cost_of = [&](long long wide, int n, long long small) {
+    const long long cw = n + kTileFixedCols, cs = kPairTile / 2 + kTileFixedCols;
+    const long long full = wide / pairs, r = wide % pairs;
+    const long long first = pairs - r;                   // small tiles that level the pairs out
+    if (small <= first) {
+      const long long a = (full + (r > 0 ? 1 : 0)) * cw, b = full * cw + (small > 0 ? cs : 0);
+      return a > b ? a : b;
+    }
+    const long long extra = small - first;
+    const long long a = r > 0 ? (full + 1) * cw + (extra + pairs - 1) / pairs * cs : 0;
+    const long long b = full * cw + cs + (extra > r ? (extra - r + pairs - 1) / pairs * cs : 0);
+    return a > b ? a : b;
+  };
+  auto tiles_of = [&](int n, int64_t less) {
+    long long tiles = 0;
+    for (int i = 0; i < n_seg; ++i)
+      if (dense == nullptr || dense[i] == 0) tiles += ((i == widest ? N[i] - less : N[i]) + n - 1) / n * m_tiles;
+    return tiles;
+  };
+  long long best_cost = 0;
+  for (int n = kPairTile; n >= 128; n -= 64) {
+    if (n == 192 && k_blocks < 8) continue;              // so short a tile is mostly the fixed part
+    const long long cost = cost_of(tiles_of(n, 0), n, 0);
+    if (best_cost == 0 || cost < best_cost) { best = TilePlan{n, -1, 0}; best_cost = cost; }
+  }
+  if (!may_split || n_seg == BQ_MAX_SEGMENTS || k_blocks < 8) return best;
+  const int64_t columns = (N[widest] + kPairTile - 1) / kPairTile;
+  for (int j = 1; j <= 6 && j < columns; ++j) {
+    const int64_t at = (columns - j) * kPairTile, tail = N[widest] - at;
+    const long long small = (tail + kPairTile / 2 - 1) / (kPairTile / 2) * m_tiles;
+    const long long cost = cost_of(tiles_of(kPairTile, tail), kPairTile, small);
+    // a split has to give something: one tile's fixed part at least
+    if (cost + kTileFixedCols < best_cost) { best = TilePlan{kPairTile, widest, at}; best_cost = cost; }
+  }
+  return best;
+}
+
 int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg,
                 const void* const* wq, const float* const* sw, void* const* y, const int64_t* N,
                 const int64_t* ldy, int out_dtype, void* ws, size_t ws_bytes, void* stream_v,
@@ -2196,19 +2265,38 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   }
   const bool pair_path = !stream_path;
   p.m_tiles = pair_path ? (int)((M + kPairTile - 1) / kPairTile) : (int)((M + kRowTile - 1) / kRowTile);
-  // plain prefill form of ONE narrow weight: 128-column tiles when all of them still run at once,
-  // i.e. when 256-column ones would leave half of the CTA pairs without a tile (the sums are the
-  // same, tile by tile; a 128-column tile takes 0.6-0.75 of a 256-column one, so a second round
-  // of them costs more than the idle pairs do)
-  p.pair_n = kPairTile;
-  if (pair_path && pair == nullptr && n_seg == 1) {
-    const long long wide_tiles = ((N[0] + kPairTile - 1) / kPairTile) * p.m_tiles;
-    const long long pairs = device_sms() / 2;
-    const bool narrow = g_opt_pair_narrow > 0 || (g_opt_pair_narrow < 0 && wide_tiles * 2 <= pairs);
-    if (narrow) p.pair_n = kPairTile / 2;
+  // plain prefill form: the tiles' columns, and perhaps the end of a weight as a segment of its own
+  const void* part_w[BQ_MAX_SEGMENTS];
+  const float* part_sw[BQ_MAX_SEGMENTS];
+  void* part_y[BQ_MAX_SEGMENTS];
+  const void* part_res[BQ_MAX_SEGMENTS];
+  int64_t part_n[BQ_MAX_SEGMENTS], part_ld[BQ_MAX_SEGMENTS], part_ld_res[BQ_MAX_SEGMENTS];
+  int part_kind[BQ_MAX_SEGMENTS];
+  DenseArgs part_dn;
+  TilePlan plan{kPairTile, -1, 0};
+  if (pair_path && pair == nullptr) {
+    plan = plan_tiles(N, dn != nullptr ? dn->kind : nullptr, n_seg, p.m_tiles, p.k_blocks, push == nullptr);
+    if (plan.split >= 0) {
+      const size_t es = out_dtype == BQ_DTYPE_F32 ? 4 : 2;
+      for (int i = 0; i <= n_seg; ++i) {
+        const int from = i < n_seg ? i : plan.split;
+        const int64_t at = i < n_seg ? 0 : plan.split_at;
+        part_w[i] = static_cast<const uint8_t*>(wq[from]) + at * K;
+        part_sw[i] = sw[from];
+        part_y[i] = static_cast<uint8_t*>(y[from]) + at * es;
+        part_n[i] = i == plan.split ? plan.split_at : N[from] - at;
+        part_ld[i] = ldy[from];
+        part_res[i] = res != nullptr && res[from] != nullptr ? static_cast<const uint8_t*>(res[from]) + at * es : nullptr;
+        part_ld_res[i] = res != nullptr ? ld_res[from] : 0;
+        part_kind[i] = i < n_seg && dn != nullptr ? dn->kind[i] : 0;
+      }
+      wq = part_w; sw = part_sw; y = part_y; N = part_n; ldy = part_ld;
+      if (res != nullptr) { res = part_res; ld_res = part_ld_res; }
+      if (dn != nullptr) { part_dn = DenseArgs{dn->x, dn->dtype, part_kind}; dn = &part_dn; }
+      p.n_seg = ++n_seg;
+    }
   }
-  const int w_box_rows = (pair_path && pair == nullptr) ? p.pair_n / 2 : kRowTile;
-  const int tile_n = pair_path ? ((pair && pair->prefill) ? kPairTile / 2 : p.pair_n) : kRowTile;
+  const bool plain_pair = pair_path && pair == nullptr;
   OutMaps ymaps;
   memset(&ymaps, 0, sizeof(ymaps));
   int tiles = 0;
@@ -2223,12 +2311,15 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     p.seg[i].n = (int)N[i];
     p.seg[i].dense = (dn != nullptr && dn->kind[i] != 0) ? 1 : 0;
     p.seg[i].tile_begin = tiles;
-    if (pair_path && p.seg[i].dense) p.seg[i].un = (int)((N[i] + 31) / 32 * 32);   // MMA N granularity of a pair
+    if (plain_pair)     // a 16-bit weight is one tile column, in the MMA N granularity of a pair
+      p.seg[i].un = p.seg[i].dense ? (int)((N[i] + 31) / 32 * 32)
+                                   : (plan.split >= 0 && i == n_seg - 1 ? kPairTile / 2 : plan.cols);
+    const int tile_n = plain_pair ? p.seg[i].un : (pair_path ? kPairTile / 2 : kRowTile);
     if (pair_path && res != nullptr && res[i] != nullptr) {
       const size_t es = out_dtype == BQ_DTYPE_F32 ? 4 : 2;
       p.seg[i].wide = aligned_to(res[i], 16) && (ld_res[i] * es) % 16 == 0 ? 1 : 0;
     }
-    const long long nt = pair_path && p.seg[i].dense ? 1 : (N[i] + tile_n - 1) / tile_n;
+    const long long nt = (N[i] + tile_n - 1) / tile_n;
     const long long add = stream_path ? nt : nt * p.m_tiles;
     if (tiles + add > 0x3fffffffLL) return kErrTooLarge;
     tiles += (int)add;
@@ -2255,7 +2346,7 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
       if (int rc = make_map(&maps.w[1], pair->wq_up, N[0] / 2, K, kRowTile / 2)) return rc;
     } else {
       // a 16-bit weight is described by its bytes: [N, 2K]
-      const int box_rows = pair_path && p.seg[i].dense ? p.seg[i].un / 2 : w_box_rows;
+      const int box_rows = plain_pair ? p.seg[i].un / 2 : kRowTile;
       if (int rc = make_map(&maps.w[i], wq[i], N[i], p.seg[i].dense ? 2 * K : K, box_rows)) return rc;
     }
   }

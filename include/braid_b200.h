@@ -581,8 +581,8 @@ int bq_read_device_status(void* ws, void* stream, int* status_out);
  * bq_set_option("quant_block" | "quant_held", v) quantizer launch shape overrides
  * bq_set_option("quant_ring", 0/1)      plain quantizer at prefill sizes through the shared-memory ring (default 1)
  * bq_set_option("push_tma", 0/1)        prefill push epilogue by bulk tensor stores (default 1) or 16-byte plain stores
- * bq_set_option("pair_narrow", -1/0/1) prefill kernel: 128-column tiles for a lone narrow weight (-1 = when 256-column
- *                                       tiles would leave half of the CTA pairs idle; same results either way)
+ * bq_set_option("pair_narrow", v)       prefill kernel: columns of a plain launch's tiles, -1 = by what evens out the
+ *                                       rounds, 0 = 256, 1 = 128, else 64, 128, 192 or 256; same results either way
  * Returns BQ_ERR_BAD_ARG for an unknown key.
  */
 int bq_set_option(const char* key, int64_t value);

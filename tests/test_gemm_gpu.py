@@ -166,6 +166,50 @@ def test_prefill_tiles_of_128_columns_give_the_bits_of_256(Q, M, N, K, dt):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K,dt", [(1500, 4096, 1024, torch.bfloat16), (300, 400, 2048, torch.float16),
+                                      (257, 192, 1024, torch.float32), (768, 4096, 4096, torch.bfloat16)])
+def test_prefill_tiles_of_192_columns_give_the_bits_of_256(Q, M, N, K, dt):
+    """Tiles between the two widths: every output element is the same sum in the same order, tails in N
+    and M included, alone and grouped."""
+    _, _, xq, sx, fw = _operands(Q, M, N, K, seed=M + N)
+    try:
+        Q.set_option("pair_narrow", 0)
+        wide = Q.fp8_matmul(xq, sx, fw, out_dtype=dt)
+        Q.set_option("pair_narrow", 192)
+        got = Q.fp8_matmul(xq, sx, fw, out_dtype=dt)
+        assert Q.last_gemm_launch()["mma_n"] == 192
+        pair = Q.fp8_matmul_grouped(xq, sx, (fw, fw), out_dtype=dt)
+    finally:
+        Q.set_option("pair_narrow", -1)
+    assert torch.equal(wide, got) and all(torch.equal(wide, p) for p in pair)
+    assert torch.equal(wide, Q.fp8_matmul(xq, sx, fw, out_dtype=dt))
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("M,Ns", [(4864, (1024,)), (4860, (1040,)), (1500, (8192, 1024, 16))])
+def test_prefill_weights_whose_end_is_tiled_apart_give_the_bits_of_256(Q, dt, M, Ns):
+    """Sizes whose last round is evened out with the end of the widest weight in 128-column tiles: outputs,
+    with and without a residual, equal those of 256-column tiles throughout."""
+    K = 1024
+    x = randn_cpu((M, K), seed=M, dtype=dt).cuda()
+    xq, sx = Q.quantize_act(x)
+    ws = [Q.quantize_weight(randn_cpu((n, K), seed=n, scale=0.02).cuda()) for n in Ns]
+    res = randn_cpu((M, Ns[0]), seed=1, dtype=dt).cuda()
+
+    def run():
+        return [*Q.fp8_matmul_grouped(xq, sx, ws, out_dtype=dt), Q.fp8_matmul(xq, sx, ws[0], out_dtype=dt, residual=res)]
+
+    try:
+        Q.set_option("pair_narrow", 0)
+        want = run()
+    finally:
+        Q.set_option("pair_narrow", -1)
+    for a, b in zip(run(), want):
+        assert torch.equal(a, b)
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
 @pytest.mark.parametrize("M,V,K", [(1, 248320, 4096), (128, 248320, 4096), (37, 1040, 272),
                                    (4, 4096, 256), (256, 16, 16)])
