@@ -53,7 +53,8 @@ struct NormParams {
   int phase_seq;
 };
 
-constexpr int kRehearseRows = 32;   // see rmsnorm_quant_kernel; one CTA per row
+constexpr int kWideRows = 256;      // batches whose rows get four times the threads
+constexpr int kRehearseRows = 128;   // see rmsnorm_quant_kernel; one CTA per row
 
 template <typename T> struct Vec4 { T v[kVec]; };
 
@@ -101,79 +102,112 @@ __device__ __forceinline__ float warp_tree_sum(float s) {
 // ---------------------------------------------------------------------------------------------
 // plain RMSNorm -> quantize.  One CTA of 128 threads per row; VPT = vectors held per thread.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int VPT>
-__global__ void __launch_bounds__(kNormThreads + 32) rmsnorm_quant_kernel(const NormParams p) {
+template <typename T, int VPT, int G>
+__global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(const NormParams p) {
+  // G groups of 128 threads share a row; a thread holds VG vectors of it
+  static_assert(VPT % G == 0, "whole vectors per thread");
+  constexpr int VG = VPT / G;
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
   __shared__ float s_red_of[2][4];
-  const RehearsingCta<kNormThreads> cta{threadIdx.x < kNormThreads};
+  __shared__ __align__(16) Vec4<T> s_x[G > 1 ? VPT * kNormThreads : 1];
+  const RehearsingCta<G * kNormThreads> cta{threadIdx.x < G * kNormThreads};
   const bool live = cta.live;
   float* const s_red = s_red_of[cta.slot()];
   const int lane = threadIdx.x & 31, warp = cta.warp(), t = warp * 32 + lane;
+  const int group = t / kNormThreads;
+  // vector i of this thread
+  auto vec = [&](int i) { return (t - group * kNormThreads) + (group * VG + i) * kNormThreads; };
   const int row = blockIdx.x;
   const int n_vec = p.cols / kVec;
   const T* xr = reinterpret_cast<const T*>(p.x) + static_cast<long long>(row) * p.ld_x;
   // gamma is a weight, not the previous kernel's output: fetch it before the dependency wait
-  float g[VPT][kVec];
+  float g[VG][kVec];
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = t + i * kNormThreads;
+  for (int i = 0; i < VG; ++i) {
+    const int v = vec(i);
     if (v < n_vec) {
       const float4 f = __ldg(reinterpret_cast<const float4*>(p.gamma) + v);
       g[i][0] = f.x; g[i][1] = f.y; g[i][2] = f.z; g[i][3] = f.w;
     }
   }
   // What bounds this kernel at a decode batch is neither bytes nor arithmetic but one dependent chain
-  // run once from a cold instruction cache (the previous kernel's code was there).  So a fifth
-  // warp rehearses: it runs the same instructions on zeros, without a load, store or exchange, while
-  // the others wait for the previous kernel, and they find the code in the cache.  A warp of its own,
-  // because there may be nothing to wait for (behind a kernel that was not launched with early
-  // starts): a second pass of all warps gave more in
-  // an unbroken chain (hidden 4096, four graphed layers, 1 row: 262 -> 244 us, here 255) but cost 3 us
-  // per launch in a broken one (hidden 2560: 194 -> 203 us, here 193).
-  // Only up to kRehearseRows rows: beyond, the rehearsal competes with the GEMM that is waited for
-  // (344 -> 350 us at 128 rows).
-  // The two-pass build was also 4 % faster at 128 rows (334 us, here 348), where neither form rehearses:
-  // its compiled kernels differ (118 and 80 registers for the two norms; 72 and 56 here).  What in
-  // them makes the difference has not been shown.
-  Vec4<T> x[VPT];
+  // run once.  Two things shorten it.
+  //
+  // The row is shared by G groups of 128 threads instead of one, so that a thread normalises and casts a
+  // quarter of the values; a lone warp per scheduler issues an instruction every few clocks, and the
+  // chain's length is what it has to issue.  Only the sum of squares stays with 128 threads, whose order it
+  // restates; they read the other groups' values from shared memory.  Together with 16 instead of 8 warps in
+  // the gated kernel (four graphed layers of hidden 4096, before -> gated -> both): 1 row 246 -> 238 -> 232 us,
+  // 27 rows 286 -> 281 -> 274, 128 rows 333 -> 323 -> 317; hidden 5120, 64 rows 434 -> 435 -> 421.  32 warps
+  // in the gated kernel gave no more.
+  //
+  // A further warp rehearses: it runs the same instructions on zeros, without a load, store or exchange,
+  // while the others wait for the previous kernel, and they find the code in the instruction cache, where
+  // the previous kernel's code was.  A warp of its own, because there may be nothing to wait for (behind a
+  // kernel that was not launched with early starts).  Only up to kRehearseRows rows: beyond, the
+  // rehearsal competes with the GEMM that is waited for.
+  Vec4<T> x[VG];
   if (live) {
     bq::pdl_wait_prior_grids();
     if (threadIdx.x == 0) BQ_STAMP(p, 2);
   }
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = t + i * kNormThreads;
+  for (int i = 0; i < VG; ++i) {
+    const int v = vec(i);
     if (live && v < n_vec) x[i] = load4(xr + v * kVec);
     else x[i] = Vec4<T>{};
   }
   float s = 0.0f;
+  if constexpr (G == 1) {
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = t + i * kNormThreads;
-    if (v < n_vec) {
+    for (int i = 0; i < VG; ++i) {
+      const int v = vec(i);
+      if (v < n_vec) {
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) {
-        const float f = widen(x[i].v[j]);
-        s = __fmaf_rn(f, f, s);
+        for (int j = 0; j < kVec; ++j) {
+          const float f = widen(x[i].v[j]);
+          s = __fmaf_rn(f, f, s);
+        }
+      }
+    }
+  } else {
+    // the sum's order is that of 128 threads: the first group walks the others' vectors
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < VG; ++i) s_x[vec(i)] = x[i];
+    }
+    cta.sync();
+    if (group == 0) {
+      Vec4<T> all[VPT];
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) all[i] = s_x[t + i * kNormThreads];
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        if (t + i * kNormThreads < n_vec) {
+#pragma unroll
+          for (int j = 0; j < kVec; ++j) {
+            const float f = widen(all[i].v[j]);
+            s = __fmaf_rn(f, f, s);
+          }
+        }
       }
     }
   }
-  s = warp_tree_sum(s);
-  if (lane == 0 && warp >= 2) s_red[warp - 2] = s;
+  if (group == 0) {
+    s = warp_tree_sum(s);
+    if (lane == 0) s_red[warp] = s;
+  }
   cta.sync();
-  if (lane == 0 && warp < 2) s = __fadd_rn(s, s_red[warp]);
-  cta.sync();
-  if (lane == 0 && warp == 1) s_red[0] = s;
-  cta.sync();
-  if (t == 0) s_red[1] = __fdiv_rn(__fadd_rn(s, s_red[0]), static_cast<float>(p.cols));
-  cta.sync();
-  const float rstd = rsqrtf(__fadd_rn(s_red[1], p.eps));
+  // every thread adds the four warps' sums up in the restated order
+  s = __fadd_rn(__fadd_rn(s_red[0], s_red[2]), __fadd_rn(s_red[1], s_red[3]));
+  s = __fdiv_rn(s, static_cast<float>(p.cols));
+  const float rstd = rsqrtf(__fadd_rn(s, p.eps));
 
   float m = 0.0f;
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = t + i * kNormThreads;
+  for (int i = 0; i < VG; ++i) {
+    const int v = vec(i);
     if (v < n_vec) {
 #pragma unroll
       for (int j = 0; j < kVec; ++j) {
@@ -186,8 +220,8 @@ __global__ void __launch_bounds__(kNormThreads + 32) rmsnorm_quant_kernel(const 
   if (live && p.h_out != nullptr) {
     T* hr = reinterpret_cast<T*>(p.h_out) + static_cast<long long>(row) * p.ld_h;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int v = t + i * kNormThreads;
+    for (int i = 0; i < VG; ++i) {
+      const int v = vec(i);
       if (v < n_vec) store4(hr + v * kVec, x[i]);
     }
   }
@@ -198,8 +232,8 @@ __global__ void __launch_bounds__(kNormThreads + 32) rmsnorm_quant_kernel(const 
   if (live && blockIdx.x == 0 && t == 0) p.scale[0] = sc;
   uint8_t* qr = p.q + static_cast<long long>(row) * p.cols;
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = t + i * kNormThreads;
+  for (int i = 0; i < VG; ++i) {
+    const int v = vec(i);
     if (v < n_vec) emit4(x[i], dv, qr + v * kVec, live);
   }
   grid_depart(static_cast<QuantWs*>(p.ws));
@@ -321,12 +355,13 @@ struct GatedParams {
 constexpr int kHeadDim = 128;
 constexpr int kGatedWarps = 8;
 constexpr int kMaxHeadsPerWarp = 8;    // up to 64 heads
+constexpr int kWideGatedRows = 256;    // batches whose CTAs have 16 warps
 
-template <typename T, bool Y_F32, int HPW>
-__global__ void __launch_bounds__(kGatedWarps * 32 + 32) gated_rmsnorm_quant_kernel(const GatedParams p) {
+template <typename T, bool Y_F32, int HPW, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32 + 32) gated_rmsnorm_quant_kernel(const GatedParams p) {
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
-  const RehearsingCta<kGatedWarps * 32> cta{threadIdx.x < kGatedWarps * 32};   // see rmsnorm_quant_kernel
+  const RehearsingCta<WARPS * 32> cta{threadIdx.x < WARPS * 32};   // see rmsnorm_quant_kernel
   const bool live = cta.live;
   const int lane = threadIdx.x & 31, warp = cta.warp();
   const int row = blockIdx.x;
@@ -340,7 +375,7 @@ __global__ void __launch_bounds__(kGatedWarps * 32 + 32) gated_rmsnorm_quant_ker
   }
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
-    const int head = warp + i * kGatedWarps;
+    const int head = warp + i * WARPS;
     core[i] = Vec4<T>{};
     gate[i] = Vec4<T>{};
     if (live && head < p.heads) {
@@ -360,7 +395,7 @@ __global__ void __launch_bounds__(kGatedWarps * 32 + 32) gated_rmsnorm_quant_ker
   float m = 0.0f;
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
-    const int head = warp + i * kGatedWarps;   // warp-uniform
+    const int head = warp + i * WARPS;   // warp-uniform
     if (head < p.heads) {
       float s = 0.0f;
 #pragma unroll
@@ -392,7 +427,7 @@ __global__ void __launch_bounds__(kGatedWarps * 32 + 32) gated_rmsnorm_quant_ker
   uint8_t* qr = p.q + static_cast<long long>(row) * p.heads * kHeadDim;
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
-    const int head = warp + i * kGatedWarps;
+    const int head = warp + i * WARPS;
     if (head < p.heads) emit4(core[i], dv, qr + head * kHeadDim + lane * kVec, live);
   }
   grid_depart(static_cast<QuantWs*>(p.ws));
@@ -432,22 +467,39 @@ int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t str
 template <typename T>
 int launch_rmsnorm(const NormParams& p, cudaStream_t stream) {
   const int per_thread = (p.cols / kVec + kNormThreads - 1) / kNormThreads;
-  if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2>, p.rows, kNormThreads, p, stream);
-  if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4>, p.rows, kNormThreads, p, stream);
-  if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8>, p.rows, kNormThreads, p, stream);
-  if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16>, p.rows, kNormThreads, p, stream);
+  // Decode batches: four times the threads, a quarter of the chain each (see the kernel).  Larger ones need
+  // the CTAs resident at once.
+  if (p.rows <= kWideRows) {
+    if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2, 2>, p.rows, 2 * kNormThreads, p, stream);
+    if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4, 4>, p.rows, 4 * kNormThreads, p, stream);
+    if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 4>, p.rows, 4 * kNormThreads, p, stream);
+    if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 4>, p.rows, 4 * kNormThreads, p, stream);
+  }
+  if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2, 1>, p.rows, kNormThreads, p, stream);
+  if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4, 1>, p.rows, kNormThreads, p, stream);
+  if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 1>, p.rows, kNormThreads, p, stream);
+  if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 1>, p.rows, kNormThreads, p, stream);
   return bq::kErrUnsupported;
 }
 
 template <typename T, bool Y_F32>
 int launch_gated(const GatedParams& p, cudaStream_t stream) {
+  // Decode batches: two heads per warp, 16 warps, so that the chain of a head -- sum, square root,
+  // exponentials, divisions -- is walked at most twice one after the other.  Larger batches need the
+  // CTAs resident at once.
+  if (p.rows <= kWideGatedRows && p.heads > kGatedWarps) {
+    constexpr int kWarps = 2 * kGatedWarps;
+    if (p.heads <= kWarps) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 1, kWarps>, p.rows, kWarps * 32, p, stream);
+    if (p.heads <= 2 * kWarps)
+      return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 2, kWarps>, p.rows, kWarps * 32, p, stream);
+  }
   const int hpw = (p.heads + kGatedWarps - 1) / kGatedWarps;
   const int threads = kGatedWarps * 32;
-  if (hpw <= 1) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 1>, p.rows, threads, p, stream);
-  if (hpw <= 2) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 2>, p.rows, threads, p, stream);
-  if (hpw <= 4) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 4>, p.rows, threads, p, stream);
+  if (hpw <= 1) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 1, kGatedWarps>, p.rows, threads, p, stream);
+  if (hpw <= 2) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 2, kGatedWarps>, p.rows, threads, p, stream);
+  if (hpw <= 4) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 4, kGatedWarps>, p.rows, threads, p, stream);
   if (hpw <= kMaxHeadsPerWarp)
-    return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, kMaxHeadsPerWarp>, p.rows, threads, p, stream);
+    return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, kMaxHeadsPerWarp, kGatedWarps>, p.rows, threads, p, stream);
   return bq::kErrUnsupported;
 }
 

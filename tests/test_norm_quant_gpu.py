@@ -178,6 +178,27 @@ def test_gated_rms_norm_quant_at_prefill_sizes(Q, ydt, rows, heads):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("rows", [1, 33, 256, 257])
+def test_norms_on_both_sides_of_the_wide_rows(Q, dt, rows):
+    """Up to 256 rows a row has four times the threads (rms) or twice the warps (gated): widths at the
+    edges of what a thread holds, heads that leave warps without one, on both sides of the line."""
+    for cols in (4, 516, 1028, 2052, 4100, 8192):
+        x = randn_cpu((rows, cols + 8), seed=cols, dtype=dt, scale=3.0).cuda()[:, 4:4 + cols]
+        gamma = _gamma(cols, 2, spread=0.3)
+        ref = TS.rms_norm(x, gamma, EPS)
+        qa = Q.rms_norm_quant(x, gamma, EPS, keep_dense=True)
+        assert torch.equal(u8(qa.dense), u8(ref)), f"{dt} {rows}x{cols}"
+        _same(qa, ref, f"{dt} {rows}x{cols}")
+    gamma = _gamma(128, 3, spread=0.3)
+    for heads in (8, 9, 16, 17, 32, 33):
+        y = randn_cpu((rows, heads * 128), seed=heads, dtype=torch.float32, scale=2.0).cuda()
+        z = randn_cpu((rows, heads * 128), seed=heads + 1, dtype=dt, scale=2.0).cuda()
+        ref = TS.rms_norm_gated(y.to(dt).reshape(-1, 128), z.reshape(-1, 128), gamma, EPS).reshape(rows, heads * 128)
+        _same(Q.gated_rms_norm_quant(y, z, gamma, EPS, 128), ref, f"{dt} {rows} rows, {heads} heads")
+    assert Q.device_status() == 0
+
+
 def test_consumers_take_the_quantized_activation(Q):
     """`project`, `linear` and the MLP on a pre-quantized activation equal the reference order of
     operations (norm, then the consumer quantizes) bit for bit, bf16 weights in the mix included."""
