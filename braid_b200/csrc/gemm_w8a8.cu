@@ -1263,21 +1263,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         const uint32_t idesc = dense ? idesc_f16(kPairTile, seg.un, p.dense_fmt)
                                      : idesc_e4m3(kPairTile, silu ? kPairTile : seg.un);
         const int blocks = dense ? p.k_blocks_dense : p.k_blocks;
-        for (int kb = 0; kb < blocks; ++kb, ++it) {
-          const int s = it % kPairStages, use = it / kPairStages;
-          if (!mbar_wait(full_bar(s), use & 1)) { ok = false; break; }
-          tc_fence_after();
-          const uint64_t da = smem_desc_sw128(a_tile(s));
-          const uint64_t db = smem_desc_sw128(b_tile(s));
+        // one loop per operand kind: a choice inside it cost every tile of a mixed launch 8 %
+        auto multiply = [&](auto is_dense) {
+          for (int kb = 0; kb < blocks; ++kb, ++it) {
+            const int s = it % kPairStages, use = it / kPairStages;
+            if (!mbar_wait(full_bar(s), use & 1)) { ok = false; break; }
+            tc_fence_after();
+            const uint64_t da = smem_desc_sw128(a_tile(s));
+            const uint64_t db = smem_desc_sw128(b_tile(s));
 #pragma unroll
-          for (int j = 0; j < kBK / kUmmaK; ++j) {
-            if (dense) mma_f16_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
-            else mma_f8_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
+            for (int j = 0; j < kBK / kUmmaK; ++j) {
+              if constexpr (is_dense.value)
+                mma_f16_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
+              else
+                mma_f8_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
+            }
+            // the stage is free in BOTH CTAs once these MMAs retire
+            mma_commit_pair(empty_bar(s));
+            mma_commit_pair(map_to_cta(empty_bar(s), 1));
           }
-          // the stage is free in BOTH CTAs once these MMAs retire
-          mma_commit_pair(empty_bar(s));
-          mma_commit_pair(map_to_cta(empty_bar(s), 1));
-        }
+        };
+        if (EPI == kMixed && dense) multiply(std::true_type{});
+        else multiply(std::false_type{});
         if (ok) {
           mma_commit_pair(acc_full(b));
           mma_commit_pair(map_to_cta(acc_full(b), 1));
