@@ -199,6 +199,26 @@ def test_norms_on_both_sides_of_the_wide_rows(Q, dt, rows):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("heads", [1, 3, 4, 5, 33])
+def test_gated_rms_norm_quant_with_heads_left_over(Q, dt, heads):
+    """A warp takes four heads of a row at a time: rows whose heads do not divide by four, an infinite
+    gamma (which a head that is not there must not see), rows of very different energy."""
+    rows = 20000 // heads + 2400
+    y = randn_cpu((rows, heads * 128), seed=heads, dtype=dt, scale=2.0).cuda()
+    y[::7] *= 2.0 ** -12
+    z = randn_cpu((rows, heads * 128), seed=heads + 1, dtype=dt, scale=4.0).cuda()
+    gamma = _gamma(128, 3, spread=0.3)
+    ref = TS.rms_norm_gated(y.reshape(-1, 128), z.reshape(-1, 128), gamma, EPS).reshape(rows, heads * 128)
+    _same(Q.gated_rms_norm_quant(y, z, gamma, EPS, 128), ref, f"{dt} {heads}")
+    gamma[5] = float("inf")
+    ref = TS.rms_norm_gated(y.reshape(-1, 128), z.reshape(-1, 128), gamma, EPS).reshape(rows, heads * 128)
+    qa = Q.gated_rms_norm_quant(y, z, gamma, EPS, 128)
+    sr = TS.quantize_act(ref)[1]
+    assert torch.equal(torch.isnan(qa.scale), torch.isnan(sr)) and torch.equal(qa.scale[~torch.isnan(sr)], sr[~torch.isnan(sr)])
+    assert Q.device_status() == 0
+
+
 def test_consumers_take_the_quantized_activation(Q):
     """`project`, `linear` and the MLP on a pre-quantized activation equal the reference order of
     operations (norm, then the consumer quantizes) bit for bit, bf16 weights in the mix included."""
