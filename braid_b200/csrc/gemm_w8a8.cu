@@ -135,6 +135,13 @@ struct PushParams {
   unsigned int* amax_local;       // local running max of the launch (zero between launches)
 };
 
+// The activation unquantized, for the few rows that every CTA quantizes for itself (stream kernel).
+struct QuantIn {
+  const void* x;       // [M, K] contiguous, 16-byte aligned; nullptr = codes and scale are given
+  int dtype;
+  int n8;              // groups of 8 values
+};
+
 struct GemmParams {
   Segment seg[BQ_MAX_SEGMENTS];
   int n_seg;
@@ -142,6 +149,7 @@ struct GemmParams {
   int M;               // activation rows
   int mma_n;           // stream kernel: padded batch = MMA N (multiple of 16)
   int k_blocks;        // ceil(K / 128)
+  int quant_k;         // K, where the activation arrives unquantized
   int k_blocks_dense;  // stream kernel: 128-byte K blocks of a 16-bit row, ceil(2K / 128)
   int dense_fmt;       // stream kernel: tcgen05 operand format of the 16-bit segments (0 f16, 1 bf16)
   int cluster;         // stream kernel: CTAs per cluster = largest split of the launch
@@ -156,6 +164,7 @@ struct GemmParams {
   int phase_seq;
   PairSilu pair;
   PushParams push;
+  QuantIn quant;
 };
 
 // What a launch's epilogue does and the type it writes, as template parameters of the kernels.  A decode
@@ -476,10 +485,68 @@ __device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const floa
 // tile, so every activation slot given up is a weight tile more in flight.
 // The tile area is reused after the main loop as the fp32 staging buffer
 // part[m][128] that the cluster reduction reads.
+//
+// QUANT (fewer rows still): the activation arrives unquantized, and every CTA quantizes it for itself: the
+// warps that have nothing to do until the accumulator is complete read the whole activation (a few
+// dozen KB, from L2) for its max |x|, then cast this CTA's K slice into the activation tiles.  The same
+// values in the same arithmetic everywhere, so every CTA finds the same scale and nothing is
+// exchanged; the quantizer's launch and its hand-over through memory are gone.  Two launches -> one, us in a
+// graph and eager: 1 row of 4096 x 4096 9.0 -> 8.2 and 10.6 -> 8.4, 4 rows of 1024 x 4096 8.7 -> 6.6 and 10.6 -> 7.3,
+// 8 rows of 512 x 1024 6.7 -> 4.9 and 10.7 -> 5.4, 16 rows of 2048 x 2048 8.2 -> 7.3 and 10.7 -> 8.7.  At 64 KB the
+// reading evens out in a graph (8 rows of 4096 x 4096 9.8 -> 9.9; eager 11.3 -> 10.4): the line lies there.
+constexpr int kQuantWarps = kStreamWarps - 2;           // all but the weight loads' and the MMAs'
+constexpr int kQuantThreads = kQuantWarps * 32;
+constexpr int kQuantAhead = 8;                          // groups of 8 a thread asks for at once
+
+// Returns the scale.  Called by warps 2.. with all lanes.
+template <typename T>
+__device__ __forceinline__ float quantize_slice(const QuantIn& in, int M, int K, int kx0, int kb_count, uint8_t* b_tiles,
+                                                int b_tile_bytes, float* s_red) {
+  using namespace bq::qd;
+  const int t = threadIdx.x - (kStreamThreads - kQuantThreads), lane = threadIdx.x & 31, warp = t >> 5;
+  const T* const x = static_cast<const T*>(in.x);
+  float m = 0.0f;
+  for (int g0 = t; g0 < in.n8; g0 += kQuantThreads * kQuantAhead / (sizeof(T) / 2)) {
+    Pack8<T> v[kQuantAhead / (sizeof(T) / 2)];
+#pragma unroll
+    for (int u = 0; u < kQuantAhead / (int)(sizeof(T) / 2); ++u)
+      if (g0 + u * kQuantThreads < in.n8) v[u] = load8<T>(x + static_cast<size_t>(g0 + u * kQuantThreads) * kGroup);
+#pragma unroll
+    for (int u = 0; u < kQuantAhead / (int)(sizeof(T) / 2); ++u)
+      if (g0 + u * kQuantThreads < in.n8) m = absmax8(v[u], m);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
+  if (lane == 0) s_red[warp] = m;
+  asm volatile("bar.sync 2, %0;" ::"n"(kQuantThreads) : "memory");
+  m = s_red[0];
+#pragma unroll
+  for (int i = 1; i < kQuantWarps; ++i) m = nan_max(m, s_red[i]);
+  const float scale = scale_from_amax(m);
+  const ScaleDiv dv(scale);
+  // 16 codes at a time, where TMA would have put them: 16-byte chunk c of row m at c ^ (m & 7).  K is a
+  // multiple of 16; what a last K block has beyond K reads as zero.
+  const int chunks = kb_count * (kBK / 16);             // of a row, in this slice
+  for (int i = t; i < M * chunks; i += kQuantThreads) {
+    const int row = i / chunks, c = i - row * chunks;
+    const int k = kx0 + c * 16;
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    if (k < K) {
+      const T* const src = x + static_cast<size_t>(row) * K + k;
+      const uint2 lo = codes8<T, true>(load8<T>(src), dv), hi = codes8<T, true>(load8<T>(src + 8), dv);
+      w = make_uint4(lo.x, lo.y, hi.x, hi.y);
+    }
+    *reinterpret_cast<uint4*>(b_tiles + (c >> 3) * b_tile_bytes + row * kBK + (((c & 7) ^ (row & 7)) << 4)) = w;
+  }
+  fence_proxy_async_smem();                             // the MMAs read through the async proxy
+  asm volatile("bar.sync 2, %0;" ::"n"(kQuantThreads) : "memory");
+  return scale;
+}
+
 #ifndef BQ_STREAM_MIN_CTAS
 #define BQ_STREAM_MIN_CTAS 2
 #endif
-template <int EPI, int DT>
+template <int EPI, int DT, bool QUANT>
 __global__ void __launch_bounds__(kStreamThreads, BQ_STREAM_MIN_CTAS)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xd,
                    const __grid_constant__ WeightMaps tm_w, const __grid_constant__ GemmParams p,
@@ -508,6 +575,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       reinterpret_cast<volatile uint32_t*>(base_ptr + smem_tile_bytes + 8 * (n_bars + 1));
   volatile uint32_t* const abort_flag = tmem_slot + 1;
   float* const s_quant = reinterpret_cast<float*>(const_cast<uint32_t*>(tmem_slot) + 2);   // one float per warp
+  volatile float* const s_scale = reinterpret_cast<volatile float*>(base_ptr + smem_tile_bytes + kBarrierBytes - 8);
 
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 0); }
   pdl_launch_dependents();   // the next kernel may start its own set-up right away
@@ -543,7 +611,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   while (tmem_cols < static_cast<uint32_t>(p.mma_n)) tmem_cols <<= 1;
 
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(x_map);
+    if (!QUANT) tma_prefetch_desc(x_map);
     tma_prefetch_desc(&tm_w.w[sg]);
     if (pair_on) tma_prefetch_desc(&tm_w.w[1]);
     for (int s = 0; s < p.stages; ++s) {
@@ -602,6 +670,20 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       }
     }
     __syncwarp();
+  } else if (QUANT && warp >= 2) {
+    if constexpr (QUANT) {
+      pdl_wait_prior_grids();   // the kernel that produces the activation has completed
+      const int kx0 = kb_begin * kBK;
+      uint8_t* const tiles = base_ptr + (b_base - base);
+      using T = typename std::conditional<DT == BQ_DTYPE_F32, float,
+                                          typename std::conditional<DT == BQ_DTYPE_F16, __half, __nv_bfloat16>::type>::type;
+      const float sc = quantize_slice<T>(p.quant, p.M, p.quant_k, kx0, kb_count, tiles, b_tile_bytes, s_quant);
+      if (threadIdx.x == kStreamThreads - kQuantThreads) {
+        *s_scale = sc;
+        mbar_arrive(full_bar_b(0));
+      }
+    }
+    __syncwarp();
   } else if (warp == 2) {
     if (elect_one()) {
       // the activation tile is shared by every row tile: keep it in L2
@@ -635,7 +717,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       int s = 0, sb = 0;
       uint32_t phase = 0, phase_b = 0;
       for (int i = 0; i < kb_count; ++i) {
-        if (!mbar_wait(full_bar(s), phase) || !mbar_wait(full_bar_b(sb), phase_b)) {
+        if (!mbar_wait(full_bar(s), phase) || ((!QUANT || i == 0) && !mbar_wait(full_bar_b(sb), phase_b))) {
           *abort_flag = 1;
           break;
         }
@@ -664,12 +746,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   // the epilogue warps get here at once and have the scale ready long before
   // the accumulator is
   const float sw = dense ? 1.0f : __ldg(seg.sw);
-  const float sx_ready = dense ? 1.0f : ld_coherent4(p.sx);
+  float sx_ready = 1.0f;
+  if (!QUANT && !dense) sx_ready = ld_coherent4(p.sx);
   bool ok = mbar_wait(accum_bar, 0);
   tc_fence_after();
   if (threadIdx.x == 0) BQ_STAMP(p, 4);
   if (!ok) *abort_flag = 1;
   __syncthreads();
+  if (QUANT) sx_ready = *s_scale;
   ok = (*abort_flag == 0);
   const float scale = sx_ready * sw;
   float* const part = reinterpret_cast<float*>(base_ptr);   // [mma_n][128]
@@ -1519,22 +1603,26 @@ long long g_opt_push_tma = 1;   // prefill push epilogue: bulk tensor stores (0:
 long long g_opt_pair_narrow = -1;   // prefill: columns of a plain launch's tiles (-1 by rule, 0: 256, 1: 128, else so many)
 long long g_opt_pdl = 1;   // programmatic dependent launch on by default
 long long g_opt_b_stages = 0;   // activation ring depth: 0 = heuristic, -1 = as deep as the weight ring
+long long g_opt_quant_inside = 65536;   // bytes of an activation that every CTA quantizes for itself
 long long g_opt_smem_cap = 0;   // 0 = no cap on pipeline bytes per CTA
 thread_local int g_argmax_slots = 0;     // pairs per batch row the last launch wrote (greedy pick)
 thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
 
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
-using StreamKernel = decltype(&gemm_stream_kernel<kAny, kAnyType>);
+using StreamKernel = decltype(&gemm_stream_kernel<kAny, kAnyType, false>);
 using WideKernel = decltype(&gemm_wide_kernel<1, kAny, kAnyType>);
 using PairKernel = decltype(&gemm_pair_kernel<kAny, kAnyType>);
 
 // The kernels by [epilogue][type]; the types are BQ_DTYPE_F32, BF16, F16 = 0, 1, 2.
 const StreamKernel kStream[3][3] = {
-    {gemm_stream_kernel<kPlain, 0>, gemm_stream_kernel<kPlain, 1>, gemm_stream_kernel<kPlain, 2>},
-    {gemm_stream_kernel<kResidual, 0>, gemm_stream_kernel<kResidual, 1>, gemm_stream_kernel<kResidual, 2>},
-    {gemm_stream_kernel<kGateUp, 0>, gemm_stream_kernel<kGateUp, 1>, gemm_stream_kernel<kGateUp, 2>}};
-const StreamKernel kStreamAny = gemm_stream_kernel<kAny, kAnyType>;
+    {gemm_stream_kernel<kPlain, 0, false>, gemm_stream_kernel<kPlain, 1, false>, gemm_stream_kernel<kPlain, 2, false>},
+    {gemm_stream_kernel<kResidual, 0, false>, gemm_stream_kernel<kResidual, 1, false>, gemm_stream_kernel<kResidual, 2, false>},
+    {gemm_stream_kernel<kGateUp, 0, false>, gemm_stream_kernel<kGateUp, 1, false>, gemm_stream_kernel<kGateUp, 2, false>}};
+const StreamKernel kStreamQuant[2][3] = {
+    {gemm_stream_kernel<kPlain, 0, true>, gemm_stream_kernel<kPlain, 1, true>, gemm_stream_kernel<kPlain, 2, true>},
+    {gemm_stream_kernel<kResidual, 0, true>, gemm_stream_kernel<kResidual, 1, true>, gemm_stream_kernel<kResidual, 2, true>}};
+const StreamKernel kStreamAny = gemm_stream_kernel<kAny, kAnyType, false>;
 template <int MODE>
 struct WideKernels {
   static constexpr WideKernel any = gemm_wide_kernel<MODE, kAny, kAnyType>;
@@ -1580,6 +1668,7 @@ int configure_once() {
         if (kPair[e][d] != nullptr) set((const void*)kPair[e][d]);
         if (e == 3) continue;
         set((const void*)kStream[e][d]);
+        if (e < 2) set((const void*)kStreamQuant[e][d]);
         set((const void*)WideKernels<1>::of[e][d]);
         set((const void*)WideKernels<2>::of[e][d]);
       }
@@ -1705,6 +1794,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   if (stages < 2) stages = kb_max < 2 ? kb_max : 2;
   if (g_opt_stages > 0 && g_opt_stages < stages) stages = (int)g_opt_stages;
   int b_stages = stages;
+  const bool quant = p.quant.x != nullptr;
   // Wide batch tiles: a shallow activation ring (its tiles are L2 hits), the rest goes to
   // weight tiles in flight.  Two slots cover the L2 latency at the rate one CTA of a two-per-SM
   // launch consumes tiles; a CTA that has the SM to itself consumes twice as fast.
@@ -1717,6 +1807,13 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
     if (stages > 24) stages = 24;
     if (b_stages > stages) b_stages = stages;
   }
+  if (quant) {     // the whole slice's activation tiles stay; the weight ring gets the rest
+    b_stages = kb_max;
+    stages = (budget - b_stages * b_tile) / kATileBytes;
+    if (stages > kb_max) stages = kb_max;
+    if (stages > 24) stages = 24;
+    if (stages < (kb_max < 4 ? kb_max : 4) || 2 * stages + b_stages + 1 > 100) return kErrUnsupported;
+  }
   p.stages = stages;
   p.b_stages = b_stages;
   int tile_bytes = stages * kATileBytes + b_stages * b_tile;
@@ -1724,7 +1821,9 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   const int smem = tile_bytes + kBarrierBytes + 1024;
   if (smem > kMaxSmem) return kErrUnsupported;
   const int epi = epilogue_of(p, false);
-  const StreamKernel kernel = epi == kAny ? kStreamAny : kStream[epi][p.out_dtype];
+  if (quant && epi != kPlain && epi != kResidual) return kErrUnsupported;
+  const StreamKernel kernel =
+      quant ? kStreamQuant[epi][p.out_dtype] : (epi == kAny ? kStreamAny : kStream[epi][p.out_dtype]);
   if (p.pair.on) p.pair.expected = (unsigned)((p.seg[0].n / kRowTile) * p.seg[0].split);
   if (p.push.n > 0)
     p.push.expected = (unsigned)(((p.seg[0].n + kRowTile - 1) / kRowTile) * p.seg[0].split);
@@ -1990,6 +2089,11 @@ int bq::gemm_set_option(const char* key, long long value) {
     g_opt_pair_narrow = value < 0 ? -1 : value;
     return kOk;
   }
+  if (strcmp(key, "decode_quant_inside") == 0) {
+    if (value < 0 || value > 262144) return kErrBadArg;
+    g_opt_quant_inside = value;
+    return kOk;
+  }
   if (strcmp(key, "decode_smem_cap") == 0) { g_opt_smem_cap = value; return kOk; }
   if (strcmp(key, "decode_wide") == 0) { g_opt_wide = value < 0 ? -1 : (value ? 1 : 0); return kOk; }
   if (strcmp(key, "decode_cta_target") == 0) {
@@ -2186,13 +2290,13 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
                 const void* const* res = nullptr,
                 const int64_t* ld_res = nullptr, const PairSilu* pair = nullptr,
                 int split_forced = 0, const PushParams* push = nullptr,
-                const DenseArgs* dn = nullptr, const ArgmaxOut* am = nullptr) {
-  if (!xq || !sx || !wq || !sw || !y || !N || !ldy || M <= 0 || K <= 0) return kErrBadArg;
+                const DenseArgs* dn = nullptr, const ArgmaxOut* am = nullptr, const QuantIn* qi = nullptr) {
+  if ((qi == nullptr && (!xq || !sx)) || (qi != nullptr && !qi->x) || !wq || !sw || !y || !N || !ldy || M <= 0 || K <= 0) return kErrBadArg;
   if (n_seg < 1 || n_seg > BQ_MAX_SEGMENTS) return kErrBadArg;
   if (out_dtype != BQ_DTYPE_F32 && out_dtype != BQ_DTYPE_BF16 && out_dtype != BQ_DTYPE_F16)
     return kErrBadArg;
   if (ws == nullptr || ws_bytes < 16u || !aligned_to(ws, 16)) return kErrWorkspace;
-  if (K % 16 || !aligned_to(xq, 16)) return kErrUnsupported;
+  if (K % 16 || !aligned_to(qi != nullptr ? qi->x : xq, 16)) return kErrUnsupported;
   if (M > 0x7fffff00LL || K > 0x7fffff00LL) return kErrTooLarge;
   const int out_align = out_dtype == BQ_DTYPE_F32 ? 16 : 8;
   for (int i = 0; i < n_seg; ++i) {   // argument checks first: no CUDA call before they pass
@@ -2207,6 +2311,10 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     if (N[i] > 0x7fffff00LL) return kErrTooLarge;
   }
   const bool stream_path = M <= g_opt_stream_max_m;
+  if (qi != nullptr) {
+    const long long es = qi->dtype == BQ_DTYPE_F32 ? 4 : 2;
+    if (dn || push || am || pair || g_opt_wide > 0 || M > 16 || M * K * es > g_opt_quant_inside) return kErrUnsupported;
+  }
   if (dn != nullptr) {
     if (pair || push || res) return kErrUnsupported;
     // prefill sizes: 16-bit weights of one tile column (gates); wider ones are a library GEMM's business
@@ -2247,6 +2355,11 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   p.k_blocks_dense = (int)((2 * K + kBK - 1) / kBK);
   p.dense_fmt = (dn != nullptr && dn->dtype == BQ_DTYPE_BF16) ? 1 : 0;
   p.out_dtype = out_dtype;
+  if (qi != nullptr) {
+    p.quant = *qi;
+    p.quant.n8 = (int)(M * K / 8);
+    p.quant_k = (int)K;
+  }
   // the sticky status word is the 4th word of the scratch, as in the quantizer
   p.status = static_cast<unsigned int*>(ws) + 3;
   if (pair) {
@@ -2266,7 +2379,7 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     p.push.amax_local = (push->amax_dst[0] != nullptr) ? static_cast<unsigned int*>(ws) + 1 : nullptr;
   }
 
-  if (stream_path && (p.M > 32 || g_opt_wide > 0)) {
+  if (stream_path && qi == nullptr && (p.M > 32 || g_opt_wide > 0)) {
     const int rc = run_wide(p, xq, K, wq, sw, y, N, ldy, res, ld_res, dn, stream);
     if (rc != kErrUnsupported) return rc;
   }
@@ -2361,6 +2474,7 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   CUtensorMap tm_x;
   if (stream_path) {
     const int mma_n = (int)(((M + 15) / 16) * 16);
+    if (qi != nullptr) return launch_stream(maps.w[0], maps.w[0], maps, p, stream);   // no map of the activation
     if (int rc = make_map(&tm_x, xq, M, K, mma_n)) return rc;
     CUtensorMap tm_xd = tm_x;
     if (dn != nullptr)
@@ -2381,6 +2495,18 @@ extern "C" int bq_gemm_w8a8_grouped(const void* xq, const float* sx, int64_t M, 
                                     const int64_t* N, const int64_t* ldy, int out_dtype, void* ws,
                                     size_t ws_bytes, void* stream_v) {
   return run_grouped(xq, sx, M, K, n_seg, wq, sw, y, N, ldy, out_dtype, ws, ws_bytes, stream_v);
+}
+
+extern "C" int bq_linear_w8a8(const void* x, int dtype, int64_t M, int64_t K, int n_seg, const void* const* wq,
+                              const float* const* sw, const void* residual, int64_t ld_res, void* const* y,
+                              const int64_t* N, const int64_t* ldy, void* ws, size_t ws_bytes, void* stream) {
+  if (x == nullptr || (residual != nullptr && n_seg != 1)) return kErrBadArg;
+  const QuantIn qi{x, dtype, 0};
+  const void* rs[1] = {residual};
+  const int64_t ldrs[1] = {ld_res};
+  return run_grouped(nullptr, nullptr, M, K, n_seg, wq, sw, y, N, ldy, dtype, ws, ws_bytes, stream,
+                     residual != nullptr ? rs : nullptr, residual != nullptr ? ldrs : nullptr, nullptr, 0, nullptr, nullptr,
+                     nullptr, &qi);
 }
 
 extern "C" int bq_project_mixed(const void* xq, const float* sx, const void* x_dense, int dense_dtype,

@@ -3,13 +3,13 @@
 //
 // An eager decode or prompt call launches kernels of 3 to 30 us; made from Python through ctypes a
 // launch costs about 18 us of host time (allocations with keyword arguments, stream lookup,
-// argument conversion), from here about 5, so from there the host is what bounds it: a projection of 8 rows
-// 36.3 -> 10.4 us, the MLP of one row 51 -> 39, a decoder layer of 16 rows 164 -> 74, which is its kernels' time.
-// Each function here does what its namesake in
-// quant.py does for the plain case -- ordinary CUDA tensors of the current device, no dispatch mode or
-// transform, operands the kernels take -- and returns None for everything else; quant.py then runs its
-// own code, which decides, converts and raises as it always did.  Nothing is kept between calls but
-// the scratch slots' counter, which quant.py shares.
+// argument conversion), from here about 5.  A projection of 8 rows 36.3 -> 10.8 us (9.9 as one launch), the
+// MLP of one row 51 -> 38, a decoder layer of 16 rows 162 -> 73; the last two are their kernels' time.
+//
+// Each function here does what its namesake in quant.py does for the plain case -- ordinary CUDA tensors
+// of the current device, no dispatch mode or transform, operands the kernels take -- and returns None for
+// everything else; quant.py then runs its own code, which decides, converts and raises as it always did.
+// Nothing is kept between calls but the scratch slots' counter, which quant.py shares.
 //
 // The kernels' library is not linked: quant.py hands over the addresses of the functions it has loaded.
 #define PY_SSIZE_T_CLEAN
@@ -44,6 +44,7 @@ struct Lib {
   decltype(&bq_sigmoid_mul_dense_scale) sigmoid_mul_dense_scale;
   decltype(&bq_gemm_w8a8_grouped) gemm_grouped;
   decltype(&bq_gemm_w8a8_residual) gemm_residual;
+  decltype(&bq_linear_w8a8) linear;
   decltype(&bq_project_mixed) project_mixed;
   decltype(&bq_gate_up_silu_quant_w8a8) gate_up_silu_quant;
   decltype(&bq_gate_up_silu_w8a8) gate_up_silu;
@@ -340,6 +341,8 @@ PyObject* sigmoid_gate_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+constexpr int64_t kInsideRows = 16, kInsideBytes = 65536;      // bq_linear_w8a8 takes no more
+
 // ---- the GEMMs ------------------------------------------------------------------------------
 // One weight, with or without the residual added; undefined where quant.py has to decide.
 at::Tensor gemm(const Here& h, const at::Tensor& xq, const at::Tensor& sx, const at::Tensor& w, const at::Tensor& sw,
@@ -377,7 +380,7 @@ at::Tensor as_rows(const at::Tensor& t, int64_t cols) {     // undefined stays u
   return !t.defined() || t.dim() == 2 ? t : t.reshape({-1, cols});
 }
 
-// linear(x, w, sw, residual or None): quantize, multiply, leading dimensions kept
+// linear(x, w, sw, residual or None): quantize, multiply, leading dimensions kept.  Few rows: one launch.
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   BQ_ARGS(4)
@@ -399,16 +402,35 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       residual = residual.view({-1, N});
     }
   }
+  auto shaped = [&](const at::Tensor& y) {
+    if (x.dim() == 2) return y;
+    std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = N;
+    return y.view(shape);
+  };
+  int rc;
+  const int64_t M = x.numel() / K;
+  const int code = dtype_code(x.scalar_type());
+  if (M <= kInsideRows && x.numel() * x.element_size() <= kInsideBytes && code >= 0 && aligned(x.data_ptr(), 16) &&
+      (!res || (residual.scalar_type() == x.scalar_type() && residual.size(0) == M && residual.stride(1) == 1))) {
+    at::Tensor y = empty(h, {M, N}, x.scalar_type());
+    void* slot = take_slot(h.dev);
+    const void* wq = w.data_ptr();
+    const float* swp = sw.data_ptr<float>();
+    void* yp = y.data_ptr();
+    {
+      NoGil no_gil;
+      rc = g_lib.linear(x.data_ptr(), code, M, K, 1, &wq, &swp, res ? residual.data_ptr() : nullptr,
+                        res ? residual.stride(0) : 0, &yp, &N, &N, slot, 16, h.stream);
+    }
+    if (rc == BQ_OK) return wrap(shaped(y));
+    g_launches.fetch_sub(1, std::memory_order_relaxed);
+  }
   const Quantized r = quantize(h, x);
   if (!r.q.defined()) Py_RETURN_NONE;
   if (r.rc != BQ_OK) return refused();
-  int rc;
   at::Tensor y = gemm(h, x.dim() == 2 ? r.q : r.q.view({-1, K}), r.scale, w, sw, x.scalar_type(), residual, rc);
-  if (y.defined() && rc == BQ_OK && x.dim() != 2) {
-    std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
-    shape.back() = N;
-    y = y.view(shape);
-  }
+  if (y.defined() && rc == BQ_OK) y = shaped(y);
   return gemm_result(y, rc);
   END_HANDLE_TH_ERRORS
 }
@@ -616,7 +638,7 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !get("bq_sigmoid_gate_quant", g_lib.sigmoid_gate_quant) ||
       !get("bq_sigmoid_mul_dense_scale", g_lib.sigmoid_mul_dense_scale) ||
       !get("bq_gemm_w8a8_grouped", g_lib.gemm_grouped) || !get("bq_gemm_w8a8_residual", g_lib.gemm_residual) ||
-      !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_w8a8", g_lib.gate_up_silu_quant) ||
+      !get("bq_linear_w8a8", g_lib.linear) || !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_w8a8", g_lib.gate_up_silu_quant) ||
       !get("bq_gate_up_silu_w8a8", g_lib.gate_up_silu) || !get("bq_lm_head_argmax", g_lib.lm_head_argmax) ||
       !get("bq_lm_head_argmax_workspace_bytes", g_lib.lm_head_argmax_workspace))
     return nullptr;

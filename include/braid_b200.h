@@ -278,6 +278,17 @@ int bq_gated_rmsnorm_scale(const void* y, int y_dtype, int64_t ld_y, const void*
                            size_t ws_bytes, void* stream);
 
 /*
+ * bq_quantize_act and bq_gemm_w8a8_grouped (or, with one weight, bq_gemm_w8a8_residual) in one launch for
+ * few rows: x [M, K] of `dtype` (also the outputs' type), contiguous; every CTA quantizes it for itself.
+ * The same bits as the two calls.  BQ_ERR_UNSUPPORTED beyond 16 rows or 64 KB of x.
+ *
+ * Replaces: braid/model/quant.py:244-252 (`fp8_linear`) at those sizes.
+ */
+int bq_linear_w8a8(const void* x, int dtype, int64_t M, int64_t K, int n_seg, const void* const* wq,
+                   const float* const* sw, const void* residual, int64_t ld_res, void* const* y,
+                   const int64_t* N, const int64_t* ldy, void* ws, size_t ws_bytes, void* stream);
+
+/*
  * Bytes of scratch the GEMM entry points need: 16 (the sticky status word and
  * the counters of the paired / push epilogues).  Split-K partial sums travel
  * through distributed shared memory and never reach global memory.  Zero the

@@ -552,6 +552,29 @@ def test_shape_guards(Q):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("K,N", [(4096, 4096), (1040, 1024), (16, 16), (272, 144), (512, 40000), (12288, 1024)])
+def test_linear_of_few_rows_as_one_launch(Q, dt, K, N):
+    """Up to 16 rows and 64 KB every CTA quantizes the activation for itself: the bits of quantizer and GEMM
+    apart, K tails, 1, 2 and 4 K slices, several clusters, a residual, both sides of both limits, NaN."""
+    fw = Q.quantize_weight(randn_cpu((N, K), seed=1, scale=0.02).cuda())
+    for M in (1, 2, 7, 8, 9, 16, 17):
+        x = randn_cpu((M, K), seed=M, dtype=dt).cuda()
+        x[0, 3] = 50.0
+        res = randn_cpu((M, N), seed=2, dtype=dt).cuda()
+        small = M <= 16 and M * K * x.element_size() <= 65536
+        for r in (None, res):
+            n0 = Q.launch_count()
+            got = Q.linear(x, fw, residual=r)
+            assert Q._NATIVE is None or Q.launch_count() - n0 == (1 if small else 2)
+            xq, sx = Q.quantize_act(x)
+            assert torch.equal(got, Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=r)), (M, r is not None)
+        assert torch.equal(Q.linear(x.view(M, 1, K), fw), Q.linear(x, fw).view(M, 1, N))
+        x[M - 1, K - 1] = float("nan")
+        assert torch.isnan(Q.linear(x, fw)).all()
+    assert Q.device_status() == 0
+
+
 # -- residual add in the epilogue ---------------------------------------------------------------
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
 @pytest.mark.parametrize("M", [1, 8, 37, 128, 256, 512])

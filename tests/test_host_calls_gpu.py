@@ -1,5 +1,5 @@
 """The native calls (`csrc/host_calls.cpp`) against the Python code they stand in for: same bits, same
-shapes, same launches, and whatever they do not take is decided by that code."""
+shapes, no more launches, and whatever they do not take is decided by that code."""
 from __future__ import annotations
 
 import pytest
@@ -29,7 +29,7 @@ def _both(Q, monkeypatch, fn):
     with monkeypatch.context() as m:
         m.setattr(Q, "_NATIVE", None)
         python = _flat(fn())
-    assert n1 - n0 == Q.launch_count() - n1
+    assert n1 - n0 <= Q.launch_count() - n1        # few rows: `linear` is one launch there
     assert len(native) == len(python)
     for a, b in zip(native, python):
         assert a.shape == b.shape and a.dtype is b.dtype and a.stride() == b.stride()
