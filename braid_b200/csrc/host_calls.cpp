@@ -7,8 +7,8 @@
 // MLP of one row 51 -> 38, a decoder layer of 16 rows 162 -> 73; the last two are their kernels' time.
 //
 // Each function here does what its namesake in quant.py does for the plain case -- ordinary CUDA tensors
-// of the current device, no dispatch mode or transform, operands the kernels take -- and returns None for
-// everything else; quant.py then runs its own code, which decides, converts and raises as it always did.
+// of the current device, no dispatch mode, transform, forward-mode level or tracer, operands the kernels take
+// -- and returns None for everything else; quant.py then runs its own code, which decides, converts and raises as it always did.
 // Nothing is kept between calls but the scratch slots' counter, which quant.py shares.
 //
 // The kernels' library is not linked: quant.py hands over the addresses of the functions it has loaded.
@@ -16,6 +16,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/autocast_mode.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
@@ -23,6 +24,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <array>
@@ -69,14 +71,16 @@ void* take_slot(int dev) {
   return reinterpret_cast<void*>(g_scratch[dev].base.load(std::memory_order_relaxed) + uint64_t(slot) * g_slot_bytes);
 }
 
-// What a call needs of its surroundings; false = leave it to quant.py.
+// What a call needs of its surroundings; false = leave it to quant.py.  A dual tensor is an ordinary strided
+// one with nothing in its keys to tell it by, so an open forward-mode level is asked for by itself, as quant.py does.
 struct Here {
   int dev = -1;
   void* stream = nullptr;
   bool ok = false;
   explicit Here(const at::Tensor& t) {
     if (!g_ready || !t.defined() || !t.is_cuda() || c10::impl::TorchDispatchModeTLS::stack_len() > 0 ||
-        c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+        c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) ||
+        at::tracer::impl::is_dispatch_enabled() || torch::autograd::ForwardADLevel::try_get_by_idx(0) != nullptr)
       return;
     dev = t.device().index();
     if (dev < 0 || dev >= kMaxDevices || dev != c10::cuda::current_device() ||
@@ -141,8 +145,9 @@ struct NoGil {
   ~NoGil() { PyEval_RestoreThread(s); }
 };
 
-// A positional argument as a tensor; not a tensor = undefined.
-at::Tensor arg(PyObject* o) { return THPVariable_Check(o) ? THPVariable_Unpack(o) : at::Tensor(); }
+// A positional argument as a tensor; undefined = not a tensor, or a subclass other than Parameter, whose results
+// torch would wrap.
+at::Tensor arg(PyObject* o) { return THPVariable_CheckExact(o) ? THPVariable_Unpack(o) : at::Tensor(); }
 PyObject* wrap(const at::Tensor& t) { return THPVariable_Wrap(t); }
 PyObject* pair(const at::Tensor& a, const at::Tensor& b) {
   PyObject* r = PyTuple_New(2);

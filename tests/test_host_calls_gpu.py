@@ -4,6 +4,8 @@ from __future__ import annotations
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fwad
+import torch.nn.functional as F
 
 from _util import randn_cpu, u8
 
@@ -99,6 +101,37 @@ def test_what_the_python_code_refuses_stays_refused(Q, weights):
                 lambda: Q.project(x[:, :256].contiguous(), w["a"], w["b"])):
         with pytest.raises(ValueError):
             bad()
+
+
+class _Tagged(torch.Tensor):
+    """A subclass without a dispatch of its own: only its Python type tells it from a tensor."""
+
+
+def test_what_torch_follows_above_256_rows_stays_a_torch_operation(Q, weights):
+    """The residual add and the 16-bit gates of a prompt are torch operations where torch follows them:
+    forward-mode tangents are carried, subclasses keep their type, a tracer sees the addition."""
+    M, H, w = 300, 512, weights
+    x, res, t = (randn_cpu((M, H), seed=s).cuda() for s in (1, 2, 3))
+    gate, tg = (randn_cpu((16, H), seed=s, scale=0.02).cuda() for s in (4, 5))
+    xq, sx = Q.quantize_act(x)
+    adds = {"matmul": lambda r: Q.fp8_matmul(xq, sx, w["a"], residual=r), "linear": lambda r: Q.linear(x, w["a"], residual=r),
+            "mlp": lambda r: Q.mlp_forward(x, w["gate"], w["up"], w["down"], residual=r)}
+    for name, add in adds.items():
+        with fwad.dual_level():
+            out = fwad.unpack_dual(add(fwad.make_dual(res, t)))
+            assert out.tangent is not None and torch.equal(out.tangent, t), name
+            assert torch.equal(out.primal, add(res)), name
+        assert type(add(res.as_subclass(_Tagged))) is _Tagged, name
+        traced = torch.jit.trace(add, (res,), check_trace=False)
+        assert torch.equal(traced(t), add(t)), name
+    with fwad.dual_level():
+        for got, want in ((Q.project(fwad.make_dual(x, t), w["a"], gate)[1], F.linear(t, gate)),
+                          (Q.project(x, w["a"], fwad.make_dual(gate, tg))[1], F.linear(x, tg))):
+            tangent = fwad.unpack_dual(got).tangent
+            assert tangent is not None and torch.equal(tangent, want)
+    assert type(Q.project(x.as_subclass(_Tagged), w["a"], gate)[1]) is _Tagged
+    assert type(Q.project(x, w["a"], gate.as_subclass(_Tagged))[1]) is _Tagged
+    assert Q.device_status() == 0
 
 
 def test_native_calls_from_threads_and_streams(Q, weights):
