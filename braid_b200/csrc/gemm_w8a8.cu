@@ -2313,7 +2313,9 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   const bool stream_path = M <= g_opt_stream_max_m;
   if (qi != nullptr) {
     const long long es = qi->dtype == BQ_DTYPE_F32 ? 4 : 2;
-    if (dn || push || am || pair || g_opt_wide > 0 || M > 16 || M * K * es > g_opt_quant_inside) return kErrUnsupported;
+    // the weight-streaming kernel alone has this form: the others read codes and scale, which are not given
+    if (!stream_path || dn || push || am || pair || g_opt_wide > 0 || M > 16 || M * K * es > g_opt_quant_inside)
+      return kErrUnsupported;
   }
   if (dn != nullptr) {
     if (pair || push || res) return kErrUnsupported;

@@ -593,6 +593,27 @@ def test_residual_epilogue_equals_gemm_then_add(Q, dt, M, N, K):
     assert torch.equal(got, want), f"{int((got != want).sum())} of {got.numel()} differ"
 
 
+@pytest.mark.parametrize("key,value,back", [("stream_max_m", 8, 256), ("decode_wide", 1, -1)])
+def test_linear_of_few_rows_leaves_forced_kernels_to_two_launches(Q, key, value, back):
+    """An option that sends the batch to another kernel: quantizer and that GEMM, bit for bit (the other
+    kernel sums K in another order: one rounding of the output away from the one launch)."""
+    fw = Q.quantize_weight(randn_cpu((1024, 512), seed=1, scale=0.02).cuda())
+    x = randn_cpu((16, 512), seed=2).cuda()
+    n0 = Q.launch_count()
+    want = Q.linear(x, fw)
+    assert Q._NATIVE is None or Q.launch_count() - n0 == 1
+    try:
+        Q.set_option(key, value)
+        n0 = Q.launch_count()
+        got = Q.linear(x, fw)
+        assert Q.launch_count() - n0 == 2
+        assert torch.equal(got, Q.fp8_matmul(*Q.quantize_act(x), fw))
+    finally:
+        Q.set_option(key, back)
+    assert max_rel(got, want) <= 2 ** -8
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
 @pytest.mark.parametrize("M,N,K", [(257, 4096, 512), (300, 272, 256), (413, 1040, 1040), (512, 16, 16), (1000, 4112, 2048)])
 def test_prefill_residual_epilogue_over_row_pitches(Q, dt, M, N, K):

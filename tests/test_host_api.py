@@ -143,6 +143,24 @@ def test_argument_validation_returns_before_any_cuda_call(lib):
         _lib.check(_lib.BQ_ERR_DEVICE_WAIT, "x")
 
 
+def test_linear_of_few_rows_is_refused_where_an_option_rules_it_out(lib):
+    """The one-launch form is the weight-streaming kernel's.  Options that send the batch to another kernel
+    leave the call to the two launches, before any CUDA call is made."""
+    from braid_b200 import _lib
+    ptr, n = (ctypes.c_void_p * 1)(16), (ctypes.c_int64 * 1)(64)
+
+    def rc(M):
+        return lib.bq_linear_w8a8(16, 1, M, 64, 1, ptr, ptr, None, 0, ptr, n, n, 16, 16, None)
+
+    for key, value, back, rows in (("stream_max_m", 8, 256, 9), ("decode_wide", 1, -1, 1)):
+        assert lib.bq_set_option(key.encode(), value) == _lib.BQ_OK
+        try:
+            assert rc(rows) == _lib.BQ_ERR_UNSUPPORTED, (key, value)
+        finally:
+            assert lib.bq_set_option(key.encode(), back) == _lib.BQ_OK
+    assert rc(17) == _lib.BQ_ERR_UNSUPPORTED
+
+
 def test_a_missing_library_is_loud(monkeypatch, tmp_path):
     from braid_b200 import _lib, quant
     monkeypatch.setattr(_lib, "_lib", None)
