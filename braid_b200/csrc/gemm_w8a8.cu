@@ -2313,8 +2313,10 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   const bool stream_path = M <= g_opt_stream_max_m;
   if (qi != nullptr) {
     const long long es = qi->dtype == BQ_DTYPE_F32 ? 4 : 2;
-    // the weight-streaming kernel alone has this form: the others read codes and scale, which are not given
-    if (!stream_path || dn || push || am || pair || g_opt_wide > 0 || M > 16 || M * K * es > g_opt_quant_inside)
+    // the weight-streaming kernel alone has this form: the others read codes and scale, which are not given.  Its
+    // rings are cut to the activation, so forced depths are left to the two launches.
+    if (!stream_path || dn || push || am || pair || g_opt_wide > 0 || g_opt_stages > 0 || g_opt_b_stages != 0 || M > 16 ||
+        M * K * es > g_opt_quant_inside)
       return kErrUnsupported;
   }
   if (dn != nullptr) {

@@ -593,10 +593,12 @@ def test_residual_epilogue_equals_gemm_then_add(Q, dt, M, N, K):
     assert torch.equal(got, want), f"{int((got != want).sum())} of {got.numel()} differ"
 
 
-@pytest.mark.parametrize("key,value,back", [("stream_max_m", 8, 256), ("decode_wide", 1, -1)])
+@pytest.mark.parametrize("key,value,back", [("stream_max_m", 8, 256), ("decode_wide", 1, -1), ("decode_stages", 2, 0),
+                                            ("decode_b_stages", 1, 0)])
 def test_linear_of_few_rows_leaves_forced_kernels_to_two_launches(Q, key, value, back):
-    """An option that sends the batch to another kernel: quantizer and that GEMM, bit for bit (the other
-    kernel sums K in another order: one rounding of the output away from the one launch)."""
+    """An option that sends the batch to another kernel or forces a ring's depth: quantizer and that GEMM,
+    bit for bit (another kernel sums K in another order: one rounding of the output away from the one
+    launch)."""
     fw = Q.quantize_weight(randn_cpu((1024, 512), seed=1, scale=0.02).cuda())
     x = randn_cpu((16, 512), seed=2).cuda()
     n0 = Q.launch_count()
@@ -608,6 +610,7 @@ def test_linear_of_few_rows_leaves_forced_kernels_to_two_launches(Q, key, value,
         got = Q.linear(x, fw)
         assert Q.launch_count() - n0 == 2
         assert torch.equal(got, Q.fp8_matmul(*Q.quantize_act(x), fw))
+        assert key != "decode_stages" or Q.last_gemm_launch()["stages"] <= value
     finally:
         Q.set_option(key, back)
     assert max_rel(got, want) <= 2 ** -8

@@ -144,15 +144,17 @@ def test_argument_validation_returns_before_any_cuda_call(lib):
 
 
 def test_linear_of_few_rows_is_refused_where_an_option_rules_it_out(lib):
-    """The one-launch form is the weight-streaming kernel's.  Options that send the batch to another kernel
-    leave the call to the two launches, before any CUDA call is made."""
+    """The one-launch form is the weight-streaming kernel's, with the rings it chooses itself.  Options that send
+    the batch to another kernel or force a ring's depth leave the call to the two launches, before any
+    CUDA call is made."""
     from braid_b200 import _lib
     ptr, n = (ctypes.c_void_p * 1)(16), (ctypes.c_int64 * 1)(64)
 
     def rc(M):
         return lib.bq_linear_w8a8(16, 1, M, 64, 1, ptr, ptr, None, 0, ptr, n, n, 16, 16, None)
 
-    for key, value, back, rows in (("stream_max_m", 8, 256, 9), ("decode_wide", 1, -1, 1)):
+    for key, value, back, rows in (("stream_max_m", 8, 256, 9), ("decode_wide", 1, -1, 1), ("decode_stages", 2, 0, 1),
+                                   ("decode_b_stages", 2, 0, 1), ("decode_b_stages", -1, 0, 1)):
         assert lib.bq_set_option(key.encode(), value) == _lib.BQ_OK
         try:
             assert rc(rows) == _lib.BQ_ERR_UNSUPPORTED, (key, value)
