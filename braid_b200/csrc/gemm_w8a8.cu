@@ -492,8 +492,8 @@ __device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const floa
 // values in the same arithmetic everywhere, so every CTA finds the same scale and nothing is
 // exchanged; the quantizer's launch and its hand-over through memory are gone.  Two launches -> one, us in a
 // graph and eager: 1 row of 4096 x 4096 9.0 -> 8.2 and 10.6 -> 8.4, 4 rows of 1024 x 4096 8.7 -> 6.6 and 10.6 -> 7.3,
-// 8 rows of 512 x 1024 6.7 -> 4.9 and 10.7 -> 5.4, 16 rows of 2048 x 2048 8.2 -> 7.3 and 10.7 -> 8.7.  At 64 KB the
-// reading evens out in a graph (8 rows of 4096 x 4096 9.8 -> 9.9; eager 11.3 -> 10.4): the line lies there.
+// 8 rows of 512 x 1024 6.7 -> 4.9 and 10.7 -> 5.4, 16 rows of 2048 x 2048 8.2 -> 7.3 and 10.7 -> 8.7.  Where it stops
+// paying: quantize_inside_pays.
 constexpr int kQuantWarps = kStreamWarps - 2;           // all but the weight loads' and the MMAs'
 constexpr int kQuantThreads = kQuantWarps * 32;
 constexpr int kQuantAhead = 8;                          // groups of 8 a thread asks for at once
@@ -1603,7 +1603,7 @@ long long g_opt_push_tma = 1;   // prefill push epilogue: bulk tensor stores (0:
 long long g_opt_pair_narrow = -1;   // prefill: columns of a plain launch's tiles (-1 by rule, 0: 256, 1: 128, else so many)
 long long g_opt_pdl = 1;   // programmatic dependent launch on by default
 long long g_opt_b_stages = 0;   // activation ring depth: 0 = heuristic, -1 = as deep as the weight ring
-long long g_opt_quant_inside = 65536;   // bytes of an activation that every CTA quantizes for itself
+long long g_opt_quant_inside = -1;   // bytes of an activation that every CTA quantizes for itself (-1 by rule)
 long long g_opt_smem_cap = 0;   // 0 = no cap on pipeline bytes per CTA
 thread_local int g_argmax_slots = 0;     // pairs per batch row the last launch wrote (greedy pick)
 thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
@@ -1746,6 +1746,35 @@ int split_for_weight(long long n_rows, int k_blocks) {
   return s;
 }
 
+// Few rows: is the launch whose CTAs quantize the activation for themselves the faster form?  It saves a launch;
+// every CTA reads all of the activation and casts its K slice, and its weights wait for that.  So what counts is
+// the bytes a CTA reads plus those it casts.  us in a graph, one launch and two, at the bytes of the activation and the
+// K slices of the weight: 48 KB in 4 (6 rows of 4096 x 4096) 9.8 and 9.8, 64 KB in 4 (8 rows) 10.0 and 9.8; 40 KB in 2
+// (5 rows of 8192 x 4096) 12.6 and 12.7, 48 KB in 2 (6 rows) 13.6 and 12.9; 24 KB in 1 (6 rows of 12288 x 2048) 10.7
+// and 10.9, 32 KB in 1 (8 rows) 11.3 and 10.8, 64 KB in 1 (16 rows) 13.9 and 10.9.  A weight of 64 CTAs or fewer
+// reads less in all (8 rows of 2048 x 4096 8.3 and 9.0).  A call that is not captured pays the host for its second
+// launch as well: 64 KB in 4 10.2 and 11.3, 60 KB in 2 (6 rows of 8192 x 5120) 14.6 and 15.3, 64 KB in 2 (8 rows of
+// 6144 x 4096) 13.2 and 12.5; 40 KB in 1 (5 rows of 12288 x 4096) 15.2 and 16.0, 48 KB in 1 (12 rows of
+// 12288 x 2048) 12.5 and 11.5.
+constexpr int64_t kInsideBytes = 65536, kInsideWork = 61440, kInsideWorkEager = 92160;
+
+bool quantize_inside_pays(int64_t M, int64_t K, int element_size, int n_seg, const int64_t* N, cudaStream_t stream) {
+  const int64_t bytes = M * K * element_size;
+  if (g_opt_quant_inside >= 0) return bytes <= g_opt_quant_inside;
+  const int k_blocks = (int)((K + kBK - 1) / kBK);
+  int64_t cast = 0, ctas = 0;
+  for (int i = 0; i < n_seg; ++i) {
+    const int split = split_for_weight(N[i], k_blocks);
+    if (bytes / split > cast) cast = bytes / split;
+    ctas += (N[i] + kRowTile - 1) / kRowTile * split;
+  }
+  if (bytes > kInsideBytes || bytes + cast > kInsideWorkEager) return false;
+  if (bytes + cast <= kInsideWork || ctas <= 64) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) (void)cudaGetLastError();
+  return status == cudaStreamCaptureStatusNone;
+}
+
 int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightMaps& maps,
                   GemmParams& p, cudaStream_t stream) {
   const int sms = device_sms();
@@ -1812,6 +1841,8 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
     stages = (budget - b_stages * b_tile) / kATileBytes;
     if (stages > kb_max) stages = kb_max;
     if (stages > 24) stages = 24;
+    // long slices of few rows: tiles padded to 16 rows would crowd out the weights (1 row of 8192 x 20480: 33 -> 36 us)
+    if (2 * b_stages * b_tile > budget) return kErrUnsupported;
     if (stages < (kb_max < 4 ? kb_max : 4) || 2 * stages + b_stages + 1 > 100) return kErrUnsupported;
   }
   p.stages = stages;
@@ -2090,8 +2121,8 @@ int bq::gemm_set_option(const char* key, long long value) {
     return kOk;
   }
   if (strcmp(key, "decode_quant_inside") == 0) {
-    if (value < 0 || value > 262144) return kErrBadArg;
-    g_opt_quant_inside = value;
+    if (value > 262144) return kErrBadArg;
+    g_opt_quant_inside = value < 0 ? -1 : value;
     return kOk;
   }
   if (strcmp(key, "decode_smem_cap") == 0) { g_opt_smem_cap = value; return kOk; }
@@ -2312,11 +2343,11 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   }
   const bool stream_path = M <= g_opt_stream_max_m;
   if (qi != nullptr) {
-    const long long es = qi->dtype == BQ_DTYPE_F32 ? 4 : 2;
     // the weight-streaming kernel alone has this form: the others read codes and scale, which are not given.  Its
     // rings are cut to the activation, so forced depths are left to the two launches.
-    if (!stream_path || dn || push || am || pair || g_opt_wide > 0 || g_opt_stages > 0 || g_opt_b_stages != 0 || M > 16 ||
-        M * K * es > g_opt_quant_inside)
+    if (!stream_path || dn || push || am || pair || g_opt_wide > 0 || g_opt_stages > 0 || g_opt_b_stages != 0 ||
+        M > BQ_LINEAR_MAX_ROWS ||
+        !quantize_inside_pays(M, K, qi->dtype == BQ_DTYPE_F32 ? 4 : 2, n_seg, N, static_cast<cudaStream_t>(stream_v)))
       return kErrUnsupported;
   }
   if (dn != nullptr) {

@@ -346,12 +346,11 @@ PyObject* sigmoid_gate_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-constexpr int64_t kInsideRows = 16, kInsideBytes = 65536;      // bq_linear_w8a8 takes no more
-
 // ---- the GEMMs ------------------------------------------------------------------------------
-// One weight, with or without the residual added; undefined where quant.py has to decide.
+// One weight, with or without the residual added, into `y` if there is one already; undefined where quant.py has
+// to decide.
 at::Tensor gemm(const Here& h, const at::Tensor& xq, const at::Tensor& sx, const at::Tensor& w, const at::Tensor& sw,
-                at::ScalarType out, const at::Tensor& residual, int& rc) {
+                at::ScalarType out, const at::Tensor& residual, int& rc, at::Tensor y = {}) {
   rc = BQ_OK;
   const int code = dtype_code(out);
   if (code < 0 || !is_codes(h, xq) || !is_scale(h, sx) || !is_scale(h, sw) || !is_weight(h, w, xq.size(1))) return {};
@@ -360,7 +359,7 @@ at::Tensor gemm(const Here& h, const at::Tensor& xq, const at::Tensor& sx, const
   if (res && (!plain(h, residual) || residual.dim() != 2 || residual.size(0) != M || residual.size(1) != N ||
               residual.scalar_type() != out || residual.stride(1) != 1 || recorded(residual)))
     return {};
-  at::Tensor y = empty(h, {M, N}, out);
+  if (!y.defined()) y = empty(h, {M, N}, out);
   void* slot = take_slot(h.dev);
   const void* wq = w.data_ptr();
   const float* swp = sw.data_ptr<float>();
@@ -416,9 +415,10 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   int rc;
   const int64_t M = x.numel() / K;
   const int code = dtype_code(x.scalar_type());
-  if (M <= kInsideRows && x.numel() * x.element_size() <= kInsideBytes && code >= 0 && aligned(x.data_ptr(), 16) &&
+  at::Tensor y;
+  if (M <= BQ_LINEAR_MAX_ROWS && code >= 0 && aligned(x.data_ptr(), 16) &&
       (!res || (residual.scalar_type() == x.scalar_type() && residual.size(0) == M && residual.stride(1) == 1))) {
-    at::Tensor y = empty(h, {M, N}, x.scalar_type());
+    y = empty(h, {M, N}, x.scalar_type());
     void* slot = take_slot(h.dev);
     const void* wq = w.data_ptr();
     const float* swp = sw.data_ptr<float>();
@@ -434,7 +434,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const Quantized r = quantize(h, x);
   if (!r.q.defined()) Py_RETURN_NONE;
   if (r.rc != BQ_OK) return refused();
-  at::Tensor y = gemm(h, x.dim() == 2 ? r.q : r.q.view({-1, K}), r.scale, w, sw, x.scalar_type(), residual, rc);
+  y = gemm(h, x.dim() == 2 ? r.q : r.q.view({-1, K}), r.scale, w, sw, x.scalar_type(), residual, rc, y);
   if (y.defined() && rc == BQ_OK) y = shaped(y);
   return gemm_result(y, rc);
   END_HANDLE_TH_ERRORS

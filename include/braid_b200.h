@@ -280,10 +280,12 @@ int bq_gated_rmsnorm_scale(const void* y, int y_dtype, int64_t ld_y, const void*
 /*
  * bq_quantize_act and bq_gemm_w8a8_grouped (or, with one weight, bq_gemm_w8a8_residual) in one launch for
  * few rows: x [M, K] of `dtype` (also the outputs' type), contiguous; every CTA quantizes it for itself.
- * The same bits as the two calls.  BQ_ERR_UNSUPPORTED beyond 16 rows or 64 KB of x.
+ * The same bits as the two calls.  BQ_ERR_UNSUPPORTED beyond BQ_LINEAR_MAX_ROWS rows and wherever the two calls
+ * are the faster form (64 KB of x at most; less for wide weights and while `stream` is captured).
  *
  * Replaces: braid/model/quant.py:244-252 (`fp8_linear`) at those sizes.
  */
+#define BQ_LINEAR_MAX_ROWS 16
 int bq_linear_w8a8(const void* x, int dtype, int64_t M, int64_t K, int n_seg, const void* const* wq,
                    const float* const* sw, const void* residual, int64_t ld_res, void* const* y,
                    const int64_t* N, const int64_t* ldy, void* ws, size_t ws_bytes, void* stream);
@@ -587,6 +589,8 @@ int bq_read_device_status(void* ws, void* stream, int* status_out);
  * bq_set_option("decode_wide", v)       decode batches on the CTA-pair kernel: -1 by size, 0 never, 1 always
  * bq_set_option("decode_cta_target", v) CTAs a small weight is sliced to reach (default 160)
  * bq_set_option("decode_smem_cap", v)   0 = none, else cap pipeline bytes per CTA
+ * bq_set_option("decode_quant_inside", v) few rows quantized inside the GEMM launch: -1 by size, 0 never, else up to
+ *                                       so many bytes of activation (<= 262144; same results either way)
  * bq_set_option("stream_max_m", v)      largest M the weight-streaming kernel takes (<= 256)
  * bq_set_option("gemm_pdl" | "quant_pdl", 0/1)  programmatic dependent launch
  * bq_set_option("quant_block" | "quant_held", v) quantizer launch shape overrides

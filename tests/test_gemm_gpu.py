@@ -593,6 +593,32 @@ def test_residual_epilogue_equals_gemm_then_add(Q, dt, M, N, K):
     assert torch.equal(got, want), f"{int((got != want).sum())} of {got.numel()} differ"
 
 
+@pytest.mark.parametrize("M,K,N,eager,captured", [(6, 4096, 4096, 1, 1), (8, 4096, 4096, 1, 2), (8, 4096, 2048, 1, 1),
+                                                  (5, 4096, 8192, 1, 1), (6, 4096, 8192, 1, 2), (6, 2048, 12288, 1, 1),
+                                                  (8, 2048, 12288, 1, 2), (8, 4096, 6144, 2, 2), (16, 2048, 12288, 2, 2),
+                                                  (1, 20480, 8192, 2, 2)])
+def test_linear_of_few_rows_in_one_launch_only_where_that_is_faster(Q, M, K, N, eager, captured):
+    """Both sides of each line of the rule, by 1, 2 and 4 K slices, eager and captured: the launches, and the
+    same bits either way."""
+    x = randn_cpu((M, K), seed=M).cuda()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    codes = torch.randint(0, 120, (N, K), generator=g, device="cuda", dtype=torch.uint8).view(Q.FP8)
+    fw = Q.FP8Weight(codes, torch.full((1, 1), 1e-3, device="cuda"), (N, K))
+    want = Q.fp8_matmul(*Q.quantize_act(x), fw)
+    n0 = Q.launch_count()
+    assert torch.equal(Q.linear(x, fw), want)
+    assert Q._NATIVE is None or Q.launch_count() - n0 == eager
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    n0 = Q.launch_count()
+    with torch.cuda.graph(graph):
+        y = Q.linear(x, fw)
+    assert Q._NATIVE is None or Q.launch_count() - n0 == captured
+    graph.replay()
+    assert torch.equal(y, want)
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("key,value,back", [("stream_max_m", 8, 256), ("decode_wide", 1, -1), ("decode_stages", 2, 0),
                                             ("decode_b_stages", 1, 0)])
 def test_linear_of_few_rows_leaves_forced_kernels_to_two_launches(Q, key, value, back):
