@@ -303,9 +303,10 @@ def _scratch_for(device_index: int) -> torch.Tensor:
                 buf = torch.zeros(_SLOTS * _SLOT_BYTES, dtype=torch.uint8,
                                   device=torch.device("cuda", device_index))
                 torch.cuda.synchronize(device_index)
-                _scratch[device_index] = buf
+                # the native calls first: whoever finds `buf` without the lock takes a slot from them
                 if _HOST is not None:
                     _HOST.set_scratch(device_index, buf.data_ptr())
+                _scratch[device_index] = buf
     return buf
 
 

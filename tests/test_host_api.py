@@ -174,6 +174,29 @@ def test_a_missing_library_is_loud(monkeypatch, tmp_path):
     assert quant.fused_state().startswith("unavailable: LibraryMissing")
 
 
+def test_scratch_is_published_after_the_native_calls_know_it(monkeypatch):
+    """A second thread that finds a device's scratch without the lock takes its slot from the native
+    counter at once, so that has to know the slots by then."""
+    from braid_b200 import quant
+    found = []
+
+    class Host:
+        def set_scratch(self, device, address):
+            found.append((device, address, device in quant._scratch))
+
+        def next_slot(self, device):
+            return 0
+
+    zeros = torch.zeros
+    monkeypatch.setattr(quant, "_HOST", Host())
+    monkeypatch.setattr(quant, "_scratch", {})
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
+    monkeypatch.setattr(torch, "zeros", lambda *size, device=None, **kw: zeros(*size, **kw))
+    buf = quant._scratch_for(3)
+    assert found == [(3, buf.data_ptr(), False)] and quant._scratch == {3: buf}
+
+
 def test_cpu_tensors_are_refused_not_emulated():
     from braid_b200 import quant
     x = torch.zeros(4, 16, dtype=torch.bfloat16)
