@@ -43,10 +43,33 @@ HOST_SRC = CSRC / "host_calls.cpp"
 HOST = PKG / "_host.so"
 
 
+HOST_MARK = b"braid_b200 native calls for "
+
+
+def host_key() -> str:
+    """The torch and the Python that the native calls have to be compiled against to run in this process."""
+    import sysconfig
+
+    import torch
+    return (f"torch {torch.__version__} ({torch.version.git_version}), cxx11 abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, "
+            f"{sysconfig.get_config_var('SOABI')}")
+
+
+def host_problem() -> str | None:
+    """Why the native calls cannot be loaded here, None if they can.  Looks at the file without loading it: the
+    code reads torch's objects by the layout it was compiled with, and another torch need not refuse it."""
+    if not HOST.exists():
+        return f"{HOST.name} is not built"
+    built = HOST.read_bytes()
+    at = built.find(HOST_MARK)
+    key = built[at + len(HOST_MARK):built.index(b"\0", at)].decode() if at >= 0 else "an unknown torch"
+    return None if key == host_key() else f"{HOST.name} was built for {key}; this is {host_key()}"
+
+
 def build_host(force: bool = False) -> Path:
     """Compile the native calls of quant.py against the torch that is installed."""
     deps = (HOST_SRC, PKG.parent / "include" / "braid_b200.h")
-    if not force and HOST.exists() and all(d.stat().st_mtime <= HOST.stat().st_mtime for d in deps):
+    if not force and host_problem() is None and all(d.stat().st_mtime <= HOST.stat().st_mtime for d in deps):
         return HOST
     import sysconfig
 
@@ -57,6 +80,7 @@ def build_host(force: bool = False) -> Path:
     includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
     cmd = ["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DBQ_HOST_KEY="{host_key()}"',
            *(arg for path in includes for arg in ("-isystem", path)),
            str(HOST_SRC), "-o", str(HOST), f"-L{torch_lib}",
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]

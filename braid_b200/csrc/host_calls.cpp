@@ -33,6 +33,14 @@
 
 #include "../../include/braid_b200.h"
 
+// What this file was compiled against: it reads fields of torch's and Python's objects by their layout there.  build.py
+// finds the text in the built file and leaves a file of another torch or Python unloaded.
+#ifndef BQ_HOST_KEY
+#error "compile with braid_b200/build.py"
+#endif
+extern "C" __attribute__((visibility("default"), used)) const char bq_host_built_for[] =
+    "braid_b200 native calls for " BQ_HOST_KEY;
+
 namespace {
 
 struct Lib {

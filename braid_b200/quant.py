@@ -224,6 +224,9 @@ def _load_host(lib) -> None:
     global _HOST
     if _HOST is not None:
         return
+    from . import build
+    if build.host_problem() is not None:
+        return
     try:
         from . import _host
     except ImportError:

@@ -174,6 +174,21 @@ def test_a_missing_library_is_loud(monkeypatch, tmp_path):
     assert quant.fused_state().startswith("unavailable: LibraryMissing")
 
 
+def test_native_calls_of_another_torch_are_not_loaded(lib, monkeypatch):
+    """The module reads torch's objects by the layout it was compiled with: a file of another torch or Python is
+    stale for the build and stays unloaded, also where it would load."""
+    from braid_b200 import build, quant
+    build.build_host()
+    assert build.host_problem() is None
+    here = build.host_key()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert here in build.host_problem() and build.host_key() in build.host_problem()
+    for name, value in (("_HOST", None), ("_NATIVE", None), ("_FUSED", None), ("_FUSED_STATE", "not tried")):
+        monkeypatch.setattr(quant, name, value)
+    assert quant.warm_fused(True)
+    assert quant._HOST is None and quant._NATIVE is None
+
+
 def test_scratch_is_published_after_the_native_calls_know_it(monkeypatch):
     """A second thread that finds a device's scratch without the lock takes its slot from the native
     counter at once, so that has to know the slots by then."""
