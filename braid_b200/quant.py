@@ -190,7 +190,7 @@ _launches = 0      # kernels of this library launched (or captured) so far
 # `csrc/host_calls.cpp`: the plain case of the calls below, checks, allocations and launch in one native
 # call (a launch from here costs about 18 us of host time, from there about 5; figures there).  Each returns None for
 # whatever is not plain, and the code below decides.  `_HOST` is the module, None where it cannot be
-# loaded (another torch build): everything then runs through the code below.  `_NATIVE` is the
+# loaded (`fused_state()` says why): everything then runs through the code below.  `_NATIVE` is the
 # same module while the kernels are active.
 _HOST = None
 _NATIVE = None
@@ -219,24 +219,27 @@ def launch_count() -> int:
     return _launches + (_HOST.launch_count() if _HOST is not None else 0)
 
 
-def _load_host(lib) -> None:
-    """Load the native calls once and give them the library's functions and the slots made so far."""
+def _load_host(lib) -> str | None:
+    """Load the native calls once and give them the library's functions and the slots made so far.  Returns
+    why they cannot be loaded, None if they are."""
     global _HOST
     if _HOST is not None:
-        return
+        return None
     from . import build
-    if build.host_problem() is not None:
-        return
+    problem = build.host_problem()
+    if problem is not None:
+        return problem
     try:
         from . import _host
-    except ImportError:
-        return
+    except ImportError as e:
+        return str(e).split(chr(10), 1)[0][:120]
     _host.init({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _lib.SIGNATURES},
                _SLOTS, _SLOT_BYTES, _TWO_LAUNCH_FROM)
     with _LOCK:
         for index, buf in _scratch.items():
             _host.set_scratch(index, buf.data_ptr())
         _HOST = _host
+    return None
 
 
 def warm_fused(enable: bool = True) -> bool:
@@ -245,9 +248,10 @@ def warm_fused(enable: bool = True) -> bool:
     Same contract as braid/model/quant.py:161-201: call it before any CUDA-graph
     capture; `warm_fused(False)` forces the torch spelling for the parity gate;
     the return value says whether the kernels are active and `fused_state()`
-    gives the one-line report.  Unlike the reference, a library that cannot be
-    loaded RAISES: there is no slower arm that would make a benchmark look
-    plausible without the kernels.
+    gives the one-line report: "active", or "active, calls from Python: <why>" where the
+    native calls cannot be loaded and an eager call takes up to three times as long.
+    Unlike the reference, a library that cannot be loaded RAISES: there is no slower arm
+    that would make a benchmark look plausible without the kernels.
     """
     global _FUSED, _FUSED_STATE, _NATIVE
     if not enable:
@@ -261,8 +265,9 @@ def warm_fused(enable: bool = True) -> bool:
         _FUSED = None
         _FUSED_STATE = f"unavailable: {type(e).__name__}: {str(e).split(chr(10), 1)[0][:120]}"
         raise
-    _load_host(lib)
-    _FUSED, _FUSED_STATE, _NATIVE = lib, "active", _HOST
+    problem = _load_host(lib)
+    state = "active" if problem is None else f"active, calls from Python: {problem}"
+    _FUSED, _FUSED_STATE, _NATIVE = lib, state, _HOST
     if torch.cuda.is_available():
         _scratch_for(torch.cuda.current_device())
     return True

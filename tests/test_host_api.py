@@ -187,6 +187,7 @@ def test_native_calls_of_another_torch_are_not_loaded(lib, monkeypatch):
         monkeypatch.setattr(quant, name, value)
     assert quant.warm_fused(True)
     assert quant._HOST is None and quant._NATIVE is None
+    assert quant.fused_state() == f"active, calls from Python: {build.host_problem()}"
 
 
 def test_scratch_is_published_after_the_native_calls_know_it(monkeypatch):
