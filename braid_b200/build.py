@@ -108,7 +108,7 @@ def build(force: bool = False, verbose: bool = False, defines: tuple[str, ...] =
         build_host(force)
     if out is None and not defines and not force and not is_stale():
         return LIB
-    LIB = out if out is not None else globals()["LIB"]
+    lib = out if out is not None else LIB
     cmd = [
         nvcc_path(), "-std=c++17", "-O3", "-lineinfo",
         "-gencode", "arch=compute_100a,code=sm_100a",
@@ -116,7 +116,7 @@ def build(force: bool = False, verbose: bool = False, defines: tuple[str, ...] =
         "--ftz=false", "--prec-div=true", "--prec-sqrt=true", "--fmad=true",
         "-cudart", "static",
         "-I", str(PKG.parent / "include"),
-        "-o", str(LIB),
+        "-o", str(lib),
     ]
     cmd += [f"-D{d}" for d in defines]
     if verbose or os.environ.get("BRAID_B200_VERBOSE") == "1":
@@ -127,7 +127,7 @@ def build(force: bool = False, verbose: bool = False, defines: tuple[str, ...] =
         raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
     if verbose:
         sys.stderr.write(proc.stdout + proc.stderr)
-    return LIB
+    return lib
 
 
 if __name__ == "__main__":

@@ -190,6 +190,13 @@ def test_native_calls_of_another_torch_are_not_loaded(lib, monkeypatch):
     assert quant.fused_state() == f"active, calls from Python: {build.host_problem()}"
 
 
+def test_a_build_that_is_current_is_returned(monkeypatch):
+    from braid_b200 import build
+    monkeypatch.setattr(build, "is_stale", lambda: False)
+    monkeypatch.setattr(build, "build_host", lambda force=False: build.HOST)
+    assert build.build() == build.LIB
+
+
 def test_scratch_is_published_after_the_native_calls_know_it(monkeypatch):
     """A second thread that finds a device's scratch without the lock takes its slot from the native
     counter at once, so that has to know the slots by then."""
