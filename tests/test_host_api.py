@@ -190,6 +190,25 @@ def test_native_calls_of_another_torch_are_not_loaded(lib, monkeypatch):
     assert quant.fused_state() == f"active, calls from Python: {build.host_problem()}"
 
 
+def test_the_library_is_built_without_the_native_calls(monkeypatch):
+    """No g++ or no torch headers: the library is compiled all the same, and the build says what is missing."""
+    import subprocess
+    from types import SimpleNamespace
+    from braid_b200 import build
+    ran = []
+
+    def run(cmd, **kw):
+        ran.append(cmd[0])
+        if cmd[0] == "g++":
+            raise FileNotFoundError("g++")
+        return SimpleNamespace(returncode=0, stdout="", stderr="")
+
+    monkeypatch.setattr(subprocess, "run", run)
+    with pytest.warns(UserWarning, match="native calls .* g\\+\\+"):
+        assert build.build(force=True) == build.LIB
+    assert len(ran) == 2 and ran[0].endswith("nvcc") and ran[1] == "g++"
+
+
 def test_a_build_that_is_current_is_returned(monkeypatch):
     from braid_b200 import build
     monkeypatch.setattr(build, "is_stale", lambda: False)
