@@ -100,7 +100,8 @@ __device__ __forceinline__ float warp_tree_sum(float s) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// plain RMSNorm -> quantize.  One CTA of 128 threads per row; VPT = vectors held per thread.
+// plain RMSNorm -> quantize.  One CTA per row, of G groups of 128 threads; VPT = vectors that a thread would hold
+// if it were 128 threads in all.
 // ---------------------------------------------------------------------------------------------
 template <typename T, int VPT, int G>
 __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(const NormParams p) {
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
   __shared__ float s_red_of[2][4];
-  __shared__ __align__(16) Vec4<T> s_x[G > 1 ? VPT * kNormThreads : 1];
+  __shared__ __align__(16) Vec4<T> s_x[G > 1 ? VPT * kNormThreads + 32 : 1];   // the last 32: the rehearsing warp's
   const RehearsingCta<G * kNormThreads> cta{threadIdx.x < G * kNormThreads};
   const bool live = cta.live;
   float* const s_red = s_red_of[cta.slot()];
@@ -172,16 +173,16 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
       }
     }
   } else {
-    // the sum's order is that of 128 threads: the first group walks the others' vectors
-    if (live) {
+    // the sum's order is that of 128 threads: the first group walks the others' vectors (the rehearsing warp,
+    // which passes no barrier with them, words of its own)
+    const int put = live ? vec(0) : VPT * kNormThreads + lane, get = live ? t : put, step = live ? kNormThreads : 0;
 #pragma unroll
-      for (int i = 0; i < VG; ++i) s_x[vec(i)] = x[i];
-    }
+    for (int i = 0; i < VG; ++i) s_x[put + i * step] = x[i];
     cta.sync();
     if (group == 0) {
       Vec4<T> all[VPT];
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) all[i] = s_x[t + i * kNormThreads];
+      for (int i = 0; i < VPT; ++i) all[i] = s_x[get + i * step];
 #pragma unroll
       for (int i = 0; i < VPT; ++i) {
         if (t + i * kNormThreads < n_vec) {
