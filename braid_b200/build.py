@@ -23,6 +23,7 @@ import shutil
 import subprocess
 import sys
 import warnings
+from importlib.machinery import EXTENSION_SUFFIXES
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -49,11 +50,9 @@ HOST_MARK = b"braid_b200 native calls for "
 
 def host_key() -> str:
     """The torch and the Python that the native calls have to be compiled against to run in this process."""
-    import sysconfig
-
     import torch
     return (f"torch {torch.__version__} ({torch.version.git_version}), cxx11 abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, "
-            f"{sysconfig.get_config_var('SOABI')}")
+            f"python{EXTENSION_SUFFIXES[0]}")
 
 
 def host_problem() -> str | None:
