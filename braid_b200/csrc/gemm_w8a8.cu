@@ -2081,6 +2081,8 @@ int launch_pair(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
   int pairs = p.total_tiles < sms / 2 ? p.total_tiles : sms / 2;
   if (pairs < 1) pairs = 1;
   const int epi = epilogue_of(p, true);
+  // the general form of this kernel is the column-parallel one's: it adds no residual
+  if (epi == kAny && p.push.n == 0) return kErrUnsupported;
   if (p.push.n > 0) p.push.expected = (unsigned)(2 * pairs);   // every CTA has a tile and stores
   g_last_launch[0] = 2; g_last_launch[1] = 2 * pairs; g_last_launch[2] = 2;
   g_last_launch[3] = kPairStages; g_last_launch[4] = smem; g_last_launch[5] = p.pair.on ? kPairTile : p.seg[0].un;
