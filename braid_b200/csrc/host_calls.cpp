@@ -388,10 +388,6 @@ PyObject* gemm_result(const at::Tensor& y, int rc) {
   return wrap(y);
 }
 
-at::Tensor as_rows(const at::Tensor& t, int64_t cols) {     // undefined stays undefined
-  return !t.defined() || t.dim() == 2 ? t : t.reshape({-1, cols});
-}
-
 // linear(x, w, sw, residual or None): quantize, multiply, leading dimensions kept.  Few rows: one launch.
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
@@ -512,7 +508,6 @@ PyObject* project(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     N[i] = w.size(0);
   }
   const void* dp = nullptr;
-  at::Tensor d2;
   if (mixed) {
     if (!dense.defined() || !plain(h, dense) || dense.scalar_type() != out || code == BQ_DTYPE_F32 ||
         !dense.is_contiguous() || dense.numel() != M * K || !aligned(dense.data_ptr(), 16) || (M > 256 && recorded(dense)))
