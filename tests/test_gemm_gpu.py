@@ -593,6 +593,25 @@ def test_residual_epilogue_equals_gemm_then_add(Q, dt, M, N, K):
     assert torch.equal(got, want), f"{int((got != want).sum())} of {got.numel()} differ"
 
 
+def test_linear_of_few_rows_over_several_weights(Q):
+    """The entry point takes several weights, of one and of four K slices: each output has the bits of its own
+    launch."""
+    import ctypes
+    from braid_b200 import _lib
+    M, K, Ns = 5, 1024, (12288, 272, 16)
+    ws = [Q.quantize_weight(randn_cpu((n, K), seed=n, scale=0.02).cuda()) for n in Ns]
+    x = randn_cpu((M, K), seed=1).cuda()
+    ys = [torch.empty(M, n, device="cuda", dtype=x.dtype) for n in Ns]
+    ptrs = lambda ts: (ctypes.c_void_p * 3)(*[t.data_ptr() for t in ts])  # noqa: E731
+    n = (ctypes.c_int64 * 3)(*Ns)
+    _lib.check(_lib.load().bq_linear_w8a8(x.data_ptr(), 1, M, K, 3, ptrs([w.data for w in ws]), ptrs([w.scale for w in ws]),
+                                          None, 0, ptrs(ys), n, n, Q._take_slot(x.device), 16, Q._stream_ptr(x.device)),
+               "linear")
+    xq, sx = Q.quantize_act(x)
+    assert all(torch.equal(y, Q.fp8_matmul(xq, sx, w)) for y, w in zip(ys, ws))
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("M,K,N,eager,captured", [(6, 4096, 4096, 1, 1), (8, 4096, 4096, 1, 2), (8, 4096, 2048, 1, 1),
                                                   (5, 4096, 8192, 1, 1), (6, 4096, 8192, 1, 2), (6, 2048, 12288, 1, 1),
                                                   (8, 2048, 12288, 1, 2), (8, 4096, 6144, 2, 2), (16, 2048, 12288, 2, 2),
