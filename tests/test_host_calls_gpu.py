@@ -136,7 +136,9 @@ def test_what_torch_follows_above_256_rows_stays_a_torch_operation(Q, weights):
 
 def test_native_calls_from_threads_and_streams(Q, weights):
     """Slots are counted in one place whichever way a call takes; threads on their own streams get the
-    bits of a lone call."""
+    bits of a lone call.  Small projections alone: their launches do not wait for one another's CTAs.  Launches
+    that do (norms, larger quantizers, gate/up) are for one stream per device, and at most 256 launches may be in
+    flight before a slot is taken again."""
     import threading
     w, x = weights, randn_cpu((4, 512), seed=1).cuda()
     want = Q.mlp_forward(x, w["gate"], w["up"], w["down"])
