@@ -18,9 +18,9 @@
 // rounds once more.  tests/test_norm_quant_gpu.py pins all of this against torch on the device.
 //
 // After the norm the values stay in registers; amax, grid-wide exchange and cast are the
-// activation quantizer's (quant_act.cu).  One CTA per token row, so grids are <= 2048 rows
-// (all CTAs must be co-resident for the exchange); larger inputs are refused and the caller runs
-// the norm and the quantizer separately.
+// activation quantizer's (quant_act.cu).  One CTA per token row, all of them co-resident for the exchange;
+// larger inputs are refused, and the caller takes the norm with its rows looped (bq_rmsnorm_scale,
+// bq_gated_rmsnorm_scale) and the cast pass.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -143,9 +143,9 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
   // 27 rows 286 -> 281 -> 274, 128 rows 333 -> 323 -> 317; hidden 5120, 64 rows 434 -> 435 -> 421.  32 warps
   // in the gated kernel gave no more.
   //
-  // A further warp rehearses: it runs the same instructions on zeros, without a load, store or exchange,
-  // while the others wait for the previous kernel, and they find the code in the instruction cache, where
-  // the previous kernel's code was.  A warp of its own, because there may be nothing to wait for (behind a
+  // A further warp rehearses: it runs the same instructions on zeros and words of its own, without an access to
+  // global memory and without the exchange, while the others wait for the previous kernel, and they find the
+  // code in the instruction cache, where the previous kernel's code was.  A warp of its own, because there may be nothing to wait for (behind a
   // kernel that was not launched with early starts).  Only up to kRehearseRows rows: beyond, the
   // rehearsal competes with the GEMM that is waited for.
   Vec4<T> x[VG];
