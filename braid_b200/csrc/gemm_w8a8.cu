@@ -640,34 +640,33 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   }
 
   if (warp == 0) {
-    if (elect_one()) {
-      // Weights do not depend on any earlier kernel: this thread never waits for the kernel
-      // that produces the activation, it only follows the MMAs through the weight ring.
-      // weights are read once: evict first
-      const uint64_t pol_w = policy_evict_first();
-      // one 128-row box, or (paired gate/up) two 64-row boxes from the two weights
-      const bool paired = pair_on;
-      const int half_row0 = tile_in_seg * (kRowTile / 2);
-      // slot and phase are carried along: an integer division by a run-time depth costs a
-      // single issuing thread more than the loads it issues
-      int s = 0;
-      uint32_t phase = 1;                      // parity of the completion that frees slot s
-      for (int i = 0; i < kb_count; ++i) {
-        if (i >= p.stages && !mbar_wait(empty_bar(s), phase)) {
-          *abort_flag = 1;
-          break;
-        }
-        mbar_expect_tx(full_bar(s), kATileBytes);
-        const int kx = (kb_begin + i) * kBK;
-        const uint32_t dst = a_base + s * kATileBytes;
-        if (paired) {
-          tma_load_2d(dst, &tm_w.w[0], full_bar(s), kx, half_row0, pol_w);
-          tma_load_2d(dst + kATileBytes / 2, &tm_w.w[1], full_bar(s), kx, half_row0, pol_w);
-        } else {
-          tma_load_2d(dst, &tm_w.w[sg], full_bar(s), kx, row0, pol_w);
-        }
-        if (++s == p.stages) { s = 0; phase ^= 1u; }
+    // Weights do not depend on any earlier kernel: this warp never waits for the kernel that produces the
+    // activation, it only follows the MMAs through the weight ring.  See ptx.cuh for why the whole warp
+    // walks the loop.  Weights are read once: evict first.
+    const uint32_t issue = elect_one() ? 1u : 0u;
+    const uint64_t pol_w = policy_evict_first();
+    // one 128-row box, or (paired gate/up) two 64-row boxes from the two weights
+    const bool paired = pair_on;
+    const int half_row0 = tile_in_seg * (kRowTile / 2);
+    // slot and phase are carried along: an integer division by a run-time depth costs a
+    // single issuing thread more than the loads it issues
+    int s = 0;
+    uint32_t phase = 1;                      // parity of the completion that frees slot s
+    for (int i = 0; i < kb_count; ++i) {
+      if (i >= p.stages && !mbar_wait(empty_bar(s), phase)) {
+        *abort_flag = 1;
+        break;
       }
+      mbar_expect_tx(issue, full_bar(s), kATileBytes);
+      const int kx = (kb_begin + i) * kBK;
+      const uint32_t dst = a_base + s * kATileBytes;
+      if (paired) {
+        tma_load_2d(issue, dst, &tm_w.w[0], full_bar(s), kx, half_row0, pol_w);
+        tma_load_2d(issue, dst + kATileBytes / 2, &tm_w.w[1], full_bar(s), kx, half_row0, pol_w);
+      } else {
+        tma_load_2d(issue, dst, &tm_w.w[sg], full_bar(s), kx, row0, pol_w);
+      }
+      if (++s == p.stages) { s = 0; phase ^= 1u; }
     }
     __syncwarp();
   } else if (QUANT && warp >= 2) {
@@ -685,59 +684,66 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     }
     __syncwarp();
   } else if (warp == 2) {
-    if (elect_one()) {
-      // the activation tile is shared by every row tile: keep it in L2
-      const uint64_t pol_x = policy_evict_last();
-      pdl_wait_prior_grids();   // the kernel that produces the activation has completed
-      BQ_STAMP(p, 2);
-      // Activation slot s was last read by the MMAs of block j = i - b_stages, whose completion
-      // is completion number j / stages of weight slot j % stages.  That barrier cannot complete
-      // a second time before this thread has looked: block j + stages >= i needs THIS load first
-      // (the host keeps b_stages <= stages).
-      int s = 0, js = 0;                       // activation slot of block i, weight slot of block j
-      uint32_t jphase = 0;                     // parity of completion j / stages
-      for (int i = 0; i < kb_count; ++i) {
-        if (i >= p.b_stages) {
-          if (!mbar_wait(empty_bar(js), jphase)) {
-            *abort_flag = 1;
-            break;
-          }
-          if (++js == p.stages) { js = 0; jphase ^= 1u; }
-        }
-        mbar_expect_tx(full_bar_b(s), b_tile_bytes);
-        tma_load_2d(b_base + s * b_tile_bytes, x_map, full_bar_b(s), (kb_begin + i) * kBK, 0, pol_x);
-        if (++s == p.b_stages) s = 0;
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (elect_one()) {
-      const uint32_t idesc = dense ? idesc_f16(kRowTile, p.mma_n, p.dense_fmt)
-                                   : idesc_e4m3(kRowTile, p.mma_n);
-      int s = 0, sb = 0;
-      uint32_t phase = 0, phase_b = 0;
-      for (int i = 0; i < kb_count; ++i) {
-        if (!mbar_wait(full_bar(s), phase) || ((!QUANT || i == 0) && !mbar_wait(full_bar_b(sb), phase_b))) {
+    // the activation tile is shared by every row tile: keep it in L2
+    const uint32_t issue = elect_one() ? 1u : 0u;
+    const uint64_t pol_x = policy_evict_last();
+    pdl_wait_prior_grids();   // the kernel that produces the activation has completed
+    if (issue) BQ_STAMP(p, 2);
+    // Activation slot s was last read by the MMAs of block j = i - b_stages, whose completion
+    // is completion number j / stages of weight slot j % stages.  That barrier cannot complete
+    // a second time before this thread has looked: block j + stages >= i needs THIS load first
+    // (the host keeps b_stages <= stages).
+    int s = 0, js = 0;                       // activation slot of block i, weight slot of block j
+    uint32_t jphase = 0;                     // parity of completion j / stages
+    for (int i = 0; i < kb_count; ++i) {
+      if (i >= p.b_stages) {
+        if (!mbar_wait(empty_bar(js), jphase)) {
           *abort_flag = 1;
           break;
         }
+        if (++js == p.stages) { js = 0; jphase ^= 1u; }
+      }
+      mbar_expect_tx(issue, full_bar_b(s), b_tile_bytes);
+      tma_load_2d(issue, b_base + s * b_tile_bytes, x_map, full_bar_b(s), (kb_begin + i) * kBK, 0, pol_x);
+      if (++s == p.b_stages) s = 0;
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    const uint32_t issue = elect_one() ? 1u : 0u;
+    const uint32_t idesc = dense ? idesc_f16(kRowTile, p.mma_n, p.dense_fmt)
+                                 : idesc_e4m3(kRowTile, p.mma_n);
+    auto multiply = [&](auto is_dense) {
+      int s = 0, sb = 0;
+      uint32_t phase = 0, phase_b = 0;
+      bool ready = false, ready_b = false;
+      for (int i = 0; i < kb_count; ++i) {
+        if ((!ready && !mbar_wait(full_bar(s), phase)) ||
+            ((!QUANT || i == 0) && !ready_b && !mbar_wait(full_bar_b(sb), phase_b))) {
+          *abort_flag = 1;
+          break;
+        }
+        const uint32_t a_tile = a_base + s * kATileBytes, b_tile = b_base + sb * b_tile_bytes, empty = empty_bar(s);
+        if (++s == p.stages) { s = 0; phase ^= 1u; }
+        if (++sb == p.b_stages) { sb = 0; phase_b ^= 1u; }
+        // look at the next block's barriers now: the answers arrive while this block's MMAs are issued
+        ready = mbar_test(full_bar(s), phase);
+        if (!QUANT) ready_b = mbar_test(full_bar_b(sb), phase_b);
         tc_fence_after();
-        if (i == 0) BQ_STAMP(p, 3);
-        const uint64_t da = smem_desc_sw128(a_base + s * kATileBytes);
-        const uint64_t db = smem_desc_sw128(b_base + sb * b_tile_bytes);
+        if (issue && i == 0) BQ_STAMP(p, 3);
+        const uint64_t da = smem_desc_sw128(a_tile), db = smem_desc_sw128(b_tile);
 #pragma unroll
         for (int j = 0; j < kBK / kUmmaK; ++j) {
           // +32 bytes along K inside the swizzle span = +2 in descriptor units (32 e4m3 or 16
           // 16-bit elements: one MMA's K either way)
-          if (dense) mma_f16(tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
-          else mma_f8(tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
+          if constexpr (is_dense.value) mma_f16(issue, tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
+          else mma_f8(issue, tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
         }
-        mma_commit(empty_bar(s));   // both slots are free once these MMAs retire
-        if (++s == p.stages) { s = 0; phase ^= 1u; }
-        if (++sb == p.b_stages) { sb = 0; phase_b ^= 1u; }
+        mma_commit(issue, empty);   // both slots are free once these MMAs retire
       }
-      mma_commit(accum_bar);        // accumulator complete
-    }
+    };
+    if (dense) multiply(std::true_type{});
+    else multiply(std::false_type{});
+    mma_commit(issue, accum_bar);     // accumulator complete
     __syncwarp();
   }
 
@@ -1303,40 +1309,43 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   pdl_wait_prior_grids();
 
   if (warp == 0) {
-    if (elect_one()) {
-      const uint64_t pol = policy_evict_last();
-      int it = 0;
-      bool ok = true;
-      for (int t = pair; t < p.total_tiles && ok; t += n_pairs) {
-        const int sg = find_segment(p, t);
-        const int local = t - p.seg[sg].tile_begin;
-        const bool dense = EPI == kMixed && p.seg[sg].dense != 0;
-        int m_idx, n_idx;
-        const int n_step = tile_cols(p.seg[sg]);
-        pair_tile_coords(local, m_tiles, (p.seg[sg].n + n_step - 1) / n_step, m_idx, n_idx);
-        const int m0 = m_idx * kPairTile + rank * kRowTile;
-        // plain: this CTA's half of the tile's weight rows; SiLU form: the leader loads 128
-        // gate rows, its peer the 128 up rows of the same output columns
-        const int rows = silu ? kRowTile : n_step / 2;
-        const int n0 = silu ? n_idx * kRowTile : n_idx * n_step + rank * rows;
-        const CUtensorMap* const w_map = silu ? &tm_w.w[rank] : &tm_w.w[sg];
-        const CUtensorMap* const x_map = dense ? &tm_xd : &tm_x;
-        const int blocks = dense ? p.k_blocks_dense : p.k_blocks;
-        for (int kb = 0; kb < blocks; ++kb, ++it) {
-          const int s = it % kPairStages, use = it / kPairStages;
-          if (use > 0 && !mbar_wait(empty_bar(s), (use - 1) & 1)) { ok = false; break; }
-          if (rank == 0) mbar_expect_tx(full_bar(s), 2u * (kATileBytes + (uint32_t)rows * kBK));
-          tma_load_2d_pair(a_tile(s), x_map, full_bar(s), kb * kBK, m0, pol);
-          tma_load_2d_pair(b_tile(s), w_map, full_bar(s), kb * kBK, n0, pol);
-        }
+    const uint32_t issue = elect_one() ? 1u : 0u, expect = rank == 0 ? issue : 0u;
+    const uint64_t pol = policy_evict_last();
+    int s = 0;
+    uint32_t phase = 1;                          // a fresh barrier counts as completed
+    bool ok = true;
+    for (int t = pair; t < p.total_tiles && ok; t += n_pairs) {
+      const int sg = find_segment(p, t);
+      const int local = t - p.seg[sg].tile_begin;
+      const bool dense = EPI == kMixed && p.seg[sg].dense != 0;
+      int m_idx, n_idx;
+      const int n_step = tile_cols(p.seg[sg]);
+      pair_tile_coords(local, m_tiles, (p.seg[sg].n + n_step - 1) / n_step, m_idx, n_idx);
+      const int m0 = m_idx * kPairTile + rank * kRowTile;
+      // plain: this CTA's half of the tile's weight rows; SiLU form: the leader loads 128
+      // gate rows, its peer the 128 up rows of the same output columns
+      const int rows = silu ? kRowTile : n_step / 2;
+      const int n0 = silu ? n_idx * kRowTile : n_idx * n_step + rank * rows;
+      const CUtensorMap* const w_map = silu ? &tm_w.w[rank] : &tm_w.w[sg];
+      const CUtensorMap* const x_map = dense ? &tm_xd : &tm_x;
+      const int blocks = dense ? p.k_blocks_dense : p.k_blocks;
+      const uint32_t bytes = 2u * (kATileBytes + (uint32_t)rows * kBK);
+      for (int kb = 0; kb < blocks; ++kb) {
+        if (!mbar_wait(empty_bar(s), phase)) { ok = false; break; }
+        mbar_expect_tx(expect, full_bar(s), bytes);
+        tma_load_2d_pair(issue, a_tile(s), x_map, full_bar(s), kb * kBK, m0, pol);
+        tma_load_2d_pair(issue, b_tile(s), w_map, full_bar(s), kb * kBK, n0, pol);
+        if (++s == kPairStages) { s = 0; phase ^= 1u; }
       }
-      if (!ok) *abort_flag = 1;
     }
+    if (!ok) *abort_flag = 1;
     __syncwarp();
   } else if (warp == 1) {
-    if (rank == 0 && elect_one()) {
-      int it = 0, tile_iter = 0;
-      bool ok = true;
+    if (rank == 0) {
+      const uint32_t issue = elect_one() ? 1u : 0u;
+      int s = 0, tile_iter = 0;
+      uint32_t phase = 0;
+      bool ok = true, ready = false;
       for (int t = pair; t < p.total_tiles && ok; t += n_pairs, ++tile_iter) {
         const int b = tile_iter & 1, use_b = tile_iter >> 1;
         if (use_b > 0 && !mbar_wait(acc_empty(b), (use_b - 1) & 1)) { ok = false; break; }
@@ -1349,30 +1358,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         const int blocks = dense ? p.k_blocks_dense : p.k_blocks;
         // one loop per operand kind: a choice inside it cost every tile of a mixed launch 8 %
         auto multiply = [&](auto is_dense) {
-          for (int kb = 0; kb < blocks; ++kb, ++it) {
-            const int s = it % kPairStages, use = it / kPairStages;
-            if (!mbar_wait(full_bar(s), use & 1)) { ok = false; break; }
+          for (int kb = 0; kb < blocks; ++kb) {
+            if (!ready && !mbar_wait(full_bar(s), phase)) { ok = false; break; }
+            const uint64_t da = smem_desc_sw128(a_tile(s)), db = smem_desc_sw128(b_tile(s));
+            const uint32_t empty = empty_bar(s);
+            if (++s == kPairStages) { s = 0; phase ^= 1u; }
+            // look at the next stage's barrier now: the answer arrives while this one's MMAs are issued
+            ready = mbar_test(full_bar(s), phase);
             tc_fence_after();
-            const uint64_t da = smem_desc_sw128(a_tile(s));
-            const uint64_t db = smem_desc_sw128(b_tile(s));
 #pragma unroll
             for (int j = 0; j < kBK / kUmmaK; ++j) {
               if constexpr (is_dense.value)
-                mma_f16_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
+                mma_f16_pair(issue, tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
               else
-                mma_f8_pair(tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
+                mma_f8_pair(issue, tmem_d, da + 2u * j, db + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
             }
-            // the stage is free in BOTH CTAs once these MMAs retire
-            mma_commit_pair(empty_bar(s));
-            mma_commit_pair(map_to_cta(empty_bar(s), 1));
+            mma_commit_pair(issue, empty);   // the stage is free in BOTH CTAs once these MMAs retire
           }
         };
         if (EPI == kMixed && dense) multiply(std::true_type{});
         else multiply(std::false_type{});
-        if (ok) {
-          mma_commit_pair(acc_full(b));
-          mma_commit_pair(map_to_cta(acc_full(b), 1));
-        }
+        if (ok) mma_commit_pair(issue, acc_full(b));
       }
       if (!ok) *abort_flag = 1;
     }

@@ -334,7 +334,8 @@ struct RingPos {
 // are template parameters, descriptors are one 64-bit add.
 template <int MODE, bool DENSE, int NM>
 __device__ __forceinline__ bool issue_unit(const GemmParams& p, const RingShape& sh, const Segment& seg, RingPos& pos,
-                                           uint32_t bar_base, uint32_t a_base, uint32_t w_base, uint32_t d) {
+                                           uint32_t bar_base, uint32_t a_base, uint32_t w_base, uint32_t d,
+                                           uint32_t issue) {
   const uint32_t idesc = DENSE ? idesc_f16(LaneMap<MODE>::kMmaM, seg.un, p.dense_fmt)
                                : idesc_e4m3(LaneMap<MODE>::kMmaM, seg.un);
   const int cols = LaneMap<MODE>::cols(seg.un);
@@ -370,8 +371,8 @@ __device__ __forceinline__ bool issue_unit(const GemmParams& p, const RingShape&
           // +32 bytes along K inside the swizzle span = +2 in descriptor units (32 e4m3 or 16
           // 16-bit elements: one MMA's K either way)
           const uint32_t accumulate = q == 0 ? acc : 1u;
-          if constexpr (DENSE) mma_f16_pair(dst, da + 2u * q, dh + 2u * q, idesc, accumulate);
-          else mma_f8_pair(dst, da + 2u * q, dh + 2u * q, idesc, accumulate);
+          if constexpr (DENSE) mma_f16_pair(issue, dst, da + 2u * q, dh + 2u * q, idesc, accumulate);
+          else mma_f8_pair(issue, dst, da + 2u * q, dh + 2u * q, idesc, accumulate);
         }
       }
       da += a_blk;
@@ -384,8 +385,7 @@ __device__ __forceinline__ bool issue_unit(const GemmParams& p, const RingShape&
       }
     }
     // both slots are free, in both CTAs of a pair, once these MMAs retire
-    mma_commit_pair(empty);
-    mma_commit_pair(map_to_cta(empty, 1));
+    mma_commit_pair(issue, empty);
   }
   return true;
 }
@@ -461,69 +461,68 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   tc_fence_after();
 
   if (warp == 0) {
-    if (lane == 0) {
-      // Weights do not depend on any earlier kernel: this thread never waits for the kernel that
-      // produces the activation, it only follows the MMAs through the ring.  Read once: evict
-      // first.  Slot and phase are carried along: an integer division by a run-time depth costs a
-      // single issuing thread more than the loads it issues.
-      const uint64_t pol_w = policy_evict_first();
-      int s = 0;
-      uint32_t phase = 1;                      // a fresh barrier counts as completed
-      bool ok = true;
-      for (int unit = unit0; unit < sh.units && ok; unit += unit_step) {
-        const int sg = segment_of(unit);
-        const Segment& seg = p.seg[sg];
-        const int box = seg.un / 2;            // weight rows of one box
-        const int row = (unit - seg.unit_begin) * seg.un + crank * box;
-        const CUtensorMap* const map = &tm_w.w[sg];
-        const uint32_t half = rs.kb_stage * box * kBK;         // bytes of one box
-        const int blocks = seg.dense ? p.k_blocks_dense : p.k_blocks;
-        for (int kb = 0; kb < blocks; kb += rs.kb_stage) {
-          if (!mbar_wait(empty_w(s), phase)) { ok = false; break; }
-          if (crank == 0) mbar_expect_tx(full_w(s), 2 * sh.nm * half);
-          const uint32_t dst = w_base + s * w_bytes;
-          const int x = sh.flat ? kb * kBK : 0, z = sh.flat ? 0 : kb;
-          tma_load_3d_pair(dst, map, full_w(s), x, row, z, pol_w);
-          if (paired) tma_load_3d_pair(dst + half, &tm_w.w[1], full_w(s), x, row, z, pol_w);
-          if (++s == rs.w_stages) { s = 0; phase ^= 1u; }
-        }
+    // Weights do not depend on any earlier kernel: this warp never waits for the kernel that
+    // produces the activation, it only follows the MMAs through the ring.  Read once: evict
+    // first.  Slot and phase are carried along: an integer division by a run-time depth costs a
+    // single issuing thread more than the loads it issues.
+    const uint32_t issue = elect_one() ? 1u : 0u, expect = crank == 0 ? issue : 0u;
+    const uint64_t pol_w = policy_evict_first();
+    int s = 0;
+    uint32_t phase = 1;                      // a fresh barrier counts as completed
+    bool ok = true;
+    for (int unit = unit0; unit < sh.units && ok; unit += unit_step) {
+      const int sg = segment_of(unit);
+      const Segment& seg = p.seg[sg];
+      const int box = seg.un / 2;            // weight rows of one box
+      const int row = (unit - seg.unit_begin) * seg.un + crank * box;
+      const CUtensorMap* const map = &tm_w.w[sg];
+      const uint32_t half = rs.kb_stage * box * kBK;         // bytes of one box
+      const int blocks = seg.dense ? p.k_blocks_dense : p.k_blocks;
+      for (int kb = 0; kb < blocks; kb += rs.kb_stage) {
+        if (!mbar_wait(empty_w(s), phase)) { ok = false; break; }
+        mbar_expect_tx(expect, full_w(s), 2 * sh.nm * half);
+        const uint32_t dst = w_base + s * w_bytes;
+        const int x = sh.flat ? kb * kBK : 0, z = sh.flat ? 0 : kb;
+        tma_load_3d_pair(issue, dst, map, full_w(s), x, row, z, pol_w);
+        if (paired) tma_load_3d_pair(issue, dst + half, &tm_w.w[1], full_w(s), x, row, z, pol_w);
+        if (++s == rs.w_stages) { s = 0; phase ^= 1u; }
       }
-      if (!ok) *abort_flag = 1;
     }
+    if (!ok) *abort_flag = 1;
     __syncwarp();
   } else if (warp == 2) {
-    if (lane == 0) {
-      // the activation is shared by every unit: keep it in L2
-      const uint64_t pol_x = policy_evict_last();
-      pdl_wait_prior_grids();   // the kernel that produces the activation has completed
-      BQ_STAMP(p, 2);
-      // Activation slot s was last read by the MMAs of stage j = i - a_stages, whose completion is
-      // completion number j / w_stages of weight slot j % w_stages.  That barrier cannot complete
-      // a second time before this thread has looked: stage j + w_stages >= i needs THIS load
-      // first (the host keeps a_stages <= w_stages).
-      int s = 0, js = 0, i = 0;
-      uint32_t jphase = 0;
-      bool ok = true;
-      for (int unit = unit0; unit < sh.units && ok; unit += unit_step) {
-        const Segment& seg = p.seg[segment_of(unit)];
-        const CUtensorMap* const map = seg.dense ? &tm_xd : &tm_x;
-        const int blocks = seg.dense ? p.k_blocks_dense : p.k_blocks;
-        for (int kb = 0; kb < blocks; kb += rs.kb_stage, ++i) {
-          if (i >= rs.a_stages) {
-            if (!mbar_wait(empty_w(js), jphase)) { ok = false; break; }
-            if (++js == rs.w_stages) { js = 0; jphase ^= 1u; }
-          }
-          if (crank == 0) mbar_expect_tx(full_a(s), 2 * a_bytes);
-          const int x = sh.flat ? kb * kBK : 0, z = sh.flat ? 0 : kb;
-          tma_load_3d_pair(a_base + s * a_bytes, map, full_a(s), x, m0, z, pol_x);
-          if (++s == rs.a_stages) s = 0;
+    // the activation is shared by every unit: keep it in L2
+    const uint32_t issue = elect_one() ? 1u : 0u, expect = crank == 0 ? issue : 0u;
+    const uint64_t pol_x = policy_evict_last();
+    pdl_wait_prior_grids();   // the kernel that produces the activation has completed
+    if (issue) BQ_STAMP(p, 2);
+    // Activation slot s was last read by the MMAs of stage j = i - a_stages, whose completion is
+    // completion number j / w_stages of weight slot j % w_stages.  That barrier cannot complete
+    // a second time before this thread has looked: stage j + w_stages >= i needs THIS load
+    // first (the host keeps a_stages <= w_stages).
+    int s = 0, js = 0, i = 0;
+    uint32_t jphase = 0;
+    bool ok = true;
+    for (int unit = unit0; unit < sh.units && ok; unit += unit_step) {
+      const Segment& seg = p.seg[segment_of(unit)];
+      const CUtensorMap* const map = seg.dense ? &tm_xd : &tm_x;
+      const int blocks = seg.dense ? p.k_blocks_dense : p.k_blocks;
+      for (int kb = 0; kb < blocks; kb += rs.kb_stage, ++i) {
+        if (i >= rs.a_stages) {
+          if (!mbar_wait(empty_w(js), jphase)) { ok = false; break; }
+          if (++js == rs.w_stages) { js = 0; jphase ^= 1u; }
         }
+        mbar_expect_tx(expect, full_a(s), 2 * a_bytes);
+        const int x = sh.flat ? kb * kBK : 0, z = sh.flat ? 0 : kb;
+        tma_load_3d_pair(issue, a_base + s * a_bytes, map, full_a(s), x, m0, z, pol_x);
+        if (++s == rs.a_stages) s = 0;
       }
-      if (!ok) *abort_flag = 1;
     }
+    if (!ok) *abort_flag = 1;
     __syncwarp();
   } else if (warp == 1) {
-    if (crank == 0 && elect_one()) {
+    if (crank == 0) {
+      const uint32_t issue = elect_one() ? 1u : 0u;
       const uint32_t tmem = *tmem_slot;
       RingPos pos;
       int round = 0;
@@ -534,11 +533,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         if (round >= 2 && !mbar_wait(acc_empty(b), ((round >> 1) - 1) & 1)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem + b * sh.acc_cols;
-        if (paired) ok = issue_unit<MODE, false, 2>(p, rs, seg, pos, bar_base, a_base, w_base, d);
-        else if (seg.dense) ok = issue_unit<MODE, true, 1>(p, rs, seg, pos, bar_base, a_base, w_base, d);
-        else ok = issue_unit<MODE, false, 1>(p, rs, seg, pos, bar_base, a_base, w_base, d);
-        mma_commit_pair(acc_full(b));
-        mma_commit_pair(map_to_cta(acc_full(b), 1));
+        if (paired) ok = issue_unit<MODE, false, 2>(p, rs, seg, pos, bar_base, a_base, w_base, d, issue);
+        else if (seg.dense) ok = issue_unit<MODE, true, 1>(p, rs, seg, pos, bar_base, a_base, w_base, d, issue);
+        else ok = issue_unit<MODE, false, 1>(p, rs, seg, pos, bar_base, a_base, w_base, d, issue);
+        mma_commit_pair(issue, acc_full(b));
       }
       if (!ok) *abort_flag = 1;
     }

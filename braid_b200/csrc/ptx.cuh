@@ -52,6 +52,15 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx(uint32_t issue, uint32_t bar, uint32_t bytes) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "setp.ne.b32 e, %2, 0;\n"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+      "}\n" ::"r"(bar), "r"(bytes), "r"(issue)
+      : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -104,18 +113,31 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
   return p;
 }
 
+// ---- instructions that one thread issues ------------------------------------------
+// TMA copies, MMAs and commits take an `issue` operand and are predicated on it: the whole warp walks the
+// issuing loop in step and one elected lane issues.  Their operands live in uniform registers; inside
+// `if (elect_one())` every descriptor was moved there lane-wise first.  Clocks of the MMA warp per K block of the
+// K-sliced decode kernel, all tiles in shared memory: 390 inside the branch (50 for an MMA, 45 for the commit, 60 for
+// each of two barriers that had completed), 275 in step (16, 40, 85), of which the barriers are taken off the
+// path by looking at the next block's before this one's MMAs.  Four graphed decoder layers of hidden 4096:
+// 1 row 233.0 -> 216.5 us, 27 rows 277.9 -> 265.2, 128 rows 317.4 -> 313.2.
+
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tm) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tm) : "memory");
 }
 // 2-D tiled load into this CTA's shared memory; x is the innermost (K, bytes for
 // u8 tensors) coordinate and must be a multiple of 16.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, uint32_t bar,
+__device__ __forceinline__ void tma_load_2d(uint32_t issue, uint32_t dst, const CUtensorMap* tm, uint32_t bar,
                                             int x, int y, uint64_t policy) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      ".L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y), "l"(policy)
+      "{\n"
+      ".reg .pred e;\n"
+      "setp.ne.b32 e, %6, 0;\n"
+      "@e cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      ".L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;\n"
+      "}\n"
+      ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y), "l"(policy), "r"(issue)
       : "memory");
 }
 
@@ -161,35 +183,41 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem], e4m3 x e4m3 -> fp32; one thread issues.
-__device__ __forceinline__ void mma_f8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                       uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f8(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                       uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, e;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+      "setp.ne.b32 e, %5, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem], 16-bit x 16-bit (f16 or bf16, per the instruction descriptor)
 // -> fp32; K = 16 elements per instruction.
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                        uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                       uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, e;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "setp.ne.b32 e, %5, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
 // Arrive on an mbarrier once every MMA issued so far by this thread has retired.
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar)
-               : "memory");
+__device__ __forceinline__ void mma_commit(uint32_t issue, uint32_t bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "setp.ne.b32 e, %1, 0;\n"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar), "r"(issue)
+      : "memory");
 }
 // 16 consecutive fp32 columns of this warp's 32 TMEM lanes -> registers.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -243,22 +271,30 @@ constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;
 
 // 2-D tiled load into THIS CTA's shared memory whose completion is counted on the
 // mbarrier at the same offset in the pair's leader CTA.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* tm,
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t issue, uint32_t dst, const CUtensorMap* tm,
                                                  uint32_t bar_in_leader, int x, int y,
                                                  uint64_t policy) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      ".L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(dst), "l"(tm), "r"(bar_in_leader & kPeerBitMask), "r"(x), "r"(y), "l"(policy)
+      "{\n"
+      ".reg .pred e;\n"
+      "setp.ne.b32 e, %6, 0;\n"
+      "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      ".L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;\n"
+      "}\n"
+      ::"r"(dst), "l"(tm), "r"(bar_in_leader & kPeerBitMask), "r"(x), "r"(y), "l"(policy), "r"(issue)
       : "memory");
 }
 // 3-D form of the same.
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* tm, uint32_t bar_in_leader, int x,
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t issue, uint32_t dst, const CUtensorMap* tm, uint32_t bar_in_leader, int x,
                                                  int y, int z, uint64_t policy) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      ".L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
-      ::"r"(dst), "l"(tm), "r"(bar_in_leader & kPeerBitMask), "r"(x), "r"(y), "r"(z), "l"(policy)
+      "{\n"
+      ".reg .pred e;\n"
+      "setp.ne.b32 e, %7, 0;\n"
+      "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      ".L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;\n"
+      "}\n"
+      ::"r"(dst), "l"(tm), "r"(bar_in_leader & kPeerBitMask), "r"(x), "r"(y), "r"(z), "l"(policy), "r"(issue)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_result, uint32_t ncols) {
@@ -276,35 +312,43 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // D[256 x N] (+)= A[256 x 32] * B[N x 32]^T over the pair: each CTA holds 128 rows of A,
 // N/2 rows of B and 128 rows of D.  Issued by one thread of the leader CTA.
-__device__ __forceinline__ void mma_f8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                            uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f8_pair(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                       uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, e;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+      "setp.ne.b32 e, %5, 0;\n"
+      "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
 // The same for one 16-bit type (f16 or bf16, per the instruction descriptor), K = 16 elements.
-__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                             uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16_pair(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                       uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, e;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "setp.ne.b32 e, %5, 0;\n"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
-// Arrive on the mbarrier at a cluster-wide shared address (this CTA's or the peer's) once
-// every pair MMA issued so far by this thread has retired.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar_cluster_addr)
-               : "memory");
+// Arrive on the mbarrier at this offset in BOTH CTAs of the pair once every pair MMA issued so far by this
+// thread has retired.
+__device__ __forceinline__ void mma_commit_pair(uint32_t issue, uint32_t bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      ".reg .b16 both;\n"
+      "mov.b16 both, 3;\n"
+      "setp.ne.b32 e, %1, 0;\n"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n"
+      "}\n" ::"r"(bar), "r"(issue)
+      : "memory");
 }
 // Plain arrival on an mbarrier that may live in another CTA of the cluster.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
