@@ -61,6 +61,8 @@ SIGNATURES = {
                                      _vp, _sz, _vp]),
     "bq_gate_up_silu_quant_w8a8": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _int, _vp,
                                           _vp, _vp, _sz, _vp]),
+    "bq_mlp_w8a8": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _vp,
+                           _i64, _vp, _sz, _vp]),
     "bq_linear_w8a8": (_int, [_vp, _int, _i64, _i64, _int, ctypes.POINTER(_vp), ctypes.POINTER(_vp), _vp, _i64,
                               ctypes.POINTER(_vp), ctypes.POINTER(_i64), ctypes.POINTER(_i64), _vp, _sz, _vp]),
     "bq_enable_peer_access": (_int, [_int]),

@@ -90,6 +90,8 @@ struct PairSilu {
                            // and the scale of h; the codes are a separate cast pass
   const void* wq_up;       // device: the up weight [I, K] (segment 0's weight pointer is the gate weight)
   const float* sw_up;      // device: dequant scale of the up half (seg.sw is the gate half's)
+  void* h;                 // decode: h itself goes here ([M, I], activation type) and its max to words[0]; the
+                           // product that follows casts it.  nullptr: codes and scale, behind a grid-wide exchange
   uint8_t* hq;             // device: e4m3 codes of h, [M, ld_hq]
   long long ld_hq;
   float* sh;               // device: the scale of h
@@ -140,6 +142,9 @@ struct QuantIn {
   const void* x;       // [M, K] contiguous, 16-byte aligned; nullptr = codes and scale are given
   int dtype;
   int n8;              // groups of 8 values
+  unsigned int* words; // nullptr, or scratch: [0] bits of max |x|, which need not be looked for then, [1] CTAs that have
+                       // read it; the last one returns both to zero
+  unsigned int expected;
 };
 
 struct GemmParams {
@@ -176,7 +181,7 @@ struct GemmParams {
 // 449 -> 435; hidden 1024, 8 rows 157 -> 149.  At prefill sizes the residual and 16-bit forms in the one
 // kernel had cost every launch 8 %.  kAny, with the type taken at run time, is the column-parallel and greedy
 // forms, and launches whose segments differ in their form.
-enum Epi { kAny = -1, kPlain = 0, kResidual = 1, kGateUp = 2, kMixed = 3 };
+enum Epi { kAny = -1, kPlain = 0, kResidual = 1, kGateUp = 2, kMixed = 3, kGateUpDense = 4 };
 constexpr int kAnyType = -1;
 
 struct alignas(64) WeightMaps {
@@ -393,11 +398,12 @@ __global__ void __launch_bounds__(128) argmax_finish_kernel(const uint2* partial
 // same 64 output columns.  Sums the K slices like reduce_store, rounds both halves to the
 // activation type T exactly as the plain GEMM would have stored them, forms
 // h = T(T(silu(gate)) * up) (the two roundings of the separate torch kernels,
-// braid/model/mlp.py:48), and parks h (64 values of T per row) at the start of the row's
-// staging slot in THIS CTA's buffer -- rows of this CTA's share are read by no peer.
+// braid/model/mlp.py:48), and puts h (64 values of T per row) at `park`, row m at m * pitch: the start of
+// the row's staging slot in THIS CTA's buffer -- rows of this CTA's share are read by no peer -- or
+// the h of the whole batch.
 // Lane L < 16 ends up with columns 4L, 4L+1; lane L+16 with 4L+2, 4L+3.  Returns max |h|.
 template <int SPLIT, typename T>
-__device__ __forceinline__ float silu_pair_rows(const EpilogueArgs& e, float scale_up, float* part_rw) {
+__device__ __forceinline__ float silu_pair_rows(const EpilogueArgs& e, float scale_up, T* park, long long pitch) {
   using namespace bq::qd;
   constexpr int kRows = ((SPLIT < 8) ? 8 / SPLIT : 1) > (kStreamWarps > 8 ? 2 : 1)
                             ? ((SPLIT < 8) ? 8 / SPLIT : 1) / (kStreamWarps > 8 ? 2 : 1)
@@ -447,9 +453,8 @@ __device__ __forceinline__ float silu_pair_rows(const EpilogueArgs& e, float sca
         const T h1 = narrow<T>(widen(s1) * u1);
         mx = nan_max(mx, fabsf(widen(h0)));
         mx = nan_max(mx, fabsf(widen(h1)));
-        T* hrow = reinterpret_cast<T*>(part_rw + m * kRowTile);
-        hrow[hcol] = h0;
-        hrow[hcol + 1] = h1;
+        struct alignas(2 * sizeof(T)) Two { T a, b; };
+        *reinterpret_cast<Two*>(park + m * pitch + hcol) = Two{h0, h1};
       }
     }
   }
@@ -497,16 +502,19 @@ __device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const floa
 constexpr int kQuantWarps = kStreamWarps - 2;           // all but the weight loads' and the MMAs'
 constexpr int kQuantThreads = kQuantWarps * 32;
 constexpr int kQuantAhead = 8;                          // groups of 8 a thread asks for at once
+// Chunks of 16 that a thread asks for at once where it casts: behind a weight stream a round trip to L2 takes 2 to 3 us.
+template <typename T, bool GIVEN> constexpr int kChunksAhead = !GIVEN ? 1 : (sizeof(T) == 2 ? 4 : 2);
 
-// Returns the scale.  Called by warps 2.. with all lanes.
-template <typename T>
+// Returns the scale.  Called by warps 2.. with all lanes.  GIVEN: max |x| is in `in.words`.
+template <typename T, bool GIVEN>
 __device__ __forceinline__ float quantize_slice(const QuantIn& in, int M, int K, int kx0, int kb_count, uint8_t* b_tiles,
                                                 int b_tile_bytes, float* s_red) {
   using namespace bq::qd;
   const int t = threadIdx.x - (kStreamThreads - kQuantThreads), lane = threadIdx.x & 31, warp = t >> 5;
   const T* const x = static_cast<const T*>(in.x);
   float m = 0.0f;
-  for (int g0 = t; g0 < in.n8; g0 += kQuantThreads * kQuantAhead / (sizeof(T) / 2)) {
+  if constexpr (GIVEN) m = __uint_as_float(__ldcg(in.words));
+  for (int g0 = t; !GIVEN && g0 < in.n8; g0 += kQuantThreads * kQuantAhead / (sizeof(T) / 2)) {
     Pack8<T> v[kQuantAhead / (sizeof(T) / 2)];
 #pragma unroll
     for (int u = 0; u < kQuantAhead / (int)(sizeof(T) / 2); ++u)
@@ -515,44 +523,68 @@ __device__ __forceinline__ float quantize_slice(const QuantIn& in, int M, int K,
     for (int u = 0; u < kQuantAhead / (int)(sizeof(T) / 2); ++u)
       if (g0 + u * kQuantThreads < in.n8) m = absmax8(v[u], m);
   }
+  if constexpr (!GIVEN) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
-  if (lane == 0) s_red[warp] = m;
-  asm volatile("bar.sync 2, %0;" ::"n"(kQuantThreads) : "memory");
-  m = s_red[0];
+    for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
+    if (lane == 0) s_red[warp] = m;
+    asm volatile("bar.sync 2, %0;" ::"n"(kQuantThreads) : "memory");
+    m = s_red[0];
 #pragma unroll
-  for (int i = 1; i < kQuantWarps; ++i) m = nan_max(m, s_red[i]);
+    for (int i = 1; i < kQuantWarps; ++i) m = nan_max(m, s_red[i]);
+  }
   const float scale = scale_from_amax(m);
   const ScaleDiv dv(scale);
   // 16 codes at a time, where TMA would have put them: 16-byte chunk c of row m at c ^ (m & 7).  K is a
-  // multiple of 16; what a last K block has beyond K reads as zero.
-  const int chunks = kb_count * (kBK / 16);             // of a row, in this slice
-  for (int i = t; i < M * chunks; i += kQuantThreads) {
-    const int row = i / chunks, c = i - row * chunks;
-    const int k = kx0 + c * 16;
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    if (k < K) {
-      const T* const src = x + static_cast<size_t>(row) * K + k;
-      const uint2 lo = codes8<T, true>(load8<T>(src), dv), hi = codes8<T, true>(load8<T>(src + 8), dv);
-      w = make_uint4(lo.x, lo.y, hi.x, hi.y);
+  // multiple of 16.
+  constexpr int kAhead = kChunksAhead<T, GIVEN>;
+  const int chunks = kb_count * (kBK / 16), total = M * chunks;     // of a row in this slice, of the slice
+  for (int i0 = t; i0 < total; i0 += kQuantThreads * kAhead) {
+    constexpr int kWords = sizeof(T);                   // 16-byte words of a chunk
+    uint4 raw[kAhead][kWords];
+    int at[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      at[u] = -1;
+      if (u > 0 && i0 - t + u * kQuantThreads >= total) continue;       // the same for all threads
+      const int i = i0 + u * kQuantThreads, row = i / chunks, c = i - row * chunks, k = kx0 + c * 16;
+      at[u] = i < total ? (c >> 3) * b_tile_bytes + row * kBK + (((c & 7) ^ (row & 7)) << 4) : -1;
+      const bool in = i < total && k < K;               // what a last K block has beyond K casts to zeros
+      const uint4* const src = reinterpret_cast<const uint4*>(x + (in ? static_cast<size_t>(row) * K + k : 0));
+#pragma unroll
+      for (int q = 0; q < kWords; ++q) {
+        raw[u][q] = __ldcg(src + q);                    // coherent (see load8)
+        if (!in) raw[u][q] = make_uint4(0u, 0u, 0u, 0u);
+      }
     }
-    *reinterpret_cast<uint4*>(b_tiles + (c >> 3) * b_tile_bytes + row * kBK + (((c & 7) ^ (row & 7)) << 4)) = w;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (at[u] < 0) continue;
+      Pack8<T> lo, hi;
+#pragma unroll
+      for (int q = 0; q < kWords; ++q) reinterpret_cast<uint4*>(q < kWords / 2 ? &lo : &hi)[q % (kWords / 2)] = raw[u][q];
+      const uint2 a = codes8<T, true>(lo, dv), b = codes8<T, true>(hi, dv);
+      *reinterpret_cast<uint4*>(b_tiles + at[u]) = make_uint4(a.x, a.y, b.x, b.y);
+    }
   }
   fence_proxy_async_smem();                             // the MMAs read through the async proxy
   asm volatile("bar.sync 2, %0;" ::"n"(kQuantThreads) : "memory");
+  if (GIVEN && t == 0 && atomicAdd(&in.words[1], 1u) == in.expected - 1u) {
+    in.words[0] = 0u;
+    in.words[1] = 0u;
+  }
   return scale;
 }
 
 #ifndef BQ_STREAM_MIN_CTAS
 #define BQ_STREAM_MIN_CTAS 2
 #endif
-template <int EPI, int DT, bool QUANT>
+template <int EPI, int DT, int QUANT>      // QUANT: 1 the activation's maximum is looked for, 2 it is given
 __global__ void __launch_bounds__(kStreamThreads, BQ_STREAM_MIN_CTAS)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xd,
                    const __grid_constant__ WeightMaps tm_w, const __grid_constant__ GemmParams p,
                    const int smem_tile_bytes) {
   extern __shared__ uint8_t smem_dyn[];
-  const bool pair_on = EPI == kAny ? p.pair.on != 0 : EPI == kGateUp;
+  const bool pair_on = EPI == kAny ? p.pair.on != 0 : (EPI == kGateUp || EPI == kGateUpDense);
   const bool argmax_on = EPI == kAny && p.argmax.on;
   const PushParams* const push = EPI == kAny && p.push.n > 0 ? &p.push : nullptr;
   const int out_dtype = DT == kAnyType ? p.out_dtype : DT;
@@ -676,7 +708,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       uint8_t* const tiles = base_ptr + (b_base - base);
       using T = typename std::conditional<DT == BQ_DTYPE_F32, float,
                                           typename std::conditional<DT == BQ_DTYPE_F16, __half, __nv_bfloat16>::type>::type;
-      const float sc = quantize_slice<T>(p.quant, p.M, p.quant_k, kx0, kb_count, tiles, b_tile_bytes, s_quant);
+      const float sc = quantize_slice<T, QUANT == 2>(p.quant, p.M, p.quant_k, kx0, kb_count, tiles, b_tile_bytes, s_quant);
       if (threadIdx.x == kStreamThreads - kQuantThreads) {
         *s_scale = sc;
         mbar_arrive(full_bar_b(0));
@@ -797,18 +829,35 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     if (pair_on) {
       const float scale_up = sx_ready * __ldg(p.pair.sw_up);
       float mx;
-#define BQ_PAIR_ROWS(TT)                                                          \
-      switch (split) {                                                             \
-        case 1: mx = silu_pair_rows<1, TT>(ea, scale_up, part); break;             \
-        case 2: mx = silu_pair_rows<2, TT>(ea, scale_up, part); break;             \
-        case 4: mx = silu_pair_rows<4, TT>(ea, scale_up, part); break;             \
-        default: mx = silu_pair_rows<8, TT>(ea, scale_up, part); break;            \
+#define BQ_PAIR_ROWS(TT)                                                                           \
+      constexpr bool dense_h = EPI == kGateUpDense;                                                 \
+      TT* const park = dense_h ? static_cast<TT*>(p.pair.h) + tile_in_seg * (kRowTile / 2)          \
+                               : reinterpret_cast<TT*>(part);                                       \
+      const long long pitch = dense_h ? seg.n / 2 : kRowTile * 4 / (int)sizeof(TT);                 \
+      switch (split) {                                                                              \
+        case 1: mx = silu_pair_rows<1, TT>(ea, scale_up, park, pitch); break;                       \
+        case 2: mx = silu_pair_rows<2, TT>(ea, scale_up, park, pitch); break;                       \
+        case 4: mx = silu_pair_rows<4, TT>(ea, scale_up, park, pitch); break;                       \
+        default: mx = silu_pair_rows<8, TT>(ea, scale_up, park, pitch); break;                      \
       }
       if (out_dtype == BQ_DTYPE_BF16) { BQ_PAIR_ROWS(__nv_bfloat16) }
       else if (out_dtype == BQ_DTYPE_F16) { BQ_PAIR_ROWS(__half) }
       else { BQ_PAIR_ROWS(float) }
 #undef BQ_PAIR_ROWS
       pair_max = mx;
+      if (EPI == kGateUpDense) {
+        // nobody waits for anybody: the bits of |h| order like the values, NaN on top, and whoever reads the word
+        // does so behind the end of this launch
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) mx = bq::qd::nan_max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        if (lane == 0) s_quant[warp] = mx;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll
+          for (int i = 1; i < kStreamWarps; ++i) mx = bq::qd::nan_max(mx, s_quant[i]);
+          atomicMax(&p.pair.words[0], __float_as_uint(mx));
+        }
+      }
     } else if (argmax_on) {
       uint2* const mine = p.argmax.partial + static_cast<size_t>(tile_in_seg) * p.M;
       if (out_dtype == BQ_DTYPE_BF16) argmax_rows<__nv_bfloat16>(ea, seg.n, mine);
@@ -855,7 +904,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         }
       }
     }
-  } else if (pair_on) {
+  } else if (pair_on && EPI != kGateUpDense) {
     // ---- grid-wide max |h| -> scale -> codes of this CTA's rows (h is parked in `part`) ----
     using namespace bq::qd;
 #pragma unroll
@@ -1616,19 +1665,23 @@ thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
 
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
-using StreamKernel = decltype(&gemm_stream_kernel<kAny, kAnyType, false>);
+using StreamKernel = decltype(&gemm_stream_kernel<kAny, kAnyType, 0>);
 using WideKernel = decltype(&gemm_wide_kernel<1, kAny, kAnyType>);
 using PairKernel = decltype(&gemm_pair_kernel<kAny, kAnyType>);
 
 // The kernels by [epilogue][type]; the types are BQ_DTYPE_F32, BF16, F16 = 0, 1, 2.
 const StreamKernel kStream[3][3] = {
-    {gemm_stream_kernel<kPlain, 0, false>, gemm_stream_kernel<kPlain, 1, false>, gemm_stream_kernel<kPlain, 2, false>},
-    {gemm_stream_kernel<kResidual, 0, false>, gemm_stream_kernel<kResidual, 1, false>, gemm_stream_kernel<kResidual, 2, false>},
-    {gemm_stream_kernel<kGateUp, 0, false>, gemm_stream_kernel<kGateUp, 1, false>, gemm_stream_kernel<kGateUp, 2, false>}};
-const StreamKernel kStreamQuant[2][3] = {
-    {gemm_stream_kernel<kPlain, 0, true>, gemm_stream_kernel<kPlain, 1, true>, gemm_stream_kernel<kPlain, 2, true>},
-    {gemm_stream_kernel<kResidual, 0, true>, gemm_stream_kernel<kResidual, 1, true>, gemm_stream_kernel<kResidual, 2, true>}};
-const StreamKernel kStreamAny = gemm_stream_kernel<kAny, kAnyType, false>;
+    {gemm_stream_kernel<kPlain, 0, 0>, gemm_stream_kernel<kPlain, 1, 0>, gemm_stream_kernel<kPlain, 2, 0>},
+    {gemm_stream_kernel<kResidual, 0, 0>, gemm_stream_kernel<kResidual, 1, 0>, gemm_stream_kernel<kResidual, 2, 0>},
+    {gemm_stream_kernel<kGateUp, 0, 0>, gemm_stream_kernel<kGateUp, 1, 0>, gemm_stream_kernel<kGateUp, 2, 0>}};
+const StreamKernel kStreamGateUpDense[3] = {gemm_stream_kernel<kGateUpDense, 0, 0>, gemm_stream_kernel<kGateUpDense, 1, 0>,
+                                           gemm_stream_kernel<kGateUpDense, 2, 0>};
+const StreamKernel kStreamQuant[2][2][3] = {     // [is the maximum given?]
+    {{gemm_stream_kernel<kPlain, 0, 1>, gemm_stream_kernel<kPlain, 1, 1>, gemm_stream_kernel<kPlain, 2, 1>},
+     {gemm_stream_kernel<kResidual, 0, 1>, gemm_stream_kernel<kResidual, 1, 1>, gemm_stream_kernel<kResidual, 2, 1>}},
+    {{gemm_stream_kernel<kPlain, 0, 2>, gemm_stream_kernel<kPlain, 1, 2>, gemm_stream_kernel<kPlain, 2, 2>},
+     {gemm_stream_kernel<kResidual, 0, 2>, gemm_stream_kernel<kResidual, 1, 2>, gemm_stream_kernel<kResidual, 2, 2>}}};
+const StreamKernel kStreamAny = gemm_stream_kernel<kAny, kAnyType, 0>;
 template <int MODE>
 struct WideKernels {
   static constexpr WideKernel any = gemm_wide_kernel<MODE, kAny, kAnyType>;
@@ -1648,7 +1701,7 @@ const PairKernel kPairAny = gemm_pair_kernel<kAny, kAnyType>;
 // segments (elsewhere they are a matter of a segment)?
 int epilogue_of(const GemmParams& p, bool mixed) {
   if (p.push.n > 0 || p.argmax.on) return kAny;
-  if (p.pair.on) return kGateUp;
+  if (p.pair.on) return p.pair.h != nullptr ? kGateUpDense : kGateUp;
   int with = 0, dense = 0;
   for (int i = 0; i < p.n_seg; ++i) {
     with += p.seg[i].res != nullptr;
@@ -1669,12 +1722,13 @@ int configure_once() {
     set((const void*)WideKernels<1>::any);
     set((const void*)WideKernels<2>::any);
     set((const void*)kPairAny);
+    for (int d = 0; d < 3; ++d) set((const void*)kStreamGateUpDense[d]);
     for (int e = 0; e < 4; ++e)
       for (int d = 0; d < 3; ++d) {
         if (kPair[e][d] != nullptr) set((const void*)kPair[e][d]);
         if (e == 3) continue;
         set((const void*)kStream[e][d]);
-        if (e < 2) set((const void*)kStreamQuant[e][d]);
+        for (int g = 0; e < 2 && g < 2; ++g) set((const void*)kStreamQuant[g][e][d]);
         set((const void*)WideKernels<1>::of[e][d]);
         set((const void*)WideKernels<2>::of[e][d]);
       }
@@ -1781,6 +1835,35 @@ bool quantize_inside_pays(int64_t M, int64_t K, int element_size, int n_seg, con
   return status == cudaStreamCaptureStatusNone;
 }
 
+// Shared memory of a CTA for rings: what lets the whole grid be resident at once (up to 2 CTAs per SM), so that one
+// CTA's epilogue overlaps its neighbour's loads.
+int stream_budget(long long grid, int sms, int* per_sm_out = nullptr) {
+  int per_sm = (int)((grid + sms - 1) / sms);
+  if (per_sm < 1) per_sm = 1;
+  if (per_sm > 2) per_sm = 2;
+  if (per_sm_out != nullptr) *per_sm_out = per_sm;
+  return kMaxSmem / per_sm - 1024 - kBarrierBytes - 1024;
+}
+
+// Rings of a launch whose CTAs cast the activation for themselves: a slice's activation tiles all stay, the weight
+// ring gets the rest.  0: no room.
+int cast_stages(int budget, int b_tile, int kb_max) {
+  int stages = (budget - kb_max * b_tile) / kATileBytes;
+  if (stages > kb_max) stages = kb_max;
+  if (stages > 24) stages = 24;
+  // long slices of few rows: tiles padded to 16 rows would crowd out the weights (1 row of 8192 x 20480: 33 -> 36 us)
+  if (2 * kb_max * b_tile > budget) return 0;
+  return stages < (kb_max < 4 ? kb_max : 4) || 2 * stages + kb_max + 1 > 100 ? 0 : stages;
+}
+
+// Few rows: where the CTAs of the down projection cast h for themselves.  It takes the grid-wide exchange and the
+// cast out of the gate/up launch, behind whose stream HBM idles for them; down's CTAs do the cast while
+// their first weights arrive, as long as one round of loads of 4 chunks a thread covers a slice (6 rows of a 16-bit
+// type; each round is 2 to 3 us, and 5 chunks spill).  Four graphed layers, us, before and after: hidden 4096,
+// 1 row 215.7 -> 202.5, 4 rows 235.2 -> 220.1, 6 rows 237.5 -> 229.1, 8 rows 240.5 and 238.3, 16 rows 249 and 257.  A
+// smaller down weight has arrived before the cast is done: hidden 2560 (20 MB), 4 rows 241.8 and 241.3, 8 rows
+// 312.3 and 313.8; hidden 2048 (13 MB), 1 row 123.7 and 124.5.
+
 int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightMaps& maps,
                   GemmParams& p, cudaStream_t stream) {
   const int sms = device_sms();
@@ -1813,13 +1896,8 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
       if (kb > kb_max) kb_max = kb;
     }
   const int staging = p.mma_n * kRowTile * 4;
-  // Shared memory per CTA: small enough that the whole grid is resident at once
-  // (up to 2 CTAs per SM: 256 threads x ~128 registers each), so one CTA's
-  // epilogue overlaps its neighbour's loads.
-  int per_sm = (int)((grid + sms - 1) / sms);
-  if (per_sm < 1) per_sm = 1;
-  if (per_sm > 2) per_sm = 2;
-  int budget = kMaxSmem / per_sm - 1024 - kBarrierBytes - 1024;
+  int per_sm = 1;
+  int budget = stream_budget(grid, sms, &per_sm);
   // Leave room for the NEXT kernel's CTAs: with programmatic dependent launch they
   // become resident while this kernel still runs and pre-load their weights.
   if (g_opt_smem_cap > 0 && budget > g_opt_smem_cap) budget = (int)g_opt_smem_cap;
@@ -1842,14 +1920,10 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
     if (stages > 24) stages = 24;
     if (b_stages > stages) b_stages = stages;
   }
-  if (quant) {     // the whole slice's activation tiles stay; the weight ring gets the rest
+  if (quant) {
     b_stages = kb_max;
-    stages = (budget - b_stages * b_tile) / kATileBytes;
-    if (stages > kb_max) stages = kb_max;
-    if (stages > 24) stages = 24;
-    // long slices of few rows: tiles padded to 16 rows would crowd out the weights (1 row of 8192 x 20480: 33 -> 36 us)
-    if (2 * b_stages * b_tile > budget) return kErrUnsupported;
-    if (stages < (kb_max < 4 ? kb_max : 4) || 2 * stages + b_stages + 1 > 100) return kErrUnsupported;
+    stages = cast_stages(budget, b_tile, kb_max);
+    if (stages == 0) return kErrUnsupported;
   }
   p.stages = stages;
   p.b_stages = b_stages;
@@ -1860,11 +1934,13 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   const int epi = epilogue_of(p, false);
   if (quant && epi != kPlain && epi != kResidual) return kErrUnsupported;
   const StreamKernel kernel =
-      quant ? kStreamQuant[epi][p.out_dtype] : (epi == kAny ? kStreamAny : kStream[epi][p.out_dtype]);
+      quant ? kStreamQuant[p.quant.words != nullptr ? 1 : 0][epi][p.out_dtype]
+            : (epi == kAny ? kStreamAny : (epi == kGateUpDense ? kStreamGateUpDense[p.out_dtype] : kStream[epi][p.out_dtype]));
   if (p.pair.on) p.pair.expected = (unsigned)((p.seg[0].n / kRowTile) * p.seg[0].split);
   if (p.push.n > 0)
     p.push.expected = (unsigned)(((p.seg[0].n + kRowTile - 1) / kRowTile) * p.seg[0].split);
-  if (p.pair.on && p.push.n == 0) {
+  if (quant) p.quant.expected = (unsigned)(((p.seg[0].n + kRowTile - 1) / kRowTile) * p.seg[0].split);
+  if (p.pair.on && p.push.n == 0 && p.pair.h == nullptr) {
     // the epilogue's amax exchange waits on the whole grid: every CTA must be resident
     const int cap = max_resident_ctas(kernel, cluster, smem);
     if (getenv("BQ_DEBUG"))
@@ -2354,8 +2430,9 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
     // the weight-streaming kernel alone has this form: the others read codes and scale, which are not given.  Its
     // rings are cut to the activation, so forced depths are left to the two launches.
     if (!stream_path || dn || push || am || pair || g_opt_wide > 0 || g_opt_stages > 0 || g_opt_b_stages != 0 ||
-        M > BQ_LINEAR_MAX_ROWS ||
-        !quantize_inside_pays(M, K, qi->dtype == BQ_DTYPE_F32 ? 4 : 2, n_seg, N, static_cast<cudaStream_t>(stream_v)))
+        M > BQ_LINEAR_MAX_ROWS || (qi->words != nullptr && n_seg != 1) ||
+        (qi->words == nullptr &&
+         !quantize_inside_pays(M, K, qi->dtype == BQ_DTYPE_F32 ? 4 : 2, n_seg, N, static_cast<cudaStream_t>(stream_v))))
       return kErrUnsupported;
   }
   if (dn != nullptr) {
@@ -2544,7 +2621,7 @@ extern "C" int bq_linear_w8a8(const void* x, int dtype, int64_t M, int64_t K, in
                               const float* const* sw, const void* residual, int64_t ld_res, void* const* y,
                               const int64_t* N, const int64_t* ldy, void* ws, size_t ws_bytes, void* stream) {
   if (x == nullptr || (residual != nullptr && n_seg != 1)) return kErrBadArg;
-  const QuantIn qi{x, dtype, 0};
+  const QuantIn qi{x, dtype, 0, nullptr, 0};
   const void* rs[1] = {residual};
   const int64_t ldrs[1] = {ld_res};
   return run_grouped(nullptr, nullptr, M, K, n_seg, wq, sw, y, N, ldy, dtype, ws, ws_bytes, stream,
@@ -2648,6 +2725,54 @@ extern "C" int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const
   const int split = (K > 0 && K <= 0x7fffff00LL) ? split_for_weight((int)I, k_blocks) : 1;
   return run_grouped(xq, sx, M, K, 1, wqs, sws, ys, Ns, ldys, act_dtype, ws, ws_bytes, stream,
                      nullptr, nullptr, &pair, split);
+}
+
+extern "C" int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate, const void* wq_up, const void* wq_down,
+                           const float* sw_gate, const float* sw_up, const float* sw_down, const void* residual,
+                           int64_t ld_res, int64_t M, int64_t K, int64_t I, int64_t N, int act_dtype, void* h, void* y,
+                           int64_t ldy, void* ws, size_t ws_bytes, void* stream) {
+  if (!xq || !sx || !wq_gate || !wq_up || !wq_down || !sw_gate || !sw_up || !sw_down || !h || !y || M <= 0 || K <= 0 ||
+      I <= 0 || N <= 0)
+    return kErrBadArg;
+  if (act_dtype != BQ_DTYPE_F32 && act_dtype != BQ_DTYPE_BF16 && act_dtype != BQ_DTYPE_F16) return kErrBadArg;
+  // Everything the second launch would refuse is refused before the first one runs.
+  const int out_align = act_dtype == BQ_DTYPE_F32 ? 16 : 8;
+  if (M * (act_dtype == BQ_DTYPE_F32 ? 4 : 2) > 2 * BQ_MLP_MAX_ROWS || I * N < BQ_MLP_MIN_WEIGHT || M > g_opt_stream_max_m || g_opt_wide > 0 || g_opt_stages > 0 || g_opt_b_stages != 0 ||
+      g_opt_smem_cap > 0 || g_opt_quant_inside >= 0)
+    return kErrUnsupported;
+  if (I % (kRowTile / 2) || N % 16 || I > 0x3fffff00LL || N > 0x7fffff00LL || !aligned_to(wq_up, 16) ||
+      !aligned_to(wq_down, 16) || !aligned_to(h, 16) || ldy < N || ldy % 4 || !aligned_to(y, out_align))
+    return kErrUnsupported;
+  if (residual != nullptr && (ld_res < N || ld_res % 4 || !aligned_to(residual, out_align))) return kErrUnsupported;
+  const int sms = device_sms();
+  if (sms <= 0) return kErrLaunch;
+  const int blocks = (int)((I + kBK - 1) / kBK), split = split_for_weight(N, blocks);
+  if (cast_stages(stream_budget((N + kRowTile - 1) / kRowTile * split, sms), (int)((M + 15) / 16 * 16) * kBK,
+                  (blocks + split - 1) / split) == 0)
+    return kErrUnsupported;
+  PairSilu pair;
+  memset(&pair, 0, sizeof(pair));
+  pair.wq_up = wq_up;
+  pair.sw_up = sw_up;
+  pair.h = h;
+  const void* wqs[1] = {wq_gate};
+  const float* sws[1] = {sw_gate};
+  void* none[1] = {nullptr};
+  const int64_t Ns[1] = {2 * I}, zero[1] = {0};
+  const int k_blocks = (int)((K + kBK - 1) / kBK);
+  if (int rc = run_grouped(xq, sx, M, K, 1, wqs, sws, none, Ns, zero, act_dtype, ws, ws_bytes, stream, nullptr, nullptr,
+                           &pair, K <= 0x7fffff00LL ? split_for_weight(I, k_blocks) : 1))
+    return rc;
+  const QuantIn qi{h, act_dtype, 0, static_cast<unsigned int*>(ws), 0};
+  const void* wds[1] = {wq_down};
+  const float* sds[1] = {sw_down};
+  void* ys[1] = {y};
+  const int64_t Nd[1] = {N}, ldys[1] = {ldy}, ldrs[1] = {ld_res};
+  const void* rs[1] = {residual};
+  const int rc = run_grouped(nullptr, nullptr, M, I, 1, wds, sds, ys, Nd, ldys, act_dtype, ws, ws_bytes, stream,
+                             residual != nullptr ? rs : nullptr, residual != nullptr ? ldrs : nullptr, nullptr, 0, nullptr,
+                             nullptr, nullptr, &qi);
+  return rc == kErrUnsupported ? kErrLaunch : rc;      // cannot be: checked above
 }
 
 extern "C" int bq_gate_up_silu_w8a8(const void* xq, const float* sx, const void* wq_gate,

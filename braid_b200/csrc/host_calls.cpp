@@ -58,6 +58,7 @@ struct Lib {
   decltype(&bq_project_mixed) project_mixed;
   decltype(&bq_gate_up_silu_quant_w8a8) gate_up_silu_quant;
   decltype(&bq_gate_up_silu_w8a8) gate_up_silu;
+  decltype(&bq_mlp_w8a8) mlp;
   decltype(&bq_lm_head_argmax) lm_head_argmax;
   decltype(&bq_lm_head_argmax_workspace_bytes) lm_head_argmax_workspace;
 } g_lib;
@@ -560,11 +561,25 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
        residual.scalar_type() != out || residual.stride(1) != 1 || residual.stride(0) < N || residual.stride(0) % 4 ||
        !aligned(residual.data_ptr(), out == at::kFloat ? 16 : 8) || recorded(residual)))
     Py_RETURN_NONE;
+  int rc;
+  if (M <= BQ_MLP_MAX_ROWS && I * N >= BQ_MLP_MIN_WEIGHT) {        // both products in one call, where that form takes them
+    const at::Tensor act = empty(h, {M, I}, out), y = empty(h, {M, N}, out);
+    void* slot = take_slot(h.dev);
+    {
+      NoGil no_gil;
+      rc = g_lib.mlp(xq.data_ptr(), sx.data_ptr<float>(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(), sg.data_ptr<float>(),
+                     su.data_ptr<float>(), sd.data_ptr<float>(), residual.defined() ? residual.data_ptr() : nullptr,
+                     residual.defined() ? residual.stride(0) : 0, M, K, I, N, code, act.data_ptr(), y.data_ptr(), N, slot, 16,
+                     h.stream);
+    }
+    if (rc == BQ_OK) g_launches.fetch_add(1, std::memory_order_relaxed);      // the slot counted one of the two
+    if (rc != BQ_ERR_UNSUPPORTED) return gemm_result(y, rc);
+    g_launches.fetch_sub(1, std::memory_order_relaxed);
+  }
   at::Tensor hq, sh = empty(h, {1, 1}, at::kFloat), dense;
   if (M <= 256) hq = empty(h, {M, I}, at::kFloat8_e4m3fn);
   else dense = empty(h, {M, I}, out);
   void* slot = take_slot(h.dev);
-  int rc;
   {
     NoGil no_gil;
     rc = M <= 256 ? g_lib.gate_up_silu_quant(xq.data_ptr(), sx.data_ptr<float>(), wg.data_ptr(), wu.data_ptr(),
@@ -646,7 +661,7 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !get("bq_sigmoid_gate_quant", g_lib.sigmoid_gate_quant) ||
       !get("bq_sigmoid_mul_dense_scale", g_lib.sigmoid_mul_dense_scale) ||
       !get("bq_gemm_w8a8_grouped", g_lib.gemm_grouped) || !get("bq_gemm_w8a8_residual", g_lib.gemm_residual) ||
-      !get("bq_linear_w8a8", g_lib.linear) || !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_w8a8", g_lib.gate_up_silu_quant) ||
+      !get("bq_linear_w8a8", g_lib.linear) || !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_w8a8", g_lib.gate_up_silu_quant) || !get("bq_mlp_w8a8", g_lib.mlp) ||
       !get("bq_gate_up_silu_w8a8", g_lib.gate_up_silu) || !get("bq_lm_head_argmax", g_lib.lm_head_argmax) ||
       !get("bq_lm_head_argmax_workspace_bytes", g_lib.lm_head_argmax_workspace))
     return nullptr;

@@ -421,6 +421,29 @@ int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const void* wq_g
                                void* ws, size_t ws_bytes, void* stream);
 
 /*
+ * The whole quantized MLP of a decode batch of few rows (M <= BQ_MLP_MAX_ROWS) in TWO launches that exchange
+ * nothing inside:
+ *   y = bq_gemm_w8a8[_residual](bq_gate_up_silu_quant_w8a8(xq, gate, up), down)
+ * with the same bits.  The first launch writes h in the activation type and its max |h|, the second one's
+ * CTAs cast the K slice they multiply for themselves.
+ *
+ * Replaces: braid/model/mlp.py:46-49.
+ *
+ *   residual   optional [M, N], row stride ld_res, added after y has been rounded to its type; or NULL
+ *   h          device, [M, I] of act_dtype, contiguous, 16-byte aligned (written and read)
+ *   y          device, [M, N] of act_dtype, row stride ldy
+ *   ws         16 bytes, zero before the first call, self-resetting (as for bq_quantize_act)
+ * Returns BQ_ERR_UNSUPPORTED, with nothing launched, where the separate calls are to be used (more rows, small
+ * down weights, slices of h too long for shared memory, a layout forced by an option, shapes and alignments they refuse as well).
+ */
+#define BQ_MLP_MAX_ROWS 6                /* fp32: half as many */
+#define BQ_MLP_MIN_WEIGHT (32 << 20)     /* values of the down weight */
+int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate, const void* wq_up, const void* wq_down,
+                const float* sw_gate, const float* sw_up, const float* sw_down, const void* residual, int64_t ld_res,
+                int64_t M, int64_t K, int64_t I, int64_t N, int act_dtype, void* h, void* y, int64_t ldy,
+                void* ws, size_t ws_bytes, void* stream);
+
+/*
  * Column-parallel forms for one NVLink/NVSwitch node (no counterpart in the reference, which is
  * single-GPU; the benchmark configuration defines an N-split MLP with gathered outputs).  The
  * GEMM of a rank's weight shard stores its output tile straight into the gathered buffer of

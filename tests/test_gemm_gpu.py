@@ -763,6 +763,39 @@ def test_prefill_gate_up_silu_equals_the_separate_kernels(Q, dt, M, I, K):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M,I,dt", [(1, 12288, torch.bfloat16), (6, 12288, torch.bfloat16), (7, 12288, torch.bfloat16),
+                                    (5, 12288, torch.float16), (3, 12288, torch.float32), (4, 12288, torch.float32),
+                                    (6, 8256, torch.bfloat16), (2, 8128, torch.bfloat16)])
+def test_mlp_of_few_rows_casts_h_in_the_down_projection(Q, M, I, dt):
+    """Up to 6 rows (3 of fp32) and from a down weight of 32 Mi values on, h is cast by the CTAs of the down projection:
+    the bits of the separate launches at either side of both lines, with a last K block that is half full, with an
+    infinity and a NaN in h, and again with the scratch that the calls before returned to zero."""
+    H = 4096
+    mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
+    wg, wu, wd = mk(I, H, 3), mk(I, H, 4), mk(H, I, 5)
+    r = randn_cpu((M, H), seed=M + 1, dtype=dt).cuda()
+    big = torch.finfo(torch.float16).max if dt is torch.float16 else torch.finfo(dt).max
+    for case in ("plain", "zeros", "inf", "nan"):
+        x = randn_cpu((M, H), seed=M, dtype=dt).cuda()
+        if case == "zeros":
+            x.zero_()
+        xq, sx = Q.quantize_act(x)
+        if case in ("inf", "nan"):
+            sx = torch.full_like(sx, big if case == "inf" else float("nan"))
+        h = Q.QuantizedActivation(xq, sx, x.shape, dt)
+        Q.set_paired_mlp(False)
+        want, want_r = Q.mlp_forward(h, wg, wu, wd), Q.mlp_forward(h, wg, wu, wd, residual=r)
+        Q.set_paired_mlp(True)
+        for _ in range(2):
+            n0 = Q.launch_count()
+            got = Q.mlp_forward(h, wg, wu, wd)
+            assert Q.launch_count() - n0 == 2
+            got_r = Q.mlp_forward(h, wg, wu, wd, residual=r)
+            for a, b in ((got, want), (got_r, want_r)):
+                assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(), b.nan_to_num()), case
+    assert Q.device_status() == 0
+
+
 def test_paired_mlp_equals_the_four_launch_mlp_and_replays(Q):
     H, I = 4096, 12288
     mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
