@@ -158,6 +158,7 @@ struct GemmParams {
   int k_blocks_dense;  // stream kernel: 128-byte K blocks of a 16-bit row, ceil(2K / 128)
   int dense_fmt;       // stream kernel: tcgen05 operand format of the 16-bit segments (0 f16, 1 bf16)
   int cluster;         // stream kernel: CTAs per cluster = largest split of the launch
+  int handover;        // stream kernel: slices are handed to the CTA that sums them (see handover_bytes)
   int stages;          // stream kernel: depth of the weight ring; pair kernel: pipeline depth
   int b_stages;        // stream kernel: depth of the activation ring
   int out_dtype;
@@ -220,6 +221,7 @@ struct EpilogueArgs {
   const float* part;       // this CTA's staging buffer [mma_n][128] fp32
   uint32_t part_addr;      // its shared-memory address
   int peer0;               // cluster rank of K slice 0 of this tile
+  int slice_rows;          // > 0: the partials were handed over, slice r of row m lies here at (r * slice_rows + m - m_begin)
   int m_begin, m_end;      // output rows this CTA reduces and writes
   int warp, lane;
   int row0;                // first weight row (output column) of the tile
@@ -270,6 +272,22 @@ __device__ __forceinline__ float4 add_res4(float4 v, uint4 raw, int out_dtype) {
   return v;
 }
 
+// The SPLIT partial sums of four columns of a row, from this CTA's memory or from its peers'.
+template <int SPLIT>
+__device__ __forceinline__ void load_slices(const EpilogueArgs& e, int m, int n4, float4 (&v)[SPLIT]) {
+  if constexpr (SPLIT == 1) {
+    v[0] = *reinterpret_cast<const float4*>(e.part + m * kRowTile + n4);
+  } else if (e.slice_rows > 0) {
+#pragma unroll
+    for (int r = 0; r < SPLIT; ++r)
+      v[r] = *reinterpret_cast<const float4*>(e.part + (r * e.slice_rows + m - e.m_begin) * kRowTile + n4);
+  } else {
+    const uint32_t off = e.part_addr + static_cast<uint32_t>(m * kRowTile + n4) * 4u;
+#pragma unroll
+    for (int r = 0; r < SPLIT; ++r) v[r] = ld_cluster_f4(map_to_cta(off, e.peer0 + r));
+  }
+}
+
 // Sums the SPLIT partial tiles of this CTA's rows in rank order (fixed order:
 // the result does not depend on timing) and stores them.  Every thread asks
 // for all the partials of a batch of rows before it uses any of them, so the
@@ -297,16 +315,7 @@ __device__ __forceinline__ void reduce_store(const EpilogueArgs& e) {
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
       const int m = m0 + i * kWarps;
-      if (m < e.m_end) {
-        const uint32_t off = e.part_addr + static_cast<uint32_t>(m * kRowTile + n4) * 4u;
-#pragma unroll
-        for (int r = 0; r < SPLIT; ++r) {
-          if constexpr (SPLIT == 1)
-            v[i][0] = *reinterpret_cast<const float4*>(e.part + m * kRowTile + n4);
-          else
-            v[i][r] = ld_cluster_f4(map_to_cta(off, e.peer0 + r));
-        }
-      }
+      if (m < e.m_end) load_slices<SPLIT>(e, m, n4, v[i]);
     }
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
@@ -419,16 +428,7 @@ __device__ __forceinline__ float silu_pair_rows(const EpilogueArgs& e, float sca
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
       const int m = m0 + i * kWarps;
-      if (m < e.m_end) {
-        const uint32_t off = e.part_addr + static_cast<uint32_t>(m * kRowTile + n4) * 4u;
-#pragma unroll
-        for (int r = 0; r < SPLIT; ++r) {
-          if constexpr (SPLIT == 1)
-            v[i][0] = *reinterpret_cast<const float4*>(e.part + m * kRowTile + n4);
-          else
-            v[i][r] = ld_cluster_f4(map_to_cta(off, e.peer0 + r));
-        }
-      }
+      if (m < e.m_end) load_slices<SPLIT>(e, m, n4, v[i]);
     }
     __syncwarp();   // every lane has its slice of the rows before any lane overwrites them
 #pragma unroll
@@ -665,9 +665,12 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) BQ_STAMP(p, 1);
 
+  // slices are written into a peer's memory: once it has started, which this says
+  if (p.handover) cluster_arrive_relaxed();
   if (!active) {
     // nothing to multiply: it only matches the two cluster barriers of the working CTAs
-    if (p.cluster > 1) { cluster_sync_all(); cluster_sync_all(); }
+    if (p.handover) { cluster_wait(); cluster_sync_all(); }
+    else if (p.cluster > 1) { cluster_sync_all(); cluster_sync_all(); }
     return;
   }
 
@@ -795,7 +798,27 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   ok = (*abort_flag == 0);
   const float scale = sx_ready * sw;
   float* const part = reinterpret_cast<float*>(base_ptr);   // [mma_n][128]
-  if (ok) {
+  float* const slices = reinterpret_cast<float*>(base_ptr + smem_tile_bytes + kBarrierBytes);   // [split][per][128]
+  const int per = (p.M + split - 1) / split;               // rows that a CTA sums
+  const bool handover = p.handover && split > 1;
+  if (p.handover) cluster_wait();
+  if (ok && handover) {
+    const int quad = warp & 3;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const uint32_t mine = smem_u32(slices) + static_cast<uint32_t>(krank * per * kRowTile + quad * 32 + lane) * 4u;
+    for (int c = (warp >> 2) * 16; c < p.M; c += 4 * kStreamWarps) {
+      uint32_t r[16];
+      tmem_ld16(lane_addr + c, r);
+      tmem_ld_wait();
+      int owner = c / per, row = c - owner * per;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        if (c + j < p.M)
+          st_cluster_f1(map_to_cta(mine + row * (kRowTile * 4), group * split + owner), __uint_as_float(r[j]));
+        if (++row == per) { row = 0; ++owner; }
+      }
+    }
+  } else if (ok) {
     // 8 warps: warp w reads TMEM lanes 32*(w%4).. (the only ones it may touch)
     // and every other 16-column chunk, starting at chunk w/4
     const int quad = warp & 3;
@@ -817,15 +840,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
 
   // ---- reduce the K slices in rank order and write this CTA's share of rows --
   float pair_max = 0.0f;
-  const int per = (p.M + split - 1) / split;
   const int m_begin = krank * per;
   const int m_end = (m_begin + per < p.M) ? (m_begin + per) : p.M;
   if (ok) {
     const bool col_ok = (row0 + lane * 4) < seg.n;      // n is a multiple of 16
     const uint32_t part_addr = smem_u32(part);
     const int peer0 = group * split;
-    const EpilogueArgs ea{part, part_addr, peer0, m_begin, m_end, warp, lane, row0, scale, col_ok,
-                          seg.y, seg.ldy, out_dtype, seg.res, seg.ld_res, push};
+    const EpilogueArgs ea{handover ? slices : part, part_addr, peer0, handover ? per : 0, m_begin, m_end, warp, lane, row0,
+                          scale, col_ok, seg.y, seg.ldy, out_dtype, seg.res, seg.ld_res, push};
     if (pair_on) {
       const float scale_up = sx_ready * __ldg(p.pair.sw_up);
       float mx;
@@ -882,7 +904,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   }
   if (threadIdx.x == 0) BQ_STAMP(p, 6);
   // nobody leaves while a peer may still read its staging buffer
-  if (p.cluster > 1) cluster_sync_all(); else __syncthreads();
+  if (p.cluster > 1 && !p.handover) cluster_sync_all(); else __syncthreads();
   if (pair_on && push != nullptr) {
     // ---- column-parallel form: h itself goes to every rank's gathered buffer; the amax needs
     // all ranks' shards and is taken by the quantizer that follows the exchange ----
@@ -943,7 +965,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     __syncthreads();
     const float sc = s_quant[0];
     if (ok) {
-      const EpilogueArgs ea{part, smem_u32(part), 0, m_begin, m_end, warp, lane, row0, 0.0f, true,
+      const EpilogueArgs ea{part, smem_u32(part), 0, 0, m_begin, m_end, warp, lane, row0, 0.0f, true,
                             nullptr, 0, out_dtype, nullptr, 0, push};
       const int col0 = tile_in_seg * (kRowTile / 2);
       if (out_dtype == BQ_DTYPE_BF16)
@@ -1835,6 +1857,15 @@ bool quantize_inside_pays(int64_t M, int64_t K, int element_size, int n_seg, con
   return status == cudaStreamCaptureStatusNone;
 }
 
+// Where the K slices of a tile are summed.  Up to 48 rows every CTA writes its share of a tile straight from its
+// accumulator into the memory of the CTA that sums those rows, and one cluster barrier ends the exchange; more
+// rows would take the memory of too many weight tiles, and are staged and fetched between two barriers.
+// us, fetched -> handed over: linear of 8 rows of 4096 x 4096 8.8 -> 7.9; four graphed layers of hidden 4096, 16 rows
+// 249.2 -> 246.6, 27 rows 263 -> 257.5, 48 rows 274 -> 273, 1 row the same; hidden 1024, 16 rows 147 -> 145.8.
+int handover_bytes(int64_t M, int split) {
+  return split > 1 && M <= 48 ? (int)((M + split - 1) / split) * split * kRowTile * 4 : 0;
+}
+
 // Shared memory of a CTA for rings: what lets the whole grid be resident at once (up to 2 CTAs per SM), so that one
 // CTA's epilogue overlaps its neighbour's loads.
 int stream_budget(long long grid, int sms, int* per_sm_out = nullptr) {
@@ -1896,8 +1927,13 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
       if (kb > kb_max) kb_max = kb;
     }
   const int staging = p.mma_n * kRowTile * 4;
-  int per_sm = 1;
-  int budget = stream_budget(grid, sms, &per_sm);
+  int per_sm = 1, handover = 0;
+  for (int i = 0; i < p.n_seg; ++i) {
+    const int bytes = handover_bytes(p.M, p.seg[i].split);
+    if (bytes > handover) handover = bytes;
+  }
+  p.handover = handover > 0 ? 1 : 0;
+  int budget = stream_budget(grid, sms, &per_sm) - handover;
   // Leave room for the NEXT kernel's CTAs: with programmatic dependent launch they
   // become resident while this kernel still runs and pre-load their weights.
   if (g_opt_smem_cap > 0 && budget > g_opt_smem_cap) budget = (int)g_opt_smem_cap;
@@ -1929,7 +1965,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   p.b_stages = b_stages;
   int tile_bytes = stages * kATileBytes + b_stages * b_tile;
   if (tile_bytes < staging) tile_bytes = staging;
-  const int smem = tile_bytes + kBarrierBytes + 1024;
+  const int smem = tile_bytes + kBarrierBytes + handover + 1024;
   if (smem > kMaxSmem) return kErrUnsupported;
   const int epi = epilogue_of(p, false);
   if (quant && epi != kPlain && epi != kResidual) return kErrUnsupported;
@@ -2747,7 +2783,7 @@ extern "C" int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate,
   const int sms = device_sms();
   if (sms <= 0) return kErrLaunch;
   const int blocks = (int)((I + kBK - 1) / kBK), split = split_for_weight(N, blocks);
-  if (cast_stages(stream_budget((N + kRowTile - 1) / kRowTile * split, sms), (int)((M + 15) / 16 * 16) * kBK,
+  if (cast_stages(stream_budget((N + kRowTile - 1) / kRowTile * split, sms) - handover_bytes(M, split), (int)((M + 15) / 16 * 16) * kBK,
                   (blocks + split - 1) / split) == 0)
     return kErrUnsupported;
   PairSilu pair;

@@ -427,6 +427,13 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The two halves of it; the first one orders nothing.
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // Address of the same shared-memory offset inside CTA `rank` of this cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
   uint32_t r;
@@ -439,6 +446,9 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                : "r"(addr));
   return v;
+}
+__device__ __forceinline__ void st_cluster_f1(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 __device__ __forceinline__ float ld_cluster_f1(uint32_t addr) {
   float v;

@@ -763,6 +763,29 @@ def test_prefill_gate_up_silu_equals_the_separate_kernels(Q, dt, M, I, K):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 15, 16, 17, 31, 33, 47, 48, 49])
+def test_slices_handed_over_add_up_to_the_fetched_sum(Q, M):
+    """Up to 48 rows the K slices of a tile are written into the CTA that sums them, beyond they are fetched: a row's
+    bits do not depend on which, for 2 and 4 slices, weights that end inside a tile and rows that no CTA owns."""
+    K = 4096
+    x = randn_cpu((60, K), seed=5).cuda()
+    xq, sx = Q.quantize_act(x)
+    ws = [Q.quantize_weight(randn_cpu((n, K), seed=n, scale=0.02).cuda()) for n in (8192, 4096, 1040, 16)]
+    r = randn_cpu((60, 4096), seed=6).cuda()
+    Q.set_option("decode_wide", 0)
+    try:
+        far = Q.fp8_matmul_grouped(xq, sx, ws)                       # 60 rows: fetched
+        near = Q.fp8_matmul_grouped(xq[:M].contiguous(), sx, ws)
+        assert not Q.last_gemm_launch()["wide"]
+        for a, b in zip(near, far):
+            assert torch.equal(a, b[:M])
+        assert torch.equal(Q.fp8_matmul(xq[:M].contiguous(), sx, ws[1], residual=r[:M]),
+                           Q.fp8_matmul(xq, sx, ws[1], residual=r)[:M])
+    finally:
+        Q.set_option("decode_wide", -1)
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("M,I,dt", [(1, 12288, torch.bfloat16), (6, 12288, torch.bfloat16), (7, 12288, torch.bfloat16),
                                     (5, 12288, torch.float16), (3, 12288, torch.float32), (4, 12288, torch.float32),
                                     (6, 8256, torch.bfloat16), (2, 8128, torch.bfloat16)])
