@@ -242,6 +242,95 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
 }
 
 // ---------------------------------------------------------------------------------------------
+// plain RMSNorm -> quantize of a short prompt: CTAs of four groups of 128 threads, R rows per group.  A row's
+// arithmetic is that of rmsnorm_quant_kernel; what differs is how many CTAs meet in the exchange.  With one CTA
+// per row its three atomics per CTA, all on one word pair, were most of the launch (1500 rows: 4500 of them).
+// us, one CTA per row -> this: 1500 x 4096 bf16 14.5 -> 11.5, 2300 x 4096 18.2 -> 13.4, 1000 x 4096 fp32 13.2 -> 8.6,
+// 1500 x 1024 bf16 12.5 -> 7.1, 2000 x 2560 13.1 -> 10.7, 1000 x 5120 13.7 -> 10.7.  Of fewer rows a block has four to
+// wait for where one would do: 500 x 4096 8.0 and 9.2, 700 x 4096 10.3 and 10.8 (700 x 1024 6.9 and 5.7).
+// ---------------------------------------------------------------------------------------------
+constexpr int kRowGroups = 4;
+constexpr int kGroupedRows = 768;     // more rows than these
+template <typename T, int VPT, int R>
+__global__ void __launch_bounds__(kRowGroups * kNormThreads) rmsnorm_rows_quant_kernel(const NormParams p) {
+  bq::pdl_launch_dependents();
+  __shared__ float s_red[kRowGroups][R][4];
+  extern __shared__ float4 s_gamma[];
+  const int group = threadIdx.x / kNormThreads, t = threadIdx.x - group * kNormThreads, lane = t & 31, warp = t >> 5;
+  const int n_vec = p.cols / kVec;
+  for (int v = threadIdx.x; v < n_vec; v += kRowGroups * kNormThreads) s_gamma[v] = __ldg(reinterpret_cast<const float4*>(p.gamma) + v);
+  __syncthreads();
+  const int row0 = (blockIdx.x * kRowGroups + group) * R;
+  bq::pdl_wait_prior_grids();
+  Vec4<T> x[R][VPT];
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const T* xr = reinterpret_cast<const T*>(p.x) + static_cast<long long>(row0 + k) * p.ld_x;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int v = t + i * kNormThreads;
+      x[k][i] = Vec4<T>{};
+      if (row0 + k < p.rows && v < n_vec) x[k][i] = load4(xr + v * kVec);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    float s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      if (t + i * kNormThreads < n_vec) {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+          const float f = widen(x[k][i].v[j]);
+          s = __fmaf_rn(f, f, s);
+        }
+      }
+    }
+    s = warp_tree_sum(s);
+    if (lane == 0) s_red[group][k][warp] = s;
+  }
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kNormThreads) : "memory");
+  float m = 0.0f;
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const float* const r = s_red[group][k];
+    float s = __fadd_rn(__fadd_rn(r[0], r[2]), __fadd_rn(r[1], r[3]));
+    s = __fdiv_rn(s, static_cast<float>(p.cols));
+    const float rstd = rsqrtf(__fadd_rn(s, p.eps));
+    T* hr = reinterpret_cast<T*>(p.h_out) + static_cast<long long>(row0 + k) * p.ld_h;
+    const bool row_ok = row0 + k < p.rows;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int v = t + i * kNormThreads;
+      if (row_ok && v < n_vec) {
+        const float4 gv = s_gamma[v];
+        const float g[kVec] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+          const float y = __fmul_rn(g[j], __fmul_rn(rstd, widen(x[k][i].v[j])));
+          x[k][i].v[j] = narrow<T>(y);
+          m = nan_max(m, fabsf(widen(x[k][i].v[j])));
+        }
+        if (p.h_out != nullptr) store4(hr + v * kVec, x[k][i]);
+      }
+    }
+  }
+  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
+  const ScaleDiv dv(sc);
+  if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    uint8_t* qr = p.q + static_cast<long long>(row0 + k) * p.cols;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int v = t + i * kNormThreads;
+      if (v < n_vec) emit4(x[k][i], dv, qr + v * kVec, row0 + k < p.rows);
+    }
+  }
+  grid_depart(static_cast<QuantWs*>(p.ws));
+}
+
+// ---------------------------------------------------------------------------------------------
 // plain RMSNorm at prefill sizes: more rows than one co-resident grid has CTAs.  Every CTA loops
 // over rows (row arithmetic exactly as above), writes the normalised activation h, and keeps the
 // running max |h|; nobody waits for anybody: each CTA folds its max into one word with an
@@ -465,6 +554,44 @@ int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t str
   return bq::kOk;
 }
 
+// The fewest rows per CTA whose grid is resident at once; kErrTooLarge if none is.
+template <typename T, int VPT, int R>
+int launch_row_groups_of(const NormParams& p, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  const size_t smem = static_cast<size_t>(p.cols) * sizeof(float);     // gamma
+  const int threads = kRowGroups * kNormThreads;
+  const int per_sm = resident_per_sm(rmsnorm_rows_quant_kernel<T, VPT, R>, threads, smem);
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1) {
+    (void)cudaGetLastError();
+    return bq::kErrTooLarge;
+  }
+  const int grid = (p.rows + kRowGroups * R - 1) / (kRowGroups * R);
+  if (static_cast<long long>(grid) > static_cast<long long>(sms) * per_sm) return bq::kErrTooLarge;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, rmsnorm_rows_quant_kernel<T, VPT, R>, p);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
+  return bq::kOk;
+}
+template <typename T, int VPT>
+int launch_row_groups(const NormParams& p, cudaStream_t stream) {
+  if (static_cast<size_t>(p.cols) * sizeof(float) > 40 * 1024) return bq::kErrTooLarge;
+  int rc = launch_row_groups_of<T, VPT, 1>(p, stream);
+  if constexpr (VPT * sizeof(T) <= 32) {           // two rows of the longest fp32 ones would not stay in registers
+    if (rc == bq::kErrTooLarge) rc = launch_row_groups_of<T, VPT, 2>(p, stream);
+  }
+  return rc;
+}
+
 template <typename T>
 int launch_rmsnorm(const NormParams& p, cudaStream_t stream) {
   const int per_thread = (p.cols / kVec + kNormThreads - 1) / kNormThreads;
@@ -476,6 +603,13 @@ int launch_rmsnorm(const NormParams& p, cudaStream_t stream) {
     if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 4>, p.rows, 4 * kNormThreads, p, stream);
     if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 4>, p.rows, 4 * kNormThreads, p, stream);
   }
+  int rc = bq::kErrTooLarge;
+  if (p.rows <= kGroupedRows) {}
+  else if (per_thread <= 2) rc = launch_row_groups<T, 2>(p, stream);
+  else if (per_thread <= 4) rc = launch_row_groups<T, 4>(p, stream);
+  else if (per_thread <= 8) rc = launch_row_groups<T, 8>(p, stream);
+  else if (per_thread <= 16) rc = launch_row_groups<T, 16>(p, stream);
+  if (rc != bq::kErrTooLarge) return rc;
   if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2, 1>, p.rows, kNormThreads, p, stream);
   if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4, 1>, p.rows, kNormThreads, p, stream);
   if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 1>, p.rows, kNormThreads, p, stream);

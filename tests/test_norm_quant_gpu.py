@@ -48,6 +48,26 @@ def test_rms_norm_quant_is_bit_identical(Q, dt, shape):
         assert Q.rms_norm_quant(x, gamma, EPS).dense is None
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("rows,cols", [(768, 4096), (769, 4096), (770, 64), (803, 5120), (1777, 4096), (2366, 4096), (1003, 8192),
+                                       (899, 516)])
+def test_rms_norm_quant_with_several_rows_per_block(Q, dt, rows, cols):
+    """Beyond 768 rows a block normalises four or eight rows: both counts, blocks with rows left over, vectors that end
+    inside a thread's share, strided rows, and a NaN in the last row."""
+    x = randn_cpu((rows, 2 * cols), seed=rows, dtype=dt, scale=2.0).cuda()[:, :cols]
+    gamma = _gamma(cols, 7)
+    ref = TS.rms_norm(x, gamma, EPS)
+    for keep in (True, False):
+        qa = Q.rms_norm_quant(x, gamma, EPS, keep_dense=keep)
+        if keep:
+            assert int((u8(qa.dense) != u8(ref)).sum()) == 0
+        _same(qa, ref, f"{rows} x {cols}")
+    x[-1, -1] = float("nan")
+    assert Q.rms_norm_quant(x, gamma, EPS).scale.isnan().all()
+    assert not Q.rms_norm_quant(x[:-1], gamma, EPS).scale.isnan().any()
+    assert Q.device_status() == 0
+
+
 def test_rms_norm_quant_many_rows_of_real_width(Q):
     """2048 independent rows x 3 magnitudes: a reduction-order mismatch shows up as a last-bit
     difference in a few percent of rows, so this is the statistical net under the exact cases."""
