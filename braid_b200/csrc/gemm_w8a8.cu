@@ -1830,7 +1830,8 @@ int split_for_weight(long long n_rows, int k_blocks) {
 
 // Few rows: is the launch whose CTAs quantize the activation for themselves the faster form?  It saves a launch;
 // every CTA reads all of the activation and casts its K slice, and its weights wait for that.  So what counts is
-// the bytes a CTA reads plus those it casts.  us in a graph, one launch and two, at the bytes of the activation and the
+// the bytes a CTA reads plus those it casts.  us in a graph, one launch and two (before the slices were
+// handed over and whole warps walked the issue loops; both sides are faster since), at the bytes of the activation and the
 // K slices of the weight: 48 KB in 4 (6 rows of 4096 x 4096) 9.8 and 9.8, 64 KB in 4 (8 rows) 10.0 and 9.8; 40 KB in 2
 // (5 rows of 8192 x 4096) 12.6 and 12.7, 48 KB in 2 (6 rows) 13.6 and 12.9; 24 KB in 1 (6 rows of 12288 x 2048) 10.7
 // and 10.9, 32 KB in 1 (8 rows) 11.3 and 10.8, 64 KB in 1 (16 rows) 13.9 and 10.9.  A weight of 64 CTAs or fewer
