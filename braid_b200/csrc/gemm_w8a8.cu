@@ -1075,8 +1075,11 @@ __global__ void wait_flag_scale_kernel(const unsigned int* flag, unsigned int* s
 // at M and N by the tensor map); the next piece waits until the store has read the box.  Outputs whose base or row pitch is not 16-byte aligned
 // cannot be described to TMA: the same staged box is then written with coalesced 128-byte
 // row segments by the warp itself.
-constexpr int kPairStageBytes = 2 * kATileBytes;    // 16 KB activation rows + 16 KB weight rows
-constexpr int kPairStages = 6;
+// Ring: six stages of 16 KB of activation rows and 16 KB of weight rows, or, where no tile of the launch is wider than
+// 128 columns, eight of 16 + 8 KB: a launch of one round waits for its copies, not for its MMAs.  us at 333 rows, six
+// stages -> eight: 4096 x 12288 28.3 -> 24.2, 4096 x 4096 13.7 -> 12.5.
+constexpr int kPairRingBytes = 6 * 2 * kATileBytes;
+constexpr int kPairMaxStages = 8;
 constexpr int kPairTile = 256;
 constexpr int kPairEpiWarps = 8;                    // two per TMEM lane quarter
 constexpr int kTileThreads = 64 + 32 * kPairEpiWarps;
@@ -1330,19 +1333,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   const int push_n = EPI == kAny ? p.push.n : 0;
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
-  const uint32_t bar_base = base + kPairStages * kPairStageBytes;
-  auto a_tile = [&](int s) { return base + s * kPairStageBytes; };
-  auto b_tile = [&](int s) { return base + s * kPairStageBytes + kATileBytes; };
+  const uint32_t bar_base = base + kPairRingBytes;
+  const int stages = p.stages;
+  const uint32_t stage_bytes = stages == kPairMaxStages ? kPairRingBytes / kPairMaxStages : 2 * kATileBytes;
+  auto a_tile = [&](int s) { return base + s * stage_bytes; };
+  auto b_tile = [&](int s) { return base + s * stage_bytes + kATileBytes; };
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (kPairStages + s); };
-  auto acc_full = [&](int b) { return bar_base + 8u * (2 * kPairStages + b); };
-  auto acc_empty = [&](int b) { return bar_base + 8u * (2 * kPairStages + 2 + b); };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (kPairMaxStages + s); };
+  auto acc_full = [&](int b) { return bar_base + 8u * (2 * kPairMaxStages + b); };
+  auto acc_empty = [&](int b) { return bar_base + 8u * (2 * kPairMaxStages + 2 + b); };
   volatile uint32_t* const tmem_slot = reinterpret_cast<volatile uint32_t*>(
-      base_ptr + kPairStages * kPairStageBytes + 8 * (2 * kPairStages + 4));
+      base_ptr + kPairRingBytes + 8 * (2 * kPairMaxStages + 4));
   volatile uint32_t* const abort_flag = tmem_slot + 1;
   // store boxes of the epilogue warps, after the barrier block (1024-byte aligned: the swizzle
   // pattern of a box is a function of its address bits)
-  uint8_t* const staging = base_ptr + kPairStages * kPairStageBytes + kBarrierBytes;
+  uint8_t* const staging = base_ptr + kPairRingBytes + kBarrierBytes;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank());     // 0 = leader of the pair
@@ -1352,12 +1357,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   // output columns per tile: 128 of h in the SiLU form, in the plain form what the host chose for the
   // segment (the sums are the same either way)
   auto tile_cols = [&](const Segment& g) { return silu ? kPairTile / 2 : g.un; };
-  float* const s_amax = reinterpret_cast<float*>(base_ptr + kPairStages * kPairStageBytes + 512);
+  float* const s_amax = reinterpret_cast<float*>(base_ptr + kPairRingBytes + 512);
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm_x);
     for (int i = 0; i < p.n_seg; ++i) tma_prefetch_desc(&tm_w.w[i]);
-    for (int s = 0; s < kPairStages; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(full_bar(s), 1);     // the leader's producer arrives, bytes of both CTAs expected
       mbar_init(empty_bar(s), 1);    // one MMA commit per use
     }
@@ -1406,7 +1411,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         mbar_expect_tx(expect, full_bar(s), bytes);
         tma_load_2d_pair(issue, a_tile(s), x_map, full_bar(s), kb * kBK, m0, pol);
         tma_load_2d_pair(issue, b_tile(s), w_map, full_bar(s), kb * kBK, n0, pol);
-        if (++s == kPairStages) { s = 0; phase ^= 1u; }
+        if (++s == stages) { s = 0; phase ^= 1u; }
       }
     }
     if (!ok) *abort_flag = 1;
@@ -1433,7 +1438,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
             if (!ready && !mbar_wait(full_bar(s), phase)) { ok = false; break; }
             const uint64_t da = smem_desc_sw128(a_tile(s)), db = smem_desc_sw128(b_tile(s));
             const uint32_t empty = empty_bar(s);
-            if (++s == kPairStages) { s = 0; phase ^= 1u; }
+            if (++s == stages) { s = 0; phase ^= 1u; }
             // look at the next stage's barrier now: the answer arrives while this one's MMAs are issued
             ready = mbar_test(full_bar(s), phase);
             tc_fence_after();
@@ -2194,8 +2199,8 @@ int launch_pair(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
                 cudaStream_t stream) {
   const int sms = device_sms();
   if (sms <= 0) return kErrLaunch;
-  const int smem = kPairStages * kPairStageBytes + kBarrierBytes + kPairStagingBytes + 1024;
-  static_assert(kPairStages * kPairStageBytes + kBarrierBytes + kPairStagingBytes + 1024 <= kMaxSmem,
+  const int smem = kPairRingBytes + kBarrierBytes + kPairStagingBytes + 1024;
+  static_assert(kPairRingBytes + kBarrierBytes + kPairStagingBytes + 1024 <= kMaxSmem,
                 "pair kernel: pipeline + store boxes exceed the shared memory of an SM");
   int pairs = p.total_tiles < sms / 2 ? p.total_tiles : sms / 2;
   if (pairs < 1) pairs = 1;
@@ -2204,7 +2209,10 @@ int launch_pair(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
   if (epi == kAny && p.push.n == 0) return kErrUnsupported;
   if (p.push.n > 0) p.push.expected = (unsigned)(2 * pairs);   // every CTA has a tile and stores
   g_last_launch[0] = 2; g_last_launch[1] = 2 * pairs; g_last_launch[2] = 2;
-  g_last_launch[3] = kPairStages; g_last_launch[4] = smem; g_last_launch[5] = p.pair.on ? kPairTile : p.seg[0].un;
+  p.stages = kPairMaxStages;
+  for (int i = 0; i < p.n_seg; ++i)
+    if (p.pair.on || p.seg[i].un > kPairTile / 2) p.stages = 6;
+  g_last_launch[3] = p.stages; g_last_launch[4] = smem; g_last_launch[5] = p.pair.on ? kPairTile : p.seg[0].un;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);

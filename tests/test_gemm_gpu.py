@@ -166,6 +166,26 @@ def test_prefill_tiles_of_128_columns_give_the_bits_of_256(Q, M, N, K, dt):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("K", [16, 128, 768, 896, 1024, 1152, 2064])
+def test_prefill_ring_of_eight_stages_gives_the_bits_of_six(Q, K):
+    """Launches of 128-column tiles alone have eight stages: K blocks fewer than, as many as and more than either
+    ring holds, several tiles per pair, with a residual and grouped."""
+    M, N = 600, 5136
+    _, _, xq, sx, fw = _operands(Q, M, N, K, seed=K)
+    res = randn_cpu((M, N), seed=3).cuda()
+    got = {}
+    try:
+        for narrow, stages in ((0, 6), (1, 8)):
+            Q.set_option("pair_narrow", narrow)
+            got[stages] = [Q.fp8_matmul(xq, sx, fw), Q.fp8_matmul(xq, sx, fw, residual=res),
+                           *Q.fp8_matmul_grouped(xq, sx, (fw, fw))]
+            assert Q.last_gemm_launch()["stages"] == stages
+    finally:
+        Q.set_option("pair_narrow", -1)
+    assert all(torch.equal(a, b) for a, b in zip(got[6], got[8]))
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K,dt", [(1500, 4096, 1024, torch.bfloat16), (300, 400, 2048, torch.float16),
                                       (257, 192, 1024, torch.float32), (768, 4096, 4096, torch.bfloat16)])
 def test_prefill_tiles_of_192_columns_give_the_bits_of_256(Q, M, N, K, dt):
