@@ -1863,6 +1863,24 @@ bool quantize_inside_pays(int64_t M, int64_t K, int element_size, int n_seg, con
   return status == cudaStreamCaptureStatusNone;
 }
 
+// The same question where such a launch has no room beside the slices handed over (handover_bytes below), and would
+// fetch them: the longest slices that fit, one or two rows, on 82 to 160 CTAs.  us, one launch and two: 1 row of
+// 9600 x 5760 eager 13.8 and 15.2, in a graph 13.7 and 13.9; 1 row of 9472 x 14336 eager 25.0 and 26.9, 25.4 and 26.1; 5248 x
+// 14336 17.6 and 19.0, 17.6 and 17.6; 2 rows of 5120 x 11520 (45 KB) eager 15.2 and 15.6, 14.7 and 14.4; beyond
+// kInsideWork two launches win eager as well: 5 rows of 9600 x 5760 16.3 and 15.8, 2 rows of 5248 x 14336 19.4 and 18.7,
+// 1 row of 2048 x 28672 17.4 and 17.0.
+constexpr int64_t kInsideFetched = 32768;
+
+bool fetched_inside_pays(const GemmParams& p, int split, cudaStream_t stream) {
+  const int64_t bytes = (int64_t)p.M * p.quant_k * (p.out_dtype == BQ_DTYPE_F32 ? 4 : 2);
+  if (g_opt_quant_inside >= 0) return true;           // the caller has chosen
+  if (bytes + bytes / split > kInsideWork) return false;
+  if (bytes <= kInsideFetched) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) (void)cudaGetLastError();
+  return status == cudaStreamCaptureStatusNone;
+}
+
 // Where the K slices of a tile are summed.  Up to 48 rows every CTA writes its share of a tile straight from its
 // accumulator into the memory of the CTA that sums those rows, and one cluster barrier ends the exchange; more
 // rows would take the memory of too many weight tiles, and are staged and fetched between two barriers.
@@ -1939,10 +1957,11 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
     if (bytes > handover) handover = bytes;
   }
   p.handover = handover > 0 ? 1 : 0;
-  int budget = stream_budget(grid, sms, &per_sm) - handover;
+  int whole = stream_budget(grid, sms, &per_sm), budget = whole - handover;
   // Leave room for the NEXT kernel's CTAs: with programmatic dependent launch they
   // become resident while this kernel still runs and pre-load their weights.
-  if (g_opt_smem_cap > 0 && budget > g_opt_smem_cap) budget = (int)g_opt_smem_cap;
+  if (g_opt_smem_cap > 0 && whole > g_opt_smem_cap) whole = (int)g_opt_smem_cap;
+  if (budget > whole) budget = whole;
   int stages = budget / stage_bytes;            // both rings equally deep: the starting point
   if (stages > kb_max) stages = kb_max;
   if (stages > 24) stages = 24;
@@ -1965,6 +1984,10 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   if (quant) {
     b_stages = kb_max;
     stages = cast_stages(budget, b_tile, kb_max);
+    if (stages == 0 && handover > 0 && p.quant.words == nullptr && fetched_inside_pays(p, min_split, stream)) {
+      handover = p.handover = 0;
+      stages = cast_stages(whole, b_tile, kb_max);
+    }
     if (stages == 0) return kErrUnsupported;
   }
   p.stages = stages;

@@ -658,6 +658,32 @@ def test_linear_of_few_rows_in_one_launch_only_where_that_is_faster(Q, M, K, N, 
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N,dt,eager,captured", [
+    (1, 5760, 9600, torch.bfloat16, 1, 1), (3, 5888, 10240, torch.bfloat16, 1, 2), (5, 5760, 9600, torch.bfloat16, 2, 2),
+    (1, 5760, 9984, torch.float32, 1, 1), (1, 11392, 4864, torch.float16, 1, 1), (2, 11776, 5120, torch.bfloat16, 1, 2),
+    (1, 14336, 8192, torch.bfloat16, 1, 1), (1, 14208, 5248, torch.bfloat16, 1, 1), (2, 14336, 8192, torch.bfloat16, 2, 2),
+    (1, 28672, 2048, torch.bfloat16, 2, 2), (1, 14464, 8192, torch.bfloat16, 2, 2)])
+def test_linear_of_few_rows_whose_slices_leave_no_room_to_be_handed_over(Q, M, K, N, dt, eager, captured):
+    """Slices as long as they can be: the launch fetches the partial sums, where that is still faster than two
+    launches; the bits of quantizer and GEMM apart either way."""
+    fw = Q.quantize_weight(randn_cpu((N, K), seed=1, scale=0.02).cuda())
+    x, r = randn_cpu((M, K), seed=M, dtype=dt).cuda(), randn_cpu((M, N), seed=2, dtype=dt).cuda()
+    n0 = Q.launch_count()
+    got = Q.linear(x, fw, residual=r)
+    assert Q._NATIVE is None or Q.launch_count() - n0 == eager
+    xq, sx = Q.quantize_act(x)
+    want = Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=r)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        n0 = Q.launch_count()
+        again = Q.linear(x, fw, residual=r)
+        assert Q._NATIVE is None or Q.launch_count() - n0 == captured
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and torch.equal(again, want)
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("key,value,back", [("stream_max_m", 8, 256), ("decode_wide", 1, -1), ("decode_stages", 2, 0),
                                             ("decode_b_stages", 1, 0)])
 def test_linear_of_few_rows_leaves_forced_kernels_to_two_launches(Q, key, value, back):
