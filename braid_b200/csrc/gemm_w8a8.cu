@@ -1687,6 +1687,7 @@ long long g_opt_pdl = 1;   // programmatic dependent launch on by default
 long long g_opt_b_stages = 0;   // activation ring depth: 0 = heuristic, -1 = as deep as the weight ring
 long long g_opt_quant_inside = -1;   // bytes of an activation that every CTA quantizes for itself (-1 by rule)
 long long g_opt_smem_cap = 0;   // 0 = no cap on pipeline bytes per CTA
+thread_local long long g_fail_in = 0;   // tests: so many weight-streaming launches from now, one is not made
 thread_local int g_argmax_slots = 0;     // pairs per batch row the last launch wrote (greedy pick)
 thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
 
@@ -2035,6 +2036,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
 #endif
+  if (g_fail_in > 0 && --g_fail_in == 0) return kErrLaunch;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm_x, tm_xd, maps, p, tile_bytes);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
@@ -2277,6 +2279,7 @@ int bq::gemm_set_option(const char* key, long long value) {
     g_opt_quant_inside = value < 0 ? -1 : value;
     return kOk;
   }
+  if (strcmp(key, "fail_stream_launch") == 0) { g_fail_in = value; return kOk; }
   if (strcmp(key, "decode_smem_cap") == 0) { g_opt_smem_cap = value; return kOk; }
   if (strcmp(key, "decode_wide") == 0) { g_opt_wide = value < 0 ? -1 : (value ? 1 : 0); return kOk; }
   if (strcmp(key, "decode_cta_target") == 0) {
@@ -2840,7 +2843,11 @@ extern "C" int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate,
   const int rc = run_grouped(nullptr, nullptr, M, I, 1, wds, sds, ys, Nd, ldys, act_dtype, ws, ws_bytes, stream,
                              residual != nullptr ? rs : nullptr, residual != nullptr ? ldrs : nullptr, nullptr, 0, nullptr,
                              nullptr, nullptr, &qi);
-  return rc == kErrUnsupported ? kErrLaunch : rc;      // cannot be: checked above
+  if (rc == kOk) return kOk;
+  // The first launch leaves max |h| in the scratch and only the second returns it to zero; whoever takes the scratch next
+  // would start from it.
+  if (cudaMemsetAsync(ws, 0, 8, static_cast<cudaStream_t>(stream)) != cudaSuccess) (void)cudaGetLastError();
+  return rc == kErrUnsupported ? kErrLaunch : rc;      // unsupported cannot be: checked above
 }
 
 extern "C" int bq_gate_up_silu_w8a8(const void* xq, const float* sx, const void* wq_gate,

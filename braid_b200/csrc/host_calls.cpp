@@ -165,7 +165,7 @@ PyObject* pair(const at::Tensor& a, const at::Tensor& b) {
   PyTuple_SET_ITEM(r, 1, wrap(b));
   return r;
 }
-// A status other than OK: nothing was launched by that call, and quant.py makes it again and raises.
+// A status other than OK: that call launched nothing whose result is kept, and quant.py makes it again and raises.
 PyObject* refused() {
   g_launches.fetch_sub(1, std::memory_order_relaxed);
   Py_RETURN_NONE;

@@ -432,7 +432,8 @@ int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const void* wq_g
  *   residual   optional [M, N], row stride ld_res, added after y has been rounded to its type; or NULL
  *   h          device, [M, I] of act_dtype, contiguous, 16-byte aligned (written and read)
  *   y          device, [M, N] of act_dtype, row stride ldy
- *   ws         16 bytes, zero before the first call, self-resetting (as for bq_quantize_act)
+ *   ws         16 bytes, zero before the first call, self-resetting (as for bq_quantize_act), also where the second
+ *              launch cannot be made (BQ_ERR_LAUNCH)
  * Returns BQ_ERR_UNSUPPORTED, with nothing launched, where the separate calls are to be used (more rows, small
  * down weights, slices of h too long for shared memory, a layout forced by an option, shapes and alignments they refuse as well).
  */
@@ -621,6 +622,8 @@ int bq_read_device_status(void* ws, void* stream, int* status_out);
  * bq_set_option("push_tma", 0/1)        prefill push epilogue by bulk tensor stores (default 1) or 16-byte plain stores
  * bq_set_option("pair_narrow", v)       prefill kernel: columns of a plain launch's tiles, -1 = by what evens out the
  *                                       rounds, 0 = 256, 1 = 128, else 64, 128, 192 or 256; same results either way
+ * bq_set_option("fail_stream_launch", v) 0 = none, else the v-th weight-streaming launch of the calling thread from now on
+ *                                       is not made and reports BQ_ERR_LAUNCH (failure injection on the host)
  * Returns BQ_ERR_BAD_ARG for an unknown key.
  */
 int bq_set_option(const char* key, int64_t value);

@@ -865,6 +865,33 @@ def test_mlp_of_few_rows_casts_h_in_the_down_projection(Q, M, I, dt):
     assert Q.device_status() == 0
 
 
+def test_mlp_of_few_rows_leaves_its_scratch_clean_when_the_second_launch_fails(Q):
+    """The maximum of h stays in the scratch between the two launches: a second one that cannot be made (injected on the
+    host) returns it to zero, and the call is made again by the separate launches."""
+    from braid_b200 import _lib
+    H, I = 4096, 8192
+    mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
+    wg, wu, wd = mk(I, H, 3), mk(I, H, 4), mk(H, I, 5)
+    x = randn_cpu((2, H), seed=1).cuda()
+    xq, sx = Q.quantize_act(x)
+    want = Q.mlp_forward(x, wg, wu, wd)
+    lib, h, y = _lib.load(), torch.empty(2, I, device="cuda", dtype=x.dtype), torch.empty_like(x)
+    slot = torch.zeros(4, device="cuda", dtype=torch.int32)
+    call = lambda: lib.bq_mlp_w8a8(  # noqa: E731
+        xq.data_ptr(), sx.data_ptr(), *[w.data.data_ptr() for w in (wg, wu, wd)], *[w.scale.data_ptr() for w in (wg, wu, wd)],
+        None, 0, 2, H, I, H, 1, h.data_ptr(), y.data_ptr(), H, slot.data_ptr(), 16, Q._stream_ptr(x.device))
+    try:
+        Q.set_option("fail_stream_launch", 2)
+        assert call() == _lib.BQ_ERR_LAUNCH
+        assert slot.tolist() == [0, 0, 0, 0] and h.abs().max() > 0         # the first launch ran
+        assert call() == _lib.BQ_OK and torch.equal(y, want) and slot.tolist() == [0, 0, 0, 0]
+        Q.set_option("fail_stream_launch", 2)
+        assert torch.equal(Q.mlp_forward(x, wg, wu, wd), want)
+    finally:
+        Q.set_option("fail_stream_launch", 0)
+    assert Q.device_status() == 0
+
+
 def test_paired_mlp_equals_the_four_launch_mlp_and_replays(Q):
     H, I = 4096, 12288
     mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
