@@ -61,6 +61,7 @@ SIGNATURES = {
                                      _vp, _sz, _vp]),
     "bq_gate_up_silu_quant_w8a8": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _int, _vp,
                                           _vp, _vp, _sz, _vp]),
+    "bq_mlp_w8a8_takes": (_int, [_i64, _i64, _i64, _int]),
     "bq_mlp_w8a8": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _vp,
                            _i64, _vp, _sz, _vp]),
     "bq_linear_w8a8": (_int, [_vp, _int, _i64, _i64, _int, ctypes.POINTER(_vp), ctypes.POINTER(_vp), _vp, _i64,

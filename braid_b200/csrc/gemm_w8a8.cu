@@ -1912,14 +1912,6 @@ int cast_stages(int budget, int b_tile, int kb_max) {
   return stages < (kb_max < 4 ? kb_max : 4) || 2 * stages + kb_max + 1 > 100 ? 0 : stages;
 }
 
-// Few rows: where the CTAs of the down projection cast h for themselves.  It takes the grid-wide exchange and the
-// cast out of the gate/up launch, behind whose stream HBM idles for them; down's CTAs do the cast while
-// their first weights arrive, as long as one round of loads of 4 chunks a thread covers a slice (6 rows of a 16-bit
-// type; each round is 2 to 3 us, and 5 chunks spill).  Four graphed layers, us, before and after: hidden 4096,
-// 1 row 215.7 -> 202.5, 4 rows 235.2 -> 220.1, 6 rows 237.5 -> 229.1, 8 rows 240.5 and 238.3, 16 rows 249 and 257.  A
-// smaller down weight has arrived before the cast is done: hidden 2560 (20 MB), 4 rows 241.8 and 241.3, 8 rows
-// 312.3 and 313.8; hidden 2048 (13 MB), 1 row 123.7 and 124.5.
-
 int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightMaps& maps,
                   GemmParams& p, cudaStream_t stream) {
   const int sms = device_sms();
@@ -2798,6 +2790,40 @@ extern "C" int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const
                      nullptr, nullptr, &pair, split);
 }
 
+// Few rows: where the CTAs of the down projection cast h for themselves.  It takes the grid-wide exchange and the
+// cast out of the gate/up launch, behind whose stream HBM idles for them; down's CTAs do the cast while their first
+// weights arrive, 4 chunks of 16 values a thread and round of loads (5 spill), a round 2 to 3 us.
+//
+// Rows: us of one MLP in a graph, separate launches -> this.  One round, 4096 x 12288: 1 row 34.4 -> 30.9, 4 rows 34.8 ->
+// 32.9, 6 rows 35.5 -> 33.8.  Two: 6 rows of 4096 x 14336 39.5 -> 38.4, of 3584 x 18944 43.8 -> 42.0; of 8192 x 12288
+// 4 rows 58.9 -> 58.2, 6 rows 58.9 and 59.9.  Three: 6 rows of 6144 x 14080 52.2 and 54.1, 1 row 51.7 -> 49.6.  The last
+// two lose less than what a call made outside a graph saves where gate/up has more CTAs than are resident at once and
+// would go through a [M, 2I] buffer: 6 rows of 4096 x 28160 66.5 and 68.3 in a graph, 87.8 -> 68.2 eager.  Four layers
+// of hidden 4096, before slices were handed over: 8 rows 240.5 and 238.3, 16 rows 249 and 257.
+// Weights: a smaller down weight has arrived before the cast is done.  Hidden 2560 (20 MB), four layers: 4 rows 241.8 and
+// 241.3, 8 rows 312.3 and 313.8; hidden 2048 (13 MB), 1 row 123.7 and 124.5.
+// Width: the slice of h, in tiles padded to 16 rows, may take half of the rings' memory (see cast_stages) and has to leave
+// four weight tiles.
+namespace {
+bool mlp_sizes_go(int64_t M, int64_t I, int64_t N, int act_dtype) {
+  return M > 0 && I > 0 && N > 0 && I <= 0x3fffff00LL && N <= 0x7fffff00LL && I % (kRowTile / 2) == 0 && N % 16 == 0 &&
+         M <= (act_dtype == BQ_DTYPE_F32 ? BQ_MLP_MAX_ROWS / 2 : BQ_MLP_MAX_ROWS) && I * N >= BQ_MLP_MIN_WEIGHT &&
+         M <= g_opt_stream_max_m && g_opt_wide <= 0 && g_opt_stages <= 0 && g_opt_b_stages == 0 && g_opt_smem_cap <= 0 &&
+         g_opt_quant_inside < 0;
+}
+bool mlp_slice_fits(int64_t M, int64_t I, int64_t N, int sms) {
+  const int blocks = (int)((I + kBK - 1) / kBK), split = split_for_weight(N, blocks);
+  const int budget = stream_budget((N + kRowTile - 1) / kRowTile * split, sms) - handover_bytes(M, split);
+  return cast_stages(budget, (int)((M + 15) / 16 * 16) * kBK, (blocks + split - 1) / split) > 0;
+}
+}  // namespace
+
+extern "C" int bq_mlp_w8a8_takes(int64_t M, int64_t I, int64_t N, int act_dtype) {
+  if (!mlp_sizes_go(M, I, N, act_dtype)) return 0;
+  const int sms = device_sms();
+  return sms > 0 && mlp_slice_fits(M, I, N, sms) ? 1 : 0;
+}
+
 extern "C" int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate, const void* wq_up, const void* wq_down,
                            const float* sw_gate, const float* sw_up, const float* sw_down, const void* residual,
                            int64_t ld_res, int64_t M, int64_t K, int64_t I, int64_t N, int act_dtype, void* h, void* y,
@@ -2808,19 +2834,14 @@ extern "C" int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate,
   if (act_dtype != BQ_DTYPE_F32 && act_dtype != BQ_DTYPE_BF16 && act_dtype != BQ_DTYPE_F16) return kErrBadArg;
   // Everything the second launch would refuse is refused before the first one runs.
   const int out_align = act_dtype == BQ_DTYPE_F32 ? 16 : 8;
-  if (M * (act_dtype == BQ_DTYPE_F32 ? 4 : 2) > 2 * BQ_MLP_MAX_ROWS || I * N < BQ_MLP_MIN_WEIGHT || M > g_opt_stream_max_m || g_opt_wide > 0 || g_opt_stages > 0 || g_opt_b_stages != 0 ||
-      g_opt_smem_cap > 0 || g_opt_quant_inside >= 0)
-    return kErrUnsupported;
-  if (I % (kRowTile / 2) || N % 16 || I > 0x3fffff00LL || N > 0x7fffff00LL || !aligned_to(wq_up, 16) ||
-      !aligned_to(wq_down, 16) || !aligned_to(h, 16) || ldy < N || ldy % 4 || !aligned_to(y, out_align))
+  if (!aligned_to(wq_up, 16) || !aligned_to(wq_down, 16) || !aligned_to(h, 16) || ldy < N || ldy % 4 ||
+      !aligned_to(y, out_align))
     return kErrUnsupported;
   if (residual != nullptr && (ld_res < N || ld_res % 4 || !aligned_to(residual, out_align))) return kErrUnsupported;
+  if (!mlp_sizes_go(M, I, N, act_dtype)) return kErrUnsupported;
   const int sms = device_sms();
   if (sms <= 0) return kErrLaunch;
-  const int blocks = (int)((I + kBK - 1) / kBK), split = split_for_weight(N, blocks);
-  if (cast_stages(stream_budget((N + kRowTile - 1) / kRowTile * split, sms) - handover_bytes(M, split), (int)((M + 15) / 16 * 16) * kBK,
-                  (blocks + split - 1) / split) == 0)
-    return kErrUnsupported;
+  if (!mlp_slice_fits(M, I, N, sms)) return kErrUnsupported;
   PairSilu pair;
   memset(&pair, 0, sizeof(pair));
   pair.wq_up = wq_up;

@@ -58,6 +58,7 @@ struct Lib {
   decltype(&bq_project_mixed) project_mixed;
   decltype(&bq_gate_up_silu_quant_w8a8) gate_up_silu_quant;
   decltype(&bq_gate_up_silu_w8a8) gate_up_silu;
+  decltype(&bq_mlp_w8a8_takes) mlp_takes;
   decltype(&bq_mlp_w8a8) mlp;
   decltype(&bq_lm_head_argmax) lm_head_argmax;
   decltype(&bq_lm_head_argmax_workspace_bytes) lm_head_argmax_workspace;
@@ -562,7 +563,8 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
        !aligned(residual.data_ptr(), out == at::kFloat ? 16 : 8) || recorded(residual)))
     Py_RETURN_NONE;
   int rc;
-  if (M <= BQ_MLP_MAX_ROWS && I * N >= BQ_MLP_MIN_WEIGHT) {        // both products in one call, where that form takes them
+  // both products in one call, where that form takes them: asked before anything is allocated
+  if (M <= BQ_MLP_MAX_ROWS && g_lib.mlp_takes(M, I, N, code) != 0) {
     const at::Tensor act = empty(h, {M, I}, out), y = empty(h, {M, N}, out);
     void* slot = take_slot(h.dev);
     {
@@ -662,6 +664,7 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !get("bq_sigmoid_mul_dense_scale", g_lib.sigmoid_mul_dense_scale) ||
       !get("bq_gemm_w8a8_grouped", g_lib.gemm_grouped) || !get("bq_gemm_w8a8_residual", g_lib.gemm_residual) ||
       !get("bq_linear_w8a8", g_lib.linear) || !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_w8a8", g_lib.gate_up_silu_quant) || !get("bq_mlp_w8a8", g_lib.mlp) ||
+      !get("bq_mlp_w8a8_takes", g_lib.mlp_takes) ||
       !get("bq_gate_up_silu_w8a8", g_lib.gate_up_silu) || !get("bq_lm_head_argmax", g_lib.lm_head_argmax) ||
       !get("bq_lm_head_argmax_workspace_bytes", g_lib.lm_head_argmax_workspace))
     return nullptr;

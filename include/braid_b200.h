@@ -434,11 +434,19 @@ int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const void* wq_g
  *   y          device, [M, N] of act_dtype, row stride ldy
  *   ws         16 bytes, zero before the first call, self-resetting (as for bq_quantize_act), also where the second
  *              launch cannot be made (BQ_ERR_LAUNCH)
- * Returns BQ_ERR_UNSUPPORTED, with nothing launched, where the separate calls are to be used (more rows, small
- * down weights, slices of h too long for shared memory, a layout forced by an option, shapes and alignments they refuse as well).
+ * Returns BQ_ERR_UNSUPPORTED, with nothing launched, where bq_mlp_w8a8_takes says 0, for K, leading dimensions or
+ * addresses that the separate calls refuse as well, and for a workspace they refuse BQ_ERR_WORKSPACE.
+ *
+ * bq_mlp_w8a8_takes: 1 where these sizes go this way on the current device, without a launch.  0 for more rows
+ * (BQ_MLP_MAX_ROWS, fp32 half as many), for a small down weight (BQ_MLP_MIN_WEIGHT), where an option forces a layout,
+ * I not a multiple of 64 or N not of 16, and where a CTA's K slice of h is too long for shared memory.  On 148 SMs
+ * a down weight of up to 4736 rows (4 slices) takes I <= 28160, of up to 5120 rows I <= 10752, of up to 9472 rows (2
+ * slices) I <= 14080, of up to 10240 rows I <= 5376, of up to 18944 rows (1 slice) I <= 7168: of the MLPs with
+ * I = 3 x hidden those of hidden 3350 to 4736.
  */
 #define BQ_MLP_MAX_ROWS 6                /* fp32: half as many */
 #define BQ_MLP_MIN_WEIGHT (32 << 20)     /* values of the down weight */
+int bq_mlp_w8a8_takes(int64_t M, int64_t I, int64_t N, int act_dtype);
 int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate, const void* wq_up, const void* wq_down,
                 const float* sw_gate, const float* sw_up, const float* sw_down, const void* residual, int64_t ld_res,
                 int64_t M, int64_t K, int64_t I, int64_t N, int act_dtype, void* h, void* y, int64_t ldy,

@@ -865,6 +865,28 @@ def test_mlp_of_few_rows_casts_h_in_the_down_projection(Q, M, I, dt):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M,H,I,dt,takes", [(2, 4096, 8192, torch.bfloat16, 1), (4, 4096, 8192, torch.float32, 0),
+                                            (2, 5120, 11328, torch.bfloat16, 0), (2, 4096, 28224, torch.bfloat16, 0)])
+def test_mlp_of_few_rows_that_is_refused_allocates_nothing_for_it(Q, M, H, I, dt, takes):
+    """h and y where both products are one call, else codes, scale and y: what is refused by its rows or its width is
+    known to be before any of them is made."""
+    if Q._NATIVE is None:
+        pytest.skip("the native calls are not loaded")
+    from braid_b200 import _lib
+    codes = lambda n, k: Q.FP8Weight(torch.zeros(n, k, device="cuda", dtype=torch.uint8).view(Q.FP8),  # noqa: E731
+                                     torch.ones(1, 1, device="cuda"), (n, k))
+    wg, wu, wd = codes(I, H), codes(I, H), codes(H, I)
+    assert _lib.load().bq_mlp_w8a8_takes(M, I, H, {torch.bfloat16: 1, torch.float32: 0}[dt]) == takes
+    x = Q.QuantizedActivation(*Q.quantize_act(randn_cpu((M, H), seed=1, dtype=dt).cuda()), (M, H), dt)
+    if I == 28224:                      # more gate/up tiles than are resident at once: four launches, made from Python
+        Q.mlp_forward(x, wg, wu, wd)
+        return
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    Q.mlp_forward(x, wg, wu, wd)
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] - before == (2 if takes else 3)
+    assert Q.device_status() == 0
+
+
 def test_mlp_of_few_rows_leaves_its_scratch_clean_when_the_second_launch_fails(Q):
     """The maximum of h stays in the scratch between the two launches: a second one that cannot be made (injected on the
     host) returns it to zero, and the call is made again by the separate launches."""

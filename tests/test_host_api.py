@@ -163,6 +163,32 @@ def test_linear_of_few_rows_is_refused_where_an_option_rules_it_out(lib):
     assert rc(17) == _lib.BQ_ERR_UNSUPPORTED
 
 
+def test_mlp_of_few_rows_is_refused_before_anything_is_launched(lib):
+    """Sizes, addresses and options that the two-launch MLP leaves to the separate calls.  Without a device the calls it
+    would take end with another error."""
+    from braid_b200 import _lib
+
+    def rc(M=2, K=4096, I=12288, N=4096, code=1, down=16, h=16, ldy=None, residual=None, ld_res=0):
+        return lib.bq_mlp_w8a8(16, 16, 16, 16, down, 16, 16, 16, residual, ld_res, M, K, I, N, code, h, 16,
+                               N if ldy is None else ldy, 16, 16, None)
+
+    for refused in (dict(M=7), dict(M=4, code=0), dict(I=8128), dict(I=12288 + 32), dict(N=4104), dict(down=24), dict(h=8),
+                    dict(ldy=4098), dict(ldy=4092), dict(residual=16, ld_res=4092), dict(residual=20, ld_res=4096)):
+        assert rc(**refused) == _lib.BQ_ERR_UNSUPPORTED, refused
+        sizes = {"M": 2, "I": 12288, "N": 4096, "code": 1, **refused}
+        if not set(refused) - {"M", "I", "N", "code"}:
+            assert lib.bq_mlp_w8a8_takes(sizes["M"], sizes["I"], sizes["N"], sizes["code"]) == 0, refused
+    for bad in (dict(M=0), dict(N=0), dict(code=3), dict(h=None)):
+        assert rc(**bad) == _lib.BQ_ERR_BAD_ARG, bad
+    for key, value, back in (("stream_max_m", 1, 256), ("decode_wide", 1, -1), ("decode_stages", 2, 0), ("decode_b_stages", 2, 0),
+                             ("decode_smem_cap", 65536, 0), ("decode_quant_inside", 0, -1)):
+        assert lib.bq_set_option(key.encode(), value) == _lib.BQ_OK
+        try:
+            assert rc() == _lib.BQ_ERR_UNSUPPORTED and lib.bq_mlp_w8a8_takes(2, 12288, 4096, 1) == 0, key
+        finally:
+            assert lib.bq_set_option(key.encode(), back) == _lib.BQ_OK
+
+
 def test_a_missing_library_is_loud(monkeypatch, tmp_path):
     from braid_b200 import _lib, quant
     monkeypatch.setattr(_lib, "_lib", None)
