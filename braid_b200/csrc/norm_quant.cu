@@ -18,9 +18,9 @@
 // rounds once more.  tests/test_norm_quant_gpu.py pins all of this against torch on the device.
 //
 // After the norm the values stay in registers; amax, grid-wide exchange and cast are the
-// activation quantizer's (quant_act.cu).  One CTA per token row, all of them co-resident for the exchange;
-// larger inputs are refused, and the caller takes the norm with its rows looped (bq_rmsnorm_scale,
-// bq_gated_rmsnorm_scale) and the cast pass.
+// activation quantizer's (quant_act.cu).  A CTA holds one token row, or four or eight (rmsnorm_rows_quant_kernel), and all
+// of them are co-resident for the exchange; larger inputs are refused, and the caller takes the norm with its rows
+// looped (bq_rmsnorm_scale, bq_gated_rmsnorm_scale) and the cast pass.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -243,14 +243,25 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
 
 // ---------------------------------------------------------------------------------------------
 // plain RMSNorm -> quantize of a short prompt: CTAs of four groups of 128 threads, R rows per group.  A row's
-// arithmetic is that of rmsnorm_quant_kernel; what differs is how many CTAs meet in the exchange.  With one CTA
-// per row its three atomics per CTA, all on one word pair, were most of the launch (1500 rows: 4500 of them).
-// us, one CTA per row -> this: 1500 x 4096 bf16 14.5 -> 11.5, 2300 x 4096 18.2 -> 13.4, 1000 x 4096 fp32 13.2 -> 8.6,
-// 1500 x 1024 bf16 12.5 -> 7.1, 2000 x 2560 13.1 -> 10.7, 1000 x 5120 13.7 -> 10.7.  Of fewer rows a block has four to
-// wait for where one would do: 500 x 4096 8.0 and 9.2, 700 x 4096 10.3 and 10.8 (700 x 1024 6.9 and 5.7).
+// arithmetic is that of rmsnorm_quant_kernel.  Gamma is in shared memory, not in registers, so that more rows are
+// resident at once, and a quarter or an eighth of the CTAs meet in the exchange (three atomics each on one word pair).
+// Narrow rows gain by the exchange, one launch before and now, us: 1500 x 64 bf16 10.9 -> 5.8, 1500 x 1024 12.1 -> 7.2,
+// 1300 x 2048 11.4 -> 7.8, 1036 x 4096 11.8 -> 10.8.  Wider ones gain the second launch: one CTA per row ends at 1036 rows
+// of 4096 columns (16-bit; fp32 740), beyond were a looped norm and a cast pass: 1500 x 4096 bf16 14.4 -> 11.9, 2368 x
+// 4096 18.5 -> 13.9, 1036 x 4096 fp32 13.9 -> 8.9, 1184 x 8192 bf16 18.9 -> 13.5.
+// Resident on 148 SMs: 16-bit rows of up to 2048 columns 3552, up to 4096 columns 2368, up to 8192 columns 1184; fp32
+// 3552 (1024 columns), 2368 (2048), 1184 (4096), longer ones never.  Beyond, the two launches: 2600 x 4096 bf16 19.2,
+// 1300 x 5120 bf16 15.4, 1300 x 4096 fp32 15.9, 900 x 5120 fp32 15.9.
+// Of fewer rows a block has four to wait for where one would do: 500 x 4096 8.0 and 9.2, 700 x 4096 10.3 and 10.8 (700 x
+// 1024 6.9 and 5.7).
 // ---------------------------------------------------------------------------------------------
 constexpr int kRowGroups = 4;
 constexpr int kGroupedRows = 768;     // more rows than these
+// The forms that hold more rows than the one before them.  A thread has VPT * sizeof(T) registers of a row: two rows of
+// 32 make 80 registers and one CTA of eight rows per SM, no more than two CTAs of four; one row of 64 makes one CTA of
+// four, 592 rows in all.
+template <typename T, int VPT> constexpr bool kOneRowPerGroup = VPT * sizeof(T) <= 32;
+template <typename T, int VPT> constexpr bool kTwoRowsPerGroup = VPT * sizeof(T) <= 16;
 template <typename T, int VPT, int R>
 __global__ void __launch_bounds__(kRowGroups * kNormThreads) rmsnorm_rows_quant_kernel(const NormParams p) {
   bq::pdl_launch_dependents();
@@ -585,8 +596,9 @@ int launch_row_groups_of(const NormParams& p, cudaStream_t stream) {
 template <typename T, int VPT>
 int launch_row_groups(const NormParams& p, cudaStream_t stream) {
   if (static_cast<size_t>(p.cols) * sizeof(float) > 40 * 1024) return bq::kErrTooLarge;
-  int rc = launch_row_groups_of<T, VPT, 1>(p, stream);
-  if constexpr (VPT * sizeof(T) <= 32) {           // two rows of the longest fp32 ones would not stay in registers
+  int rc = bq::kErrTooLarge;
+  if constexpr (kOneRowPerGroup<T, VPT>) rc = launch_row_groups_of<T, VPT, 1>(p, stream);
+  if constexpr (kTwoRowsPerGroup<T, VPT>) {
     if (rc == bq::kErrTooLarge) rc = launch_row_groups_of<T, VPT, 2>(p, stream);
   }
   return rc;

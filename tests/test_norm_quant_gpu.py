@@ -50,15 +50,21 @@ def test_rms_norm_quant_is_bit_identical(Q, dt, shape):
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
 @pytest.mark.parametrize("rows,cols", [(768, 4096), (769, 4096), (770, 64), (803, 5120), (1777, 4096), (2366, 4096), (1003, 8192),
-                                       (899, 516)])
+                                       (899, 516), (2369, 1024), (3552, 64), (3553, 1024), (1776, 2048), (1777, 2048),
+                                       (2369, 2048), (1184, 4096), (1185, 4096), (2369, 4096), (1185, 8192)])
 def test_rms_norm_quant_with_several_rows_per_block(Q, dt, rows, cols):
-    """Beyond 768 rows a block normalises four or eight rows: both counts, blocks with rows left over, vectors that end
-    inside a thread's share, strided rows, and a NaN in the last row."""
+    """Beyond 768 rows a block normalises four or eight rows, as long as all of them are resident at once: both counts of
+    each type, either side of each limit (seen in the launches), blocks with rows left over, vectors that end inside a
+    thread's share, strided rows, and a NaN in the last row."""
     x = randn_cpu((rows, 2 * cols), seed=rows, dtype=dt, scale=2.0).cuda()[:, :cols]
     gamma = _gamma(cols, 7)
     ref = TS.rms_norm(x, gamma, EPS)
+    per_sm = {torch.bfloat16: ((2048, 24), (4096, 16), (8192, 8)), torch.float32: ((1024, 24), (2048, 16), (4096, 8))}[dt]
+    room = next((n for c, n in per_sm if cols <= c), 0) * torch.cuda.get_device_properties(0).multi_processor_count
     for keep in (True, False):
+        n0 = Q.launch_count()
         qa = Q.rms_norm_quant(x, gamma, EPS, keep_dense=keep)
+        assert rows <= 768 or Q.launch_count() - n0 == (1 if rows <= room else 2)
         if keep:
             assert int((u8(qa.dense) != u8(ref)).sum()) == 0
         _same(qa, ref, f"{rows} x {cols}")
