@@ -101,6 +101,7 @@ SIGNATURES = {
     "bq_read_device_status": (_int, [_vp, _vp, ctypes.POINTER(_int)]),
     "bq_set_option": (_int, [ctypes.c_char_p, _i64]),
     "bq_last_gemm_launch": (_int, [ctypes.POINTER(_i64)]),
+    "bq_last_gemm_quantizes": (_int, []),
 }
 
 _lib: ctypes.CDLL | None = None

@@ -1690,6 +1690,7 @@ long long g_opt_smem_cap = 0;   // 0 = no cap on pipeline bytes per CTA
 thread_local long long g_fail_in = 0;   // tests: so many weight-streaming launches from now, one is not made
 thread_local int g_argmax_slots = 0;     // pairs per batch row the last launch wrote (greedy pick)
 thread_local long long g_last_launch[6] = {0, 0, 0, 0, 0, 0};
+thread_local int g_last_quantizes = 0;     // its CTAs cast the activation for themselves
 
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
@@ -2022,6 +2023,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_opt_pdl ? 2 : 1;
+  g_last_quantizes = quant ? 1 : 0;
   g_last_launch[0] = 0; g_last_launch[1] = grid; g_last_launch[2] = cluster;
   g_last_launch[3] = stages; g_last_launch[4] = smem; g_last_launch[5] = p.mma_n;
   g_argmax_slots = (p.seg[0].n + kRowTile - 1) / kRowTile;   // one pair per row tile
@@ -2197,6 +2199,7 @@ int launch_wide(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_opt_pdl ? 2 : 1;
+  g_last_quantizes = 0;
   g_last_launch[0] = 1; g_last_launch[1] = sh.grid; g_last_launch[2] = p.seg[0].split;
   g_last_launch[3] = sh.ring[0].w_stages; g_last_launch[4] = smem; g_last_launch[5] = 64 << sh.mode;
   g_argmax_slots = argmax_slots(sh);
@@ -2225,6 +2228,7 @@ int launch_pair(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
   // the general form of this kernel is the column-parallel one's: it adds no residual
   if (epi == kAny && p.push.n == 0) return kErrUnsupported;
   if (p.push.n > 0) p.push.expected = (unsigned)(2 * pairs);   // every CTA has a tile and stores
+  g_last_quantizes = 0;
   g_last_launch[0] = 2; g_last_launch[1] = 2 * pairs; g_last_launch[2] = 2;
   p.stages = kPairMaxStages;
   for (int i = 0; i < p.n_seg; ++i)
@@ -3044,6 +3048,8 @@ extern "C" int bq_gemm_w8a8_residual(const void* xq, const void* wq, const float
                      rs, ldrs);
 }
 
+
+extern "C" int bq_last_gemm_quantizes(void) { return g_last_quantizes; }
 
 extern "C" int bq_last_gemm_launch(int64_t out[6]) {
   if (!out) return kErrBadArg;

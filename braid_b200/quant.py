@@ -370,12 +370,14 @@ def set_option(key: str, value: int) -> None:
 
 def last_gemm_launch() -> dict:
     """What the last GEMM call of this thread launched: the kernel ("stream" for a decode batch, "pair"
-    for prefill), whether a decode batch ran on CTA pairs (`wide`), grid, split, stages, smem, tile."""
+    for prefill), whether a decode batch ran on CTA pairs (`wide`), grid, split, stages, smem, tile, and whether its
+    CTAs cast the activation for themselves (`quantizes`)."""
     out = (ctypes.c_int64 * 6)()
     _lib.check(_require_lib().bq_last_gemm_launch(out), "last_gemm_launch")
     return {"kernel": {0: "stream", 1: "stream", 2: "pair"}.get(int(out[0]), "?"), "wide": int(out[0]) == 1,
             "grid": out[1], "split": out[2],
-            "stages": out[3], "smem": out[4], "mma_n": out[5]}
+            "stages": out[3], "smem": out[4], "mma_n": out[5],
+            "quantizes": bool(_require_lib().bq_last_gemm_quantizes())}
 
 
 # ---------------------------------------------------------------------------

@@ -643,6 +643,8 @@ int bq_set_option(const char* key, int64_t value);
  * out[4]=dynamic smem bytes out[5]=batch rows of one MMA (0, 1) or weight rows of one tile (2)
  */
 int bq_last_gemm_launch(int64_t out[6]);
+/* 1 if the CTAs of that launch cast the activation for themselves (bq_linear_w8a8, the down projection of bq_mlp_w8a8). */
+int bq_last_gemm_quantizes(void);
 
 #ifdef __cplusplus
 }

@@ -670,7 +670,7 @@ def test_linear_of_few_rows_whose_slices_leave_no_room_to_be_handed_over(Q, M, K
     x, r = randn_cpu((M, K), seed=M, dtype=dt).cuda(), randn_cpu((M, N), seed=2, dtype=dt).cuda()
     n0 = Q.launch_count()
     got = Q.linear(x, fw, residual=r)
-    assert Q._NATIVE is None or Q.launch_count() - n0 == eager
+    assert Q._NATIVE is None or (Q.launch_count() - n0 == eager and Q.last_gemm_launch()["quantizes"] == (eager == 1))
     xq, sx = Q.quantize_act(x)
     want = Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=r)
     graph = torch.cuda.CUDAGraph()
@@ -837,9 +837,10 @@ def test_slices_handed_over_add_up_to_the_fetched_sum(Q, M):
                                     (6, 8256, torch.bfloat16), (2, 8128, torch.bfloat16)])
 def test_mlp_of_few_rows_casts_h_in_the_down_projection(Q, M, I, dt):
     """Up to 6 rows (3 of fp32) and from a down weight of 32 Mi values on, h is cast by the CTAs of the down projection:
-    the bits of the separate launches at either side of both lines, with a last K block that is half full, with an
-    infinity and a NaN in h, and again with the scratch that the calls before returned to zero."""
+    the bits of the separate launches at either side of both lines (seen in the last launch), with a last K block that is
+    half full, with an infinity and a NaN in h, and again with the scratch that the calls before returned to zero."""
     H = 4096
+    takes = Q._NATIVE is not None and M <= (3 if dt is torch.float32 else 6) and I * H >= 32 << 20
     mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
     wg, wu, wd = mk(I, H, 3), mk(I, H, 4), mk(H, I, 5)
     r = randn_cpu((M, H), seed=M + 1, dtype=dt).cuda()
@@ -858,15 +859,45 @@ def test_mlp_of_few_rows_casts_h_in_the_down_projection(Q, M, I, dt):
         for _ in range(2):
             n0 = Q.launch_count()
             got = Q.mlp_forward(h, wg, wu, wd)
-            assert Q.launch_count() - n0 == 2
+            assert Q.launch_count() - n0 == 2 and Q.last_gemm_launch()["quantizes"] == takes
             got_r = Q.mlp_forward(h, wg, wu, wd, residual=r)
             for a, b in ((got, want), (got_r, want_r)):
                 assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(), b.nan_to_num()), case
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M,H,I,takes", [(4, 5120, 11264, 1), (5, 5120, 11264, 0), (6, 5120, 10752, 1), (6, 4096, 14336, 1),
+                                         (1, 4736, 28160, 1), (3, 9216, 4096, 1), (2, 9216, 14144, 0), (2, 10368, 3328, 1),
+                                         (2, 10368, 7232, 0)])
+def test_mlp_of_few_rows_at_other_widths(Q, M, H, I, takes):
+    """1, 2 and 4 slices of h, one and two CTAs per SM, slices that take two rounds of loads, either side of what fits:
+    the bits of the separate launches, and which form ran."""
+    from braid_b200 import _lib
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("what fits is a matter of the SMs")
+    g = torch.Generator(device="cuda").manual_seed(H + I)
+
+    def weight(n, k):
+        codes = torch.randint(0, 0x60, (n, k), generator=g, device="cuda", dtype=torch.uint8)
+        codes |= torch.randint(0, 2, (n, k), generator=g, device="cuda", dtype=torch.uint8) << 7
+        return Q.FP8Weight(codes.view(Q.FP8), torch.full((1, 1), 1e-3, device="cuda"), (n, k))
+
+    wg, wu, wd = weight(I, H), weight(I, H), weight(H, I)
+    x, r = randn_cpu((M, H), seed=M).cuda(), randn_cpu((M, H), seed=M + 1).cuda()
+    h = Q.QuantizedActivation(*Q.quantize_act(x), x.shape, x.dtype)
+    assert _lib.load().bq_mlp_w8a8_takes(M, I, H, 1) == takes
+    got = Q.mlp_forward(h, wg, wu, wd, residual=r)
+    assert Q.last_gemm_launch()["quantizes"] == (takes == 1 and Q._NATIVE is not None)
+    Q.set_paired_mlp(False)
+    try:
+        assert torch.equal(got, Q.mlp_forward(h, wg, wu, wd, residual=r))
+    finally:
+        Q.set_paired_mlp(True)
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("M,H,I,dt,takes", [(2, 4096, 8192, torch.bfloat16, 1), (4, 4096, 8192, torch.float32, 0),
-                                            (2, 5120, 11328, torch.bfloat16, 0), (2, 4096, 28224, torch.bfloat16, 0)])
+                                            (2, 5120, 11328, torch.bfloat16, 0)])
 def test_mlp_of_few_rows_that_is_refused_allocates_nothing_for_it(Q, M, H, I, dt, takes):
     """h and y where both products are one call, else codes, scale and y: what is refused by its rows or its width is
     known to be before any of them is made."""
@@ -878,9 +909,6 @@ def test_mlp_of_few_rows_that_is_refused_allocates_nothing_for_it(Q, M, H, I, dt
     wg, wu, wd = codes(I, H), codes(I, H), codes(H, I)
     assert _lib.load().bq_mlp_w8a8_takes(M, I, H, {torch.bfloat16: 1, torch.float32: 0}[dt]) == takes
     x = Q.QuantizedActivation(*Q.quantize_act(randn_cpu((M, H), seed=1, dtype=dt).cuda()), (M, H), dt)
-    if I == 28224:                      # more gate/up tiles than are resident at once: four launches, made from Python
-        Q.mlp_forward(x, wg, wu, wd)
-        return
     before = torch.cuda.memory_stats()["allocation.all.allocated"]
     Q.mlp_forward(x, wg, wu, wd)
     assert torch.cuda.memory_stats()["allocation.all.allocated"] - before == (2 if takes else 3)
