@@ -67,9 +67,12 @@ bool g_ready = false;
 int64_t g_two_launch_from = 0;
 
 constexpr int kMaxDevices = 64;
+constexpr uint32_t kMaxSlots = 256;
 struct Scratch {
   std::atomic<uint64_t> base{0};      // device address of the slots, 0 = none yet
   std::atomic<uint32_t> next{0};
+  std::atomic<uint32_t> next_held{0};
+  std::atomic<bool> held[kMaxSlots]{};
 };
 Scratch g_scratch[kMaxDevices];
 uint32_t g_slots = 1, g_slot_bytes = 64;
@@ -80,6 +83,26 @@ void* take_slot(int dev) {
   const uint32_t slot = g_scratch[dev].next.fetch_add(1, std::memory_order_relaxed) % g_slots;
   return reinterpret_cast<void*>(g_scratch[dev].base.load(std::memory_order_relaxed) + uint64_t(slot) * g_slot_bytes);
 }
+
+// A slot for a call of two launches that leaves something in it between them.  The slots above pass from hand to
+// hand by count alone: a thread that is not scheduled between its two launches would find that another one, 256
+// calls later, has taken its slot and returned it to zero.  So these are as many slots behind those, nobody else's,
+// and each is held until both launches are in the stream.
+struct HeldSlot {
+  Scratch& pool;
+  uint32_t index;
+  explicit HeldSlot(int dev) : pool(g_scratch[dev]) {
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    do index = pool.next_held.fetch_add(1, std::memory_order_relaxed) % g_slots;
+    while (pool.held[index].exchange(true, std::memory_order_acquire));
+  }
+  ~HeldSlot() { pool.held[index].store(false, std::memory_order_release); }
+  HeldSlot(const HeldSlot&) = delete;
+  HeldSlot& operator=(const HeldSlot&) = delete;
+  void* address() const {
+    return reinterpret_cast<void*>(pool.base.load(std::memory_order_relaxed) + uint64_t(g_slots + index) * g_slot_bytes);
+  }
+};
 
 // What a call needs of its surroundings; false = leave it to quant.py.  A dual tensor is an ordinary strided
 // one with nothing in its keys to tell it by, so an open forward-mode level is asked for by itself, as quant.py does.
@@ -566,13 +589,13 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   // both products in one call, where that form takes them: asked before anything is allocated
   if (M <= BQ_MLP_MAX_ROWS && g_lib.mlp_takes(M, I, N, code) != 0) {
     const at::Tensor act = empty(h, {M, I}, out), y = empty(h, {M, N}, out);
-    void* slot = take_slot(h.dev);
     {
       NoGil no_gil;
+      const HeldSlot slot(h.dev);
       rc = g_lib.mlp(xq.data_ptr(), sx.data_ptr<float>(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(), sg.data_ptr<float>(),
                      su.data_ptr<float>(), sd.data_ptr<float>(), residual.defined() ? residual.data_ptr() : nullptr,
-                     residual.defined() ? residual.stride(0) : 0, M, K, I, N, code, act.data_ptr(), y.data_ptr(), N, slot, 16,
-                     h.stream);
+                     residual.defined() ? residual.stride(0) : 0, M, K, I, N, code, act.data_ptr(), y.data_ptr(), N,
+                     slot.address(), 16, h.stream);
     }
     if (rc == BQ_OK) g_launches.fetch_add(1, std::memory_order_relaxed);      // the slot counted one of the two
     if (rc != BQ_ERR_UNSUPPORTED) return gemm_result(y, rc);
@@ -672,11 +695,15 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   g_slot_bytes = (uint32_t)PyLong_AsUnsignedLong(a[2]);
   g_two_launch_from = PyLong_AsLongLong(a[3]);
   if (PyErr_Occurred()) return nullptr;
-  g_ready = g_slots > 0;
+  if (g_slots < 1 || g_slots > kMaxSlots) {
+    PyErr_SetString(PyExc_ValueError, "between 1 and 256 slots");
+    return nullptr;
+  }
+  g_ready = true;
   Py_RETURN_NONE;
 }
 
-// set_scratch(device, address): the zeroed slots of a device
+// set_scratch(device, address): the zeroed slots of a device, and as many that calls hold
 PyObject* set_scratch(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   BQ_ARGS(2)
   const long dev = PyLong_AsLong(a[0]);

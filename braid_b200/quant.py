@@ -177,7 +177,8 @@ _LOCK = threading.Lock()
 # Scratch for the kernels: 16-byte slots (amax word, two barrier counters, a
 # sticky status word), zeroed once and returned to zero by the kernels.  Calls
 # take slots round-robin so that launches in flight on different streams do not
-# share barrier words.
+# share barrier words.  Behind them lie as many slots for native calls of two launches that
+# leave something in theirs between the two: held by the call, never handed out meanwhile.
 _SLOTS = 256
 # From this many elements on (beyond what the one-launch prologue quantizers hold in registers)
 # the SiLU*mul and sigmoid-gate quantizers run as two launches: product + scale, then the cast.
@@ -308,7 +309,7 @@ def _scratch_for(device_index: int) -> torch.Tensor:
         with _LOCK:
             buf = _scratch.get(device_index)
             if buf is None:
-                buf = torch.zeros(_SLOTS * _SLOT_BYTES, dtype=torch.uint8,
+                buf = torch.zeros(2 * _SLOTS * _SLOT_BYTES, dtype=torch.uint8,
                                   device=torch.device("cuda", device_index))
                 torch.cuda.synchronize(device_index)
                 # the native calls first: whoever finds `buf` without the lock takes a slot from them
@@ -352,7 +353,7 @@ def device_status(device: torch.device | int | None = None) -> int:
     if buf is None:
         return 0
     torch.cuda.synchronize(idx)
-    words = buf.view(torch.int32).view(_SLOTS, _SLOT_BYTES // 4)[:, 3]
+    words = buf.view(torch.int32).view(2 * _SLOTS, _SLOT_BYTES // 4)[:, 3]
     bad = int(words.max().item())
     if bad:
         words.zero_()

@@ -433,7 +433,8 @@ int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const void* wq_g
  *   h          device, [M, I] of act_dtype, contiguous, 16-byte aligned (written and read)
  *   y          device, [M, N] of act_dtype, row stride ldy
  *   ws         16 bytes, zero before the first call, self-resetting (as for bq_quantize_act), also where the second
- *              launch cannot be made (BQ_ERR_LAUNCH)
+ *              launch cannot be made (BQ_ERR_LAUNCH).  It holds max |h| between the two launches: no other thread may use
+ *              it before this call has returned
  * Returns BQ_ERR_UNSUPPORTED, with nothing launched, where bq_mlp_w8a8_takes says 0, for K, leading dimensions or
  * addresses that the separate calls refuse as well, and for a workspace they refuse BQ_ERR_WORKSPACE.
  *

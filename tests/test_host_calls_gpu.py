@@ -134,6 +134,38 @@ def test_what_torch_follows_above_256_rows_stays_a_torch_operation(Q, weights):
     assert Q.device_status() == 0
 
 
+def test_mlp_of_two_launches_holds_a_slot_of_its_own(Q):
+    """Between its launches the maximum of h lies in its scratch: not in one that a call of another thread may be handed
+    meanwhile.  The common slots are not touched, the one it held is zero again, and threads that share a stream get
+    the bits of a lone call."""
+    import threading
+    mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
+    wg, wu, wd = mk(8192, 4096, 1), mk(8192, 4096, 2), mk(4096, 8192, 3)
+    xs = [randn_cpu((2, 4096), seed=i).cuda() * (1 + 3 * i) for i in range(4)]
+    hs = [Q.QuantizedActivation(*Q.quantize_act(x), x.shape, x.dtype) for x in xs]
+    want = [Q.mlp_forward(h, wg, wu, wd) for h in hs]
+    n0, taken = Q.launch_count(), Q._next_slot[0]
+    Q.mlp_forward(hs[0], wg, wu, wd)
+    assert Q.last_gemm_launch()["quantizes"] and Q.launch_count() - n0 == 2 and Q._next_slot[0] == taken
+    wrong = []
+
+    def work(i):
+        for _ in range(60):
+            got = [Q.mlp_forward(hs[i], wg, wu, wd) for _ in range(3)]
+            for _ in range(6):
+                Q.linear(xs[i], wg)
+            wrong.extend(1 for y in got if not torch.equal(y, want[i]))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    torch.cuda.synchronize()
+    assert not Q._scratch[0].view(torch.int32).any() and Q.device_status() == 0
+
+
 def test_native_calls_from_threads_and_streams(Q, weights):
     """Slots are counted in one place whichever way a call takes; threads on their own streams get the
     bits of a lone call.  Small projections alone: their launches do not wait for one another's CTAs.  Launches
