@@ -66,6 +66,7 @@ SIGNATURES = {
                            _i64, _vp, _sz, _vp]),
     "bq_linear_w8a8": (_int, [_vp, _int, _i64, _i64, _int, ctypes.POINTER(_vp), ctypes.POINTER(_vp), _vp, _i64,
                               ctypes.POINTER(_vp), ctypes.POINTER(_i64), ctypes.POINTER(_i64), _vp, _sz, _vp]),
+    "bq_stream_is_captured": (_int, [_vp]),
     "bq_enable_peer_access": (_int, [_int]),
     "bq_peer_alloc": (_int, [_sz, ctypes.POINTER(_vp), _vp]),
     "bq_peer_free": (_int, [_vp]),

@@ -50,6 +50,15 @@ extern "C" int bq_read_device_status(void* ws, void* stream, int* status_out) {
   return BQ_OK;
 }
 
+extern "C" int bq_stream_is_captured(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &status) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return status != cudaStreamCaptureStatusNone ? 1 : 0;
+}
+
 extern "C" int bq_enable_peer_access(int peer_device) {
   int dev = -1, can = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return BQ_ERR_LAUNCH; }

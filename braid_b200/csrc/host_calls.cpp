@@ -59,6 +59,7 @@ struct Lib {
   decltype(&bq_gate_up_silu_quant_w8a8) gate_up_silu_quant;
   decltype(&bq_gate_up_silu_w8a8) gate_up_silu;
   decltype(&bq_mlp_w8a8_takes) mlp_takes;
+  decltype(&bq_stream_is_captured) stream_is_captured;
   decltype(&bq_mlp_w8a8) mlp;
   decltype(&bq_lm_head_argmax) lm_head_argmax;
   decltype(&bq_lm_head_argmax_workspace_bytes) lm_head_argmax_workspace;
@@ -87,21 +88,27 @@ void* take_slot(int dev) {
 // A slot for a call of two launches that leaves something in it between them.  The slots above pass from hand to
 // hand by count alone: a thread that is not scheduled between its two launches would find that another one, 256
 // calls later, has taken its slot and returned it to zero.  So these are as many slots behind those, nobody else's,
-// and each is held until both launches are in the stream.
+// and each is held until both launches are in the stream.  While a graph is captured it is a common one: the graph puts both
+// launches into a stream at once whenever it is replayed, and keeps the slot for longer than it could be held.
 struct HeldSlot {
   Scratch& pool;
-  uint32_t index;
-  explicit HeldSlot(int dev) : pool(g_scratch[dev]) {
+  void* address;
+  int64_t index = -1;       // held; -1: a common one
+  HeldSlot(int dev, void* stream) : pool(g_scratch[dev]) {
+    if (g_lib.stream_is_captured(stream) != 0) {
+      address = take_slot(dev);
+      return;
+    }
     g_launches.fetch_add(1, std::memory_order_relaxed);
     do index = pool.next_held.fetch_add(1, std::memory_order_relaxed) % g_slots;
     while (pool.held[index].exchange(true, std::memory_order_acquire));
+    address = reinterpret_cast<void*>(pool.base.load(std::memory_order_relaxed) + uint64_t(g_slots + index) * g_slot_bytes);
   }
-  ~HeldSlot() { pool.held[index].store(false, std::memory_order_release); }
+  ~HeldSlot() {
+    if (index >= 0) pool.held[index].store(false, std::memory_order_release);
+  }
   HeldSlot(const HeldSlot&) = delete;
   HeldSlot& operator=(const HeldSlot&) = delete;
-  void* address() const {
-    return reinterpret_cast<void*>(pool.base.load(std::memory_order_relaxed) + uint64_t(g_slots + index) * g_slot_bytes);
-  }
 };
 
 // What a call needs of its surroundings; false = leave it to quant.py.  A dual tensor is an ordinary strided
@@ -591,11 +598,11 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const at::Tensor act = empty(h, {M, I}, out), y = empty(h, {M, N}, out);
     {
       NoGil no_gil;
-      const HeldSlot slot(h.dev);
+      const HeldSlot slot(h.dev, h.stream);
       rc = g_lib.mlp(xq.data_ptr(), sx.data_ptr<float>(), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(), sg.data_ptr<float>(),
                      su.data_ptr<float>(), sd.data_ptr<float>(), residual.defined() ? residual.data_ptr() : nullptr,
                      residual.defined() ? residual.stride(0) : 0, M, K, I, N, code, act.data_ptr(), y.data_ptr(), N,
-                     slot.address(), 16, h.stream);
+                     slot.address, 16, h.stream);
     }
     if (rc == BQ_OK) g_launches.fetch_add(1, std::memory_order_relaxed);      // the slot counted one of the two
     if (rc != BQ_ERR_UNSUPPORTED) return gemm_result(y, rc);
@@ -687,7 +694,7 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !get("bq_sigmoid_mul_dense_scale", g_lib.sigmoid_mul_dense_scale) ||
       !get("bq_gemm_w8a8_grouped", g_lib.gemm_grouped) || !get("bq_gemm_w8a8_residual", g_lib.gemm_residual) ||
       !get("bq_linear_w8a8", g_lib.linear) || !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_w8a8", g_lib.gate_up_silu_quant) || !get("bq_mlp_w8a8", g_lib.mlp) ||
-      !get("bq_mlp_w8a8_takes", g_lib.mlp_takes) ||
+      !get("bq_mlp_w8a8_takes", g_lib.mlp_takes) || !get("bq_stream_is_captured", g_lib.stream_is_captured) ||
       !get("bq_gate_up_silu_w8a8", g_lib.gate_up_silu) || !get("bq_lm_head_argmax", g_lib.lm_head_argmax) ||
       !get("bq_lm_head_argmax_workspace_bytes", g_lib.lm_head_argmax_workspace))
     return nullptr;

@@ -468,6 +468,9 @@ int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate, const void
  * (destinations and their row pitch then 16-byte aligned).
  */
 
+/* 1 while `stream` is captured into a graph. */
+int bq_stream_is_captured(void* stream);
+
 /*
  * Lets kernels launched on the CURRENT device dereference memory of `peer_device` that this
  * process has mapped (cudaDeviceEnablePeerAccess; already-enabled is success).  A peer buffer

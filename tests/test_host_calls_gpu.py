@@ -137,7 +137,7 @@ def test_what_torch_follows_above_256_rows_stays_a_torch_operation(Q, weights):
 def test_mlp_of_two_launches_holds_a_slot_of_its_own(Q):
     """Between its launches the maximum of h lies in its scratch: not in one that a call of another thread may be handed
     meanwhile.  The common slots are not touched, the one it held is zero again, and threads that share a stream get
-    the bits of a lone call."""
+    the bits of a lone call.  A captured call keeps a common slot, which no call outside a graph holds."""
     import threading
     mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
     wg, wu, wd = mk(8192, 4096, 1), mk(8192, 4096, 2), mk(4096, 8192, 3)
@@ -147,6 +147,12 @@ def test_mlp_of_two_launches_holds_a_slot_of_its_own(Q):
     n0, taken = Q.launch_count(), Q._next_slot[0]
     Q.mlp_forward(hs[0], wg, wu, wd)
     assert Q.last_gemm_launch()["quantizes"] and Q.launch_count() - n0 == 2 and Q._next_slot[0] == taken
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        again = Q.mlp_forward(hs[1], wg, wu, wd)
+    assert Q._next_slot[0] == (taken + 1) % 256
+    graph.replay()
+    assert torch.equal(again, want[1])
     wrong = []
 
     def work(i):
