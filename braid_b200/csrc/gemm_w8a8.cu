@@ -482,22 +482,24 @@ __device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const floa
 // Weight-streaming kernel (swap-AB, cluster split-K)
 // ---------------------------------------------------------------------------
 // Shared memory, after aligning the dynamic base to 1024 bytes:
-//   [stages x 16 KiB weight tiles][b_stages x (mma_n*128) activation tiles] ... [barrier block]
+//   [stages x 16 KiB weight tiles][b_stages x (mma_n*128) activation tiles] ... [barrier block][slices]
 // Two rings with their own barriers and their own producer thread.  The weight ring is as deep
 // as the shared memory allows: its tiles come from HBM, and the bytes in flight per SM are what
 // sets the streaming rate.  The activation ring is shallow (2 to 4 tiles at wide batches): its
 // tiles are L2 hits shared by every row tile, and a wide batch tile is as large as a weight
 // tile, so every activation slot given up is a weight tile more in flight.
 // The tile area is reused after the main loop as the fp32 staging buffer
-// part[m][128] that the cluster reduction reads.
+// part[m][128] that the cluster reduction reads.  Up to 48 rows of a sliced weight (handover_bytes) the reduction
+// reads the slices instead, [split][rows that this CTA sums][128] fp32 behind the barriers: every CTA of the cluster
+// writes its own there from its accumulator, and nothing is staged.
 //
 // QUANT (fewer rows still): the activation arrives unquantized, and every CTA quantizes it for itself: the
 // warps that have nothing to do until the accumulator is complete read the whole activation (a few
 // dozen KB, from L2) for its max |x|, then cast this CTA's K slice into the activation tiles.  The same
 // values in the same arithmetic everywhere, so every CTA finds the same scale and nothing is
 // exchanged; the quantizer's launch and its hand-over through memory are gone.  Two launches -> one, us in a
-// graph and eager: 1 row of 4096 x 4096 9.0 -> 8.2 and 10.6 -> 8.4, 4 rows of 1024 x 4096 8.7 -> 6.6 and 10.6 -> 7.3,
-// 8 rows of 512 x 1024 6.7 -> 4.9 and 10.7 -> 5.4, 16 rows of 2048 x 2048 8.2 -> 7.3 and 10.7 -> 8.7.  Where it stops
+// graph and eager: 1 row of 4096 x 4096 7.5 -> 6.6 and 10.7 -> 6.8, 4 rows of 1024 x 4096 7.3 -> 5.2 and 10.6 -> 6.0,
+// 8 rows of 512 x 1024 6.1 -> 4.2 and 10.6 -> 6.0, 16 rows of 2048 x 2048 7.3 -> 6.2 and 10.5 -> 6.8.  Where it stops
 // paying: quantize_inside_pays.
 constexpr int kQuantWarps = kStreamWarps - 2;           // all but the weight loads' and the MMAs'
 constexpr int kQuantThreads = kQuantWarps * 32;
@@ -1837,15 +1839,15 @@ int split_for_weight(long long n_rows, int k_blocks) {
 
 // Few rows: is the launch whose CTAs quantize the activation for themselves the faster form?  It saves a launch;
 // every CTA reads all of the activation and casts its K slice, and its weights wait for that.  So what counts is
-// the bytes a CTA reads plus those it casts.  us in a graph, one launch and two (before the slices were
-// handed over and whole warps walked the issue loops; both sides are faster since), at the bytes of the activation and the
-// K slices of the weight: 48 KB in 4 (6 rows of 4096 x 4096) 9.8 and 9.8, 64 KB in 4 (8 rows) 10.0 and 9.8; 40 KB in 2
-// (5 rows of 8192 x 4096) 12.6 and 12.7, 48 KB in 2 (6 rows) 13.6 and 12.9; 24 KB in 1 (6 rows of 12288 x 2048) 10.7
-// and 10.9, 32 KB in 1 (8 rows) 11.3 and 10.8, 64 KB in 1 (16 rows) 13.9 and 10.9.  A weight of 64 CTAs or fewer
-// reads less in all (8 rows of 2048 x 4096 8.3 and 9.0).  A call that is not captured pays the host for its second
-// launch as well: 64 KB in 4 10.2 and 11.3, 60 KB in 2 (6 rows of 8192 x 5120) 14.6 and 15.3, 64 KB in 2 (8 rows of
-// 6144 x 4096) 13.2 and 12.5; 40 KB in 1 (5 rows of 12288 x 4096) 15.2 and 16.0, 48 KB in 1 (12 rows of
-// 12288 x 2048) 12.5 and 11.5.
+// the bytes a CTA reads plus those it casts.  us in a graph, one launch and two, at the bytes of the activation and the
+// K slices of the weight: 48 KB in 4 (6 rows of 4096 x 4096) 7.9 and 8.9, 64 KB in 4 (8 rows) 8.3 and 8.9; 40 KB in 2
+// (5 rows of 8192 x 4096) 9.8 and 10.8, 48 KB in 2 (6 rows) 10.5 and 10.9; 24 KB in 1 (6 rows of 12288 x 2048) 8.0
+// and 9.0, 32 KB in 1 (8 rows) 8.5 and 9.0, 48 KB in 1 (12 rows) 9.8 and 9.1, 64 KB in 1 10.9 and 9.3.  The line of a
+// captured call, 60 KB of both, dates from when one launch and two were equal there; they now are at 80 KB.
+// A weight of 64 CTAs or fewer reads less in all (8 rows of 2048 x 4096 6.5 and 7.7).  A call that is not captured pays
+// the host for its second launch as well: 64 KB in 4 8.4 and 10.7, 60 KB in 2 (6 rows of 8192 x 5120) 11.9 and 13.5,
+// 64 KB in 2 (8 rows of 6144 x 4096) 10.3 and 11.0; 40 KB in 1 (5 rows of 12288 x 4096) 12.7 and 13.7, 48 KB in 1 13.6
+// and 13.8, 64 KB in 1 (16 rows of 12288 x 2048) 11.0 and 10.7.
 constexpr int64_t kInsideBytes = 65536, kInsideWork = 61440, kInsideWorkEager = 92160;
 
 bool quantize_inside_pays(int64_t M, int64_t K, int element_size, int n_seg, const int64_t* N, cudaStream_t stream) {
@@ -2406,10 +2408,12 @@ int run_wide(GemmParams p, const void* xq, int64_t K, const void* const* wq, con
 // are visited last, where that evens out the last round.  A launch takes as long as its busiest CTA pair
 // (tiles are dealt out in turn), a tile its columns plus a part that does not shrink with them: the
 // activation rows' loads and MMA passes, the epilogue.  Measured, us with tiles of 256 / 192 / 128 columns:
-// 4096 x 12288 at 300 rows 45.0 / 37.9 / 31.6, at 600 45.1 / 38.2 / 56.5, at 1024 45.6 / 67.9 / 56.8, at 1500
-// 81.7 / 68.9 / 81.9, at 3000 126.5 / 138.2 / 182.8: one round of n columns costs n + 128, within the launch's
-// own 3 us.  64 columns never won by more than 2 %.  Split: q, k and v of 8192 + 1024 + 1024 columns at 1500 rows
-// 58.0 -> 54.8, 2560 x 7680 at 4096 rows 76.8 -> 69.7.
+// 4096 x 12288 at 300 rows 34.3 / 28.5 / 21.9, at 600 35.6 / 30.5 / 36.9, at 1100 64.0 / 53.9 / 56.3, at 1500
+// 66.4 / 60.2 / 62.8, at 3000 115.9 / 121.5 / 127.4: one round of n columns costs n + 128 within 6 % (128 columns alone,
+// with their deeper ring, n + 114).  Of 13 weights at 16 batches of 257 to 4000 rows, the choices timed in turn, the rule's is
+// more than 3 % behind the best at 7 of 208 (2560 x 7680 at 2600 rows 43.9 where 128 columns take 41.5, 15360 x 5120
+// at 1100 rows 78.8 with a split and 76.4 without; the others below 0.7 us).  64 columns never won by more than 2 %.  Split: q, k and v of 8192 + 1024 + 1024 columns at 1500 rows
+// 58.0 -> 54.8, 2560 x 7680 at 4096 rows 76.8 -> 69.7 (both before the issue loops were walked by whole warps).
 struct TilePlan {
   int cols;            // columns of a tile
   int split;           // weight whose end becomes a segment of 128-column tiles, -1: none

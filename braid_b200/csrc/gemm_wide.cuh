@@ -201,8 +201,7 @@ __device__ __forceinline__ void pair_park(const PairTile<T>& t, uint32_t taddr, 
 }
 
 // Which (row, group of 8 columns) a thread takes: the groups of all rows in turn.  (Whole rows per warp left 8 of 32
-// lanes idle at 192 columns, and took six rounds instead of four for 64 rows: four graphed layers of 128 rows 308.6 us, now
-// 305.9.)
+// lanes idle at 192 columns, and took six rounds instead of four for 64 rows: four graphed layers of 128 rows take 0.9 % less.)
 template <typename T, typename F>
 __device__ __forceinline__ void for_each_group(const PairTile<T>& t, F f) {
   const int per_row = t.un / 8, rows = kWideThreads / per_row, left = kWideThreads - rows * per_row;   // of one round

@@ -1342,8 +1342,8 @@ def mlp_forward(x: torch.Tensor, gate_proj: FP8Weight, up_proj: FP8Weight,
     """The quantized branch of `MLP.forward` (braid/model/mlp.py:44-49) in 3 launches at decode
     sizes: quantize(x) -> gate and up as one GEMM (tiles put together from both weights) with
     SiLU*mul and the quantization of h in its epilogue -> down GEMM (with `residual` added in its epilogue).
-    Up to 6 rows of a large MLP (native calls) the first of the two GEMMs writes h and the second one's CTAs cast it, so
-    that nothing is exchanged inside a launch.
+    Up to 6 rows of some widths (native calls; `bq_mlp_w8a8_takes`) the first of the two GEMMs writes h and the second
+    one's CTAs cast it, so that nothing is exchanged inside a launch.
     Larger M: 4 launches (quantize -> gate and up as one CTA-pair GEMM that writes h = silu(gate)*up
     and its scale -> cast of h -> down).  Unpaired shapes or `set_paired_mlp(False)`: 4 launches
     (quantize -> grouped GEMM writing gate|up into one `[M, 2I]` buffer -> SiLU*mul inside the
