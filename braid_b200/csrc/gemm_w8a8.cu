@@ -1890,6 +1890,10 @@ bool fetched_inside_pays(const GemmParams& p, int split, cudaStream_t stream) {
 // rows would take the memory of too many weight tiles, and are staged and fetched between two barriers.
 // us, fetched -> handed over: linear of 8 rows of 4096 x 4096 8.8 -> 7.9; four graphed layers of hidden 4096, 16 rows
 // 249.2 -> 246.6, 27 rows 263 -> 257.5, 48 rows 274 -> 273, 1 row the same; hidden 1024, 16 rows 147 -> 145.8.
+// Two CTAs per SM have room for three stages beside it from 45 rows on, which the long slices of halves pay for: 48 rows of
+// 9728 x 5760 14.4 fetched, 14.8 with three stages (13.9 fetched with the present loops), four layers of hidden 3072 250.4 and
+// 245.0 so; slices of quarters gain all the same (48 rows of 5120 x 2560 6.7 and 6.3, 5120 x 7680 11.4 and 11.0).
+constexpr int kHandoverStages = 4;
 int handover_bytes(int64_t M, int split) {
   return split > 1 && M <= 48 ? (int)((M + split - 1) / split) * split * kRowTile * 4 : 0;
 }
@@ -1952,8 +1956,12 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
     const int bytes = handover_bytes(p.M, p.seg[i].split);
     if (bytes > handover) handover = bytes;
   }
+  const bool quant = p.quant.x != nullptr;
+  int whole = stream_budget(grid, sms, &per_sm);
+  const int beside = (whole - handover) / stage_bytes;      // stages that the handed-over slices leave
+  if (!quant && min_split == 2 && beside < kHandoverStages && beside < kb_max) handover = 0;
   p.handover = handover > 0 ? 1 : 0;
-  int whole = stream_budget(grid, sms, &per_sm), budget = whole - handover;
+  int budget = whole - handover;
   // Leave room for the NEXT kernel's CTAs: with programmatic dependent launch they
   // become resident while this kernel still runs and pre-load their weights.
   if (g_opt_smem_cap > 0 && whole > g_opt_smem_cap) whole = (int)g_opt_smem_cap;
@@ -1964,7 +1972,6 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   if (stages < 2) stages = kb_max < 2 ? kb_max : 2;
   if (g_opt_stages > 0 && g_opt_stages < stages) stages = (int)g_opt_stages;
   int b_stages = stages;
-  const bool quant = p.quant.x != nullptr;
   // Wide batch tiles: a shallow activation ring (its tiles are L2 hits), the rest goes to
   // weight tiles in flight.  Two slots cover the L2 latency at the rate one CTA of a two-per-SM
   // launch consumes tiles; a CTA that has the SM to itself consumes twice as fast.

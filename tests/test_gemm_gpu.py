@@ -832,6 +832,26 @@ def test_slices_handed_over_add_up_to_the_fetched_sum(Q, M):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M", [44, 45, 48])
+@pytest.mark.parametrize("N,K", [(9728, 5760), (10240, 2048), (5120, 2560)])
+def test_slices_of_halves_are_handed_over_only_beside_four_stages(Q, M, N, K):
+    """Two CTAs per SM: the area for the slices is not bought with the weight ring, where slices are long; the bits of
+    the fetched sum."""
+    x = randn_cpu((60, K), seed=5).cuda()
+    xq, sx = Q.quantize_act(x)
+    w = Q.quantize_weight(randn_cpu((N, K), seed=N, scale=0.02).cuda())
+    Q.set_option("decode_wide", 0)
+    try:
+        far = Q.fp8_matmul(xq, sx, w)
+        near = Q.fp8_matmul(xq[:M].contiguous(), sx, w)
+        launch = Q.last_gemm_launch()
+        assert not launch["wide"] and (launch["split"] != 2 or launch["stages"] >= 4)
+        assert torch.equal(near, far[:M])
+    finally:
+        Q.set_option("decode_wide", -1)
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("M,I,dt", [(1, 12288, torch.bfloat16), (6, 12288, torch.bfloat16), (7, 12288, torch.bfloat16),
                                     (5, 12288, torch.float16), (3, 12288, torch.float32), (4, 12288, torch.float32),
                                     (6, 8256, torch.bfloat16), (2, 8128, torch.bfloat16)])
