@@ -1898,6 +1898,9 @@ int handover_bytes(int64_t M, int split) {
   return split > 1 && M <= 48 ? (int)((M + split - 1) / split) * split * kRowTile * 4 : 0;
 }
 
+// Shared memory that three CTAs of an SM cannot have (228 KB, of which 1 KB per CTA is reserved).
+constexpr int kThirdOfSmem = (233472 / 3 - 1024) / 128 * 128 + 128;
+
 // Shared memory of a CTA for rings: what lets the whole grid be resident at once (up to 2 CTAs per SM), so that one
 // CTA's epilogue overlaps its neighbour's loads.
 int stream_budget(long long grid, int sms, int* per_sm_out = nullptr) {
@@ -1997,7 +2000,10 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   p.b_stages = b_stages;
   int tile_bytes = stages * kATileBytes + b_stages * b_tile;
   if (tile_bytes < staging) tile_bytes = staging;
-  const int smem = tile_bytes + kBarrierBytes + handover + 1024;
+  int smem = tile_bytes + kBarrierBytes + handover + 1024;
+  // More than 128 rows take half of an SM's tensor memory: a third CTA there would wait for it until one of the two
+  // is done, and where they wait for the whole grid's maximum that is never.  So no third one gets in.
+  if (p.mma_n > 128 && smem < kThirdOfSmem) smem = kThirdOfSmem;
   if (smem > kMaxSmem) return kErrUnsupported;
   const int epi = epilogue_of(p, false);
   if (quant && epi != kPlain && epi != kResidual) return kErrUnsupported;

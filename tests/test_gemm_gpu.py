@@ -962,6 +962,39 @@ def test_mlp_of_few_rows_leaves_its_scratch_clean_when_the_second_launch_fails(Q
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("M", [129, 144, 200, 256])
+def test_mlps_of_more_than_128_rows_back_to_back(Q, M):
+    """More than 128 rows take half of an SM's tensor memory, and gate/up waits for the whole grid: launches of small
+    weights, of which three CTAs would fit an SM, take the shared memory that keeps the third out.  MLPs without a launch
+    between them, captured and replayed, have the bits of the four-launch form, and no wait runs out."""
+    H, I = 1024, 3072
+    ws = [[Q.quantize_weight(randn_cpu((n, k), seed=s + j, scale=0.02).cuda()) for j, (n, k) in enumerate(((I, H), (I, H), (H, I)))]
+          for s in (1, 11, 21)]
+    x = randn_cpu((M, H), seed=M).cuda()
+    h = Q.QuantizedActivation(*Q.quantize_act(x), x.shape, x.dtype)
+    Q.set_paired_mlp(False)
+    want = [Q.mlp_forward(h, *w) for w in ws]
+    Q.set_paired_mlp(True)
+    Q.set_option("decode_wide", 0)
+    try:
+        got = [Q.mlp_forward(h, *w) for w in ws]
+        launch = Q.last_gemm_launch()
+        assert launch["kernel"] == "stream" and not launch["wide"] and 3 * (launch["smem"] + 1024) > 233472
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            again = [Q.mlp_forward(h, *w) for w in ws for _ in range(2)]
+        graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert Q.device_status() == 0
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+        for a, b in zip(again, [b for b in want for _ in range(2)]):
+            assert torch.equal(a, b)
+    finally:
+        Q.set_option("decode_wide", -1)
+
+
 def test_paired_mlp_equals_the_four_launch_mlp_and_replays(Q):
     H, I = 4096, 12288
     mk = lambda n, k, s: Q.quantize_weight(randn_cpu((n, k), seed=s, scale=0.02).cuda())  # noqa: E731
