@@ -612,7 +612,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   volatile float* const s_scale = reinterpret_cast<volatile float*>(base_ptr + smem_tile_bytes + kBarrierBytes - 8);
 
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 0); }
-  pdl_launch_dependents();   // the next kernel may start its own set-up right away
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // A cluster of p.cluster CTAs works on p.cluster / split row tiles of one weight
   // at a time: CTAs [g*split, (g+1)*split) of the cluster hold the K slices of
@@ -661,6 +660,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), tmem_cols);
     tmem_relinquish();
   }
+  // The next kernel may start its own set-up -- only now: a CTA of it that shares this SM takes tensor memory too and
+  // keeps it until this kernel is done.
+  if (warp == 1) pdl_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
