@@ -93,6 +93,51 @@ __device__ __forceinline__ float grid_amax(float m, QuantWs* ws, const Cta& cta 
   return s_amax;
 }
 
+// The exchange of a grid that is ONE cluster: every CTA stores its max into every other's shared memory, where the
+// bytes are counted, and no word of global memory is involved.  A grid-wide exchange is three trips to L2 one after the
+// other (max, arrival, poll), each 0.7 us and more while the next GEMM's weights stream.
+constexpr int kMaxCluster = 16;      // beyond 8 a kernel has to allow it
+struct ClusterAmax {
+  uint64_t full;
+  uint32_t slot[kMaxCluster];        // one word per CTA of the cluster
+};
+
+// All threads of the CTA, before anything else.
+__device__ __forceinline__ void cluster_amax_begin(ClusterAmax& s) {
+  if (threadIdx.x == 0) {
+    bq::mbar_init(bq::smem_u32(&s.full), 1);
+    bq::fence_mbar_init();
+    bq::mbar_expect_tx(bq::smem_u32(&s.full), 4u * gridDim.x);
+  }
+  __syncwarp();
+  bq::cluster_arrive();              // says that this CTA runs and its barrier is set up
+}
+
+// As grid_amax; nothing is owed to the scratch afterwards.  A CTA has every other's word when it leaves, so none is
+// stored to that has ended.
+template <typename Cta>
+__device__ __forceinline__ float cluster_amax(float m, ClusterAmax& s, QuantWs* ws, const Cta& cta) {
+  __shared__ uint32_t s_warp_of[2][32];
+  uint32_t* const s_warp = s_warp_of[cta.slot()];
+  const int lane = threadIdx.x & 31, warp = cta.warp();
+  // |x| >= 0 or NaN with the sign cleared: bit patterns order like the values, NaN on top
+  const uint32_t mine = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+  if (lane == 0) s_warp[warp] = mine;
+  cta.sync();
+  uint32_t all = __reduce_max_sync(0xffffffffu, lane < cta.warps() ? s_warp[lane] : 0u);
+  if (!cta.live) return __uint_as_float(all);
+  if (warp == 0) {
+    bq::cluster_wait();              // every CTA's barrier is set up
+    if (lane < gridDim.x)
+      bq::st_async_cluster(bq::map_to_cta(bq::smem_u32(&s.slot[blockIdx.x]), lane), all,
+                           bq::map_to_cta(bq::smem_u32(&s.full), lane));
+  }
+  if (!bq::mbar_wait_cluster(bq::smem_u32(&s.full), 0) && threadIdx.x == 0)
+    atomicExch(&ws->status, (unsigned int)bq::kErrDeviceWait);
+  all = lane < gridDim.x ? *static_cast<volatile uint32_t*>(&s.slot[lane]) : 0u;
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, all));
+}
+
 // CTA-wide max alone, to every thread.  Blocks of whole warps, 1024 threads at most.
 __device__ __forceinline__ float cta_amax(float m) {
   __shared__ float s_warp[32];
@@ -169,6 +214,64 @@ inline int resident_per_sm(Kernel kernel, int threads, size_t dynamic_smem) {
   }
   known[next++ % 32] = Known{key, dev, threads, dynamic_smem, per_sm};
   return per_sm;
+}
+
+// Host side: can a cluster of `n` CTAs of this kernel be scheduled at all?  Asked once per thread, kernel and size.
+extern bool g_cluster_exchange;       // quant_act.cu: option "quant_cluster"
+
+template <typename Kernel>
+inline bool cluster_fits(Kernel kernel, int threads, int n) {
+  struct Known { const void* kernel; int dev, threads, n; bool fits; };
+  static thread_local Known known[32];
+  static thread_local unsigned int next = 0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+  const void* const key = reinterpret_cast<const void*>(kernel);
+  for (const Known& k : known)
+    if (k.kernel == key && k.dev == dev && k.threads == threads && k.n == n) return k.fits;
+  bool fits = n <= 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  if (fits) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(n), 1, 1);
+    cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(n);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    fits = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+  }
+  if (!fits) (void)cudaGetLastError();
+  known[next++ % 32] = Known{key, dev, threads, n, fits};
+  return fits;
+}
+
+// Host side: launches a grid that is one cluster of `ctas` CTAs; kErrTooLarge where such a cluster cannot be scheduled.
+template <typename Kernel, typename Params>
+inline int launch_cluster(Kernel kernel, int ctas, int threads, cudaStream_t stream, Params p) {
+  if (!cluster_fits(kernel, threads, ctas)) return bq::kErrTooLarge;
+#ifdef BQ_PHASES
+  p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
+#endif
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
+  return bq::kOk;
 }
 
 // Host side: launches a grid-stride kernel with at most as many CTAs as the device holds at

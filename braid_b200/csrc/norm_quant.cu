@@ -17,9 +17,9 @@
 // multiplies by gamma in fp32, multiplies by silu(z) evaluated in fp32 (x / (1 + expf(-x))) and
 // rounds once more.  tests/test_norm_quant_gpu.py pins all of this against torch on the device.
 //
-// After the norm the values stay in registers; amax, grid-wide exchange and cast are the
-// activation quantizer's (quant_act.cu).  A CTA holds one token row, or four or eight (rmsnorm_rows_quant_kernel), and all
-// of them are co-resident for the exchange; larger inputs are refused, and the caller takes the norm with its rows
+// After the norm the values stay in registers; amax, exchange and cast are the activation quantizer's (quant_act.cu).
+// The exchange of up to 64 rows stays inside one cluster; beyond it is grid-wide: a CTA holds one token row, or four or
+// eight (rmsnorm_rows_quant_kernel), and all of them are co-resident for it; larger inputs are refused, and the caller takes the norm with its rows
 // looped (bq_rmsnorm_scale, bq_gated_rmsnorm_scale) and the cast pass.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -55,6 +55,7 @@ struct NormParams {
 
 constexpr int kWideRows = 256;      // batches whose rows get four times the threads
 constexpr int kRehearseRows = 128;   // see rmsnorm_quant_kernel; one CTA per row
+constexpr int with_rehearsal(int threads) { return threads < 1024 ? threads + 32 : threads; }    // CTAs of 1024 have no room for it
 
 template <typename T> struct Vec4 { T v[kVec]; };
 
@@ -100,26 +101,32 @@ __device__ __forceinline__ float warp_tree_sum(float s) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// plain RMSNorm -> quantize.  One CTA per row, of G groups of 128 threads; VPT = vectors that a thread would hold
-// if it were 128 threads in all.
+// plain RMSNorm -> quantize.  R rows per CTA (more than one only where the grid is one cluster, see launch_rmsnorm_cluster),
+// each of G groups of 128 threads; VPT = vectors that a thread would hold if a row were 128 threads in all.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int VPT, int G>
-__global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(const NormParams p) {
+template <typename T, int VPT, int G, int R, bool CLUSTER>
+__global__ void __launch_bounds__(with_rehearsal(R * G * kNormThreads)) rmsnorm_quant_kernel(const NormParams p) {
+  static_assert(R == 1 || CLUSTER, "several rows per CTA: one cluster");
   // G groups of 128 threads share a row; a thread holds VG vectors of it
   static_assert(VPT % G == 0, "whole vectors per thread");
   constexpr int VG = VPT / G;
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
-  __shared__ float s_red_of[2][4];
-  __shared__ __align__(16) Vec4<T> s_x[G > 1 ? VPT * kNormThreads + 32 : 1];   // the last 32: the rehearsing warp's
-  const RehearsingCta<G * kNormThreads> cta{threadIdx.x < G * kNormThreads};
+  __shared__ float s_red_of[1 + R][4];
+  __shared__ __align__(16) Vec4<T> s_x_of[G > 1 ? R * VPT * kNormThreads + 32 : 1];   // the last 32: the rehearsing warp's
+  __shared__ ClusterAmax s_cluster;
+  if constexpr (CLUSTER) cluster_amax_begin(s_cluster);
+  const RehearsingCta<R * G * kNormThreads> cta{threadIdx.x < R * G * kNormThreads};
   const bool live = cta.live;
-  float* const s_red = s_red_of[cta.slot()];
-  const int lane = threadIdx.x & 31, warp = cta.warp(), t = warp * 32 + lane;
+  const int lane = threadIdx.x & 31, of_row = (cta.warp() * 32 + lane) / (G * kNormThreads);   // row of this CTA
+  const int t = cta.warp() * 32 + lane - of_row * (G * kNormThreads), warp = t >> 5;            // thread of that row
   const int group = t / kNormThreads;
+  float* const s_red = s_red_of[live ? of_row : R];
+  Vec4<T>* const s_x = s_x_of + (G > 1 && live ? of_row * (VPT * kNormThreads) : 0);
   // vector i of this thread
   auto vec = [&](int i) { return (t - group * kNormThreads) + (group * VG + i) * kNormThreads; };
-  const int row = blockIdx.x;
+  const int row = blockIdx.x * R + of_row;
+  const bool row_ok = live && (R == 1 || row < p.rows);
   const int n_vec = p.cols / kVec;
   const T* xr = reinterpret_cast<const T*>(p.x) + static_cast<long long>(row) * p.ld_x;
   // gamma is a weight, not the previous kernel's output: fetch it before the dependency wait
@@ -156,7 +163,7 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
 #pragma unroll
   for (int i = 0; i < VG; ++i) {
     const int v = vec(i);
-    if (live && v < n_vec) x[i] = load4(xr + v * kVec);
+    if (row_ok && v < n_vec) x[i] = load4(xr + v * kVec);
     else x[i] = Vec4<T>{};
   }
   float s = 0.0f;
@@ -175,7 +182,7 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
   } else {
     // the sum's order is that of 128 threads: the first group walks the others' vectors (the rehearsing warp,
     // which passes no barrier with them, words of its own)
-    const int put = live ? vec(0) : VPT * kNormThreads + lane, get = live ? t : put, step = live ? kNormThreads : 0;
+    const int put = live ? vec(0) : R * VPT * kNormThreads + lane, get = live ? t : put, step = live ? kNormThreads : 0;
 #pragma unroll
     for (int i = 0; i < VG; ++i) s_x[put + i * step] = x[i];
     cta.sync();
@@ -209,7 +216,7 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
 #pragma unroll
   for (int i = 0; i < VG; ++i) {
     const int v = vec(i);
-    if (v < n_vec) {
+    if (v < n_vec && (R == 1 || row_ok || !live)) {
 #pragma unroll
       for (int j = 0; j < kVec; ++j) {
         const float y = __fmul_rn(g[i][j], __fmul_rn(rstd, widen(x[i].v[j])));
@@ -218,7 +225,7 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
       }
     }
   }
-  if (live && p.h_out != nullptr) {
+  if (row_ok && p.h_out != nullptr) {
     T* hr = reinterpret_cast<T*>(p.h_out) + static_cast<long long>(row) * p.ld_h;
 #pragma unroll
     for (int i = 0; i < VG; ++i) {
@@ -227,17 +234,20 @@ __global__ void __launch_bounds__(G * kNormThreads + 32) rmsnorm_quant_kernel(co
     }
   }
   if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
-  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), cta));
+  float amax;
+  if constexpr (CLUSTER) amax = cluster_amax(m, s_cluster, static_cast<QuantWs*>(p.ws), cta);
+  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws), cta);
+  const float sc = scale_from_amax(amax);
   if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
   const ScaleDiv dv(sc);
-  if (live && blockIdx.x == 0 && t == 0) p.scale[0] = sc;
+  if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
   uint8_t* qr = p.q + static_cast<long long>(row) * p.cols;
 #pragma unroll
   for (int i = 0; i < VG; ++i) {
     const int v = vec(i);
-    if (v < n_vec) emit4(x[i], dv, qr + v * kVec, live);
+    if (v < n_vec) emit4(x[i], dv, qr + v * kVec, row_ok);
   }
-  grid_depart(static_cast<QuantWs*>(p.ws));
+  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws));
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
@@ -447,6 +457,7 @@ struct GatedParams {
   float* scale;
   void* ws;
   int rows, heads;
+  int cta_rows;        // rows per CTA (a grid that is one cluster; else 1)
   long long ld_y, ld_z;
   float eps;
   unsigned long long* phase_ring;   // development builds (BQ_PHASES) only, else nullptr
@@ -458,14 +469,23 @@ constexpr int kGatedWarps = 8;
 constexpr int kMaxHeadsPerWarp = 8;    // up to 64 heads
 constexpr int kWideGatedRows = 256;    // batches whose CTAs have 16 warps
 
-template <typename T, bool Y_F32, int HPW, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32 + 32) gated_rmsnorm_quant_kernel(const GatedParams p) {
+template <typename T, bool Y_F32, int HPW, int WARPS, bool CLUSTER>
+__global__ void __launch_bounds__(with_rehearsal(WARPS * 32)) gated_rmsnorm_quant_kernel(const GatedParams p) {
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 1); }
   bq::pdl_launch_dependents();
+  __shared__ ClusterAmax s_cluster;
+  if constexpr (CLUSTER) cluster_amax_begin(s_cluster);
   const RehearsingCta<WARPS * 32> cta{threadIdx.x < WARPS * 32};   // see rmsnorm_quant_kernel
   const bool live = cta.live;
   const int lane = threadIdx.x & 31, warp = cta.warp();
-  const int row = blockIdx.x;
+  // head i of this warp: the CTA's rows lie one after the other
+  const int first_row = CLUSTER ? blockIdx.x * p.cta_rows : blockIdx.x;
+  const int cta_heads = CLUSTER ? (p.rows - first_row < p.cta_rows ? p.rows - first_row : p.cta_rows) * p.heads : p.heads;
+  auto place = [&](int at, int& row, int& head) {
+    row = CLUSTER ? at / p.heads : 0;
+    head = at - row * p.heads;
+    row += first_row;
+  };
   const float4 gm = __ldg(reinterpret_cast<const float4*>(p.gamma) + lane);
   const float gmv[kVec] = {gm.x, gm.y, gm.z, gm.w};
   Vec4<T> core[HPW];
@@ -476,10 +496,11 @@ __global__ void __launch_bounds__(WARPS * 32 + 32) gated_rmsnorm_quant_kernel(co
   }
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
-    const int head = warp + i * WARPS;
     core[i] = Vec4<T>{};
     gate[i] = Vec4<T>{};
-    if (live && head < p.heads) {
+    if (live && warp + i * WARPS < cta_heads) {
+      int row, head;
+      place(warp + i * WARPS, row, head);
       const long long off = static_cast<long long>(head) * kHeadDim + lane * kVec;
       if constexpr (Y_F32) {
         // the reference rounds the scan output to the activation type first (gdn.py:383)
@@ -496,8 +517,7 @@ __global__ void __launch_bounds__(WARPS * 32 + 32) gated_rmsnorm_quant_kernel(co
   float m = 0.0f;
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
-    const int head = warp + i * WARPS;   // warp-uniform
-    if (head < p.heads) {
+    if (warp + i * WARPS < cta_heads) {   // warp-uniform
       float s = 0.0f;
 #pragma unroll
       for (int j = 0; j < kVec; ++j) {
@@ -521,17 +541,20 @@ __global__ void __launch_bounds__(WARPS * 32 + 32) gated_rmsnorm_quant_kernel(co
     }
   }
   if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
-  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), cta));
+  float amax;
+  if constexpr (CLUSTER) amax = cluster_amax(m, s_cluster, static_cast<QuantWs*>(p.ws), cta);
+  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws), cta);
+  const float sc = scale_from_amax(amax);
   if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
   const ScaleDiv dv(sc);
-  if (live && blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
-  uint8_t* qr = p.q + static_cast<long long>(row) * p.heads * kHeadDim;
+  if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
+  uint8_t* qr = p.q + static_cast<long long>(first_row) * p.heads * kHeadDim;      // codes are contiguous
 #pragma unroll
   for (int i = 0; i < HPW; ++i) {
     const int head = warp + i * WARPS;
-    if (head < p.heads) emit4(core[i], dv, qr + head * kHeadDim + lane * kVec, live);
+    if (head < cta_heads) emit4(core[i], dv, qr + head * kHeadDim + lane * kVec, live);
   }
-  grid_depart(static_cast<QuantWs*>(p.ws));
+  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws));
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
@@ -563,6 +586,63 @@ int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t str
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
   return bq::kOk;
+}
+
+// Decode batches of up to 64 rows: a grid that is one cluster of up to 16 CTAs, and the exchange goes through its shared
+// memory (cluster_amax).  Four graphed layers of hidden 4096, grid-wide exchange -> this, us: norms of 8 rows 240.2 ->
+// 225.4, 16 rows 248.3 -> 232.0, 27 rows 259.0 -> 239.1, 48 rows 271.8 -> 257; with the gated norm 8 rows 221.4, 16 rows 225.7,
+// 27 rows 237.1.  Eight CTAs at most (what a cluster may be without asking) leave 27 rows at 259.
+//
+// A CTA takes one row while there are 16 at most: with R rows it has R times the bytes to wait for.  Two groups of 128
+// threads to a row from there on: one loses (four rows per CTA, 40 rows 264.4 and 258.0), four give the same up to 4096
+// columns and take more of an SM; longer rows need them (hidden 5120, 17 rows, grid-wide 386.4, two groups 390.9, four 366.3).
+// Seven rows per CTA lose: 96 rows 296 and 310.  Where values of 4 bytes or long rows leave no room for R rows,
+// kErrTooLarge: the grid-wide exchange takes them.
+constexpr int kClusterRows = 64;
+template <typename T, int VPT>
+int launch_rmsnorm_cluster(const NormParams& p, cudaStream_t stream) {
+  constexpr int kOne = VPT == 2 ? 2 : 4;              // groups of one row
+  constexpr int kRow = VPT * (int)sizeof(T);          // registers of a row, were it one group's
+  const int ctas = kMaxCluster;
+  if (p.rows <= ctas)
+    return launch_cluster(rmsnorm_quant_kernel<T, VPT, kOne, 1, true>, p.rows, with_rehearsal(kOne * kNormThreads), stream, p);
+  if constexpr (VPT == 16 && kRow <= 32) {
+    if (p.rows <= 2 * ctas)
+      return launch_cluster(rmsnorm_quant_kernel<T, VPT, 4, 2, true>, (p.rows + 1) / 2, with_rehearsal(8 * kNormThreads), stream, p);
+  } else if constexpr (kRow <= 32) {
+    if (p.rows <= 2 * ctas)
+      return launch_cluster(rmsnorm_quant_kernel<T, VPT, 2, 2, true>, (p.rows + 1) / 2, with_rehearsal(4 * kNormThreads), stream, p);
+  }
+  if constexpr (kRow <= 16) {
+    if (p.rows <= 3 * ctas)
+      return launch_cluster(rmsnorm_quant_kernel<T, VPT, 2, 3, true>, (p.rows + 2) / 3, with_rehearsal(6 * kNormThreads), stream, p);
+    if (p.rows <= 4 * ctas)
+      return launch_cluster(rmsnorm_quant_kernel<T, VPT, 2, 4, true>, (p.rows + 3) / 4, with_rehearsal(8 * kNormThreads), stream, p);
+  }
+  return bq::kErrTooLarge;
+}
+
+// The gated norm: 16 warps for a row; two rows take 32, so that no warp has more heads than it would have of one (27
+// rows 239.1 -> 237.1; with 16 warps 242).  Three rows lose (40 rows 264 and 267).
+template <typename T, bool Y_F32>
+int launch_gated_cluster(GatedParams p, cudaStream_t stream) {
+  constexpr int kWarps = 2 * kGatedWarps;
+  p.cta_rows = p.rows <= kMaxCluster ? 1 : 2;
+  const int ctas = (p.rows + p.cta_rows - 1) / p.cta_rows, heads = p.cta_rows * p.heads;
+  if (ctas > kMaxCluster) return bq::kErrTooLarge;
+  if (p.cta_rows == 1) {
+    if (heads <= kWarps) return launch_cluster(gated_rmsnorm_quant_kernel<T, Y_F32, 1, kWarps, true>, ctas, with_rehearsal(kWarps * 32), stream, p);
+    if (heads <= 2 * kWarps) return launch_cluster(gated_rmsnorm_quant_kernel<T, Y_F32, 2, kWarps, true>, ctas, with_rehearsal(kWarps * 32), stream, p);
+    if (heads <= 4 * kWarps) return launch_cluster(gated_rmsnorm_quant_kernel<T, Y_F32, 4, kWarps, true>, ctas, with_rehearsal(kWarps * 32), stream, p);
+  } else {
+    if (heads <= 2 * kWarps)
+      return launch_cluster(gated_rmsnorm_quant_kernel<T, Y_F32, 1, 2 * kWarps, true>, ctas, with_rehearsal(2 * kWarps * 32), stream, p);
+    if (heads <= 4 * kWarps)
+      return launch_cluster(gated_rmsnorm_quant_kernel<T, Y_F32, 2, 2 * kWarps, true>, ctas, with_rehearsal(2 * kWarps * 32), stream, p);
+    if (heads <= 8 * kWarps)
+      return launch_cluster(gated_rmsnorm_quant_kernel<T, Y_F32, 4, 2 * kWarps, true>, ctas, with_rehearsal(2 * kWarps * 32), stream, p);
+  }
+  return bq::kErrTooLarge;
 }
 
 // The fewest rows per CTA whose grid is resident at once; kErrTooLarge if none is.
@@ -609,11 +689,19 @@ int launch_rmsnorm(const NormParams& p, cudaStream_t stream) {
   const int per_thread = (p.cols / kVec + kNormThreads - 1) / kNormThreads;
   // Decode batches: four times the threads, a quarter of the chain each (see the kernel).  Larger ones need
   // the CTAs resident at once.
+  if (p.rows > 1 && p.rows <= kClusterRows && g_cluster_exchange) {
+    int rc = bq::kErrTooLarge;
+    if (per_thread <= 2) rc = launch_rmsnorm_cluster<T, 2>(p, stream);
+    else if (per_thread <= 4) rc = launch_rmsnorm_cluster<T, 4>(p, stream);
+    else if (per_thread <= 8) rc = launch_rmsnorm_cluster<T, 8>(p, stream);
+    else if (per_thread <= 16) rc = launch_rmsnorm_cluster<T, 16>(p, stream);
+    if (rc != bq::kErrTooLarge) return rc;
+  }
   if (p.rows <= kWideRows) {
-    if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2, 2>, p.rows, 2 * kNormThreads, p, stream);
-    if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4, 4>, p.rows, 4 * kNormThreads, p, stream);
-    if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 4>, p.rows, 4 * kNormThreads, p, stream);
-    if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 4>, p.rows, 4 * kNormThreads, p, stream);
+    if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2, 2, 1, false>, p.rows, 2 * kNormThreads, p, stream);
+    if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4, 4, 1, false>, p.rows, 4 * kNormThreads, p, stream);
+    if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 4, 1, false>, p.rows, 4 * kNormThreads, p, stream);
+    if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 4, 1, false>, p.rows, 4 * kNormThreads, p, stream);
   }
   int rc = bq::kErrTooLarge;
   if (p.rows <= kGroupedRows) {}
@@ -622,10 +710,10 @@ int launch_rmsnorm(const NormParams& p, cudaStream_t stream) {
   else if (per_thread <= 8) rc = launch_row_groups<T, 8>(p, stream);
   else if (per_thread <= 16) rc = launch_row_groups<T, 16>(p, stream);
   if (rc != bq::kErrTooLarge) return rc;
-  if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2, 1>, p.rows, kNormThreads, p, stream);
-  if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4, 1>, p.rows, kNormThreads, p, stream);
-  if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 1>, p.rows, kNormThreads, p, stream);
-  if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 1>, p.rows, kNormThreads, p, stream);
+  if (per_thread <= 2) return launch_rows(rmsnorm_quant_kernel<T, 2, 1, 1, false>, p.rows, kNormThreads, p, stream);
+  if (per_thread <= 4) return launch_rows(rmsnorm_quant_kernel<T, 4, 1, 1, false>, p.rows, kNormThreads, p, stream);
+  if (per_thread <= 8) return launch_rows(rmsnorm_quant_kernel<T, 8, 1, 1, false>, p.rows, kNormThreads, p, stream);
+  if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 1, 1, false>, p.rows, kNormThreads, p, stream);
   return bq::kErrUnsupported;
 }
 
@@ -634,19 +722,23 @@ int launch_gated(const GatedParams& p, cudaStream_t stream) {
   // Decode batches: two heads per warp, 16 warps, so that the chain of a head -- sum, square root,
   // exponentials, divisions -- is walked at most twice one after the other.  Larger batches need the
   // CTAs resident at once.
+  if (p.rows > 1 && p.rows <= 2 * kMaxCluster && g_cluster_exchange) {
+    const int rc = launch_gated_cluster<T, Y_F32>(p, stream);
+    if (rc != bq::kErrTooLarge) return rc;
+  }
   if (p.rows <= kWideGatedRows && p.heads > kGatedWarps) {
     constexpr int kWarps = 2 * kGatedWarps;
-    if (p.heads <= kWarps) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 1, kWarps>, p.rows, kWarps * 32, p, stream);
+    if (p.heads <= kWarps) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 1, kWarps, false>, p.rows, kWarps * 32, p, stream);
     if (p.heads <= 2 * kWarps)
-      return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 2, kWarps>, p.rows, kWarps * 32, p, stream);
+      return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 2, kWarps, false>, p.rows, kWarps * 32, p, stream);
   }
   const int hpw = (p.heads + kGatedWarps - 1) / kGatedWarps;
   const int threads = kGatedWarps * 32;
-  if (hpw <= 1) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 1, kGatedWarps>, p.rows, threads, p, stream);
-  if (hpw <= 2) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 2, kGatedWarps>, p.rows, threads, p, stream);
-  if (hpw <= 4) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 4, kGatedWarps>, p.rows, threads, p, stream);
+  if (hpw <= 1) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 1, kGatedWarps, false>, p.rows, threads, p, stream);
+  if (hpw <= 2) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 2, kGatedWarps, false>, p.rows, threads, p, stream);
+  if (hpw <= 4) return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, 4, kGatedWarps, false>, p.rows, threads, p, stream);
   if (hpw <= kMaxHeadsPerWarp)
-    return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, kMaxHeadsPerWarp, kGatedWarps>, p.rows, threads, p, stream);
+    return launch_rows(gated_rmsnorm_quant_kernel<T, Y_F32, kMaxHeadsPerWarp, kGatedWarps, false>, p.rows, threads, p, stream);
   return bq::kErrUnsupported;
 }
 

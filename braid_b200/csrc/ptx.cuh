@@ -427,6 +427,9 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
 // The two halves of it; the first one orders nothing.
 __device__ __forceinline__ void cluster_arrive_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
@@ -449,6 +452,29 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
 }
 __device__ __forceinline__ void st_cluster_f1(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+// A word into another CTA's shared memory, its four bytes counted on a barrier there.
+__device__ __forceinline__ void st_async_cluster(uint32_t addr, uint32_t v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar)
+               : "memory");
+}
+// mbar_wait for a barrier that other CTAs of the cluster complete with what they stored.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  for (;;) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok != 0) return true;
+    if (clock64() - t0 > kSpinLimitCycles) return false;
+  }
 }
 __device__ __forceinline__ float ld_cluster_f1(uint32_t addr) {
   float v;

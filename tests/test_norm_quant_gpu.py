@@ -388,3 +388,33 @@ def test_silu_of_the_looped_gated_norm_is_the_ieee_quotient(Q, lib, dt):
                                               1, 1, 128, h[i].data_ptr(), 128, scale.data_ptr(), ws.data_ptr(), 16,
                                               stream) == 0
         assert torch.equal(h.float().cpu().flatten(), want)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("cols", [128, 1000, 1024, 4096, 5120, 8192])
+def test_exchange_inside_a_cluster_equals_the_grid_wide_one(Q, dt, cols):
+    """Up to 64 rows the CTAs of a norm or quantizer are one cluster that exchanges the maximum in shared memory (option
+    `quant_cluster`), with one to four rows per CTA: either side of every count, rows left over, the largest value in the
+    first, a middle and the last row, and a NaN there.  The same bits as through the grid-wide exchange."""
+    heads = max(1, cols // 128)
+    gamma, g128 = _gamma(cols, 3, spread=0.3), _gamma(128, 4)
+    for rows in (2, 3, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65):
+        for peak in (0, rows // 2, rows - 1):
+            for value in (300.0, float("nan")):
+                x = randn_cpu((rows, cols), seed=rows, dtype=dt).cuda()
+                x[peak, -1] = value
+                y, z = x[:, :heads * 128 if cols >= 128 else cols].float(), torch.randn(rows, heads * 128, device="cuda").to(dt)
+                got = []
+                for on in (0, 1):
+                    Q.set_option("quant_cluster", on)
+                    try:
+                        a = Q.rms_norm_quant(x, gamma, EPS, keep_dense=True)
+                        b = Q.gated_rms_norm_quant(y, z, g128, EPS, 128) if cols % 128 == 0 and heads <= 64 else a
+                        c = Q.quantize_act(x)
+                        d = Q.sigmoid_gate_quant(x, x)
+                    finally:
+                        Q.set_option("quant_cluster", 1)
+                    got.append([u8(a.dense), u8(a.q), u8(a.scale), u8(b.q), u8(b.scale), u8(c[0]), u8(c[1]), u8(d[0]), u8(d[1])])
+                for i, (p, q) in enumerate(zip(*got)):
+                    assert torch.equal(p, q), f"{rows} x {cols}, peak {peak} {value}: output {i}"
+    assert Q.device_status() == 0
