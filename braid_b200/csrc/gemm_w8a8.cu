@@ -847,7 +847,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   const int m_begin = krank * per;
   const int m_end = (m_begin + per < p.M) ? (m_begin + per) : p.M;
   if (ok) {
-    const bool col_ok = (row0 + lane * 4) < seg.n;      // n is a multiple of 16
+    const bool col_ok = (row0 + lane * 4) < seg.n;      // n is a multiple of 4
     const uint32_t part_addr = smem_u32(part);
     const int peer0 = group * split;
     const EpilogueArgs ea{handover ? slices : part, part_addr, peer0, handover ? per : 0, m_begin, m_end, warp, lane, row0,
@@ -1304,12 +1304,13 @@ __device__ __forceinline__ void pair_epilogue_rows(const GemmParams& p, const Se
         const int row = pass * 4 + (lane >> 3);
         const int m = m_row0 + row;
         const uint4 v = *reinterpret_cast<const uint4*>(box + row * 128 + ((piece ^ (row & 7)) << 4));
-        if (m < p.M && col < seg.n) {         // n is a multiple of 16: a piece is in or out as a whole
-          // rows are 8-byte aligned at least (checked by the host)
+        if (m < p.M && col < seg.n) {
+          // rows are 8-byte aligned at least (checked by the host); n is a multiple of 16, or of 4 for a 16-bit weight,
+          // whose last piece may be in by half
           if (!PUSH || p.push.n == 0) {
             uint8_t* dst = static_cast<uint8_t*>(seg.y) + ((long long)m * seg.ldy + col) * ES;
             *reinterpret_cast<uint2*>(dst) = make_uint2(v.x, v.y);
-            *reinterpret_cast<uint2*>(dst + 8) = make_uint2(v.z, v.w);
+            if (ES == 4 || col + 4 < seg.n) *reinterpret_cast<uint2*>(dst + 8) = make_uint2(v.z, v.w);
           } else {
             // column-parallel form: the same piece into every rank's gathered buffer (plain
             // stores through peer-mapped pointers, this rank's own buffer included)
@@ -2503,7 +2504,7 @@ int run_grouped(const void* xq, const float* sx, int64_t M, int64_t K, int n_seg
   for (int i = 0; i < n_seg; ++i) {   // argument checks first: no CUDA call before they pass
     const bool is_dense = dn != nullptr && dn->kind[i] != 0;
     if (!wq[i] || (!sw[i] && !is_dense) || N[i] <= 0) return kErrBadArg;
-    if (N[i] % 16 || !aligned_to(wq[i], 16)) return kErrUnsupported;
+    if (N[i] % (is_dense ? 4 : 16) || !aligned_to(wq[i], 16)) return kErrUnsupported;
     if ((pair == nullptr || pair->prefill) && push == nullptr &&
         !(am != nullptr && !am->store_logits)) {   // forms that write y
       if (!y[i]) return kErrBadArg;

@@ -142,8 +142,18 @@ struct UnitOut {
 template <typename T, int EPI>
 __device__ __forceinline__ void store_chunk(const UnitOut& o, int c, float (&v)[16]) {
   const int col = o.row0 + c;
-  if (!o.row_ok || col >= o.seg.n) return;        // n is a multiple of 16: a chunk is in or out
+  if (!o.row_ok || col >= o.seg.n) return;        // n is a multiple of 16: a chunk is in or out ...
   const bool wide = o.seg.wide != 0;
+  if constexpr (sizeof(T) == 2 && EPI != kResidual) {
+    if (o.seg.n - col < 16) {                     // ... but a 16-bit weight's is one of 4
+      T* const dst = static_cast<T*>(o.seg.y) + (long long)o.m * o.seg.ldy + col;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (col + 4 * q < o.seg.n)
+          reinterpret_cast<uint2*>(dst)[q] = make_uint2(bq::qd::pack2<T>(v[4 * q], v[4 * q + 1]), bq::qd::pack2<T>(v[4 * q + 2], v[4 * q + 3]));
+      return;
+    }
+  }
   if (EPI == kResidual || (EPI == kAny && o.seg.res != nullptr))
     add_res16<T>(v, static_cast<const T*>(o.seg.res) + (long long)o.m * o.seg.ld_res + col, wide);
   if (EPI != kAny || o.p.push.n == 0) {

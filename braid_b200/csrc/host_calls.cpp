@@ -518,15 +518,17 @@ PyObject* project(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   void* yp[BQ_MAX_SEGMENTS];
   int64_t N[BQ_MAX_SEGMENTS];
   int kind[BQ_MAX_SEGMENTS];
-  bool mixed = false;
+  bool mixed = false, ragged = false;
   for (Py_ssize_t i = 0; i < n; ++i) {
     const at::Tensor w = arg(PyTuple_GET_ITEM(a[4], i));
     PyObject* const so = PyTuple_GET_ITEM(a[5], i);
     if (!w.defined()) Py_RETURN_NONE;
     if (so == Py_None) {
-      if (!plain(h, w) || w.scalar_type() != out || w.dim() != 2 || w.size(1) != K || w.size(0) % 16 || w.size(0) == 0 ||
-          !w.is_contiguous() || !aligned(w.data_ptr(), 16) || (M > 256 && (w.size(0) > 256 || recorded(w))))
+      if (!plain(h, w) || w.scalar_type() != out || w.dim() != 2 || w.size(1) != K || w.size(0) % 4 || w.size(0) == 0 ||
+          !w.is_contiguous() || !aligned(w.data_ptr(), 16) || (M > 256 && w.size(0) > 256) ||
+          ((M > 256 || w.size(0) % 16) && recorded(w)))
         Py_RETURN_NONE;
+      ragged = ragged || w.size(0) % 16 != 0;
       kind[i] = 1;
       sw[i] = nullptr;
       mixed = true;
@@ -542,7 +544,7 @@ PyObject* project(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const void* dp = nullptr;
   if (mixed) {
     if (!dense.defined() || !plain(h, dense) || dense.scalar_type() != out || code == BQ_DTYPE_F32 ||
-        !dense.is_contiguous() || dense.numel() != M * K || !aligned(dense.data_ptr(), 16) || (M > 256 && recorded(dense)))
+        !dense.is_contiguous() || dense.numel() != M * K || !aligned(dense.data_ptr(), 16) || ((M > 256 || ragged) && recorded(dense)))
       Py_RETURN_NONE;
     dp = dense.data_ptr();
   }

@@ -1030,7 +1030,8 @@ def _project_mixed(xq, sx, dense: torch.Tensor, weights, lead, K):
     if (not _DENSE_SEGMENTS or M == 0 or dt not in (torch.bfloat16, torch.float16)
             or len(weights) > _lib.BQ_MAX_SEGMENTS):
         return None
-    if M > 256 and _recorded(dense, *(w for w in weights if not isinstance(w, FP8Weight))):
+    dense_w = [w for w in weights if not isinstance(w, FP8Weight)]
+    if (M > 256 or any(w.dim() == 2 and w.shape[0] % 16 for w in dense_w)) and _recorded(dense, *dense_w):
         return None
     d2 = dense.reshape(-1, K)
     if not d2.is_contiguous() or d2.data_ptr() % 16:
@@ -1039,9 +1040,9 @@ def _project_mixed(xq, sx, dense: torch.Tensor, weights, lead, K):
         if isinstance(w, FP8Weight):
             if w.data.shape[1] != K or not w.data.is_contiguous():
                 return None
-        elif (w.dtype != dt or w.dim() != 2 or w.shape[1] != K or w.shape[0] % 16
+        elif (w.dtype != dt or w.dim() != 2 or w.shape[1] != K or w.shape[0] % 4
               or not w.is_contiguous() or w.data_ptr() % 16 or not w.is_cuda
-              or (M > 256 and (w.shape[0] > 256 or w.device != dense.device))):
+              or (M > 256 and w.shape[0] > 256) or ((M > 256 or w.shape[0] % 16) and w.device != dense.device)):
             return None
     lib = _require_lib()
     n = len(weights)

@@ -600,7 +600,8 @@ int bq_gemm_w8a8_grouped(const void* xq, const float* sx, int64_t M, int64_t K, 
  *
  *   x_dense      device, [M, K] of dense_dtype (BQ_DTYPE_BF16 or BQ_DTYPE_F16), contiguous,
  *                16-byte aligned; out_dtype must equal dense_dtype when a 16-bit segment exists
- *   w[i]         device, e4m3 codes (kind 0) or 16-bit values (kind != 0), contiguous [N_i, K]
+ *   w[i]         device, e4m3 codes (kind 0) or 16-bit values (kind != 0), contiguous [N_i, K];
+ *                N_i a multiple of 16, of a 16-bit weight a multiple of 4
  * Returns BQ_ERR_UNSUPPORTED for M > 256 with a 16-bit segment of more than 256 rows: call
  * bq_gemm_w8a8_grouped and a dense GEMM instead.
  */

@@ -461,6 +461,36 @@ def test_prefill_mixed_projection_as_one_launch(Q, dt, M, K, widths):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("M", [1, 16, 48, 49, 100, 128, 161, 256, 257, 300])
+def test_sixteen_bit_weights_of_few_odd_rows_ride_along(Q, dt, M):
+    """Gates of 8, 20 or 40 rows (hidden 1024, 2560, 5120), and of 4, 36 or 244: a 16-bit weight's rows are a multiple of 4.
+    One launch on each of the three kernels, FP8 members bit-equal to their own, 16-bit ones within half a unit of the type of
+    the exact product; nothing beyond a row's end is written; what records gradients or has another count of rows
+    goes through `F.linear`, as before."""
+    K = 1040
+    x = randn_cpu((M, K), seed=M, dtype=dt).cuda()
+    w = Q.quantize_weight(randn_cpu((2 * K, K), seed=1, scale=0.02).cuda())
+    xq, sx = Q.quantize_act(x)
+    pre = Q.QuantizedActivation(xq, sx, x.shape, dt, dense=x)
+    for widths in ((8, 20), (40, 4), (36, 244, 48)):
+        dense = [randn_cpu((n, K), seed=2 + n, dtype=dt, scale=0.02).cuda() for n in widths]
+        n0 = Q.launch_count()
+        ys = Q.project(pre, w, *dense)
+        assert Q.launch_count() - n0 == 1
+        assert torch.equal(ys[0], Q.fp8_matmul(xq, sx, w, out_dtype=dt))
+        for y, d in zip(ys[1:], dense):
+            assert y.dtype is dt and y.shape == (M, d.shape[0]) and y.is_contiguous()
+            assert max_rel(y, F.linear(x.double(), d.double())) <= (2 ** -8 if dt is torch.bfloat16 else 2 ** -10)
+        assert all(torch.equal(p, q) for p, q in zip(ys, Q.project(x, w, *dense)))
+    odd = randn_cpu((18, K), seed=5, dtype=dt, scale=0.02).cuda()
+    assert torch.equal(Q.project(pre, w, odd)[1], F.linear(x, odd))
+    d = randn_cpu((20, K), seed=6, dtype=dt, scale=0.02).cuda().requires_grad_()
+    got = Q.project(pre, w, d)[1]
+    assert got.requires_grad and torch.equal(got, F.linear(x, d))
+    assert Q.device_status() == 0
+
+
 def test_leading_dims_and_dispatch(Q):
     x = randn_cpu((2, 3, 256), seed=19).cuda()
     w = randn_cpu((512, 256), seed=20, scale=0.02).cuda()
