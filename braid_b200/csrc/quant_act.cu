@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
     if (tid == 0) p.scale[0] = sc;
   }
   if constexpr (PHASE != kScaleOnly) {
-    const ScaleDiv dv(sc);
+    const ScaleMul<T> dv(sc);
     // Every thread re-reads exactly the groups it read in pass 1 (the L2 keeps a line on
     // the side of the chip whose SM asked for it, so the same SM finds it again), last
     // iteration first: what pass 1 read last is the likeliest to be still there.
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       const T* src = reinterpret_cast<const T*>(p.a) + static_cast<size_t>(p.n_groups) * kGroup;
       uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;
       for (unsigned int i = 0; i < p.tail; ++i)
-        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(src + i)), dv),
+        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(src + i)), dv.div),
                                        __NV_SATFINITE, __NV_E4M3);
     }
   }
@@ -229,13 +229,13 @@ __device__ __forceinline__ float unit_absmax(const uint4& raw, float m) {
 
 // codes of the 16 bytes `raw` holds: 8 for a 16-bit type, 4 for fp32
 template <typename T, bool OWN_SCALE>
-__device__ __forceinline__ void unit_emit(const uint4& raw, const ScaleDiv& dv, uint8_t* dst) {
+__device__ __forceinline__ void unit_emit(const uint4& raw, const ScaleMul<T>& dv, uint8_t* dst) {
   if constexpr (sizeof(T) == 2) {
     emit8<T, OWN_SCALE>(*reinterpret_cast<const Pack8<T>*>(&raw), dv, dst);
   } else {
     float f[4] = {__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z),
                   __uint_as_float(raw.w)};
-    divide_group<T, 4, OWN_SCALE>(dv, f);
+    divide_group<T, 4, OWN_SCALE>(dv.div, f);
     const uint32_t a = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
     const uint32_t b = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
     *reinterpret_cast<uint32_t*>(dst) = (a & 0xFFFFu) | ((b & 0xFFFFu) << 16);
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
     if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
   }
   {
-    const ScaleDiv dv(sc);
+    const ScaleMul<T> dv(kCasts ? sc : 0.0f);      // a scale of 0: nothing to prepare
     float m = 0.0f;
     if (producer) {
       if (lane == 0) {
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
       if (owns_tail) {
         uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;
         for (unsigned int i = 0; i < p.tail; ++i)
-          dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(tail_src + i)), dv), __NV_SATFINITE, __NV_E4M3);
+          dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(tail_src + i)), dv.div), __NV_SATFINITE, __NV_E4M3);
       }
     } else if constexpr (PHASE == kMaxOnly) {
       m = cta_amax(m);
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
   }
   // ---- backward pass of the whole quantizer: the ring's contents first, then re-fetches ----
   if constexpr (PHASE == kBoth) {
-    const ScaleDiv dv(sc);
+    const ScaleMul<T> dv(sc);
     const int refetch = count - kRingStages;   // chunks [0, refetch) are no longer in the ring
     if (producer) {
       if (lane == 0 && s_failed == 0u) {
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
     if (owns_tail) {
       uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;
       for (unsigned int i = 0; i < p.tail; ++i)
-        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(tail_src + i)), dv), __NV_SATFINITE, __NV_E4M3);
+        dst[i] = __nv_cvt_float_to_fp8(quant_one(widen(__ldcg(tail_src + i)), dv.div), __NV_SATFINITE, __NV_E4M3);
     }
   }
   // no bulk copy is in flight here unless a wait ran out: every issued copy was waited for by

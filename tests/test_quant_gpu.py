@@ -506,3 +506,25 @@ def test_quantize_weight_can_be_traced_and_transformed(Q):
     assert same(f(neg), b.neg())
     with pytest.raises(RuntimeError):          # as with the torch spelling
         torch.func.vmap(f)(torch.stack([a, b]))
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+def test_codes_by_one_product_under_the_scale_of_every_maximum(Q, dt):
+    """The passes over large inputs take a code from ONE product where the scale allows it (`ScaleMul`); max |x| / 448 is the
+    scale that lies closest to the ties, since 3/4 of the maximum may be one exactly.  Every mantissa a maximum can have, all
+    values of the type up to it, through the quantizer (ring kernel) and the cast alone, and under scales one and two units
+    away; against the torch spelling."""
+    bits = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).cuda().view(dt)
+    mant = 7 if dt is torch.bfloat16 else 10
+    base = (127 << 7) if dt is torch.bfloat16 else (18 << 10)
+    for m in range(0, 1 << mant, 1 if mant == 7 else 5):
+        top = torch.tensor([base + m], dtype=torch.int16).cuda().view(dt)
+        x = torch.where((bits.float().abs() <= top.float()), bits, torch.zeros_like(bits)).repeat(32).contiguous()
+        q, s = Q.quantize_act(x)
+        qr, sr = TS.quantize_act(x)
+        _assert_same(q, s, qr, sr, f"{dt} maximum {top.item()}")
+        for ulps in (-2, -1, 1, 2):
+            other = (sr.view(torch.int32) + ulps).view(torch.float32)
+            want = (bits.float() / other).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
+            assert torch.equal(u8(Q.cast_act(bits, other)).reshape(-1), u8(want).reshape(-1)), f"{dt} {top.item()} {ulps}"
+    assert Q.device_status() == 0
