@@ -46,6 +46,7 @@ namespace {
 struct Lib {
   decltype(&bq_quantize_act) quantize_act;
   decltype(&bq_rmsnorm_quant) rmsnorm_quant;
+  decltype(&bq_rmsnorm_quant_rows) rmsnorm_quant_rows;
   decltype(&bq_rmsnorm_scale) rmsnorm_scale;
   decltype(&bq_gated_rmsnorm_quant) gated_rmsnorm_quant;
   decltype(&bq_gated_rmsnorm_scale) gated_rmsnorm_scale;
@@ -272,7 +273,15 @@ PyObject* rms_norm_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     rc = g_lib.rmsnorm_quant(x.data_ptr(), code, r.rows, K, r.ld, gamma.data_ptr<float>(), (float)eps, hp, K, q.data_ptr(),
                              scale.data_ptr<float>(), slot, 16, h.stream);
   }
-  if (rc == BQ_ERR_TOO_LARGE) {
+  if (rc == BQ_ERR_TOO_LARGE && !keep) {
+    const at::Tensor rstd = empty(h, {r.rows}, at::kFloat);
+    NoGil no_gil;
+    rc = g_lib.rmsnorm_quant_rows(x.data_ptr(), code, r.rows, K, r.ld, gamma.data_ptr<float>(), (float)eps, q.data_ptr(),
+                                  scale.data_ptr<float>(), rstd.data_ptr<float>(), slot, 16, h.stream);
+    if (rc == BQ_OK) g_launches.fetch_add(1, std::memory_order_relaxed);
+    if (rc == BQ_ERR_UNSUPPORTED) rc = BQ_ERR_TOO_LARGE;
+  }
+  if (rc == BQ_ERR_TOO_LARGE) {      // h is wanted, or rows are no whole 16-byte pieces: h and its scale, then the cast of h
     at::Tensor norm = keep ? dense : empty(h, {r.rows, K}, x.scalar_type());
     {
       NoGil no_gil;
@@ -689,7 +698,7 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return true;
   };
   if (!get("bq_quantize_act", g_lib.quantize_act) || !get("bq_rmsnorm_quant", g_lib.rmsnorm_quant) ||
-      !get("bq_rmsnorm_scale", g_lib.rmsnorm_scale) ||
+      !get("bq_rmsnorm_quant_rows", g_lib.rmsnorm_quant_rows) || !get("bq_rmsnorm_scale", g_lib.rmsnorm_scale) ||
       !get("bq_gated_rmsnorm_quant", g_lib.gated_rmsnorm_quant) ||
       !get("bq_gated_rmsnorm_scale", g_lib.gated_rmsnorm_scale) || !get("bq_cast_act", g_lib.cast_act) ||
       !get("bq_sigmoid_gate_quant", g_lib.sigmoid_gate_quant) ||

@@ -45,6 +45,7 @@ struct NormParams {
   void* h_out;        // optional normalised activation in the activation type
   uint8_t* q;
   float* scale;
+  float* rstd;        // prefill: [rows], from the first launch to the second
   void* ws;
   int rows, cols;
   long long ld_x, ld_h;
@@ -352,17 +353,58 @@ __global__ void __launch_bounds__(kRowGroups * kNormThreads) rmsnorm_rows_quant_
 }
 
 // ---------------------------------------------------------------------------------------------
-// plain RMSNorm at prefill sizes: more rows than one co-resident grid has CTAs.  Every CTA loops
-// over rows (row arithmetic exactly as above), writes the normalised activation h, and keeps the
-// running max |h|; nobody waits for anybody: each CTA folds its max into one word with an
-// atomicMax and counts itself, and the CTA that counts last turns the word into the scale and
-// returns the scratch to zero.  The codes are then one cast pass over h under that scale
-// (bq_cast_act), in stream order.
+// plain RMSNorm at prefill sizes: more rows than one co-resident grid has CTAs.  Two launches, and nobody waits for
+// anybody.  The first finds every row's rstd and max |h|: each CTA loops over rows (row arithmetic as above), folds its
+// max into one word with an atomicMax and counts itself, and the CTA that counts last turns the word into the scale and
+// returns the scratch to zero.  The second reads x again -- last rows first, of which L2 still has some -- normalises it once
+// more with the rstd found, and casts: 9658 x 4096 bf16 are 79 + 79 + 40 MB, where a first launch that writes h and a cast of
+// h move 79 + 79 + 79 + 40: 53.9 -> 39.7 us (fp32 85 -> 62).  Those (DENSE, 53.9 -> 44.4 with the loops below; bq_rmsnorm_scale and bq_cast_act) are what is left where h is wanted anyway.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int VPT>
+// Running max |.| of values of T.
+template <typename T>
+struct AbsMax {
+  float m = 0.0f;
+  uint32_t pairs = 0u;      // 16-bit types: two at a time
+  __device__ __forceinline__ void add(const Vec4<T>& v) {
+    if constexpr (sizeof(T) == 2) {
+      const uint2 w = *reinterpret_cast<const uint2*>(&v);
+      pairs = absmax2<T>(absmax2<T>(pairs, w.x), w.y);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kVec; ++j) m = nan_max(m, fabsf(widen(v.v[j])));
+    }
+  }
+  __device__ __forceinline__ float value() const {
+    if constexpr (sizeof(T) == 2) {
+      const float2 f = unpack2<T>(pairs);
+      return nan_max(f.x, f.y);
+    } else {
+      return m;
+    }
+  }
+};
+
+// v <- T(gamma * (rstd * v)), two values rounded at an instruction where T has 16 bits.
+template <typename T, int N>
+__device__ __forceinline__ void scale_norm(T (&v)[N], const float (&g)[N], float rstd) {
+  if constexpr (sizeof(T) == 2) {
+    uint32_t* const w = reinterpret_cast<uint32_t*>(v);
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const float2 y = mul2(make_float2(g[i], g[i + 1]), mul2(make_float2(rstd, rstd), unpack2<T>(w[i / 2])));
+      w[i / 2] = pack2<T>(y.x, y.y);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = __fmul_rn(g[i], __fmul_rn(rstd, v[i]));
+  }
+}
+
+// DENSE: h is written, and nobody reads rstd.
+template <typename T, int VPT, bool DENSE>
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_scale_kernel(const NormParams p) {
   bq::pdl_launch_dependents();
-  __shared__ float s_red[4];
+  __shared__ float s_red_of[2][4];
   __shared__ float s_max[4];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int n_vec = p.cols / kVec;
@@ -372,55 +414,79 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_scale_kernel(const NormP
   for (int v = t; v < n_vec; v += kNormThreads) s_gamma[v] = __ldg(reinterpret_cast<const float4*>(p.gamma) + v);
   __syncthreads();
   bq::pdl_wait_prior_grids();
-  float m = 0.0f;
-  for (int row = blockIdx.x; row < p.rows; row += gridDim.x) {
-    const T* xr = reinterpret_cast<const T*>(p.x) + static_cast<long long>(row) * p.ld_x;
-    Vec4<T> x[VPT];
+  AbsMax<T> mx;
+  // One loop for rows of VPT whole vectors per thread, one for the others.  A third of the instructions of the second are
+  // its comparisons, and a launch is bound by its instructions as much as by its bytes.
+  auto walk = [&](auto full) {
+    constexpr bool kFull = decltype(full)::value;
+    auto has = [&](int i) { return kFull || t + i * kNormThreads < n_vec; };
+    // where the registers allow it the next row is asked for before this one is summed
+    constexpr bool kAhead = VPT * sizeof(T) <= 16;
+    const long long step = static_cast<long long>(gridDim.x) * p.ld_x;
+    const T* xr = reinterpret_cast<const T*>(p.x) + static_cast<long long>(blockIdx.x) * p.ld_x + t * kVec;
+    Vec4<T> buffer[kAhead ? 2 : 1][VPT];
+    auto load_row = [&](const T* from, Vec4<T>* to) {
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int v = t + i * kNormThreads;
-      if (v < n_vec) x[i] = load4(xr + v * kVec);
-    }
-    float s = 0.0f;
+      for (int i = 0; i < VPT; ++i)
+        if (has(i)) to[i] = load4(from + i * (kNormThreads * kVec));
+    };
+    auto one_row = [&](int row, Vec4<T>* x, float* r) {
+      float s = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int v = t + i * kNormThreads;
-      if (v < n_vec) {
+      for (int i = 0; i < VPT; ++i) {
+        if (has(i)) {
 #pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-          const float f = widen(x[i].v[j]);
-          s = __fmaf_rn(f, f, s);
+          for (int j = 0; j < kVec; ++j) {
+            const float f = widen(x[i].v[j]);
+            s = __fmaf_rn(f, f, s);
+          }
         }
       }
-    }
-    s = warp_tree_sum(s);
-    if (lane == 0 && warp >= 2) s_red[warp - 2] = s;
-    __syncthreads();
-    if (lane == 0 && warp < 2) s = __fadd_rn(s, s_red[warp]);
-    __syncthreads();
-    if (lane == 0 && warp == 1) s_red[0] = s;
-    __syncthreads();
-    if (t == 0) s_red[1] = __fdiv_rn(__fadd_rn(s, s_red[0]), static_cast<float>(p.cols));
-    __syncthreads();
-    const float rstd = rsqrtf(__fadd_rn(s_red[1], p.eps));
-    T* hr = reinterpret_cast<T*>(p.h_out) + static_cast<long long>(row) * p.ld_h;
+      s = warp_tree_sum(s);
+      if (lane == 0) r[warp] = s;
+      __syncthreads();                       // the other words may still be read
+      s = __fadd_rn(__fadd_rn(r[0], r[2]), __fadd_rn(r[1], r[3]));
+      s = __fdiv_rn(s, static_cast<float>(p.cols));
+      const float rstd = rsqrtf(__fadd_rn(s, p.eps));
+      if (!DENSE && t == 0) p.rstd[row] = rstd;
+      T* const hr = reinterpret_cast<T*>(p.h_out) + static_cast<long long>(row) * p.ld_h + t * kVec;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int v = t + i * kNormThreads;
-      if (v < n_vec) {
-        const float4 gv = s_gamma[v];
-        const float g[kVec] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-          const float y = __fmul_rn(g[j], __fmul_rn(rstd, widen(x[i].v[j])));
-          x[i].v[j] = narrow<T>(y);
-          m = nan_max(m, fabsf(widen(x[i].v[j])));
+      for (int i = 0; i < VPT; ++i) {
+        if (has(i)) {
+          const float4 gv = s_gamma[t + i * kNormThreads];
+          const float g[kVec] = {gv.x, gv.y, gv.z, gv.w};
+          scale_norm<T, kVec>(x[i].v, g, rstd);
+          mx.add(x[i]);
+          if constexpr (DENSE) store4(hr + i * (kNormThreads * kVec), x[i]);
         }
-        store4(hr + v * kVec, x[i]);
+      }
+    };
+    int row = blockIdx.x;
+    if (row >= p.rows) return;
+    if constexpr (kAhead) {
+      load_row(xr, buffer[0]);
+      for (;;) {
+        xr += step;
+        if (row + (int)gridDim.x < p.rows) load_row(xr, buffer[1]);
+        one_row(row, buffer[0], s_red_of[0]);
+        row += gridDim.x;
+        if (row >= p.rows) break;
+        xr += step;
+        if (row + (int)gridDim.x < p.rows) load_row(xr, buffer[0]);
+        one_row(row, buffer[1], s_red_of[1]);
+        row += gridDim.x;
+        if (row >= p.rows) break;
+      }
+    } else {
+      for (int parity = 0; row < p.rows; row += gridDim.x, xr += step, parity ^= 1) {
+        load_row(xr, buffer[0]);
+        one_row(row, buffer[0], s_red_of[parity]);
       }
     }
-    __syncthreads();   // s_red is written again by the next row
-  }
+  };
+  if (n_vec == VPT * kNormThreads) walk(std::true_type{});
+  else walk(std::false_type{});
+  float m = mx.value();
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
   if (lane == 0) s_max[warp] = m;
@@ -440,6 +506,43 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_scale_kernel(const NormP
       ws->arrive = 0u;
       __threadfence();
     }
+  }
+}
+
+// The second launch: a thread keeps gamma of its 8 columns and walks rows, kCastRows of them in flight.
+constexpr int kCastThreads = 256;
+constexpr int kCastRows = 4;
+template <typename T>
+__global__ void __launch_bounds__(kCastThreads) rmsnorm_cast_kernel(const NormParams p) {
+  bq::pdl_launch_dependents();
+  const int group = blockIdx.x * kCastThreads + threadIdx.x;
+  const bool live = group < p.cols / kGroup;
+  float g[kGroup];
+#pragma unroll
+  for (int i = 0; i < kGroup; i += 4) {
+    const float4 f = live ? __ldg(reinterpret_cast<const float4*>(p.gamma) + group * 2 + i / 4) : make_float4(0, 0, 0, 0);
+    g[i] = f.x; g[i + 1] = f.y; g[i + 2] = f.z; g[i + 3] = f.w;
+  }
+  bq::pdl_wait_prior_grids();
+  const ScaleMul<T> dv(__ldcg(p.scale));
+  if (!live) return;
+  const T* const x = reinterpret_cast<const T*>(p.x) + group * kGroup;
+  for (int top = p.rows - 1 - blockIdx.y * kCastRows; top >= 0; top -= gridDim.y * kCastRows) {
+    Pack8<T> v[kCastRows];
+    float rstd[kCastRows];
+#pragma unroll
+    for (int k = 0; k < kCastRows; ++k)
+      if (top - k >= 0) {
+        v[k] = load8<T>(x + static_cast<long long>(top - k) * p.ld_x);
+        rstd[k] = __ldcg(p.rstd + top - k);
+      }
+#pragma unroll
+    for (int k = 0; k < kCastRows; ++k)
+      if (top - k >= 0) {
+        const int row = top - k;
+        scale_norm<T, kGroup>(v[k].v, g, rstd[k]);
+        emit8<T, true>(v[k], dv, p.q + static_cast<long long>(row) * p.cols + group * kGroup);
+      }
   }
 }
 
@@ -758,30 +861,6 @@ inline bool known_dtype(int d) { return d == BQ_DTYPE_F32 || d == BQ_DTYPE_BF16 
 // flight per warp.  With the cast pass, 9658 x 32 heads, fp32 scan output: 121 -> 95 us; 4096 rows 57 -> 44.
 constexpr int kQuad = 4;
 
-// Running max |.| of values of T.
-template <typename T>
-struct AbsMax {
-  float m = 0.0f;
-  uint32_t pairs = 0u;      // 16-bit types: two at a time
-  __device__ __forceinline__ void add(const Vec4<T>& v) {
-    if constexpr (sizeof(T) == 2) {
-      const uint2 w = *reinterpret_cast<const uint2*>(&v);
-      pairs = absmax2<T>(absmax2<T>(pairs, w.x), w.y);
-    } else {
-#pragma unroll
-      for (int j = 0; j < kVec; ++j) m = nan_max(m, fabsf(widen(v.v[j])));
-    }
-  }
-  __device__ __forceinline__ float value() const {
-    if constexpr (sizeof(T) == 2) {
-      const float2 f = unpack2<T>(pairs);
-      return nan_max(f.x, f.y);
-    } else {
-      return m;
-    }
-  }
-};
-
 // The shuffle-down tree sums of four values at once.  Every step halves the lanes of a value and hands
 // the other half's lanes to another value, so that 6 shuffles do the work of 20; what is added to
 // what is the tree of warp_tree_sum (operands in either order: addition commutes).  Lane l
@@ -828,8 +907,7 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_scale_kernel(c
         if constexpr (Y_F32) {
           const float4 f = __ldcg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.y) + row * p.ld_y +
                                                                   off + h * kHeadDim));
-          core[h].v[0] = narrow<T>(f.x); core[h].v[1] = narrow<T>(f.y);
-          core[h].v[2] = narrow<T>(f.z); core[h].v[3] = narrow<T>(f.w);
+          *reinterpret_cast<uint2*>(&core[h]) = make_uint2(pack2<T>(f.x, f.y), pack2<T>(f.z, f.w));
         } else {
           core[h] = load4(reinterpret_cast<const T*>(p.y) + row * p.ld_y + off + h * kHeadDim);
         }
@@ -854,10 +932,19 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_scale_kernel(c
       const float rstd = __shfl_sync(0xffffffffu, rstd8, h * 8);
       float silu[kVec] = {widen(gate[h].v[0]), widen(gate[h].v[1]), widen(gate[h].v[2]), widen(gate[h].v[3])};
       gate_group<T, kSilu, kVec>(silu);
+      if constexpr (sizeof(T) == 2) {
+        uint32_t* const w = reinterpret_cast<uint32_t*>(&core[h]);
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) {
-        const T xn = narrow<T>(__fmul_rn(rstd, widen(core[h].v[j])));
-        core[h].v[j] = narrow<T>(__fmul_rn(__fmul_rn(gmv[j], widen(xn)), silu[j]));
+        for (int j = 0; j < kVec; j += 2) {
+          const float2 r = mul2(make_float2(rstd, rstd), unpack2<T>(w[j / 2]));
+          const float2 xn = unpack2<T>(pack2<T>(r.x, r.y));
+          const float2 y = mul2(mul2(make_float2(gmv[j], gmv[j + 1]), xn), make_float2(silu[j], silu[j + 1]));
+          w[j / 2] = pack2<T>(y.x, y.y);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j)
+          core[h].v[j] = __fmul_rn(__fmul_rn(gmv[j], __fmul_rn(rstd, core[h].v[j])), silu[j]);
       }
       if (h < live) {
         mx.add(core[h]);
@@ -891,7 +978,7 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_scale_kernel(c
 }
 
 namespace {
-template <typename T>
+template <typename T, bool DENSE>
 int launch_rmsnorm_scale(const NormParams& p, cudaStream_t stream) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -903,11 +990,39 @@ int launch_rmsnorm_scale(const NormParams& p, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(p.cols) * sizeof(float);     // gamma
   if (smem > 48 * 1024) return bq::kErrUnsupported;
   cudaError_t e;
-  if (per_thread <= 2) e = launch_resident_smem(rmsnorm_scale_kernel<T, 2>, p.rows, kNormThreads, sms, true, smem, stream, p);
-  else if (per_thread <= 4) e = launch_resident_smem(rmsnorm_scale_kernel<T, 4>, p.rows, kNormThreads, sms, true, smem, stream, p);
-  else if (per_thread <= 8) e = launch_resident_smem(rmsnorm_scale_kernel<T, 8>, p.rows, kNormThreads, sms, true, smem, stream, p);
-  else if (per_thread <= 16) e = launch_resident_smem(rmsnorm_scale_kernel<T, 16>, p.rows, kNormThreads, sms, true, smem, stream, p);
+  if (per_thread <= 2) e = launch_resident_smem(rmsnorm_scale_kernel<T, 2, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
+  else if (per_thread <= 4) e = launch_resident_smem(rmsnorm_scale_kernel<T, 4, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
+  else if (per_thread <= 8) e = launch_resident_smem(rmsnorm_scale_kernel<T, 8, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
+  else if (per_thread <= 16) e = launch_resident_smem(rmsnorm_scale_kernel<T, 16, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
   else return bq::kErrUnsupported;
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
+  return bq::kOk;
+}
+
+// CTAs that are resident at once, the rows dealt out among those of one column block.
+template <typename T>
+int launch_rmsnorm_cast(const NormParams& p, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  const int per_sm = resident_per_sm(rmsnorm_cast_kernel<T>, kCastThreads, 0);
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1) {
+    (void)cudaGetLastError();
+    return bq::kErrLaunch;
+  }
+  const int columns = (p.cols / kGroup + kCastThreads - 1) / kCastThreads;
+  int slices = per_sm * sms / columns;
+  if (slices > (p.rows + kCastRows - 1) / kCastRows) slices = (p.rows + kCastRows - 1) / kCastRows;
+  if (slices < 1) slices = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(columns), static_cast<unsigned>(slices), 1);
+  cfg.blockDim = dim3(kCastThreads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, rmsnorm_cast_kernel<T>, p);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
   return bq::kOk;
 }
@@ -932,9 +1047,39 @@ extern "C" int bq_rmsnorm_scale(const void* x, int dtype, int64_t rows, int64_t 
   p.ld_x = ld_x; p.ld_h = ld_h; p.eps = eps;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case BQ_DTYPE_F32: return launch_rmsnorm_scale<float>(p, s);
-    case BQ_DTYPE_BF16: return launch_rmsnorm_scale<__nv_bfloat16>(p, s);
-    default: return launch_rmsnorm_scale<__half>(p, s);
+    case BQ_DTYPE_F32: return launch_rmsnorm_scale<float, true>(p, s);
+    case BQ_DTYPE_BF16: return launch_rmsnorm_scale<__nv_bfloat16, true>(p, s);
+    default: return launch_rmsnorm_scale<__half, true>(p, s);
+  }
+}
+
+extern "C" int bq_rmsnorm_quant_rows(const void* x, int dtype, int64_t rows, int64_t cols, int64_t ld_x, const float* gamma,
+                                     float eps, void* q_out, float* scale_out, float* rstd, void* ws, size_t ws_bytes, void* stream) {
+  if (!x || !gamma || !q_out || !scale_out || !rstd || rows <= 0 || cols <= 0) return bq::kErrBadArg;
+  if (!known_dtype(dtype)) return bq::kErrBadArg;
+  if (ws == nullptr || ws_bytes < sizeof(QuantWs) || !aligned_to(ws, 16)) return bq::kErrWorkspace;
+  const size_t es = elem_size(dtype);
+  if (cols % kGroup || ld_x < cols || (ld_x * es) % 16 || !aligned_to(x, 16) || !aligned_to(gamma, 16) ||
+      !aligned_to(q_out, 8) || !aligned_to(rstd, 4))
+    return bq::kErrUnsupported;
+  if (rows > 0x7fffffffLL || cols > 0x7fffffffLL) return bq::kErrTooLarge;
+  NormParams p{};
+  p.x = x; p.gamma = gamma;
+  p.q = static_cast<uint8_t*>(q_out); p.scale = scale_out; p.rstd = rstd; p.ws = ws;
+  p.rows = static_cast<int>(rows); p.cols = static_cast<int>(cols);
+  p.ld_x = ld_x; p.eps = eps;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  int rc;
+  switch (dtype) {
+    case BQ_DTYPE_F32: rc = launch_rmsnorm_scale<float, false>(p, s); break;
+    case BQ_DTYPE_BF16: rc = launch_rmsnorm_scale<__nv_bfloat16, false>(p, s); break;
+    default: rc = launch_rmsnorm_scale<__half, false>(p, s);
+  }
+  if (rc != bq::kOk) return rc;
+  switch (dtype) {
+    case BQ_DTYPE_F32: return launch_rmsnorm_cast<float>(p, s);
+    case BQ_DTYPE_BF16: return launch_rmsnorm_cast<__nv_bfloat16>(p, s);
+    default: return launch_rmsnorm_cast<__half>(p, s);
   }
 }
 

@@ -25,6 +25,21 @@ constexpr int kGroup = 8;      // elements per group (one 128-bit load of a 16-b
 
 enum Mode { kPlain = 0, kSiluMul = 1, kSigmoidGate = 2 };
 
+// n / d for 32-bit n without a division: floor((n * mul) >> 32 >> shift) with the round-up multiplier of Granlund and
+// Montgomery (PLDI 1994), exact for n < 2^31.
+struct FastDiv {
+  unsigned int d, mul, shift;
+  static FastDiv by(unsigned int d) {
+    unsigned int l = 0;
+    while ((1ull << l) < d) ++l;
+    const unsigned long long m = ((1ull << (31 + l)) + d - 1) / d;      // 2^31 <= m < 2^32 unless d is 1
+    return l == 0 ? FastDiv{d, 0u, 0u} : FastDiv{d, static_cast<unsigned int>(m), l - 1};
+  }
+  __device__ __forceinline__ unsigned int operator()(unsigned int n) const {
+    return mul == 0u ? n : __umulhi(n, mul) >> shift;
+  }
+};
+
 struct QParams {
   const void* a;        // x | gate | o
   const void* b;        // - | up   | gate
@@ -34,9 +49,9 @@ struct QParams {
   float* partial;       // weight quantizer: the CTAs' maxima, from its first launch to its second
   unsigned int n_groups;      // full groups of 8
   unsigned int tail;          // plain mode only: leftover elements (< 8)
-  unsigned int groups_per_row;
+  FastDiv groups_per_row;
   long long ld_a, ld_b;       // row strides in elements (prologue modes)
-  unsigned int chunk;         // sigmoid gate: head width of the strided gate view
+  FastDiv chunk;              // sigmoid gate: head width of the strided gate view
   long long chunk_stride;     // sigmoid gate: distance between heads
   int held;                   // groups each thread keeps (hold kernel)
   // column-parallel form: the input is a gathered buffer other ranks store into; wait until the
@@ -100,6 +115,17 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) {
   if constexpr (std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<const __half2*>(&w));
   else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
 }
+// Two fp32 products at an instruction, each rounded as by itself.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long x, y, z;
+  float2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(z) : "l"(x), "l"(y));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(z));
+  return r;
+}
+
 // max(m, |v[0..7]|), NaN-propagating.  The 16-bit types take the maximum on packed pairs
 // (`abs` and `max.NaN` on two values per instruction; the maximum of 16-bit values is one of
 // them, so nothing is rounded) and widen once at the end.
@@ -251,14 +277,7 @@ __device__ __forceinline__ uint32_t codes4_mul(uint32_t lo, uint32_t hi, float m
   uint32_t out[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const float2 v = unpack2<T>(i == 0 ? lo : hi);
-    unsigned long long p, q, mm;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(v.x), "f"(v.y));
-    asm("mov.b64 %0, {%1, %1};" : "=l"(mm) : "f"(mul));
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(p), "l"(mm));
-    float a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(q));
-    out[i] = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
+    out[i] = __nv_cvt_float2_to_fp8x2(mul2(unpack2<T>(i == 0 ? lo : hi), make_float2(mul, mul)), __NV_SATFINITE, __NV_E4M3);
   }
   return __byte_perm(out[0], out[1], 0x5410);
 }
@@ -311,6 +330,13 @@ __device__ __forceinline__ float corrected_quotient(float x, float d) {
   return copysignf(__fmaf_rn(__fmaf_rn(-d, q, x), y, q), x);
 }
 
+// 1 / d of the same: the first quotient is the estimate itself, and nothing is negative.
+__device__ __forceinline__ float corrected_reciprocal(float d) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return __fmaf_rn(__fmaf_rn(-d, y, 1.0f), y, y);
+}
+
 enum Gate { kSilu, kSigmoid };
 
 template <typename T, Gate G, int N>
@@ -321,7 +347,10 @@ __device__ __forceinline__ void gate_group(float (&x)[N]) {
     for (int i = 0; i < N; ++i) ok = ok && fabsf(x[i]) <= 80.0f;
     if (ok) {
 #pragma unroll
-      for (int i = 0; i < N; ++i) x[i] = corrected_quotient(G == kSilu ? x[i] : 1.0f, 1.0f + expf(-x[i]));
+      for (int i = 0; i < N; ++i) {
+        const float d = 1.0f + expf(-x[i]);
+        x[i] = G == kSilu ? corrected_quotient(x[i], d) : corrected_reciprocal(d);
+      }
       return;
     }
   }
@@ -347,8 +376,8 @@ __device__ __forceinline__ void gated_product(float (&gated)[N], const float (&o
   if constexpr (sizeof(T) == 2) {
 #pragma unroll
     for (int i = 0; i < N; i += 2) {
-      const float2 s = unpack2<T>(pack2<T>(gated[i], gated[i + 1]));
-      const float2 h = unpack2<T>(pack2<T>(s.x * other[i], s.y * other[i + 1]));
+      const float2 p = mul2(unpack2<T>(pack2<T>(gated[i], gated[i + 1])), make_float2(other[i], other[i + 1]));
+      const float2 h = unpack2<T>(pack2<T>(p.x, p.y));
       gated[i] = h.x;
       gated[i + 1] = h.y;
     }
@@ -364,16 +393,16 @@ __device__ __forceinline__ void load_raw(const QParams& p, unsigned int g, Pack8
   if constexpr (MODE == kPlain) {
     a = load8<T>(reinterpret_cast<const T*>(p.a) + static_cast<size_t>(g) * kGroup);
   } else {
-    const unsigned int row = g / p.groups_per_row;
-    const unsigned int col = (g - row * p.groups_per_row) * kGroup;
+    const unsigned int row = p.groups_per_row(g);
+    const unsigned int col = (g - row * p.groups_per_row.d) * kGroup;
     const T* pa = reinterpret_cast<const T*>(p.a) + static_cast<long long>(row) * p.ld_a + col;
     const T* pb;
     if constexpr (MODE == kSiluMul) {
       pb = reinterpret_cast<const T*>(p.b) + static_cast<long long>(row) * p.ld_b + col;
     } else {
-      const unsigned int head = col / p.chunk;
+      const unsigned int head = p.chunk(col);
       pb = reinterpret_cast<const T*>(p.b) + static_cast<long long>(row) * p.ld_b +
-           static_cast<long long>(head) * p.chunk_stride + (col - head * p.chunk);
+           static_cast<long long>(head) * p.chunk_stride + (col - head * p.chunk.d);
     }
     a = load8<T>(pa);
     b = load8<T>(pb);
@@ -384,17 +413,37 @@ __device__ __forceinline__ void load_raw(const QParams& p, unsigned int g, Pack8
 // LARGE: the kernel runs this many times over (see gate_group).
 template <typename T, int MODE, bool LARGE = false>
 __device__ __forceinline__ void apply_prologue(Pack8<T>& a, const Pack8<T>& b) {
-  if constexpr (MODE != kPlain && LARGE) {
+  if constexpr (MODE != kPlain && LARGE && sizeof(T) == 2) {
+    // the operand of the gate function: gate of SiLU(gate) * up, gate of o * sigmoid(gate)
+    const uint4 gw = *reinterpret_cast<const uint4*>(MODE == kSiluMul ? &a : &b);
+    const uint4 ow = *reinterpret_cast<const uint4*>(MODE == kSiluMul ? &b : &a);
+    const uint32_t g[4] = {gw.x, gw.y, gw.z, gw.w}, o[4] = {ow.x, ow.y, ow.z, ow.w};
+    float x[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 v = unpack2<T>(g[i]);
+      x[2 * i] = v.x;
+      x[2 * i + 1] = v.y;
+    }
+    gate_group<T, MODE == kSiluMul ? kSilu : kSigmoid, 8>(x);
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      // two roundings to T, as of the separate kernels
+      const float2 h = mul2(unpack2<T>(pack2<T>(x[2 * i], x[2 * i + 1])), unpack2<T>(o[i]));
+      w[i] = pack2<T>(h.x, h.y);
+    }
+    *reinterpret_cast<uint4*>(&a) = make_uint4(w[0], w[1], w[2], w[3]);
+  } else if constexpr (MODE != kPlain && LARGE) {
     float x[8], y[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      // the operand of the gate function first: gate of SiLU(gate) * up, gate of o * sigmoid(gate)
       x[i] = widen(MODE == kSiluMul ? a.v[i] : b.v[i]);
       y[i] = widen(MODE == kSiluMul ? b.v[i] : a.v[i]);
     }
     gated_product<T, MODE == kSiluMul ? kSilu : kSigmoid, 8>(x, y);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) a.v[i] = narrow<T>(x[i]);   // exact: values of T already
+    for (int i = 0; i < 8; ++i) a.v[i] = narrow<T>(x[i]);
   } else if constexpr (MODE != kPlain) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {

@@ -714,8 +714,19 @@ def rms_norm_quant(x: torch.Tensor, gamma: torch.Tensor, eps: float,
         if rc == _lib.BQ_ERR_TOO_LARGE:
             global _launches
             _launches -= 1            # the refused call launched nothing
-            # prefill: more rows than CTAs can wait for one another -- rows looped per CTA, h and
-            # its scale from one launch with no grid-wide wait, then the cast pass
+            # prefill: more rows than CTAs can wait for one another -- rows looped per CTA in two launches with no
+            # grid-wide wait: the rows' 1 / rms and the scale, then a second read of x
+            if h is None:
+                rstd = torch.empty((rows,), dtype=torch.float32, device=x.device)
+                rc = lib.bq_rmsnorm_quant_rows(x2.data_ptr(), code, rows, K, x2.stride(0), gamma.data_ptr(), float(eps),
+                                               q.data_ptr(), scale.data_ptr(), rstd.data_ptr(), _take_slot(x.device), 16,
+                                               _stream_ptr(x.device))
+                if rc != _lib.BQ_ERR_UNSUPPORTED:
+                    _lib.check(rc, "rms_norm_quant_rows")
+                    _launches += 1
+                    return QuantizedActivation(q, scale, x.shape, x.dtype)
+                _launches -= 1
+            # h is wanted, or rows are no whole 16-byte pieces: h and its scale, then the cast of h
             if h is None:
                 h = torch.empty((rows, K), dtype=x.dtype, device=x.device)
             rc = lib.bq_rmsnorm_scale(x2.data_ptr(), code, rows, K, x2.stride(0), gamma.data_ptr(),

@@ -235,6 +235,18 @@ int bq_rmsnorm_quant(const void* x, int dtype, int64_t rows, int64_t cols, int64
                      float* scale_out, void* ws, size_t ws_bytes, void* stream);
 
 /*
+ * bq_rmsnorm_quant for any number of rows, as two launches of which neither waits for another CTA: the rows' 1 / rms and
+ * the scale, then a second read of x that normalises and casts.  The normalised activation is not kept (bq_rmsnorm_scale
+ * keeps it).  Bit-identical to bq_rmsnorm_quant.
+ *
+ *   rstd         device, [rows] fp32 scratch of the caller's, written by the first launch and read by the second
+ * x 16-byte aligned in base and row pitch, q_out 8-byte, cols a multiple of 8 and at most 8192; otherwise
+ * BQ_ERR_UNSUPPORTED.
+ */
+int bq_rmsnorm_quant_rows(const void* x, int dtype, int64_t rows, int64_t cols, int64_t ld_x, const float* gamma, float eps,
+                          void* q_out, float* scale_out, float* rstd, void* ws, size_t ws_bytes, void* stream);
+
+/*
  * The same norm for more rows than one co-resident grid has CTAs (prefill): every CTA loops
  * over rows, writes the normalised activation h_out (required here) and the grid leaves the
  * quantization scale of h in *scale_out without anybody waiting for anybody (one atomicMax and

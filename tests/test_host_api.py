@@ -107,6 +107,8 @@ def test_argument_validation_returns_before_any_cuda_call(lib):
     # the prefill-size and column-parallel entry points: every check precedes any CUDA call
     assert lib.bq_cast_act(None, 1, 8, 16, 16, None) == _lib.BQ_ERR_BAD_ARG
     assert lib.bq_cast_act(24, 1, 8, 16, 16, None) == _lib.BQ_ERR_UNSUPPORTED
+    assert lib.bq_rmsnorm_quant_rows(16, 1, 4, 64, 64, 16, 1e-6, 16, 16, None, 16, 16, None) == _lib.BQ_ERR_BAD_ARG
+    assert lib.bq_rmsnorm_quant_rows(16, 1, 4, 60, 64, 16, 1e-6, 16, 16, 16, 16, 16, None) == _lib.BQ_ERR_UNSUPPORTED
     assert lib.bq_rmsnorm_scale(16, 1, 4, 64, 64, 16, 1e-6, None, 64, 16, 16, 16, None) == _lib.BQ_ERR_BAD_ARG
     assert lib.bq_rmsnorm_scale(16, 1, 4, 64, 64, 16, 1e-6, 16, 64, 16, None, 0, None) == _lib.BQ_ERR_WORKSPACE
     assert lib.bq_rmsnorm_scale(16, 1, 4, 62, 64, 16, 1e-6, 16, 64, 16, 16, 16, None) == _lib.BQ_ERR_UNSUPPORTED

@@ -418,3 +418,22 @@ def test_exchange_inside_a_cluster_equals_the_grid_wide_one(Q, dt, cols):
                 for i, (p, q) in enumerate(zip(*got)):
                     assert torch.equal(p, q), f"{rows} x {cols}, peak {peak} {value}: output {i}"
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("rows,cols", [(4000, 512), (4001, 504), (3999, 500), (3000, 2560), (2500, 4096), (2371, 4088), (1500, 5120), (1300, 8192)])
+def test_rms_norm_quant_that_reads_its_rows_twice(Q, dt, rows, cols):
+    """Beyond the rows that are resident at once: rows of whole and of partial vectors per thread, rows that are no whole
+    16-byte pieces (through h), strided rows, more column blocks than one, with and without the dense form."""
+    x = randn_cpu((rows, cols + 16), seed=rows, dtype=dt, scale=2.0).cuda()[:, :cols]
+    x[::7] *= 20.0
+    gamma = _gamma(cols, 9, spread=0.3)
+    ref = TS.rms_norm(x, gamma, EPS)
+    for keep in (False, True):
+        qa = Q.rms_norm_quant(x, gamma, EPS, keep_dense=keep)
+        if keep:
+            assert torch.equal(u8(qa.dense), u8(ref))
+        _same(qa, ref, f"{rows} x {cols}")
+    x[rows - 1, cols - 1] = float("nan")
+    assert Q.rms_norm_quant(x, gamma, EPS).scale.isnan().all()
+    assert Q.device_status() == 0

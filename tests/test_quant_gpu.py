@@ -528,3 +528,23 @@ def test_codes_by_one_product_under_the_scale_of_every_maximum(Q, dt):
             want = (bits.float() / other).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
             assert torch.equal(u8(Q.cast_act(bits, other)).reshape(-1), u8(want).reshape(-1)), f"{dt} {top.item()} {ulps}"
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("rows,cols,chunk", [(1184, 1024, 256), (1185, 1024, 256), (2368, 1024, 128), (2369, 1024, 128), (4095, 1024, 64),
+                                             (4097, 1000, 8), (2600, 1000, 40), (1747, 2400, 24), (40001, 104, 104), (3, 24, 24)])
+def test_prologues_held_in_registers_up_to_the_two_launches(Q, dt, rows, cols, chunk):
+    """One launch up to 2^22 elements: one to eight groups per thread (either side of four, and of two for fp32), groups left
+    over, and row lengths and head widths that are no powers of two (their divisions are multiplications); beyond, the
+    two-launch form with the same coordinates."""
+    gu = randn_cpu((rows, 2 * cols), seed=rows, dtype=dt, scale=3.0).cuda()
+    gate, up = gu[:, :cols], gu[:, cols:]
+    n0 = Q.launch_count()
+    q, s = Q.silu_mul_quant(gate, up)
+    assert Q.launch_count() - n0 == (1 if rows * cols < 1 << 22 else 2)
+    _assert_same(q, s, *TS.quantize_act(TS.silu_mul(gate.contiguous(), up.contiguous())), f"silu {rows} x {cols}")
+    qg = randn_cpu((rows, cols // chunk, 2 * chunk), seed=rows + 1, dtype=dt, scale=3.0).cuda()
+    view, o = qg[..., chunk:], up.contiguous()
+    q, s = Q.sigmoid_gate_quant(o, view)
+    _assert_same(q, s, *TS.quantize_act(TS.sigmoid_gate(o, view.reshape(rows, cols))), f"sigmoid {rows} x {cols} by {chunk}")
+    assert Q.device_status() == 0
