@@ -180,9 +180,11 @@ struct GemmParams {
 // which a launch runs a tenth (35 to 52 KB now).  Four graphed decoder layers, one kernel -> these: hidden
 // 4096, 1 row 252 -> 246 us, 128 rows 339 -> 334; hidden 2560, 16 rows 231 -> 224; hidden 5120, 64 rows
 // 449 -> 435; hidden 1024, 8 rows 157 -> 149.  At prefill sizes the residual and 16-bit forms in the one
-// kernel had cost every launch 8 %.  kAny, with the type taken at run time, is the column-parallel and greedy
+// kernel had cost every launch 8 %.  kAny, with the type taken at run time, is the column-parallel
 // forms, and launches whose segments differ in their form.
-enum Epi { kAny = -1, kPlain = 0, kResidual = 1, kGateUp = 2, kMixed = 3, kGateUpDense = 4 };
+enum Epi { kAny = -1, kPlain = 0, kResidual = 1, kGateUp = 2, kMixed = 3, kGateUpDense = 4, kArgmax = 5 };
+// The greedy pick has kernels of its own too; in the general ones, a vocabulary of 248320 x 4096 with its logits, repeated: 16
+// rows 169 -> 163 us, 64 rows 212 -> 198, 128 rows 231 -> 205.
 constexpr int kAnyType = -1;
 
 struct alignas(64) WeightMaps {
@@ -343,30 +345,50 @@ __device__ __forceinline__ void reduce_store(const EpilogueArgs& e) {
   }
 }
 
-// Per batch row of this CTA's share: the best of the tile's 128 logits (see ArgmaxOut).  K is
-// not split in an argmax launch, so the staged tile is final.
+// The order of the greedy pick as one unsigned comparison: NaN on top, -0 and 0 alike.
+__device__ __forceinline__ uint32_t argmax_key(float v) {
+  const uint32_t b = __float_as_uint(__fadd_rn(v, 0.0f));
+  return v != v ? 0xFFFFFFFFu : ((b >> 31) != 0u ? ~b : b | 0x80000000u);
+}
+__device__ __forceinline__ uint32_t argmax_bits(uint32_t key) {      // the fp32 bits of its value
+  return key == 0xFFFFFFFFu ? 0x7FFFFFFFu : ((key >> 31) != 0u ? key & 0x7FFFFFFFu : ~key);
+}
+
+// Per batch row of this CTA's share: the best of the tile's 128 logits (see ArgmaxOut), and the logits themselves where
+// they are wanted.  K is not split in an argmax launch, so the staged tile is final.  A lane's four, then the warp's 32 in two
+// reductions (the largest key, the lowest index that has it); four rows at a time, since a row by itself is one chain.
 template <typename T>
-__device__ __forceinline__ void argmax_rows(const EpilogueArgs& e, int n_total, uint2* partial_tile) {
+__device__ __forceinline__ void argmax_rows(const EpilogueArgs& e, uint2* partial_tile, bool store) {
   using namespace bq::qd;
+  constexpr int kRows = 4;
   const int n4 = e.lane * 4;
-  for (int m = e.m_begin + e.warp; m < e.m_end; m += kStreamWarps) {
-    const float4 v = *reinterpret_cast<const float4*>(e.part + m * kRowTile + n4);
-    const float r[4] = {widen(narrow<T>(v.x * e.scale)), widen(narrow<T>(v.y * e.scale)),
-                        widen(narrow<T>(v.z * e.scale)), widen(narrow<T>(v.w * e.scale))};
-    float bv = 0.0f;
-    int bi = kNoIndex;                      // "nothing yet": loses against any real column
+  for (int m0 = e.m_begin + e.warp; m0 < e.m_end; m0 += kStreamWarps * kRows) {
+    float4 v[kRows];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int idx = e.row0 + n4 + j;
-      if (idx < n_total && (bi == kNoIndex || argmax_beats(r[j], idx, bv, bi))) { bv = r[j]; bi = idx; }
-    }
+    for (int i = 0; i < kRows; ++i)
+      if (m0 + i * kStreamWarps < e.m_end)
+        v[i] = *reinterpret_cast<const float4*>(e.part + (m0 + i * kStreamWarps) * kRowTile + n4);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-      if (oi != kNoIndex && (bi == kNoIndex || argmax_beats(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+    for (int i = 0; i < kRows; ++i) {
+      const int m = m0 + i * kStreamWarps;            // warp-uniform
+      if (m < e.m_end) {
+        v[i].x *= e.scale; v[i].y *= e.scale; v[i].z *= e.scale; v[i].w *= e.scale;
+        if (store && e.col_ok) store_out4(e.y, (long long)m * e.ldy + e.row0 + n4, e.out_dtype, v[i]);
+        uint32_t key = 0u;                            // below every value's
+        int at = 0;
+        if (e.col_ok) {                               // n is a multiple of 16: four columns are in or out
+          key = argmax_key(widen(narrow<T>(v[i].x)));
+          const uint32_t k1 = argmax_key(widen(narrow<T>(v[i].y))), k2 = argmax_key(widen(narrow<T>(v[i].z)));
+          const uint32_t k3 = argmax_key(widen(narrow<T>(v[i].w)));
+          if (k1 > key) { key = k1; at = 1; }
+          if (k2 > key) { key = k2; at = 2; }
+          if (k3 > key) { key = k3; at = 3; }
+        }
+        const uint32_t best = __reduce_max_sync(0xffffffffu, key);
+        const int first = __reduce_min_sync(0xffffffffu, key == best && e.col_ok ? e.row0 + n4 + at : kNoIndex);
+        if (e.lane == 0) partial_tile[m] = make_uint2(argmax_bits(best), static_cast<unsigned int>(first));
+      }
     }
-    if (e.lane == 0) partial_tile[m] = make_uint2(__float_as_uint(bv), static_cast<unsigned int>(bi));
   }
 }
 
@@ -587,7 +609,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                    const int smem_tile_bytes) {
   extern __shared__ uint8_t smem_dyn[];
   const bool pair_on = EPI == kAny ? p.pair.on != 0 : (EPI == kGateUp || EPI == kGateUpDense);
-  const bool argmax_on = EPI == kAny && p.argmax.on;
   const PushParams* const push = EPI == kAny && p.push.n > 0 ? &p.push : nullptr;
   const int out_dtype = DT == kAnyType ? p.out_dtype : DT;
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -755,6 +776,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       // A commit per block tells the loading warps that its slots are free; where none is filled twice nobody asks (four
       // graphed layers of hidden 4096, 1 row 199.9 -> 197.7 us, 48 rows 250.9 -> 249.9).  (Copies of the activation that bring 2
       // or 4 blocks save its warp 100 clocks a block, 0.3 % of those layers, and counting boxes in this loop costs 2 %.)
+      // Where this kernel casts the activation itself the test costs more than it saves: linear of 8 rows 7.93 and 8.13.
       const bool reuse = kb_count > p.stages || kb_count > p.b_stages;
       int s = 0, sb = 0;
       uint32_t phase = 0, phase_b = 0;
@@ -781,7 +803,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
           if constexpr (is_dense.value) mma_f16(issue, tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
           else mma_f8(issue, tmem_base, da + 2u * j, db + 2u * j, idesc, (i | j) != 0 ? 1u : 0u);
         }
-        if (reuse) mma_commit(issue, empty);   // both slots are free once these MMAs retire
+        if (QUANT || reuse) mma_commit(issue, empty);   // both slots are free once these MMAs retire
       }
     };
     if (dense) multiply(std::true_type{});
@@ -888,12 +910,12 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
           atomicMax(&p.pair.words[0], __float_as_uint(mx));
         }
       }
-    } else if (argmax_on) {
+    } else if (EPI == kArgmax) {
       uint2* const mine = p.argmax.partial + static_cast<size_t>(tile_in_seg) * p.M;
-      if (out_dtype == BQ_DTYPE_BF16) argmax_rows<__nv_bfloat16>(ea, seg.n, mine);
-      else if (out_dtype == BQ_DTYPE_F16) argmax_rows<__half>(ea, seg.n, mine);
-      else argmax_rows<float>(ea, seg.n, mine);
-      if (p.argmax.store_logits) reduce_store<1, false>(ea);
+      const bool store = p.argmax.store_logits != 0;
+      if (out_dtype == BQ_DTYPE_BF16) argmax_rows<__nv_bfloat16>(ea, mine, store);
+      else if (out_dtype == BQ_DTYPE_F16) argmax_rows<__half>(ea, mine, store);
+      else argmax_rows<float>(ea, mine, store);
     } else if (EPI == kPlain || (EPI == kAny && seg.res == nullptr)) {
       switch (split) {
         case 1: reduce_store<1, false>(ea); break;
@@ -1719,6 +1741,8 @@ const StreamKernel kStreamQuant[2][2][3] = {     // [is the maximum given?]
      {gemm_stream_kernel<kResidual, 0, 1>, gemm_stream_kernel<kResidual, 1, 1>, gemm_stream_kernel<kResidual, 2, 1>}},
     {{gemm_stream_kernel<kPlain, 0, 2>, gemm_stream_kernel<kPlain, 1, 2>, gemm_stream_kernel<kPlain, 2, 2>},
      {gemm_stream_kernel<kResidual, 0, 2>, gemm_stream_kernel<kResidual, 1, 2>, gemm_stream_kernel<kResidual, 2, 2>}}};
+const StreamKernel kStreamArgmax[3] = {gemm_stream_kernel<kArgmax, 0, 0>, gemm_stream_kernel<kArgmax, 1, 0>,
+                                      gemm_stream_kernel<kArgmax, 2, 0>};
 const StreamKernel kStreamAny = gemm_stream_kernel<kAny, kAnyType, 0>;
 template <int MODE>
 struct WideKernels {
@@ -1727,6 +1751,8 @@ struct WideKernels {
       {gemm_wide_kernel<MODE, kPlain, 0>, gemm_wide_kernel<MODE, kPlain, 1>, gemm_wide_kernel<MODE, kPlain, 2>},
       {gemm_wide_kernel<MODE, kResidual, 0>, gemm_wide_kernel<MODE, kResidual, 1>, gemm_wide_kernel<MODE, kResidual, 2>},
       {gemm_wide_kernel<MODE, kGateUp, 0>, gemm_wide_kernel<MODE, kGateUp, 1>, gemm_wide_kernel<MODE, kGateUp, 2>}};
+  static constexpr WideKernel argmax[3] = {gemm_wide_kernel<MODE, kArgmax, 0>, gemm_wide_kernel<MODE, kArgmax, 1>,
+                                           gemm_wide_kernel<MODE, kArgmax, 2>};
 };
 const PairKernel kPair[4][3] = {
     {gemm_pair_kernel<kPlain, 0>, gemm_pair_kernel<kPlain, 1>, gemm_pair_kernel<kPlain, 2>},
@@ -1738,7 +1764,8 @@ const PairKernel kPairAny = gemm_pair_kernel<kAny, kAnyType>;
 // The form all segments of a launch share, or kAny.  `mixed`: does the kernel have a form for 16-bit
 // segments (elsewhere they are a matter of a segment)?
 int epilogue_of(const GemmParams& p, bool mixed) {
-  if (p.push.n > 0 || p.argmax.on) return kAny;
+  if (p.argmax.on) return kArgmax;
+  if (p.push.n > 0) return kAny;
   if (p.pair.on) return p.pair.h != nullptr ? kGateUpDense : kGateUp;
   int with = 0, dense = 0;
   for (int i = 0; i < p.n_seg; ++i) {
@@ -1760,7 +1787,12 @@ int configure_once() {
     set((const void*)WideKernels<1>::any);
     set((const void*)WideKernels<2>::any);
     set((const void*)kPairAny);
-    for (int d = 0; d < 3; ++d) set((const void*)kStreamGateUpDense[d]);
+    for (int d = 0; d < 3; ++d) {
+      set((const void*)kStreamGateUpDense[d]);
+      set((const void*)kStreamArgmax[d]);
+      set((const void*)WideKernels<1>::argmax[d]);
+      set((const void*)WideKernels<2>::argmax[d]);
+    }
     for (int e = 0; e < 4; ++e)
       for (int d = 0; d < 3; ++d) {
         if (kPair[e][d] != nullptr) set((const void*)kPair[e][d]);
@@ -2016,7 +2048,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   if (quant && epi != kPlain && epi != kResidual) return kErrUnsupported;
   const StreamKernel kernel =
       quant ? kStreamQuant[p.quant.words != nullptr ? 1 : 0][epi][p.out_dtype]
-            : (epi == kAny ? kStreamAny : (epi == kGateUpDense ? kStreamGateUpDense[p.out_dtype] : kStream[epi][p.out_dtype]));
+            : (epi == kAny ? kStreamAny : epi == kArgmax ? kStreamArgmax[p.out_dtype] : (epi == kGateUpDense ? kStreamGateUpDense[p.out_dtype] : kStream[epi][p.out_dtype]));
   if (p.pair.on) p.pair.expected = (unsigned)((p.seg[0].n / kRowTile) * p.seg[0].split);
   if (p.push.n > 0)
     p.push.expected = (unsigned)(((p.seg[0].n + kRowTile - 1) / kRowTile) * p.seg[0].split);
@@ -2230,8 +2262,10 @@ int launch_wide(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const WeightM
 #endif
   const int epi = epilogue_of(p, false);
   const WideKernel kernel =
-      sh.mode == 1 ? (epi == kAny ? WideKernels<1>::any : WideKernels<1>::of[epi][p.out_dtype])
-                   : (epi == kAny ? WideKernels<2>::any : WideKernels<2>::of[epi][p.out_dtype]);
+      sh.mode == 1 ? (epi == kAny ? WideKernels<1>::any : epi == kArgmax ? WideKernels<1>::argmax[p.out_dtype]
+                                                                         : WideKernels<1>::of[epi][p.out_dtype])
+                   : (epi == kAny ? WideKernels<2>::any : epi == kArgmax ? WideKernels<2>::argmax[p.out_dtype]
+                                                                         : WideKernels<2>::of[epi][p.out_dtype]);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm_x, tm_xd, maps, p, sh);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return kErrLaunch; }
   return kOk;
@@ -2346,7 +2380,11 @@ struct DenseArgs {
 //    at 161 rows; 2560 x 7680: 0.96 alone, but the layers 324 -> 328 us: the line lies between).
 //
 // Several rounds (a vocabulary) pay an epilogue per round.  Where K is long it is hidden (60016 x 4096:
-// 33 rows 1.05, 129 rows 1.09), where K is short the batch has to be larger (60016 x 1024: 65 rows 1.14,
+// 129 rows 1.09).  Up to 48 rows the two are within 4 % of one another at full clock there (248320 x 4096 with the greedy pick, 48
+// rows 167 us on the K-sliced kernel and 163 here), but a stream of that length runs into the power limit when it is
+// repeated, and this kernel multiplies 128 rows whatever the batch: 176 to 180 and 186 to 195 us; 64 rows 197 and 185 to 205, 195
+// and 170 at full clock.  With fewer tiles than one and a half times what the K-sliced kernel holds it has a nearly
+// empty last wave (40000 x 4096, 33 rows 1.05).  Where K is short the batch has to be larger (60016 x 1024: 65 rows 1.14,
 // 129 rows 1.06).  The K-sliced kernel holds up to two CTAs per SM at once; while its tiles fit and fill
 // three quarters of that room, only its wide accumulators (more than 96 rows, and again more than 160) are
 // slower (32000 x 4096: 49 rows 0.95, 97 rows 1.01, 129 rows 0.88, 161 rows 1.06; 24576 x 4096: 1.08,
@@ -2363,7 +2401,8 @@ bool wide_applies(const GemmParams& p, const WideShape& sh) {
   if (sh.rounds > 1) {
     if (ctas <= 2 * sms && short_k) return p.M > 208;
     if (ctas <= 2 * sms && 2 * ctas > 3 * sms && p.k_blocks >= 16) return p.M > 96 && !between;
-    return p.k_blocks >= 16 ? p.M > 32 : p.M > 64 && !between;
+    if (p.k_blocks >= 16) return p.M > (ctas >= 3 * sms ? 48 : 32);
+    return p.M > 64 && !between;
   }
   if (p.M <= 48 || between) return false;
   if (p.pair.on) return true;

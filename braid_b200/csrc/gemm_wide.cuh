@@ -170,10 +170,22 @@ __device__ __forceinline__ void argmax_chunk(const UnitOut& o, int c, const floa
   using namespace bq::qd;
   const int col = o.row0 + c;
   if (col >= o.seg.n) return;
+  // columns come in ascending order: what is not larger than the best so far loses, by its index if by nothing else
+  float r[16];
+  bool ordered = true;
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    const float r = widen(narrow<T>(v[i]));
-    if (bi == kNoIndex || argmax_beats(r, col + i, bv, bi)) { bv = r; bi = col + i; }
+    r[i] = widen(narrow<T>(v[i]));
+    ordered = ordered && r[i] == r[i];
+  }
+  if (bi == kNoIndex) { bv = r[0]; bi = col; }
+  if (ordered) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (r[i] > bv) { bv = r[i]; bi = col + i; }
+  } else {
+    for (int i = 0; i < 16; ++i)
+      if (argmax_beats(r[i], col + i, bv, bi)) { bv = r[i]; bi = col + i; }
   }
 }
 
@@ -410,7 +422,6 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                    const __grid_constant__ WideShape sh) {
   using Lanes = LaneMap<MODE>;
   const int out_dtype = DT == kAnyType ? p.out_dtype : DT;
-  const bool argmax_on = EPI == kAny && p.argmax.on;
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
@@ -609,7 +620,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           load_sums(taddr + c, seg.split, cols, v);
 #pragma unroll
           for (int q = 0; q < 16; ++q) v[q] *= scale;
-          if (argmax_on) {
+          if constexpr (EPI == kArgmax) {
             if (out_dtype == BQ_DTYPE_BF16) argmax_chunk<__nv_bfloat16>(o, c, v, bv, bi);
             else if (out_dtype == BQ_DTYPE_F16) argmax_chunk<__half>(o, c, v, bv, bi);
             else argmax_chunk<float>(o, c, v, bv, bi);
@@ -627,7 +638,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         if (lane == 0) mbar_arrive_cluster(map_to_cta(acc_empty(b), 0));
       }
     }
-    if (argmax_on && row_ok) {
+    if (EPI == kArgmax && row_ok) {
       // a pair of 128 holds a row's columns in two lane quarters: two slots per column group
       const int slot = (unit0 * n_groups + col_group) * (MODE == 1 ? 2 : 1) + (MODE == 1 ? quad >> 1 : 0);
       p.argmax.partial[static_cast<size_t>(slot) * p.M + m0 + row] =
