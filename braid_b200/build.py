@@ -83,7 +83,7 @@ def build_host(force: bool = False) -> Path:
            f'-DBQ_HOST_KEY="{host_key()}"',
            *(arg for path in includes for arg in ("-isystem", path)),
            str(HOST_SRC), "-o", str(HOST), f"-L{torch_lib}",
-           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError("g++ failed:\n" + proc.stdout + proc.stderr)

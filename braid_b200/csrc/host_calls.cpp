@@ -18,6 +18,7 @@
 #include <ATen/ATen.h>
 #include <ATen/TracerMode.h>
 #include <ATen/autocast_mode.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -45,6 +46,8 @@ namespace {
 
 struct Lib {
   decltype(&bq_quantize_act) quantize_act;
+  decltype(&bq_quantize_weight) quantize_weight;
+  decltype(&bq_quantize_weight_workspace_bytes) quantize_weight_workspace;
   decltype(&bq_rmsnorm_quant) rmsnorm_quant;
   decltype(&bq_rmsnorm_quant_rows) rmsnorm_quant_rows;
   decltype(&bq_rmsnorm_scale) rmsnorm_scale;
@@ -177,8 +180,10 @@ bool recorded(const at::Tensor& t) {
   return (t.requires_grad() && c10::GradMode::is_enabled()) || at::autocast::is_autocast_enabled(at::kCUDA);
 }
 
+// Memory that is written whole before anybody reads it, from the allocator without the dispatcher (0.5 us of a call's 5):
+// the modes that would see a torch.empty are what Here leaves to quant.py.
 at::Tensor empty(const Here& h, at::IntArrayRef sizes, at::ScalarType t) {
-  return at::empty(sizes, at::TensorOptions().dtype(t).device(at::kCUDA, h.dev));
+  return at::Tensor(at::detail::empty_cuda(sizes, t, c10::Device(at::kCUDA, (c10::DeviceIndex)h.dev), std::nullopt));
 }
 
 struct NoGil {
@@ -237,6 +242,30 @@ PyObject* quantize_act(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!r.q.defined()) Py_RETURN_NONE;
   if (r.rc != BQ_OK) return refused();
   return pair(r.q, r.scale);
+  END_HANDLE_TH_ERRORS
+}
+
+// quantize_weight(w) -> (q, scale): a loader's call, 22 us from Python and 9 from here, which is its time for weights of up to
+// a few MB
+PyObject* quantize_weight(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  BQ_ARGS(1)
+  const at::Tensor w = arg(a[0]);
+  const Here h(w);
+  if (!h.ok || !plain(h, w)) Py_RETURN_NONE;
+  const int code = dtype_code(w.scalar_type());
+  if (code < 0 || w.dim() != 2 || w.numel() == 0 || !w.is_contiguous() || !aligned(w.data_ptr(), 16) || recorded(w)) Py_RETURN_NONE;
+  const at::Tensor q = empty(h, w.sizes(), at::kFloat8_e4m3fn), scale = empty(h, {1, 1}, at::kFloat);
+  const size_t bytes = g_lib.quantize_weight_workspace();
+  const at::Tensor ws = empty(h, {(int64_t)bytes}, at::kByte);
+  int rc;
+  {
+    NoGil no_gil;
+    rc = g_lib.quantize_weight(w.data_ptr(), code, w.numel(), q.data_ptr(), scale.data_ptr<float>(), ws.data_ptr(), bytes,
+                               h.stream);
+  }
+  if (rc != BQ_OK) Py_RETURN_NONE;
+  return pair(q, scale);
   END_HANDLE_TH_ERRORS
 }
 
@@ -578,11 +607,13 @@ PyObject* project(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// mlp(xq, sx, dtype, gate, s_gate, up, s_up, down, s_down, residual or None) -> [M, H]
+// mlp(xq, sx, dtype, gate, s_gate, up, s_up, down, s_down, residual or None) -> [M, H]; with sx None, xq is the [M, K] activation
+// itself, and what is quantized here before a refusal comes back as (xq, sx)
 PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   BQ_ARGS(10)
-  const at::Tensor xq = arg(a[0]), sx = arg(a[1]);
+  at::Tensor xq = arg(a[0]), sx = arg(a[1]);
+  const bool quantized = a[1] != Py_None;
   at::ScalarType out;
   const Here h(xq);
   if (!h.ok || !scalar_type_of(a[2], out)) Py_RETURN_NONE;
@@ -590,7 +621,10 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const at::Tensor wg = arg(a[3]), sg = arg(a[4]), wu = arg(a[5]), su = arg(a[6]), wd = arg(a[7]), sd = arg(a[8]);
   const at::Tensor residual = arg(a[9]);
   if (a[9] != Py_None && !residual.defined()) Py_RETURN_NONE;
-  if (code < 0 || !is_codes(h, xq) || !is_scale(h, sx)) Py_RETURN_NONE;
+  if (code < 0) Py_RETURN_NONE;
+  if (quantized ? !is_codes(h, xq) || !is_scale(h, sx)
+                : !plain(h, xq) || xq.scalar_type() != out || xq.dim() != 2 || xq.numel() == 0 || xq.size(1) % 16)
+    Py_RETURN_NONE;
   const int64_t M = xq.size(0), K = xq.size(1);
   if (!wg.defined() || !wu.defined() || !wd.defined() || !is_weight(h, wg, K) || !is_weight(h, wu, K) ||
       wu.size(0) != wg.size(0) || !is_weight(h, wd, wg.size(0)) || !is_scale(h, sg) || !is_scale(h, su) || !is_scale(h, sd))
@@ -604,6 +638,18 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
        !aligned(residual.data_ptr(), out == at::kFloat ? 16 : 8) || recorded(residual)))
     Py_RETURN_NONE;
   int rc;
+  if (!quantized) {
+    const Quantized r = quantize(h, xq);
+    if (!r.q.defined()) Py_RETURN_NONE;
+    if (r.rc != BQ_OK) return refused();
+    xq = r.q;
+    sx = r.scale;
+  }
+  auto given_back = [&]() -> PyObject* {
+    g_launches.fetch_sub(1, std::memory_order_relaxed);
+    if (!quantized) return pair(xq, sx);
+    Py_RETURN_NONE;
+  };
   // both products in one call, where that form takes them: asked before anything is allocated
   if (M <= BQ_MLP_MAX_ROWS && g_lib.mlp_takes(M, I, N, code) != 0) {
     const at::Tensor act = empty(h, {M, I}, out), y = empty(h, {M, N}, out);
@@ -615,8 +661,11 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
                      residual.defined() ? residual.stride(0) : 0, M, K, I, N, code, act.data_ptr(), y.data_ptr(), N,
                      slot.address, 16, h.stream);
     }
-    if (rc == BQ_OK) g_launches.fetch_add(1, std::memory_order_relaxed);      // the slot counted one of the two
-    if (rc != BQ_ERR_UNSUPPORTED) return gemm_result(y, rc);
+    if (rc == BQ_OK) {
+      g_launches.fetch_add(1, std::memory_order_relaxed);      // the slot counted one of the two
+      return wrap(y);
+    }
+    if (rc != BQ_ERR_UNSUPPORTED) return given_back();
     g_launches.fetch_sub(1, std::memory_order_relaxed);
   }
   at::Tensor hq, sh = empty(h, {1, 1}, at::kFloat), dense;
@@ -632,13 +681,14 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
                                        sg.data_ptr<float>(), su.data_ptr<float>(), M, I, K, code, dense.data_ptr(), I,
                                        sh.data_ptr<float>(), slot, 16, h.stream);
   }
-  if (rc != BQ_OK) return refused();
+  if (rc != BQ_OK) return given_back();
   if (M > 256) {
     rc = cast(h, dense, sh, hq);
-    if (rc != BQ_OK) return refused();
+    if (rc != BQ_OK) return given_back();
   }
   const at::Tensor y = gemm(h, hq, sh, wd, sd, out, residual, rc);
-  return gemm_result(y, rc);
+  if (!y.defined() || rc != BQ_OK) return given_back();
+  return wrap(y);
   END_HANDLE_TH_ERRORS
 }
 
@@ -697,7 +747,8 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     std::memcpy(&fn, &p, sizeof(p));
     return true;
   };
-  if (!get("bq_quantize_act", g_lib.quantize_act) || !get("bq_rmsnorm_quant", g_lib.rmsnorm_quant) ||
+  if (!get("bq_quantize_act", g_lib.quantize_act) || !get("bq_quantize_weight", g_lib.quantize_weight) ||
+      !get("bq_quantize_weight_workspace_bytes", g_lib.quantize_weight_workspace) || !get("bq_rmsnorm_quant", g_lib.rmsnorm_quant) ||
       !get("bq_rmsnorm_quant_rows", g_lib.rmsnorm_quant_rows) || !get("bq_rmsnorm_scale", g_lib.rmsnorm_scale) ||
       !get("bq_gated_rmsnorm_quant", g_lib.gated_rmsnorm_quant) ||
       !get("bq_gated_rmsnorm_scale", g_lib.gated_rmsnorm_scale) || !get("bq_cast_act", g_lib.cast_act) ||
@@ -763,6 +814,7 @@ PyMethodDef kMethods[] = {BQ_METHOD("init", init),
                           BQ_METHOD("next_slot", next_slot),
                           BQ_METHOD("launch_count", launch_count),
                           BQ_METHOD("quantize_act", quantize_act),
+                          BQ_METHOD("quantize_weight", quantize_weight),
                           BQ_METHOD("rms_norm_quant", rms_norm_quant),
                           BQ_METHOD("gated_rms_norm_quant", gated_rms_norm_quant),
                           BQ_METHOD("sigmoid_gate_quant", sigmoid_gate_quant),

@@ -155,7 +155,9 @@ def quantize_weight(w: torch.Tensor) -> FP8Weight:
         raise ValueError(
             f"_scaled_mm needs both weight dims to be multiples of 16; got "
             f"[{N}, {K}]. Leave this projection in bf16.")
-    fused = _quantize_weight_fused(w)
+    fused = _NATIVE.quantize_weight(w) if _NATIVE is not None else None
+    if fused is None:
+        fused = _quantize_weight_fused(w)
     if fused is not None:
         return FP8Weight(data=fused[0], scale=fused[1], shape=(N, K))
     scale = _weight_scale(w)
@@ -987,13 +989,17 @@ class residual_into:
         return False
 
 
+def _is_rows(t: torch.Tensor, cols: int) -> bool:
+    return t.dim() == 2 and t.shape[1] == cols
+
+
 def _claim_residual(w, lead, n, dtype):
     slot = _PENDING_RESIDUAL
     if (slot is None or slot.taken or slot.w is not w or slot.residual.dtype != dtype
             or tuple(slot.residual.shape) != (*lead, n)):
         return None
     slot.taken = True
-    return slot.residual.reshape(-1, n)
+    return slot.residual if slot.residual.dim() == 2 else slot.residual.reshape(-1, n)
 
 
 def fp8_linear(x: torch.Tensor, w: FP8Weight, residual: torch.Tensor | None = None) -> torch.Tensor:
@@ -1001,9 +1007,13 @@ def fp8_linear(x: torch.Tensor, w: FP8Weight, residual: torch.Tensor | None = No
     `residual` (same shape as the result) is added in the GEMM epilogue."""
     *lead, K = x.shape
     N = w.shape[0]
-    res2 = residual.reshape(-1, N) if residual is not None else _claim_residual(w, lead, N, x.dtype)
+    if residual is None:
+        res2 = _claim_residual(w, lead, N, x.dtype) if _PENDING_RESIDUAL is not None else None
+    else:
+        res2 = residual if _is_rows(residual, N) else residual.reshape(-1, N)
     if isinstance(x, QuantizedActivation):
-        return fp8_matmul(x.q, x.scale, w, out_dtype=x.dtype, residual=res2).reshape(*lead, N)
+        y = fp8_matmul(x.q, x.scale, w, out_dtype=x.dtype, residual=res2)
+        return y if len(lead) == 1 and lead[0] == y.shape[0] else y.reshape(*lead, N)
     pre = _attached(x)
     if pre is None and _NATIVE is not None:
         y = _NATIVE.linear(x, w.data, w.scale, res2)
@@ -1098,6 +1108,22 @@ def project(x: torch.Tensor, *weights: torch.Tensor | FP8Weight) -> list[torch.T
     `set_dense_segments(False)`) they take `F.linear`, as in the reference.
     """
     pre = x if isinstance(x, QuantizedActivation) else None
+    if pre is not None and _NATIVE is not None:
+        # the plain case of a decoder: everything given, all members in one launch
+        data, scales, sixteen_bit = [], [], 0
+        for w in weights:
+            if isinstance(w, FP8Weight):
+                data.append(w.data)
+                scales.append(w.scale)
+            else:
+                data.append(w)
+                scales.append(None)
+                sixteen_bit += 1
+        if sixteen_bit == 0 or sixteen_bit < len(weights) and pre.dense is not None and _DENSE_SEGMENTS:
+            dense = pre.dense if sixteen_bit else None
+            ys = _NATIVE.project(pre.q, pre.scale, dense, pre.dtype if dense is None else dense.dtype, tuple(data), tuple(scales))
+            if ys is not None:
+                return ys if len(pre.shape) == 2 else [y.reshape(*pre.shape[:-1], y.shape[1]) for y in ys]
     if not any(isinstance(w, FP8Weight) for w in weights):
         dense = pre.require_dense() if pre is not None else x
         return [F.linear(dense, w) for w in weights]
@@ -1365,18 +1391,19 @@ def mlp_forward(x: torch.Tensor, gate_proj: FP8Weight, up_proj: FP8Weight,
     """
     *lead, K = x.shape
     pre = x if isinstance(x, QuantizedActivation) else None
-    x2 = None if pre is not None else x.reshape(-1, K)
+    x2 = None if pre is not None else (x if len(lead) == 1 else x.reshape(-1, K))
     M = pre.q.shape[0] if pre is not None else x2.shape[0]
     I = gate_proj.shape[0]
-    res2 = residual.reshape(-1, down_proj.shape[0]) if residual is not None else None
+    res2 = residual if residual is None or _is_rows(residual, down_proj.shape[0]) else residual.reshape(-1, down_proj.shape[0])
     if (_PAIR_MLP and _NATIVE is not None and isinstance(gate_proj, FP8Weight) and isinstance(up_proj, FP8Weight)
             and isinstance(down_proj, FP8Weight)):
-        xq, sx = (pre.q, pre.scale) if pre is not None else quantize_act(x2)
+        xq, sx = (pre.q, pre.scale) if pre is not None else (x2, None)
         y = _NATIVE.mlp(xq, sx, x.dtype, gate_proj.data, gate_proj.scale, up_proj.data, up_proj.scale,
                         down_proj.data, down_proj.scale, res2)
-        if y is not None:
+        if type(y) is tuple:           # refused behind the quantizer: do not quantize twice
+            pre = QuantizedActivation(y[0], y[1], x.shape, x.dtype)
+        elif y is not None:
             return y if len(lead) == 1 else y.reshape(*lead, down_proj.shape[0])
-        pre = QuantizedActivation(xq, sx, x.shape, x.dtype)     # do not quantize twice
     if _PAIR_MLP and M <= 256 and x.device.type == "cuda":
         xq, sx = (pre.q, pre.scale) if pre is not None else quantize_act(x2)
         paired = gate_up_silu_quant(xq, sx, gate_proj, up_proj, x.dtype)
@@ -1406,5 +1433,7 @@ def gated_output_projection(o: torch.Tensor, gate: torch.Tensor, o_proj: FP8Weig
     *lead, K = o.shape
     oq, so = sigmoid_gate_quant(o, gate)
     res2 = _claim_residual(o_proj, lead, o_proj.shape[0], o.dtype)
+    if len(lead) == 1:
+        return fp8_matmul(oq, so, o_proj, out_dtype=o.dtype, residual=res2)
     return fp8_matmul(oq.reshape(-1, K), so, o_proj, out_dtype=o.dtype,
                       residual=res2).reshape(*lead, o_proj.shape[0])

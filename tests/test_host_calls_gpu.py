@@ -199,3 +199,39 @@ def test_native_calls_from_threads_and_streams(Q, weights):
     assert not wrong
     assert torch.equal(want, Q.mlp_forward(x, w["gate"], w["up"], w["down"]))
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,I", [(1, 256, 512), (16, 256, 512), (300, 256, 512), (16, 256, 28160), (16, 256, 576)])
+def test_mlp_quantizes_its_input_once(Q, M, K, I):
+    """A plain activation is quantized inside the native MLP call; where that call is refused behind the quantizer (28160 columns:
+    more CTAs than are resident at once) the codes are used, not made again.  Same bits and one launch more than from codes."""
+    g = torch.Generator(device="cuda").manual_seed(I + M)
+    gate, up, down = (Q.quantize_weight((torch.randn(n, k, generator=g, device="cuda") * 0.05).bfloat16())
+                      for n, k in ((I, K), (I, K), (K, I)))
+    x, res = (torch.randn(M, K, generator=g, device="cuda").bfloat16() for _ in range(2))
+    n0 = Q.launch_count()
+    y = Q.mlp_forward(x, gate, up, down, residual=res)
+    n1 = Q.launch_count()
+    qa = Q.QuantizedActivation(*Q.quantize_act(x), x.shape, x.dtype)
+    n2 = Q.launch_count()
+    want = Q.mlp_forward(qa, gate, up, down, residual=res)
+    assert torch.equal(y, want) and n1 - n0 == Q.launch_count() - n2 + 1
+    assert torch.equal(Q.mlp_forward(x.view(1, M, K), gate, up, down, residual=res.view(1, M, K)), want.view(1, M, K))
+    assert Q.device_status() == 0
+
+
+def test_native_weight_quantizer_gives_the_same_weight(Q):
+    """`quantize_weight` as a native call and from Python: same codes and scale; what torch would follow, strided weights
+    and odd types go the other ways they went."""
+    for dt in (torch.bfloat16, torch.float16, torch.float32):
+        w = torch.randn(272, 1040, device="cuda").to(dt)
+        a, b = Q.quantize_weight(w), Q._quantize_weight_fused(w)
+        assert torch.equal(a.data.view(torch.uint8), b[0].view(torch.uint8)) and torch.equal(a.scale, b[1])
+        assert a.shape == (272, 1040) and a.data.shape == (272, 1040) and a.scale.shape == (1, 1)
+        p = torch.nn.Parameter(w)
+        with torch.no_grad():
+            assert torch.equal(Q.quantize_weight(p).scale, a.scale)
+        t = w.t().contiguous().t()
+        assert torch.equal(Q.quantize_weight(t).data.view(torch.uint8), a.data.view(torch.uint8))
+    with pytest.raises(ValueError):
+        Q.quantize_weight(torch.randn(8, 16, device="cuda"))
