@@ -97,7 +97,23 @@ struct PairSilu {
   float* sh;               // device: the scale of h
   unsigned int* words;     // [0] amax bits [1] arrivals [2] departures ([3] is the sticky status)
   unsigned int expected;   // CTAs that take part in the exchange (the active ones)
+  const uint8_t* next;     // device: what the launch behind this one streams first, next_bytes of it (0: nothing)
+  unsigned int next_bytes;
 };
+
+// Behind the last load of a gate/up launch HBM idles for its tail: the exchange, the cast, the start of the down projection.  One
+// warp of every CTA asks its share of the first megabytes of the down weight into L2 meanwhile; behind the exchange, whose trips
+// to L2 a saturated memory would delay, and not more than the tail brings in.  Four graphed layers of hidden 4096, none / 8 MB
+// / 16 MB / 32 MB: 1 row 198.5 / 196.5 / 196.5 / 203.5 us, 8 rows 217.7 / 214.1 / 213.7 / 220.3, 16 rows 223.7 / 220.3 /
+// 219.9 / 225.8, 48 rows 251.2 / 249.0 / 250.6 / 255.0; before the exchange 8 MB give 217.1 at 8 rows and nothing at 27.  In pieces of
+// less than 1 KB, so that every CTA of the down projection gets its share, the instructions cost more than that (8 rows
+// 220 to 225).  A down weight of less than that loses (hidden 1024, 3 MB: 8 rows 103.3 and 105.4), and so does the kernel for
+// wider batches (64 rows 274.6 -> 278.3).
+constexpr unsigned int kNextBytes = 8u << 20, kNextPiece = 4096;
+__device__ __forceinline__ void prefetch_next(const PairSilu& pr) {
+  for (unsigned int at = (blockIdx.x * 32u + (threadIdx.x & 31u)) * kNextPiece; at < pr.next_bytes; at += gridDim.x * 32u * kNextPiece)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pr.next + at), "n"(kNextPiece) : "memory");
+}
 
 // Greedy pick fused into the lm_head GEMM: every CTA (one 128-row tile of the vocabulary, K not
 // split) reduces, per batch row, the largest of ITS 128 logits -- taken after the rounding to the
@@ -728,6 +744,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       }
       if (++s == p.stages) { s = 0; phase ^= 1u; }
     }
+    if (EPI == kGateUpDense) prefetch_next(p.pair);      // no exchange to wait for
     __syncwarp();
   } else if (QUANT && warp >= 2) {
     if constexpr (QUANT) {
@@ -993,6 +1010,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       s_quant[0] = sc;
     }
     __syncthreads();
+    if (EPI == kGateUp && warp == 0) prefetch_next(p.pair);
     const float sc = s_quant[0];
     if (ok) {
       const EpilogueArgs ea{part, smem_u32(part), 0, 0, m_begin, m_end, warp, lane, row0, 0.0f, true,
@@ -2830,11 +2848,26 @@ extern "C" int bq_lm_head_argmax(const void* xq, const void* wq, const float* sx
   return kOk;
 }
 
-extern "C" int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const void* wq_gate,
-                                          const void* wq_up, const float* sw_gate,
-                                          const float* sw_up, int64_t M,
-                                          int64_t I, int64_t K, int act_dtype, void* hq_out,
-                                          float* sh_out, void* ws, size_t ws_bytes, void* stream) {
+namespace {
+void set_next(PairSilu* pair, const void* next, int64_t bytes) {
+  pair->next = static_cast<const uint8_t*>(next);
+  pair->next_bytes = next != nullptr && bytes >= (int64_t)kNextBytes ? kNextBytes : 0u;
+}
+}  // namespace
+
+extern "C" int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const void* wq_gate, const void* wq_up,
+                                          const float* sw_gate, const float* sw_up, int64_t M, int64_t I, int64_t K,
+                                          int act_dtype, void* hq_out, float* sh_out, void* ws, size_t ws_bytes,
+                                          void* stream) {
+  return bq_gate_up_silu_quant_next_w8a8(xq, sx, wq_gate, wq_up, sw_gate, sw_up, M, I, K, act_dtype, hq_out, sh_out, nullptr, 0,
+                                         ws, ws_bytes, stream);
+}
+
+extern "C" int bq_gate_up_silu_quant_next_w8a8(const void* xq, const float* sx, const void* wq_gate, const void* wq_up,
+                                               const float* sw_gate, const float* sw_up, int64_t M, int64_t I, int64_t K,
+                                               int act_dtype, void* hq_out, float* sh_out, const void* next,
+                                               int64_t next_bytes, void* ws, size_t ws_bytes, void* stream) {
+  if (!aligned_to(next, 16)) return kErrUnsupported;
   if (!wq_gate || !wq_up || !sw_gate || !sw_up || !hq_out || !sh_out || I <= 0) return kErrBadArg;
   if (I % (kRowTile / 2) || !aligned_to(hq_out, 2) || !aligned_to(wq_up, 16)) return kErrUnsupported;
   PairSilu pair;
@@ -2844,6 +2877,7 @@ extern "C" int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const
   pair.hq = static_cast<uint8_t*>(hq_out);
   pair.ld_hq = I;
   pair.sh = sh_out;
+  set_next(&pair, next, next_bytes);
   const void* wqs[1] = {wq_gate};
   const float* sws[1] = {sw_gate};
   void* ys[1] = {nullptr};
@@ -2914,6 +2948,7 @@ extern "C" int bq_mlp_w8a8(const void* xq, const float* sx, const void* wq_gate,
   pair.wq_up = wq_up;
   pair.sw_up = sw_up;
   pair.h = h;
+  set_next(&pair, wq_down, I * N);
   const void* wqs[1] = {wq_gate};
   const float* sws[1] = {sw_gate};
   void* none[1] = {nullptr};

@@ -60,7 +60,7 @@ struct Lib {
   decltype(&bq_gemm_w8a8_residual) gemm_residual;
   decltype(&bq_linear_w8a8) linear;
   decltype(&bq_project_mixed) project_mixed;
-  decltype(&bq_gate_up_silu_quant_w8a8) gate_up_silu_quant;
+  decltype(&bq_gate_up_silu_quant_next_w8a8) gate_up_silu_quant;
   decltype(&bq_gate_up_silu_w8a8) gate_up_silu;
   decltype(&bq_mlp_w8a8_takes) mlp_takes;
   decltype(&bq_stream_is_captured) stream_is_captured;
@@ -676,7 +676,7 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     NoGil no_gil;
     rc = M <= 256 ? g_lib.gate_up_silu_quant(xq.data_ptr(), sx.data_ptr<float>(), wg.data_ptr(), wu.data_ptr(),
                                              sg.data_ptr<float>(), su.data_ptr<float>(), M, I, K, code, hq.data_ptr(),
-                                             sh.data_ptr<float>(), slot, 16, h.stream)
+                                             sh.data_ptr<float>(), wd.data_ptr(), N * I, slot, 16, h.stream)
                   : g_lib.gate_up_silu(xq.data_ptr(), sx.data_ptr<float>(), wg.data_ptr(), wu.data_ptr(),
                                        sg.data_ptr<float>(), su.data_ptr<float>(), M, I, K, code, dense.data_ptr(), I,
                                        sh.data_ptr<float>(), slot, 16, h.stream);
@@ -755,7 +755,7 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !get("bq_sigmoid_gate_quant", g_lib.sigmoid_gate_quant) ||
       !get("bq_sigmoid_mul_dense_scale", g_lib.sigmoid_mul_dense_scale) ||
       !get("bq_gemm_w8a8_grouped", g_lib.gemm_grouped) || !get("bq_gemm_w8a8_residual", g_lib.gemm_residual) ||
-      !get("bq_linear_w8a8", g_lib.linear) || !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_w8a8", g_lib.gate_up_silu_quant) || !get("bq_mlp_w8a8", g_lib.mlp) ||
+      !get("bq_linear_w8a8", g_lib.linear) || !get("bq_project_mixed", g_lib.project_mixed) || !get("bq_gate_up_silu_quant_next_w8a8", g_lib.gate_up_silu_quant) || !get("bq_mlp_w8a8", g_lib.mlp) ||
       !get("bq_mlp_w8a8_takes", g_lib.mlp_takes) || !get("bq_stream_is_captured", g_lib.stream_is_captured) ||
       !get("bq_gate_up_silu_w8a8", g_lib.gate_up_silu) || !get("bq_lm_head_argmax", g_lib.lm_head_argmax) ||
       !get("bq_lm_head_argmax_workspace_bytes", g_lib.lm_head_argmax_workspace))
