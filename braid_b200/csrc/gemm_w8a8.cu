@@ -535,15 +535,98 @@ __device__ __forceinline__ void silu_pair_emit(const EpilogueArgs& e, const floa
 // warps that have nothing to do until the accumulator is complete read the whole activation (a few
 // dozen KB, from L2) for its max |x|, then cast this CTA's K slice into the activation tiles.  The same
 // values in the same arithmetic everywhere, so every CTA finds the same scale and nothing is
-// exchanged; the quantizer's launch and its hand-over through memory are gone.  Two launches -> one, us in a
-// graph and eager: 1 row of 4096 x 4096 7.5 -> 6.6 and 10.7 -> 6.8, 4 rows of 1024 x 4096 7.3 -> 5.2 and 10.6 -> 6.0,
-// 8 rows of 512 x 1024 6.1 -> 4.2 and 10.6 -> 6.0, 16 rows of 2048 x 2048 7.3 -> 6.2 and 10.5 -> 6.8.  Where it stops
-// paying: quantize_inside_pays.
+// exchanged (SliceMax is the other form); the quantizer's launch and its hand-over through memory are gone.  Two launches ->
+// one, us in a graph and eager: 1 row of 4096 x 4096 6.3 -> 6.5 and 8.5 -> 6.7, 4 rows of 1024 x 4096 5.3 -> 5.0 and 8.4 ->
+// 5.5, 8 rows of 2048 x 2048 4.9 -> 5.0 and 8.7 -> 5.4.  Where it stops paying: quantize_inside_pays.
 constexpr int kQuantWarps = kStreamWarps - 2;           // all but the weight loads' and the MMAs'
 constexpr int kQuantThreads = kQuantWarps * 32;
 constexpr int kQuantAhead = 8;                          // groups of 8 a thread asks for at once
 // Chunks of 16 that a thread asks for at once where it casts: behind a weight stream a round trip to L2 takes 2 to 3 us.
 template <typename T, bool GIVEN> constexpr int kChunksAhead = !GIVEN ? 1 : (sizeof(T) == 2 ? 4 : 2);
+
+// Where a weight is sliced, the slices of a tile are whole x between them: every CTA finds the maximum of its own slice, which it
+// keeps in registers for the cast if it is not too long, and the CTAs of the tile exchange four bytes each (see ClusterAmax):
+// a quarter of the reads and one pass fewer for one trip inside the cluster.  8 rows of 4096 x 4096 eager 7.9 -> 7.1 us, in
+// a graph 8.1 -> 7.2; 16 rows 10.4 -> 8.2.  Where it is taken: own_slices_pay.
+struct SliceMax {
+  uint32_t bar, slots;     // shared-memory addresses: the barrier that counts the words, one word per slice
+  int split, krank, peer0; // slices of the tile, this one, the cluster rank of the first
+};
+template <typename T> constexpr int kHeldChunks = 8 / (int)sizeof(T);      // 32 registers
+
+// 16 codes where TMA would have put them: 16-byte chunk c of row m at c ^ (m & 7).
+template <typename T>
+__device__ __forceinline__ void emit_chunk(const uint4 (&raw)[sizeof(T)], const bq::qd::ScaleDiv& dv, uint8_t* dst) {
+  using namespace bq::qd;
+  constexpr int kWords = sizeof(T);
+  Pack8<T> lo, hi;
+#pragma unroll
+  for (int q = 0; q < kWords; ++q) reinterpret_cast<uint4*>(q < kWords / 2 ? &lo : &hi)[q % (kWords / 2)] = raw[q];
+  const uint2 a = codes8<T, true>(lo, dv), b = codes8<T, true>(hi, dv);
+  *reinterpret_cast<uint4*>(dst) = make_uint4(a.x, a.y, b.x, b.y);
+}
+
+template <typename T>
+__device__ __forceinline__ float quantize_own_slice(const QuantIn& in, int M, int K, int kx0, int kb_count, uint8_t* b_tiles,
+                                                    int b_tile_bytes, float* s_red, const SliceMax& sm, unsigned int* status) {
+  using namespace bq::qd;
+  constexpr int kWords = sizeof(T), kHeld = kHeldChunks<T>;
+  const int t = threadIdx.x - (kStreamThreads - kQuantThreads), lane = threadIdx.x & 31, warp = t >> 5;
+  const T* const x = static_cast<const T*>(in.x);
+  const int chunks = kb_count * (kBK / 16), total = M * chunks;     // of a row in this slice, of the slice
+  auto load = [&](int i, uint4 (&raw)[kWords]) {                     // K is a multiple of 16; beyond K: zeros
+    const int row = i / chunks, k = kx0 + (i - row * chunks) * 16;
+    const uint4* const src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * K + k);
+#pragma unroll
+    for (int q = 0; q < kWords; ++q) raw[q] = k < K ? __ldcg(src + q) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  auto largest = [&](const uint4 (&raw)[kWords], float m) {
+#pragma unroll
+    for (int q = 0; q < kWords; q += kWords / 2) m = absmax8(*reinterpret_cast<const Pack8<T>*>(&raw[q]), m);
+    return m;
+  };
+  auto at = [&](int i) {
+    const int row = i / chunks, c = i - row * chunks;
+    return b_tiles + (c >> 3) * b_tile_bytes + row * kBK + (((c & 7) ^ (row & 7)) << 4);
+  };
+  uint4 held[kHeld][kWords];
+  float m = 0.0f;
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u)
+    if (t + u * kQuantThreads < total) load(t + u * kQuantThreads, held[u]);
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u)
+    if (t + u * kQuantThreads < total) m = largest(held[u], m);
+  for (int i = t + kHeld * kQuantThreads; i < total; i += kQuantThreads) {
+    uint4 raw[kWords];
+    load(i, raw);
+    m = largest(raw, m);
+  }
+  uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));      // bit patterns order like the values, NaN on top
+  if (lane == 0) s_red[warp] = __uint_as_float(bits);
+  asm volatile("bar.sync 2, %0;" ::"n"(kQuantThreads) : "memory");
+  if (warp == 0) {
+    bits = __reduce_max_sync(0xffffffffu, lane < kQuantWarps ? __float_as_uint(s_red[lane]) : 0u);
+    if (lane < sm.split)
+      st_async_cluster(map_to_cta(sm.slots + 4u * sm.krank, sm.peer0 + lane), bits, map_to_cta(sm.bar, sm.peer0 + lane));
+  }
+  if (!mbar_wait_cluster(sm.bar, 0) && t == 0) atomicExch(status, (unsigned int)kErrDeviceWait);
+  bits = 0u;
+  if (lane < sm.split) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(bits) : "r"(sm.slots + 4u * lane) : "memory");
+  const float scale = scale_from_amax(__uint_as_float(__reduce_max_sync(0xffffffffu, bits)));
+  const ScaleDiv dv(scale);
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u)
+    if (t + u * kQuantThreads < total) emit_chunk<T>(held[u], dv, at(t + u * kQuantThreads));
+  for (int i = t + kHeld * kQuantThreads; i < total; i += kQuantThreads) {
+    uint4 raw[kWords];
+    load(i, raw);
+    emit_chunk<T>(raw, dv, at(i));
+  }
+  fence_proxy_async_smem();                             // the MMAs read through the async proxy
+  asm volatile("bar.sync 2, %0;" ::"n"(kQuantThreads) : "memory");
+  return scale;
+}
 
 // Returns the scale.  Called by warps 2.. with all lanes.  GIVEN: max |x| is in `in.words`.
 template <typename T, bool GIVEN>
@@ -618,7 +701,7 @@ __device__ __forceinline__ float quantize_slice(const QuantIn& in, int M, int K,
 #ifndef BQ_STREAM_MIN_CTAS
 #define BQ_STREAM_MIN_CTAS 2
 #endif
-template <int EPI, int DT, int QUANT>      // QUANT: 1 the activation's maximum is looked for, 2 it is given
+template <int EPI, int DT, int QUANT>      // QUANT: 1 the activation's maximum is looked for, 2 it is given, 3 each slice looks for its own
 __global__ void __launch_bounds__(kStreamThreads, BQ_STREAM_MIN_CTAS)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xd,
                    const __grid_constant__ WeightMaps tm_w, const __grid_constant__ GemmParams p,
@@ -646,6 +729,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       reinterpret_cast<volatile uint32_t*>(base_ptr + smem_tile_bytes + 8 * (n_bars + 1));
   volatile uint32_t* const abort_flag = tmem_slot + 1;
   float* const s_quant = reinterpret_cast<float*>(const_cast<uint32_t*>(tmem_slot) + 2);   // one float per warp
+  const uint32_t slice_bar = bar_base + 896u;       // QUANT: SliceMax, behind whatever the others need
   volatile float* const s_scale = reinterpret_cast<volatile float*>(base_ptr + smem_tile_bytes + kBarrierBytes - 8);
 
   if (threadIdx.x == 0) { BQ_STAMP(p, 0); BQ_STAMP_META(p, 0); }
@@ -690,8 +774,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     }
     for (int s = 0; s < p.b_stages; ++s) mbar_init(full_bar_b(s), 1);
     mbar_init(accum_bar, 1);
+    if (QUANT == 3) mbar_init(slice_bar, 1);
     *abort_flag = 0;
     fence_mbar_init();
+    if (QUANT == 3) mbar_expect_tx(slice_bar, 4u * split);
   }
   if (warp == 1 && active) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), tmem_cols);
@@ -706,10 +792,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) BQ_STAMP(p, 1);
 
-  // slices are written into a peer's memory: once it has started, which this says
-  if (p.handover) cluster_arrive_relaxed();
+  // slices (and maxima) are written into a peer's memory: once it has started, which this says
+  if (QUANT == 3 || p.handover) cluster_arrive_relaxed();
   if (!active) {
-    // nothing to multiply: it only matches the two cluster barriers of the working CTAs
+    // nothing to multiply: it only matches the cluster barriers of the working CTAs
+    if (QUANT == 3 && !p.handover) cluster_wait();
     if (p.handover) { cluster_wait(); cluster_sync_all(); }
     else if (p.cluster > 1) { cluster_sync_all(); cluster_sync_all(); }
     return;
@@ -753,7 +840,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       uint8_t* const tiles = base_ptr + (b_base - base);
       using T = typename std::conditional<DT == BQ_DTYPE_F32, float,
                                           typename std::conditional<DT == BQ_DTYPE_F16, __half, __nv_bfloat16>::type>::type;
-      const float sc = quantize_slice<T, QUANT == 2>(p.quant, p.M, p.quant_k, kx0, kb_count, tiles, b_tile_bytes, s_quant);
+      float sc;
+      if constexpr (QUANT == 3) {
+        cluster_wait();
+        sc = quantize_own_slice<T>(p.quant, p.M, p.quant_k, kx0, kb_count, tiles, b_tile_bytes, s_quant,
+                                   SliceMax{slice_bar, slice_bar + 8u, split, krank, group * split}, p.status);
+      } else {
+        sc = quantize_slice<T, QUANT == 2>(p.quant, p.M, p.quant_k, kx0, kb_count, tiles, b_tile_bytes, s_quant);
+      }
       if (threadIdx.x == kStreamThreads - kQuantThreads) {
         *s_scale = sc;
         mbar_arrive(full_bar_b(0));
@@ -848,7 +942,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   float* const slices = reinterpret_cast<float*>(base_ptr + smem_tile_bytes + kBarrierBytes);   // [split][per][128]
   const int per = (p.M + split - 1) / split;               // rows that a CTA sums
   const bool handover = p.handover && split > 1;
-  if (p.handover) cluster_wait();
+  if (QUANT == 3 ? warp < 2 : p.handover) cluster_wait();      // QUANT == 3: the others have waited
   if (ok && handover) {
     const int quad = warp & 3;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
@@ -1754,11 +1848,11 @@ const StreamKernel kStream[3][3] = {
     {gemm_stream_kernel<kGateUp, 0, 0>, gemm_stream_kernel<kGateUp, 1, 0>, gemm_stream_kernel<kGateUp, 2, 0>}};
 const StreamKernel kStreamGateUpDense[3] = {gemm_stream_kernel<kGateUpDense, 0, 0>, gemm_stream_kernel<kGateUpDense, 1, 0>,
                                            gemm_stream_kernel<kGateUpDense, 2, 0>};
-const StreamKernel kStreamQuant[2][2][3] = {     // [is the maximum given?]
-    {{gemm_stream_kernel<kPlain, 0, 1>, gemm_stream_kernel<kPlain, 1, 1>, gemm_stream_kernel<kPlain, 2, 1>},
-     {gemm_stream_kernel<kResidual, 0, 1>, gemm_stream_kernel<kResidual, 1, 1>, gemm_stream_kernel<kResidual, 2, 1>}},
-    {{gemm_stream_kernel<kPlain, 0, 2>, gemm_stream_kernel<kPlain, 1, 2>, gemm_stream_kernel<kPlain, 2, 2>},
-     {gemm_stream_kernel<kResidual, 0, 2>, gemm_stream_kernel<kResidual, 1, 2>, gemm_stream_kernel<kResidual, 2, 2>}}};
+#define BQ_QUANT_KERNELS(Q)                                                                                       \
+  {{gemm_stream_kernel<kPlain, 0, Q>, gemm_stream_kernel<kPlain, 1, Q>, gemm_stream_kernel<kPlain, 2, Q>},        \
+   {gemm_stream_kernel<kResidual, 0, Q>, gemm_stream_kernel<kResidual, 1, Q>, gemm_stream_kernel<kResidual, 2, Q>}}
+const StreamKernel kStreamQuant[3][2][3] = {BQ_QUANT_KERNELS(1), BQ_QUANT_KERNELS(2), BQ_QUANT_KERNELS(3)};
+#undef BQ_QUANT_KERNELS
 const StreamKernel kStreamArgmax[3] = {gemm_stream_kernel<kArgmax, 0, 0>, gemm_stream_kernel<kArgmax, 1, 0>,
                                       gemm_stream_kernel<kArgmax, 2, 0>};
 const StreamKernel kStreamAny = gemm_stream_kernel<kAny, kAnyType, 0>;
@@ -1816,7 +1910,7 @@ int configure_once() {
         if (kPair[e][d] != nullptr) set((const void*)kPair[e][d]);
         if (e == 3) continue;
         set((const void*)kStream[e][d]);
-        for (int g = 0; e < 2 && g < 2; ++g) set((const void*)kStreamQuant[g][e][d]);
+        for (int g = 0; e < 2 && g < 3; ++g) set((const void*)kStreamQuant[g][e][d]);
         set((const void*)WideKernels<1>::of[e][d]);
         set((const void*)WideKernels<2>::of[e][d]);
       }
@@ -1896,15 +1990,12 @@ int split_for_weight(long long n_rows, int k_blocks) {
 
 // Few rows: is the launch whose CTAs quantize the activation for themselves the faster form?  It saves a launch;
 // every CTA reads all of the activation and casts its K slice, and its weights wait for that.  So what counts is
-// the bytes a CTA reads plus those it casts.  us in a graph, one launch and two, at the bytes of the activation and the
-// K slices of the weight: 48 KB in 4 (6 rows of 4096 x 4096) 7.9 and 8.9, 64 KB in 4 (8 rows) 8.3 and 8.9; 40 KB in 2
-// (5 rows of 8192 x 4096) 9.8 and 10.8, 48 KB in 2 (6 rows) 10.5 and 10.9; 24 KB in 1 (6 rows of 12288 x 2048) 8.0
-// and 9.0, 32 KB in 1 (8 rows) 8.5 and 9.0, 48 KB in 1 (12 rows) 9.8 and 9.1, 64 KB in 1 10.9 and 9.3.  The line of a
-// captured call, 60 KB of both, dates from when one launch and two were equal there; they now are at 80 KB.
-// A weight of 64 CTAs or fewer reads less in all (8 rows of 2048 x 4096 6.5 and 7.7).  A call that is not captured pays
-// the host for its second launch as well: 64 KB in 4 8.4 and 10.7, 60 KB in 2 (6 rows of 8192 x 5120) 11.9 and 13.5,
-// 64 KB in 2 (8 rows of 6144 x 4096) 10.3 and 11.0; 40 KB in 1 (5 rows of 12288 x 4096) 12.7 and 13.7, 48 KB in 1 13.6
-// and 13.8, 64 KB in 1 (16 rows of 12288 x 2048) 11.0 and 10.7.
+// the bytes a CTA reads plus those it casts.  us of an eager call, one launch and two, at the bytes of the activation and
+// the K slices of the weight: 8 KB in 4 (1 row of 4096 x 4096) 6.7 and 8.5, 64 KB in 4 (8 rows) 7.4 and 8.4; 64 KB in 4 (8
+// rows of 1024 x 4096) 5.9 and 8.5; 32 KB in 1 (8 rows of 12288 x 2048) 8.4 and 8.6, 64 KB in 1 (16 rows) 10.7 and 8.5.  In a graph
+// the second launch costs no host, and since its quantizer exchanges inside a cluster it costs less on the device too:
+// 6.5 and 6.3, 7.2 and 6.6, 5.6 and 5.3, 8.2 and 7.0, 10.6 and 7.2.  The line of a captured call, 60 KB of both, is where
+// the two were equal before that; what it gives up below is 0 to 1.2 us, against one scratch slot and launch less.
 constexpr int64_t kInsideBytes = 65536, kInsideWork = 61440, kInsideWorkEager = 92160;
 
 bool quantize_inside_pays(int64_t M, int64_t K, int element_size, int n_seg, const int64_t* N, cudaStream_t stream) {
@@ -1940,6 +2031,16 @@ bool fetched_inside_pays(const GemmParams& p, int split, cudaStream_t stream) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) (void)cudaGetLastError();
   return status == cudaStreamCaptureStatusNone;
+}
+
+// Where every weight is sliced the CTAs may look at their own slices alone (quantize_own_slice) instead of at all of x.  us in a
+// graph, all of x and own slices, at the bytes of x and the slices: 8 KB in 4 (1 row of 1024 x 4096) 4.7 and 5.1, 32 KB in 4 (4
+// rows) 5.0 and 5.2, 48 KB in 4 6.1 and 5.6; 4096 x 4096 32 KB 6.8 and 6.7, 48 KB 7.9 and 7.1, 64 KB (8 rows) 8.1 and 7.2; 32
+// KB in 2 (4 rows of 8192 x 4096) 9.4 and 9.2, 48 KB in 2 10.1 and 9.5; 40 KB in 4 (4 rows of 2560 x 5120) 6.1 and 6.2,
+// 60 KB in 4 7.4 and 6.5; 80 KB in 2 (8 rows of 9728 x 5120) 15.4 and 13.8.
+constexpr int64_t kOwnSliceBytes = 32768;
+bool own_slices_pay(const GemmParams& p, int min_split) {
+  return min_split > 1 && (int64_t)p.M * p.quant_k * (p.out_dtype == BQ_DTYPE_F32 ? 4 : 2) > kOwnSliceBytes;
 }
 
 // Where the K slices of a tile are summed.  Up to 48 rows every CTA writes its share of a tile straight from its
@@ -2065,7 +2166,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   const int epi = epilogue_of(p, false);
   if (quant && epi != kPlain && epi != kResidual) return kErrUnsupported;
   const StreamKernel kernel =
-      quant ? kStreamQuant[p.quant.words != nullptr ? 1 : 0][epi][p.out_dtype]
+      quant ? kStreamQuant[p.quant.words != nullptr ? 1 : (own_slices_pay(p, min_split) ? 2 : 0)][epi][p.out_dtype]
             : (epi == kAny ? kStreamAny : epi == kArgmax ? kStreamArgmax[p.out_dtype] : (epi == kGateUpDense ? kStreamGateUpDense[p.out_dtype] : kStream[epi][p.out_dtype]));
   if (p.pair.on) p.pair.expected = (unsigned)((p.seg[0].n / kRowTile) * p.seg[0].split);
   if (p.push.n > 0)

@@ -662,6 +662,64 @@ def test_linear_of_few_rows_over_several_weights(Q):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("M,K,N,split", [(8, 2048, 4096, 0), (4, 4112, 4096, 0), (9, 2064, 8192, 0), (16, 2048, 5008, 2),
+                                         (16, 4096, 8192, 0), (15, 6160, 1024, 0), (13, 4096, 2048, 8)])
+def test_linear_whose_slices_look_at_their_own_columns(Q, dt, M, K, N, split):
+    """Above 32 KB and over sliced weights a CTA looks for the maximum of its own K slice and the slices exchange theirs:
+    the bits of quantizer and GEMM apart, on both sides of that line, K tails, 2, 4 and 8 slices, slices that fit the
+    registers and that do not (from 40 KB), the largest value and a NaN in any slice, a residual, a replay."""
+    fw = Q.quantize_weight(randn_cpu((N, K), seed=1, scale=0.02).cuda())
+    res = randn_cpu((M, N), seed=2, dtype=dt).cuda()
+    try:
+        Q.set_option("decode_quant_inside", 262144)
+        Q.set_option("decode_split_k", split)
+        for at in (0, K // 2 - 1, K - 1):
+            x = randn_cpu((M, K), seed=at, dtype=dt).cuda()
+            x[M - 1, at] = -40.0
+            xq, sx = Q.quantize_act(x)
+            n0 = Q.launch_count()
+            got = Q.linear(x, fw, residual=res)
+            assert Q._NATIVE is None or Q.launch_count() - n0 == (1 if x.nbytes <= 262144 else 2)
+            assert torch.equal(got, Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=res)), at
+            x[0, K - 1 - at] = float("nan")
+            assert torch.isnan(Q.linear(x, fw)).all(), at
+        graph, ins = torch.cuda.CUDAGraph(), randn_cpu((M, K), seed=5, dtype=dt).cuda()
+        with torch.cuda.graph(graph):
+            out = Q.linear(ins, fw)
+        for seed in (6, 7):
+            ins.copy_(randn_cpu((M, K), seed=seed, dtype=dt, scale=float(seed)))
+            graph.replay()
+            assert torch.equal(out, Q.fp8_matmul(*Q.quantize_act(ins), fw, out_dtype=dt))
+    finally:
+        Q.set_option("decode_quant_inside", -1)
+        Q.set_option("decode_split_k", 0)
+    assert Q.device_status() == 0
+
+
+def test_linear_whose_weights_have_unlike_slices(Q):
+    """Weights of 4, 2 and 4 K slices in one launch, and one that is not sliced beside them (no exchange then)."""
+    import ctypes
+    from braid_b200 import _lib
+    M, K = 8, 2560
+    x = randn_cpu((M, K), seed=1).cuda()
+    xq, sx = Q.quantize_act(x)
+    for Ns in ((4096, 8192, 272), (4096, 12288)):
+        ws = [Q.quantize_weight(randn_cpu((n, K), seed=n, scale=0.02).cuda()) for n in Ns]
+        ys = [torch.empty(M, n, device="cuda", dtype=x.dtype) for n in Ns]
+        ptrs = lambda ts: (ctypes.c_void_p * len(ts))(*[t.data_ptr() for t in ts])  # noqa: E731
+        n = (ctypes.c_int64 * len(Ns))(*Ns)
+        try:
+            Q.set_option("decode_quant_inside", 262144)
+            _lib.check(_lib.load().bq_linear_w8a8(x.data_ptr(), 1, M, K, len(Ns), ptrs([w.data for w in ws]),
+                                                  ptrs([w.scale for w in ws]), None, 0, ptrs(ys), n, n,
+                                                  Q._take_slot(x.device), 16, Q._stream_ptr(x.device)), "linear")
+        finally:
+            Q.set_option("decode_quant_inside", -1)
+        assert all(torch.equal(y, Q.fp8_matmul(xq, sx, w)) for y, w in zip(ys, ws))
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("M,K,N,eager,captured", [(6, 4096, 4096, 1, 1), (8, 4096, 4096, 1, 2), (8, 4096, 2048, 1, 1),
                                                   (5, 4096, 8192, 1, 1), (6, 4096, 8192, 1, 2), (6, 2048, 12288, 1, 1),
                                                   (8, 2048, 12288, 1, 2), (8, 4096, 6144, 2, 2), (16, 2048, 12288, 2, 2),
