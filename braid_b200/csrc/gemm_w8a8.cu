@@ -39,6 +39,7 @@
 #include "../../include/braid_b200.h"
 #include "ptx.cuh"
 #include "quant_device.cuh"
+#include "grid_amax.cuh"
 
 namespace {
 
@@ -1070,38 +1071,19 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   } else if (pair_on && EPI != kGateUpDense) {
     // ---- grid-wide max |h| -> scale -> codes of this CTA's rows (h is parked in `part`) ----
     using namespace bq::qd;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-      pair_max = nan_max(pair_max, __shfl_xor_sync(0xffffffffu, pair_max, off));
+    pair_max = bq::qd::warp_amax(pair_max);
     if (lane == 0) s_quant[warp] = pair_max;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float w = s_quant[0];
-#pragma unroll
-      for (int i = 1; i < kStreamWarps; ++i) w = nan_max(w, s_quant[i]);
-      unsigned int* const words = p.pair.words;
-      if (p.pair.expected > 1) {
+    if (warp == 0) {
+      float w = warp_amax(lane < kStreamWarps ? s_quant[lane] : 0.0f);
+      __syncwarp();
+      if (lane == 0) {
         // an aborted CTA still arrives (with 0), so the others are not left waiting
-        atomicMax(&words[0], __float_as_uint(w));
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&words[1]) : "memory");
-        unsigned int amax_bits = 0, arrived = 0;
-        const long long t0 = clock64();
-        for (;;) {
-          asm volatile("ld.acquire.gpu.global.v2.u32 {%0, %1}, [%2];"
-                       : "=r"(amax_bits), "=r"(arrived)
-                       : "l"(words)
-                       : "memory");
-          if (arrived >= p.pair.expected) break;
-          if (clock64() - t0 > kSpinLimitCycles) {
-            atomicExch(p.status, (unsigned int)kErrDeviceWait);
-            break;
-          }
-        }
-        w = __uint_as_float(amax_bits);
+        if (p.pair.expected > 1) w = exchange_max(w, p.pair.words, p.pair.expected, p.status);
+        const float sc = scale_from_amax(w);
+        if (blockIdx.x == 0) p.pair.sh[0] = sc;
+        s_quant[0] = sc;
       }
-      const float sc = scale_from_amax(w);
-      if (blockIdx.x == 0) p.pair.sh[0] = sc;
-      s_quant[0] = sc;
     }
     __syncthreads();
     if (EPI == kGateUp && warp == 0) prefetch_next(p.pair);
@@ -1117,14 +1099,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       else
         silu_pair_emit<float>(ea, part, sc, p.pair.hq, p.pair.ld_hq, col0);
     }
-    if (threadIdx.x == 0 && p.pair.expected > 1) {
-      unsigned int* const words = p.pair.words;
-      const unsigned int old = atomicAdd(&words[2], 1u);
-      if (old == p.pair.expected - 1) {
-        words[0] = 0u; words[1] = 0u; words[2] = 0u;
-        __threadfence();
-      }
-    }
+    if (threadIdx.x == 0 && p.pair.expected > 1) exchange_end(p.pair.words, p.pair.expected, exchange_leave(p.pair.words));
   }
   if (push != nullptr) {
     // The stores of all threads of this CTA are ordered before thread 0's fence by the barrier

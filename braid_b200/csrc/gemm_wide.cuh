@@ -306,45 +306,28 @@ __device__ __forceinline__ void pair_finish(const GemmParams& p, uint8_t* smem, 
     if (ok) pair_push(t, p.push, m0, col0, cols);
     return;      // the amax needs every rank's shard: the quantizer behind the exchange takes it
   }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = nan_max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  mx = warp_amax(mx);
   if (lane == 0) s_red[warp] = mx;
   __syncthreads();
-  unsigned int* const words = p.pair.words;
-  if (threadIdx.x == 0) {
-    float w = s_red[0];
-#pragma unroll
-    for (int i = 1; i < kWideWarps; ++i) w = nan_max(w, s_red[i]);
-    if (gridDim.x > 1) {
+  unsigned int ticket = 0u;
+  if (warp == 0) {
+    float w = warp_amax(lane < kWideWarps ? s_red[lane] : 0.0f);
+    __syncwarp();
+    if (lane == 0) {
       // an aborted CTA still arrives (with 0), so the others are not left waiting
-      atomicMax(&words[0], __float_as_uint(w));
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&words[1]) : "memory");
-      unsigned int amax_bits = 0, arrived = 0;
-      const long long t0 = clock64();
-      for (;;) {
-        asm volatile("ld.acquire.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(amax_bits), "=r"(arrived) : "l"(words) : "memory");
-        if (arrived >= gridDim.x) break;
-        if (clock64() - t0 > kSpinLimitCycles) {
-          atomicExch(p.status, (unsigned int)kErrDeviceWait);
-          break;
-        }
+      if (gridDim.x > 1) {
+        w = exchange_max(w, p.pair.words, gridDim.x, p.status);
+        ticket = exchange_leave(p.pair.words);
       }
-      w = __uint_as_float(amax_bits);
+      const float sc = scale_from_amax(w);
+      if (blockIdx.x == 0) p.pair.sh[0] = sc;
+      s_red[0] = sc;
     }
-    const float sc = scale_from_amax(w);
-    if (blockIdx.x == 0) p.pair.sh[0] = sc;
-    s_red[0] = sc;
   }
   __syncthreads();
   if (threadIdx.x == 0) BQ_STAMP(p, 5);
   if (ok) pair_emit(t, s_red[0], p.pair.hq, p.pair.ld_hq, m0, col0, cols);
-  if (threadIdx.x == 0 && gridDim.x > 1) {
-    const unsigned int old = atomicAdd(&words[2], 1u);
-    if (old == gridDim.x - 1) {
-      words[0] = 0u; words[1] = 0u; words[2] = 0u;
-      __threadfence();
-    }
-  }
+  if (threadIdx.x == 0 && gridDim.x > 1) exchange_end(p.pair.words, gridDim.x, ticket);
 }
 
 // ---- the kernel -----------------------------------------------------------------------------
@@ -647,7 +630,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     if (threadIdx.x == 0) BQ_STAMP(p, 6);
   }
   tc_fence_before();
-  cluster_sync_all();   // nobody frees tensor memory while the peer may still use the pair
+  // Nobody frees tensor memory while the peer may still use the pair.  That wants no order of the outputs' stores, for
+  // whose way to L2 (0.5 us) a releasing barrier waits; where a peer counts arrivals here, or the stores are counted, it does.
+  if (many || EPI == kAny) cluster_sync_all();
+  else { cluster_arrive_relaxed(); cluster_wait(); }
   if (EPI == kAny && p.push.n > 0 && threadIdx.x == 0) {
     // The stores of all threads of this CTA are ordered before thread 0's fence by the barrier
     // (fences are cumulative); the fence orders them before this CTA's count; the last CTA sees

@@ -18,10 +18,48 @@ struct QuantWs {
   unsigned int status;     // sticky: non-zero once a bounded wait ran out
 };
 
+// One thread of each of `expected` CTAs: publishes w (>= 0, or NaN with the sign cleared) and returns the largest of all,
+// once all have published theirs (bounded).  It owes exchange_leave() and exchange_end() afterwards.
+// words: [0] the maximum's bits [1] arrivals [2] departures.
+__device__ __forceinline__ float exchange_max(float w, unsigned int* words, unsigned int expected, unsigned int* status) {
+  // The unsigned order of the bit patterns is the order of the values, NaN on top.  The max is published first; the
+  // release on the counter orders it before the arrival.
+  atomicMax(&words[0], __float_as_uint(w));
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&words[1]) : "memory");
+  // amax word and arrival counter sit in one aligned 8-byte pair: one acquire load sees both
+  unsigned int amax_bits = 0, arrived = 0;
+  const long long t0 = clock64();
+  bool ok = true;
+  for (;;) {
+    asm volatile("ld.acquire.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(amax_bits), "=r"(arrived) : "l"(words) : "memory");
+    if (arrived >= expected) break;
+    if (clock64() - t0 > bq::kSpinLimitCycles) { ok = false; break; }
+  }
+  if (!ok) atomicExch(status, (unsigned int)bq::kErrDeviceWait);
+  return __uint_as_float(amax_bits);
+}
+// The place among those that check out.  Asked for before the codes are written and looked at behind them, so that a launch does
+// not end a trip to L2 (0.7 us) later: with the barrier at the end of gemm_wide_kernel, four graphed layers of 128 rows 304.5 ->
+// 297.8 us, 64 rows 273.0 -> 271.1; hidden 1024, 256 rows 180.6 -> 173.0.  The K-sliced gate/up launch asks behind its
+// codes: earlier 16 rows lose (217.0 -> 218.9), the warp that asks also prefetches.
+__device__ __forceinline__ unsigned int exchange_leave(unsigned int* words) { return atomicAdd(&words[2], 1u); }
+// True for the last one, which has returned the words to zero, so that the next launch (and a graph replay) starts
+// clean.
+__device__ __forceinline__ bool exchange_end(unsigned int* words, unsigned int expected, unsigned int ticket) {
+  if (ticket != expected - 1u) return false;
+  words[0] = 0u; words[1] = 0u; words[2] = 0u;
+  __threadfence();
+  return true;
+}
+
+// The largest of a warp's values, each >= 0 or NaN with the sign cleared.
+__device__ __forceinline__ float warp_amax(float m) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+}
+
 // CTA-wide max, then the grid-wide exchange.  Returns the global amax to every
 // thread.  A single-CTA grid never touches global memory here.  Thread 0 of every
-// CTA of a multi-CTA grid owes the scratch a grid_depart() call afterwards; that
-// part is kept off the critical path on purpose.
+// CTA of a multi-CTA grid owes the scratch a grid_depart() call afterwards.
 struct WholeCta {
   static constexpr bool live = true;
   __device__ int warp() const { return threadIdx.x >> 5; }
@@ -47,46 +85,23 @@ struct RehearsingCta {
 
 // `cta.live` = false: this warp's own max without the exchange.
 template <typename Cta = WholeCta>
-__device__ __forceinline__ float grid_amax(float m, QuantWs* ws, const Cta& cta = Cta{}) {
+__device__ __forceinline__ float grid_amax(float m, QuantWs* ws, unsigned int& ticket, const Cta& cta = Cta{}) {
   __shared__ float s_warp_of[2][32];
   __shared__ float s_amax_of[2];
   float* const s_warp = s_warp_of[cta.slot()];
   float& s_amax = s_amax_of[cta.slot()];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
+  m = warp_amax(m);
   const int lane = threadIdx.x & 31, warp = cta.warp();
   if (lane == 0) s_warp[warp] = m;
   cta.sync();
   if (warp == 0) {
-    const int nwarps = cta.warps();
-    float w = (lane < nwarps) ? s_warp[lane] : 0.0f;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) w = nan_max(w, __shfl_xor_sync(0xffffffffu, w, off));
+    float w = warp_amax(lane < cta.warps() ? s_warp[lane] : 0.0f);
     if (lane == 0) {
-      if (gridDim.x == 1 || !cta.live) {
-        s_amax = w;
-      } else {
-        // |x| >= 0 or NaN with the sign cleared: the unsigned order of the bit
-        // patterns is the order of the values, NaN on top.  The max is published
-        // first; the release on the counter orders it before the arrival.
-        atomicMax(&ws->amax_bits, __float_as_uint(w));
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ws->arrive) : "memory");
-        // amax word and arrival counter sit in one aligned 8-byte pair: one
-        // acquire load sees both
-        unsigned int amax_bits = 0, arrived = 0;
-        const long long t0 = clock64();
-        bool ok = true;
-        for (;;) {
-          asm volatile("ld.acquire.gpu.global.v2.u32 {%0, %1}, [%2];"
-                       : "=r"(amax_bits), "=r"(arrived)
-                       : "l"(ws)
-                       : "memory");
-          if (arrived >= gridDim.x) break;
-          if (clock64() - t0 > bq::kSpinLimitCycles) { ok = false; break; }
-        }
-        if (!ok) atomicExch(&ws->status, (unsigned int)bq::kErrDeviceWait);
-        s_amax = __uint_as_float(amax_bits);
+      if (gridDim.x > 1 && cta.live) {
+        w = exchange_max(w, &ws->amax_bits, gridDim.x, &ws->status);
+        ticket = exchange_leave(&ws->amax_bits);
       }
+      s_amax = w;
     }
   }
   cta.sync();
@@ -174,24 +189,12 @@ __device__ __forceinline__ void grid_wait_arrivals(const unsigned int* flag, con
   __syncthreads();
 }
 
-// Called by thread 0 of every CTA of a multi-CTA grid after it has the global
-// amax: the last CTA to check out returns the scratch to zero, so the next
-// launch (and a graph replay) starts clean.
-__device__ __forceinline__ void grid_depart(QuantWs* ws, unsigned int* wait_seen = nullptr,
+// Called by all threads when grid_amax is behind them, with the ticket it gave.
+__device__ __forceinline__ void grid_depart(QuantWs* ws, unsigned int ticket, unsigned int* wait_seen = nullptr,
                                             unsigned int wait_count = 0u) {
   if (threadIdx.x != 0) return;
-  if (gridDim.x == 1) {
-    if (wait_seen != nullptr) *wait_seen += wait_count;
-    return;
-  }
-  const unsigned int old = atomicAdd(&ws->depart, 1u);
-  if (old == gridDim.x - 1) {
-    if (wait_seen != nullptr) *wait_seen += wait_count;   // every CTA has read the old value
-    ws->amax_bits = 0u;
-    ws->arrive = 0u;
-    ws->depart = 0u;
-    __threadfence();
-  }
+  // the last one to leave: every CTA has read the old value
+  if ((gridDim.x == 1 || exchange_end(&ws->amax_bits, gridDim.x, ticket)) && wait_seen != nullptr) *wait_seen += wait_count;
 }
 
 // Host side: CTAs of a kernel that an SM of the current device holds at once, 0 where CUDA cannot say.  The

@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(with_rehearsal(R * G * kNormThreads)) rmsnorm_
   }
   if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
   float amax;
+  unsigned int ticket = 0u;
   if constexpr (CLUSTER) amax = cluster_amax(m, s_cluster, static_cast<QuantWs*>(p.ws), cta);
-  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws), cta);
+  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws), ticket, cta);
   const float sc = scale_from_amax(amax);
   if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
   const ScaleDiv dv(sc);
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(with_rehearsal(R * G * kNormThreads)) rmsnorm_
     const int v = vec(i);
     if (v < n_vec) emit4(x[i], dv, qr + v * kVec, row_ok);
   }
-  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws));
+  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws), ticket);
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
@@ -337,7 +338,8 @@ __global__ void __launch_bounds__(kRowGroups * kNormThreads) rmsnorm_rows_quant_
       }
     }
   }
-  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
+  unsigned int ticket = 0u;
+  const float sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), ticket));
   const ScaleDiv dv(sc);
   if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
 #pragma unroll
@@ -349,7 +351,7 @@ __global__ void __launch_bounds__(kRowGroups * kNormThreads) rmsnorm_rows_quant_
       if (v < n_vec) emit4(x[k][i], dv, qr + v * kVec, row0 + k < p.rows);
     }
   }
-  grid_depart(static_cast<QuantWs*>(p.ws));
+  grid_depart(static_cast<QuantWs*>(p.ws), ticket);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -645,8 +647,9 @@ __global__ void __launch_bounds__(with_rehearsal(WARPS * 32)) gated_rmsnorm_quan
   }
   if (live && threadIdx.x == 0) BQ_STAMP(p, 3);
   float amax;
+  unsigned int ticket = 0u;
   if constexpr (CLUSTER) amax = cluster_amax(m, s_cluster, static_cast<QuantWs*>(p.ws), cta);
-  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws), cta);
+  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws), ticket, cta);
   const float sc = scale_from_amax(amax);
   if (live && threadIdx.x == 0) BQ_STAMP(p, 4);
   const ScaleDiv dv(sc);
@@ -657,7 +660,7 @@ __global__ void __launch_bounds__(with_rehearsal(WARPS * 32)) gated_rmsnorm_quan
     const int head = warp + i * WARPS;
     if (head < cta_heads) emit4(core[i], dv, qr + head * kHeadDim + lane * kVec, live);
   }
-  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws));
+  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws), ticket);
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 

@@ -93,8 +93,9 @@ __global__ void __launch_bounds__(512, 1) quant_hold_kernel(const QParams p) {
     }
   }
   float amax;
+  unsigned int ticket = 0u;
   if constexpr (CLUSTER) amax = cluster_amax(m, s_cluster, static_cast<QuantWs*>(p.ws), WholeCta{});
-  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws));
+  else amax = grid_amax(m, static_cast<QuantWs*>(p.ws), ticket);
   const float sc = scale_from_amax(amax);
   const ScaleDiv dv(sc);
   if (threadIdx.x == 0) BQ_STAMP(p, 4);
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(512, 1) quant_hold_kernel(const QParams p) {
     for (unsigned int i = 0; i < p.tail; ++i)
       dst[i] = __nv_cvt_float_to_fp8(quant_one(tail_v[i], dv), __NV_SATFINITE, __NV_E4M3);
   }
-  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws), p.wait_flag != nullptr ? p.wait_seen : nullptr, p.wait_count);
+  if constexpr (!CLUSTER) grid_depart(static_cast<QuantWs*>(p.ws), ticket, p.wait_flag != nullptr ? p.wait_seen : nullptr, p.wait_count);
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
     grid_wait_arrivals(p.wait_flag, p.wait_seen, p.wait_count, static_cast<QuantWs*>(p.ws));
   const bool owns_tail = (MODE == kPlain) && p.tail != 0 && tid == nthreads - 1;
   float sc;
+  unsigned int ticket = 0u;
   if constexpr (PHASE == kCastOnly) {
     sc = __ldcg(p.scale);
   } else {
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       for (unsigned int i = 0; i < p.tail; ++i)
         m = nan_max(m, fabsf(widen(__ldcg(src + i))));
     }
-    sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
+    sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), ticket));
     if (tid == 0) p.scale[0] = sc;
   }
   if constexpr (PHASE != kScaleOnly) {
@@ -204,7 +206,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
     }
   }
   if constexpr (PHASE != kCastOnly)
-    grid_depart(static_cast<QuantWs*>(p.ws), p.wait_flag != nullptr ? p.wait_seen : nullptr, p.wait_count);
+    grid_depart(static_cast<QuantWs*>(p.ws), ticket, p.wait_flag != nullptr ? p.wait_seen : nullptr, p.wait_count);
 }
 
 // Sticky status of the launches that run without scratch words from the caller (the cast half alone,
@@ -310,6 +312,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
   constexpr int kPerUnit = 16 / (int)sizeof(T);   // elements (and code bytes) per 16 bytes of input
 
   float sc = 1.0f;
+  unsigned int ticket = 0u;
   // ---- forward pass: |x| max (kBoth, kScaleOnly, kMaxOnly) or the cast itself ----
   if constexpr (PHASE == kCastOnly) sc = __ldcg(p.scale);
   if constexpr (PHASE == kWeightCast) {
@@ -383,7 +386,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
       if (owns_tail)
         for (unsigned int i = 0; i < p.tail; ++i) m = nan_max(m, fabsf(widen(__ldcg(tail_src + i))));
       if (threadIdx.x == 0) BQ_STAMP(p, 3);
-      sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws)));
+      sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), ticket));
       if (threadIdx.x == 0) BQ_STAMP(p, 4);
       if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
     }
@@ -452,7 +455,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
     }
     __syncthreads();
   }
-  if constexpr (PHASE == kBoth || PHASE == kScaleOnly) grid_depart(static_cast<QuantWs*>(p.ws));
+  if constexpr (PHASE == kBoth || PHASE == kScaleOnly) grid_depart(static_cast<QuantWs*>(p.ws), ticket);
   if (threadIdx.x == 0) BQ_STAMP(p, 7);
 }
 
