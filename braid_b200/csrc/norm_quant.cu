@@ -257,25 +257,27 @@ __global__ void __launch_bounds__(with_rehearsal(R * G * kNormThreads)) rmsnorm_
 // plain RMSNorm -> quantize of a short prompt: CTAs of four groups of 128 threads, R rows per group.  A row's
 // arithmetic is that of rmsnorm_quant_kernel.  Gamma is in shared memory, not in registers, so that more rows are
 // resident at once, and a quarter or an eighth of the CTAs meet in the exchange (three atomics each on one word pair).
-// Narrow rows gain by the exchange, one launch before and now, us: 1500 x 64 bf16 10.9 -> 5.8, 1500 x 1024 12.1 -> 7.2,
-// 1300 x 2048 11.4 -> 7.8, 1036 x 4096 11.8 -> 10.8.  Wider ones gain the second launch: one CTA per row ends at 1036 rows
-// of 4096 columns (16-bit; fp32 740), beyond were a looped norm and a cast pass: 1500 x 4096 bf16 14.4 -> 11.9, 2368 x
-// 4096 18.5 -> 13.9, 1036 x 4096 fp32 13.9 -> 8.9, 1184 x 8192 bf16 18.9 -> 13.5.
+// What bounds it are the rows' loads in flight, so the registers decide: held to 40 for a third CTA per SM, the compiler asks
+// for a row's vectors one after the other.  That form (PER_SM = 3) is taken where two CTAs per SM do not hold the rows.
+// One CTA per row / 40 registers / 64, us: 16-bit 512 x 4096 7.5 / 9.2 / 7.0, 768 x 4096 8.9 / 10.8 / 7.4, 1036 x 4096 - / 10.3 /
+// 7.5, 1500 x 4096 - / 10.5 / - (two rows per group 11.7); 600 x 1024 5.8 / 4.9 / 4.5.
 // Resident on 148 SMs: 16-bit rows of up to 2048 columns 3552, up to 4096 columns 2368, up to 8192 columns 1184; fp32
-// 3552 (1024 columns), 2368 (2048), 1184 (4096), longer ones never.  Beyond, the two launches: 2600 x 4096 bf16 19.2,
-// 1300 x 5120 bf16 15.4, 1300 x 4096 fp32 15.9, 900 x 5120 fp32 15.9.
-// Of fewer rows a block has four to wait for where one would do: 500 x 4096 8.0 and 9.2, 700 x 4096 10.3 and 10.8 (700 x
-// 1024 6.9 and 5.7).
+// 3552 (1024 columns), 2368 (2048), 1184 (4096), longer ones never.  Beyond, the two launches: 2600 x 4096 bf16 12.7,
+// 1300 x 5120 bf16 10, 1300 x 4096 fp32 12.5.
+// Of few rows a block has four to wait for where one would do.  One CTA per row and this, us: 16-bit 257 x 2048 4.8 and
+// 4.7, 333 x 4096 6.3 and 6.4, 413 x 4096 6.8 and 6.6, fp32 333 x 4096 6.3 and 6.3, 413 x 4096 6.7 and 6.6; bf16
+// 257 x 8192 8.5 and 8.7, 600 x 8192 9.8 and 11.1, 900 x 8192 12.3 and 11.5.
 // ---------------------------------------------------------------------------------------------
 constexpr int kRowGroups = 4;
-constexpr int kGroupedRows = 768;     // more rows than these
-// The forms that hold more rows than the one before them.  A thread has VPT * sizeof(T) registers of a row: two rows of
+// more rows than these, for rows of up to 2048, 4096 and 8192 columns
+constexpr int grouped_rows(int per_thread) { return per_thread <= 4 ? 256 : per_thread <= 8 ? 384 : 768; }
+// The forms that hold more rows than the one before them (of R = 1, PER_SM 2 and then 3).  A thread has VPT * sizeof(T) registers of a row: two rows of
 // 32 make 80 registers and one CTA of eight rows per SM, no more than two CTAs of four; one row of 64 makes one CTA of
 // four, 592 rows in all.
 template <typename T, int VPT> constexpr bool kOneRowPerGroup = VPT * sizeof(T) <= 32;
 template <typename T, int VPT> constexpr bool kTwoRowsPerGroup = VPT * sizeof(T) <= 16;
-template <typename T, int VPT, int R>
-__global__ void __launch_bounds__(kRowGroups * kNormThreads) rmsnorm_rows_quant_kernel(const NormParams p) {
+template <typename T, int VPT, int R, int PER_SM>
+__global__ void __launch_bounds__(kRowGroups * kNormThreads, PER_SM) rmsnorm_rows_quant_kernel(const NormParams p) {
   bq::pdl_launch_dependents();
   __shared__ float s_red[kRowGroups][R][4];
   extern __shared__ float4 s_gamma[];
@@ -751,13 +753,14 @@ int launch_gated_cluster(GatedParams p, cudaStream_t stream) {
   return bq::kErrTooLarge;
 }
 
-// The fewest rows per CTA whose grid is resident at once; kErrTooLarge if none is.
-template <typename T, int VPT, int R>
+// kErrTooLarge where the grid is not resident at once.  launch_row_groups: the most registers and the fewest rows per CTA
+// whose grid is.
+template <typename T, int VPT, int R, int PER_SM>
 int launch_row_groups_of(const NormParams& p, cudaStream_t stream) {
   int dev = 0, sms = 0;
   const size_t smem = static_cast<size_t>(p.cols) * sizeof(float);     // gamma
   const int threads = kRowGroups * kNormThreads;
-  const int per_sm = resident_per_sm(rmsnorm_rows_quant_kernel<T, VPT, R>, threads, smem);
+  const int per_sm = resident_per_sm(rmsnorm_rows_quant_kernel<T, VPT, R, PER_SM>, threads, smem);
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1) {
     (void)cudaGetLastError();
@@ -775,7 +778,7 @@ int launch_row_groups_of(const NormParams& p, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, rmsnorm_rows_quant_kernel<T, VPT, R>, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, rmsnorm_rows_quant_kernel<T, VPT, R, PER_SM>, p);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
   return bq::kOk;
 }
@@ -783,9 +786,10 @@ template <typename T, int VPT>
 int launch_row_groups(const NormParams& p, cudaStream_t stream) {
   if (static_cast<size_t>(p.cols) * sizeof(float) > 40 * 1024) return bq::kErrTooLarge;
   int rc = bq::kErrTooLarge;
-  if constexpr (kOneRowPerGroup<T, VPT>) rc = launch_row_groups_of<T, VPT, 1>(p, stream);
+  if constexpr (kOneRowPerGroup<T, VPT>) rc = launch_row_groups_of<T, VPT, 1, 2>(p, stream);
   if constexpr (kTwoRowsPerGroup<T, VPT>) {
-    if (rc == bq::kErrTooLarge) rc = launch_row_groups_of<T, VPT, 2>(p, stream);
+    if (rc == bq::kErrTooLarge) rc = launch_row_groups_of<T, VPT, 1, 3>(p, stream);
+    if (rc == bq::kErrTooLarge) rc = launch_row_groups_of<T, VPT, 2, VPT * sizeof(T) <= 8 ? 3 : 2>(p, stream);
   }
   return rc;
 }
@@ -810,7 +814,7 @@ int launch_rmsnorm(const NormParams& p, cudaStream_t stream) {
     if (per_thread <= 16) return launch_rows(rmsnorm_quant_kernel<T, 16, 4, 1, false>, p.rows, 4 * kNormThreads, p, stream);
   }
   int rc = bq::kErrTooLarge;
-  if (p.rows <= kGroupedRows) {}
+  if (p.rows <= grouped_rows(per_thread)) {}
   else if (per_thread <= 2) rc = launch_row_groups<T, 2>(p, stream);
   else if (per_thread <= 4) rc = launch_row_groups<T, 4>(p, stream);
   else if (per_thread <= 8) rc = launch_row_groups<T, 8>(p, stream);

@@ -74,6 +74,26 @@ def test_rms_norm_quant_with_several_rows_per_block(Q, dt, rows, cols):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.float32], ids=["fp16", "fp32"])
+@pytest.mark.parametrize("rows,cols", [(256, 2048), (257, 2048), (259, 64), (384, 4096), (385, 4096), (387, 2052), (511, 1028)])
+def test_rms_norm_quant_from_where_rows_share_a_block(Q, dt, rows, cols):
+    """Rows of up to 2048 columns share a block from 257 rows on, of up to 4096 from 385: either side of both lines, rows
+    left over in the last block, vectors that end inside a thread's share, strided rows, with and without the dense output."""
+    x = randn_cpu((rows, 2 * cols), seed=rows, dtype=dt, scale=2.0).cuda()[:, cols:]
+    gamma = _gamma(cols, 9)
+    ref = TS.rms_norm(x, gamma, EPS)
+    for keep in (True, False):
+        n0 = Q.launch_count()
+        qa = Q.rms_norm_quant(x, gamma, EPS, keep_dense=keep)
+        assert Q.launch_count() - n0 == 1
+        if keep:
+            assert int((u8(qa.dense) != u8(ref)).sum()) == 0
+        _same(qa, ref, f"{rows} x {cols}")
+    x[-1, 0] = float("nan")
+    assert Q.rms_norm_quant(x, gamma, EPS).scale.isnan().all()
+    assert Q.device_status() == 0
+
+
 def test_rms_norm_quant_many_rows_of_real_width(Q):
     """2048 independent rows x 3 magnitudes: a reduction-order mismatch shows up as a last-bit
     difference in a few percent of rows, so this is the statistical net under the exact cases."""
