@@ -211,11 +211,6 @@ inline int resident_per_sm(Kernel kernel, int threads, size_t dynamic_smem) {
   for (const Known& k : known)
     if (k.kernel == key && k.dev == dev && k.threads == threads && k.smem == dynamic_smem) return k.per_sm;
   int per_sm = 0;
-  if (dynamic_smem > 48 * 1024 &&           // what a kernel gets without asking; each has one size beyond it at most
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic_smem) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return 0;
-  }
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dynamic_smem) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;

@@ -667,14 +667,6 @@ __global__ void __launch_bounds__(with_rehearsal(WARPS * 32)) gated_rmsnorm_quan
 }
 
 // ---------------------------------------------------------------------------------------------
-// From 33 rows to one per SM, a CTA asks for more than half of an SM's shared memory, so that it gets one to itself: they come
-// in while the CTAs of a GEMM leave, several to the SM that is free first, and share its schedulers in a chain that all
-// others wait for.  Four graphed layers, without and with, us: hidden 4096, 56 rows 268.5 -> 268.0, 72 rows 281.5 -> 278.3, 128
-// rows 298.3 -> 296.5, 144 rows 334.8 -> 327.7; hidden 2048 183 -> 178 (72), 192 -> 188 (128); hidden 5120 367 -> 362 (72);
-// it loses at 128 rows of hidden 2560, 216.1 -> 217.2.  Of two and more per SM it loses too: an
-// eager layer of 257 rows 137.7 -> 139.1, 1000 rows 233 -> 240.
-constexpr int kAloneRows = 32;
-constexpr size_t kAloneBytes = 116 * 1024;
 template <typename Kernel, typename Params>
 int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t stream) {
 #ifdef BQ_PHASES
@@ -683,17 +675,14 @@ int launch_rows(Kernel kernel, int rows, int threads, Params p, cudaStream_t str
   if (rows <= kRehearseRows) threads += 32;   // the rehearsing warp
   // every CTA waits for every other: the whole grid must fit on the device at once
   int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+  const int per_sm = resident_per_sm(kernel, threads, 0);
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1) {
     (void)cudaGetLastError();
     return bq::kErrLaunch;
   }
-  size_t smem = rows > kAloneRows && rows <= sms ? kAloneBytes : 0;
-  int per_sm = resident_per_sm(kernel, threads, smem);
-  if (per_sm < 1 && smem > 0) per_sm = resident_per_sm(kernel, threads, smem = 0);
-  if (per_sm < 1) return bq::kErrLaunch;
   if (static_cast<long long>(rows) > static_cast<long long>(sms) * per_sm) return bq::kErrTooLarge;
   cudaLaunchConfig_t cfg = {};
-  cfg.dynamicSmemBytes = smem;
   cfg.gridDim = dim3(static_cast<unsigned>(rows), 1, 1);
   cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
   cfg.stream = stream;

@@ -94,27 +94,6 @@ def test_rms_norm_quant_from_where_rows_share_a_block(Q, dt, rows, cols):
     assert Q.device_status() == 0
 
 
-@pytest.mark.parametrize("rows", [32, 33, 64, 65, 147, 148, 149])
-def test_norms_with_an_sm_to_each_row(Q, rows):
-    """From 33 rows to one per SM a block has an SM to itself: either side of both lines, rows of each width class, eager
-    and captured beside a GEMM."""
-    for cols, dt in ((4096, torch.bfloat16), (516, torch.float16), (8192, torch.float32), (6144, torch.float32)):
-        x = randn_cpu((rows, cols), seed=rows, dtype=dt, scale=2.0).cuda()
-        gamma = _gamma(cols, 11)
-        _same(Q.rms_norm_quant(x, gamma, EPS), TS.rms_norm(x, gamma, EPS), f"{rows} x {cols}")
-    fw = Q.quantize_weight(randn_cpu((4096, 4096), seed=3, scale=0.02).cuda())
-    x, gamma = randn_cpu((rows, 4096), seed=4).cuda(), _gamma(4096, 5)
-    step = lambda: Q.project(Q.rms_norm_quant(Q.project(Q.rms_norm_quant(x, gamma, EPS), fw)[0], gamma, EPS), fw)[0]  # noqa: E731
-    want = step()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
-        got = step()
-    for _ in range(3):
-        graph.replay()
-    assert torch.equal(got, want)
-    assert Q.device_status() == 0
-
-
 def test_rms_norm_quant_many_rows_of_real_width(Q):
     """2048 independent rows x 3 magnitudes: a reduction-order mismatch shows up as a last-bit
     difference in a few percent of rows, so this is the statistical net under the exact cases."""
