@@ -16,9 +16,9 @@
 // (gemm_w8a8.cu): a 64-row form of this one took 3.6 us instead of 2.5 from the activation's arrival
 // to the last MMA of a 4096 x 4096 weight; four graphed decoder layers were 4 % slower with it at
 // 1 row and 1 % at 27, and it was not kept.  At 128 rows those layers (hidden 4096, bf16) take 341 us
-// here and 376 on the K-sliced kernel.  Graphed norm + greedy pick with logits over a 248320 x 4096
-// vocabulary: 180 and 223 us at 64 rows, 273 and 742 at 256; eager calls add their host time (212 us at
-// 64 rows).
+// here and 376 on the K-sliced kernel (before both had kernels of their own per epilogue; 298 now).  Norm + greedy pick with logits
+// over a 248320 x 4096 vocabulary, eager and repeated: 200 to 203 us at 64 rows, 205 at 128, at the clock that the power
+// cap leaves.
 //
 // Sums.  Weights of few rows are summed in 2 or 4 K slices, each with an accumulator of its own,
 // added in order at the end: the order of summation is a function of the weight's shape alone and

@@ -4,7 +4,7 @@
 // An eager decode or prompt call launches kernels of 3 to 30 us; made from Python through ctypes a
 // launch costs about 18 us of host time (allocations with keyword arguments, stream lookup,
 // argument conversion), from here about 5.  A projection of 8 rows 36.3 -> 10.8 us (7.9 as one launch), the
-// MLP of one row 51 -> 38 (32 now), a decoder layer of 16 rows 162 -> 73 (64 now); the last two are their kernels' time.
+// MLP of one row 51 -> 38 (30 now), a decoder layer of 16 rows 162 -> 73 (55 now); the last two are their kernels' time.
 //
 // Each function here does what its namesake in quant.py does for the plain case -- ordinary CUDA tensors
 // of the current device, no dispatch mode, transform, forward-mode level or tracer, operands the kernels take

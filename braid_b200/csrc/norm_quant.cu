@@ -18,8 +18,8 @@
 // rounds once more.  tests/test_norm_quant_gpu.py pins all of this against torch on the device.
 //
 // After the norm the values stay in registers; amax, exchange and cast are the activation quantizer's (quant_act.cu).
-// The exchange of up to 64 rows stays inside one cluster; beyond it is grid-wide: a CTA holds one token row, or four or
-// eight (rmsnorm_rows_quant_kernel), and all of them are co-resident for it; larger inputs are refused, and the caller takes the norm with its rows
+// The exchange of up to 64 rows stays inside one cluster; beyond it is grid-wide: a CTA holds one token row, or from 257 rows on
+// four or eight (rmsnorm_rows_quant_kernel), and all of them are co-resident for it; larger inputs are refused, and the caller takes the norm with its rows
 // looped (bq_rmsnorm_scale, bq_gated_rmsnorm_scale) and the cast pass.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

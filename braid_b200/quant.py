@@ -686,8 +686,8 @@ def rms_norm_quant(x: torch.Tensor, gamma: torch.Tensor, eps: float,
                    keep_dense: bool = False) -> QuantizedActivation:
     """`quantize_act(rms_norm(x, gamma, eps))` in one launch (braid/model/layer.py:49,59 feeding
     `project` / the MLP).  Bit-identical to the two steps.  More rows than fit on the device at
-    once (prefill) take two launches: the norm with rows looped per CTA, which also leaves the
-    scale, and the cast; inputs with odd strides run the two torch-spelled steps."""
+    once (prefill) take two launches: the scale first, rows looped per CTA, then the codes, from the dense output where it
+    is kept and else from `x` read a second time; inputs with odd strides run the two torch-spelled steps."""
     if _NATIVE is not None:
         got = _NATIVE.rms_norm_quant(x, gamma, eps, keep_dense)
         if got is not None:
