@@ -2556,7 +2556,7 @@ int run_wide(GemmParams p, const void* xq, int64_t K, const void* const* wq, con
   return launch_wide(tm_x, tm_xd, maps, p, sh, stream);
 }
 
-// Tiles of a plain prefill launch: 256, 192 or 128 columns (the sums are the same, tile by tile; whole
+// Tiles of a plain prefill launch: 256, 192, 128 or 64 columns (the sums are the same, tile by tile; whole
 // 128-byte pieces of 16-bit output), and the last columns of its widest weight as 128-column tiles that
 // are visited last, where that evens out the last round.  A launch takes as long as its busiest CTA pair
 // (tiles are dealt out in turn), a tile its columns plus a part that does not shrink with them: the
@@ -2565,7 +2565,11 @@ int run_wide(GemmParams p, const void* xq, int64_t K, const void* const* wq, con
 // 66.4 / 60.2 / 62.8, at 3000 115.9 / 121.5 / 127.4: one round of n columns costs n + 128 within 6 % (128 columns alone,
 // with their deeper ring, n + 114).  Of 13 weights at 16 batches of 257 to 4000 rows, the choices timed in turn, the rule's is
 // more than 3 % behind the best at 7 of 208 (2560 x 7680 at 2600 rows 43.9 where 128 columns take 41.5, 15360 x 5120
-// at 1100 rows 78.8 with a split and 76.4 without; the others below 0.7 us).  64 columns never won by more than 2 %.  Split: q, k and v of 8192 + 1024 + 1024 columns at 1500 rows
+// at 1100 rows 78.8 with a split and 76.4 without; the others below 0.7 us).
+// 64 columns where half of the pairs hold such tiles: a K block's turn is shorter by more than its share of the round, us with 128
+// and with 64: 1024 x 4096 at 413 rows fp32 9.8 / 8.6, 16-bit 9.1 / 8.2, 1024 x 12288 18.3 / 16.5, 256 x 1024 at 2000
+// rows 5.6 / 5.1; at more tiles the gain goes, 48 tiles of 1024 x 4096 9.1 / 8.7, 64 tiles 9.3 / 9.0 (2048 x 1024 5.6 / 5.6).  Of K
+// below 8 blocks 512 x 512 at 512 rows takes 5.1 / 4.5; those stay at 128, as above.  Split: q, k and v of 8192 + 1024 + 1024 columns at 1500 rows
 // 58.0 -> 54.8, 2560 x 7680 at 4096 rows 76.8 -> 69.7 (both before the issue loops were walked by whole warps).
 struct TilePlan {
   int cols;            // columns of a tile
@@ -2611,6 +2615,7 @@ TilePlan plan_tiles(const int64_t* N, const int* dense, int n_seg, int m_tiles, 
     const long long cost = cost_of(tiles_of(n, 0), n, 0);
     if (best_cost == 0 || cost < best_cost) { best = TilePlan{n, -1, 0}; best_cost = cost; }
   }
+  if (k_blocks >= 8 && 2 * tiles_of(64, 0) <= pairs) return TilePlan{64, -1, 0};
   if (!may_split || n_seg == BQ_MAX_SEGMENTS || k_blocks < 8) return best;
   const int64_t columns = (N[widest] + kPairTile - 1) / kPairTile;
   for (int j = 1; j <= 6 && j < columns; ++j) {

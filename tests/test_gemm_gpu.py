@@ -207,6 +207,35 @@ def test_prefill_tiles_of_192_columns_give_the_bits_of_256(Q, M, N, K, dt):
 
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("M,N,K,cols", [(257, 16, 1024, 64), (413, 1024, 4096, 64), (512, 1152, 1024, 64), (2300, 208, 2064, 64),
+                                        (513, 784, 1040, 128), (512, 1200, 1024, 128), (300, 1024, 912, 64), (300, 1024, 896, 128)])
+def test_prefill_tiles_of_64_columns_give_the_bits_of_256(Q, M, N, K, cols, dt):
+    """Tiles of 64 columns while half of the pairs hold them: both sides of that line (37 of 74 pairs) and of eight K blocks,
+    tails in M, N and K, more K blocks than stages, residuals of either row stride, grouped."""
+    _, _, xq, sx, fw = _operands(Q, M, N, K, seed=M + N)
+    res = randn_cpu((M, N), seed=2, dtype=dt).cuda()
+    res_rows = randn_cpu((M, N + 4), seed=3, dtype=dt).cuda()[:, :N]
+
+    def run():
+        return [Q.fp8_matmul(xq, sx, fw, out_dtype=dt), Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=res),
+                Q.fp8_matmul(xq, sx, fw, out_dtype=dt, residual=res_rows), *Q.fp8_matmul_grouped(xq, sx, (fw, fw), out_dtype=dt)]
+
+    auto = Q.fp8_matmul(xq, sx, fw, out_dtype=dt)
+    assert Q.last_gemm_launch()["mma_n"] == cols
+    try:
+        Q.set_option("pair_narrow", 0)
+        want = run()
+        Q.set_option("pair_narrow", 64)
+        got = run()
+        assert Q.last_gemm_launch()["mma_n"] == 64
+    finally:
+        Q.set_option("pair_narrow", -1)
+    assert torch.equal(auto, want[0]) and all(torch.equal(a, b) for a, b in zip(got, want))
+    assert all(torch.equal(a, b) for a, b in zip(run(), want))
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
 @pytest.mark.parametrize("M,Ns", [(4864, (1024,)), (4860, (1040,)), (1500, (8192, 1024, 16))])
 def test_prefill_weights_whose_end_is_tiled_apart_give_the_bits_of_256(Q, dt, M, Ns):
     """Sizes whose last round is evened out with the end of the widest weight in 128-column tiles: outputs,
