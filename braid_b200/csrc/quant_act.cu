@@ -656,14 +656,16 @@ int launch_ring(const QParams& p, int sms, cudaStream_t stream) {
   const unsigned long long body = (unsigned long long)p.n_groups * kGroup * sizeof(T);
   const unsigned long long unit_chunk = (unsigned long long)kRingThreads * 16;
   const unsigned long long ctas = 2ull * sms;
-  const int units = body >= 3 * ctas * 4 * unit_chunk ? 4 : (body >= 3 * ctas * 2 * unit_chunk ? 2 : 1);
+  // the whole quantizer holds what would be chunks of one unit (launch_quant)
+  const int units = body >= 3 * ctas * 4 * unit_chunk ? 4 : (PHASE == kBoth || body >= 3 * ctas * 2 * unit_chunk ? 2 : 1);
   unsigned long long chunks = (body + units * unit_chunk - 1) / (units * unit_chunk);
   if (chunks < 1) chunks = 1;
   const int grid = (int)(chunks < ctas ? chunks : ctas);
   const int block = kRingThreads + 32;
   if (units == 4) return launch_with_pdl(quant_ring_kernel<T, PHASE, 4>, grid, block, p, stream, kRingSmem);
   if (units == 2) return launch_with_pdl(quant_ring_kernel<T, PHASE, 2>, grid, block, p, stream, kRingSmem);
-  return launch_with_pdl(quant_ring_kernel<T, PHASE, 1>, grid, block, p, stream, kRingSmem);
+  if constexpr (PHASE != kBoth) return launch_with_pdl(quant_ring_kernel<T, PHASE, 1>, grid, block, p, stream, kRingSmem);
+  return bq::kErrUnsupported;
 }
 
 constexpr int kWeightCtas = 1024;   // room for one maximum per CTA of the weight quantizer's first launch
@@ -679,9 +681,11 @@ template <typename T, int MODE>
 int launch_quant(QParams p, cudaStream_t stream) {
   const int sms = device_sms();
   if (sms <= 0) return bq::kErrLaunch;
-  // registers a thread may spend on held values: 8 groups of a 16-bit type in
-  // the plain mode; half of that when two operands are staged or T is fp32
-  constexpr int kMaxH = MODE == kPlain && sizeof(T) == 4 ? 4 : 8;
+  // Groups that a thread may hold, in 64 registers: 16 of a 16-bit type, 8 of fp32, and 8 of a prologue's product.  What is held
+  // is read once and waits for one exchange; the ring, which takes over, has its barriers besides.  us, ring and held: fp32
+  // 600 x 4096 8.2 and 6.5, 700 x 4096 8.9 and 6.6, 1000 x 4096 9.2 and 7.6, 1184 x 4096 (the last) 9.8 and 8.2; bf16
+  // 1300 x 4096 8.6 and 7.1, 413 x 12288 8.5 and 7.1, 700 x 12288 10.4 and 8.5, 2368 x 4096 (the last) 10.1 and 8.7.
+  constexpr int kMaxH = MODE == kPlain && sizeof(T) == 2 ? 16 : 8;
   const unsigned long long groups = p.n_groups;
   // One group per thread while that covers the input with 256-thread CTAs on
   // every SM; after that 512-thread CTAs, deepening each thread up to kMaxH;
@@ -717,8 +721,8 @@ int launch_quant(QParams p, cudaStream_t stream) {
     if (held <= 1) return launch_with_pdl(quant_hold_kernel<T, MODE, 1>, grid, block, p, stream);
     if (held <= 2 && kMaxH >= 2)
       return launch_with_pdl(quant_hold_kernel<T, MODE, (kMaxH >= 2 ? 2 : kMaxH)>, grid, block, p, stream);
-    if (held <= 4 && kMaxH >= 4)
-      return launch_with_pdl(quant_hold_kernel<T, MODE, (kMaxH >= 4 ? 4 : kMaxH)>, grid, block, p, stream);
+    if (held <= 4) return launch_with_pdl(quant_hold_kernel<T, MODE, 4>, grid, block, p, stream);
+    if (held <= 8 && kMaxH > 8) return launch_with_pdl(quant_hold_kernel<T, MODE, 8>, grid, block, p, stream);
     return launch_with_pdl(quant_hold_kernel<T, MODE, kMaxH>, grid, block, p, stream);
   }
   p.held = 0;

@@ -80,6 +80,23 @@ def test_ragged_sizes_through_the_shared_memory_ring(Q, dt, n):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+def test_values_held_up_to_64_registers(Q, dt):
+    """Every count of groups that a thread holds has its last size, one group more and a tail; beyond the last count the ring
+    takes over.  The largest value is the last one, and a NaN anywhere makes the scale NaN."""
+    per = torch.cuda.get_device_properties(0).multi_processor_count * 512 * 8
+    most = 8 if dt is torch.float32 else 16
+    for held in (4, most // 2, most - 1, most):
+        for n in (per * held, per * held + 8, per * held - 3):
+            x = randn_cpu((n,), seed=held, dtype=dt, scale=1.7).cuda()
+            x[-1] = 50.0
+            qr, sr = TS.quantize_act(x)
+            _assert_same(*Q.quantize_act(x), qr, sr, f"{dt} {held} {n}")
+    x[n // 2] = float("nan")
+    assert Q.quantize_act(x)[1].isnan().all()
+    assert Q.device_status() == 0
+
+
 @pytest.mark.parametrize("cols", [4096, 12288])
 def test_config_4_activations_on_the_streaming_kernel(Q, cols):
     """16 packed sequences (M ~ 8192 rows) of width 4096 (layer input) and
