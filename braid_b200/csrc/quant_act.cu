@@ -11,7 +11,7 @@
 // same scale bits.
 //
 // Shape of the kernel (HBM-bound, 3 bytes moved per bf16 element):
-//   * every thread pulls up to kMaxHeld groups of 8 elements with 128-bit loads
+//   * every thread pulls up to 16 groups of 8 elements with 128-bit loads
 //     and KEEPS them in registers;
 //   * |x| max: per thread -> warp shuffles -> shared memory -> one atomicMax per
 //     CTA on the bit pattern of the non-negative float (exact; NaN patterns sort
