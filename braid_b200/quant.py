@@ -1397,9 +1397,13 @@ def mlp_forward(x: torch.Tensor, gate_proj: FP8Weight, up_proj: FP8Weight,
     res2 = residual if residual is None or _is_rows(residual, down_proj.shape[0]) else residual.reshape(-1, down_proj.shape[0])
     if (_PAIR_MLP and _NATIVE is not None and isinstance(gate_proj, FP8Weight) and isinstance(up_proj, FP8Weight)
             and isinstance(down_proj, FP8Weight)):
+        weights = (gate_proj.data, gate_proj.scale, up_proj.data, up_proj.scale, down_proj.data, down_proj.scale)
         xq, sx = (pre.q, pre.scale) if pre is not None else (x2, None)
-        y = _NATIVE.mlp(xq, sx, x.dtype, gate_proj.data, gate_proj.scale, up_proj.data, up_proj.scale,
-                        down_proj.data, down_proj.scale, res2)
+        y = _NATIVE.mlp(xq, sx, x.dtype, *weights, res2)
+        if y is None and pre is None:
+            # its quantizer takes contiguous aligned rows that nothing records; its products take codes, whoever made them
+            pre = QuantizedActivation(*quantize_act(x2), x.shape, x.dtype)
+            y = _NATIVE.mlp(pre.q, pre.scale, x.dtype, *weights, res2)
         if type(y) is tuple:           # refused behind the quantizer: do not quantize twice
             pre = QuantizedActivation(y[0], y[1], x.shape, x.dtype)
         elif y is not None:

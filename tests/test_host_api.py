@@ -267,6 +267,31 @@ def test_scratch_is_published_after_the_native_calls_know_it(monkeypatch):
     assert found == [(3, buf.data_ptr(), False)] and quant._scratch == {3: buf}
 
 
+def test_mlp_whose_input_the_native_quantizer_refuses_takes_the_native_products(monkeypatch):
+    """A strided, misaligned or recorded input is quantized outside the native MLP call, which then takes the codes; one
+    that it takes as it is is not quantized outside."""
+    from braid_b200 import quant
+    calls, made = [], []
+
+    class Native:
+        def mlp(self, xq, sx, dtype, *rest):
+            calls.append((xq, sx))
+            return rest[-1] if sx is not None or xq.is_contiguous() else None
+
+    def quantize(x):
+        made.append(x)
+        return torch.zeros(x.shape).to(quant.FP8), torch.ones(1, 1)
+
+    monkeypatch.setattr(quant, "_NATIVE", Native())
+    monkeypatch.setattr(quant, "quantize_act", quantize)
+    w = quant.FP8Weight(torch.zeros(32, 32).to(quant.FP8), torch.ones(1, 1), (32, 32))
+    wide, out = torch.zeros(4, 64, dtype=torch.bfloat16), torch.zeros(4, 32, dtype=torch.bfloat16)
+    assert quant.mlp_forward(wide[:, :32], w, w, w, residual=out) is out
+    assert len(calls) == 2 and len(made) == 1 and calls[1][0].dtype is quant.FP8
+    assert quant.mlp_forward(wide[:, :32].contiguous(), w, w, w, residual=out) is out
+    assert len(calls) == 3 and len(made) == 1
+
+
 def test_cpu_tensors_are_refused_not_emulated():
     from braid_b200 import quant
     x = torch.zeros(4, 16, dtype=torch.bfloat16)
