@@ -254,7 +254,7 @@ inline bool cluster_fits(Kernel kernel, int threads, int n) {
 
 // Host side: launches a grid that is one cluster of `ctas` CTAs; kErrTooLarge where such a cluster cannot be scheduled.
 template <typename Kernel, typename Params>
-inline int launch_cluster(Kernel kernel, int ctas, int threads, cudaStream_t stream, Params p) {
+inline int launch_cluster(Kernel kernel, int ctas, int threads, cudaStream_t stream, Params p, bool pdl = true) {
   if (!cluster_fits(kernel, threads, ctas)) return bq::kErrTooLarge;
 #ifdef BQ_PHASES
   p.phase_ring = bq::phase_ring_for_launch(&p.phase_seq);
@@ -264,14 +264,14 @@ inline int launch_cluster(Kernel kernel, int ctas, int threads, cudaStream_t str
   cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(ctas);
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = pdl ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
   return bq::kOk;

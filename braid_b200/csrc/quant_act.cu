@@ -695,15 +695,17 @@ int launch_quant(QParams p, cudaStream_t stream) {
   // Decode batches: a grid that is one cluster (see cluster_amax), while a thread has one group or two.  The sigmoid product
   // of one attention layer in four, graphed layers of hidden 4096, us: 8 rows 221.3 -> 219.5, 16 rows 230.8 -> 228.6, 27 rows
   // 239.2 -> 238.3, 48 rows 262.6 -> 262.0; with four groups 64 rows 278.9 and 279.2.
-  if (g_cluster_exchange && p.wait_flag == nullptr) {
+  // An option that forces the launch's shape means the grid-wide one.
+  if (g_cluster_exchange && p.wait_flag == nullptr && g_opt_quant_block == 0 && g_opt_quant_held == 0) {
     const unsigned long long per_cta = (groups + kMaxCluster - 1) / kMaxCluster;
     const int threads = per_cta <= 256 ? 256 : 512;
     const int held = (int)((per_cta + threads - 1) / threads);
     const int grid = held > 0 ? (int)((groups + threads * held - 1) / (threads * held)) : 0;
-    if (grid > 1 && held <= (kMaxH < 2 ? 1 : 2)) {
+    if (grid > 1 && held <= 2) {
       p.held = held;
-      const int rc = held == 1 ? launch_cluster(quant_hold_kernel<T, MODE, 1, true>, grid, threads, stream, p)
-                               : launch_cluster(quant_hold_kernel<T, MODE, 2, true>, grid, threads, stream, p);
+      const bool pdl = g_opt_quant_pdl != 0;
+      const int rc = held == 1 ? launch_cluster(quant_hold_kernel<T, MODE, 1, true>, grid, threads, stream, p, pdl)
+                               : launch_cluster(quant_hold_kernel<T, MODE, 2, true>, grid, threads, stream, p, pdl);
       if (rc != bq::kErrTooLarge) return rc;
     }
   }
@@ -719,8 +721,7 @@ int launch_quant(QParams p, cudaStream_t stream) {
     // The smallest instantiation that holds `held` groups: fewer registers per
     // thread, so the next GEMM's CTAs fit on the SM beside a waiting quantizer CTA.
     if (held <= 1) return launch_with_pdl(quant_hold_kernel<T, MODE, 1>, grid, block, p, stream);
-    if (held <= 2 && kMaxH >= 2)
-      return launch_with_pdl(quant_hold_kernel<T, MODE, (kMaxH >= 2 ? 2 : kMaxH)>, grid, block, p, stream);
+    if (held <= 2) return launch_with_pdl(quant_hold_kernel<T, MODE, 2>, grid, block, p, stream);
     if (held <= 4) return launch_with_pdl(quant_hold_kernel<T, MODE, 4>, grid, block, p, stream);
     if (held <= 8 && kMaxH > 8) return launch_with_pdl(quant_hold_kernel<T, MODE, 8>, grid, block, p, stream);
     return launch_with_pdl(quant_hold_kernel<T, MODE, kMaxH>, grid, block, p, stream);

@@ -650,8 +650,10 @@ int bq_read_device_status(void* ws, void* stream, int* status_out);
  * bq_set_option("decode_quant_inside", v) few rows quantized inside the GEMM launch: -1 by size, 0 never, else up to
  *                                       so many bytes of activation (<= 262144; same results either way)
  * bq_set_option("stream_max_m", v)      largest M the weight-streaming kernel takes (<= 256)
- * bq_set_option("gemm_pdl" | "quant_pdl", 0/1)  programmatic dependent launch
- * bq_set_option("quant_block" | "quant_held", v) quantizer launch shape overrides
+ * bq_set_option("gemm_pdl" | "quant_pdl", 0/1)  programmatic dependent launch (of the GEMMs, of the quantizers)
+ * bq_set_option("quant_block" | "quant_held", v) quantizer launch shape overrides; 0 = by size
+ * bq_set_option("quant_cluster", 0/1)   norms and quantizers of decode batches as one cluster (default 1) or with the
+ *                                       grid-wide exchange, which a forced quantizer launch shape takes in any case
  * bq_set_option("quant_ring", 0/1)      plain quantizer at prefill sizes through the shared-memory ring (default 1)
  * bq_set_option("push_tma", 0/1)        prefill push epilogue by bulk tensor stores (default 1) or 16-byte plain stores
  * bq_set_option("pair_narrow", v)       prefill kernel: columns of a plain launch's tiles, -1 = by what evens out the

@@ -1,6 +1,8 @@
 """Helpers shared by the tests: bit views, seeded inputs, numpy bridges."""
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 
@@ -49,3 +51,35 @@ def config1_inputs(seed: int = 0):
 def max_rel(y: torch.Tensor, ref: torch.Tensor) -> float:
     y, ref = y.double(), ref.double()
     return float((y - ref).abs().max() / ref.abs().max().clamp_min(1e-300))
+
+
+def captured_kernels(fn):
+    """The kernels that `fn()` launches, captured and not run: per kernel its (mangled) name, CTAs, threads and CTAs per cluster; and how
+    many of the edges between them are programmatic."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1:] if len(result) > 2 else result[1]
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    handle = driver.CUgraph(graph.raw_cuda_graph())
+    nodes, _ = ok(driver.cuGraphGetNodes(handle, ok(driver.cuGraphGetNodes(handle))[1]))
+    found = []
+    for node in nodes:
+        if ok(driver.cuGraphNodeGetType(node)) != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        params = ok(driver.cuGraphKernelNodeGetParams(node))
+        name = ok(driver.cuFuncGetName(params.func)) if int(params.func) else ok(driver.cuKernelGetName(params.kern))
+        cluster = ok(driver.cuGraphKernelNodeGetAttribute(node, driver.CUlaunchAttributeID.CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION))
+        found.append({"name": name.decode(), "ctas": params.gridDimX * params.gridDimY, "threads": params.blockDimX,
+                      "cluster": cluster.clusterDim.x})
+    # cuda-python hands out edge data that it has freed
+    libcuda, n = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t(len(nodes) ** 2)
+    ends = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)()
+    data = (ctypes.c_uint8 * (8 * n.value))()         # from port, to port, type, five reserved
+    assert libcuda.cuGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), *ends, data, ctypes.byref(n)) == 0
+    programmatic = sum(data[8 * i + 2] == int(driver.CUgraphDependencyType.CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC) for i in range(n.value))
+    return found, programmatic

@@ -10,7 +10,7 @@ import torch.nn.functional as F
 
 import oracle
 from oracle import torch_spelling as TS
-from _util import codes_np, f32_bits, from_bits16, randn_cpu, to_np_f32, u8
+from _util import captured_kernels, codes_np, f32_bits, from_bits16, randn_cpu, to_np_f32, u8
 
 pytestmark = pytest.mark.gpu
 
@@ -564,4 +564,23 @@ def test_prologues_held_in_registers_up_to_the_two_launches(Q, dt, rows, cols, c
     view, o = qg[..., chunk:], up.contiguous()
     q, s = Q.sigmoid_gate_quant(o, view)
     _assert_same(q, s, *TS.quantize_act(TS.sigmoid_gate(o, view.reshape(rows, cols))), f"sigmoid {rows} x {cols} by {chunk}")
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("option,value,kernels", [
+    ("quant_cluster", 1, (16, 512, 16, 1)), ("quant_pdl", 0, (16, 512, 16, 0)), ("quant_cluster", 0, (32, 256, 0, 1)),
+    ("quant_block", 512, (16, 512, 0, 1)), ("quant_block", 256, (32, 256, 0, 1)), ("quant_held", 2, (16, 256, 0, 1))])
+def test_launch_options_hold_for_decode_batches(Q, option, value, kernels):
+    """A batch that would be one cluster takes the launch that the options ask for: its CTAs, threads, CTAs per cluster, and
+    whether the next launch may start early; the same codes."""
+    x = randn_cpu((16, 4096), seed=1).cuda()
+    qr, sr = TS.quantize_act(x)
+    default = {"quant_cluster": 1, "quant_pdl": 1}.get(option, 0)
+    try:
+        Q.set_option(option, value)
+        _assert_same(*Q.quantize_act(x), qr, sr)
+        found, programmatic = captured_kernels(lambda: (Q.quantize_act(x), Q.quantize_act(x)))
+    finally:
+        Q.set_option(option, default)
+    assert [(k["ctas"], k["threads"], k["cluster"], programmatic) for k in found] == [kernels] * 2
     assert Q.device_status() == 0
