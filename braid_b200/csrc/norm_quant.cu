@@ -531,23 +531,25 @@ __global__ void __launch_bounds__(kCastThreads) rmsnorm_cast_kernel(const NormPa
   const ScaleMul<T> dv(__ldcg(p.scale));
   if (!live) return;
   const T* const x = reinterpret_cast<const T*>(p.x) + group * kGroup;
-  for (int top = p.rows - 1 - blockIdx.y * kCastRows; top >= 0; top -= gridDim.y * kCastRows) {
-    Pack8<T> v[kCastRows];
-    float rstd[kCastRows];
+  by_scale(dv, [&](const auto& scale) {
+    for (int top = p.rows - 1 - blockIdx.y * kCastRows; top >= 0; top -= gridDim.y * kCastRows) {
+      Pack8<T> v[kCastRows];
+      float rstd[kCastRows];
 #pragma unroll
-    for (int k = 0; k < kCastRows; ++k)
-      if (top - k >= 0) {
-        v[k] = load8<T>(x + static_cast<long long>(top - k) * p.ld_x);
-        rstd[k] = __ldcg(p.rstd + top - k);
-      }
+      for (int k = 0; k < kCastRows; ++k)
+        if (top - k >= 0) {
+          v[k] = load8<T>(x + static_cast<long long>(top - k) * p.ld_x);
+          rstd[k] = __ldcg(p.rstd + top - k);
+        }
 #pragma unroll
-    for (int k = 0; k < kCastRows; ++k)
-      if (top - k >= 0) {
-        const int row = top - k;
-        scale_norm<T, kGroup>(v[k].v, g, rstd[k]);
-        emit8<T, true>(v[k], dv, p.q + static_cast<long long>(row) * p.cols + group * kGroup);
-      }
-  }
+      for (int k = 0; k < kCastRows; ++k)
+        if (top - k >= 0) {
+          const int row = top - k;
+          scale_norm<T, kGroup>(v[k].v, g, rstd[k]);
+          emit8<T, true>(v[k], scale, p.q + static_cast<long long>(row) * p.cols + group * kGroup);
+        }
+    }
+  });
 }
 
 // ---------------------------------------------------------------------------------------------

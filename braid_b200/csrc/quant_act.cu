@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
     if (tid == 0) p.scale[0] = sc;
   }
   if constexpr (PHASE != kScaleOnly) {
-    const ScaleMul<T> dv(sc);
+    const ScaleMul<T> dv(sc, p.n_groups > static_cast<unsigned long long>(nthreads) * kProofPays);
     // Every thread re-reads exactly the groups it read in pass 1 (the L2 keeps a line on
     // the side of the chip whose SM asked for it, so the same SM finds it again), last
     // iteration first: what pass 1 read last is the likeliest to be still there.
@@ -193,7 +193,8 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
         const long long g = g0 + (long long)u * nthreads;
         if (g < (long long)p.n_groups) {
           apply_prologue<T, MODE, true>(a[u], b[MODE == kPlain ? 0 : u]);
-          emit8<T, PHASE == kBoth>(a[u], dv, p.q + static_cast<size_t>(g) * kGroup);
+          // one loop for either: two of them spill (64 registers)
+          by_scale(dv, [&](const auto& scale) { emit8<T, PHASE == kBoth>(a[u], scale, p.q + static_cast<size_t>(g) * kGroup); });
         }
       }
     }
@@ -239,14 +240,14 @@ __device__ __forceinline__ float unit_absmax(const uint4& raw, float m) {
 }
 
 // codes of the 16 bytes `raw` holds: 8 for a 16-bit type, 4 for fp32
-template <typename T, bool OWN_SCALE>
-__device__ __forceinline__ void unit_emit(const uint4& raw, const ScaleMul<T>& dv, uint8_t* dst) {
+template <typename T, bool OWN_SCALE, typename Scale>
+__device__ __forceinline__ void unit_emit(const uint4& raw, const Scale& dv, uint8_t* dst) {
   if constexpr (sizeof(T) == 2) {
     emit8<T, OWN_SCALE>(*reinterpret_cast<const Pack8<T>*>(&raw), dv, dst);
   } else {
     float f[4] = {__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z),
                   __uint_as_float(raw.w)};
-    divide_group<T, 4, OWN_SCALE>(dv.div, f);
+    divide_group<T, 4, OWN_SCALE>(dv, f);
     const uint32_t a = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
     const uint32_t b = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
     *reinterpret_cast<uint32_t*>(dst) = (a & 0xFFFFu) | ((b & 0xFFFFu) << 16);
@@ -323,24 +324,11 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
     if (blockIdx.x == 0 && threadIdx.x == 0) p.scale[0] = sc;
   }
   {
-    const ScaleMul<T> dv(kCasts ? sc : 0.0f);      // a scale of 0: nothing to prepare
+    // the producer's copies need no scale, and are on their way while the consumers prepare theirs
+    const bool worth = kCasts && !producer && p.n_groups > static_cast<unsigned long long>(gridDim.x) * kRingThreads * kProofPays;
+    const ScaleMul<T> dv(kCasts ? sc : 0.0f, worth);
     float m = 0.0f;
-    if (producer) {
-      if (lane == 0) {
-        for (int k = 0; k < count; ++k) {
-          const int s = k % kRingStages;
-          if (k >= kRingStages &&
-              !bq::mbar_wait(bq::smem_u32(&bars[1][s]), (uint32_t)((k / kRingStages - 1) & 1))) {
-            fail();
-            break;
-          }
-          const uint32_t bytes = chunk_bytes(chunk_at(k));
-          bq::mbar_expect_tx(bq::smem_u32(&bars[0][s]), bytes);
-          bq::bulk_load_1d(bq::smem_u32(ring + s * kRingChunk), src + chunk_offset(chunk_at(k)), bytes,
-                           bq::smem_u32(&bars[0][s]), policy);
-        }
-      }
-    } else {
+    auto consume = [&](const auto& scale) {
       for (int k = 0; k < count; ++k) {
         const int s = k % kRingStages;
         if (!bq::mbar_wait(bq::smem_u32(&bars[0][s]), (uint32_t)((k / kRingStages) & 1))) {
@@ -359,7 +347,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
           const uint32_t unit = threadIdx.x + u * kRingThreads;
           if (unit * 16u < have) {
             if constexpr (kCasts) {
-              unit_emit<T, PHASE == kWeightCast>(raw[u], dv,
+              unit_emit<T, PHASE == kWeightCast>(raw[u], scale,
                                                  p.q + (chunk_offset(chunk_at(k)) / 16 + unit) * kPerUnit);
             } else {
               m = unit_absmax<T>(raw[u], m);
@@ -372,6 +360,26 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
           if (lane == 0) bq::mbar_arrive(bq::smem_u32(&bars[1][s]));
         }
       }
+    };
+    if (producer) {
+      if (lane == 0) {
+        for (int k = 0; k < count; ++k) {
+          const int s = k % kRingStages;
+          if (k >= kRingStages &&
+              !bq::mbar_wait(bq::smem_u32(&bars[1][s]), (uint32_t)((k / kRingStages - 1) & 1))) {
+            fail();
+            break;
+          }
+          const uint32_t bytes = chunk_bytes(chunk_at(k));
+          bq::mbar_expect_tx(bq::smem_u32(&bars[0][s]), bytes);
+          bq::bulk_load_1d(bq::smem_u32(ring + s * kRingChunk), src + chunk_offset(chunk_at(k)), bytes,
+                           bq::smem_u32(&bars[0][s]), policy);
+        }
+      }
+    } else if constexpr (kCasts) {
+      by_scale(dv, consume);
+    } else {
+      consume(0);
     }
     if constexpr (kCasts) {
       if (owns_tail) {
@@ -393,7 +401,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
   }
   // ---- backward pass of the whole quantizer: the ring's contents first, then re-fetches ----
   if constexpr (PHASE == kBoth) {
-    const ScaleMul<T> dv(sc);
+    const ScaleMul<T> dv(sc, !producer);
     const int refetch = count - kRingStages;   // chunks [0, refetch) are no longer in the ring
     if (producer) {
       if (lane == 0 && s_failed == 0u) {
@@ -408,30 +416,32 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2) quant_ring_kernel(const 
         }
       }
     } else if (s_failed == 0u) {
-      for (int k = count - 1; k >= 0; --k) {
-        const int s = k % kRingStages;
-        if (k < refetch) {
-          const uint32_t parity = (uint32_t)(((refetch - 1 - k) / kRingStages) & 1);
-          if (!bq::mbar_wait(bq::smem_u32(&bars[2][s]), parity)) { fail(); break; }
-        }
-        const uint32_t have = chunk_bytes(k);
-        uint4 raw[kRingUnits];
+      by_scale(dv, [&](const auto& scale) {
+        for (int k = count - 1; k >= 0; --k) {
+          const int s = k % kRingStages;
+          if (k < refetch) {
+            const uint32_t parity = (uint32_t)(((refetch - 1 - k) / kRingStages) & 1);
+            if (!bq::mbar_wait(bq::smem_u32(&bars[2][s]), parity)) { fail(); break; }
+          }
+          const uint32_t have = chunk_bytes(k);
+          uint4 raw[kRingUnits];
 #pragma unroll
-        for (int u = 0; u < kRingUnits; ++u) {
-          const uint32_t unit = threadIdx.x + u * kRingThreads;
-          if (unit * 16u < have) raw[u] = *reinterpret_cast<const uint4*>(ring + s * kRingChunk + unit * 16);
-        }
+          for (int u = 0; u < kRingUnits; ++u) {
+            const uint32_t unit = threadIdx.x + u * kRingThreads;
+            if (unit * 16u < have) raw[u] = *reinterpret_cast<const uint4*>(ring + s * kRingChunk + unit * 16);
+          }
 #pragma unroll
-        for (int u = 0; u < kRingUnits; ++u) {
-          const uint32_t unit = threadIdx.x + u * kRingThreads;
-          if (unit * 16u < have)
-            unit_emit<T, true>(raw[u], dv, p.q + (chunk_offset(k) / 16 + unit) * kPerUnit);
+          for (int u = 0; u < kRingUnits; ++u) {
+            const uint32_t unit = threadIdx.x + u * kRingThreads;
+            if (unit * 16u < have)
+              unit_emit<T, true>(raw[u], scale, p.q + (chunk_offset(k) / 16 + unit) * kPerUnit);
+          }
+          if (k >= kRingStages) {   // chunk k - kRingStages comes into this stage next
+            __syncwarp();
+            if (lane == 0) bq::mbar_arrive(bq::smem_u32(&bars[3][s]));
+          }
         }
-        if (k >= kRingStages) {   // chunk k - kRingStages comes into this stage next
-          __syncwarp();
-          if (lane == 0) bq::mbar_arrive(bq::smem_u32(&bars[3][s]));
-        }
-      }
+      });
     }
     if (owns_tail) {
       uint8_t* dst = p.q + static_cast<size_t>(p.n_groups) * kGroup;

@@ -238,18 +238,25 @@ __device__ __forceinline__ uint2 codes8(const Pack8<T>& v, const ScaleDiv& sc) {
 // infinity and in NaN both saturate alike).  Tried are the rounded reciprocal and its two neighbours: one of them
 // does for 99.99 % of all scales of bf16 values, 99.98 % of fp16's, and for 90 % of the scales that are max|x| / 448 of a value
 // of the type itself, where x = 3/4 max|x| may lie on a tie exactly.  The others take ScaleDiv's correction, 4 instructions
-// an element where this is half of one: a 12288 x 4096 weight 45.0 -> 41.3 us, cast of 9658 x 4096 bf16 22.9 -> 19.9, of
-// 9658 x 12288 64.0 -> 60.9 (5.8 TB/s).  For kernels that cast many groups a thread: the proof is a division and two
-// ballots per warp, which a CTA of one row per group pays for once and loses by (1500 x 4096 normed 11.6 -> 12.1).
+// an element where this is half of one.  us, quotients / one product, and a scale that takes the quotients: a 12288 x 4096
+// weight 43.2 / 38.4 / 44.2, cast of 9658 x 4096 bf16 21.9 / 17.5 / 21.5, of 9658 x 12288 62.3 / 57.9 / 61.5, 9658 x 4096 bf16
+// quantized 34.0 / 29.7 / 34.2.  Each has a loop of its own (by_scale): with the choice inside the loop those were 39.7 and
+// 44.9, 17.9 and 22.0, 58.9 and 62.1, 31.7 and 35.9.
+// For kernels that cast many groups a thread: the proof is a division and two ballots per warp, which a CTA of one row per
+// group pays for once and loses by (1500 x 4096 normed 11.6 -> 12.1), and so does a thread of one group: cast of 32768
+// values 1.8 -> 2.05, of 1.21 M (one each) 2.85 -> 3.1; 2.46 M (two) 3.6 -> 3.35, 3.16 M (2.6) 4.1 -> 3.6.
+constexpr int kProofPays = 2;      // more groups of 8 per thread
+template <typename T> struct OneProduct { float mul; };
+
 template <typename T>
 struct ScaleMul {
   ScaleDiv div;
   float mul;
   bool one;
-  // By whole warps.
-  __device__ __forceinline__ explicit ScaleMul(float s) : div(s), mul(0.0f), one(false) {
+  // By whole warps, of one mind about `worth`.
+  __device__ __forceinline__ explicit ScaleMul(float s, bool worth = true) : div(s), mul(0.0f), one(false) {
     if constexpr (sizeof(T) == 2) {
-      if (!div.fast) return;
+      if (!div.fast || !worth) return;
       constexpr int kBits = std::is_same<T, __half>::value ? 11 : 8;
       const unsigned int lane = threadIdx.x & 31u, n = 16u + (lane & 15u);
       const float tie = static_cast<float>(n) * 0.0625f;
@@ -283,14 +290,18 @@ __device__ __forceinline__ uint32_t codes4_mul(uint32_t lo, uint32_t hi, float m
 }
 
 template <typename T, bool OWN_SCALE = false>
-__device__ __forceinline__ uint2 codes8(const Pack8<T>& v, const ScaleMul<T>& sc) {
+__device__ __forceinline__ uint2 codes8(const Pack8<T>& v, const OneProduct<T>& sc) {
+  const uint4 w = *reinterpret_cast<const uint4*>(&v);
+  return make_uint2(codes4_mul<T>(w.x, w.y, sc.mul), codes4_mul<T>(w.z, w.w, sc.mul));
+}
+
+// f(scale) with what the codes are taken by.
+template <typename T, typename F>
+__device__ __forceinline__ void by_scale(const ScaleMul<T>& s, F&& f) {
   if constexpr (sizeof(T) == 2) {
-    if (sc.one) {
-      const uint4 w = *reinterpret_cast<const uint4*>(&v);
-      return make_uint2(codes4_mul<T>(w.x, w.y, sc.mul), codes4_mul<T>(w.z, w.w, sc.mul));
-    }
+    if (s.one) { f(OneProduct<T>{s.mul}); return; }
   }
-  return codes8<T, OWN_SCALE>(v, sc.div);
+  f(s.div);
 }
 
 template <typename T, bool OWN_SCALE = false, typename Scale>

@@ -529,21 +529,33 @@ def test_quantize_weight_can_be_traced_and_transformed(Q):
 def test_codes_by_one_product_under_the_scale_of_every_maximum(Q, dt):
     """The passes over large inputs take a code from ONE product where the scale allows it (`ScaleMul`); max |x| / 448 is the
     scale that lies closest to the ties, since 3/4 of the maximum may be one exactly.  Every mantissa a maximum can have, all
-    values of the type up to it, through the quantizer (ring kernel) and the cast alone, and under scales one and two units
-    away; against the torch spelling."""
+    values of the type up to it: the quantizer held in registers and as a ring (beyond what registers hold), the weight
+    quantizer, and the cast alone, with few groups per thread (quotients) and with many, under the maximum's own scale and
+    under scales one and two units away; against the torch spelling."""
     bits = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).cuda().view(dt)
     mant = 7 if dt is torch.bfloat16 else 10
     base = (127 << 7) if dt is torch.bfloat16 else (18 << 10)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    ring = sms * 512 * 16 * 8 // bits.numel() + 1         # copies that no longer fit the registers
+    many = bits.repeat(2 * 2 * sms * 512 * 8 // bits.numel() + 1)
     for m in range(0, 1 << mant, 1 if mant == 7 else 5):
         top = torch.tensor([base + m], dtype=torch.int16).cuda().view(dt)
-        x = torch.where((bits.float().abs() <= top.float()), bits, torch.zeros_like(bits)).repeat(32).contiguous()
+        x1 = torch.where((bits.float().abs() <= top.float()), bits, torch.zeros_like(bits))
+        x = x1.repeat(32).contiguous()
         q, s = Q.quantize_act(x)
         qr, sr = TS.quantize_act(x)
         _assert_same(q, s, qr, sr, f"{dt} maximum {top.item()}")
-        for ulps in (-2, -1, 1, 2):
+        want1 = u8(qr).reshape(-1)[:bits.numel()]
+        q, s = Q.quantize_act(x1.repeat(ring))
+        assert torch.equal(s, sr) and bool((u8(q).view(ring, -1) == want1).all()), f"{dt} ring, maximum {top.item()}"
+        w = Q.quantize_weight(x.view(-1, 1024))
+        _assert_same(w.data.reshape(-1), w.scale, qr, sr, f"{dt} weight, maximum {top.item()}")
+        for ulps in (-2, -1, 0, 1, 2):
             other = (sr.view(torch.int32) + ulps).view(torch.float32)
             want = (bits.float() / other).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
             assert torch.equal(u8(Q.cast_act(bits, other)).reshape(-1), u8(want).reshape(-1)), f"{dt} {top.item()} {ulps}"
+            got = u8(Q.cast_act(many, other)).view(-1, bits.numel())
+            assert bool((got == u8(want).reshape(-1)).all()), f"{dt} {top.item()} {ulps}, many groups per thread"
     assert Q.device_status() == 0
 
 
