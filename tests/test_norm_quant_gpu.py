@@ -457,3 +457,19 @@ def test_rms_norm_quant_that_reads_its_rows_twice(Q, dt, rows, cols):
     x[rows - 1, cols - 1] = float("nan")
     assert Q.rms_norm_quant(x, gamma, EPS).scale.isnan().all()
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("rows,cols", [(3553, 8), (9001, 16), (30001, 24), (7105, 88), (40007, 64), (20003, 344), (6001, 1024), (6001, 1032)])
+def test_narrow_rows_cast_next_to_one_another(Q, dt, rows, cols):
+    """Rows of up to 128 groups of 8 lie next to one another in a CTA of the second launch, as many as put all rows on the device
+    at once and at most what fits its 256 threads: counts that leave threads over, rows left over, one group per row, and the
+    widest such row and the first that is not."""
+    x = randn_cpu((rows, cols + 8), seed=rows, dtype=dt, scale=2.0).cuda()[:, :cols]
+    x[::7] *= 20.0
+    gamma = _gamma(cols, 9, spread=0.3)
+    n0 = Q.launch_count()
+    qa = Q.rms_norm_quant(x, gamma, EPS)
+    assert Q.launch_count() - n0 == 2
+    _same(qa, TS.rms_norm(x, gamma, EPS), f"{rows} x {cols}")
+    assert Q.device_status() == 0
