@@ -2008,14 +2008,15 @@ bool fetched_inside_pays(const GemmParams& p, int split, cudaStream_t stream) {
   return status == cudaStreamCaptureStatusNone;
 }
 
-// Where every weight is sliced the CTAs may look at their own slices alone (quantize_own_slice) instead of at all of x.  us in a
-// graph, all of x and own slices, at the bytes of x and the slices: 8 KB in 4 (1 row of 1024 x 4096) 4.7 and 5.1, 32 KB in 4 (4
-// rows) 5.0 and 5.2, 48 KB in 4 6.1 and 5.6; 4096 x 4096 32 KB 6.8 and 6.7, 48 KB 7.9 and 7.1, 64 KB (8 rows) 8.1 and 7.2; 32
-// KB in 2 (4 rows of 8192 x 4096) 9.4 and 9.2, 48 KB in 2 10.1 and 9.5; 40 KB in 4 (4 rows of 2560 x 5120) 6.1 and 6.2,
-// 60 KB in 4 7.4 and 6.5; 80 KB in 2 (8 rows of 9728 x 5120) 15.4 and 13.8.
-constexpr int64_t kOwnSliceBytes = 32768;
-bool own_slices_pay(const GemmParams& p, int min_split) {
-  return min_split > 1 && (int64_t)p.M * p.quant_k * (p.out_dtype == BQ_DTYPE_F32 ? 4 : 2) > kOwnSliceBytes;
+// Where every weight is sliced the CTAs may look at their own slices alone (quantize_own_slice) instead of at all of x.  In a
+// graph, the time with all of x over that with own slices, 13 weights of 512 to 10240 rows by 9 of 1024 to 12288 columns, by KB of x:
+// 16 bits, halves: 31 to 41 KB 0.98, to 46 KB 1.04, to 60 KB 1.05; quarters 1.00, 1.085, 1.10; where two CTAs share an SM 1.04 to
+// 1.06, 1.11 to 1.13, 1.14; fp32 1.09 to 1.14, 1.19 to 1.24, 1.15 to 1.24.  So the line lies at 32 KB, and for 16 bits with an SM
+// per CTA at 40 KB (between them 5 rows of 8192 x 4096 8.2 and 8.5 us, 2 rows of 5760 x 9728 10.2 and 11.0).
+constexpr int64_t kOwnSliceBytes = 32768, kOwnSliceBytes16 = 40960;
+bool own_slices_pay(const GemmParams& p, int min_split, int per_sm) {
+  const bool fp32 = p.out_dtype == BQ_DTYPE_F32;
+  return min_split > 1 && (int64_t)p.M * p.quant_k * (fp32 ? 4 : 2) > (fp32 || per_sm > 1 ? kOwnSliceBytes : kOwnSliceBytes16);
 }
 
 // Where the K slices of a tile are summed.  Up to 48 rows every CTA writes its share of a tile straight from its
@@ -2141,7 +2142,7 @@ int launch_stream(const CUtensorMap& tm_x, const CUtensorMap& tm_xd, const Weigh
   const int epi = epilogue_of(p, false);
   if (quant && epi != kPlain && epi != kResidual) return kErrUnsupported;
   const StreamKernel kernel =
-      quant ? kStreamQuant[p.quant.words != nullptr ? 1 : (own_slices_pay(p, min_split) ? 2 : 0)][epi][p.out_dtype]
+      quant ? kStreamQuant[p.quant.words != nullptr ? 1 : (own_slices_pay(p, min_split, per_sm) ? 2 : 0)][epi][p.out_dtype]
             : (epi == kAny ? kStreamAny : epi == kArgmax ? kStreamArgmax[p.out_dtype] : (epi == kGateUpDense ? kStreamGateUpDense[p.out_dtype] : kStream[epi][p.out_dtype]));
   if (p.pair.on) p.pair.expected = (unsigned)((p.seg[0].n / kRowTile) * p.seg[0].split);
   if (p.push.n > 0)

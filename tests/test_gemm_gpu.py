@@ -13,7 +13,7 @@ import torch.nn.functional as F
 
 import oracle
 from oracle import torch_spelling as TS
-from _util import codes_np, config1_inputs, from_bits16, from_bits32, max_rel, randn_cpu, u8
+from _util import captured_kernels, codes_np, config1_inputs, from_bits16, from_bits32, max_rel, randn_cpu, u8
 
 pytestmark = pytest.mark.gpu
 
@@ -695,8 +695,8 @@ def test_linear_of_few_rows_over_several_weights(Q):
 @pytest.mark.parametrize("M,K,N,split", [(8, 2048, 4096, 0), (4, 4112, 4096, 0), (9, 2064, 8192, 0), (16, 2048, 5008, 2),
                                          (16, 4096, 8192, 0), (15, 6160, 1024, 0), (13, 4096, 2048, 8)])
 def test_linear_whose_slices_look_at_their_own_columns(Q, dt, M, K, N, split):
-    """Above 32 KB and over sliced weights a CTA looks for the maximum of its own K slice and the slices exchange theirs:
-    the bits of quantizer and GEMM apart, on both sides of that line, K tails, 2, 4 and 8 slices, slices that fit the
+    """Above 32 KB (16 bits: 40 KB) and over sliced weights a CTA looks for the maximum of its own K slice and the slices exchange
+    theirs: the bits of quantizer and GEMM apart, on both sides of that line, K tails, 2, 4 and 8 slices, slices that fit the
     registers and that do not (from 40 KB), the largest value and a NaN in any slice, a residual, a replay."""
     fw = Q.quantize_weight(randn_cpu((N, K), seed=1, scale=0.02).cuda())
     res = randn_cpu((M, N), seed=2, dtype=dt).cuda()
@@ -723,6 +723,27 @@ def test_linear_whose_slices_look_at_their_own_columns(Q, dt, M, K, N, split):
     finally:
         Q.set_option("decode_quant_inside", -1)
         Q.set_option("decode_split_k", 0)
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt,M,K,N,own", [
+    (torch.bfloat16, 5, 4096, 8192, False), (torch.float16, 2, 9728, 5760, False), (torch.bfloat16, 4, 5136, 1024, True),
+    (torch.bfloat16, 4, 4096, 9728, False), (torch.float16, 4, 4112, 9728, True), (torch.float32, 2, 4096, 4096, False),
+    (torch.float32, 2, 4112, 8192, True), (torch.bfloat16, 6, 4096, 14336, False)])
+def test_own_slices_only_where_they_pay(Q, dt, M, K, N, own):
+    """Both sides of the lines at 32 KB (fp32, and 16 bits where two CTAs share an SM) and at 40 KB: which kernel is launched, and
+    the same bits.  A weight that is not sliced has no slices to look at."""
+    fw = Q.quantize_weight(randn_cpu((N, K), seed=1, scale=0.02).cuda())
+    x = randn_cpu((M, K), seed=M, dtype=dt).cuda()
+    try:
+        Q.set_option("decode_quant_inside", 262144)
+        assert torch.equal(Q.linear(x, fw), Q.fp8_matmul(*Q.quantize_act(x), fw, out_dtype=dt))
+        torch.cuda.synchronize()
+        (kernel,), _ = captured_kernels(lambda: Q.linear(x, fw))
+    finally:
+        Q.set_option("decode_quant_inside", -1)
+    # the kernel's last template argument: 1 looks at all of x, 3 at its own slice
+    assert ("Li3EEEv" if own else "Li1EEEv") in kernel["name"], kernel["name"]
     assert Q.device_status() == 0
 
 
