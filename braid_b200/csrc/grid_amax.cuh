@@ -83,9 +83,9 @@ struct RehearsingCta {
   }
 };
 
-// `cta.live` = false: this warp's own max without the exchange.
+// `cta.live` = false: this warp's own max without the exchange.  `late`: the ticket is drawn by grid_depart.
 template <typename Cta = WholeCta>
-__device__ __forceinline__ float grid_amax(float m, QuantWs* ws, unsigned int& ticket, const Cta& cta = Cta{}) {
+__device__ __forceinline__ float grid_amax(float m, QuantWs* ws, unsigned int& ticket, const Cta& cta = Cta{}, bool late = false) {
   __shared__ float s_warp_of[2][32];
   __shared__ float s_amax_of[2];
   float* const s_warp = s_warp_of[cta.slot()];
@@ -99,7 +99,7 @@ __device__ __forceinline__ float grid_amax(float m, QuantWs* ws, unsigned int& t
     if (lane == 0) {
       if (gridDim.x > 1 && cta.live) {
         w = exchange_max(w, &ws->amax_bits, gridDim.x, &ws->status);
-        ticket = exchange_leave(&ws->amax_bits);
+        if (!late) ticket = exchange_leave(&ws->amax_bits);
       }
       s_amax = w;
     }
@@ -168,7 +168,7 @@ __device__ __forceinline__ float cta_amax(float m) {
 // Column-parallel form: every CTA waits (bounded, thread 0 polls with a system-scope acquire)
 // until the arrival counter has advanced by `count` beyond *seen -- i.e. until every rank's push
 // launch has stored its share of the buffer this kernel is about to read.  *seen is advanced by
-// grid_wait_done() once every CTA has read it.
+// grid_depart once every CTA has read it for the last time.
 __device__ __forceinline__ void grid_wait_arrivals(const unsigned int* flag, const unsigned int* seen,
                                                    unsigned int count, QuantWs* ws) {
   if (threadIdx.x == 0) {
@@ -189,11 +189,12 @@ __device__ __forceinline__ void grid_wait_arrivals(const unsigned int* flag, con
   __syncthreads();
 }
 
-// Called by all threads when grid_amax is behind them, with the ticket it gave.
+// Called by all threads when grid_amax is behind them, with the ticket it gave; `late`: behind the last read of what was waited
+// for, so that the last one to leave knows that every CTA has read it, and the old *wait_seen.
 __device__ __forceinline__ void grid_depart(QuantWs* ws, unsigned int ticket, unsigned int* wait_seen = nullptr,
-                                            unsigned int wait_count = 0u) {
+                                            unsigned int wait_count = 0u, bool late = false) {
   if (threadIdx.x != 0) return;
-  // the last one to leave: every CTA has read the old value
+  if (late && gridDim.x > 1) ticket = exchange_leave(&ws->amax_bits);
   if ((gridDim.x == 1 || exchange_end(&ws->amax_bits, gridDim.x, ticket)) && wait_seen != nullptr) *wait_seen += wait_count;
 }
 

@@ -139,6 +139,8 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
   if (p.wait_flag != nullptr)
     grid_wait_arrivals(p.wait_flag, p.wait_seen, p.wait_count, static_cast<QuantWs*>(p.ws));
   const bool owns_tail = (MODE == kPlain) && p.tail != 0 && tid == nthreads - 1;
+  // what peers have stored is read twice (the register-held kernel has read it once when it takes its ticket)
+  auto late = [&] { return MODE == kPlain && PHASE == kBoth && p.wait_flag != nullptr; };
   float sc;
   unsigned int ticket = 0u;
   if constexpr (PHASE == kCastOnly) {
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
       for (unsigned int i = 0; i < p.tail; ++i)
         m = nan_max(m, fabsf(widen(__ldcg(src + i))));
     }
-    sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), ticket));
+    sc = scale_from_amax(grid_amax(m, static_cast<QuantWs*>(p.ws), ticket, WholeCta{}, late()));
     if (tid == 0) p.scale[0] = sc;
   }
   if constexpr (PHASE != kScaleOnly) {
@@ -206,8 +208,10 @@ __global__ void __launch_bounds__(512, 2) quant_stream_kernel(const QParams p) {
                                        __NV_SATFINITE, __NV_E4M3);
     }
   }
-  if constexpr (PHASE != kCastOnly)
-    grid_depart(static_cast<QuantWs*>(p.ws), ticket, p.wait_flag != nullptr ? p.wait_seen : nullptr, p.wait_count);
+  if constexpr (PHASE != kCastOnly) {
+    if (late()) __syncthreads();
+    grid_depart(static_cast<QuantWs*>(p.ws), ticket, p.wait_flag != nullptr ? p.wait_seen : nullptr, p.wait_count, late());
+  }
 }
 
 // Sticky status of the launches that run without scratch words from the caller (the cast half alone,

@@ -596,3 +596,18 @@ def test_launch_options_hold_for_decode_batches(Q, option, value, kernels):
         Q.set_option(option, default)
     assert [(k["ctas"], k["threads"], k["cluster"], programmatic) for k in found] == [kernels] * 2
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt,n", [(torch.bfloat16, 2048), (torch.bfloat16, 64 * 4096 + 3), (torch.bfloat16, 9_000_001), (torch.bfloat16, 9_800_005),
+                                  (torch.float16, 20_000_000), (torch.float32, 4_700_000), (torch.float32, 5_000_001)])
+def test_a_gathered_buffer_is_quantized_and_counted_as_seen(Q, dt, n):
+    """`quantize_act_after` with its arrivals in place: one CTA, values held in registers, and beyond (read twice, by the streaming
+    kernel); the codes of `quantize_act`, `seen` advanced once, the scratch clean for the next call."""
+    x = randn_cpu((n,), seed=n % 1000, dtype=dt, scale=1.7).cuda()
+    qr, sr = TS.quantize_act(x)
+    flag, seen = (torch.tensor([v], dtype=torch.int32, device="cuda") for v in (8, 5))
+    for count, total in ((3, 8), (2, 10)):
+        flag.fill_(total)
+        _assert_same(*Q.quantize_act_after(x, flag, seen, count), qr, sr, f"{dt} {n}")
+        assert seen.item() == total
+    assert Q.device_status() == 0
