@@ -13,7 +13,7 @@ import torch
 import torch.nn.functional as F
 
 from oracle import torch_spelling as TS
-from _util import randn_cpu, u8
+from _util import captured_kernels, randn_cpu, u8
 
 pytestmark = pytest.mark.gpu
 
@@ -437,6 +437,29 @@ def test_exchange_inside_a_cluster_equals_the_grid_wide_one(Q, dt, cols):
                     got.append([u8(a.dense), u8(a.q), u8(a.scale), u8(b.q), u8(b.scale), u8(c[0]), u8(c[1]), u8(d[0]), u8(d[1])])
                 for i, (p, q) in enumerate(zip(*got)):
                     assert torch.equal(p, q), f"{rows} x {cols}, peak {peak} {value}: output {i}"
+    assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("call,dt,rows,cols,ctas", [
+    ("norm", torch.bfloat16, 1, 4096, 0), ("norm", torch.bfloat16, 2, 4096, 2), ("norm", torch.bfloat16, 16, 8192, 16),
+    ("norm", torch.bfloat16, 17, 4096, 9), ("norm", torch.bfloat16, 27, 8192, 14), ("norm", torch.bfloat16, 33, 4096, 11),
+    ("norm", torch.float16, 48, 1024, 16), ("norm", torch.bfloat16, 49, 4096, 13), ("norm", torch.float16, 64, 512, 16),
+    ("norm", torch.bfloat16, 65, 4096, 0), ("norm", torch.bfloat16, 33, 5120, 0), ("norm", torch.float32, 16, 8192, 16),
+    ("norm", torch.float32, 17, 8192, 0), ("norm", torch.float32, 32, 4096, 16), ("norm", torch.float32, 33, 4096, 0),
+    ("norm", torch.float32, 64, 2048, 16), ("gated", torch.bfloat16, 16, 4096, 16), ("gated", torch.bfloat16, 32, 4096, 16),
+    ("gated", torch.float32, 17, 1024, 9), ("gated", torch.bfloat16, 33, 4096, 0), ("quantizer", torch.bfloat16, 1, 2048, 0),
+    ("quantizer", torch.bfloat16, 1, 2056, 2), ("quantizer", torch.bfloat16, 32, 4096, 16), ("quantizer", torch.bfloat16, 33, 4096, 0),
+    ("product", torch.float32, 27, 4096, 14), ("product", torch.bfloat16, 48, 4096, 0)])
+def test_where_the_exchange_stays_inside_a_cluster(Q, call, dt, rows, cols, ctas):
+    """The launch that a decode batch takes: one cluster of so many CTAs, or (0) a grid without one; by rows, width and type."""
+    x, z = (torch.randn(rows, cols, device="cuda").to(dt) for _ in range(2))
+    y, gamma, g128 = x.float(), _gamma(cols, 3), _gamma(128, 4)
+    run = {"norm": lambda: Q.rms_norm_quant(x, gamma, EPS), "gated": lambda: Q.gated_rms_norm_quant(y, z, g128, EPS, 128),
+           "quantizer": lambda: Q.quantize_act(x), "product": lambda: Q.sigmoid_gate_quant(x, z)}[call]
+    run()
+    torch.cuda.synchronize()
+    (kernel,), _ = captured_kernels(run)
+    assert kernel["cluster"] == ctas and (ctas == 0 or kernel["ctas"] == ctas), kernel
     assert Q.device_status() == 0
 
 

@@ -53,16 +53,23 @@ def test_ragged_small_and_streaming_sizes(Q, shape, dt):
 @pytest.mark.parametrize("dt,n", [(torch.bfloat16, 4_850_000 + 4099), (torch.bfloat16, 9_000_001),
                                   (torch.bfloat16, 20_000_003), (torch.bfloat16, 296 * 3 * 16384 + 8),
                                   (torch.bfloat16, 296 * 4 * 16384), (torch.float16, 7_777_777),
-                                  (torch.float32, 2_500_001), (torch.float32, 9_000_005)],
-                         ids=["bf16-8KB-chunks", "bf16-16KB-chunks", "bf16-refetch", "bf16-ring-full+1",
-                              "bf16-4-each", "fp16", "fp32-resident", "fp32-refetch"])
+                                  (torch.float32, 2_500_001), (torch.float32, 9_000_005),
+                                  (torch.bfloat16, 9_699_328 + 11), (torch.bfloat16, 12_000_007), (torch.float16, 9_699_328 + 9),
+                                  (torch.float16, 296 * 3 * 16384 + 13), (torch.float16, 20_000_003), (torch.float32, 4_849_664 + 9),
+                                  (torch.float32, 6_000_003), (torch.float32, 296 * 3 * 8192 + 12)],
+                         ids=["bf16-held-8", "bf16-held-16", "bf16-refetch", "bf16-ring-full+1",
+                              "bf16-4-each", "fp16-held-16", "fp32-held-8", "fp32-refetch", "bf16-first", "bf16-16KB-chunks",
+                              "fp16-first", "fp16-ring-full+1", "fp16-refetch", "fp32-first", "fp32-16KB-chunks", "fp32-ring-full+1"])
 def test_ragged_sizes_through_the_shared_memory_ring(Q, dt, n):
-    """Plain quantizer beyond the register-held regime: a ring of bulk copies per CTA (96 KB;
-    chunks of 8, 16 or 32 KB by input size).  Sizes where every chunk of a CTA stays in the ring
-    between the passes, where chunks are fetched again, where the ring is exactly full (three
-    32 KB chunks per CTA on 148 SMs), a short last chunk and a tail that is no whole group;
+    """Plain quantizer beyond the register-held regime (148 SMs: 9.7 M 16-bit values, 4.85 M of fp32; sizes below it are those of the
+    cast alone): a ring of bulk copies per CTA (96 KB; chunks of 16 or 32 KB by input size, of the cast alone 8 KB too).  The first size
+    that takes it, sizes where every chunk of a CTA stays in the ring between the passes, where chunks are fetched again,
+    where the ring is exactly full (three 32 KB chunks per CTA on 148 SMs), a short last chunk and a tail that is no whole group;
     the cast half alone at the same sizes; and the register-fed streaming kernel on the same
     input (option `quant_ring` off) gives the same bits."""
+    held = torch.cuda.get_device_properties(0).multi_processor_count * 512 * 64 * (1 if dt is torch.float32 else 2)
+    (kernel,), _ = captured_kernels(lambda x=torch.empty(n, dtype=dt, device="cuda"): Q.quantize_act(x))
+    assert ("quant_ring_kernel" in kernel["name"]) == (n >= held + 8), kernel["name"]
     x = randn_cpu((n,), seed=n % 1000, dtype=dt, scale=1.7).cuda()
     q, s = Q.quantize_act(x)
     qr, sr = TS.quantize_act(x)
