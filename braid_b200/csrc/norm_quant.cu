@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(kCastThreads) rmsnorm_cast_kernel(const NormPa
   bq::pdl_launch_dependents();
   const int row_groups = p.cols / kGroup;
   const int which = BESIDE ? threadIdx.x / row_groups : 0;
-  const int group = BESIDE ? threadIdx.x - which * row_groups : blockIdx.x * kCastThreads + threadIdx.x;
+  const int group = BESIDE ? threadIdx.x - which * row_groups : blockIdx.x * blockDim.x + threadIdx.x;
   const int slice = BESIDE ? blockIdx.y * p.beside + which : blockIdx.y;      // of the rows
   const int slices = BESIDE ? gridDim.y * p.beside : gridDim.y;
   const bool live = group < row_groups && (!BESIDE || which < p.beside);
@@ -1020,13 +1020,16 @@ int launch_rmsnorm_scale(const NormParams& p, cudaStream_t stream) {
 template <typename T, bool BESIDE>
 int launch_rmsnorm_cast_of(NormParams p, cudaStream_t stream) {
   int dev = 0, sms = 0;
-  const int per_sm = resident_per_sm(rmsnorm_cast_kernel<T, BESIDE>, kCastThreads, 0);
+  const int row_groups = p.cols / kGroup, columns = (row_groups + kCastThreads - 1) / kCastThreads;
+  // Wide rows: as many threads as their column blocks need, in whole warps; with 256 always, 2112 columns left half of them idle.
+  // us, 256 / so many: fp32 1776 x 2112 12.7 / 10.6, 9658 x 2560 41.7 / 35.3, bf16 9658 x 2560 35.9 / 30.1, 4000 x 4608 23.6 / 21.3.
+  const int threads = BESIDE ? kCastThreads : ((row_groups + columns - 1) / columns + 31) / 32 * 32;
+  const int per_sm = resident_per_sm(rmsnorm_cast_kernel<T, BESIDE>, threads, 0);
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1) {
     (void)cudaGetLastError();
     return bq::kErrLaunch;
   }
-  const int row_groups = p.cols / kGroup, columns = (row_groups + kCastThreads - 1) / kCastThreads;
   p.beside = 1;
   if (BESIDE) {
     const int once = (p.rows - 1) / (kCastRows * per_sm * sms) + 1;
@@ -1038,7 +1041,7 @@ int launch_rmsnorm_cast_of(NormParams p, cudaStream_t stream) {
   if (slices < 1) slices = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(columns), static_cast<unsigned>(slices), 1);
-  cfg.blockDim = dim3(kCastThreads, 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -496,3 +496,19 @@ def test_narrow_rows_cast_next_to_one_another(Q, dt, rows, cols):
     assert Q.launch_count() - n0 == 2
     _same(qa, TS.rms_norm(x, gamma, EPS), f"{rows} x {cols}")
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt,rows,cols,threads", [(torch.bfloat16, 3601, 1032, 160), (torch.float32, 1301, 2056, 160), (torch.float32, 1500, 2112, 160),
+                                                  (torch.float16, 2603, 4096, 256), (torch.float32, 1201, 4104, 192), (torch.bfloat16, 1301, 5120, 224),
+                                                  (torch.bfloat16, 1300, 6152, 224), (torch.float16, 1300, 8192, 256)])
+def test_wide_rows_cast_by_as_many_threads_as_their_columns_need(Q, dt, rows, cols, threads):
+    """One to four blocks of columns of a row, with threads for them in whole warps: the launch, and the bits, the last columns
+    included."""
+    x = randn_cpu((rows, cols), seed=rows, dtype=dt, scale=2.0).cuda()
+    gamma = _gamma(cols, 9, spread=0.3)
+    _same(Q.rms_norm_quant(x, gamma, EPS), TS.rms_norm(x, gamma, EPS), f"{rows} x {cols}")
+    torch.cuda.synchronize()
+    kernels, _ = captured_kernels(lambda: Q.rms_norm_quant(x, gamma, EPS))
+    (cast,) = [k for k in kernels if "rmsnorm_cast_kernel" in k["name"]]
+    assert cast["threads"] == threads
+    assert Q.device_status() == 0
