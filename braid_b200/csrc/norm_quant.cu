@@ -405,9 +405,16 @@ __device__ __forceinline__ void scale_norm(T (&v)[N], const float (&g)[N], float
   }
 }
 
-// DENSE: h is written, and nobody reads rstd.
-template <typename T, int VPT, bool DENSE>
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_scale_kernel(const NormParams p) {
+// DENSE: h is written, and nobody reads rstd.  WHOLE: are rows VPT whole vectors per thread (kAsk: asked here)?  Long rows of fp32 have a
+// kernel for either, since both loops in one cost the partial one a CTA per SM (six where they have 80 registers): h of 1776 x 5120
+// 18.7 -> 19.8 us.  Held to 80, the partial loop that writes h spills 480 bytes by itself and 16 beside the other one, so that is
+// its kernel; whole rows of 8192 want more (1776 x 8192 with 88 registers 31.1, with 80 36.1).
+enum Whole { kAsk = -1, kPartial = 0, kWhole = 1 };
+template <typename T, int VPT, bool DENSE> constexpr int kPartialKernel = sizeof(T) == 4 && VPT >= 8 && !(DENSE && VPT == 16) ? kPartial : kAsk;
+template <typename T, int VPT> constexpr int kWholeKernel = sizeof(T) == 4 && VPT >= 8 ? kWhole : kAsk;
+template <typename T, int VPT, int WHOLE> constexpr int kScalePerSm = sizeof(T) == 4 && VPT == 16 && WHOLE != kWhole ? 6 : 0;      // 0: as it comes
+template <typename T, int VPT, bool DENSE, int WHOLE>
+__global__ void __launch_bounds__(kNormThreads, kScalePerSm<T, VPT, WHOLE>) rmsnorm_scale_kernel(const NormParams p) {
   bq::pdl_launch_dependents();
   __shared__ float s_red_of[2][4];
   __shared__ float s_max[4];
@@ -489,7 +496,8 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_scale_kernel(const NormP
       }
     }
   };
-  if (n_vec == VPT * kNormThreads) walk(std::true_type{});
+  if constexpr (WHOLE != kAsk) walk(std::integral_constant<bool, WHOLE == kWhole>{});
+  else if (n_vec == VPT * kNormThreads) walk(std::true_type{});
   else walk(std::false_type{});
   float m = mx.value();
 #pragma unroll
@@ -995,6 +1003,14 @@ __global__ void __launch_bounds__(kGatedWarps * 32) gated_rmsnorm_scale_kernel(c
 }
 
 namespace {
+template <typename T, int VPT, bool DENSE>
+cudaError_t launch_rmsnorm_scale_of(const NormParams& p, int sms, size_t smem, cudaStream_t stream) {
+  auto launch = [&](auto whole) {
+    return launch_resident_smem(rmsnorm_scale_kernel<T, VPT, DENSE, decltype(whole)::value>, p.rows, kNormThreads, sms, true, smem, stream, p);
+  };
+  if (p.cols == VPT * kNormThreads * kVec) return launch(std::integral_constant<int, kWholeKernel<T, VPT>>{});
+  return launch(std::integral_constant<int, kPartialKernel<T, VPT, DENSE>>{});
+}
 template <typename T, bool DENSE>
 int launch_rmsnorm_scale(const NormParams& p, cudaStream_t stream) {
   int dev = 0, sms = 0;
@@ -1007,10 +1023,10 @@ int launch_rmsnorm_scale(const NormParams& p, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(p.cols) * sizeof(float);     // gamma
   if (smem > 48 * 1024) return bq::kErrUnsupported;
   cudaError_t e;
-  if (per_thread <= 2) e = launch_resident_smem(rmsnorm_scale_kernel<T, 2, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
-  else if (per_thread <= 4) e = launch_resident_smem(rmsnorm_scale_kernel<T, 4, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
-  else if (per_thread <= 8) e = launch_resident_smem(rmsnorm_scale_kernel<T, 8, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
-  else if (per_thread <= 16) e = launch_resident_smem(rmsnorm_scale_kernel<T, 16, DENSE>, p.rows, kNormThreads, sms, true, smem, stream, p);
+  if (per_thread <= 2) e = launch_rmsnorm_scale_of<T, 2, DENSE>(p, sms, smem, stream);
+  else if (per_thread <= 4) e = launch_rmsnorm_scale_of<T, 4, DENSE>(p, sms, smem, stream);
+  else if (per_thread <= 8) e = launch_rmsnorm_scale_of<T, 8, DENSE>(p, sms, smem, stream);
+  else if (per_thread <= 16) e = launch_rmsnorm_scale_of<T, 16, DENSE>(p, sms, smem, stream);
   else return bq::kErrUnsupported;
   if (e != cudaSuccess) { (void)cudaGetLastError(); return bq::kErrLaunch; }
   return bq::kOk;

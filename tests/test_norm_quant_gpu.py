@@ -512,3 +512,23 @@ def test_wide_rows_cast_by_as_many_threads_as_their_columns_need(Q, dt, rows, co
     (cast,) = [k for k in kernels if "rmsnorm_cast_kernel" in k["name"]]
     assert cast["threads"] == threads
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,vpt,whole", [(1301, 3072, 8, "Li0"), (1301, 4096, 8, "Li1"), (601, 4608, 16, None), (1777, 5120, 16, None),
+                                                 (601, 8192, 16, "Li1"), (601, 8188, 16, None)])
+def test_long_rows_of_fp32_take_the_kernel_of_their_width(Q, rows, cols, vpt, whole):
+    """Rows of as many vectors as a thread has room for, and shorter ones: which kernel finds the scale, with and without the dense
+    output, and the bits.  (None: the partial loop alone where h is not written, beside the whole one where it is.)"""
+    x = randn_cpu((rows, cols), seed=rows, dtype=torch.float32, scale=2.0).cuda()
+    gamma = _gamma(cols, 9, spread=0.3)
+    ref = TS.rms_norm(x, gamma, EPS)
+    for keep in (False, True):
+        qa = Q.rms_norm_quant(x, gamma, EPS, keep_dense=keep)
+        _same(qa, ref, f"{rows} x {cols}")
+        assert not keep or torch.equal(u8(qa.dense), u8(ref))
+        torch.cuda.synchronize()
+        kernels, _ = captured_kernels(lambda: Q.rms_norm_quant(x, gamma, EPS, keep_dense=keep))
+        dense = keep or cols % 8 != 0           # rows that are no whole 16-byte pieces of both types go through h
+        form = whole or ("Lin1" if dense else "Li0")
+        assert any(f"rmsnorm_scale_kernelIfLi{vpt}ELb{int(dense)}E{form}E" in k["name"] for k in kernels), kernels
+    assert Q.device_status() == 0
