@@ -259,12 +259,13 @@ __global__ void __launch_bounds__(with_rehearsal(R * G * kNormThreads)) rmsnorm_
 // arithmetic is that of rmsnorm_quant_kernel.  Gamma is in shared memory, not in registers, so that more rows are
 // resident at once, and a quarter or an eighth of the CTAs meet in the exchange (three atomics each on one word pair).
 // What bounds it are the rows' loads in flight, so the registers decide: held to 40 for a third CTA per SM, the compiler asks
-// for a row's vectors one after the other.  That form (PER_SM = 3) is taken where two CTAs per SM do not hold the rows.
-// One CTA per row / 40 registers / 64, us: 16-bit 512 x 4096 7.5 / 9.2 / 7.0, 768 x 4096 8.9 / 10.8 / 7.4, 1036 x 4096 - / 10.3 /
+// for a row's vectors one after the other; with two it takes the 47 to 50 that it wants.  The form of 40 (PER_SM = 3) is taken
+// where two CTAs per SM do not hold the rows.
+// One CTA per row / 40 registers / 50, us: 16-bit 512 x 4096 7.5 / 9.2 / 7.0, 768 x 4096 8.9 / 10.8 / 7.4, 1036 x 4096 - / 10.3 /
 // 7.5, 1500 x 4096 - / 10.5 / - (two rows per group 11.7); 600 x 1024 5.8 / 4.9 / 4.5.
 // Resident on 148 SMs: 16-bit rows of up to 2048 columns 3552, up to 4096 columns 2368, up to 8192 columns 1184; fp32
-// 3552 (1024 columns), 2368 (2048), 1184 (4096), longer ones never.  Beyond, the two launches: 2600 x 4096 bf16 12.7,
-// 1300 x 5120 bf16 10, 1300 x 4096 fp32 12.5.
+// 3552 (1024 columns), 2368 (2048), 1184 (4096), longer ones never.  Beyond, the two launches, from HBM: 2600 x 4096
+// bf16 14.5, 1300 x 5120 bf16 13.7, 1300 x 4096 fp32 13.9.
 // Of few rows a block has four to wait for where one would do.  One CTA per row and this, us: 16-bit 257 x 2048 4.8 and
 // 4.7, 333 x 4096 6.3 and 6.4, 413 x 4096 6.8 and 6.6, fp32 333 x 4096 6.3 and 6.3, 413 x 4096 6.7 and 6.6; bf16
 // 257 x 8192 8.5 and 8.7, 600 x 8192 9.8 and 11.1, 900 x 8192 12.3 and 11.5.
@@ -363,7 +364,8 @@ __global__ void __launch_bounds__(kRowGroups * kNormThreads, PER_SM) rmsnorm_row
 // max into one word with an atomicMax and counts itself, and the CTA that counts last turns the word into the scale and
 // returns the scratch to zero.  The second reads x again -- last rows first, of which L2 still has some -- normalises it once
 // more with the rstd found, and casts: 9658 x 4096 bf16 are 79 + 79 + 40 MB, where a first launch that writes h and a cast of
-// h move 79 + 79 + 79 + 40: 53.9 -> 39.7 us (fp32 85 -> 62).  Those (DENSE, 53.9 -> 44.4 with the loops below; bq_rmsnorm_scale and bq_cast_act) are what is left where h is wanted anyway.
+// h move 79 + 79 + 79 + 40: 53.9 -> 40.6 us (fp32 85 -> 61).  Those (DENSE, 45.9 with the loops below; bq_rmsnorm_scale and
+// bq_cast_act) are what is left where h is wanted anyway.
 // ---------------------------------------------------------------------------------------------
 // Running max |.| of values of T.
 template <typename T>
