@@ -100,6 +100,7 @@ struct PairSilu {
   unsigned int expected;   // CTAs that take part in the exchange (the active ones)
   const uint8_t* next;     // device: what the launch behind this one streams first, next_bytes of it (0: nothing)
   unsigned int next_bytes;
+  int next_warp;           // the warp of a CTA that asks for it
 };
 
 // Behind the last load of a gate/up launch HBM idles for its tail: the exchange, the cast, the start of the down projection.  One
@@ -108,9 +109,13 @@ struct PairSilu {
 // / 16 MB / 32 MB: 1 row 198.5 / 196.5 / 196.5 / 203.5 us, 8 rows 217.7 / 214.1 / 213.7 / 220.3, 16 rows 223.7 / 220.3 /
 // 219.9 / 225.8, 48 rows 251.2 / 249.0 / 250.6 / 255.0; before the exchange 8 MB give 217.1 at 8 rows and nothing at 27.  In pieces of
 // less than 1 KB, so that every CTA of the down projection gets its share, the instructions cost more than that (8 rows
-// 220 to 225).  A down weight of less than that loses (hidden 1024, 3 MB: 8 rows 103.3 and 105.4), and so does the kernel for
-// wider batches (64 rows 274.6 -> 278.3).
+// 220 to 225), and the kernel for wider batches loses (64 rows 274.6 -> 278.3).
+// It takes a down weight of 12 MB.  us of one MLP over cold weights, 16 rows, none / asked by warp 0 / by the last warp: 1792 x 5376 (9.6
+// MB) 13.1 / 14.7 / 13.6; 2048 x 6144 (12 MB) 14.7 / 15.6 / 15.1, but in graphed layers 127.0 / 125.7 / 124.1; 2304 x 6912 (15) 17.0 / 16.8 /
+// 16.6; 2560 x 7680 (19) 20.0 / 18.8 / 18.6; 3072 x 9216 (27) 23.4 / 22.2 / 22.3; 4096 x 12288 (48) 33.5 / 31.8 / 32.1.  The last warp has no
+// row to write where rows are few, which a short launch notices; a long one gains more by the first, which asks sooner.
 constexpr unsigned int kNextBytes = 8u << 20, kNextPiece = 4096;
+constexpr int64_t kNextFrom = 12 << 20, kNextFirstWarpFrom = 32 << 20;
 __device__ __forceinline__ void prefetch_next(const PairSilu& pr) {
   for (unsigned int at = (blockIdx.x * 32u + (threadIdx.x & 31u)) * kNextPiece; at < pr.next_bytes; at += gridDim.x * 32u * kNextPiece)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pr.next + at), "n"(kNextPiece) : "memory");
@@ -1086,7 +1091,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       }
     }
     __syncthreads();
-    if (EPI == kGateUp && warp == 0) prefetch_next(p.pair);
+    if (EPI == kGateUp && warp == p.pair.next_warp) prefetch_next(p.pair);
     const float sc = s_quant[0];
     if (ok) {
       const EpilogueArgs ea{part, smem_u32(part), 0, 0, m_begin, m_end, warp, lane, row0, 0.0f, true,
@@ -2933,7 +2938,8 @@ extern "C" int bq_lm_head_argmax(const void* xq, const void* wq, const float* sx
 namespace {
 void set_next(PairSilu* pair, const void* next, int64_t bytes) {
   pair->next = static_cast<const uint8_t*>(next);
-  pair->next_bytes = next != nullptr && bytes >= (int64_t)kNextBytes ? kNextBytes : 0u;
+  pair->next_bytes = next != nullptr && bytes >= kNextFrom ? kNextBytes : 0u;
+  pair->next_warp = bytes >= kNextFirstWarpFrom ? 0 : kStreamWarps - 1;
 }
 }  // namespace
 

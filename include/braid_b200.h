@@ -433,7 +433,7 @@ int bq_gate_up_silu_quant_w8a8(const void* xq, const float* sx, const void* wq_g
                                void* ws, size_t ws_bytes, void* stream);
 
 /* The same, with a hint: `next` (16-byte aligned, or NULL) is device memory of which the launch behind this one will stream
- * `next_bytes`, the down weight's codes: batches of up to 48 rows ask its first megabytes into L2 at their end.  Results do not
+ * `next_bytes`, the down weight's codes: batches of up to 48 rows ask its first 8 MB into L2 at their end, where it has 12.  Results do not
  * depend on it. */
 int bq_gate_up_silu_quant_next_w8a8(const void* xq, const float* sx, const void* wq_gate, const void* wq_up,
                                     const float* sw_gate, const float* sw_up, int64_t M, int64_t I, int64_t K, int act_dtype,

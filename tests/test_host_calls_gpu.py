@@ -235,3 +235,16 @@ def test_native_weight_quantizer_gives_the_same_weight(Q):
         assert torch.equal(Q.quantize_weight(t).data.view(torch.uint8), a.data.view(torch.uint8))
     with pytest.raises(ValueError):
         Q.quantize_weight(torch.randn(8, 16, device="cuda"))
+
+
+@pytest.mark.parametrize("H,I", [(1792, 5376), (2048, 6144), (3072, 9216), (3648, 9216)])
+def test_mlp_that_asks_the_down_weight_into_l2_gives_the_same_bits(Q, monkeypatch, H, I):
+    """The native MLP names the down weight to its gate/up launch, which asks 8 MB of it into L2 from 12 MB on, by the last warp and
+    from 32 MB on by the first; the Python code names nothing."""
+    g = torch.Generator(device="cuda").manual_seed(H)
+    gate, up, down = (Q.quantize_weight((torch.randn(n, k, generator=g, device="cuda") * 0.02).bfloat16())
+                      for n, k in ((I, H), (I, H), (H, I)))
+    for M in (1, 16, 48):
+        x = randn_cpu((M, H), seed=M).cuda()
+        _both(Q, monkeypatch, lambda: Q.mlp_forward(x, gate, up, down, residual=x))
+    assert Q.device_status() == 0
