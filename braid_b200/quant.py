@@ -1108,6 +1108,7 @@ def project(x: torch.Tensor, *weights: torch.Tensor | FP8Weight) -> list[torch.T
     `set_dense_segments(False)`) they take `F.linear`, as in the reference.
     """
     pre = x if isinstance(x, QuantizedActivation) else None
+    asked = False              # the native call, which would refuse a second time
     if pre is not None and _NATIVE is not None:
         # the plain case of a decoder: everything given, all members in one launch
         data, scales, sixteen_bit = [], [], 0
@@ -1120,6 +1121,7 @@ def project(x: torch.Tensor, *weights: torch.Tensor | FP8Weight) -> list[torch.T
                 scales.append(None)
                 sixteen_bit += 1
         if sixteen_bit == 0 or sixteen_bit < len(weights) and pre.dense is not None and _DENSE_SEGMENTS:
+            asked = True
             dense = pre.dense if sixteen_bit else None
             ys = _NATIVE.project(pre.q, pre.scale, dense, pre.dtype if dense is None else dense.dtype, tuple(data), tuple(scales))
             if ys is not None:
@@ -1135,14 +1137,14 @@ def project(x: torch.Tensor, *weights: torch.Tensor | FP8Weight) -> list[torch.T
         else:
             dense = x
             xq, sx = quantize_act(x.reshape(-1, K))
-        mixed = _project_native(xq, sx, dense, dense.dtype, weights, lead)
+        mixed = None if asked else _project_native(xq, sx, dense, dense.dtype, weights, lead)
         if mixed is None:
             mixed = _project_mixed(xq, sx, dense, weights, lead, K)
         if mixed is not None:
             return mixed
         pre = QuantizedActivation(xq, sx, x.shape, x.dtype, dense)     # do not quantize twice
     xq, sx = (pre.q, pre.scale) if pre is not None else quantize_act(x.reshape(-1, K))
-    if len(fp8) == len(weights):
+    if len(fp8) == len(weights) and not asked:
         ys = _project_native(xq, sx, None, x.dtype, weights, lead)
         if ys is not None:
             return ys

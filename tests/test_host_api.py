@@ -292,6 +292,25 @@ def test_mlp_whose_input_the_native_quantizer_refuses_takes_the_native_products(
     assert len(calls) == 3 and len(made) == 1
 
 
+def test_projections_that_the_native_call_refuses_are_offered_once(monkeypatch):
+    """An engine in fp32 keeps its gates as `F.linear`: the native call refuses the mixed set, and is not asked again."""
+    from braid_b200 import quant
+    calls = []
+
+    class Native:
+        def project(self, *args):
+            calls.append(args)
+
+    monkeypatch.setattr(quant, "_NATIVE", Native())
+    monkeypatch.setattr(quant, "_project_mixed", lambda *args: None)
+    monkeypatch.setattr(quant, "fp8_matmul_grouped", lambda xq, sx, ws, out_dtype: [torch.zeros(4, w.shape[0]) for w in ws])
+    w = quant.FP8Weight(torch.zeros(32, 32).to(quant.FP8), torch.ones(1, 1), (32, 32))
+    x = torch.zeros(4, 32)
+    pre = quant.QuantizedActivation(x.to(quant.FP8), torch.ones(1, 1), x.shape, x.dtype, x)
+    assert [y.shape for y in quant.project(pre, w, torch.zeros(8, 32))] == [(4, 32), (4, 8)] and len(calls) == 1
+    assert [y.shape for y in quant.project(pre, w, w)] == [(4, 32), (4, 32)] and len(calls) == 2
+
+
 def test_cpu_tensors_are_refused_not_emulated():
     from braid_b200 import quant
     x = torch.zeros(4, 16, dtype=torch.bfloat16)
